@@ -13,6 +13,7 @@
 // window may keep the sequence's first positions visible (mask_keep): the visible keys are then two ranges, [0, keep) and the
 // window, and the tiles of the gap between them are never staged. Value heads may be fewer than key heads (Gv < G: key head g
 // reads value head g mod Gv), which is how the two maps of differential attention share one set of values.
+// Prompt portions whose sizes allow it leave for attention_split.cu; decode steps, short portions and wide heads stay here.
 #include <math.h>
 
 #include "common.cuh"
@@ -466,6 +467,7 @@ int attn_bias_f32(const BiasAttnArgs& a, cudaStream_t st) {
     B2_TRY(check_args(a, "attn_bias"));
     B2_CHECK_ARG((a.out || a.out16) && (a.rel == nullptr || a.bucket_of != nullptr), "attn_bias: null argument");
     B2_CHECK_ARG(a.nsplit >= 1 && a.nsplit <= 64 && (a.nsplit == 1 || a.partial != nullptr), "attn_bias: 1..64 key splits, with scratch");
+    if (attn_split_fits(a)) return attn_split_f32(a, st);
     const int warps = a.rows * a.H;
     const bool vec = a.dk % 4 == 0 && (reinterpret_cast<uintptr_t>(a.kcache) & 15) == 0;
     const int HG = a.H / a.G;

@@ -585,8 +585,18 @@ struct BiasAttnArgs {
     float* partial = nullptr; int nsplit = 1;     // split-KV scratch [rows*H*nsplit*(dv+2)] when nsplit > 1
     int tile_rows = 0;                            // consecutive rows that share a slot (a prompt portion: its rows; a decode step: 1);
                                                   // 0: one warp per (row, head) without shared key/value tiles
+    // a prompt portion (tile_rows == rows) whose host side knows where it lies may run on the tensor cores (attention_split.cu): its slot, the
+    // slot's length behind it, and scratch for the bf16 parts of the keys and values that it sees (null: it stays on the fp32 pipe)
+    int slot = 0, key_end = 0;
+    void* parts = nullptr; size_t parts_bytes = 0;
 };
 int attn_prepare_f32(const BiasAttnArgs& a, cudaStream_t stream);  // q/k norms, temperature, cache append
+// Fewer keys take as long on the fp32 pipe, which starts faster (a layer's prompt of n tokens, fp32 pipe -> tensor cores, width 1024: n = 24
+// 107.9 -> 110.1 us, 32 109.6 -> 112.5, 48 115.5 -> 114.0, 96 131.6 -> 121.4); fewer rows leave a 128-pair tile mostly idle.
+constexpr int ATTN_SPLIT_MIN_ROWS = 16, ATTN_SPLIT_MIN_KEYS = 40;
+bool attn_split_fits(const BiasAttnArgs& a);                       // the call runs on the tensor cores
+size_t attn_split_bytes_per_key(int G, int Gv, int dk, int dv);    // scratch per visible key position
+int attn_split_f32(const BiasAttnArgs& a, cudaStream_t stream);
 int attn_bias_f32(const BiasAttnArgs& a, cudaStream_t stream);     // causal softmax attention of every row against its slot's cache
 
 }  // namespace b2

@@ -98,6 +98,7 @@ struct SeqState {
     DevBuf last_tok;                   // int32 [slots]: the token in front of the next one (hashed bigram embedding)
     DevBuf kmat, vmat;                 // latent attention, long prompt portions: per-head keys / values of one slot's positions [Smax][heads*size]
     int kmat_ld = 0, vmat_ld = 0;
+    DevBuf parts;                      // bf16 parts of the keys and values that a prompt portion sees (attention_split.cu)
     DevBuf attn_partial;
     int nsplit_max = 1;
 };
@@ -248,6 +249,13 @@ static void mask_of(const b2_seq_layer_desc& d, BiasAttnArgs& aa) {
     aa.mask_keep = d.mask_keep;
 }
 
+// a prompt portion (nseg == 1): where it lies, and the scratch with which its attention runs on the tensor cores
+static void portion_of(const SeqState& state, int nseg, int slot, int ctx_end, BiasAttnArgs& aa) {
+    if (nseg != 1 || ctx_end < aa.rows) return;
+    aa.slot = slot; aa.key_end = ctx_end;
+    aa.parts = state.parts.p; aa.parts_bytes = state.parts.bytes;
+}
+
 // Attention over a low-rank latent. S: the run's own state (rotation table); KS: the state whose cache rows it reads (its own,
 // or an earlier layer's). slot / ctx_end as for seq_forward.
 static int latent_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeights& W, SeqLayerState& S, SeqLayerState& KS, const float* h, float* target,
@@ -312,6 +320,7 @@ static int latent_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeight
         aa.kv_row_stride = state.kmat_ld; aa.kv_row_stride_v = state.vmat_ld;
         aa.out = y; aa.ldo = L.pv;
         aa.G = H; aa.dk = qh; aa.dv = dv; aa.nsplit = 1;
+        portion_of(state, nseg, slot, ctx_end, aa);
         B2_TRY(attn_bias_f32(aa, st));
     } else {
         // absorbed form: q_h -> W_uk_h^T q_h lives in the latent space (the rotated part rides behind it), so scores and values
@@ -359,7 +368,7 @@ static int latent_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeight
 // per head. With two maps (differential attention) the projection rows were ordered [map][head][dim] when the tensors were set, so the
 // maps are simply twice the query and key heads over the same value heads, and a head's two outputs are joined after the softmax.
 static int gqa_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeights& W, SeqLayerState& S, const SubIn& in, float* target, float alpha,
-                     int accumulate, int R, int nseg, cudaStream_t st) {
+                     int accumulate, int R, int nseg, int slot, int ctx_end, cudaStream_t st) {
     SeqModel& s = *m->seq;
     SeqState& state = *kv->seq;
     const b2_seq_layer_desc& d = L.d;
@@ -415,6 +424,7 @@ static int gqa_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeights& 
     if (chan_in_attn) { aa.chan_gate = gates; aa.ldg = L.lproj_ld; }
     const bool out16 = maps == 1 && !d.ga_rot_values && lin.tensor_cores(width, L.ng, target, width, R);
     if (out16) aa.out16 = s.a16.p;
+    portion_of(state, nseg, slot, ctx_end, aa);
     B2_TRY(attn_bias_f32(aa, st));
     if (out16) return lin(nullptr, 0, W.o_w, width, L.ng, target, width, R, LIN_NONE, alpha, accumulate, nullptr, 0, nullptr, s.a16.p);
     const float* yo = s.y.as<float>();
@@ -840,7 +850,7 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
                     SeqLayerState& KS = d.la_kv_from > 0 ? state.layer[s.runs[ri].kv_run] : S;
                     B2_TRY(latent_mixer(m, kv, L, W, S, KS, in1.h, x, rm, 1, R, nseg, slot, ctx_end, st));
                 } else if (d.type == B2_MIXER_GQA_ATTN) {
-                    B2_TRY(gqa_mixer(m, kv, L, W, S, in1, x, rm, 1, R, nseg, st));
+                    B2_TRY(gqa_mixer(m, kv, L, W, S, in1, x, rm, 1, R, nseg, slot, ctx_end, st));
                 } else if (d.type == B2_MIXER_MLSTM || d.type == B2_MIXER_DELTA) {
                     B2_TRY(memory_mixer(m, L, W, S, in1, x, rm, 1, R, nseg, st));
                 } else if (d.type == B2_MIXER_GLA) {
@@ -860,7 +870,7 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
                 SeqLayerState& KS = d.la_kv_from > 0 ? state.layer[s.runs[ri].kv_run] : S;
                 B2_TRY(latent_mixer(m, kv, L, W, S, KS, h, target, alpha, acc, R, nseg, slot, ctx_end, st));
             } else if (d.type == B2_MIXER_GQA_ATTN) {
-                B2_TRY(gqa_mixer(m, kv, L, W, S, h, target, alpha, acc, R, nseg, st));
+                B2_TRY(gqa_mixer(m, kv, L, W, S, h, target, alpha, acc, R, nseg, slot, ctx_end, st));
             } else if (d.type == B2_MIXER_GLA) {
                 B2_TRY(gla_mixer(m, L, W, S, h, target, alpha, acc, R, nseg, st));
             } else {
@@ -925,6 +935,7 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
             aa.tile_rows = max_n;
             if (aa.nsplit > state.nsplit_max) aa.nsplit = state.nsplit_max;
             aa.partial = state.attn_partial.as<float>();
+            portion_of(state, nseg, slot, ctx_end, aa);
             B2_TRY(attn_prepare_f32(aa, st));
             B2_TRY(attn_bias_f32(aa, st));
             B2_TRY(sigmoid_gate_f32(s.y.as<float>(), L.ng, proj + L.nq + L.nk + L.nv, L.lproj_ld, s.gated.as<float>(), L.ng, R, L.ng, st));
@@ -1708,6 +1719,17 @@ int seq_kv_alloc(b2_kv* kv) {
         B2_TRY(kv->seq->kmat.alloc(Smax * kw * F4));
         B2_TRY(kv->seq->vmat.alloc(Smax * vw * F4));
     }
+    {   // bf16 parts of what a prompt portion sees, at most PARTS_MAX: a portion that sees more keys stays on the fp32 pipe
+        size_t per_key = 0;
+        for (const SeqLayerInfo& L : s.layers) {
+            const b2_seq_layer_desc& d = L.d;
+            if (d.type == B2_MIXER_LATENT_ATTN) per_key = std::max(per_key, attn_split_bytes_per_key(d.la_heads, d.la_heads, d.la_dim + d.la_rot_dim, d.la_vdim));
+            else if (d.type == B2_MIXER_GQA_ATTN) per_key = std::max(per_key, attn_split_bytes_per_key(L.maps * d.ga_kv_heads, d.ga_kv_heads, d.ga_dim, d.ga_vdim));
+            else if (d.type == B2_MIXER_PARALLEL) per_key = std::max(per_key, attn_split_bytes_per_key(d.a_kv_heads, d.a_kv_heads, d.a_dim, d.a_vdim));
+        }
+        const size_t PARTS_MAX = (size_t)256 << 20;
+        if (per_key > 0) B2_TRY(kv->seq->parts.alloc(std::min(Smax * per_key, PARTS_MAX)));
+    }
     kv->seq->nsplit_max = 64;
     B2_TRY(kv->seq->attn_partial.alloc((size_t)8 * maxH * kv->seq->nsplit_max * (maxdv + 2) * F4));
     return 0;
@@ -1722,6 +1744,7 @@ void seq_kv_free(b2_kv* kv) {
     kv->seq->last_tok.free();
     kv->seq->kmat.free();
     kv->seq->vmat.free();
+    kv->seq->parts.free();
     kv->seq->attn_partial.free();
     delete kv->seq;
     kv->seq = nullptr;

@@ -1,0 +1,55 @@
+"""Prompt attention on the tensor cores (csrc/attention_split.cu) against the plain oracle: one attention layer in true fp32, at the edges of its
+key tiles (64, or 32 for keys above 128), query tiles (128 (row, head) pairs) and head slabs (64 entries), in one piece and in portions whose
+windows, kept positions and chunks start inside the cache; and the sizes next to those that stay on the fp32 pipe."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import sofopel_oracle as O
+from test_sofopel_gpu import build, config, diff, tokens_for, win
+
+pytestmark = pytest.mark.gpu
+
+MLP = {"kind": "dense", "ff": 8, "limit": 7.0}
+# Projections, scores and output are sums of at most 256 fp32 terms: about 2^-24 sqrt(256 / 2) = 7e-7 of their result each (2-norm), three in a row
+BOUND = 2.1e-6
+
+
+def check(mixer, portions, seed=0):
+    cfg = config([dict(mixer, mlp=MLP)], width=64, vocab=90, mult=1.0)
+    n = sum(portions)
+    model, w = build(cfg, torch.float32, seed=seed, max_batch=2, max_seq=n + 3, max_rows=max(portions))
+    toks = tokens_for(cfg, n, seed + 1)
+    eng = model._ensure_engine()
+    kv, got, at = eng.new_kv(2, n + 3), [], 0
+    for p in portions:
+        got.append(eng.append_tokens(kv, 1, toks[at:at + p], restart=at == 0, residuals=True)[1][0])
+        at += p
+    got = torch.cat(got).double().cpu().numpy()
+    ref = O.forward(cfg, w, toks, return_layers=True)[1][0]
+    add = ref - np.asarray(w["embed"], np.float64)[toks] * cfg["embedding"]["scale"]   # what the layer adds
+    model.invalidate_engine()
+    err = np.linalg.norm(got - ref) / np.linalg.norm(add)
+    assert err <= BOUND, (mixer, portions, err)
+
+
+@pytest.mark.parametrize("n", [15, 16, 31, 33, 63, 64, 65, 128, 129])
+def test_edges_of_key_and_query_tiles(n):
+    check(win(4, 1, 128, 128, None, None, 64), [n])
+
+
+@pytest.mark.parametrize("heads,kv,dim,vdim", [(1, 1, 64, 64), (2, 2, 65, 65), (3, 1, 192, 128), (5, 5, 8, 4), (6, 2, 129, 61), (7, 1, 30, 127), (2, 1, 193, 128), (2, 1, 128, 129)])
+def test_head_sizes_and_groups(heads, kv, dim, vdim):
+    check(win(heads, kv, dim, vdim, 40, 3, dim // 4 * 2), [70])
+
+
+@pytest.mark.parametrize("size,keep", [(1, 1), (7, 0), (64, 5), (30, 100), (50, 64)])
+@pytest.mark.parametrize("portions", [[150], [40, 17, 70, 16, 7], [100, 33]])
+def test_windows_and_kept_positions(size, keep, portions):
+    check(win(4, 2, 24, 40, size, keep, 8), portions)
+
+
+@pytest.mark.parametrize("chunk", [1, 16, 64, 100])
+@pytest.mark.parametrize("portions", [[150], [20, 60, 16, 41]])
+def test_two_maps_in_chunks(chunk, portions):
+    check(diff(4, 2, 64, 72, 3, chunk, 32), portions)
