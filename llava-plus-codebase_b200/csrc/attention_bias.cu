@@ -387,6 +387,7 @@ __global__ void __launch_bounds__(TL_WARPS * 32, MAXC == 16 ? 1 : 2) attn_tile_k
 // one block per (row, head): every thread turns the splits' (max, sum) into weights (nsplit <= 64 values from L1) and combines
 // its value columns in split order
 __global__ void __launch_bounds__(512) attn_merge_kernel(BiasAttnArgs a) {
+    pdl_trigger_small();
     const int w = blockIdx.x;
     const int r = w / a.H, h = w % a.H;
     if (a.row_pos[r] < 0) return;

@@ -57,6 +57,12 @@ extern unsigned long long g_launch_count;  // kernels launched by this library (
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// For small launches only (a decode step's): behind a grid of several waves the next kernel's CTAs would take SMs from its last ones
+// (a prompt of 1900 tokens through a gated-linear-attention layer: 988 -> 997 us with unconditional triggers in its casts, gates and norms).
+__device__ __forceinline__ void pdl_trigger_small() {
+    if (gridDim.x * gridDim.y * gridDim.z <= 512) pdl_trigger();
+}
+
 bool pdl_enabled();  // B2_PDL=0 turns the launch attribute off (A/B runs)
 
 // ----------------------------------------------------------------------------------------------
@@ -80,6 +86,12 @@ __device__ __forceinline__ void epi_post8(float (&x)[8], const float* op, int po
         const float4 a = *reinterpret_cast<const float4*>(op), b = *reinterpret_cast<const float4*>(op + 4);
         x[0] += a.x; x[1] += a.y; x[2] += a.z; x[3] += a.w; x[4] += b.x; x[5] += b.y; x[6] += b.z; x[7] += b.w;
     }
+}
+
+// the fp32 epilogue of the row Linears: *o = alpha * act(acc + bias[n]) (+ *o); act: LIN_* of kernels.h
+__device__ __forceinline__ void linear_store(float* o, float acc, const float* bias, int n, int act, float alpha, int accumulate) {
+    float v = alpha * epi_post_act(acc + (bias != nullptr ? bias[n] : 0.f), act);
+    *o = accumulate ? (*o + v) : v;
 }
 
 template <typename... KArgs, typename... Args>

@@ -287,7 +287,12 @@ struct LinearArgs {
     int accumulate = 0;
     int round_a = 0;                             // round A to bf16 first (bf16 compute: the product is bf16 x bf16 -> fp32)
     DytNorm norm;                                // norm.alpha non-null: A passes this norm while it is staged (linear_fuses_norm calls only)
+    const void* A16 = nullptr;                   // the same rows already rounded to bf16, pitch K (linear_stream_f32 reads these when there are 2 or more)
 };
+// A handful of rows on bf16 weights (linear_stream.cu): whether a call is one of those that stream their weights through registers
+constexpr int LINEAR_STREAM_MAX = 16;
+bool linear_streams(const LinearArgs& a);
+int linear_stream_f32(const LinearArgs& a, cudaStream_t stream);
 // whether a call of these sizes can norm A on its way in: a handful of rows with K % 8 == 0 (the weight-streaming kernel)
 bool linear_fuses_norm(int M, int K);
 int linear_f32(const LinearArgs& a, cudaStream_t stream);

@@ -406,6 +406,7 @@ __global__ void __launch_bounds__(256) linear_grouped_tiled_kernel(GroupedLinear
 template <typename TW, bool VEC>
 __global__ void __launch_bounds__(256) linear_grouped_rows_kernel(GroupedLinearArgs g) {
     const int m = blockIdx.y;
+    pdl_trigger();
     const int grp = g.tile_group[m];
     if (grp < 0) return;
     const int src = g.a_rows != nullptr ? g.a_rows[m] : m / g.a_div;

@@ -133,6 +133,7 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int32_t* __restric
 // out[r, c] = act(in[r, c], in[r, ff + c]): the gated unit (SiLU(g) u, or its bounded and shifted form)
 __global__ void glu_rows_kernel(const float* __restrict__ in, int64_t ld_in, float* __restrict__ out, int64_t ld_out, int ff,
                                 __nv_bfloat16* __restrict__ out16, int64_t ld_out16, GluAct act) {
+    pdl_trigger_small();
     const size_t r = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < ff) {

@@ -69,6 +69,7 @@ __global__ void gated_group_rmsnorm_kernel(const float* __restrict__ y, int64_t 
                                            const float* __restrict__ gamma, float* __restrict__ out, int64_t ldo, int rows, int groups, int group,
                                            int gate_first, int gamma_shared, float eps, int sigmoid_gate, const float* __restrict__ den,
                                            __nv_bfloat16* __restrict__ out16, int64_t ldo16) {
+    pdl_trigger_small();
     const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (w >= rows * groups) return;
     const int r = w / groups, g = w % groups;
@@ -144,6 +145,7 @@ __global__ void __launch_bounds__(256) concat_rows_kernel(const float* __restric
 // the difference to unit RMS
 __global__ void diff_combine_kernel(const float* __restrict__ y, int64_t ldy, float* __restrict__ out, int64_t ldo, int rows, int heads, int dv,
                                     float lambda, float out_scale, float eps) {
+    pdl_trigger_small();
     const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (w >= rows * heads) return;
     const int r = w / heads, h = w % heads;
@@ -224,6 +226,7 @@ __global__ void __launch_bounds__(256) rms_weight_reg_kernel(const float* in, in
                                                              const float* __restrict__ w, float* out, int64_t ld_out, int accumulate, int cols, float eps,
                                                              __nv_bfloat16* __restrict__ out16) {
     __shared__ float red[33];
+    pdl_trigger_small();
     const size_t r = blockIdx.x;
     const float* xr = in + (row_index != nullptr ? (size_t)row_index[r] : r) * ld_in;
     float4 x[V], g[V];

@@ -192,6 +192,8 @@ struct Lin {  // one Linear call on the model's compute dtype
         a.bias = bias; a.out = out; a.ld_out = ldo; a.M = M; a.N = N; a.K = K; a.act = act; a.alpha = alpha; a.accumulate = accumulate;
         a.round_a = s.d.compute == B2_COMPUTE_BF16;
         if (norm != nullptr) a.norm = *norm;
+        a.A16 = a16;
+        if ((M == 1 || tc_enabled()) && linear_streams(a)) return linear_stream_f32(a, st);
         // bf16 compute, a portion of a prompt: the tcgen05 GEMM on a bf16 copy of A (weights are stored with their rows
         // padded to a multiple of 8, zero-filled, so N rounds up; the pitch of every projection buffer is a multiple of 8)
         const int Np = (N + 7) / 8 * 8;
@@ -548,7 +550,7 @@ static int memory_mixer(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, SeqLa
 // W_down gelu(W_up h) in two steps, so that a parallel block can take the first product before anything joins the residual stream it reads.
 // On the tensor cores the first product's epilogue activates and writes the bf16 rows that the second one reads.
 static bool gelu_on_tensor_cores(const SeqModel& s, const Lin& lin, int ff, float* target, int R) {
-    return ff % 8 == 0 && s.f16.p != nullptr && lin.tensor_cores(ff, s.d.width, s.ff.as<float>(), (ff + 7) / 8 * 8, R) && lin.tensor_cores(s.d.width, ff, target, s.d.width, R);
+    return R > LINEAR_STREAM_MAX && ff % 8 == 0 && s.f16.p != nullptr && lin.tensor_cores(ff, s.d.width, s.ff.as<float>(), (ff + 7) / 8 * 8, R) && lin.tensor_cores(s.d.width, ff, target, s.d.width, R);
 }
 static int gelu_up(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, const SubIn& in, float* target, int R, cudaStream_t st) {
     SeqModel& s = *m->seq;
