@@ -687,6 +687,7 @@ int gemm_bf16(const GemmArgs& g, cudaStream_t stream) {
     const bool grouped = g.tile_group != nullptr;
     B2_CHECK_ARG(!grouped || (g.groups >= 1 && g.act == ACT_NONE && g.bias == nullptr && g.residual == nullptr && g.M % BM == 0),
                  "gemm: a grouped product takes whole tiles of %d rows, no bias, residual or fused activation", BM);
+    if (g.bn_override >= 1000 && !grouped) return gemm_bf16_splitk(g, g.bn_override % 1000, g.bn_override / 1000, stream);
     if (g.bn_override == 2 && !grouped) return gemm_bf16_2cta(g, stream);  // CTA-pair kernel (cta_group::2, 256x256 pair tiles)
 
     // Tile-N choice. Cost model fitted to profiles/r1b_gemm_sweep.json: a tile costs ~BN / rel(BN) (rel = tensor-pipe
@@ -710,13 +711,31 @@ int gemm_bf16(const GemmArgs& g, cudaStream_t stream) {
             const float cost = (float)waves * ((float)cand[i] / rel[i] + 24.f /*per-tile fixed cost*/);
             if (best == 0.f || cost < best) { best = cost; bn = cand[i]; }
         }
+        // K cut over a cluster of S CTAs, where its tiles then still fit the SMs at once. Measured (M = 64, weights from DRAM): N = 2048,
+        // K = 5120 23.0 us on 32 SMs, 15.5 / 11.4 us with S = 2 / 4; N = 4096, K = 11008 46.4 -> 21.6; M = 577, N = 1024, K = 4096 19.5 ->
+        // 15.1. An SM takes a k-block of 24-32 KB in 0.2 us whatever the width; meeting costs about 1.5 us, i.e. 1154 / k-blocks in
+        // this model's units. Clusters of 8 were slower throughout (19.6 us at N = 2048, K = 5120): few GPCs hold two of them, and 32 is how
+        // many clusters of 4 they hold.
+        int split_bn = 0, split_s = 0;
+        float split_best = 0.f;
+        const int kb = (g.K + BK - 1) / BK;
+        if (g.bn_override == 0 && !grouped && g.act != ACT_SWIGLU) {
+            for (int c = 2; c < 4; ++c)
+                for (int s = 2; s <= 4; s *= 2) {
+                    const long long ctas = (long long)num_m * ((g.N + cand[c] - 1) / cand[c]) * s;
+                    if (ctas > (s == 2 ? num_sms() : 128) || kb < 4 * s) continue;
+                    const float cost = (float)cand[c] / rel[c] / s + 24.f + 1154.f / kb;
+                    if (split_bn == 0 || cost < split_best) { split_best = cost; split_bn = cand[c]; split_s = s; }
+                }
+        }
         if (g.bn_override == 0 && g.M >= 512 && g.N >= 256 && !grouped) {
             const long long pairs = (long long)((g.M + 255) / 256) * ((g.N + 255) / 256);
             const long long pair_slots = num_sms() / 2;
             const long long waves = (pairs + pair_slots - 1) / pair_slots;
             const float cost = (float)waves * (256.f / 1.08f + 24.f);
-            if (cost < best) return gemm_bf16_2cta(g, stream);
+            if (cost < best && (split_bn == 0 || cost < split_best)) return gemm_bf16_2cta(g, stream);
         }
+        if (split_bn != 0 && split_best < best) return gemm_bf16_splitk(g, split_bn, split_s, stream);
     }
     if (g.bn_override == 64 || g.bn_override == 128 || g.bn_override == 192 || g.bn_override == 256) bn = g.bn_override;
     if (g.act == ACT_SWIGLU && bn % 128 != 0) bn = 128;
