@@ -533,7 +533,10 @@ struct ScanArgs {
     float* y = nullptr; int64_t ldy = 0;                                  // [rows, heads*dv]
     int heads = 0, groups = 0, dk = 0, dv = 0;
     const SeqSeg* segs = nullptr; int nseg = 0;
+    int rows = 0;                                                         // tokens of the one segment (nseg == 1); with the scratch (floats, see below) a long
+    float* chunk_scratch = nullptr; size_t chunk_floats = 0;              // prompt is walked in chunks side by side
 };
+size_t linear_scan_scratch_floats(int heads, int dk, int dv);
 int linear_scan_f32(const ScanArgs& a, cudaStream_t stream);
 
 // ---- matrix memories with one decay per head (matrix_memory.cu) ------------------------------------------------------------------

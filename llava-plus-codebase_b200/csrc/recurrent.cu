@@ -3,7 +3,7 @@
 // serves a portion of a prompt (n rows of one slot) and a decode step (one row of each of B slots): the rows come as
 // segments (kernels.h, SeqSeg). State, decays, step sizes and sums are fp32; a segment whose pos0 is 0 starts from zero
 // state whatever its slot held before, so a slot that is handed to a new request needs no clearing.
-#include <stdlib.h>
+#include <algorithm>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -132,170 +132,304 @@ __global__ void __launch_bounds__(128) token_shift_carry_kernel(const float* __r
 }
 
 // ---- linear recurrence ------------------------------------------------------------------------------------------------
-// Block = 32 value columns (threadIdx.x) x KS key slices (threadIdx.y) of one head of one segment. A thread keeps KPT keys
-// of its column's state in registers. Tokens are staged TT at a time into shared memory with the per-token preparation done
-// while staging (step size, decay, dt-scaled key), then walked in order with no barrier in between: the recurrence lives in
-// registers, and the KS partial dot products of the tile's tokens meet in shared memory once per tile.
-constexpr int TT = 16;   // KPT (template): keys of the state a thread keeps, 16, or 8 for key sizes <= 128 (twice the warps per CTA)
+// S <- D S + k v^T, y = S^T q per head, D diagonal (one decay per key, or one per token), S and all sums fp32.
+// A warp holds 64 keys x 16 columns of a head's state in registers, a lane 8 keys x 4 columns, so that a token costs a lane seven 16-byte reads
+// of shared memory for its 96 multiply-adds; a CTA takes all keys (KW warps) of 64 columns (4 warps). Tokens come in tiles of SC_TT through
+// two buffers (cp.async), the raw gates are turned into (q, k, decay) once per tile, the lanes' and warps' shares of y meet per token by
+// shuffles and per tile in shared memory.
+// A long prompt has few (head, column) CTAs and a long chain of tokens, so it is cut into chunks that run side by side, exactly (no decay is
+// divided by): a first launch walks every chunk from an empty state (the first one from the slot's state, with its outputs) and leaves the
+// chunk's final state and the product of its decays per key; a second launch starts each further chunk from what those fold to, S_c = P_c S_(c-1)
+// + L_c, and writes its outputs. The chain is then 2 / C of the tokens for 5/3 of the arithmetic.
+// 1900 tokens, 8 heads of 128 x 256 (gated linear attention): 625 -> 191 us (two walks of 90 us, 11 us for the gates beforehand; before, 8 keys x
+// one column per thread and one chain). Issue slots bound a walk (65 % with the gates' arithmetic in it: 291 us for both, hence
+// scan_prepare_kernel), then the multiply-add pipe. 600 tokens, 32 heads of 128 x 64 (state space): 152 -> 84 us, 16 heads of 64 x 64 (RWKV) 128 -> 58.
+constexpr int SC_TT = 16, SC_COLS = 64, SC_MAX_CHUNKS = 10;
 
-template <int MODE, int KPT>
-__global__ void __launch_bounds__(512) linear_scan_kernel(ScanArgs a) {
-    extern __shared__ float sm[];
-    const SeqSeg sg = a.segs[blockIdx.z];
-    if (sg.n <= 0) return;
-    const int h = blockIdx.y, j = blockIdx.x * 32 + threadIdx.x, ks = threadIdx.y, KS = blockDim.y;
-    const int dk = a.dk, dv = a.dv, dkp = KS * KPT;
-    const int tid = threadIdx.y * 32 + threadIdx.x, nthr = KS * 32;
-    float* sQ = sm;                    // [TT][dkp]
-    float* sK = sQ + TT * dkp;         // [TT][dkp]
-    float* sD = sK + TT * dkp;         // [TT][dkp] decay per key channel
-    float* sV = sD + TT * dkp;         // [TT][32]
-    float* sR = sV + TT * 32;          // [TT][KS][32] partial outputs of a tile
-    const int g = MODE == SCAN_SSD ? h / (a.heads / a.groups) : h;  // SCAN_HGRN2 has no key input: a.k is not read
-    const bool col_ok = j < dv;
-    float S[KPT], bon[KPT];
-    float* st = a.state + (((size_t)sg.slot * a.heads + h) * dk) * dv;
+struct ScanPlan {
+    int chunks = 1, len = 0;       // chunks of `len` tokens (1: the whole segment, whatever its length)
+    int z0 = 0;                    // chunk of blockIdx.z == 0
+    int second = 0;                // the launch that starts from folded states
+    int prepared = 0;              // scan_prepare_kernel has made (q, decay) of the raw gates
+    float *final_state = nullptr, *decays = nullptr;   // [chunk][head][dk][dv], [chunk][head][dk]
+};
+
+__device__ __forceinline__ void scan_cp16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void scan_cp4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+// The gates' arithmetic, on a query and a raw decay entry of key `key` of head h (SSD, one decay per token, has its own): the forget gate bounded
+// below f = l + (1 - l) sigmoid(z + b) (HGRN2: what is forgotten, 1 - f, is what is written), sigmoid(z + b)^(1 / tau) = exp(log_sigmoid(z + b) /
+// tau) with log_sigmoid(u) = min(u, 0) - log1p(exp(-|u|)) (GLA), exp(-exp(z)) (RWKV).
+template <int MODE>
+__device__ __forceinline__ float scan_decay(const ScanArgs& a, int at, float z) {   // at = h * dk + key
+    if (MODE == SCAN_HGRN2) {
+        const float low = a.gate_lower[at];
+        return fmaf(1.f - low, 1.f / (1.f + expf(-(z + a.gate_bias[at]))), low);
+    }
+    if (MODE == SCAN_GLA) {
+        const float u = z + a.gate_bias[at];
+        return expf((fminf(u, 0.f) - log1pf(expf(-fabsf(u)))) / a.tau);
+    }
+    return expf(-expf(z));
+}
+template <int MODE>
+__device__ __forceinline__ float scan_query(const ScanArgs& a, float q) { return MODE == SCAN_HGRN2 ? silu_f(q) : MODE == SCAN_GLA ? q * a.q_scale : q; }
+// ... in place over a long prompt's rows (workspaces of the call), where every column block of both launches would redo it
+template <int MODE>
+__global__ void __launch_bounds__(256) scan_prepare_kernel(ScanArgs a) {
+    const int c = blockIdx.x * 256 + threadIdx.x;
+    const size_t r = (size_t)a.segs[0].row0 + blockIdx.y;
+    if (c >= a.heads * a.dk) return;
+    float* d = const_cast<float*>(a.decay_in) + r * a.ldd + c;
+    *d = scan_decay<MODE>(a, c, *d);
+    if (MODE != SCAN_RWKV) {
+        float* q = const_cast<float*>(a.q) + r * a.ldq + c;
+        *q = scan_query<MODE>(a, *q);
+    }
+}
+
+// KW: warps over the keys (64 each); V16: every operand row is 16-byte aligned with sizes in whole fours
+template <int MODE, int KW, bool V16>
+__global__ void __launch_bounds__(KW * 128, KW == 4 ? 1 : 2) linear_scan_kernel(ScanArgs a, ScanPlan p) {
+    constexpr int DKP = KW * 64, NTHR = KW * 128;
+    constexpr bool PER_KEY = MODE != SCAN_SSD, HAS_K = MODE != SCAN_HGRN2;
+    extern __shared__ __align__(16) float sm[];
+    float* sQ = sm;                                  // [2][TT][DKP]
+    float* sD = sQ + 2 * SC_TT * DKP;                // [2][TT][DKP] decays per key (SSD: [2][2][TT] step sizes, decays)
+    float* sK = sD + 2 * SC_TT * DKP;                // [2][TT][DKP]
+    float* sV = sK + 2 * SC_TT * DKP;                // [2][TT][COLS]
+    float* sY = sV + 2 * SC_TT * SC_COLS;            // [KW][TT][COLS]
+    const int chunk = p.chunks > 1 ? p.z0 + (int)blockIdx.z : 0;
+    const SeqSeg sg = a.segs[p.chunks > 1 ? 0 : blockIdx.z];
+    const int t_lo = chunk * p.len, t_hi = p.chunks > 1 && chunk + 1 < p.chunks ? min(sg.n, t_lo + p.len) : sg.n;
+    if (t_lo >= t_hi) return;
+    const bool outputs = p.chunks == 1 || p.second != 0 || chunk == 0;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, kw = warp % KW, cw = warp / KW, kg = lane & 7, cg = lane >> 3;
+    const int h = blockIdx.y, col0 = blockIdx.x * SC_COLS, dk = a.dk, dv = a.dv;
+    const int g = MODE == SCAN_SSD ? h / (a.heads / a.groups) : h;
+    // a lane's keys: four consecutive ones out of each half of its warp's 64, so that eight key groups read 128 adjoining bytes
+    const int key0 = kw * 64 + kg * 4, c0 = cw * 16 + cg * 4;   // keys key0 + (0..3) and key0 + 32 + (0..3); columns col0 + c0 + (0..3)
+    auto key_of = [&](int i) { return key0 + (i >> 2) * 32 + (i & 3); };
+    const float* qg = a.q + (size_t)sg.row0 * a.ldq + (size_t)g * dk;
+    const float* kgm = HAS_K ? a.k + (size_t)sg.row0 * a.ldk + (size_t)g * dk : nullptr;
+    const float* dg = a.decay_in + (size_t)sg.row0 * a.ldd + (PER_KEY ? (size_t)h * dk : (size_t)h);
+    const float* vg = a.v + (size_t)sg.row0 * a.ldv + (size_t)h * dv + col0;
+    const int ncol = min(SC_COLS, dv - col0);
+    const size_t head_state = ((size_t)h * dk) * dv, all_state = (size_t)a.heads * dk * dv;
+
+    float S[8][4], pd[8];
+    auto load_state = [&](const float* st, bool fold, const float* dec) {   // S = st, or S = dec S + st
 #pragma unroll
-    for (int i = 0; i < KPT; ++i) {
-        const int key = ks * KPT + i;
-        S[i] = (sg.pos0 > 0 && col_ok && key < dk) ? st[(size_t)key * dv + j] : 0.f;
-        bon[i] = (MODE == SCAN_RWKV && key < dk) ? a.bonus[(size_t)h * dk + key] : 0.f;
+        for (int i = 0; i < 8; ++i) {
+            const int key = key_of(i);
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            if (key < dk) {
+                const float* r = st + (size_t)key * dv + col0 + c0;
+                if (V16 && c0 + 4 <= ncol) {
+                    const float4 f = *reinterpret_cast<const float4*>(r);
+                    v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) if (c0 + j < ncol) v[j] = r[j];
+                }
+            }
+            const float d = fold && key < dk ? dec[key] : 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) S[i][j] = fold ? fmaf(d, S[i][j], v[j]) : v[j];
+        }
+    };
+    auto store_state = [&](float* st) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int key = key_of(i);
+            if (key >= dk) continue;
+            float* r = st + (size_t)key * dv + col0 + c0;
+            if (V16 && c0 + 4 <= ncol) {
+                *reinterpret_cast<float4*>(r) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) if (c0 + j < ncol) r[j] = S[i][j];
+            }
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        pd[i] = 1.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) S[i][j] = 0.f;
+    }
+    auto fetch = [&](int t0, int buf) {   // raw rows of a tile; entries past dk / the last column are zeroed once, below
+        const int nt = min(SC_TT, t_hi - t0);
+        float *q = sQ + buf * SC_TT * DKP, *k = sK + buf * SC_TT * DKP, *d = sD + buf * SC_TT * DKP, *v = sV + buf * SC_TT * SC_COLS;
+        if (V16) {
+            const int n4 = dk >> 2, c4 = ncol >> 2;
+            for (int e = tid; e < nt * n4; e += NTHR) {
+                const int t = e / n4, o = (e - t * n4) * 4;
+                if (outputs) scan_cp16(q + t * DKP + o, qg + (size_t)(t0 + t) * a.ldq + o);
+                if (HAS_K) scan_cp16(k + t * DKP + o, kgm + (size_t)(t0 + t) * a.ldk + o);
+                if (PER_KEY) scan_cp16(d + t * DKP + o, dg + (size_t)(t0 + t) * a.ldd + o);
+            }
+            for (int e = tid; e < nt * c4; e += NTHR) {
+                const int t = e / c4, o = (e - t * c4) * 4;
+                scan_cp16(v + t * SC_COLS + o, vg + (size_t)(t0 + t) * a.ldv + o);
+            }
+        } else {
+            for (int e = tid; e < nt * dk; e += NTHR) {
+                const int t = e / dk, o = e - t * dk;
+                if (outputs) scan_cp4(q + t * DKP + o, qg + (size_t)(t0 + t) * a.ldq + o);
+                if (HAS_K) scan_cp4(k + t * DKP + o, kgm + (size_t)(t0 + t) * a.ldk + o);
+                if (PER_KEY) scan_cp4(d + t * DKP + o, dg + (size_t)(t0 + t) * a.ldd + o);
+            }
+            for (int e = tid; e < nt * ncol; e += NTHR) {
+                const int t = e / ncol, o = e - t * ncol;
+                scan_cp4(v + t * SC_COLS + o, vg + (size_t)(t0 + t) * a.ldv + o);
+            }
+        }
+        if (!PER_KEY && tid < nt) scan_cp4(d + tid, dg + (size_t)(t0 + tid) * a.ldd);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(t_lo, 0);
+    if (p.second != 0) {
+        load_state(p.final_state + head_state, false, nullptr);
+        for (int c = 1; c < chunk; ++c) load_state(p.final_state + (size_t)c * all_state + head_state, true, p.decays + ((size_t)c * a.heads + h) * dk);
+    } else if (chunk == 0 && sg.pos0 > 0) {
+        load_state(a.state + (size_t)sg.slot * all_state + head_state, false, nullptr);
+    }
+    float bon[8];
+    if (MODE == SCAN_RWKV) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) bon[i] = key_of(i) < dk ? a.bonus[(size_t)h * dk + key_of(i)] : 0.f;
     }
     float neg_a = 0.f, dtb = 0.f, skip = 0.f;
     if (MODE == SCAN_SSD) { neg_a = -expf(a.a_log[h]); dtb = a.dt_bias[h]; skip = a.skip[h]; }
+    // entries that no copy writes: keys past dk (queries and keys 0), columns past the last one
+    for (int e = tid; e < 2 * SC_TT * (DKP - dk); e += NTHR) {
+        const int at = (e / (DKP - dk)) * DKP + dk + e % (DKP - dk);
+        sQ[at] = 0.f; sK[at] = 0.f;
+        if (PER_KEY) sD[at] = 0.f;
+    }
+    for (int e = tid; e < 2 * SC_TT * (SC_COLS - ncol); e += NTHR) sV[(e / (SC_COLS - ncol)) * SC_COLS + ncol + e % (SC_COLS - ncol)] = 0.f;
 
-    // Staging is split in two so that global latency hides behind the walk of the previous tile: the raw inputs of tile
-    // i+1 are requested into registers before tile i is walked, and turned into (q, dt*k, decay, v) in shared memory after.
-    // A thread stages TT*KPT/32 key elements (dkp = KS*KPT over 32*KS threads) and up to TT value elements.
-    constexpr int EPT = TT * KPT / 32;
-    float rq[EPT], rk[EPT], rd[EPT], rv[TT];
-    float rtok = 0.f;  // SSD: the raw step size of token `tid` of the tile (one scalar per token and head)
-    auto fetch = [&](int t0) {
-        const int nt = min(TT, sg.n - t0);
-        if (MODE == SCAN_SSD && tid < nt) rtok = a.decay_in[(size_t)(sg.row0 + t0 + tid) * a.ldd + h];
-#pragma unroll
-        for (int u = 0; u < EPT; ++u) {
-            const int e = tid + u * nthr, t = e / dkp, key = e % dkp;
-            rq[u] = 0.f; rk[u] = 0.f; rd[u] = 0.f;
-            if (t < nt && key < dk) {
-                const size_t row = (size_t)(sg.row0 + t0 + t);
-                rq[u] = a.q[row * a.ldq + (size_t)g * dk + key];
-                if (MODE != SCAN_HGRN2) rk[u] = a.k[row * a.ldk + (size_t)g * dk + key];
-                if (MODE != SCAN_SSD) rd[u] = a.decay_in[row * a.ldd + (size_t)h * dk + key];
+    int buf = 0;
+    for (int t0 = t_lo; t0 < t_hi; t0 += SC_TT, buf ^= 1) {
+        const int nt = min(SC_TT, t_hi - t0);
+        float *q = sQ + buf * SC_TT * DKP, *k = sK + buf * SC_TT * DKP, *d = sD + buf * SC_TT * DKP, *v = sV + buf * SC_TT * SC_COLS;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        if (t0 + SC_TT < t_hi) fetch(t0 + SC_TT, buf ^ 1);   // (the other buffer was read before the barrier above)
+        // the raw gates -> (q, k, decay)
+        if (MODE == SCAN_SSD) {
+            if (tid < nt) {   // the step size multiplies the value (dt B x^T = B (dt x)^T)
+                const float dt = softplus_f(d[tid] + dtb);
+                d[tid] = dt;
+                d[SC_TT + tid] = expf(neg_a * dt);
+            }
+        } else if (p.prepared == 0 || MODE == SCAN_HGRN2) {
+            for (int at = tid; at < nt * DKP; at += NTHR) {
+                const int key = at % DKP;
+                if (key >= dk) continue;
+                float f = d[at];
+                if (p.prepared == 0) {
+                    d[at] = f = scan_decay<MODE>(a, h * dk + key, f);
+                    if (outputs && MODE != SCAN_RWKV) q[at] = scan_query<MODE>(a, q[at]);
+                }
+                if (MODE == SCAN_HGRN2) k[at] = 1.f - f;
             }
         }
+        if (MODE == SCAN_SSD || MODE == SCAN_HGRN2 || p.prepared == 0) __syncthreads();
+        if (outputs) {
+#pragma unroll 2
+            for (int t = 0; t < nt; ++t) {
+                float qv[8], kv[8], dvv[8], vv[4], y[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int u = 0; u < TT; ++u) {
-            const int e = tid + u * nthr, t = e >> 5, jj = blockIdx.x * 32 + (e & 31);
-            rv[u] = (e < nt * 32 && jj < dv) ? a.v[(size_t)(sg.row0 + t0 + t) * a.ldv + (size_t)h * dv + jj] : 0.f;
-        }
-    };
-    fetch(0);
-    for (int t0 = 0; t0 < sg.n; t0 += TT) {
-        const int nt = min(TT, sg.n - t0);
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < EPT; ++u) {
-            const int e = tid + u * nthr, key = e % dkp;
-            if (MODE == SCAN_HGRN2) {
-                // forget gate bounded below: f = l + (1 - l) sigmoid(z + b); what is forgotten, 1 - f, is what is written
-                float f = 1.f;
-                if (key < dk) {
-                    const float low = a.gate_lower[(size_t)h * dk + key];
-                    f = fmaf(1.f - low, 1.f / (1.f + expf(-(rd[u] + a.gate_bias[(size_t)h * dk + key]))), low);
-                }
-                sQ[e] = silu_f(rq[u]); sK[e] = 1.f - f; sD[e] = f;
-            } else if (MODE == SCAN_GLA) {
-                // decay per key channel: sigmoid(z + b)^(1 / tau) = exp(log_sigmoid(z + b) / tau), log_sigmoid(u) = min(u, 0) - log1p(exp(-|u|))
-                float al = 1.f;
-                if (key < dk) {
-                    const float z = rd[u] + a.gate_bias[(size_t)h * dk + key];
-                    al = expf((fminf(z, 0.f) - log1pf(expf(-fabsf(z)))) / a.tau);
-                }
-                sQ[e] = rq[u] * a.q_scale; sK[e] = rk[u]; sD[e] = al;
-            } else {
-                sQ[e] = rq[u]; sK[e] = rk[u];
-                if (MODE == SCAN_RWKV) sD[e] = key < dk ? expf(-expf(rd[u])) : 1.f;
-            }
-        }
-        // SSD: the decay and the step size are scalars per token; the step size multiplies the value (dt B x^T = B (dt x)^T),
-        // so the keys are staged as they are and sD holds [TT] step sizes followed by [TT] decays
-        if (MODE == SCAN_SSD && tid < TT) {
-            const float dt = softplus_f(rtok + dtb);
-            sD[tid] = dt;
-            sD[TT + tid] = expf(neg_a * dt);
-        }
-#pragma unroll
-        for (int u = 0; u < TT; ++u) {
-            const int e = tid + u * nthr;
-            if (e < TT * 32) sV[e] = rv[u];
-        }
-        __syncthreads();
-        if (t0 + TT < sg.n) fetch(t0 + TT);
-        float part[TT];   // this thread's share of y[t][j] for the tokens of the tile
-#pragma unroll
-        for (int t = 0; t < TT; ++t) {
-            part[t] = 0.f;
-            if (t < nt) {
-                const float v = sV[t * 32 + threadIdx.x];
-                float q[KPT], k[KPT], d[KPT];   // this slice's 16 keys of the token: four 16-byte broadcast reads per array
-#pragma unroll
-                for (int i4 = 0; i4 < KPT / 4; ++i4) {
-                    const float4 q4 = *reinterpret_cast<const float4*>(sQ + t * dkp + ks * KPT + i4 * 4);
-                    const float4 k4 = *reinterpret_cast<const float4*>(sK + t * dkp + ks * KPT + i4 * 4);
-                    q[i4 * 4] = q4.x; q[i4 * 4 + 1] = q4.y; q[i4 * 4 + 2] = q4.z; q[i4 * 4 + 3] = q4.w;
-                    k[i4 * 4] = k4.x; k[i4 * 4 + 1] = k4.y; k[i4 * 4 + 2] = k4.z; k[i4 * 4 + 3] = k4.w;
-                    if (MODE != SCAN_SSD) {
-                        const float4 d4 = *reinterpret_cast<const float4*>(sD + t * dkp + ks * KPT + i4 * 4);
-                        d[i4 * 4] = d4.x; d[i4 * 4 + 1] = d4.y; d[i4 * 4 + 2] = d4.z; d[i4 * 4 + 3] = d4.w;
+                for (int i = 0; i < 2; ++i) {
+                    const float4 q4 = *reinterpret_cast<const float4*>(q + t * DKP + key0 + 32 * i), k4 = *reinterpret_cast<const float4*>(k + t * DKP + key0 + 32 * i);
+                    qv[4 * i] = q4.x; qv[4 * i + 1] = q4.y; qv[4 * i + 2] = q4.z; qv[4 * i + 3] = q4.w;
+                    kv[4 * i] = k4.x; kv[4 * i + 1] = k4.y; kv[4 * i + 2] = k4.z; kv[4 * i + 3] = k4.w;
+                    if (PER_KEY) {
+                        const float4 d4 = *reinterpret_cast<const float4*>(d + t * DKP + key0 + 32 * i);
+                        dvv[4 * i] = d4.x; dvv[4 * i + 1] = d4.y; dvv[4 * i + 2] = d4.z; dvv[4 * i + 3] = d4.w;
                     }
                 }
-                float acc = 0.f;
-                const float vdt = MODE == SCAN_SSD ? v * sD[t] : v, dec = MODE == SCAN_SSD ? sD[TT + t] : 0.f;
+                const float4 v4 = *reinterpret_cast<const float4*>(v + t * SC_COLS + c0);
+                const float dt = PER_KEY ? 1.f : d[t], dec = PER_KEY ? 0.f : d[SC_TT + t];
+                vv[0] = v4.x * dt; vv[1] = v4.y * dt; vv[2] = v4.z * dt; vv[3] = v4.w * dt;
 #pragma unroll
-                for (int i = 0; i < KPT; ++i) {
-                    const float kv = k[i] * vdt;
-                    if (MODE == SCAN_RWKV) {
-                        acc = fmaf(q[i], fmaf(bon[i], kv, S[i]), acc);
-                        S[i] = fmaf(d[i], S[i], kv);
-                    } else if (MODE == SCAN_HGRN2 || MODE == SCAN_GLA) {
-                        S[i] = fmaf(d[i], S[i], kv);
-                        acc = fmaf(q[i], S[i], acc);
-                    } else {
-                        S[i] = fmaf(dec, S[i], kv);
-                        acc = fmaf(q[i], S[i], acc);
+                for (int i = 0; i < 8; ++i) {
+                    const float de = PER_KEY ? dvv[i] : dec;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float x = kv[i] * vv[j];
+                        if (MODE == SCAN_RWKV) {
+                            y[j] = fmaf(qv[i], fmaf(bon[i], x, S[i][j]), y[j]);
+                            S[i][j] = fmaf(de, S[i][j], x);
+                        } else {
+                            S[i][j] = fmaf(de, S[i][j], x);
+                            y[j] = fmaf(qv[i], S[i][j], y[j]);
+                        }
                     }
                 }
-                part[t] = acc;
+                // sum over the eight key groups; lane kg ends up with column 2 (kg & 1) + (kg >> 1 & 1)
+                const bool b0 = kg & 1, b1 = kg & 2;
+                float u0 = b0 ? y[2] : y[0], u1 = b0 ? y[3] : y[1];
+                u0 += __shfl_xor_sync(0xffffffffu, b0 ? y[0] : y[2], 1);
+                u1 += __shfl_xor_sync(0xffffffffu, b0 ? y[1] : y[3], 1);
+                float w0 = b1 ? u1 : u0;
+                w0 += __shfl_xor_sync(0xffffffffu, b1 ? u0 : u1, 2);
+                w0 += __shfl_xor_sync(0xffffffffu, w0, 4);
+                if (kg < 4) sY[(kw * SC_TT + t) * SC_COLS + c0 + 2 * (kg & 1) + (kg >> 1)] = w0;
+            }
+        } else {
+#pragma unroll 2
+            for (int t = 0; t < nt; ++t) {
+                float kv[8], dvv[8], vv[4];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const float4 k4 = *reinterpret_cast<const float4*>(k + t * DKP + key0 + 32 * i);
+                    kv[4 * i] = k4.x; kv[4 * i + 1] = k4.y; kv[4 * i + 2] = k4.z; kv[4 * i + 3] = k4.w;
+                    if (PER_KEY) {
+                        const float4 d4 = *reinterpret_cast<const float4*>(d + t * DKP + key0 + 32 * i);
+                        dvv[4 * i] = d4.x; dvv[4 * i + 1] = d4.y; dvv[4 * i + 2] = d4.z; dvv[4 * i + 3] = d4.w;
+                    }
+                }
+                const float4 v4 = *reinterpret_cast<const float4*>(v + t * SC_COLS + c0);
+                const float dt = PER_KEY ? 1.f : d[t], dec = PER_KEY ? 0.f : d[SC_TT + t];
+                vv[0] = v4.x * dt; vv[1] = v4.y * dt; vv[2] = v4.z * dt; vv[3] = v4.w * dt;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float de = PER_KEY ? dvv[i] : dec;
+                    pd[i] *= de;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) S[i][j] = fmaf(de, S[i][j], kv[i] * vv[j]);
+                }
             }
         }
-        // the key slices meet once per tile: partial sums through shared memory, every thread finishes some (token, column) pairs
-        if (KS > 1) {
-#pragma unroll
-            for (int t = 0; t < TT; ++t) sR[(t * KS + ks) * 32 + threadIdx.x] = part[t];
+        if (outputs) {
             __syncthreads();
-            for (int t = ks; t < nt; t += KS) {
-                float acc = 0.f;
-                for (int s2 = 0; s2 < KS; ++s2) acc += sR[(t * KS + s2) * 32 + threadIdx.x];
-                if (col_ok) {
-                    if (MODE == SCAN_SSD) acc = fmaf(skip, sV[t * 32 + threadIdx.x], acc);
-                    a.y[(size_t)(sg.row0 + t0 + t) * a.ldy + (size_t)h * dv + j] = acc;
-                }
-            }
-        } else if (col_ok) {
+            for (int e = tid; e < nt * SC_COLS; e += NTHR) {
+                const int t = e / SC_COLS, c = e % SC_COLS;
+                if (c >= ncol) continue;
+                float y = sY[e];
 #pragma unroll
-            for (int t = 0; t < TT; ++t)
-                if (t < nt) {
-                    float acc = part[t];
-                    if (MODE == SCAN_SSD) acc = fmaf(skip, sV[t * 32 + threadIdx.x], acc);
-                    a.y[(size_t)(sg.row0 + t0 + t) * a.ldy + (size_t)h * dv + j] = acc;
-                }
+                for (int w = 1; w < KW; ++w) y += sY[w * SC_TT * SC_COLS + e];
+                if (MODE == SCAN_SSD) y = fmaf(skip, v[t * SC_COLS + c], y);
+                a.y[(size_t)(sg.row0 + t0 + t) * a.ldy + (size_t)h * dv + col0 + c] = y;
+            }
         }
     }
+    if (p.chunks == 1 || chunk == p.chunks - 1) {
+        store_state(a.state + (size_t)sg.slot * all_state + head_state);
+    } else if (p.second == 0) {
+        store_state(p.final_state + (size_t)chunk * all_state + head_state);
+        if (blockIdx.x == 0 && cw == 0 && cg == 0) {
 #pragma unroll
-    for (int i = 0; i < KPT; ++i) {
-        const int key = ks * KPT + i;
-        if (col_ok && key < dk) st[(size_t)key * dv + j] = S[i];
+            for (int i = 0; i < 8; ++i)
+                if (key_of(i) < dk) p.decays[((size_t)chunk * a.heads + h) * dk + key_of(i)] = pd[i];
+        }
     }
 }
 }  // namespace
@@ -339,39 +473,72 @@ int token_shift_mix_f32(const float* x, const float* mu, float* prev, float* out
     return 0;
 }
 
-template <int MODE, int KPT>
+template <int MODE, int KW, bool V16>
 int launch_scan(const ScanArgs& a, cudaStream_t st) {
-    const int KS = (a.dk + KPT - 1) / KPT;
-    const size_t smem = ((size_t)3 * TT * KS * KPT + TT * 32 + (size_t)TT * KS * 32) * sizeof(float);
-    dim3 grid((a.dv + 31) / 32, a.heads, a.nseg), block(32, KS);
-    if (smem > 48 * 1024) B2_CUDA_CHECK(cudaFuncSetAttribute(linear_scan_kernel<MODE, KPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    linear_scan_kernel<MODE, KPT><<<grid, block, smem, st>>>(a);
+    constexpr size_t smem = (size_t)(6 * SC_TT * KW * 64 + 2 * SC_TT * SC_COLS + KW * SC_TT * SC_COLS) * sizeof(float);
+    B2_CUDA_CHECK(cudaFuncSetAttribute(linear_scan_kernel<MODE, KW, V16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int cols = (a.dv + SC_COLS - 1) / SC_COLS, ctas = cols * a.heads;
+    ScanPlan p;
+    // Chunks: enough CTAs for two per SM, of 64 tokens and more; two chunks would walk the whole chain all the same
+    // (the last chunk has no part in the first launch, the first one none in the second)
+    int chunks = a.nseg == 1 && a.chunk_scratch != nullptr ? 1 + 2 * num_sms() / ctas : 1;
+    chunks = std::min(std::min(chunks, SC_MAX_CHUNKS), a.rows / 64);
+    if (chunks >= 3 && (size_t)(chunks - 1) * a.heads * a.dk * (a.dv + 1) <= a.chunk_floats) {
+        p.len = ((a.rows + chunks - 1) / chunks + SC_TT - 1) / SC_TT * SC_TT;
+        p.chunks = (a.rows + p.len - 1) / p.len;
+    }
+    if (p.chunks >= 3) {
+        p.final_state = a.chunk_scratch;
+        p.decays = a.chunk_scratch + (size_t)(p.chunks - 1) * a.heads * a.dk * a.dv;
+        if (MODE != SCAN_SSD) {
+            scan_prepare_kernel<MODE><<<dim3((a.heads * a.dk + 255) / 256, a.rows), 256, 0, st>>>(a);
+            B2_LAUNCH_CHECK();
+            p.prepared = 1;
+        }
+        linear_scan_kernel<MODE, KW, V16><<<dim3(cols, a.heads, p.chunks - 1), KW * 128, smem, st>>>(a, p);
+        B2_LAUNCH_CHECK();
+        p.second = 1;
+        p.z0 = 1;
+        linear_scan_kernel<MODE, KW, V16><<<dim3(cols, a.heads, p.chunks - 1), KW * 128, smem, st>>>(a, p);
+    } else {
+        p.chunks = 1;
+        linear_scan_kernel<MODE, KW, V16><<<dim3(cols, a.heads, a.nseg), KW * 128, smem, st>>>(a, p);
+    }
     B2_LAUNCH_CHECK();
     return 0;
 }
+template <int MODE>
+int scan_of_size(const ScanArgs& a, cudaStream_t st) {
+    const uintptr_t ptrs = reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) | reinterpret_cast<uintptr_t>(a.v) | reinterpret_cast<uintptr_t>(a.state) |
+                           (MODE == SCAN_SSD ? 0 : reinterpret_cast<uintptr_t>(a.decay_in));
+    const int64_t sizes = a.dk | a.dv | a.ldq | (MODE == SCAN_HGRN2 ? 0 : a.ldk) | a.ldv | (MODE == SCAN_SSD ? 0 : a.ldd);
+    const bool v16 = (ptrs & 15) == 0 && sizes % 4 == 0;
+    if (a.dk <= 64) return v16 ? launch_scan<MODE, 1, true>(a, st) : launch_scan<MODE, 1, false>(a, st);
+    if (a.dk <= 128) return v16 ? launch_scan<MODE, 2, true>(a, st) : launch_scan<MODE, 2, false>(a, st);
+    return v16 ? launch_scan<MODE, 4, true>(a, st) : launch_scan<MODE, 4, false>(a, st);
+}
+
+size_t linear_scan_scratch_floats(int heads, int dk, int dv) { return (size_t)(SC_MAX_CHUNKS - 1) * heads * dk * (dv + 1); }
 
 int linear_scan_f32(const ScanArgs& a, cudaStream_t st) {
     B2_CHECK_ARG(a.q && (a.k || a.mode == SCAN_HGRN2) && a.v && a.decay_in && a.state && a.y && a.segs && a.nseg > 0, "linear_scan: null argument");
     B2_CHECK_ARG(a.heads > 0 && a.dk > 0 && a.dv > 0, "linear_scan: bad sizes");
     B2_CHECK_ARG(a.dk <= 256, "linear_scan: key size %d exceeds 256", a.dk);
-    // 8 keys per thread where 16 key slices cover the key size: twice the warps hide the shared-memory latency of the token walk
-    static const bool narrow_ok = [] { const char* e = getenv("B2_SCAN_KPT8"); return !(e != nullptr && e[0] == '0'); }();
-    const bool narrow = narrow_ok && a.dk <= 128 && a.dk > 16;
     if (a.mode == SCAN_SSD) {
         B2_CHECK_ARG(a.groups > 0 && a.heads % a.groups == 0 && a.dt_bias && a.a_log && a.skip, "linear_scan(ssd): heads %d / groups %d", a.heads, a.groups);
-        return narrow ? launch_scan<SCAN_SSD, 8>(a, st) : launch_scan<SCAN_SSD, 16>(a, st);
+        return scan_of_size<SCAN_SSD>(a, st);
     }
     if (a.mode == SCAN_HGRN2) {
         B2_CHECK_ARG(a.gate_bias && a.gate_lower, "linear_scan(hgrn2): null gate bias / lower bound");
-        return narrow ? launch_scan<SCAN_HGRN2, 8>(a, st) : launch_scan<SCAN_HGRN2, 16>(a, st);
+        return scan_of_size<SCAN_HGRN2>(a, st);
     }
     if (a.mode == SCAN_GLA) {
         B2_CHECK_ARG(a.gate_bias && a.tau > 0.f, "linear_scan(gla): null decay bias or a non-positive tau");
-        return narrow ? launch_scan<SCAN_GLA, 8>(a, st) : launch_scan<SCAN_GLA, 16>(a, st);
+        return scan_of_size<SCAN_GLA>(a, st);
     }
     B2_CHECK_ARG(a.mode == SCAN_RWKV, "linear_scan: unknown mode %d", a.mode);
     B2_CHECK_ARG(a.bonus != nullptr, "linear_scan(rwkv): null bonus");
-    return narrow ? launch_scan<SCAN_RWKV, 8>(a, st) : launch_scan<SCAN_RWKV, 16>(a, st);
+    return scan_of_size<SCAN_RWKV>(a, st);
 }
 
 }  // namespace b2

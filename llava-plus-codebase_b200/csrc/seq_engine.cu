@@ -77,6 +77,7 @@ struct SeqModel {
     int rows = 0;                      // workspace rows
     // workspaces (fp32 unless noted)
     DevBuf x, proj, act, y, gated, mixout, mixes, rp, wl1, wlog, ff, xn, tok, want;
+    DevBuf scan_chunks;                // chunk states of a long prompt's recurrences (recurrent.cu)
     DevBuf a16;                        // bf16 copy of a GEMM's A operand (tensor-core path of the bf16 compute mode)
     int a16_w = 0;
     DevBuf segs, row_slot, row_pos;
@@ -476,6 +477,7 @@ static int gla_mixer(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, SeqLayer
     sa.y = s.y.as<float>(); sa.ldy = L.pv;
     sa.heads = H; sa.groups = H; sa.dk = dk; sa.dv = dv;
     sa.segs = s.segs.as<SeqSeg>(); sa.nseg = nseg;
+    sa.rows = R; sa.chunk_scratch = s.scan_chunks.as<float>(); sa.chunk_floats = s.scan_chunks.bytes / F4;
     B2_TRY(linear_scan_f32(sa, st));
     B2_TRY(gated_group_rmsnorm_f32(s.y.as<float>(), L.pv, proj + 2 * L.pq + L.pv, L.pproj_ld, W.gnorm.as<float>(), s.gated.as<float>(), L.pv, R, L.pv, dv,
                                    0, s.d.norm_eps, st, 1));
@@ -501,6 +503,7 @@ static int hgrn2_mixer(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, SeqLay
     sa.y = s.y.as<float>(); sa.ldy = L.pv;
     sa.heads = H; sa.groups = H; sa.dk = dk; sa.dv = dv;
     sa.segs = s.segs.as<SeqSeg>(); sa.nseg = nseg;
+    sa.rows = R; sa.chunk_scratch = s.scan_chunks.as<float>(); sa.chunk_floats = s.scan_chunks.bytes / F4;
     B2_TRY(linear_scan_f32(sa, st));
     B2_TRY(group_rmsnorm_f32(s.y.as<float>(), L.pv, W.hnorm.as<float>(), 1, s.gated.as<float>(), L.pv, R, L.pv, dv, s.d.norm_eps, st));
     return lin(s.gated.as<float>(), L.pv, W.o_w, width, L.pv, target, width, R, LIN_NONE, alpha, accumulate);
@@ -915,6 +918,7 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
             sa.y = s.y.as<float>(); sa.ldy = L.inner;
             sa.heads = d.m_heads; sa.groups = d.m_groups; sa.dk = d.m_state; sa.dv = d.m_vdim;
             sa.segs = segs; sa.nseg = nseg;
+            sa.rows = R; sa.chunk_scratch = s.scan_chunks.as<float>(); sa.chunk_floats = s.scan_chunks.bytes / F4;
             B2_TRY(linear_scan_f32(sa, st));
             B2_TRY(gated_group_rmsnorm_f32(s.y.as<float>(), L.inner, proj, L.dproj_ld, W.mnorm.as<float>(), s.gated.as<float>(), L.inner, R, L.inner,
                                            L.inner / d.m_norm_groups, 1, eps, st));
@@ -965,6 +969,7 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
             sa.y = s.y.as<float>(); sa.ldy = L.rn;
             sa.heads = d.r_heads; sa.groups = d.r_heads; sa.dk = d.r_dim; sa.dv = d.r_dim;
             sa.segs = segs; sa.nseg = nseg;
+            sa.rows = R; sa.chunk_scratch = s.scan_chunks.as<float>(); sa.chunk_floats = s.scan_chunks.bytes / F4;
             B2_TRY(linear_scan_f32(sa, st));
             B2_TRY(gated_group_rmsnorm_f32(s.y.as<float>(), L.rn, rp + 3 * rs, L.rn, W.rnorm.as<float>(), s.gated.as<float>(), L.rn, R, L.rn, d.r_dim,
                                            0, eps, st));
@@ -1518,6 +1523,15 @@ int seq_finalize(b2_model* m) {
     if (s.d.loop_mix) B2_TRY(s.cat.alloc(R * 2 * width * F4));
     if (s.d.block == B2_BLOCK_PARALLEL2) B2_TRY(s.h2.alloc(R * width * F4));
     if (den_w > 0) B2_TRY(s.den.alloc(R * den_w * F4));
+    size_t chunk_floats = 0;
+    for (const SeqLayerInfo& L : s.layers) {
+        const b2_seq_layer_desc& d = L.d;
+        if (d.type == B2_MIXER_MAMBA2) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.m_heads, d.m_state, d.m_vdim));
+        else if (d.type == B2_MIXER_PARALLEL) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.r_heads, d.r_dim, d.r_dim));
+        else if (d.type == B2_MIXER_HGRN2) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.g_heads, d.g_dim, d.g_vdim));
+        else if (d.type == B2_MIXER_GLA) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.gl_heads, d.gl_dim, d.gl_vdim));
+    }
+    if (chunk_floats > 0) B2_TRY(s.scan_chunks.alloc(chunk_floats * F4));
     if (s.d.compute == B2_COMPUTE_BF16) {
         if (dyt || s.d.block == B2_BLOCK_PARALLEL_RMS || s.d.block == B2_BLOCK_PARALLEL2) B2_TRY(s.h1_16.alloc(R * width * 2));
         if (dyt) B2_TRY(s.h2_16.alloc(R * width * 2));
@@ -1583,7 +1597,7 @@ void seq_model_free(b2_model* m) {
     DevBuf* bs[] = {&s.embed, &s.head, &s.final_w, &s.final_b, &s.x, &s.proj, &s.act, &s.y, &s.gated, &s.mixout, &s.mixes, &s.rp, &s.wl1, &s.wlog,
                     &s.ff, &s.xn, &s.tok, &s.want, &s.segs, &s.row_slot, &s.row_pos, &s.a16, &s.bigram, &s.loop_step, &s.x0, &s.qabs, &s.olat, &s.ffa,
                     &s.rlogit, &s.moe_idx, &s.moe_w, &s.moe_pos, &s.moe_src, &s.moe_tile, &s.moe_h, &s.moe_a, &s.moe_y, &s.moe_a16, &s.zero_idx, &s.hin, &s.final_a, &s.loop_in, &s.cat,
-                    &s.h2, &s.h1_16, &s.h2_16, &s.f16, &s.den, &s.embed_nw};
+                    &s.h2, &s.h1_16, &s.h2_16, &s.f16, &s.den, &s.embed_nw, &s.scan_chunks};
     for (DevBuf* b : bs) b->free();
     delete m->seq;
     m->seq = nullptr;
