@@ -22,10 +22,30 @@
 #include <cuda.h>
 #include <math.h>
 
-#include "common.cuh"
 #include "kernels.h"
+#include "split.cuh"
 
 namespace b2 {
+
+// [planes][rows][pitch] bf16, box = [1][box_rows][64], SWIZZLE_128B (bf16 parts; linear_split.cu uses it too)
+int make_tmap_parts(CUtensorMap* map, const void* ptr, int pitch, int64_t nkeys, int planes, int box_rows) {
+    typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                               CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static Encode fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess ? reinterpret_cast<Encode>(f) : nullptr;
+    }();
+    if (fn == nullptr) { set_error("cuTensorMapEncodeTiled entry point unavailable"); return -2; }
+    const cuuint64_t dims[3] = {(cuuint64_t)pitch, (cuuint64_t)nkeys, (cuuint64_t)planes};
+    const cuuint64_t strides[2] = {(cuuint64_t)pitch * 2, (cuuint64_t)nkeys * pitch * 2};
+    const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1}, one[3] = {1, 1, 1};
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled(parts) failed (%d): %d x %lld x %d", (int)r, pitch, (long long)nkeys, planes); return -2; }
+    return 0;
+}
+
 namespace {
 
 constexpr int SP_M = 128, SP_THREADS = 320, SP_SLAB_Q = SP_M * 128;
@@ -34,30 +54,6 @@ __device__ __forceinline__ int split_first(int pos, int kind, int size) {   // f
     if (kind == MASK_WINDOW) return max(0, pos - size + 1);
     if (kind == MASK_CHUNK) return pos / size * size;
     return 0;
-}
-
-// two values -> their three bf16 parts, packed (first value in the low half)
-__device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    hi = pack_bf16(a, b);
-    const float a1 = a - bf16_lo(hi), b1 = b - bf16_hi(hi);
-    mid = pack_bf16(a1, b1);
-    lo = pack_bf16(a1 - bf16_lo(mid), b1 - bf16_hi(mid));
-}
-__device__ __forceinline__ void split8(const float (&x)[8], uint4& hi, uint4& mid, uint4& lo) {
-    split3(x[0], x[1], hi.x, mid.x, lo.x);
-    split3(x[2], x[3], hi.y, mid.y, lo.y);
-    split3(x[4], x[5], hi.z, mid.z, lo.z);
-    split3(x[6], x[7], hi.w, mid.w, lo.w);
-}
-// 8 floats of a row of `n`, from d on (entries past the end are zero)
-__device__ __forceinline__ void load8(const float* p, int d, int n, bool vec, float (&x)[8]) {
-    if (vec && d + 8 <= n) {
-        const float4 a = *reinterpret_cast<const float4*>(p + d), b = *reinterpret_cast<const float4*>(p + d + 4);
-        x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
-    } else {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = d + e < n ? p[d + e] : 0.f;
-    }
 }
 
 struct SplitSrc {          // rows of one operand: element (head, key, d) at base + head * hs + key * ks + d
@@ -89,10 +85,6 @@ __global__ void __launch_bounds__(256) attn_split_kv_kernel(SplitSrc k, SplitSrc
     }
 }
 
-__device__ __forceinline__ void tma_load_3d(void* dst, const void* tmap, uint64_t* bar, int c0, int c1, int c2) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-                 ::"r"(smem_u32(dst)), "l"(tmap), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2) : "memory");
-}
 // D (+)= A B with A [128 x 16] in TMEM (two bf16 of a row per column) and B by descriptor
 __device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -234,9 +226,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            // products in rising size, so that the accumulator is small while the small ones join it: (lo, hi) (hi, lo) (mid, mid) (mid, hi)
-            // (hi, mid) (hi, hi); two bits each, first product lowest. The loops stay rolled: the kernel's roles share the instruction cache.
-            constexpr uint32_t PART_A = 2u | 0u << 2 | 1u << 4 | 1u << 6 | 0u << 8 | 0u << 10, PART_B = 0u | 2u << 2 | 1u << 4 | 0u << 6 | 1u << 8 | 0u << 10;
+            // (the loops stay rolled: the kernel's roles share the instruction cache)
             constexpr uint32_t idesc_s = make_idesc_bf16_f32(SP_M, KT), idesc_o = make_idesc_bf16_f32(SP_M, 64 * DVS) | (1u << 16);
             const uint64_t q_desc = make_sw128_kmajor_desc(smem_u32(sQ)), k_desc = make_sw128_kmajor_desc(smem_u32(sK)), v_desc = make_mn_desc(smem_u32(sV), KT * 128);
 #pragma unroll 1
@@ -247,7 +237,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_
                     const uint32_t d0 = tm + ((t + 1) & 1) * DKS * KT;
 #pragma unroll 1
                     for (int i = 0; i < 6; ++i) {
-                        const uint32_t pa = (PART_A >> (2 * i)) & 3u, pb = (PART_B >> (2 * i)) & 3u;
+                        const uint32_t pa = (SPLIT_A >> (2 * i)) & 3u, pb = (SPLIT_B >> (2 * i)) & 3u;
 #pragma unroll
                         for (int s = 0; s < DKS; ++s)   // a slab of 64 entries of the head has an accumulator of its own
 #pragma unroll
@@ -264,7 +254,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_
                     tc_fence_after();
 #pragma unroll 1
                     for (int i = 0; i < 6; ++i) {
-                        const uint32_t pa = (PART_A >> (2 * i)) & 3u, pb = (PART_B >> (2 * i)) & 3u;
+                        const uint32_t pa = (SPLIT_A >> (2 * i)) & 3u, pb = (SPLIT_B >> (2 * i)) & 3u;
 #pragma unroll
                         for (int k = 0; k < KT / 16; ++k)
                             umma_ts(tm + Cfg::TM_O, tm + Cfg::TM_P + pa * KH + k * 8, v_desc + (pb * (DVS * KT * 8) + k * 128), idesc_o, (i | k) != 0 ? 1u : 0u);
@@ -411,30 +401,12 @@ __global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_
     if (warp == 1) { tc_fence_after(); tmem_dealloc(tm, 512); }
 }
 
-int parts_tmap(CUtensorMap* map, const void* ptr, int pitch, int nkeys, int planes, int box_rows) {
-    typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                               CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static Encode fn = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess ? reinterpret_cast<Encode>(f) : nullptr;
-    }();
-    if (fn == nullptr) { set_error("cuTensorMapEncodeTiled entry point unavailable"); return -2; }
-    const cuuint64_t dims[3] = {(cuuint64_t)pitch, (cuuint64_t)nkeys, (cuuint64_t)planes};
-    const cuuint64_t strides[2] = {(cuuint64_t)pitch * 2, (cuuint64_t)nkeys * pitch * 2};
-    const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1}, one[3] = {1, 1, 1};
-    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled(parts) failed (%d): %d x %d x %d", (int)r, pitch, nkeys, planes); return -2; }
-    return 0;
-}
-
 template <int DKS, int DVS, int KT>
 int launch_split(const SplitParams& p, const SplitSrc& k, const SplitSrc& v, int nkeys, cudaStream_t st) {
     using Cfg = SplitCfg<DKS, DVS, KT>;
     CUtensorMap tk, tv;
-    B2_TRY(parts_tmap(&tk, k.out, k.pitch, nkeys, 3 * k.heads, KT));
-    B2_TRY(parts_tmap(&tv, v.out, v.pitch, nkeys, 3 * v.heads, KT));
+    B2_TRY(make_tmap_parts(&tk, k.out, k.pitch, nkeys, 3 * k.heads, KT));
+    B2_TRY(make_tmap_parts(&tv, v.out, v.pitch, nkeys, 3 * v.heads, KT));
     auto kernel = p.a.softcap > 0.f || p.a.rel != nullptr ? attn_split_kernel<DKS, DVS, KT, true> : attn_split_kernel<DKS, DVS, KT, false>;
     B2_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));
     kernel<<<((p.a.rows + p.QT - 1) / p.QT) * p.a.G, SP_THREADS, Cfg::SMEM, st>>>(tk, tv, p);

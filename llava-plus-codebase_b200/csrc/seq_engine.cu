@@ -77,6 +77,7 @@ struct SeqModel {
     int rows = 0;                      // workspace rows
     // workspaces (fp32 unless noted)
     DevBuf x, proj, act, y, gated, mixout, mixes, rp, wl1, wlog, ff, xn, tok, want;
+    DevBuf lin_parts;                  // fp32 compute: bf16 parts of a product's operands (linear_split.cu)
     DevBuf scan_chunks;                // chunk states of a long prompt's recurrences (recurrent.cu)
     DevBuf a16;                        // bf16 copy of a GEMM's A operand (tensor-core path of the bf16 compute mode)
     int a16_w = 0;
@@ -108,6 +109,11 @@ namespace {
 
 const size_t F4 = sizeof(float);
 size_t esz(int dt) { return dt == DT_F32 ? 4 : 2; }
+
+// scratch that a faster path wants and that nothing depends on: a device without room for it runs the other path
+void alloc_spare(DevBuf& b, size_t bytes) {
+    if (b.alloc(bytes) != 0) cudaGetLastError();
+}
 
 int64_t numel(const int64_t* shape, int ndim) {
     int64_t n = 1;
@@ -194,6 +200,8 @@ struct Lin {  // one Linear call on the model's compute dtype
         a.round_a = s.d.compute == B2_COMPUTE_BF16;
         if (norm != nullptr) a.norm = *norm;
         a.A16 = a16;
+        a.parts = s.lin_parts.p; a.parts_bytes = s.lin_parts.bytes;
+        if (tc_enabled() && linear_splits(a)) return linear_split_f32(a, st);
         if ((M == 1 || tc_enabled()) && linear_streams(a)) return linear_stream_f32(a, st);
         // bf16 compute, a portion of a prompt: the tcgen05 GEMM on a bf16 copy of A (weights are stored with their rows
         // padded to a multiple of 8, zero-filled, so N rounds up; the pitch of every projection buffer is a multiple of 8)
@@ -1531,7 +1539,7 @@ int seq_finalize(b2_model* m) {
         else if (d.type == B2_MIXER_HGRN2) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.g_heads, d.g_dim, d.g_vdim));
         else if (d.type == B2_MIXER_GLA) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.gl_heads, d.gl_dim, d.gl_vdim));
     }
-    if (chunk_floats > 0) B2_TRY(s.scan_chunks.alloc(chunk_floats * F4));
+    alloc_spare(s.scan_chunks, chunk_floats * F4);
     if (s.d.compute == B2_COMPUTE_BF16) {
         if (dyt || s.d.block == B2_BLOCK_PARALLEL_RMS || s.d.block == B2_BLOCK_PARALLEL2) B2_TRY(s.h1_16.alloc(R * width * 2));
         if (dyt) B2_TRY(s.h2_16.alloc(R * width * 2));
@@ -1572,6 +1580,7 @@ int seq_finalize(b2_model* m) {
             kmax = std::max(kmax, std::max(std::max(std::max(L.inner, L.ng), std::max(L.rn, L.d.ff)), std::max(std::max(L.pv, std::max(L.lrow, L.d.la_q_rank)), std::max(L.d.la_dim, L.d.moe_shared_ff))));
         s.a16_w = (kmax + 7) / 8 * 8;
         if (s.d.compute == B2_COMPUTE_BF16) B2_TRY(s.a16.alloc(R * s.a16_w * 2));
+        else alloc_spare(s.lin_parts, linear_split_bytes((int)R, kmax) + ((size_t)64 << 20));   // (with room for the weights in blocks of rows)
     }
     B2_TRY(s.tok.alloc(R * 4));
     B2_TRY(s.want.alloc(R * 4));
@@ -1597,7 +1606,7 @@ void seq_model_free(b2_model* m) {
     DevBuf* bs[] = {&s.embed, &s.head, &s.final_w, &s.final_b, &s.x, &s.proj, &s.act, &s.y, &s.gated, &s.mixout, &s.mixes, &s.rp, &s.wl1, &s.wlog,
                     &s.ff, &s.xn, &s.tok, &s.want, &s.segs, &s.row_slot, &s.row_pos, &s.a16, &s.bigram, &s.loop_step, &s.x0, &s.qabs, &s.olat, &s.ffa,
                     &s.rlogit, &s.moe_idx, &s.moe_w, &s.moe_pos, &s.moe_src, &s.moe_tile, &s.moe_h, &s.moe_a, &s.moe_y, &s.moe_a16, &s.zero_idx, &s.hin, &s.final_a, &s.loop_in, &s.cat,
-                    &s.h2, &s.h1_16, &s.h2_16, &s.f16, &s.den, &s.embed_nw, &s.scan_chunks};
+                    &s.h2, &s.h1_16, &s.h2_16, &s.f16, &s.den, &s.embed_nw, &s.scan_chunks, &s.lin_parts};
     for (DevBuf* b : bs) b->free();
     delete m->seq;
     m->seq = nullptr;
@@ -1744,7 +1753,7 @@ int seq_kv_alloc(b2_kv* kv) {
             else if (d.type == B2_MIXER_PARALLEL) per_key = std::max(per_key, attn_split_bytes_per_key(d.a_kv_heads, d.a_kv_heads, d.a_dim, d.a_vdim));
         }
         const size_t PARTS_MAX = (size_t)256 << 20;
-        if (per_key > 0) B2_TRY(kv->seq->parts.alloc(std::min(Smax * per_key, PARTS_MAX)));
+        alloc_spare(kv->seq->parts, std::min(Smax * per_key, PARTS_MAX));
     }
     kv->seq->nsplit_max = 64;
     B2_TRY(kv->seq->attn_partial.alloc((size_t)8 * maxH * kv->seq->nsplit_max * (maxdv + 2) * F4));

@@ -1,0 +1,45 @@
+"""True-fp32 Linears of prompt portions on the tensor cores (csrc/linear_split.cu) against the oracle: one layer and the head, at the edges of the
+128-row tiles, of the 64-wide blocks of K and of tiles of 64 and 128 columns, at sizes that are no multiple of 8, and a head whose parts exceed
+the scratch and go in blocks of rows."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import sofopel_oracle as O
+from test_sofopel_gpu import build, config, tokens_for, win
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float(np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+def check(width, ff, vocab, n, seed=0):
+    cfg = config([dict(win(3, 1, 20, 28, None, None, 8), mlp={"kind": "dense", "ff": ff, "limit": 7.0})], width=width, vocab=vocab, mult=1.0)
+    model, w = build(cfg, torch.float32, seed=seed, max_batch=1, max_seq=n + 2, max_rows=n)
+    toks = tokens_for(cfg, n)
+    eng = model._ensure_engine()
+    logits, stream = eng.append_tokens(eng.new_kv(1, n + 2), 0, toks, list(range(n)), restart=True, residuals=True)
+    logits, stream = logits.double().cpu().numpy(), stream[0].double().cpu().numpy()
+    model.invalidate_engine()
+    ref, layers = O.forward(cfg, w, toks, return_layers=True)
+    # each product is a sum of K fp32 terms, about 2^-24 sqrt(K / 2) of a result; four follow one another (projection, scores, output / unit, head)
+    k = max(width, ff, 84)
+    bound = 4 * 2 ** -24 * (k / 2) ** 0.5 + 2 ** -22
+    assert rel(stream, layers[0]) <= bound
+    assert rel(logits, ref) <= bound
+
+
+@pytest.mark.parametrize("n", [8, 9, 24, 127, 128, 129, 260])
+def test_rows(n):
+    check(136, 200, 150, n)
+
+
+@pytest.mark.parametrize("width,ff,vocab", [(64, 64, 64), (63, 65, 129), (8, 1, 7), (200, 1000, 300), (130, 72, 8200)])
+def test_sizes(width, ff, vocab):
+    check(width, ff, vocab, 40)
+
+
+def test_weights_in_blocks_of_rows():
+    check(320, 40, 40000, 30)
