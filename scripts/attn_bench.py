@@ -22,12 +22,9 @@ def main():
     lib = _b2.load_library()
     _b2.check(lib.b2_init(0))
     dev = torch.device("cuda:0")
-    variants = [("tcgen05 2cta/SM@d64, exp2 half on FMA pipe", "1", "2", "1"), ("tcgen05 2cta/SM@d64, exp2 all MUFU", "1", "2", "0"),
-                ("tcgen05 1cta/SM", "1", "1", "1"), ("mma.sync", "0", "1", "1")]
-    for (tag, tc, ctas, poly), (B, S, H, D, causal) in [(v, sh) for sh in SHAPES for v in variants]:
-        if ctas == "1" and tc == "1" and D != 64:
-            continue  # d=128 has a single tcgen05 build
-        os.environ["B2_FLASH_TC"], os.environ["B2_FLASH_TC_CTAS"], os.environ["B2_FLASH_EXP_POLY"] = tc, ctas, poly
+    variants = [("tcgen05", "1"), ("mma.sync", "0")]
+    for (tag, tc), (B, S, H, D, causal) in [(v, sh) for sh in SHAPES for v in variants]:
+        os.environ["B2_FLASH_TC"] = tc
         g = torch.Generator(device=dev).manual_seed(1)
         q, k, v = (torch.randn(B, S, H, D, device=dev, generator=g).to(torch.bfloat16) for _ in range(3))
         o = torch.empty_like(q)

@@ -1,0 +1,65 @@
+"""bf16 flash attention (csrc/attention_tc.cu) against 64-bit softmax attention at the edges of its tiles (128 queries, 64 keys) and of its
+rings (2 or 3 tiles), with ragged lengths, and with scores that grow along the keys so that the running output is rescaled on every tile."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def attend(q, k, v, lens, causal, scale):
+    B, S, H, D = q.shape
+    out = torch.zeros_like(q, dtype=torch.float64)
+    for b in range(B):
+        n = S if lens is None else int(lens[b])
+        s = torch.einsum("shd,thd->hst", q[b].double(), k[b, :n].double()) * scale
+        if causal:
+            s = s.masked_fill(torch.arange(n, device=s.device) > torch.arange(S, device=s.device)[:, None], float("-inf"))
+        out[b] = torch.einsum("hst,thd->shd", torch.softmax(s, -1), v[b, :n].double())
+    return out
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [0, 1])
+@pytest.mark.parametrize("S", [1, 63, 64, 65, 127, 128, 129, 192, 193, 257, 577])
+@pytest.mark.parametrize("growing", [False, True])
+def test_tile_edges(S, D, causal, growing):
+    from llava import _b2
+
+    lib, P = _b2.init(0), _b2.ptr
+    B, H = 2, 3
+    g = torch.Generator(device="cuda").manual_seed(S + D)
+    q, k, v = (torch.randn(B, S, H, D, device="cuda", generator=g).bfloat16() for _ in range(3))
+    if growing:   # a common direction in q and k whose size grows along the keys: scores rise by far more than 2^8 from tile to tile
+        q[..., 0] = 8.0
+        k[..., 0] = torch.arange(S, device="cuda").div(16, rounding_mode="floor").clamp(max=200).bfloat16()[None, :, None]
+    scale = 1 / math.sqrt(D)
+    for lens in (None, torch.tensor([S, max(1, S // 2)], dtype=torch.int32, device="cuda")):
+        o = torch.empty_like(q)
+        _b2.check(lib.b2_op_flash_attn(P(q), P(k), P(v), P(o), P(lens), B, S, H, D, causal, scale, _b2.stream_ptr()))
+        ref = attend(q, k, v, lens, causal, scale)
+        # P is rounded to bf16 (2^-9 each, of weights that sum to 1) and so is the output: 2^-8 of the largest value, with room for scores of up to
+        # ~150 in fp32 (2^-24 of them in the exponent)
+        tol = 2 ** -8 * float(v.abs().max()) + 2 ** -8
+        for b in range(B):   # rows past a causal request's length are padding
+            n = S if lens is None or not causal else int(lens[b])
+            assert float((o[b, :n].double() - ref[b, :n]).abs().max()) <= tol
+
+
+@pytest.mark.parametrize("D,causal,S,B,H", [(128, 1, 704, 8, 32), (128, 0, 321, 8, 32), (64, 0, 577, 16, 16), (64, 1, 704, 8, 32), (128, 1, 128, 64, 32)])
+def test_full_grids(D, causal, S, B, H):
+    """Several waves of blocks, two on each multiprocessor: products are slow enough here for the softmax of the last tile to end before the product
+    of the tile before it, and the output may only be read after the last one."""
+    from llava import _b2
+
+    lib, P = _b2.init(0), _b2.ptr
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, k, v = (torch.randn(B, S, H, D, device="cuda", generator=g).bfloat16() for _ in range(3))
+    scale = 1 / math.sqrt(D)
+    for _ in range(3):
+        o = torch.empty_like(q)
+        _b2.check(lib.b2_op_flash_attn(P(q), P(k), P(v), P(o), None, B, S, H, D, causal, scale, _b2.stream_ptr()))
+        for b in range(B):
+            ref = attend(q[b:b + 1], k[b:b + 1], v[b:b + 1], None, causal, scale)
+            assert float((o[b:b + 1].double() - ref).abs().max()) <= 2 ** -8 * float(v[b].abs().max()) + 2 ** -8
