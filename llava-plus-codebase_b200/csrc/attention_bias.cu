@@ -49,6 +49,7 @@ __device__ __forceinline__ void store_out(const BiasAttnArgs& a, int row, int he
 
 // unit = q head (normalise, temperature, in place) | k head (normalise, append) | v head (append)
 __global__ void attn_prepare_kernel(BiasAttnArgs a) {
+    pdl_enter();
     const int units = a.H + 2 * a.G;
     const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (w >= a.rows * units) return;
@@ -82,6 +83,7 @@ constexpr int AT_WARPS = 4, AT_MAXC = 8;  // dv <= 32 * AT_MAXC
 
 template <bool VEC>
 __global__ void __launch_bounds__(AT_WARPS * 32) attn_bias_kernel(BiasAttnArgs a) {
+    pdl_enter();
     extern __shared__ float sq[];  // [AT_WARPS][dk]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int w = blockIdx.x * AT_WARPS + warp;
@@ -208,6 +210,7 @@ __device__ __forceinline__ void copy_rows_f4(float* __restrict__ dst, int dpitch
 
 template <bool VEC, int MAXC>
 __global__ void __launch_bounds__(TL_WARPS * 32, MAXC == 16 ? 1 : 2) attn_tile_kernel(BiasAttnArgs a, int QT, int HC) {
+    pdl_enter();
     extern __shared__ float sm[];
     const int HGall = a.H / a.G, chunks = (HGall + HC - 1) / HC;
     const int g = blockIdx.y / chunks, h0 = g * HGall + (blockIdx.y % chunks) * HC, HG = min(HC, g * HGall + HGall - h0);
@@ -387,7 +390,7 @@ __global__ void __launch_bounds__(TL_WARPS * 32, MAXC == 16 ? 1 : 2) attn_tile_k
 // one block per (row, head): every thread turns the splits' (max, sum) into weights (nsplit <= 64 values from L1) and combines
 // its value columns in split order
 __global__ void __launch_bounds__(512) attn_merge_kernel(BiasAttnArgs a) {
-    pdl_trigger_small();
+    pdl_enter();
     const int w = blockIdx.x;
     const int r = w / a.H, h = w % a.H;
     if (a.row_pos[r] < 0) return;
@@ -447,7 +450,7 @@ int attn_prepare_f32(const BiasAttnArgs& a, cudaStream_t st) {
     B2_TRY(check_args(a, "attn_prepare"));
     B2_CHECK_ARG(a.k && a.v && a.temp_every > 0.f, "attn_prepare: null k / v or a non-positive temperature period");
     const int warps = a.rows * (a.H + 2 * a.G);
-    attn_prepare_kernel<<<(warps + 7) / 8, 256, 0, st>>>(a);
+    launch_pdl(attn_prepare_kernel, dim3((warps + 7) / 8), dim3(256), 0, st, a);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -455,10 +458,10 @@ int attn_prepare_f32(const BiasAttnArgs& a, cudaStream_t st) {
 template <bool VEC, int MAXC>
 int launch_tile(const BiasAttnArgs& a, int QT, int HC, dim3 grid, size_t smem, cudaStream_t st) {
     if (smem > 48 * 1024) B2_CUDA_CHECK(cudaFuncSetAttribute(attn_tile_kernel<VEC, MAXC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attn_tile_kernel<VEC, MAXC><<<grid, TL_WARPS * 32, smem, st>>>(a, QT, HC);
+    launch_pdl(attn_tile_kernel<VEC, MAXC>, dim3(grid), dim3(TL_WARPS * 32), smem, st, a, QT, HC);
     B2_LAUNCH_CHECK();
     if (a.nsplit > 1) {
-        attn_merge_kernel<<<a.rows * a.H, a.dv > 256 ? 512 : (a.dv > 128 ? 256 : 128), 0, st>>>(a);
+        launch_pdl(attn_merge_kernel, dim3(a.rows * a.H), dim3(a.dv > 256 ? 512 : (a.dv > 128 ? 256 : 128)), 0, st, a);
         B2_LAUNCH_CHECK();
     }
     return 0;
@@ -489,11 +492,11 @@ int attn_bias_f32(const BiasAttnArgs& a, cudaStream_t st) {
     B2_CHECK_ARG(a.dk <= 256 && a.dv <= 32 * AT_MAXC, "attn_bias: the untiled kernel takes head sizes up to 256");
     dim3 grid((warps + AT_WARPS - 1) / AT_WARPS, a.nsplit);
     const size_t smem = (size_t)AT_WARPS * a.dk * sizeof(float);
-    if (vec) attn_bias_kernel<true><<<grid, AT_WARPS * 32, smem, st>>>(a);
-    else attn_bias_kernel<false><<<grid, AT_WARPS * 32, smem, st>>>(a);
+    if (vec) launch_pdl(attn_bias_kernel<true>, dim3(grid), dim3(AT_WARPS * 32), smem, st, a);
+    else launch_pdl(attn_bias_kernel<false>, dim3(grid), dim3(AT_WARPS * 32), smem, st, a);
     B2_LAUNCH_CHECK();
     if (a.nsplit > 1) {
-        attn_merge_kernel<<<warps, a.dv > 256 ? 512 : (a.dv > 128 ? 256 : 128), 0, st>>>(a);
+        launch_pdl(attn_merge_kernel, dim3(warps), dim3(a.dv > 256 ? 512 : (a.dv > 128 ? 256 : 128)), 0, st, a);
         B2_LAUNCH_CHECK();
     }
     return 0;

@@ -65,6 +65,7 @@ struct SplitSrc {          // rows of one operand: element (head, key, d) at bas
 };
 // index -> key: the kept first positions (nA of them), then the positions from `first` on
 __global__ void __launch_bounds__(256) attn_split_kv_kernel(SplitSrc k, SplitSrc v, int nkeys, int nA, int first) {
+    pdl_enter();
     const SplitSrc s = blockIdx.y == 0 ? k : v;
     const int chunks = s.pitch >> 3;
     const int64_t total = (int64_t)s.heads * nkeys * chunks;
@@ -134,6 +135,7 @@ __device__ __noinline__ float sigmoid_times(float gate, float v) { return v / (1
 template <int DKS, int DVS, int KT, bool EXTRA>   // EXTRA: soft-cap or distance bias
 __global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                                                                    const __grid_constant__ SplitParams p) {
+    pdl_enter();
     using Cfg = SplitCfg<DKS, DVS, KT>;
     constexpr int KH = KT / 2, CH = 32 * DVS;   // keys of a tile and value columns per softmax thread
     extern __shared__ uint8_t sp_raw[];
@@ -409,7 +411,7 @@ int launch_split(const SplitParams& p, const SplitSrc& k, const SplitSrc& v, int
     B2_TRY(make_tmap_parts(&tv, v.out, v.pitch, nkeys, 3 * v.heads, KT));
     auto kernel = p.a.softcap > 0.f || p.a.rel != nullptr ? attn_split_kernel<DKS, DVS, KT, true> : attn_split_kernel<DKS, DVS, KT, false>;
     B2_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));
-    kernel<<<((p.a.rows + p.QT - 1) / p.QT) * p.a.G, SP_THREADS, Cfg::SMEM, st>>>(tk, tv, p);
+    launch_pdl(kernel, dim3(((p.a.rows + p.QT - 1) / p.QT) * p.a.G), dim3(SP_THREADS), Cfg::SMEM, st, tk, tv, p);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -456,7 +458,7 @@ int attn_split_f32(const BiasAttnArgs& a, cudaStream_t st) {
     for (SplitSrc* s : {&k, &v}) s->vec = s->hs % 4 == 0 && s->ks % 4 == 0 && (reinterpret_cast<uintptr_t>(s->base) & 15) == 0;
     const int64_t most = (int64_t)nkeys * (k.heads * (k.pitch / 8) > v.heads * (v.pitch / 8) ? k.heads * (k.pitch / 8) : v.heads * (v.pitch / 8));
     const int64_t blocks = (most + 255) / 256, cap = (int64_t)num_sms() * 8;
-    attn_split_kv_kernel<<<dim3((unsigned)(blocks < cap ? blocks : cap), 2), 256, 0, st>>>(k, v, nkeys, p.nA0, p.first0);
+    launch_pdl(attn_split_kv_kernel, dim3((unsigned)(blocks < cap ? blocks : cap), 2), dim3(256), 0, st, k, v, nkeys, p.nA0, p.first0);
     B2_LAUNCH_CHECK();
     const bool v1 = a.dv <= 64;
     if (a.dk <= 64) return v1 ? launch_split<1, 1, 64>(p, k, v, nkeys, st) : launch_split<1, 2, 64>(p, k, v, nkeys, st);

@@ -63,6 +63,14 @@ __device__ __forceinline__ void pdl_trigger_small() {
     if (gridDim.x * gridDim.y * gridDim.z <= 512) pdl_trigger();
 }
 
+// First statement of a kernel of the layer-list path: it is launched while its predecessor drains, and its own successor while it does. A step
+// or a prompt is a chain of 30..60 kernels of 2..30 us; launched one after the other's end they stood 2.2 us apart in a prompt and ~0.4 us in a
+// captured step: prompts 500 -> 457 us (latent attention with experts, 1536 rows), 419 -> 366 (41 rows of a four-layer model), a step 276 -> 270.
+__device__ __forceinline__ void pdl_enter() {
+    pdl_trigger_small();
+    pdl_wait();
+}
+
 bool pdl_enabled();  // B2_PDL=0 turns the launch attribute off (A/B runs)
 
 // ----------------------------------------------------------------------------------------------

@@ -52,6 +52,7 @@ template <typename TW>
 __global__ void __launch_bounds__(256) linear_rows_vec_kernel(const float* __restrict__ A, int64_t lda, const TW* __restrict__ W, int64_t ldw,
                                                               const float* __restrict__ bias, float* __restrict__ out, int64_t ld_out, int M, int N,
                                                               int K, int kc_max, int act, float alpha, int accumulate, int round_a, DytNorm norm) {
+    pdl_enter();
     extern __shared__ float sA[];  // [M][kc]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ngroups = (N + 8 * RW_COLS - 1) / (8 * RW_COLS);
@@ -134,6 +135,7 @@ template <typename TW, int WPC, bool NORM>
 __global__ void __launch_bounds__(256) linear_one_row_kernel(const float* __restrict__ A, const TW* __restrict__ W, int64_t ldw,
                                                              const float* __restrict__ bias, float* __restrict__ out, int N, int K, int act,
                                                              float alpha, int accumulate, int round_a, DytNorm norm) {
+    pdl_enter();
     extern __shared__ __align__(16) float sA1[];   // [K] with NORM
     __shared__ float part[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -196,10 +198,11 @@ int launch_one_row(const LinearArgs& a, cudaStream_t st) {
     const TW* W = reinterpret_cast<const TW*>(a.W);
     const int grid = (a.N + 8 / WPC - 1) / (8 / WPC);
     if (a.norm.alpha != nullptr)
-        linear_one_row_kernel<TW, WPC, true><<<std::min(grid, 4 * num_sms()), 256, (size_t)a.K * sizeof(float), st>>>(a.A, W, a.ldw, a.bias, a.out, a.N, a.K, a.act, a.alpha, a.accumulate,
-                                                                                          a.round_a, a.norm);
+        launch_pdl(linear_one_row_kernel<TW, WPC, true>, dim3(std::min(grid, 4 * num_sms())), dim3(256), (size_t)a.K * sizeof(float), st, a.A, W, a.ldw,
+                   a.bias, a.out, a.N, a.K, a.act, a.alpha, a.accumulate, a.round_a, a.norm);
     else
-        linear_one_row_kernel<TW, WPC, false><<<grid, 256, 0, st>>>(a.A, W, a.ldw, a.bias, a.out, a.N, a.K, a.act, a.alpha, a.accumulate, a.round_a, a.norm);
+        launch_pdl(linear_one_row_kernel<TW, WPC, false>, dim3(grid), dim3(256), 0, st, a.A, W, a.ldw, a.bias, a.out, a.N, a.K, a.act, a.alpha, a.accumulate,
+                   a.round_a, a.norm);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -209,6 +212,7 @@ template <typename TW>
 __global__ void __launch_bounds__(256) linear_rows_kernel(const float* __restrict__ A, int64_t lda, const TW* __restrict__ W, int64_t ldw,
                                                           const float* __restrict__ bias, float* __restrict__ out, int64_t ld_out, int M, int N,
                                                           int K, int act, float alpha, int accumulate, int round_a) {
+    pdl_enter();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = blockIdx.x * 8 + warp;
     if (n >= N) return;
@@ -242,6 +246,7 @@ template <typename TW>
 __global__ void __launch_bounds__(256) linear_tiled_kernel(const float* __restrict__ A, int64_t lda, const TW* __restrict__ W, int64_t ldw,
                                                            const float* __restrict__ bias, float* __restrict__ out, int64_t ld_out, int M, int N,
                                                            int K, int act, float alpha, int accumulate, int round_a) {
+    pdl_enter();
     __shared__ float As[TK][TB + 4];
     __shared__ float Ws[TK][TB + 4];
     const int tid = threadIdx.x;
@@ -318,22 +323,22 @@ int launch_linear(const LinearArgs& a, cudaStream_t st) {
             if (a.K <= kc_max || a.act == LIN_NONE) {
                 const int grid = a.K <= kc_max ? std::min(ngroups, 3 * num_sms()) : ngroups;
                 const size_t smem = (size_t)a.M * std::min(kc_max, a.K) * sizeof(float);
-                linear_rows_vec_kernel<TW><<<grid, 256, smem, st>>>(a.A, a.lda, W, a.ldw, a.bias, a.out, a.ld_out, a.M, a.N, a.K, kc_max, a.act,
-                                                                  a.alpha, a.accumulate, a.round_a, a.norm);
+                launch_pdl(linear_rows_vec_kernel<TW>, dim3(grid), dim3(256), smem, st, a.A, a.lda, W, a.ldw, a.bias, a.out, a.ld_out, a.M, a.N, a.K, kc_max,
+                           a.act, a.alpha, a.accumulate, a.round_a, a.norm);
                 B2_LAUNCH_CHECK();
                 return 0;
             }
         }
         {
             B2_CHECK_ARG(a.norm.alpha == nullptr, "linear: a norm on the way in needs the vectorised row kernel (K=%d, lda=%lld)", a.K, (long long)a.lda);
-            linear_rows_kernel<TW><<<(a.N + 7) / 8, 256, 0, st>>>(a.A, a.lda, W, a.ldw, a.bias, a.out, a.ld_out, a.M, a.N, a.K, a.act, a.alpha,
-                                                                 a.accumulate, a.round_a);
+            launch_pdl(linear_rows_kernel<TW>, dim3((a.N + 7) / 8), dim3(256), 0, st, a.A, a.lda, W, a.ldw, a.bias, a.out, a.ld_out, a.M, a.N, a.K, a.act,
+                       a.alpha, a.accumulate, a.round_a);
         }
     } else {
         B2_CHECK_ARG(a.norm.alpha == nullptr, "linear: a norm on the way in is for at most %d rows (got %d)", MR, a.M);
         dim3 grid((a.N + TB - 1) / TB, (a.M + TB - 1) / TB);
-        linear_tiled_kernel<TW><<<grid, 256, 0, st>>>(a.A, a.lda, W, a.ldw, a.bias, a.out, a.ld_out, a.M, a.N, a.K, a.act, a.alpha,
-                                                      a.accumulate, a.round_a);
+        launch_pdl(linear_tiled_kernel<TW>, dim3(grid), dim3(256), 0, st, a.A, a.lda, W, a.ldw, a.bias, a.out, a.ld_out, a.M, a.N, a.K, a.act, a.alpha,
+                   a.accumulate, a.round_a);
     }
     B2_LAUNCH_CHECK();
     return 0;
@@ -342,6 +347,7 @@ int launch_linear(const LinearArgs& a, cudaStream_t st) {
 // 64-row tiles: the tiled kernel above with a per-tile weight matrix and gathered input rows. Tiles without a group return.
 template <typename TW>
 __global__ void __launch_bounds__(256) linear_grouped_tiled_kernel(GroupedLinearArgs g) {
+    pdl_enter();
     __shared__ float As[TK][TB + 4];
     __shared__ float Ws[TK][TB + 4];
     const int grp = g.tile_group[blockIdx.y];
@@ -407,6 +413,7 @@ template <typename TW, bool VEC>
 __global__ void __launch_bounds__(256) linear_grouped_rows_kernel(GroupedLinearArgs g) {
     const int m = blockIdx.y;
     pdl_trigger();
+    pdl_wait();
     const int grp = g.tile_group[m];
     if (grp < 0) return;
     const int src = g.a_rows != nullptr ? g.a_rows[m] : m / g.a_div;
@@ -451,6 +458,7 @@ __global__ void __launch_bounds__(256) linear_grouped_rows_kernel(GroupedLinearA
 // four weight loads of 16 bytes in flight per choice.
 template <typename TW, bool VEC>
 __global__ void __launch_bounds__(256) expert_sum_kernel(ExpertSumArgs a) {
+    pdl_enter();
     const int r = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = blockIdx.x * 8 + warp;
     if (n >= a.N) return;
@@ -497,8 +505,8 @@ int launch_expert_sum(const ExpertSumArgs& a, cudaStream_t st) {
     const bool vec = a.K % 8 == 0 && a.lda % 4 == 0 && a.w_group_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(a.a) & 15) == 0 &&
                      (reinterpret_cast<uintptr_t>(a.W) & 15) == 0;
     dim3 grid((a.N + 7) / 8, a.rows);
-    if (vec) expert_sum_kernel<TW, true><<<grid, 256, 0, st>>>(a);
-    else expert_sum_kernel<TW, false><<<grid, 256, 0, st>>>(a);
+    if (vec) launch_pdl(expert_sum_kernel<TW, true>, dim3(grid), dim3(256), 0, st, a);
+    else launch_pdl(expert_sum_kernel<TW, false>, dim3(grid), dim3(256), 0, st, a);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -509,6 +517,7 @@ template <typename TW, bool VEC>
 __global__ void __launch_bounds__(256) linear_batched_rows_kernel(const float* __restrict__ A, int64_t lda, int64_t a_bs, const TW* __restrict__ W,
                                                                   int64_t w_bs, float* __restrict__ out, int64_t ld_out, int64_t o_bs, int M, int N,
                                                                   int K, int round_a, const float* __restrict__ gate, int64_t ldg) {
+    pdl_enter();
     const int b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = blockIdx.x * 8 + warp;
     if (n >= N) return;
@@ -556,8 +565,9 @@ int launch_batched_rows(const float* A, int64_t lda, int64_t a_bs, const void* W
                      (reinterpret_cast<uintptr_t>(W) & 15) == 0;
     dim3 grid((N + 7) / 8, batch);
     const TW* w = reinterpret_cast<const TW*>(W);
-    if (vec) linear_batched_rows_kernel<TW, true><<<grid, 256, 0, st>>>(A, lda, a_bs, w, w_bs, out, ld_out, o_bs, M, N, K, round_a, gate, ldg);
-    else linear_batched_rows_kernel<TW, false><<<grid, 256, 0, st>>>(A, lda, a_bs, w, w_bs, out, ld_out, o_bs, M, N, K, round_a, gate, ldg);
+    if (vec) launch_pdl(linear_batched_rows_kernel<TW, true>, dim3(grid), dim3(256), 0, st, A, lda, a_bs, w, w_bs, out, ld_out, o_bs, M, N, K, round_a, gate,
+                        ldg);
+    else launch_pdl(linear_batched_rows_kernel<TW, false>, dim3(grid), dim3(256), 0, st, A, lda, a_bs, w, w_bs, out, ld_out, o_bs, M, N, K, round_a, gate, ldg);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -568,11 +578,11 @@ int launch_grouped(const GroupedLinearArgs& g, cudaStream_t st) {
         const bool vec = g.K % 8 == 0 && g.lda % 4 == 0 && g.ldw % 8 == 0 && g.w_group_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(g.A) & 15) == 0 &&
                          (reinterpret_cast<uintptr_t>(g.W) & 15) == 0;
         dim3 grid((g.N + 7) / 8, g.M);
-        if (vec) linear_grouped_rows_kernel<TW, true><<<grid, 256, 0, st>>>(g);
-        else linear_grouped_rows_kernel<TW, false><<<grid, 256, 0, st>>>(g);
+        if (vec) launch_pdl(linear_grouped_rows_kernel<TW, true>, dim3(grid), dim3(256), 0, st, g);
+        else launch_pdl(linear_grouped_rows_kernel<TW, false>, dim3(grid), dim3(256), 0, st, g);
     } else {
         dim3 grid((g.N + TB - 1) / TB, (g.M + TB - 1) / TB);
-        linear_grouped_tiled_kernel<TW><<<grid, 256, 0, st>>>(g);
+        launch_pdl(linear_grouped_tiled_kernel<TW>, dim3(grid), dim3(256), 0, st, g);
     }
     B2_LAUNCH_CHECK();
     return 0;
@@ -604,6 +614,7 @@ int expert_sum_f32(const ExpertSumArgs& a, cudaStream_t st) {
 
 namespace {
 __global__ void cast_rows_bf16_kernel(const float* __restrict__ A, int64_t lda, __nv_bfloat16* __restrict__ out, int64_t ld_out, int K) {
+    pdl_enter();
     const size_t r = blockIdx.y;
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) * 2;
     if (k + 1 < K) {
@@ -616,7 +627,7 @@ __global__ void cast_rows_bf16_kernel(const float* __restrict__ A, int64_t lda, 
 
 int cast_rows_bf16(const float* A, int64_t lda, void* out, int64_t ld_out, int M, int K, cudaStream_t st) {
     B2_CHECK_ARG(A && out && M > 0 && K > 0 && ld_out % 2 == 0, "cast_rows_bf16: bad argument");
-    cast_rows_bf16_kernel<<<dim3((K / 2 + 256) / 256, M), 256, 0, st>>>(A, lda, reinterpret_cast<__nv_bfloat16*>(out), ld_out, K);
+    launch_pdl(cast_rows_bf16_kernel, dim3((K / 2 + 256) / 256, M), dim3(256), 0, st, A, lda, reinterpret_cast<__nv_bfloat16*>(out), ld_out, K);
     B2_LAUNCH_CHECK();
     return 0;
 }

@@ -31,6 +31,7 @@ struct LxCfg {
 
 // rows of fp32 -> [part][rows][pitch] bf16, entries past K zero
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ in, int64_t ld, int rows, int K, int pitch, __nv_bfloat16* __restrict__ out, int vec) {
+    pdl_enter();
     const int chunks = pitch >> 3;
     const int64_t total = (int64_t)rows * chunks, plane = (int64_t)rows * pitch;
     for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < total; e += (int64_t)gridDim.x * 256) {
@@ -51,6 +52,7 @@ __device__ __noinline__ float lx_act(float v, int act) { return epi_post_act(v, 
 
 template <int BN>
 __global__ void __launch_bounds__(LX_THREADS, 1) linear_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w, LinearArgs a) {
+    pdl_enter();
     using Cfg = LxCfg<BN>;
     constexpr int CH = BN / 2;   // columns per epilogue thread
     extern __shared__ uint8_t lx_raw[];
@@ -167,7 +169,7 @@ __global__ void __launch_bounds__(LX_THREADS, 1) linear_split_kernel(const __gri
 int split_rows(const float* in, int64_t ld, int rows, int K, int pitch, __nv_bfloat16* out, cudaStream_t st) {
     const int vec = ld % 4 == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0;
     const int64_t blocks = ((int64_t)rows * (pitch / 8) + 255) / 256;
-    split_rows_kernel<<<(unsigned)std::min<int64_t>(blocks, 8 * num_sms()), 256, 0, st>>>(in, ld, rows, K, pitch, out, vec);
+    launch_pdl(split_rows_kernel, dim3((unsigned)std::min<int64_t>(blocks, 8 * num_sms())), dim3(256), 0, st, in, ld, rows, K, pitch, out, vec);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -178,7 +180,7 @@ int launch_split_linear(const LinearArgs& a, const __nv_bfloat16* pa, const __nv
     B2_TRY(make_tmap_parts(&ta, pa, pitch, a.M, 3, LX_M));
     B2_TRY(make_tmap_parts(&tw, pw, pitch, a.N, 3, BN));
     B2_CUDA_CHECK(cudaFuncSetAttribute(linear_split_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, LxCfg<BN>::SMEM));
-    linear_split_kernel<BN><<<((a.M + LX_M - 1) / LX_M) * ((a.N + BN - 1) / BN), LX_THREADS, LxCfg<BN>::SMEM, st>>>(ta, tw, a);
+    launch_pdl(linear_split_kernel<BN>, dim3(((a.M + LX_M - 1) / LX_M) * ((a.N + BN - 1) / BN)), dim3(LX_THREADS), LxCfg<BN>::SMEM, st, ta, tw, a);
     B2_LAUNCH_CHECK();
     return 0;
 }

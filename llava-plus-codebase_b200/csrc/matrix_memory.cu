@@ -41,6 +41,7 @@ __device__ __forceinline__ float sum32(float v) {
 // VEC: dk % 4 == 0 and q / k rows are 16-byte aligned
 template <int MODE, int KPT, bool VEC>
 __global__ void __launch_bounds__(MM_THREADS) matrix_memory_kernel(MemoryArgs a) {
+    pdl_enter();
     constexpr int DKP = KPT * MM_L;                      // keys a CTA holds (the ones past dk stay zero)
     extern __shared__ __align__(16) float sm[];
     float* sQ = sm;                                      // [2][TT][DKP]
@@ -284,7 +285,7 @@ int launch_memory(const MemoryArgs& a, cudaStream_t st) {
     const int ncol = a.mode == MEM_MLSTM ? a.dv + 1 : a.dv;
     const size_t smem = ((size_t)4 * MM_TT * KPT * MM_L + 2 * MM_TT * MM_COLS + 4 * MM_TT + 8 * MM_TT + MM_TT * MM_COLS) * sizeof(float);
     if (smem > 48 * 1024) B2_CUDA_CHECK(cudaFuncSetAttribute(matrix_memory_kernel<MODE, KPT, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    matrix_memory_kernel<MODE, KPT, VEC><<<dim3(mem_blocks(ncol), a.heads, a.nseg), MM_THREADS, smem, st>>>(a);
+    launch_pdl(matrix_memory_kernel<MODE, KPT, VEC>, dim3(mem_blocks(ncol), a.heads, a.nseg), dim3(MM_THREADS), smem, st, a);
     B2_LAUNCH_CHECK();
     return 0;
 }

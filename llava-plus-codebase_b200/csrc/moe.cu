@@ -24,6 +24,7 @@ __device__ __forceinline__ void warp_argmax(float& v, int& i) {
 
 // One warp per row. Shared memory per warp: E scores, G group scores (later: group alive flags), E taken flags, E choice scores.
 __global__ void moe_route_kernel(MoeRouteArgs a) {
+    pdl_enter();
     extern __shared__ float sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = blockIdx.x * (blockDim.x >> 5) + warp;
@@ -106,6 +107,7 @@ __global__ void moe_route_kernel(MoeRouteArgs a) {
 __global__ void __launch_bounds__(1024) moe_plan_kernel(const int32_t* __restrict__ idx, int pairs, int top, int experts, int tile, int max_tiles,
                                                         int32_t* __restrict__ pair_pos, int32_t* __restrict__ src_row,
                                                         int32_t* __restrict__ tile_group) {
+    pdl_enter();
     extern __shared__ int cnt[];   // [experts] counts, then [experts] offsets
     int* off = cnt + experts;
     for (int e = threadIdx.x; e < experts; e += blockDim.x) cnt[e] = 0;
@@ -133,7 +135,7 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int32_t* __restric
 // out[r, c] = act(in[r, c], in[r, ff + c]): the gated unit (SiLU(g) u, or its bounded and shifted form)
 __global__ void glu_rows_kernel(const float* __restrict__ in, int64_t ld_in, float* __restrict__ out, int64_t ld_out, int ff,
                                 __nv_bfloat16* __restrict__ out16, int64_t ld_out16, GluAct act) {
-    pdl_trigger_small();
+    pdl_enter();
     const size_t r = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < ff) {
@@ -145,6 +147,7 @@ __global__ void glu_rows_kernel(const float* __restrict__ in, int64_t ld_in, flo
 
 __global__ void gather_rows_bf16_kernel(const float* __restrict__ A, int64_t lda, const int32_t* __restrict__ src_row, __nv_bfloat16* __restrict__ out,
                                         int64_t ld_out, int K) {
+    pdl_enter();
     const size_t p = blockIdx.y;
     const int src = src_row[p];
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) * 2;
@@ -159,6 +162,7 @@ __global__ void gather_rows_bf16_kernel(const float* __restrict__ A, int64_t lda
 // x[r] += alpha * sum_k w[r, k] * y[pair_pos[r * top + k]] (a negative position: h[r] in y's place)
 __global__ void moe_combine_kernel(float* __restrict__ x, const float* __restrict__ y, int64_t ldy, const int32_t* __restrict__ pair_pos,
                                    const float* __restrict__ w, int top, int cols, float alpha, const float* __restrict__ h, int64_t ldh) {
+    pdl_enter();
     const size_t r = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= cols) return;
@@ -181,7 +185,7 @@ int moe_route_f32(const MoeRouteArgs& a, cudaStream_t st) {
     B2_CHECK_ARG(a.identity >= 0 && a.identity < a.experts, "moe_route: %d identity experts of %d", a.identity, a.experts);
     const size_t smem = (size_t)warps * (3 * a.experts + a.groups) * sizeof(float);
     B2_CHECK_ARG(smem <= 48 * 1024, "moe_route: %d experts exceed the router kernel's shared memory", a.experts);
-    moe_route_kernel<<<(a.rows + warps - 1) / warps, warps * 32, smem, st>>>(a);
+    launch_pdl(moe_route_kernel, dim3((a.rows + warps - 1) / warps), dim3(warps * 32), smem, st, a);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -190,7 +194,8 @@ int moe_plan(const int32_t* idx, int rows, int top, int experts, int tile, int m
              cudaStream_t st) {
     B2_CHECK_ARG(idx && pair_pos && src_row && tile_group && rows > 0 && top > 0 && experts > 0 && tile > 0, "moe_plan: bad argument");
     B2_CHECK_ARG((size_t)max_tiles * tile >= (size_t)rows * top + (size_t)experts * (tile - 1), "moe_plan: %d tiles cannot hold the padded pairs", max_tiles);
-    moe_plan_kernel<<<1, 1024, 2 * experts * sizeof(int), st>>>(idx, rows * top, top, experts, tile, max_tiles, pair_pos, src_row, tile_group);
+    launch_pdl(moe_plan_kernel, dim3(1), dim3(1024), 2 * experts * sizeof(int), st, idx, rows * top, top, experts, tile, max_tiles, pair_pos, src_row,
+               tile_group);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -198,14 +203,15 @@ int moe_plan(const int32_t* idx, int rows, int top, int experts, int tile, int m
 int glu_rows_f32(const float* in, int64_t ld_in, float* out, int64_t ld_out, int rows, int ff, const GluAct& act, cudaStream_t st, void* out16,
                  int64_t ld_out16) {
     B2_CHECK_ARG(in && (out || out16) && rows > 0 && ff > 0, "glu_rows: bad argument");
-    glu_rows_kernel<<<dim3((ff + 255) / 256, rows), 256, 0, st>>>(in, ld_in, out, ld_out, ff, reinterpret_cast<__nv_bfloat16*>(out16), ld_out16, act);
+    launch_pdl(glu_rows_kernel, dim3((ff + 255) / 256, rows), dim3(256), 0, st, in, ld_in, out, ld_out, ff, reinterpret_cast<__nv_bfloat16*>(out16),
+               ld_out16, act);
     B2_LAUNCH_CHECK();
     return 0;
 }
 
 int gather_rows_bf16(const float* A, int64_t lda, const int32_t* src_row, void* out, int64_t ld_out, int rows, int K, cudaStream_t st) {
     B2_CHECK_ARG(A && src_row && out && rows > 0 && K > 0 && ld_out % 2 == 0, "gather_rows_bf16: bad argument");
-    gather_rows_bf16_kernel<<<dim3((K / 2 + 256) / 256, rows), 256, 0, st>>>(A, lda, src_row, reinterpret_cast<__nv_bfloat16*>(out), ld_out, K);
+    launch_pdl(gather_rows_bf16_kernel, dim3((K / 2 + 256) / 256, rows), dim3(256), 0, st, A, lda, src_row, reinterpret_cast<__nv_bfloat16*>(out), ld_out, K);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -213,7 +219,7 @@ int gather_rows_bf16(const float* A, int64_t lda, const int32_t* src_row, void* 
 int moe_combine_f32(float* x, const float* y, int64_t ldy, const int32_t* pair_pos, const float* w, int rows, int top, int cols, float alpha,
                     cudaStream_t st, const float* h, int64_t ldh) {
     B2_CHECK_ARG(x && y && w && pair_pos && rows > 0 && top > 0 && cols > 0, "moe_combine: bad argument");
-    moe_combine_kernel<<<dim3((cols + 255) / 256, rows), 256, 0, st>>>(x, y, ldy, pair_pos, w, top, cols, alpha, h, ldh);
+    launch_pdl(moe_combine_kernel, dim3((cols + 255) / 256, rows), dim3(256), 0, st, x, y, ldy, pair_pos, w, top, cols, alpha, h, ldh);
     B2_LAUNCH_CHECK();
     return 0;
 }

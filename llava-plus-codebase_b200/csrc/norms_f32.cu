@@ -44,6 +44,7 @@ __device__ __forceinline__ void row_stats(const float* y, int cols, float eps, f
 
 __global__ void layernorm_add_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ gamma,
                                      const float* __restrict__ beta, int cols, float eps) {
+    pdl_enter();
     __shared__ float red[33];
     const size_t r = blockIdx.x;
     const float* yr = y + r * cols;
@@ -54,6 +55,7 @@ __global__ void layernorm_add_kernel(float* __restrict__ x, const float* __restr
 
 __global__ void layernorm_gather_kernel(const float* __restrict__ x, const int32_t* __restrict__ row_index, const float* __restrict__ gamma,
                                         const float* __restrict__ beta, float* __restrict__ out, int cols, float eps) {
+    pdl_enter();
     __shared__ float red[33];
     const size_t r = blockIdx.x;
     const float* xr = x + (size_t)(row_index != nullptr ? row_index[r] : (int)r) * cols;  // null index: row r itself
@@ -69,7 +71,7 @@ __global__ void gated_group_rmsnorm_kernel(const float* __restrict__ y, int64_t 
                                            const float* __restrict__ gamma, float* __restrict__ out, int64_t ldo, int rows, int groups, int group,
                                            int gate_first, int gamma_shared, float eps, int sigmoid_gate, const float* __restrict__ den,
                                            __nv_bfloat16* __restrict__ out16, int64_t ldo16) {
-    pdl_trigger_small();
+    pdl_enter();
     const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (w >= rows * groups) return;
     const int r = w / groups, g = w % groups;
@@ -100,6 +102,7 @@ __device__ __forceinline__ float dyt_f(float x, float alpha, float w, float b) {
 template <bool VEC>
 __global__ void __launch_bounds__(256) dyt_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ row_index, DytOuts outs, int n_outs,
                                                        int cols) {
+    pdl_enter();
     const size_t r = blockIdx.y;
     const float* xr = x + (size_t)(row_index != nullptr ? row_index[r] : (int)r) * cols;
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * (VEC ? 4 : 1);
@@ -133,6 +136,7 @@ __global__ void __launch_bounds__(256) dyt_rows_kernel(const float* __restrict__
 
 __global__ void __launch_bounds__(256) concat_rows_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out,
                                                           __nv_bfloat16* __restrict__ out16, int cols) {
+    pdl_enter();
     const size_t r = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= 2 * cols) return;
@@ -145,7 +149,7 @@ __global__ void __launch_bounds__(256) concat_rows_kernel(const float* __restric
 // the difference to unit RMS
 __global__ void diff_combine_kernel(const float* __restrict__ y, int64_t ldy, float* __restrict__ out, int64_t ldo, int rows, int heads, int dv,
                                     float lambda, float out_scale, float eps) {
-    pdl_trigger_small();
+    pdl_enter();
     const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (w >= rows * heads) return;
     const int r = w / heads, h = w % heads;
@@ -165,6 +169,7 @@ __global__ void diff_combine_kernel(const float* __restrict__ y, int64_t ldy, fl
 template <typename TT>
 __global__ void embed_rows_kernel(const int32_t* __restrict__ tokens, const TT* __restrict__ table, float* __restrict__ x, int cols, int vocab,
                                   int* err_flag, float scale) {
+    pdl_enter();
     const size_t r = blockIdx.x;
     const int t = tokens[r];
     const bool ok = t >= 0 && t < vocab;
@@ -174,6 +179,7 @@ __global__ void embed_rows_kernel(const int32_t* __restrict__ tokens, const TT* 
 
 __global__ void sigmoid_gate_kernel(const float* __restrict__ a, int64_t lda, const float* __restrict__ g, int64_t ldg, float* __restrict__ out,
                                     int64_t ldo, int cols) {
+    pdl_enter();
     const size_t r = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < cols) out[r * ldo + c] = a[r * lda + c] / (1.f + expf(-g[r * ldg + c]));
@@ -184,6 +190,7 @@ __global__ void sigmoid_gate_kernel(const float* __restrict__ a, int64_t lda, co
 // x += add[row] + vec (the opening of a pass of a looped block of layers)
 __global__ void rms_scalar_kernel(float* __restrict__ x, const int32_t* __restrict__ row_index, const float* __restrict__ g,
                                   const float* __restrict__ add, const float* __restrict__ vec, float* __restrict__ out, int cols, float eps) {
+    pdl_enter();
     __shared__ float red[33];
     const size_t r = blockIdx.x;
     const size_t src = row_index != nullptr ? (size_t)row_index[r] : r;
@@ -205,6 +212,7 @@ __global__ void rms_scalar_kernel(float* __restrict__ x, const int32_t* __restri
 // weighted RMS norm of a (gathered) row; accumulate: added onto out
 __global__ void rms_weight_kernel(const float* __restrict__ in, int64_t ld_in, const int32_t* __restrict__ row_index, const float* __restrict__ w,
                                   float* __restrict__ out, int64_t ld_out, int accumulate, int cols, float eps, __nv_bfloat16* __restrict__ out16) {
+    pdl_enter();
     __shared__ float red[33];
     const size_t r = blockIdx.x;
     const float* xr = in + (row_index != nullptr ? (size_t)row_index[r] : r) * ld_in;
@@ -225,8 +233,8 @@ template <int V>
 __global__ void __launch_bounds__(256) rms_weight_reg_kernel(const float* in, int64_t ld_in, const int32_t* __restrict__ row_index,
                                                              const float* __restrict__ w, float* out, int64_t ld_out, int accumulate, int cols, float eps,
                                                              __nv_bfloat16* __restrict__ out16) {
+    pdl_enter();
     __shared__ float red[33];
-    pdl_trigger_small();
     const size_t r = blockIdx.x;
     const float* xr = in + (row_index != nullptr ? (size_t)row_index[r] : r) * ld_in;
     float4 x[V], g[V];
@@ -269,6 +277,7 @@ __global__ void __launch_bounds__(256) rms_weight_reg_kernel(const float* in, in
 template <typename TT>
 __global__ void embed_norm_kernel(const int32_t* __restrict__ tokens, const TT* __restrict__ table, float* __restrict__ x, int cols, int vocab,
                                   int* err_flag, const float* __restrict__ w, float eps) {
+    pdl_enter();
     __shared__ float red[33];
     const size_t r = blockIdx.x;
     const int t = tokens[r];
@@ -290,6 +299,7 @@ __device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
 template <typename TT, int V>
 __global__ void __launch_bounds__(256) embed_norm_reg_kernel(const int32_t* __restrict__ tokens, const TT* __restrict__ table, float* __restrict__ x,
                                                              int cols, int vocab, int* err_flag, const float* __restrict__ w, float eps) {
+    pdl_enter();
     __shared__ float red[33];
     const size_t r = blockIdx.x;
     const int t = tokens[r];
@@ -321,10 +331,10 @@ template <typename TT>
 int launch_embed_norm(const int32_t* tokens, const TT* table, float* x, int rows, int cols, int vocab, int* err_flag, const float* w, float eps, cudaStream_t st) {
     const uintptr_t align = reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w);
     if (cols % 4 == 0 && cols <= 8192 && (align & 15) == 0) {
-        if (cols <= 2048) embed_norm_reg_kernel<TT, 2><<<rows, 256, 0, st>>>(tokens, table, x, cols, vocab, err_flag, w, eps);
-        else embed_norm_reg_kernel<TT, 8><<<rows, 256, 0, st>>>(tokens, table, x, cols, vocab, err_flag, w, eps);
+        if (cols <= 2048) launch_pdl(embed_norm_reg_kernel<TT, 2>, dim3(rows), dim3(256), 0, st, tokens, table, x, cols, vocab, err_flag, w, eps);
+        else launch_pdl(embed_norm_reg_kernel<TT, 8>, dim3(rows), dim3(256), 0, st, tokens, table, x, cols, vocab, err_flag, w, eps);
     } else {
-        embed_norm_kernel<TT><<<rows, 256, 0, st>>>(tokens, table, x, cols, vocab, err_flag, w, eps);
+        launch_pdl(embed_norm_kernel<TT>, dim3(rows), dim3(256), 0, st, tokens, table, x, cols, vocab, err_flag, w, eps);
     }
     B2_LAUNCH_CHECK();
     return 0;
@@ -332,6 +342,7 @@ int launch_embed_norm(const int32_t* tokens, const TT* table, float* x, int rows
 
 // post-norm add of one sublayer, pre-norm of the next, and (decode steps) the input convolution with its carried inputs
 __global__ void sandwich_norm_kernel(SandwichNormArgs a) {
+    pdl_enter();
     __shared__ float red[33];
     const size_t r = blockIdx.x;
     const int cols = a.cols;
@@ -387,6 +398,7 @@ __global__ void sandwich_norm_kernel(SandwichNormArgs a) {
 // row and is bound by round trips, not by bandwidth).
 template <int V, int TP>
 __global__ void __launch_bounds__(512) sandwich_norm_reg_kernel(SandwichNormArgs a) {
+    pdl_enter();
     __shared__ float red[33];
     const size_t r = blockIdx.x;
     const int cols = a.cols, tid = threadIdx.x, nt = blockDim.x;
@@ -469,6 +481,7 @@ __global__ void transpose_blocks_kernel(const T* __restrict__ src, T* __restrict
 // PolyNorm: out = a N(z) + b N(z^2) + c N(z^3) + e with z = in + bias, powers element-wise, N = division by the row's root mean square
 __global__ void polynorm_kernel(const float* __restrict__ in, int64_t ld_in, const float* __restrict__ bias, const float* __restrict__ coef,
                                 float* __restrict__ out, int64_t ld_out, int cols, float eps, int vec) {
+    pdl_enter();
     __shared__ float red[33];
     const size_t r = blockIdx.x;
     const float* zr = in + r * ld_in;
@@ -517,6 +530,7 @@ __global__ void polynorm_kernel(const float* __restrict__ in, int64_t ld_in, con
 
 // x[i] = cap * tanh(x[i] / cap)
 __global__ void softcap_kernel(float* __restrict__ x, size_t n, float cap) {
+    pdl_enter();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] = cap * tanhf(x[i] / cap);
 }
@@ -524,6 +538,7 @@ __global__ void softcap_kernel(float* __restrict__ x, size_t n, float cap) {
 // out[r, h * dv + d] = a[r, h * dv + d] * sigmoid(g[r, h]): one gate per head
 __global__ void head_gate_kernel(const float* __restrict__ a, int64_t lda, const float* __restrict__ g, int64_t ldg, float* __restrict__ out,
                                  int64_t ldo, int heads, int dv) {
+    pdl_enter();
     const size_t r = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < heads * dv) out[r * ldo + c] = a[r * lda + c] / (1.f + expf(-g[r * ldg + c / dv]));
@@ -536,6 +551,7 @@ template <typename TT>
 __global__ void embed_bigram_kernel(const int32_t* __restrict__ tokens, const SeqSeg* __restrict__ segs, const TT* __restrict__ table,
                                     const TT* __restrict__ bigram, int32_t* __restrict__ last_tok, float* __restrict__ x, float* __restrict__ x0,
                                     int cols, int vocab, int buckets, int mul_prev, int mul_cur, int* err_flag) {
+    pdl_enter();
     const SeqSeg sg = segs[blockIdx.y];
     const int t = blockIdx.x;
     if (t >= sg.n) return;
@@ -566,6 +582,7 @@ __global__ void embed_bigram_kernel(const int32_t* __restrict__ tokens, const Se
 // latent[slot][pos] = unit_rms(in[r]) * gamma: the normalised low-rank row that a token leaves in the cache
 __global__ void latent_append_kernel(const float* __restrict__ in, int64_t ld_in, const float* __restrict__ gamma, float* __restrict__ cache,
                                      const int32_t* __restrict__ row_slot, const int32_t* __restrict__ row_pos, int rank, int Smax, float eps) {
+    pdl_enter();
     __shared__ float red[33];
     const size_t r = blockIdx.x;
     const int pos = row_pos[r];
@@ -579,6 +596,7 @@ __global__ void latent_append_kernel(const float* __restrict__ in, int64_t ld_in
 }
 
 __global__ void rowmap_portion_kernel(SeqSeg* segs, int32_t* row_slot, int32_t* row_pos, int32_t* len, int slot, int n, int restart) {
+    pdl_enter();
     const int pos0 = restart ? 0 : len[slot];
     __syncthreads();
     for (int r = threadIdx.x; r < n; r += blockDim.x) { row_slot[r] = slot; row_pos[r] = pos0 + r; }
@@ -590,6 +608,7 @@ __global__ void rowmap_portion_kernel(SeqSeg* segs, int32_t* row_slot, int32_t* 
 
 __global__ void rowmap_decode_kernel(SeqSeg* segs, int32_t* row_slot, int32_t* row_pos, const int32_t* len, const SampleState* sstate,
                                      const RowState* rows_state, int slot0, int B) {
+    pdl_enter();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= B) return;
     const int slot = slot0 + b;
@@ -604,7 +623,7 @@ __global__ void rowmap_decode_kernel(SeqSeg* segs, int32_t* row_slot, int32_t* r
 
 int layernorm_add_f32(float* x, const float* y, const float* gamma, const float* beta, int rows, int cols, float eps, cudaStream_t st) {
     B2_CHECK_ARG(x && y && gamma && beta && rows > 0 && cols > 0, "layernorm_add: bad argument");
-    layernorm_add_kernel<<<rows, cols >= 1024 ? 256 : 128, 0, st>>>(x, y, gamma, beta, cols, eps);
+    launch_pdl(layernorm_add_kernel, dim3(rows), dim3(cols >= 1024 ? 256 : 128), 0, st, x, y, gamma, beta, cols, eps);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -612,7 +631,7 @@ int layernorm_add_f32(float* x, const float* y, const float* gamma, const float*
 int layernorm_gather_f32(const float* x, const int32_t* row_index, const float* gamma, const float* beta, float* out, int rows, int cols,
                          float eps, cudaStream_t st) {
     B2_CHECK_ARG(x && gamma && beta && out && rows > 0 && cols > 0, "layernorm_gather: bad argument");
-    layernorm_gather_kernel<<<rows, cols >= 1024 ? 256 : 128, 0, st>>>(x, row_index, gamma, beta, out, cols, eps);
+    launch_pdl(layernorm_gather_kernel, dim3(rows), dim3(cols >= 1024 ? 256 : 128), 0, st, x, row_index, gamma, beta, out, cols, eps);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -623,8 +642,8 @@ int gated_group_rmsnorm_f32(const float* y, int64_t ldy, const float* z, int64_t
     B2_CHECK_ARG(y && z && gamma && (out || out16) && rows > 0 && group > 0 && cols % group == 0, "gated_group_rmsnorm: cols %d is not a multiple of the group %d",
                  cols, group);
     const int groups = cols / group, warps = rows * groups;
-    gated_group_rmsnorm_kernel<<<(warps + 7) / 8, 256, 0, st>>>(y, ldy, z, ldz, gamma, out, ldo, rows, groups, group, gate_first, gamma_shared, eps,
-                                                               sigmoid_gate, den, reinterpret_cast<__nv_bfloat16*>(out16), ld_out16);
+    launch_pdl(gated_group_rmsnorm_kernel, dim3((warps + 7) / 8), dim3(256), 0, st, y, ldy, z, ldz, gamma, out, ldo, rows, groups, group, gate_first,
+               gamma_shared, eps, sigmoid_gate, den, reinterpret_cast<__nv_bfloat16*>(out16), ld_out16);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -633,8 +652,8 @@ int group_rmsnorm_f32(const float* y, int64_t ldy, const float* gamma, int gamma
                       float eps, cudaStream_t st) {
     B2_CHECK_ARG(y && gamma && out && rows > 0 && group > 0 && cols % group == 0, "group_rmsnorm: cols %d is not a multiple of the group %d", cols, group);
     const int groups = cols / group, warps = rows * groups;
-    gated_group_rmsnorm_kernel<<<(warps + 7) / 8, 256, 0, st>>>(y, ldy, nullptr, 0, gamma, out, ldo, rows, groups, group, 0, gamma_shared, eps,
-                                                               0, nullptr, nullptr, 0);
+    launch_pdl(gated_group_rmsnorm_kernel, dim3((warps + 7) / 8), dim3(256), 0, st, y, ldy, nullptr, 0, gamma, out, ldo, rows, groups, group, 0,
+               gamma_shared, eps, 0, nullptr, nullptr, 0);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -643,7 +662,7 @@ int diff_combine_f32(const float* y, int64_t ldy, float* out, int64_t ldo, int r
                      cudaStream_t st) {
     B2_CHECK_ARG(y && out && y != out && rows > 0 && heads > 0 && dv > 0, "diff_combine: bad argument");
     const int warps = rows * heads;
-    diff_combine_kernel<<<(warps + 7) / 8, 256, 0, st>>>(y, ldy, out, ldo, rows, heads, dv, lambda, out_scale, eps);
+    launch_pdl(diff_combine_kernel, dim3((warps + 7) / 8), dim3(256), 0, st, y, ldy, out, ldo, rows, heads, dv, lambda, out_scale, eps);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -656,16 +675,17 @@ int embed_rows_f32(const int32_t* tokens, const void* table, int table_dtype, fl
         return launch_embed_norm(tokens, reinterpret_cast<const __nv_bfloat16*>(table), x, rows, cols, vocab, err_flag, norm_w, eps, st);
     }
     if (table_dtype == DT_F32)
-        embed_rows_kernel<float><<<rows, 128, 0, st>>>(tokens, reinterpret_cast<const float*>(table), x, cols, vocab, err_flag, scale);
+        launch_pdl(embed_rows_kernel<float>, dim3(rows), dim3(128), 0, st, tokens, reinterpret_cast<const float*>(table), x, cols, vocab, err_flag, scale);
     else
-        embed_rows_kernel<__nv_bfloat16><<<rows, 128, 0, st>>>(tokens, reinterpret_cast<const __nv_bfloat16*>(table), x, cols, vocab, err_flag, scale);
+        launch_pdl(embed_rows_kernel<__nv_bfloat16>, dim3(rows), dim3(128), 0, st, tokens, reinterpret_cast<const __nv_bfloat16*>(table), x, cols, vocab,
+                   err_flag, scale);
     B2_LAUNCH_CHECK();
     return 0;
 }
 
 int sigmoid_gate_f32(const float* a, int64_t lda, const float* g, int64_t ldg, float* out, int64_t ldo, int rows, int cols, cudaStream_t st) {
     B2_CHECK_ARG(a && g && out && rows > 0 && cols > 0, "sigmoid_gate: bad argument");
-    sigmoid_gate_kernel<<<dim3((cols + 255) / 256, rows), 256, 0, st>>>(a, lda, g, ldg, out, ldo, cols);
+    launch_pdl(sigmoid_gate_kernel, dim3((cols + 255) / 256, rows), dim3(256), 0, st, a, lda, g, ldg, out, ldo, cols);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -673,7 +693,7 @@ int sigmoid_gate_f32(const float* a, int64_t lda, const float* g, int64_t ldg, f
 int rms_scalar_f32(float* x, const int32_t* row_index, const float* g, const float* add, const float* vec, float* out, int rows, int cols,
                    float eps, cudaStream_t st) {
     B2_CHECK_ARG(x && rows > 0 && cols > 0 && ((g && out) || (!out && (add || vec))), "rms_scalar: bad argument");
-    rms_scalar_kernel<<<rows, cols >= 1024 ? 256 : 128, 0, st>>>(x, row_index, g, add, vec, out, cols, eps);
+    launch_pdl(rms_scalar_kernel, dim3(rows), dim3(cols >= 1024 ? 256 : 128), 0, st, x, row_index, g, add, vec, out, cols, eps);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -684,12 +704,14 @@ int rms_weight_f32(const float* in, int64_t ld_in, const int32_t* row_index, con
     __nv_bfloat16* o16 = reinterpret_cast<__nv_bfloat16*>(out16);
     const uintptr_t align = reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out16);
     if (cols % 4 == 0 && ld_in % 4 == 0 && ld_out % 4 == 0 && (align & 15) == 0 && cols <= 8192) {
-        if (cols <= 512) rms_weight_reg_kernel<1><<<rows, 128, 0, st>>>(in, ld_in, row_index, w, out, ld_out, accumulate, cols, eps, o16);
-        else if (cols <= 2048) rms_weight_reg_kernel<2><<<rows, 256, 0, st>>>(in, ld_in, row_index, w, out, ld_out, accumulate, cols, eps, o16);
-        else if (cols <= 4096) rms_weight_reg_kernel<4><<<rows, 256, 0, st>>>(in, ld_in, row_index, w, out, ld_out, accumulate, cols, eps, o16);
-        else rms_weight_reg_kernel<8><<<rows, 256, 0, st>>>(in, ld_in, row_index, w, out, ld_out, accumulate, cols, eps, o16);
+        if (cols <= 512) launch_pdl(rms_weight_reg_kernel<1>, dim3(rows), dim3(128), 0, st, in, ld_in, row_index, w, out, ld_out, accumulate, cols, eps, o16);
+        else if (cols <= 2048) launch_pdl(rms_weight_reg_kernel<2>, dim3(rows), dim3(256), 0, st, in, ld_in, row_index, w, out, ld_out, accumulate, cols,
+                                          eps, o16);
+        else if (cols <= 4096) launch_pdl(rms_weight_reg_kernel<4>, dim3(rows), dim3(256), 0, st, in, ld_in, row_index, w, out, ld_out, accumulate, cols,
+                                          eps, o16);
+        else launch_pdl(rms_weight_reg_kernel<8>, dim3(rows), dim3(256), 0, st, in, ld_in, row_index, w, out, ld_out, accumulate, cols, eps, o16);
     } else {
-        rms_weight_kernel<<<rows, cols >= 1024 ? 256 : 128, 0, st>>>(in, ld_in, row_index, w, out, ld_out, accumulate, cols, eps, o16);
+        launch_pdl(rms_weight_kernel, dim3(rows), dim3(cols >= 1024 ? 256 : 128), 0, st, in, ld_in, row_index, w, out, ld_out, accumulate, cols, eps, o16);
     }
     B2_LAUNCH_CHECK();
     return 0;
@@ -705,15 +727,16 @@ int dyt_rows_f32(const float* x, const int32_t* row_index, const DytOut* outs, i
         B2_CHECK_ARG(n.alpha && n.w && n.b && (outs[i].out || outs[i].out16), "dyt_rows: norm %d lacks a tensor or an output", i);
         align |= reinterpret_cast<uintptr_t>(n.w) | reinterpret_cast<uintptr_t>(n.b) | reinterpret_cast<uintptr_t>(outs[i].out) | reinterpret_cast<uintptr_t>(outs[i].out16);
     }
-    if (cols % 4 == 0 && (align & 15) == 0) dyt_rows_kernel<true><<<dim3((cols / 4 + 255) / 256, rows), 256, 0, st>>>(x, row_index, o, n_outs, cols);
-    else dyt_rows_kernel<false><<<dim3((cols + 255) / 256, rows), 256, 0, st>>>(x, row_index, o, n_outs, cols);
+    if (cols % 4 == 0 && (align & 15) == 0) launch_pdl(dyt_rows_kernel<true>, dim3((cols / 4 + 255) / 256, rows), dim3(256), 0, st, x, row_index, o, n_outs,
+                                                       cols);
+    else launch_pdl(dyt_rows_kernel<false>, dim3((cols + 255) / 256, rows), dim3(256), 0, st, x, row_index, o, n_outs, cols);
     B2_LAUNCH_CHECK();
     return 0;
 }
 
 int concat_rows_f32(const float* a, const float* b, float* out, void* out16, int rows, int cols, cudaStream_t st) {
     B2_CHECK_ARG(a && b && (out || out16) && rows > 0 && cols > 0, "concat_rows: bad argument");
-    concat_rows_kernel<<<dim3((2 * cols + 255) / 256, rows), 256, 0, st>>>(a, b, out, reinterpret_cast<__nv_bfloat16*>(out16), cols);
+    launch_pdl(concat_rows_kernel, dim3((2 * cols + 255) / 256, rows), dim3(256), 0, st, a, b, out, reinterpret_cast<__nv_bfloat16*>(out16), cols);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -726,10 +749,12 @@ int sandwich_norm_f32(const SandwichNormArgs& a, cudaStream_t st) {
     const bool conv = a.conv_w != nullptr;
     if (a.cols <= 4096 && (!conv || a.taps <= 4)) {
         const int t4 = (a.cols + 127) / 128 * 32, t8 = (a.cols + 255) / 256 * 32;
-        if (a.cols <= 512) { if (conv) sandwich_norm_reg_kernel<4, 3><<<a.rows, t4, 0, st>>>(a); else sandwich_norm_reg_kernel<4, 0><<<a.rows, t4, 0, st>>>(a); }
-        else { if (conv) sandwich_norm_reg_kernel<8, 3><<<a.rows, t8, 0, st>>>(a); else sandwich_norm_reg_kernel<8, 0><<<a.rows, t8, 0, st>>>(a); }
+        if (a.cols <= 512) { if (conv) launch_pdl(sandwich_norm_reg_kernel<4, 3>, dim3(a.rows), dim3(t4), 0, st,
+                                                  a); else launch_pdl(sandwich_norm_reg_kernel<4, 0>, dim3(a.rows), dim3(t4), 0, st, a); }
+        else { if (conv) launch_pdl(sandwich_norm_reg_kernel<8, 3>, dim3(a.rows), dim3(t8), 0, st, a); else launch_pdl(sandwich_norm_reg_kernel<8, 0>,
+                                    dim3(a.rows), dim3(t8), 0, st, a); }
     } else {
-        sandwich_norm_kernel<<<a.rows, 256, 0, st>>>(a);
+        launch_pdl(sandwich_norm_kernel, dim3(a.rows), dim3(256), 0, st, a);
     }
     B2_LAUNCH_CHECK();
     return 0;
@@ -749,21 +774,21 @@ int polynorm_f32(const float* in, int64_t ld_in, const float* bias, const float*
     B2_CHECK_ARG(in && coef && out && rows > 0 && cols > 0, "polynorm: bad argument");
     const int vec = cols % 4 == 0 && ld_in % 4 == 0 && ld_out % 4 == 0 && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out) |
                                                                             reinterpret_cast<uintptr_t>(bias)) & 15) == 0;
-    polynorm_kernel<<<rows, cols >= 4096 ? 512 : (cols >= 1024 ? 256 : 128), 0, st>>>(in, ld_in, bias, coef, out, ld_out, cols, eps, vec);
+    launch_pdl(polynorm_kernel, dim3(rows), dim3(cols >= 4096 ? 512 : (cols >= 1024 ? 256 : 128)), 0, st, in, ld_in, bias, coef, out, ld_out, cols, eps, vec);
     B2_LAUNCH_CHECK();
     return 0;
 }
 
 int softcap_f32(float* x, size_t n, float cap, cudaStream_t st) {
     B2_CHECK_ARG(x && n > 0 && cap > 0.f, "softcap: bad argument");
-    softcap_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(x, n, cap);
+    launch_pdl(softcap_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, x, n, cap);
     B2_LAUNCH_CHECK();
     return 0;
 }
 
 int head_gate_f32(const float* a, int64_t lda, const float* g, int64_t ldg, float* out, int64_t ldo, int rows, int heads, int dv, cudaStream_t st) {
     B2_CHECK_ARG(a && g && out && rows > 0 && heads > 0 && dv > 0, "head_gate: bad argument");
-    head_gate_kernel<<<dim3((heads * dv + 255) / 256, rows), 256, 0, st>>>(a, lda, g, ldg, out, ldo, heads, dv);
+    launch_pdl(head_gate_kernel, dim3((heads * dv + 255) / 256, rows), dim3(256), 0, st, a, lda, g, ldg, out, ldo, heads, dv);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -775,13 +800,11 @@ int embed_bigram_rows_f32(const int32_t* tokens, const SeqSeg* segs, int nseg, i
     B2_CHECK_ARG(bigram == nullptr || buckets > 0, "embed_bigram_rows: a bigram table needs buckets");
     if (bigram == nullptr) buckets = 1;
     if (table_dtype == DT_F32)
-        embed_bigram_kernel<float><<<dim3(max_n, nseg), 256, 0, st>>>(tokens, segs, reinterpret_cast<const float*>(table),
-                                                                     reinterpret_cast<const float*>(bigram), last_tok, x, x0, cols, vocab, buckets,
-                                                                     mul_prev, mul_cur, err_flag);
+        launch_pdl(embed_bigram_kernel<float>, dim3(max_n, nseg), dim3(256), 0, st, tokens, segs, reinterpret_cast<const float*>(table),
+                   reinterpret_cast<const float*>(bigram), last_tok, x, x0, cols, vocab, buckets, mul_prev, mul_cur, err_flag);
     else
-        embed_bigram_kernel<__nv_bfloat16><<<dim3(max_n, nseg), 256, 0, st>>>(tokens, segs, reinterpret_cast<const __nv_bfloat16*>(table),
-                                                                             reinterpret_cast<const __nv_bfloat16*>(bigram), last_tok, x, x0, cols,
-                                                                             vocab, buckets, mul_prev, mul_cur, err_flag);
+        launch_pdl(embed_bigram_kernel<__nv_bfloat16>, dim3(max_n, nseg), dim3(256), 0, st, tokens, segs, reinterpret_cast<const __nv_bfloat16*>(table),
+                   reinterpret_cast<const __nv_bfloat16*>(bigram), last_tok, x, x0, cols, vocab, buckets, mul_prev, mul_cur, err_flag);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -789,21 +812,21 @@ int embed_bigram_rows_f32(const int32_t* tokens, const SeqSeg* segs, int nseg, i
 int latent_append_f32(const float* in, int64_t ld_in, const float* gamma, float* cache, const int32_t* row_slot, const int32_t* row_pos, int rows,
                       int rank, int Smax, float eps, cudaStream_t st) {
     B2_CHECK_ARG(in && gamma && cache && row_slot && row_pos && rows > 0 && rank > 0, "latent_append: bad argument");
-    latent_append_kernel<<<rows, rank >= 512 ? 256 : 128, 0, st>>>(in, ld_in, gamma, cache, row_slot, row_pos, rank, Smax, eps);
+    launch_pdl(latent_append_kernel, dim3(rows), dim3(rank >= 512 ? 256 : 128), 0, st, in, ld_in, gamma, cache, row_slot, row_pos, rank, Smax, eps);
     B2_LAUNCH_CHECK();
     return 0;
 }
 
 int rowmap_portion(const RowMap& rm, int32_t* len, int slot, int n, int restart, cudaStream_t st) {
     B2_CHECK_ARG(rm.segs && rm.row_slot && rm.row_pos && len && n > 0, "rowmap_portion: bad argument");
-    rowmap_portion_kernel<<<1, 256, 0, st>>>(rm.segs, rm.row_slot, rm.row_pos, len, slot, n, restart);
+    launch_pdl(rowmap_portion_kernel, dim3(1), dim3(256), 0, st, rm.segs, rm.row_slot, rm.row_pos, len, slot, n, restart);
     B2_LAUNCH_CHECK();
     return 0;
 }
 
 int rowmap_decode(const RowMap& rm, const int32_t* len, const SampleState* sstate, const RowState* rows_state, int slot0, int B, cudaStream_t st) {
     B2_CHECK_ARG(rm.segs && rm.row_slot && rm.row_pos && len && B > 0, "rowmap_decode: bad argument");
-    rowmap_decode_kernel<<<(B + 127) / 128, 128, 0, st>>>(rm.segs, rm.row_slot, rm.row_pos, len, sstate, rows_state, slot0, B);
+    launch_pdl(rowmap_decode_kernel, dim3((B + 127) / 128), dim3(128), 0, st, rm.segs, rm.row_slot, rm.row_pos, len, sstate, rows_state, slot0, B);
     B2_LAUNCH_CHECK();
     return 0;
 }

@@ -24,6 +24,7 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(const float* __restric
                                                           const float* __restrict__ bias, float* __restrict__ tail,
                                                           float* __restrict__ out, int64_t ld_out, int C, int taps,
                                                           const SeqSeg* __restrict__ segs, int own_tail) {
+    pdl_enter();
     const SeqSeg sg = segs[blockIdx.z];
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int tt0 = blockIdx.y * CONV_TILE;
@@ -79,6 +80,7 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(const float* __restric
 // tail[j] := input of token n - (taps-1) + j of the segment; tokens before the call come from the old tail (or zero)
 __global__ void __launch_bounds__(128) causal_conv_tail_kernel(const float* __restrict__ in, int64_t ld_in, float* __restrict__ tail, int C,
                                                                int taps, const SeqSeg* __restrict__ segs) {
+    pdl_enter();
     const SeqSeg sg = segs[blockIdx.y];
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C || sg.n <= 0) return;
@@ -103,6 +105,7 @@ constexpr int SHIFT_MAX_MIX = 8, SHIFT_TILE = 8;
 __global__ void __launch_bounds__(128) token_shift_mix_kernel(const float* __restrict__ x, const float* __restrict__ mu,
                                                               const float* __restrict__ prev, float* __restrict__ out, int64_t out_stride,
                                                               int cols, int n_mix, const SeqSeg* __restrict__ segs) {
+    pdl_enter();
     const SeqSeg sg = segs[blockIdx.z];
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int t0 = blockIdx.y * SHIFT_TILE;
@@ -126,6 +129,7 @@ __global__ void __launch_bounds__(128) token_shift_mix_kernel(const float* __res
 }
 __global__ void __launch_bounds__(128) token_shift_carry_kernel(const float* __restrict__ x, float* __restrict__ prev, int cols,
                                                                 const SeqSeg* __restrict__ segs) {
+    pdl_enter();
     const SeqSeg sg = segs[blockIdx.y];
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < cols && sg.n > 0) prev[(size_t)sg.slot * cols + c] = x[(size_t)(sg.row0 + sg.n - 1) * cols + c];
@@ -181,6 +185,7 @@ __device__ __forceinline__ float scan_query(const ScanArgs& a, float q) { return
 // ... in place over a long prompt's rows (workspaces of the call), where every column block of both launches would redo it
 template <int MODE>
 __global__ void __launch_bounds__(256) scan_prepare_kernel(ScanArgs a) {
+    pdl_enter();
     const int c = blockIdx.x * 256 + threadIdx.x;
     const size_t r = (size_t)a.segs[0].row0 + blockIdx.y;
     if (c >= a.heads * a.dk) return;
@@ -195,6 +200,7 @@ __global__ void __launch_bounds__(256) scan_prepare_kernel(ScanArgs a) {
 // KW: warps over the keys (64 each); V16: every operand row is 16-byte aligned with sizes in whole fours
 template <int MODE, int KW, bool V16>
 __global__ void __launch_bounds__(KW * 128, KW == 4 ? 1 : 2) linear_scan_kernel(ScanArgs a, ScanPlan p) {
+    pdl_enter();
     constexpr int DKP = KW * 64, NTHR = KW * 128;
     constexpr bool PER_KEY = MODE != SCAN_SSD, HAS_K = MODE != SCAN_HGRN2;
     extern __shared__ __align__(16) float sm[];
@@ -448,14 +454,17 @@ int causal_conv_f32(const float* in, int64_t ld_in, const float* w, const float*
     const dim3 grid((C + 127) / 128, (max_n + CONV_TILE - 1) / CONV_TILE, nseg);
     const int own = max_n <= CONV_TILE;   // one tile per segment (decode steps, short portions): no second kernel for the carried inputs
     switch (flags & (CONV_SILU | CONV_ADD_INPUT)) {
-        case 0: causal_conv_kernel<0><<<grid, 128, 0, st>>>(in, ld_in, w, bias, tail, out, ld_out, C, taps, segs, own); break;
-        case CONV_SILU: causal_conv_kernel<CONV_SILU><<<grid, 128, 0, st>>>(in, ld_in, w, bias, tail, out, ld_out, C, taps, segs, own); break;
-        case CONV_ADD_INPUT: causal_conv_kernel<CONV_ADD_INPUT><<<grid, 128, 0, st>>>(in, ld_in, w, bias, tail, out, ld_out, C, taps, segs, own); break;
-        default: causal_conv_kernel<CONV_SILU | CONV_ADD_INPUT><<<grid, 128, 0, st>>>(in, ld_in, w, bias, tail, out, ld_out, C, taps, segs, own); break;
+        case 0: launch_pdl(causal_conv_kernel<0>, dim3(grid), dim3(128), 0, st, in, ld_in, w, bias, tail, out, ld_out, C, taps, segs, own); break;
+        case CONV_SILU: launch_pdl(causal_conv_kernel<CONV_SILU>, dim3(grid), dim3(128), 0, st, in, ld_in, w, bias, tail, out, ld_out, C, taps, segs,
+                                   own); break;
+        case CONV_ADD_INPUT: launch_pdl(causal_conv_kernel<CONV_ADD_INPUT>, dim3(grid), dim3(128), 0, st, in, ld_in, w, bias, tail, out, ld_out, C, taps,
+                                        segs, own); break;
+        default: launch_pdl(causal_conv_kernel<CONV_SILU | CONV_ADD_INPUT>, dim3(grid), dim3(128), 0, st, in, ld_in, w, bias, tail, out, ld_out, C, taps,
+                            segs, own); break;
     }
     B2_LAUNCH_CHECK();
     if (taps > 1 && !own) {
-        causal_conv_tail_kernel<<<dim3((C + 127) / 128, nseg), 128, 0, st>>>(in, ld_in, tail, C, taps, segs);
+        launch_pdl(causal_conv_tail_kernel, dim3((C + 127) / 128, nseg), dim3(128), 0, st, in, ld_in, tail, C, taps, segs);
         B2_LAUNCH_CHECK();
     }
     return 0;
@@ -465,10 +474,10 @@ int token_shift_mix_f32(const float* x, const float* mu, float* prev, float* out
                         int nseg, int max_n, cudaStream_t st) {
     B2_CHECK_ARG(x && mu && prev && out && segs && cols > 0 && nseg > 0, "token_shift: bad argument");
     B2_CHECK_ARG(n_mix >= 1 && n_mix <= SHIFT_MAX_MIX, "token_shift: 1..%d mixes are supported (got %d)", SHIFT_MAX_MIX, n_mix);
-    token_shift_mix_kernel<<<dim3((cols + 127) / 128, (max_n + SHIFT_TILE - 1) / SHIFT_TILE, nseg), 128, 0, st>>>(x, mu, prev, out, out_stride, cols,
-                                                                                                                 n_mix, segs);
+    launch_pdl(token_shift_mix_kernel, dim3((cols + 127) / 128, (max_n + SHIFT_TILE - 1) / SHIFT_TILE, nseg), dim3(128), 0, st, x, mu, prev, out, out_stride,
+               cols, n_mix, segs);
     B2_LAUNCH_CHECK();
-    token_shift_carry_kernel<<<dim3((cols + 127) / 128, nseg), 128, 0, st>>>(x, prev, cols, segs);
+    launch_pdl(token_shift_carry_kernel, dim3((cols + 127) / 128, nseg), dim3(128), 0, st, x, prev, cols, segs);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -491,18 +500,18 @@ int launch_scan(const ScanArgs& a, cudaStream_t st) {
         p.final_state = a.chunk_scratch;
         p.decays = a.chunk_scratch + (size_t)(p.chunks - 1) * a.heads * a.dk * a.dv;
         if (MODE != SCAN_SSD) {
-            scan_prepare_kernel<MODE><<<dim3((a.heads * a.dk + 255) / 256, a.rows), 256, 0, st>>>(a);
+            launch_pdl(scan_prepare_kernel<MODE>, dim3((a.heads * a.dk + 255) / 256, a.rows), dim3(256), 0, st, a);
             B2_LAUNCH_CHECK();
             p.prepared = 1;
         }
-        linear_scan_kernel<MODE, KW, V16><<<dim3(cols, a.heads, p.chunks - 1), KW * 128, smem, st>>>(a, p);
+        launch_pdl(linear_scan_kernel<MODE, KW, V16>, dim3(cols, a.heads, p.chunks - 1), dim3(KW * 128), smem, st, a, p);
         B2_LAUNCH_CHECK();
         p.second = 1;
         p.z0 = 1;
-        linear_scan_kernel<MODE, KW, V16><<<dim3(cols, a.heads, p.chunks - 1), KW * 128, smem, st>>>(a, p);
+        launch_pdl(linear_scan_kernel<MODE, KW, V16>, dim3(cols, a.heads, p.chunks - 1), dim3(KW * 128), smem, st, a, p);
     } else {
         p.chunks = 1;
-        linear_scan_kernel<MODE, KW, V16><<<dim3(cols, a.heads, a.nseg), KW * 128, smem, st>>>(a, p);
+        launch_pdl(linear_scan_kernel<MODE, KW, V16>, dim3(cols, a.heads, a.nseg), dim3(KW * 128), smem, st, a, p);
     }
     B2_LAUNCH_CHECK();
     return 0;

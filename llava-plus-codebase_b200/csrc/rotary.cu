@@ -22,8 +22,14 @@ namespace {
 // the call may run in place.
 struct RotateParts { RotateArgs p[3]; };
 __device__ __forceinline__ void rotate_rows_body(const RotateArgs& a);
-__global__ void __launch_bounds__(256) rotate_rows_kernel(RotateArgs a) { rotate_rows_body(a); }
-__global__ void __launch_bounds__(256) rotate_rows_multi_kernel(RotateParts ps) { rotate_rows_body(ps.p[blockIdx.z]); }
+__global__ void __launch_bounds__(256) rotate_rows_kernel(RotateArgs a) {
+    pdl_enter();
+    rotate_rows_body(a);
+}
+__global__ void __launch_bounds__(256) rotate_rows_multi_kernel(RotateParts ps) {
+    pdl_enter();
+    rotate_rows_body(ps.p[blockIdx.z]);
+}
 __device__ __forceinline__ void rotate_rows_body(const RotateArgs& a) {
     const int units = a.size - a.pairs;
     const int r = blockIdx.y;
@@ -62,6 +68,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 // everything it writes before it writes (its own pairs and single entries), and the sum of squares is complete before any lane writes,
 // so the call may run in place.
 __global__ void __launch_bounds__(256) rotate_rows_warp_kernel(RotateParts ps, int n_parts) {
+    pdl_enter();
     const int r = blockIdx.y, lane = threadIdx.x & 31;
     int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     int pi = 0;
@@ -108,6 +115,7 @@ __global__ void __launch_bounds__(256) rotate_rows_warp_kernel(RotateParts ps, i
 // then every head's pairs turn. Parts may read the same input (values that are the raw keys), so a part writes in place only what no
 // other part reads.
 __global__ void __launch_bounds__(256) rotate_rows_block_kernel(RotateParts ps) {
+    pdl_enter();
     __shared__ float red[8];
     const RotateArgs& a = ps.p[blockIdx.y];
     const int r = blockIdx.x, tid = threadIdx.x;
@@ -151,6 +159,7 @@ __global__ void __launch_bounds__(128) latent_rot_append_kernel(const float* __r
                                                                 float* __restrict__ cache, const int32_t* __restrict__ row_slot,
                                                                 const int32_t* __restrict__ row_pos, int rank, int rot, int pairs,
                                                                 const float2* __restrict__ table, int Smax, float eps) {
+    pdl_enter();
     __shared__ float red[4];
     const size_t r = blockIdx.x;
     const int pos = row_pos[r];
@@ -180,7 +189,7 @@ int rotate_rows_f32(const RotateArgs& a, cudaStream_t st) {
     B2_CHECK_ARG(a.cache == nullptr || (a.row_slot != nullptr && a.Smax > 0), "rotate_rows: a cache destination needs slots");
     if (a.norm_w != nullptr) return rotate_rows_multi_f32(&a, 1, st);
     const int units = a.heads * (a.size - a.pairs);
-    rotate_rows_kernel<<<dim3((units + 255) / 256, a.rows), 256, 0, st>>>(a);
+    launch_pdl(rotate_rows_kernel, dim3((units + 255) / 256, a.rows), dim3(256), 0, st, a);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -204,16 +213,16 @@ int rotate_rows_multi_f32(const RotateArgs* parts, int n, cudaStream_t st) {
     }
     if (whole) {   // one CTA per row and part
         for (int i = 0; i < n; ++i) B2_CHECK_ARG(parts[i].norm_w == nullptr || parts[i].norm_all, "rotate_rows_multi: norms per head and over all heads do not mix");
-        rotate_rows_block_kernel<<<dim3(parts[0].rows, n), 256, 0, st>>>(ps);
+        launch_pdl(rotate_rows_block_kernel, dim3(parts[0].rows, n), dim3(256), 0, st, ps);
         B2_LAUNCH_CHECK();
         return 0;
     }
     if (normed) {   // a normed head needs its sum of squares: one warp per (row, head) of every part
-        rotate_rows_warp_kernel<<<dim3((heads + 7) / 8, parts[0].rows), 256, 0, st>>>(ps, n);
+        launch_pdl(rotate_rows_warp_kernel, dim3((heads + 7) / 8, parts[0].rows), dim3(256), 0, st, ps, n);
         B2_LAUNCH_CHECK();
         return 0;
     }
-    rotate_rows_multi_kernel<<<dim3((units + 255) / 256, parts[0].rows, n), 256, 0, st>>>(ps);
+    launch_pdl(rotate_rows_multi_kernel, dim3((units + 255) / 256, parts[0].rows, n), dim3(256), 0, st, ps);
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -221,7 +230,7 @@ int rotate_rows_multi_f32(const RotateArgs* parts, int n, cudaStream_t st) {
 int latent_rot_append_f32(const float* in, int64_t ld_in, const float* gamma, float* cache, const int32_t* row_slot, const int32_t* row_pos, int rows,
                           int rank, int rot, int pairs, const float2* table, int Smax, float eps, cudaStream_t st) {
     B2_CHECK_ARG(in && gamma && cache && row_slot && row_pos && rows > 0 && rank > 0 && pairs >= 0 && 2 * pairs <= rot && (pairs == 0 || table), "latent_rot_append: bad argument");
-    latent_rot_append_kernel<<<rows, 128, 0, st>>>(in, ld_in, gamma, cache, row_slot, row_pos, rank, rot, pairs, table, Smax, eps);
+    launch_pdl(latent_rot_append_kernel, dim3(rows), dim3(128), 0, st, in, ld_in, gamma, cache, row_slot, row_pos, rank, rot, pairs, table, Smax, eps);
     B2_LAUNCH_CHECK();
     return 0;
 }
