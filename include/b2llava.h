@@ -382,6 +382,11 @@ int64_t b2_kv_bytes(b2_model* m, int max_batch, int max_seq);
 /* ---- single-kernel entry points (unit-level parity tests; same kernels the hot path launches) ----------- */
 int b2_op_gemm(const void* A, int lda, const void* W, int ldw, const void* bias, const void* residual, int ld_res,
                void* out, int ld_out, int out_fp32, int M, int N, int K, int act, int bn_override, void* stream);
+// out[M, ff] = bf16(a(gate) (up + up_shift)), [gate | up] = A[M,K] W[2 ff, K]^T: the products and their gated unit in one launch; ff % 8 == 0.
+// a(g) = g sigmoid(slope g), or (kind 1) the tanh form of GELU; limit > 0 bounds gate (from above) and up first. tile_group (nullable): rows
+// come in tiles of 128, tile t multiplies with the matrix tile_group[t] of `groups` stacked ones (negative: the tile is skipped).
+int b2_op_gemm_glu(const void* A, int lda, const void* W, int ldw, void* out, int ld_out, int M, int ff, int K, float slope, float limit,
+                   float up_shift, int kind, const int32_t* tile_group, int groups, int bn_override, void* stream);
 int b2_op_gemv(const void* x, int64_t ldx, const void* W, int ldw, const void* norm_gamma, float eps,
                const void* residual, int ld_res, void* out, int ld_out, int out_fp32, int B, int N, int K, int act,
                void* stream);

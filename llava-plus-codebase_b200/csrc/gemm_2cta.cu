@@ -56,6 +56,7 @@ struct PairEpi {
     __nv_bfloat16* kcache;
     __nv_bfloat16* vcache;
     int rope_S, rope_H, rope_Smax;
+    GluAct glu;            // ACT_GLU
 };
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -182,14 +183,19 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 int m_blk, n_blk;
                 tile_coords(t, m_blk, n_blk);
                 const int a_row = m_blk * P_TM + (int)rank * P_BM;  // this CTA's 128 rows of A
-                const int b_row = n_blk * P_TN + (int)rank * P_BM;  // this CTA's 128 rows of W (half of the N tile)
+                const int b_row = n_blk * P_TN + (int)rank * P_BM;  // this CTA's 128 rows of W (half of the N tile; ACT_GLU: 64 of gate, 64 of up)
                 for (int kb = 0; kb < num_kb; ++kb) {
                     mbar_wait(&empty_bar[stage], phase ^ 1);
                     uint8_t* sa = smem + stage * P_STAGE_BYTES;
                     const uint32_t leader_full = mapa_rank(smem_u32(&full_bar[stage]), 0);
                     if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * P_STAGE_BYTES);
                     tma_load_2d_2sm(sa, &tmap_a, leader_full, kb * P_BK, a_row, kEvictNormal);
-                    tma_load_2d_2sm(sa + P_TILE_BYTES, &tmap_b, leader_full, kb * P_BK, b_row, kEvictNormal);
+                    if constexpr (ACT == ACT_GLU) {
+                        tma_load_2d_2sm(sa + P_TILE_BYTES, &tmap_b, leader_full, kb * P_BK, b_row / 2, kEvictNormal);
+                        tma_load_2d_2sm(sa + P_TILE_BYTES + P_TILE_BYTES / 2, &tmap_b, leader_full, kb * P_BK, N / 2 + b_row / 2, kEvictNormal);
+                    } else {
+                        tma_load_2d_2sm(sa + P_TILE_BYTES, &tmap_b, leader_full, kb * P_BK, b_row, kEvictNormal);
+                    }
                     if (++stage == P_STAGES) { stage = 0; phase ^= 1; }
                 }
             }
@@ -235,7 +241,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             const int row = m_blk * P_TM + (int)rank * P_BM + q * 32 + lane;
             const bool row_ok = row < M;
             const uint32_t taddr_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + as * P_TN;
-            if constexpr (ACT == ACT_SWIGLU) {
+            if constexpr (ACT == ACT_SWIGLU || ACT == ACT_GLU) {   // 64 gate columns, then 64 up columns of the same outputs
 #pragma unroll 1
                 for (int it = half * (P_TN / 128); it < (half + 1) * (P_TN / 128); ++it) {
                     const int g = it >> 1, j = it & 1;
@@ -254,9 +260,10 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                             for (int e = 0; e < 4; ++e) {
                                 const float g0 = __uint_as_float(vg[v8 * 8 + 2 * e]), g1 = __uint_as_float(vg[v8 * 8 + 2 * e + 1]);
                                 const float u0 = __uint_as_float(vu[v8 * 8 + 2 * e]), u1 = __uint_as_float(vu[v8 * 8 + 2 * e + 1]);
-                                pk[e] = pack_bf16(p_silu(g0) * u0, p_silu(g1) * u1);
+                                if constexpr (ACT == ACT_GLU) pk[e] = pack_bf16(glu_act(g0, u0, ep.glu), glu_act(g1, u1, ep.glu));
+                                else pk[e] = pack_bf16(p_silu(g0) * u0, p_silu(g1) * u1);
                             }
-                            *reinterpret_cast<uint4*>(op + v8 * 8) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                            if (ACT == ACT_SWIGLU || ocol0 + v8 * 8 < N / 2) *reinterpret_cast<uint4*>(op + v8 * 8) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
                         }
                     }
                 }
@@ -392,12 +399,14 @@ int gemm_bf16_2cta(const GemmArgs& g, cudaStream_t stream) {
     B2_CHECK_ARG(g.K % 8 == 0 && g.N % 8 == 0, "gemm_2cta: K and N must be multiples of 8 (K=%d N=%d)", g.K, g.N);
     B2_CHECK_ARG(g.act != ACT_SWIGLU || (g.N % 128 == 0 && !g.out_fp32 && g.bias == nullptr && g.residual == nullptr),
                  "gemm_2cta: swiglu needs N %% 128 == 0, no bias/residual, bf16 output");
+    B2_CHECK_ARG(g.act != ACT_GLU || (g.N % 16 == 0 && !g.out_fp32 && g.bias == nullptr && g.residual == nullptr),
+                 "gemm_2cta: glu needs N %% 16 == 0, no bias/residual, bf16 output");
     B2_CHECK_ARG((reinterpret_cast<uintptr_t>(g.out) & 15) == 0 && (g.ld_out % 8) == 0, "gemm_2cta: out alignment");
     B2_CHECK_ARG(g.residual == nullptr || ((reinterpret_cast<uintptr_t>(g.residual) & 15) == 0 && (g.ld_res % 8) == 0),
                  "gemm_2cta: residual alignment");
     CUtensorMap ta, tb;
     B2_TRY(make_tmap_bf16(&ta, g.A, g.M, g.K, g.lda, P_BM));
-    B2_TRY(make_tmap_bf16(&tb, g.W, g.N, g.K, g.ldw, P_BM));
+    B2_TRY(make_tmap_bf16(&tb, g.W, g.N, g.K, g.ldw, g.act == ACT_GLU ? P_BM / 2 : P_BM));
     PairEpi ep;
     ep.bias = reinterpret_cast<const __nv_bfloat16*>(g.bias);
     ep.residual = reinterpret_cast<const __nv_bfloat16*>(g.residual);
@@ -406,6 +415,7 @@ int gemm_bf16_2cta(const GemmArgs& g, cudaStream_t stream) {
     ep.rope_tab = reinterpret_cast<const uint32_t*>(g.rope.table);
     ep.kcache = reinterpret_cast<__nv_bfloat16*>(g.rope.kcache); ep.vcache = reinterpret_cast<__nv_bfloat16*>(g.rope.vcache);
     ep.rope_S = g.rope.S; ep.rope_H = g.rope.H; ep.rope_Smax = g.rope.Smax;
+    ep.glu = g.glu;
     if (g.act == ACT_ROPE_QKV) {
         B2_CHECK_ARG(g.rope.table && g.rope.kcache && g.rope.vcache && g.rope.S > 0 && g.rope.H > 0 && g.rope.Smax >= g.rope.S,
                      "gemm_2cta(rope_qkv): rope arguments missing");
@@ -418,6 +428,7 @@ int gemm_bf16_2cta(const GemmArgs& g, cudaStream_t stream) {
         case ACT_QUICK_GELU: return launch_pair<ACT_QUICK_GELU>(ta, tb, g.M, g.N, g.K, ep, stream);
         case ACT_GELU_ERF: return launch_pair<ACT_GELU_ERF>(ta, tb, g.M, g.N, g.K, ep, stream);
         case ACT_SWIGLU: return launch_pair<ACT_SWIGLU>(ta, tb, g.M, g.N, g.K, ep, stream);
+        case ACT_GLU: return launch_pair<ACT_GLU>(ta, tb, g.M, g.N, g.K, ep, stream);
         case ACT_ROPE_QKV: return launch_pair<ACT_ROPE_QKV>(ta, tb, g.M, g.N, g.K, ep, stream);
         default: break;
     }

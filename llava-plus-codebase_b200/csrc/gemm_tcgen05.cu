@@ -131,6 +131,7 @@ struct EpiParams {
     // rows [g * group_rows, (g + 1) * group_rows) of W, g = tile_group[m]; a negative group: the tile is unused and skipped
     const int* tile_group = nullptr;
     int group_rows = 0;
+    GluAct glu;            // ACT_GLU
 };
 
 __device__ __forceinline__ float act_quick_gelu(float x) { return __fdividef(x, 1.0f + __expf(-1.702f * x)); }
@@ -205,6 +206,15 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
         if (lane == 0) {
             // Programmatic dependent launch: the WEIGHT halves of the first ring-full of stages are requested before the
             // upstream kernel (which produces A) is known to have finished; the A halves follow after pdl_wait().
+            auto load_b = [&](uint8_t* sb, uint64_t* bar, int kb, int w_row0, int n_blk) {
+                if constexpr (ACT == ACT_GLU) {   // 64 rows of gate, then the 64 rows of up of the same outputs
+#pragma unroll
+                    for (int i = 0; i < BN / 64; ++i)
+                        tma_load_2d(sb + i * 64 * BK * 2, &tmap_b, bar, kb * BK, w_row0 + (i & 1) * (N / 2) + n_blk * (BN / 2) + (i >> 1) * 64, kEvictNormal);
+                } else {
+                    tma_load_2d(sb, &tmap_b, bar, kb * BK, w_row0 + n_blk * BN, kEvictNormal);
+                }
+            };
             int stage = 0;
             uint32_t phase = 0;
             int pre_n = 0;
@@ -214,7 +224,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
                 for (int kb = 0; kb < num_kb && pre_n < STAGES; ++kb, ++pre_n) {
                     uint8_t* sb = smem + pre_n * Cfg::STAGE_BYTES + A_TILE_BYTES;
                     mbar_arrive_expect_tx(&full_bar[pre_n], Cfg::STAGE_BYTES);
-                    tma_load_2d(sb, &tmap_b, &full_bar[pre_n], kb * BK, n_blk * BN, kEvictNormal);
+                    load_b(sb, &full_bar[pre_n], kb, 0, n_blk);
                 }
             }
             pdl_wait();
@@ -231,7 +241,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
                     if (seen >= pre_n) {
                         mbar_wait(&empty_bar[stage], phase ^ 1);
                         mbar_arrive_expect_tx(&full_bar[stage], Cfg::STAGE_BYTES);
-                        tma_load_2d(sb, &tmap_b, &full_bar[stage], kb * BK, w_row0 + n_blk * BN, kEvictNormal);
+                        load_b(sb, &full_bar[stage], kb, w_row0, n_blk);
                     }
                     tma_load_2d(sa, &tmap_a, &full_bar[stage], kb * BK, m_blk * BM, kEvictNormal);
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -294,8 +304,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
             const bool row_ok = row < M;
             const uint32_t taddr_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + as * Cfg::ACC_STRIDE;
 
-            if constexpr (ACT == ACT_SWIGLU) {
-                // W rows are block-interleaved: within each 128-col group, cols [0,64) = gate, [64,128) = up
+            if constexpr (ACT == ACT_SWIGLU || ACT == ACT_GLU) {
+                // W rows are block-interleaved (ACT_GLU: by the loads): within each 128-col group, cols [0,64) = gate, [64,128) = up
                 // for the same 64 output channels. out is [M, N/2].
                 static_assert(BN % 128 == 0, "swiglu needs BN multiple of 128");
 #pragma unroll 1
@@ -320,10 +330,11 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
                                     float g1 = __uint_as_float(vg[v8 * 8 + 2 * e + 1]);
                                     float u0 = __uint_as_float(vu[v8 * 8 + 2 * e]);
                                     float u1 = __uint_as_float(vu[v8 * 8 + 2 * e + 1]);
-                                    pk[e] = pack_bf16(act_silu(g0) * u0, act_silu(g1) * u1);
+                                    if constexpr (ACT == ACT_GLU) pk[e] = pack_bf16(glu_act(g0, u0, ep.glu), glu_act(g1, u1, ep.glu));
+                                    else pk[e] = pack_bf16(act_silu(g0) * u0, act_silu(g1) * u1);
                                 }
-                                *reinterpret_cast<uint4*>(op + v8 * 8) =
-                                    make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                                if (ACT == ACT_SWIGLU || ocol0 + v8 * 8 < N / 2)
+                                    *reinterpret_cast<uint4*>(op + v8 * 8) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
                             }
                         }
                     }
@@ -678,15 +689,17 @@ int gemm_bf16(const GemmArgs& g, cudaStream_t stream) {
     B2_CHECK_ARG(g.act != ACT_SWIGLU || g.N % 128 == 0, "gemm: swiglu needs N %% 128 == 0 (N=%d)", g.N);
     B2_CHECK_ARG(g.act != ACT_SWIGLU || (!g.out_fp32 && g.bias == nullptr && g.residual == nullptr),
                  "gemm: swiglu epilogue takes no bias/residual and writes bf16");
+    B2_CHECK_ARG(g.act != ACT_GLU || (g.N % 16 == 0 && !g.out_fp32 && g.bias == nullptr && g.residual == nullptr),
+                 "gemm: glu epilogue takes whole blocks of 8 outputs, no bias/residual, and writes bf16");
     B2_CHECK_ARG((reinterpret_cast<uintptr_t>(g.out) & 15) == 0 && (g.ld_out % 8) == 0,
                  "gemm: out must be 16B aligned with ld_out %% 8 == 0");
     B2_CHECK_ARG(g.residual == nullptr ||
                      ((reinterpret_cast<uintptr_t>(g.residual) & 15) == 0 && (g.ld_res % 8) == 0),
                  "gemm: residual must be 16B aligned with ld_res %% 8 == 0");
 
-    const bool grouped = g.tile_group != nullptr;
-    B2_CHECK_ARG(!grouped || (g.groups >= 1 && g.act == ACT_NONE && g.bias == nullptr && g.residual == nullptr && g.M % BM == 0),
-                 "gemm: a grouped product takes whole tiles of %d rows, no bias, residual or fused activation", BM);
+    const bool grouped = g.tile_group != nullptr, glu = g.act == ACT_SWIGLU || g.act == ACT_GLU;
+    B2_CHECK_ARG(!grouped || (g.groups >= 1 && (g.act == ACT_NONE || g.act == ACT_GLU) && g.bias == nullptr && g.residual == nullptr && g.M % BM == 0),
+                 "gemm: a grouped product takes whole tiles of %d rows, no bias, residual or fused activation but the gated unit", BM);
     if (g.bn_override >= 1000 && !grouped) return gemm_bf16_splitk(g, g.bn_override % 1000, g.bn_override / 1000, stream);
     if (g.bn_override == 2 && !grouped) return gemm_bf16_2cta(g, stream);  // CTA-pair kernel (cta_group::2, 256x256 pair tiles)
 
@@ -705,7 +718,7 @@ int gemm_bf16(const GemmArgs& g, cudaStream_t stream) {
         const float rel[4] = {1.00f, 0.93f, 0.81f, 0.44f};
         float best = 0.f;
         for (int i = 0; i < 4; ++i) {
-            if (g.act == ACT_SWIGLU && cand[i] % 128 != 0) continue;
+            if (glu && cand[i] % 128 != 0) continue;
             const long long tiles = (long long)num_m * ((g.N + cand[i] - 1) / cand[i]);
             const long long waves = (tiles + num_sms() - 1) / num_sms();
             const float cost = (float)waves * ((float)cand[i] / rel[i] + 24.f /*per-tile fixed cost*/);
@@ -719,7 +732,7 @@ int gemm_bf16(const GemmArgs& g, cudaStream_t stream) {
         int split_bn = 0, split_s = 0;
         float split_best = 0.f;
         const int kb = (g.K + BK - 1) / BK;
-        if (g.bn_override == 0 && !grouped && g.act != ACT_SWIGLU) {
+        if (g.bn_override == 0 && !grouped && !glu) {
             for (int c = 2; c < 4; ++c)
                 for (int s = 2; s <= 4; s *= 2) {
                     const long long ctas = (long long)num_m * ((g.N + cand[c] - 1) / cand[c]) * s;
@@ -738,12 +751,13 @@ int gemm_bf16(const GemmArgs& g, cudaStream_t stream) {
         if (split_bn != 0 && split_best < best) return gemm_bf16_splitk(g, split_bn, split_s, stream);
     }
     if (g.bn_override == 64 || g.bn_override == 128 || g.bn_override == 192 || g.bn_override == 256) bn = g.bn_override;
-    if (g.act == ACT_SWIGLU && bn % 128 != 0) bn = 128;
+    if (glu && bn % 128 != 0) bn = 128;
 
     CUtensorMap ta, tb;
     B2_TRY(make_tmap_bf16(&ta, g.A, g.M, g.K, g.lda, BM));
-    B2_TRY(make_tmap_bf16(&tb, g.W, grouped ? g.N * g.groups : g.N, g.K, g.ldw, bn));
+    B2_TRY(make_tmap_bf16(&tb, g.W, grouped ? g.N * g.groups : g.N, g.K, g.ldw, g.act == ACT_GLU ? 64 : bn));
     EpiParams ep;
+    ep.glu = g.glu;
     ep.tile_group = g.tile_group; ep.group_rows = g.N;
     ep.bias = reinterpret_cast<const __nv_bfloat16*>(g.bias);
     ep.residual = reinterpret_cast<const __nv_bfloat16*>(g.residual);
@@ -753,6 +767,10 @@ int gemm_bf16(const GemmArgs& g, cudaStream_t stream) {
     ep.out_fp32 = g.out_fp32;
     ep.post = g.out_fp32 ? g.post : 0; ep.alpha = g.out_fp32 ? g.alpha : 1.f; ep.accumulate = g.out_fp32 ? g.accumulate : 0;
 
+    if (g.act == ACT_GLU) {
+        if (bn == 256) return launch_gemm<256, ACT_GLU>(ta, tb, g.M, g.N, g.K, ep, stream);
+        return launch_gemm<128, ACT_GLU>(ta, tb, g.M, g.N, g.K, ep, stream);
+    }
     if (g.act == ACT_SWIGLU) {
         if (bn == 256) return launch_gemm<256, ACT_SWIGLU>(ta, tb, g.M, g.N, g.K, ep, stream);
         return launch_gemm<128, ACT_SWIGLU>(ta, tb, g.M, g.N, g.K, ep, stream);

@@ -7,7 +7,7 @@
 
 namespace b2 {
 
-enum { ACT_NONE = 0, ACT_QUICK_GELU = 1, ACT_GELU_ERF = 2, ACT_SWIGLU = 3, ACT_ROPE_QKV = 4 };
+enum { ACT_NONE = 0, ACT_QUICK_GELU = 1, ACT_GELU_ERF = 2, ACT_SWIGLU = 3, ACT_ROPE_QKV = 4, ACT_GLU = 5 };
 
 // ACT_ROPE_QKV (CTA-pair kernel only): the GEMM is LLaMA's fused QKV projection of a prefill, rows = b*S + t. The epilogue
 // rounds the projection to bf16, applies RoPE (HF rounding points, cos/sin from `table`) to the q and k heads, writes q to
@@ -22,9 +22,21 @@ enum { DT_BF16 = 0, DT_F16 = 1, DT_F32 = 2 };
 
 int num_sms();
 
+// The gated unit in its general form: with g = in[r, c] and u = in[r, ff + c], limit > 0 first bounds them, g = min(g, limit),
+// u = clamp(u, -limit, limit); out = a(g) (u + up_shift) with a(g) = g sigmoid(slope g), or (GLU_GELU_TANH) the tanh form of GELU,
+// a(g) = g / 2 (1 + tanh(sqrt(2 / pi) (g + 0.044715 g^3))). (slope 1, no limit, shift 0: SiLU(g) u.)
+enum { GLU_SIGMOID = 0, GLU_GELU_TANH = 1 };
+struct GluAct { float slope = 1.f, limit = 0.f, up_shift = 0.f; int kind = GLU_SIGMOID; };
+__host__ __device__ inline float glu_act(float g, float u, const GluAct& a) {
+    if (a.limit > 0.f) { g = fminf(g, a.limit); u = fminf(fmaxf(u, -a.limit), a.limit); }
+    const float v = a.kind == GLU_GELU_TANH ? 0.5f * g * (1.f + tanhf(0.7978845608028654f * fmaf(0.044715f * g * g, g, g))) : g / (1.f + expf(-a.slope * g));
+    return v * (u + a.up_shift);
+}
+
 // ---- tcgen05 GEMM (gemm_tcgen05.cu) -------------------------------------------------------------
 // out[M, N] = act(A[M,K] · W[N,K]^T + bias) + residual      (ACT_NONE / QUICK_GELU / GELU_ERF)
 // out[M, N/2] = silu(gate) * up                               (ACT_SWIGLU; W rows block-64 interleaved)
+// out[M, N/2] = glu_act(gate, up), bf16                       (ACT_GLU; W = [gate rows | up rows], N / 2 of each, N % 16 == 0)
 struct GemmArgs {
     const void* A = nullptr; int lda = 0;        // bf16 [M, K]
     const void* W = nullptr; int ldw = 0;        // bf16 [N, K]
@@ -35,6 +47,7 @@ struct GemmArgs {
     int act = ACT_NONE;
     int bn_override = 0;  // 0 = cost-model heuristic, else 64/128/192/256 (2 = CTA-pair kernel)
     RopeQkv rope;         // ACT_ROPE_QKV only
+    GluAct glu;           // ACT_GLU only
     // fp32 output only (layer-list decoders): out = alpha * post(acc + bias + residual) (+ out when accumulate); post = LIN_*
     int post = 0; float alpha = 1.f; int accumulate = 0;
     // grouped product (mixture of experts; single-CTA kernels only): M is a multiple of 128, tile t of 128 rows multiplies with
@@ -308,17 +321,6 @@ bool linear_fuses_norm(int M, int K);
 int linear_f32(const LinearArgs& a, cudaStream_t stream);
 // out[r, :K] = bf16(A[r, :K]): the A operand of a tensor-core GEMM from fp32 activations (ld_out % 8 == 0)
 int cast_rows_bf16(const float* A, int64_t lda, void* out, int64_t ld_out, int M, int K, cudaStream_t stream);
-
-// The gated unit in its general form: with g = in[r, c] and u = in[r, ff + c], limit > 0 first bounds them, g = min(g, limit),
-// u = clamp(u, -limit, limit); out = a(g) (u + up_shift) with a(g) = g sigmoid(slope g), or (GLU_GELU_TANH) the tanh form of GELU,
-// a(g) = g / 2 (1 + tanh(sqrt(2 / pi) (g + 0.044715 g^3))). (slope 1, no limit, shift 0: SiLU(g) u.)
-enum { GLU_SIGMOID = 0, GLU_GELU_TANH = 1 };
-struct GluAct { float slope = 1.f, limit = 0.f, up_shift = 0.f; int kind = GLU_SIGMOID; };
-__host__ __device__ inline float glu_act(float g, float u, const GluAct& a) {
-    if (a.limit > 0.f) { g = fminf(g, a.limit); u = fminf(fmaxf(u, -a.limit), a.limit); }
-    const float v = a.kind == GLU_GELU_TANH ? 0.5f * g * (1.f + tanhf(0.7978845608028654f * fmaf(0.044715f * g * g, g, g))) : g / (1.f + expf(-a.slope * g));
-    return v * (u + a.up_shift);
-}
 
 // Grouped Linear: output rows come in tiles of tile_rows (1 or 64) rows; tile t multiplies with the weight matrix of group
 // tile_group[t] (W + group * w_group_stride elements; a negative group: the tile is unused). Output row m reads input row

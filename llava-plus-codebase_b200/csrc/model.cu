@@ -1487,10 +1487,21 @@ int b2_argmax(const float* logits, int B, int V, int32_t* out, void* stream) {
 int b2_op_gemm(const void* A, int lda, const void* W, int ldw, const void* bias, const void* residual, int ld_res,
                void* out, int ld_out, int out_fp32, int M, int N, int K, int act, int bn_override, void* stream) {
     B2_CHECK_ARG(A && W && out, "b2_op_gemm: null argument");
+    B2_CHECK_ARG(act != ACT_GLU, "gemm: unsupported activation %d", act);
     GemmArgs g;
     g.A = A; g.lda = lda; g.W = W; g.ldw = ldw; g.bias = bias; g.residual = residual; g.ld_res = ld_res;
     g.out = out; g.ld_out = ld_out; g.out_fp32 = out_fp32; g.M = M; g.N = N; g.K = K; g.act = act;
     g.bn_override = bn_override;
+    return gemm_bf16(g, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int b2_op_gemm_glu(const void* A, int lda, const void* W, int ldw, void* out, int ld_out, int M, int ff, int K, float slope, float limit,
+                   float up_shift, int kind, const int32_t* tile_group, int groups, int bn_override, void* stream) {
+    B2_CHECK_ARG(A && W && out && (kind == GLU_SIGMOID || kind == GLU_GELU_TANH), "b2_op_gemm_glu: bad argument");
+    GemmArgs g;
+    g.A = A; g.lda = lda; g.W = W; g.ldw = ldw; g.out = out; g.ld_out = ld_out; g.M = M; g.N = 2 * ff; g.K = K; g.act = ACT_GLU;
+    g.glu = GluAct{slope, limit, up_shift, kind};
+    g.tile_group = tile_group; g.groups = groups; g.bn_override = bn_override;
     return gemm_bf16(g, reinterpret_cast<cudaStream_t>(stream));
 }
 

@@ -670,6 +670,24 @@ static int sandwich_input(SeqModel& s, const float* post, const DevBuf& norm, co
     return 0;
 }
 
+// Whether a gated unit of a portion of a prompt runs inside its first product (and the second reads the bf16 rows that it leaves in s.ff): from
+// 17 rows on, i.e. wherever that product is a tile GEMM. The product alone wrote 2 ff fp32 values a row and the unit read them back: at width
+// 2048, ff 5632 and 2048 rows 78 us of product and 44 of unit, one launch of 68 now; a window-attention layer 431 -> 384 us, 1900 rows of gated
+// linear attention 532 -> 482, 41 rows through four layers 366 -> 364. Fewer rows stream their weights (linear_stream.cu).
+static bool glu_in_product(const Lin& lin, int ff, float* target, int R) {
+    const SeqModel& s = *lin.m->seq;
+    return R > LINEAR_STREAM_MAX && ff % 8 == 0 && lin.tensor_cores(2 * ff, s.d.width, s.ff.as<float>(), 2 * ff, R) && lin.tensor_cores(s.d.width, ff, target, s.d.width, R);
+}
+static int glu_product(const Lin& lin, const SubIn& in, const DevBuf& W, int ff, const GluAct& act, int R) {
+    const SeqModel& s = *lin.m->seq;
+    const int width = s.d.width;
+    if (in.h16 == nullptr) B2_TRY(cast_rows_bf16(in.h, width, s.a16.p, width, R, width, lin.st));
+    GemmArgs g;
+    g.A = in.h16 != nullptr ? in.h16 : s.a16.p; g.lda = width; g.W = W.p; g.ldw = width; g.out = s.ff.p; g.ld_out = ff;
+    g.M = R; g.N = 2 * ff; g.K = width; g.act = ACT_GLU; g.glu = act;
+    return gemm_bf16(g, lin.st);
+}
+
 // The feed-forward of a pre-norm, sandwich or parallel block in its kinds. in.h holds the fp32 rows always, in.h16 their rounded copy sometimes.
 static int seq_feed_forward(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, const SubIn& in, float* target, float alpha, int accumulate, int R,
                             cudaStream_t st) {
@@ -699,6 +717,9 @@ static int seq_feed_forward(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, c
             gs.M = R; gs.N = ff; gs.K = width; gs.round_a = s.d.compute == B2_COMPUTE_BF16; gs.swiglu = 1;
             gs.glu = act;
             B2_TRY(linear_grouped_f32(gs, st));
+        } else if (glu_in_product(lin, ff, target, R)) {
+            B2_TRY(glu_product(lin, in, W.up_w, ff, act, R));
+            return lin(nullptr, 0, W.down_w, width, ff, target, width, R, LIN_NONE, alpha, accumulate, nullptr, 0, nullptr, s.ff.p);
         } else {
             B2_TRY(lin(h, width, W.up_w, 2 * ff, width, s.ff.as<float>(), ffl, R, LIN_NONE, 1.f, 0, nullptr, 0, nullptr, in.h16));
             if (lin.tensor_cores(width, ff, target, width, R)) {   // the unit writes the bf16 rows that the second product reads
@@ -739,17 +760,21 @@ static int seq_feed_forward(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, c
             B2_TRY(lin(s.ff.as<float>(), sfl, W.sd_w, width, sf, target, width, R, LIN_NONE, alpha, accumulate));
         } else {
             const int sfl = (2 * sf + 7) / 8 * 8;
+            const void* down16 = nullptr;
             if (R <= 8) {   // decode step: both projections and the gate in one launch (the shared expert is "group 0" of its matrix)
                 GroupedLinearArgs gs;
                 gs.A = h; gs.lda = width; gs.a_div = 1; gs.W = W.sgu_w.p; gs.ldw = width; gs.w_group_stride = 0; gs.w_dtype = s.w_dtype;
                 gs.tile_group = s.zero_idx.as<int32_t>(); gs.tile_rows = 1; gs.out = s.ffa.as<float>(); gs.ld_out = sf;
                 gs.M = R; gs.N = sf; gs.K = width; gs.round_a = round_a; gs.swiglu = 1; gs.glu = act;
                 B2_TRY(linear_grouped_f32(gs, st));
+            } else if (glu_in_product(lin, sf, target, R)) {
+                B2_TRY(glu_product(lin, in, W.sgu_w, sf, act, R));
+                down16 = s.ff.p;
             } else {
                 B2_TRY(lin(h, width, W.sgu_w, 2 * sf, width, s.ff.as<float>(), sfl, R));
                 B2_TRY(glu_rows_f32(s.ff.as<float>(), sfl, s.ffa.as<float>(), sf, R, sf, act, st));
             }
-            B2_TRY(lin(s.ffa.as<float>(), sf, W.sd_w, width, sf, target, width, R, LIN_NONE, alpha, accumulate));
+            B2_TRY(lin(s.ffa.as<float>(), sf, W.sd_w, width, sf, target, width, R, LIN_NONE, alpha, accumulate, nullptr, 0, nullptr, down16));
         }
     } else if (!accumulate) {
         B2_CUDA_CHECK(cudaMemsetAsync(target, 0, (size_t)R * width * F4, st));
@@ -791,10 +816,10 @@ static int seq_feed_forward(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, c
         GemmArgs g1;
         g1.A = a16; g1.lda = width; g1.W = W.egu_w.p; g1.ldw = width; g1.out = s.moe_h.p; g1.ld_out = un; g1.out_fp32 = 1;
         g1.M = P; g1.N = un; g1.K = width; g1.tile_group = s.moe_tile.as<int32_t>(); g1.groups = E;
-        if (!gated) g1.post = LIN_RELU_SQ;
+        if (gated) { g1.act = ACT_GLU; g1.glu = act; g1.out = h16; g1.ld_out = ff; g1.out_fp32 = 0; }
+        else g1.post = LIN_RELU_SQ;
         B2_TRY(gemm_bf16(g1, st));
-        if (gated) B2_TRY(glu_rows_f32(s.moe_h.as<float>(), 2 * ff, nullptr, 0, P, ff, act, st, h16, ff));
-        else B2_TRY(cast_rows_bf16(s.moe_h.as<float>(), ff, h16, ff, P, ff, st));
+        if (!gated) B2_TRY(cast_rows_bf16(s.moe_h.as<float>(), ff, h16, ff, P, ff, st));
         GemmArgs g2;
         g2.A = h16; g2.lda = ff; g2.W = W.ed_w.p; g2.ldw = ff; g2.out = s.moe_y.p; g2.ld_out = width; g2.out_fp32 = 1;
         g2.M = P; g2.N = width; g2.K = ff; g2.tile_group = s.moe_tile.as<int32_t>(); g2.groups = E;
