@@ -261,6 +261,9 @@ int convert_to_bf16(const void* src, int src_dtype, void* dst, int64_t n, cudaSt
 int convert_to_f32(const void* src, int src_dtype, float* dst, int64_t n, cudaStream_t stream);  // src on the device
 // out[2I, h]: within each 128-row group g: rows [0,64) = gate[g*64 .. +64), rows [64,128) = up[g*64 .. +64)
 int interleave_gate_up(const void* gate, const void* up, void* out, int I, int h, cudaStream_t stream);
+// tok[:B] = tokens[:B], *step_counter = 0; and behind the step logits_out[:n] = logits[:n] (16-byte aligned), next[:B] = tok[:B]
+int decode_begin(int32_t* tok, const int32_t* tokens, int B, int32_t* step_counter, cudaStream_t stream);
+int decode_end(float* logits_out, const float* logits, int64_t n, int32_t* next, const int32_t* tok, int B, cudaStream_t stream);
 int store_token(const int32_t* src, int32_t* dst_base, const int32_t* step_counter, int B, cudaStream_t stream);
 
 // =====================================================================================================================

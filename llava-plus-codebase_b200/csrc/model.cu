@@ -1238,6 +1238,12 @@ static bool is_device_pointer(const void* p) {
     if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) { cudaGetLastError(); return false; }
     return attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
 }
+// memory of this device that a kernel may read or write `align` bytes at a time (host pointers, other devices' and odd addresses take copies)
+static bool on_device(const void* p, int device, size_t align) {
+    cudaPointerAttributes attr;
+    if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) { cudaGetLastError(); return false; }
+    return attr.type == cudaMemoryTypeDevice && attr.device == device && (reinterpret_cast<uintptr_t>(p) & (align - 1)) == 0;
+}
 
 int b2_decode_step(b2_model* m, b2_kv* kv, const int32_t* tokens, int B, void* logits_out, int32_t* next_tokens_out,
                    void* stream) {
@@ -1259,8 +1265,13 @@ int b2_decode_step_slots(b2_model* m, b2_kv* kv, const int32_t* tokens, int B, i
                      "b2_decode_step: sample %d has cache length %d (capacity %d; prefill first)", b, kv->len_host[b],
                      kv->max_seq);
     B2_TRY(ws_enter(m, st));
-    B2_CUDA_CHECK(cudaMemcpyAsync(kv->tok.as<int32_t>() + slot0, tokens, (size_t)B * 4, cudaMemcpyDefault, st));
-    B2_CUDA_CHECK(cudaMemsetAsync(kv->step_counter.p, 0, 4, st));
+    int32_t* tok = kv->tok.as<int32_t>() + slot0;
+    if (on_device(tokens, m->device, 4)) {
+        B2_TRY(decode_begin(tok, tokens, B, kv->step_counter.as<int32_t>(), st));
+    } else {
+        B2_CUDA_CHECK(cudaMemcpyAsync(tok, tokens, (size_t)B * 4, cudaMemcpyDefault, st));
+        B2_CUDA_CHECK(cudaMemsetAsync(kv->step_counter.p, 0, 4, st));
+    }
     B2_TRY(set_greedy_unpublished(kv, st));
     cudaStream_t run = nullptr;
     B2_TRY(fork_stream(kv, st, &run));
@@ -1268,10 +1279,15 @@ int b2_decode_step_slots(b2_model* m, b2_kv* kv, const int32_t* tokens, int B, i
     else B2_TRY(seq_decode_launch(m, kv, B, slot0, run));  // the captured step covers slots from 0: others run launch by launch
     B2_TRY(join_stream(kv, st, run));
     for (int b = slot0; b < slot0 + B; ++b) kv->len_host[b]++;
+    if ((logits_out || next_tokens_out) && (!logits_out || on_device(logits_out, m->device, 16)) && (!next_tokens_out || on_device(next_tokens_out, m->device, 4))) {
+        B2_TRY(decode_end(reinterpret_cast<float*>(logits_out), m->logits.as<float>(), logits_out ? (int64_t)B * m->d.vocab : 0, next_tokens_out, tok,
+                          next_tokens_out ? B : 0, st));
+        return ws_leave(m, st);
+    }
     if (logits_out)
         B2_CUDA_CHECK(cudaMemcpyAsync(logits_out, m->logits.p, (size_t)B * m->d.vocab * 4, cudaMemcpyDefault, st));
     if (next_tokens_out)
-        B2_CUDA_CHECK(cudaMemcpyAsync(next_tokens_out, kv->tok.as<int32_t>() + slot0, (size_t)B * 4, cudaMemcpyDefault, st));
+        B2_CUDA_CHECK(cudaMemcpyAsync(next_tokens_out, tok, (size_t)B * 4, cudaMemcpyDefault, st));
     B2_TRY(ws_leave(m, st));
     if ((next_tokens_out && !is_device_pointer(next_tokens_out)) || (logits_out && !is_device_pointer(logits_out)))
         B2_CUDA_CHECK(cudaStreamSynchronize(st));

@@ -96,6 +96,70 @@ __global__ void gated_group_rmsnorm_kernel(const float* __restrict__ y, int64_t 
     }
 }
 
+// Groups of up to 128 NV channels, 16 bytes at a time: a lane requests all that it will use of a group before it computes anything. The loop
+// above is a chain of dependent 4-byte loads: a step's row of 1024 channels in groups of 256 8.8 -> 5.5 us, 1900 rows 30.7 -> 10.3 us.
+template <int NV>
+__global__ void __launch_bounds__(256) gated_group_rmsnorm_vec_kernel(const float* __restrict__ y, int64_t ldy, const float* __restrict__ z, int64_t ldz,
+                                                                      const float* __restrict__ gamma, float* __restrict__ out, int64_t ldo, int rows,
+                                                                      int groups, int group, int gate_first, int gamma_shared, float eps, int sigmoid_gate,
+                                                                      const float* __restrict__ den, __nv_bfloat16* __restrict__ out16, int64_t ldo16) {
+    pdl_enter();
+    const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (w >= rows * groups) return;
+    const int r = w / groups, g = w % groups;
+    const float* yr = y + (size_t)r * ldy + (size_t)g * group;
+    const float* zr = z != nullptr ? z + (size_t)r * ldz + (size_t)g * group : nullptr;
+    const float* gm = gamma + (gamma_shared ? 0 : (size_t)g * group);
+    float yv[NV][4], gz[NV][4], wv[NV][4];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int c = (lane + 32 * i) * 4;
+        const bool in = c < group;
+        *reinterpret_cast<float4*>(yv[i]) = in ? *reinterpret_cast<const float4*>(yr + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        *reinterpret_cast<float4*>(gz[i]) = in && zr != nullptr ? *reinterpret_cast<const float4*>(zr + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        *reinterpret_cast<float4*>(wv[i]) = in ? *reinterpret_cast<const float4*>(gm + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const float pre = den != nullptr ? 1.f / den[(size_t)r * groups + g] : 1.f;
+    float q = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            gz[i][e] = zr == nullptr ? 1.f : (sigmoid_gate ? 1.f / (1.f + expf(-gz[i][e])) : silu_f(gz[i][e]));
+            const float v = (gate_first ? yv[i][e] * gz[i][e] : yv[i][e]) * pre;
+            q = fmaf(v, v, q);   // (entries past the group are zeros)
+        }
+    q = warp_sum(q);
+    const float rinv = pre / sqrtf(q / (float)group + eps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int c = (lane + 32 * i) * 4;
+        if (c >= group) break;
+        float v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = gate_first ? (yv[i][e] * gz[i][e]) * rinv * wv[i][e] : yv[i][e] * rinv * wv[i][e] * gz[i][e];
+        if (out16 != nullptr) *reinterpret_cast<uint2*>(out16 + (size_t)r * ldo16 + (size_t)g * group + c) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+        else *reinterpret_cast<float4*>(out + (size_t)r * ldo + (size_t)g * group + c) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+}
+
+int launch_group_norm(const float* y, int64_t ldy, const float* z, int64_t ldz, const float* gamma, float* out, int64_t ldo, int rows, int groups,
+                      int group, int gate_first, int gamma_shared, float eps, int sigmoid_gate, const float* den, void* out16, int64_t ldo16, cudaStream_t st) {
+    const dim3 grid((rows * groups + 7) / 8), block(256);
+    __nv_bfloat16* o16 = reinterpret_cast<__nv_bfloat16*>(out16);
+    const uintptr_t align = reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(gamma) | (out16 != nullptr ? 0 : reinterpret_cast<uintptr_t>(out));
+    const bool vec = group % 4 == 0 && group <= 512 && (align & 15) == 0 && ldy % 4 == 0 && (z == nullptr || ldz % 4 == 0) &&
+                     (out16 != nullptr ? (reinterpret_cast<uintptr_t>(out16) & 7) == 0 && ldo16 % 4 == 0 : ldo % 4 == 0) &&
+                     !(gate_first && sigmoid_gate);   // (that pair norms one gate and applies another: the loop does it)
+    auto run = [&](auto kernel) { launch_pdl(kernel, grid, block, 0, st, y, ldy, z, ldz, gamma, out, ldo, rows, groups, group, gate_first, gamma_shared, eps, sigmoid_gate, den, o16, ldo16); };
+    if (!vec) run(gated_group_rmsnorm_kernel);
+    else if (group <= 128) run(gated_group_rmsnorm_vec_kernel<1>);
+    else if (group <= 256) run(gated_group_rmsnorm_vec_kernel<2>);
+    else run(gated_group_rmsnorm_vec_kernel<4>);
+    B2_LAUNCH_CHECK();
+    return 0;
+}
+
 // one or two dynamic-tanh norms of a row: the row is read once, 16 bytes at a time where the width allows
 struct DytOuts { DytOut o[2]; };
 __device__ __forceinline__ float dyt_f(float x, float alpha, float w, float b) { return fmaf(tanhf(alpha * x), w, b); }
@@ -166,7 +230,17 @@ __global__ void diff_combine_kernel(const float* __restrict__ y, int64_t ldy, fl
     for (int c = lane; c < dv; c += 32) o[c] = fmaf(-lambda, a2[c], a1[c]) * mul;
 }
 
-template <typename TT>
+__device__ __forceinline__ void ld8(const float* p, float (&v)[8]) {
+    *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p);
+    *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(p + 4);
+}
+__device__ __forceinline__ void ld8(const __nv_bfloat16* p, float (&v)[8]) {
+    const uint4 u = *reinterpret_cast<const uint4*>(p);
+    v[0] = bf16_lo(u.x); v[1] = bf16_hi(u.x); v[2] = bf16_lo(u.y); v[3] = bf16_hi(u.y);
+    v[4] = bf16_lo(u.z); v[5] = bf16_hi(u.z); v[6] = bf16_lo(u.w); v[7] = bf16_hi(u.w);
+}
+// VEC: 8 entries of a row per thread (one entry per thread and step made 16 rounds of loads of a 2048-wide row: 7.4 -> 4.3 us of a step, 1900 rows 11.4 -> 6.4)
+template <typename TT, bool VEC>
 __global__ void embed_rows_kernel(const int32_t* __restrict__ tokens, const TT* __restrict__ table, float* __restrict__ x, int cols, int vocab,
                                   int* err_flag, float scale) {
     pdl_enter();
@@ -174,7 +248,21 @@ __global__ void embed_rows_kernel(const int32_t* __restrict__ tokens, const TT* 
     const int t = tokens[r];
     const bool ok = t >= 0 && t < vocab;
     if (!ok && threadIdx.x == 0 && err_flag != nullptr) err_flag[0] = 1;  // slot 0 = B2_ERR_TOKEN_RANGE
-    for (int c = threadIdx.x; c < cols; c += blockDim.x) x[r * cols + c] = ok ? (float)table[(size_t)t * cols + c] * scale : 0.f;
+    if (VEC) {
+        for (int c = threadIdx.x * 8; c < cols; c += blockDim.x * 8) {
+            float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (ok) {
+                ld8(table + (size_t)t * cols + c, v);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[e] *= scale;
+            }
+            float4* d = reinterpret_cast<float4*>(x + r * cols + c);
+            d[0] = make_float4(v[0], v[1], v[2], v[3]);
+            d[1] = make_float4(v[4], v[5], v[6], v[7]);
+        }
+    } else {
+        for (int c = threadIdx.x; c < cols; c += blockDim.x) x[r * cols + c] = ok ? (float)table[(size_t)t * cols + c] * scale : 0.f;
+    }
 }
 
 __global__ void sigmoid_gate_kernel(const float* __restrict__ a, int64_t lda, const float* __restrict__ g, int64_t ldg, float* __restrict__ out,
@@ -641,21 +729,13 @@ int gated_group_rmsnorm_f32(const float* y, int64_t ldy, const float* z, int64_t
                             void* out16, int64_t ld_out16) {
     B2_CHECK_ARG(y && z && gamma && (out || out16) && rows > 0 && group > 0 && cols % group == 0, "gated_group_rmsnorm: cols %d is not a multiple of the group %d",
                  cols, group);
-    const int groups = cols / group, warps = rows * groups;
-    launch_pdl(gated_group_rmsnorm_kernel, dim3((warps + 7) / 8), dim3(256), 0, st, y, ldy, z, ldz, gamma, out, ldo, rows, groups, group, gate_first,
-               gamma_shared, eps, sigmoid_gate, den, reinterpret_cast<__nv_bfloat16*>(out16), ld_out16);
-    B2_LAUNCH_CHECK();
-    return 0;
+    return launch_group_norm(y, ldy, z, ldz, gamma, out, ldo, rows, cols / group, group, gate_first, gamma_shared, eps, sigmoid_gate, den, out16, ld_out16, st);
 }
 
 int group_rmsnorm_f32(const float* y, int64_t ldy, const float* gamma, int gamma_shared, float* out, int64_t ldo, int rows, int cols, int group,
                       float eps, cudaStream_t st) {
     B2_CHECK_ARG(y && gamma && out && rows > 0 && group > 0 && cols % group == 0, "group_rmsnorm: cols %d is not a multiple of the group %d", cols, group);
-    const int groups = cols / group, warps = rows * groups;
-    launch_pdl(gated_group_rmsnorm_kernel, dim3((warps + 7) / 8), dim3(256), 0, st, y, ldy, nullptr, 0, gamma, out, ldo, rows, groups, group, 0,
-               gamma_shared, eps, 0, nullptr, nullptr, 0);
-    B2_LAUNCH_CHECK();
-    return 0;
+    return launch_group_norm(y, ldy, nullptr, 0, gamma, out, ldo, rows, cols / group, group, 0, gamma_shared, eps, 0, nullptr, nullptr, 0, st);
 }
 
 int diff_combine_f32(const float* y, int64_t ldy, float* out, int64_t ldo, int rows, int heads, int dv, float lambda, float out_scale, float eps,
@@ -674,11 +754,16 @@ int embed_rows_f32(const int32_t* tokens, const void* table, int table_dtype, fl
         if (table_dtype == DT_F32) return launch_embed_norm(tokens, reinterpret_cast<const float*>(table), x, rows, cols, vocab, err_flag, norm_w, eps, st);
         return launch_embed_norm(tokens, reinterpret_cast<const __nv_bfloat16*>(table), x, rows, cols, vocab, err_flag, norm_w, eps, st);
     }
-    if (table_dtype == DT_F32)
-        launch_pdl(embed_rows_kernel<float>, dim3(rows), dim3(128), 0, st, tokens, reinterpret_cast<const float*>(table), x, cols, vocab, err_flag, scale);
-    else
-        launch_pdl(embed_rows_kernel<__nv_bfloat16>, dim3(rows), dim3(128), 0, st, tokens, reinterpret_cast<const __nv_bfloat16*>(table), x, cols, vocab,
-                   err_flag, scale);
+    const bool vec = cols % 8 == 0 && ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
+    const dim3 grid(rows), block(vec ? (cols >= 2048 ? 256 : 128) : 128);
+    auto run = [&](auto kernel, auto* tab) { launch_pdl(kernel, grid, block, 0, st, tokens, tab, x, cols, vocab, err_flag, scale); };
+    if (table_dtype == DT_F32) {
+        const float* tab = reinterpret_cast<const float*>(table);
+        if (vec) run(embed_rows_kernel<float, true>, tab); else run(embed_rows_kernel<float, false>, tab);
+    } else {
+        const __nv_bfloat16* tab = reinterpret_cast<const __nv_bfloat16*>(table);
+        if (vec) run(embed_rows_kernel<__nv_bfloat16, true>, tab); else run(embed_rows_kernel<__nv_bfloat16, false>, tab);
+    }
     B2_LAUNCH_CHECK();
     return 0;
 }
