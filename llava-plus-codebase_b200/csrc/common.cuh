@@ -152,6 +152,10 @@ __device__ __forceinline__ uint4 ld_stream_16(const void* p) {
     return r;
 }
 
+// One lane of a converged warp. The loops that issue tcgen05.mma are walked by their whole warp, and only the products and their commit are the
+// elected lane's: descriptors and barrier addresses then stay warp-uniform. With the next stage's barrier looked at before this stage's products
+// (mbar_try_wait) a k-block of 64 takes its thread 335-385 clk; walked by one lane that waits for each barrier in turn 430, whatever the tile's
+// width, which is more than the products themselves take up to N = 192 (four of 48 / 64 / 96 clk at N = 64 / 128 / 192).
 __device__ __forceinline__ bool elect_one() {
     uint32_t pred = 0;
     asm volatile(
@@ -185,7 +189,7 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
                  : "memory");
 }
 // Spin on try_wait (HW-suspended wait with a time hint). A bounded spin count turns a protocol bug
-// into a trap instead of a GPU hang (a hang costs a gpurun strike; a trap is a clean CUDA error).
+// into a trap instead of a GPU hang (a trap is a clean CUDA error).
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
     uint32_t addr = smem_u32(bar);
     uint32_t done = 0;

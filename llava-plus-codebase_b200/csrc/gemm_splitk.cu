@@ -28,6 +28,7 @@ struct KsEpi {
     void* out;
     int ld_out, ld_res, out_fp32, post, accumulate;
     float alpha;
+    int a_bytes;           // of A per k-block: gemm_a_rows(M) rows
 };
 
 __device__ __forceinline__ uint32_t ks_rank() {
@@ -80,7 +81,7 @@ __global__ void __launch_bounds__(KS_THREADS, 1) gemm_splitk_kernel(const __grid
             // the weight halves of the first stages travel in front of the programmatic-dependent-launch wait, A follows behind it
             const int pre = kb1 - kb0 < STAGES ? kb1 - kb0 : STAGES;
             for (int i = 0; i < pre; ++i) {
-                mbar_arrive_expect_tx(&full[i], Cfg::STAGE);
+                mbar_arrive_expect_tx(&full[i], ep.a_bytes + BN * KS_BK * 2);
                 tma_load_2d(smem + i * Cfg::STAGE + KS_A, &tmap_b, &full[i], (kb0 + i) * KS_BK, n0, kEvictNormal);
             }
             pdl_wait();
@@ -90,7 +91,7 @@ __global__ void __launch_bounds__(KS_THREADS, 1) gemm_splitk_kernel(const __grid
                 uint8_t* sa = smem + stage * Cfg::STAGE;
                 if (kb - kb0 >= pre) {
                     mbar_wait(&empty[stage], phase ^ 1);
-                    mbar_arrive_expect_tx(&full[stage], Cfg::STAGE);
+                    mbar_arrive_expect_tx(&full[stage], ep.a_bytes + BN * KS_BK * 2);
                     tma_load_2d(sa + KS_A, &tmap_b, &full[stage], kb * KS_BK, n0, kEvictNormal);
                 }
                 tma_load_2d(sa, &tmap_a, &full[stage], kb * KS_BK, m0, kEvictNormal);
@@ -99,23 +100,27 @@ __global__ void __launch_bounds__(KS_THREADS, 1) gemm_splitk_kernel(const __grid
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc_bf16_f32(KS_BM, BN);
-            int stage = 0;
-            uint32_t phase = 0;
-            for (int kb = kb0; kb < kb1; ++kb) {
-                mbar_wait(&full[stage], phase);
-                tc_fence_after();
-                const uint32_t sa = smem_u32(smem + stage * Cfg::STAGE);
-                const uint64_t da = make_sw128_kmajor_desc(sa), db = make_sw128_kmajor_desc(sa + KS_A);
+        constexpr uint32_t idesc = make_idesc_bf16_f32(KS_BM, BN);
+        int stage = 0;
+        uint32_t phase = 0, ready = 0;
+        for (int kb = kb0; kb < kb1; ++kb) {
+            if (!ready) mbar_wait(&full[stage], phase);
+            const int next = stage + 1 == STAGES ? 0 : stage + 1;
+            const uint32_t next_phase = next == 0 ? phase ^ 1 : phase;
+            ready = __all_sync(0xffffffffu, kb + 1 < kb1 ? mbar_try_wait(&full[next], next_phase) : 0u);
+            tc_fence_after();
+            const uint32_t sa = smem_u32(smem + stage * Cfg::STAGE);
+            const uint64_t da = make_sw128_kmajor_desc(sa), db = make_sw128_kmajor_desc(sa + KS_A);
+            if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < KS_BK / 16; ++k) umma_bf16(tmem, da + 2 * k, db + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
                 umma_commit(&empty[stage]);
                 if (kb == kb1 - 1) umma_commit(done);
-                if (++stage == STAGES) { stage = 0; phase ^= 1; }
             }
+            __syncwarp();
+            stage = next;
+            phase = next_phase;
         }
-        __syncwarp();
     } else {
         // the accumulator into the drained ring (every load has landed and every product has read it when `done` completes): [4 columns][128 rows]
         const int q = warp & 3, half = (warp - 2) >> 2, row = q * 32 + lane;
@@ -139,7 +144,7 @@ __global__ void __launch_bounds__(KS_THREADS, 1) gemm_splitk_kernel(const __grid
         pdl_wait();   // residual and output may be written by the kernels in front
         const int t = threadIdx.x - 64, row = t & 127, per = BN / S / 8;   // 8-column groups of this CTA's share
         const uint32_t base = smem_u32(smem);
-        for (int j = t >> 7; j < per; j += 2) {
+        for (int j = t >> 7; j < per && m0 + row < M; j += 2) {
             const int c8 = rank * per + j;   // group of 8 columns inside the tile
             float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             for (int s = 0; s < S; ++s) {
@@ -147,7 +152,7 @@ __global__ void __launch_bounds__(KS_THREADS, 1) gemm_splitk_kernel(const __grid
                 x[0] += u.x; x[1] += u.y; x[2] += u.z; x[3] += u.w; x[4] += w.x; x[5] += w.y; x[6] += w.z; x[7] += w.w;
             }
             const int m = m0 + row, n = n0 + c8 * 8;
-            if (m >= M || n >= N) continue;
+            if (n >= N) continue;
             if (ep.bias != nullptr) {
                 const uint4 b = *reinterpret_cast<const uint4*>(ep.bias + n);
                 x[0] += bf16_lo(b.x); x[1] += bf16_hi(b.x); x[2] += bf16_lo(b.y); x[3] += bf16_hi(b.y);
@@ -182,7 +187,7 @@ __global__ void __launch_bounds__(KS_THREADS, 1) gemm_splitk_kernel(const __grid
 template <int BN, int ACT>
 int launch_splitk(const GemmArgs& g, int S, const KsEpi& ep, cudaStream_t st) {
     CUtensorMap ta, tb;
-    B2_TRY(make_tmap_bf16(&ta, g.A, g.M, g.K, g.lda, KS_BM));
+    B2_TRY(make_tmap_bf16(&ta, g.A, g.M, g.K, g.lda, gemm_a_rows(g.M)));
     B2_TRY(make_tmap_bf16(&tb, g.W, g.N, g.K, g.ldw, BN));
     auto kernel = gemm_splitk_kernel<BN, ACT>;
     B2_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KsCfg<BN>::SMEM));
@@ -210,6 +215,7 @@ int gemm_bf16_splitk(const GemmArgs& g, int bn, int S, cudaStream_t st) {
     B2_CHECK_ARG((bn == 64 || bn == 128) && (S == 2 || S == 4) && S <= (g.K + KS_BK - 1) / KS_BK && g.act != ACT_SWIGLU && g.act != ACT_ROPE_QKV && g.tile_group == nullptr,
                  "gemm(split K): bad plan bn=%d S=%d K=%d", bn, S, g.K);
     KsEpi ep;
+    ep.a_bytes = gemm_a_rows(g.M) * KS_BK * 2;
     ep.bias = reinterpret_cast<const __nv_bfloat16*>(g.bias); ep.residual = reinterpret_cast<const __nv_bfloat16*>(g.residual);
     ep.out = g.out; ep.ld_out = g.ld_out; ep.ld_res = g.ld_res; ep.out_fp32 = g.out_fp32;
     ep.post = g.out_fp32 ? g.post : 0; ep.alpha = g.out_fp32 ? g.alpha : 1.f; ep.accumulate = g.out_fp32 ? g.accumulate : 0;

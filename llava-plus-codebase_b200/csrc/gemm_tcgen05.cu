@@ -132,6 +132,7 @@ struct EpiParams {
     const int* tile_group = nullptr;
     int group_rows = 0;
     GluAct glu;            // ACT_GLU
+    int a_bytes = BM * BK * 2;   // of A per k-block: gemm_a_rows(M) rows
 };
 
 __device__ __forceinline__ float act_quick_gelu(float x) { return __fdividef(x, 1.0f + __expf(-1.702f * x)); }
@@ -223,7 +224,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
                 tile_coords(blockIdx.x, m_blk, n_blk);
                 for (int kb = 0; kb < num_kb && pre_n < STAGES; ++kb, ++pre_n) {
                     uint8_t* sb = smem + pre_n * Cfg::STAGE_BYTES + A_TILE_BYTES;
-                    mbar_arrive_expect_tx(&full_bar[pre_n], Cfg::STAGE_BYTES);
+                    mbar_arrive_expect_tx(&full_bar[pre_n], ep.a_bytes + Cfg::B_TILE_BYTES);
                     load_b(sb, &full_bar[pre_n], kb, 0, n_blk);
                 }
             }
@@ -240,7 +241,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
                     uint8_t* sb = sa + A_TILE_BYTES;
                     if (seen >= pre_n) {
                         mbar_wait(&empty_bar[stage], phase ^ 1);
-                        mbar_arrive_expect_tx(&full_bar[stage], Cfg::STAGE_BYTES);
+                        mbar_arrive_expect_tx(&full_bar[stage], ep.a_bytes + Cfg::B_TILE_BYTES);
                         load_b(sb, &full_bar[stage], kb, w_row0, n_blk);
                     }
                     tma_load_2d(sa, &tmap_a, &full_bar[stage], kb * BK, m_blk * BM, kEvictNormal);
@@ -249,11 +250,14 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
             }
         }
     } else if (warp == 1) {
-        // ===================== MMA issuer (one thread) =====================
-        if (lane == 0) {
+        // ===================== MMA issuer (one warp, an elected lane) =====================
+        // Walked by the whole warp up to BN = 128 (elect_one, common.cuh). A wider tile's products cover what one lane's loop takes, and 32 lanes at
+        // its barriers cost it more than that: M = 32, N = 22016, K = 4096 in tiles of 256 36.4 us by one lane, 38.0 by the warp.
+        constexpr bool WARP = BN <= 128;
+        if (WARP || lane == 0) {
             constexpr uint32_t idesc = make_idesc_bf16_f32(BM, BN);
             int stage = 0;
-            uint32_t phase = 0;
+            uint32_t phase = 0, ready = 0;
             int local = 0;
             if (ep.tile_group != nullptr) pdl_wait();   // the group table comes from the upstream kernel
             for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
@@ -269,19 +273,26 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + as * Cfg::ACC_STRIDE;
                 for (int kb = 0; kb < num_kb; ++kb) {
-                    mbar_wait(&full_bar[stage], phase);  // TMA bytes have landed
+                    if (!ready) mbar_wait(&full_bar[stage], phase);  // TMA bytes have landed
+                    const int next = stage + 1 == STAGES ? 0 : stage + 1;
+                    const uint32_t next_phase = next == 0 ? phase ^ 1 : phase;
+                    if constexpr (WARP) ready = __all_sync(0xffffffffu, kb + 1 < num_kb ? mbar_try_wait(&full_bar[next], next_phase) : 0u);
                     tc_fence_after();
                     const uint32_t sa = smem_u32(smem + stage * Cfg::STAGE_BYTES);
                     const uint64_t da = make_sw128_kmajor_desc(sa);
                     const uint64_t db = make_sw128_kmajor_desc(sa + A_TILE_BYTES);
+                    if (!WARP || elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < BK / 16; ++k) {
-                        // advance 16 bf16 = 32 B along K inside the 128B swizzle atom: +2 in the addr field
-                        umma_bf16(tmem_d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                        for (int k = 0; k < BK / 16; ++k) {
+                            // advance 16 bf16 = 32 B along K inside the 128B swizzle atom: +2 in the addr field
+                            umma_bf16(tmem_d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                        }
+                        umma_commit(&empty_bar[stage]);  // smem slot reusable once these MMAs retire
+                        if (kb == num_kb - 1) umma_commit(&tmem_full[as]);  // accumulator complete
                     }
-                    umma_commit(&empty_bar[stage]);  // smem slot reusable once these MMAs retire
-                    if (kb == num_kb - 1) umma_commit(&tmem_full[as]);  // accumulator complete
-                    if (++stage == STAGES) { stage = 0; phase ^= 1; }
+                    if constexpr (WARP) __syncwarp();
+                    stage = next;
+                    phase = next_phase;
                 }
             }
         }
@@ -754,10 +765,11 @@ int gemm_bf16(const GemmArgs& g, cudaStream_t stream) {
     if (glu && bn % 128 != 0) bn = 128;
 
     CUtensorMap ta, tb;
-    B2_TRY(make_tmap_bf16(&ta, g.A, g.M, g.K, g.lda, BM));
+    B2_TRY(make_tmap_bf16(&ta, g.A, g.M, g.K, g.lda, gemm_a_rows(g.M)));
     B2_TRY(make_tmap_bf16(&tb, g.W, grouped ? g.N * g.groups : g.N, g.K, g.ldw, g.act == ACT_GLU ? 64 : bn));
     EpiParams ep;
     ep.glu = g.glu;
+    ep.a_bytes = gemm_a_rows(g.M) * BK * 2;
     ep.tile_group = g.tile_group; ep.group_rows = g.N;
     ep.bias = reinterpret_cast<const __nv_bfloat16*>(g.bias);
     ep.residual = reinterpret_cast<const __nv_bfloat16*>(g.residual);

@@ -55,6 +55,9 @@ struct GemmArgs {
     const int* tile_group = nullptr; int groups = 1;
 };
 int gemm_bf16(const GemmArgs& g, cudaStream_t stream);
+// Rows of A that a tile of 128 rows loads per k-block: with fewer rows in all, the rest of the tile is left as it lies in shared memory (a row of
+// A touches its own row of the accumulator only, and those rows are not stored).
+inline int gemm_a_rows(int M) { return M >= 128 ? 128 : (M + 7) / 8 * 8; }
 // mm_projector mlp2x_gelu as ONE kernel (gemm_tcgen05.cu, projector_fused_kernel): out = gelu_erf(X W1^T + b1) W2^T + b2.
 // H [M,N1] bf16 and row_done int[ceil(M/128)] are caller scratch.
 int projector_fused_bf16(const void* X, int ldx, const void* W1, const void* b1, const void* W2, const void* b2, void* H,

@@ -111,9 +111,14 @@ int gemv(const void* x, int64_t ldx, const void* W, int ldw, const void* gamma, 
     return gemv_bf16(g, st);
 }
 
-// decode Linear at batch 9..128: swap-AB stream-K tcgen05 GEMM over the kv-owned workspace
+// Decode Linear at batch 7..128: the tile GEMMs (a tile loads the rows of x that there are; K cut over clusters where few tiles would be left).
+// Measured against the stream-K GEMM over the kv-owned workspace, whose shared tiles cost it 8 us of fix-up (h = 4096, weights from memory; B = 9 /
+// 32 / 128): [B, 12288] 26.6 -> 22.9, 27.3 -> 22.8, 39.5 -> 24.1 us; [B, 4096] 14.6 -> 10.5, 15.4 -> 10.9, 35.3 -> 12.2; gate/up 36.5 -> 36.1, 37.6 ->
+// 36.6, 57.7 -> 37.7; down 22.3 -> 20.1, 23.2 -> 20.4, 43.2 -> 22.2; 32000 columns 51.4 -> 46.6, 52.3 -> 46.9, 76.9 -> 50.7. It stays for sizes that
+// the tile GEMMs refuse, and for fp8 weights.
 int skinny(b2_kv* kv, const void* x, int ldx, const void* W, int ldw, const void* res, int ld_res, void* out, int ld_out,
            int out_fp32, int B, int N, int K, int act, cudaStream_t st) {
+    if (N % 8 == 0 && ld_out % 8 == 0 && (res == nullptr || ld_res % 8 == 0)) return gemm(x, ldx, W, ldw, nullptr, res, ld_res, out, ld_out, out_fp32, B, N, K, act, st);
     SkinnyArgs g;
     g.x = x; g.ldx = ldx; g.W = W; g.ldw = ldw; g.residual = res; g.ld_res = ld_res;
     g.out = out; g.ld_out = ld_out; g.out_fp32 = out_fp32; g.B = B; g.N = N; g.K = K; g.act = act;
