@@ -309,6 +309,8 @@ struct LinearArgs {
     int round_a = 0;                             // round A to bf16 first (bf16 compute: the product is bf16 x bf16 -> fp32)
     DytNorm norm;                                // norm.alpha non-null: A passes this norm while it is staged (linear_fuses_norm calls only)
     void* parts = nullptr; size_t parts_bytes = 0;   // scratch of linear_split_f32
+    int gated = 0; GluAct glu;                   // linear_stream_f32 only: W = [gate | up] of N rows each, out = glu_act(gate, up); no act, bias, alpha
+    void* out16 = nullptr;                       // with gated: bf16 rows of pitch ld_out in place of out
     const void* A16 = nullptr;                   // the same rows already rounded to bf16, pitch K (linear_stream_f32 reads these when there are 2 or more)
 };
 // True fp32, a portion of a prompt (linear_split.cu): whether a call runs on the tensor cores as products of bf16 parts. Scratch: the parts of A and

@@ -9,7 +9,8 @@
 // 2..16 rows: mma.sync m16n8k16 (weights are the 16-row operand, the rows of A the 8 columns; 9..16 rows take two column tiles): tcgen05 wants
 // 128 rows of A or a 128-row weight tile per CTA, which cuts these matrices into too few pieces. One row: the same stream on the FMA pipe.
 // A four-layer model of width 2048 (weights 0.49 GB a step), one decode step: 8 slots 420 -> 274 us (before: a cast and the 128-row tile GEMM,
-// 17-31 us a product; here 9), one slot 285 -> 256 us (before: one warp or a few per column).
+// 17-31 us a product; here 9), one slot 285 -> 256 us (before: one warp or a few per column). With the gated unit of a feed-forward inside its
+// first product: 48 steps 12.23 -> 12.03 ms (one slot; before: one warp per output), 14.81 -> 14.53 (8 slots; before: a product and a launch of its own).
 #include <algorithm>
 
 #include "common.cuh"
@@ -25,24 +26,25 @@ __device__ __forceinline__ void mma_16x8x16(float (&c)[4], uint32_t a0, uint32_t
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// NT: column tiles of 8 rows of A (0: one row on the FMA pipe). A16: A lies there as bf16 rows of pitch K.
-template <int NT, bool A16>
+// NT: column tiles of 8 rows of A (0: one row on the FMA pipe). A16: A lies there as bf16 rows of pitch K. GLU: a tile is 8 outputs of a gated unit,
+// rows 0..7 their gate weights and 8..15 their up weights.
+template <int NT, bool A16, bool GLU>
 __global__ void __launch_bounds__(LS_WARPS * 32, 2) linear_stream_kernel(LinearArgs a) {
-    constexpr int COLS = NT == 0 ? 1 : 8 * NT;
+    constexpr int COLS = NT == 0 ? 1 : 8 * NT, OUTS = GLU ? LS_N / 2 : LS_N;   // outputs per tile
     __shared__ float red[LS_WARPS][LS_N][COLS + (NT == 0 ? 0 : 1)];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = lane >> 2, kq = (lane & 3) * 8;
     const int units = (a.K + LS_UNIT - 1) / LS_UNIT, upw = (units + LS_WARPS - 1) / LS_WARPS;   // units per warp and tile
-    const int tiles = (a.N + LS_N - 1) / LS_N, mine = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int tiles = (a.N + OUTS - 1) / OUTS, mine = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
     const int steps = mine * upw;
     const __nv_bfloat16* W = reinterpret_cast<const __nv_bfloat16*>(a.W);
 
     uint4 w[2][4][2];
     auto load_w = [&](int s, uint4 (&u)[4][2]) {   // step s: tile s / upw of this CTA, unit (s % upw) * 8 + warp
-        const int n0 = ((int)blockIdx.x + (s / upw) * (int)gridDim.x) * LS_N, k0 = ((s % upw) * LS_WARPS + warp) * LS_UNIT + kq;
+        const int n0 = ((int)blockIdx.x + (s / upw) * (int)gridDim.x) * OUTS, k0 = ((s % upw) * LS_WARPS + warp) * LS_UNIT + kq;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int n = n0 + row + 8 * h;
-            const __nv_bfloat16* p = W + (size_t)(n < a.N ? n : 0) * a.ldw + k0;
+            const int n = n0 + row + (GLU ? 0 : 8 * h);
+            const __nv_bfloat16* p = W + (size_t)(n < a.N ? n + (GLU ? h * a.N : 0) : 0) * a.ldw + k0;
 #pragma unroll
             for (int c = 0; c < 4; ++c) u[c][h] = s < steps && n < a.N && k0 + 32 * c < a.K ? ld_stream_16(p + 32 * c) : make_uint4(0, 0, 0, 0);
         }
@@ -112,7 +114,7 @@ __global__ void __launch_bounds__(LS_WARPS * 32, 2) linear_stream_kernel(LinearA
     };
     auto finish = [&](int s) {   // the last unit of a tile: the warps' sums meet, every thread writes some outputs
         if (s % upw != upw - 1) return;
-        const int n0 = ((int)blockIdx.x + (s / upw) * (int)gridDim.x) * LS_N;
+        const int n0 = ((int)blockIdx.x + (s / upw) * (int)gridDim.x) * OUTS;
         __syncthreads();   // the previous tile's sums have been read
         if (NT == 0) {
             float v0 = acc[0][0] + acc[0][1], v1 = acc[0][2] + acc[0][3];
@@ -132,12 +134,19 @@ __global__ void __launch_bounds__(LS_WARPS * 32, 2) linear_stream_kernel(LinearA
 #pragma unroll
             for (int i = 0; i < 4; ++i) acc[t][i] = 0.f;
         __syncthreads();
-        const int i = threadIdx.x & 15, m = threadIdx.x >> 4, n = n0 + i;
+        const int i = threadIdx.x % OUTS, m = threadIdx.x / OUTS, n = n0 + i;
         if (m < a.M && m < COLS && n < a.N) {
             float v = 0.f;
 #pragma unroll
             for (int q = 0; q < LS_WARPS; ++q) v += red[q][i][m];
-            linear_store(a.out + (size_t)m * a.ld_out + n, v, a.bias, n, a.act, a.alpha, a.accumulate);
+            if constexpr (GLU) {
+                float u = 0.f;
+#pragma unroll
+                for (int q = 0; q < LS_WARPS; ++q) u += red[q][i + OUTS][m];
+                v = glu_act(v, u, a.glu);
+                if (a.out16 != nullptr) reinterpret_cast<__nv_bfloat16*>(a.out16)[(size_t)m * a.ld_out + n] = __float2bfloat16_rn(v);
+                else a.out[(size_t)m * a.ld_out + n] = v;
+            } else linear_store(a.out + (size_t)m * a.ld_out + n, v, a.bias, n, a.act, a.alpha, a.accumulate);
         }
     };
     for (int s = 0; s < steps; s += 2) {
@@ -152,10 +161,10 @@ __global__ void __launch_bounds__(LS_WARPS * 32, 2) linear_stream_kernel(LinearA
     }
 }
 
-template <int NT, bool A16>
+template <int NT, bool A16, bool GLU>
 int launch_stream(const LinearArgs& a, cudaStream_t st) {
-    const int tiles = (a.N + LS_N - 1) / LS_N;
-    B2_CUDA_CHECK(launch_pdl(linear_stream_kernel<NT, A16>, dim3(std::min(tiles, 2 * num_sms())), dim3(LS_WARPS * 32), 0, st, a));
+    const int tiles = GLU ? (a.N + LS_N / 2 - 1) / (LS_N / 2) : (a.N + LS_N - 1) / LS_N;
+    B2_CUDA_CHECK(launch_pdl(linear_stream_kernel<NT, A16, GLU>, dim3(std::min(tiles, 2 * num_sms())), dim3(LS_WARPS * 32), 0, st, a));
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -167,10 +176,13 @@ bool linear_streams(const LinearArgs& a) {
            (a.M > 1 && a.A16 != nullptr ? (reinterpret_cast<uintptr_t>(a.A16) & 15) == 0 : a.A != nullptr && (a.M == 1 || a.lda % 4 == 0) && (reinterpret_cast<uintptr_t>(a.A) & 15) == 0);
 }
 
-int linear_stream_f32(const LinearArgs& a, cudaStream_t st) {
-    if (a.M == 1) return launch_stream<0, false>(a, st);
-    if (a.M <= 8) return a.A16 != nullptr ? launch_stream<1, true>(a, st) : launch_stream<1, false>(a, st);
-    return a.A16 != nullptr ? launch_stream<2, true>(a, st) : launch_stream<2, false>(a, st);
+template <bool GLU>
+static int stream_rows(const LinearArgs& a, cudaStream_t st) {
+    if (a.M == 1) return launch_stream<0, false, GLU>(a, st);
+    if (a.M <= 8) return a.A16 != nullptr ? launch_stream<1, true, GLU>(a, st) : launch_stream<1, false, GLU>(a, st);
+    return a.A16 != nullptr ? launch_stream<2, true, GLU>(a, st) : launch_stream<2, false, GLU>(a, st);
 }
+
+int linear_stream_f32(const LinearArgs& a, cudaStream_t st) { return a.gated ? stream_rows<true>(a, st) : stream_rows<false>(a, st); }
 
 }  // namespace b2

@@ -710,6 +710,15 @@ static int seq_feed_forward(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, c
         const int ff = d.ff, ffl = (2 * ff + 7) / 8 * 8;
         GluAct act = clamp_glu;
         if (d.ff_kind == B2_FF_GELU_GLU) { act = GluAct{}; act.kind = GLU_GELU_TANH; }
+        LinearArgs up;   // a handful of rows: both products and the unit in one stream of the weights
+        up.A = h; up.lda = width; up.A16 = in.h16; up.W = W.up_w.p; up.ldw = width; up.w_dtype = s.w_dtype; up.out = s.ffa.as<float>(); up.ld_out = ff;
+        up.M = R; up.N = ff; up.K = width; up.round_a = s.d.compute == B2_COMPUTE_BF16; up.gated = 1; up.glu = act;
+        if ((R == 1 || tc_enabled()) && linear_streams(up)) {
+            if (R > 1 && lin.tensor_cores(width, ff, target, width, R)) up.out16 = s.ff.p;   // bf16 rows for the second product
+            B2_TRY(linear_stream_f32(up, st));
+            return lin(up.out16 != nullptr ? nullptr : s.ffa.as<float>(), ff, W.down_w, width, ff, target, width, R, LIN_NONE, alpha, accumulate, nullptr, 0, nullptr,
+                       up.out16);
+        }
         if (R == 1) {
             GroupedLinearArgs gs;
             gs.A = h; gs.lda = width; gs.a_div = 1; gs.W = W.up_w.p; gs.ldw = width; gs.w_group_stride = 0; gs.w_dtype = s.w_dtype;

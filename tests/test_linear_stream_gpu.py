@@ -32,7 +32,7 @@ def residuals(cfg, w, n, steps):
     return out
 
 
-@pytest.mark.parametrize("width,ff", [(64, 24), (72, 136), (136, 40), (264, 1032), (1160, 272)])
+@pytest.mark.parametrize("width,ff", [(64, 24), (64, 100), (72, 136), (136, 40), (264, 1032), (1160, 272)])
 @pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 15, 16, 17])
 def test_streamed_weights_equal_the_fma_kernels(width, ff, n, monkeypatch):
     cfg = config([dict(win(5, 1, 24, 40, None, None, 8), mlp={"kind": "dense", "ff": ff, "limit": 7.0})], width=width, vocab=101)
