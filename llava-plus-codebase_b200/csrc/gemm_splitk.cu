@@ -212,8 +212,9 @@ int splitk_act(const GemmArgs& g, int S, const KsEpi& ep, cudaStream_t st) {
 }  // namespace
 
 int gemm_bf16_splitk(const GemmArgs& g, int bn, int S, cudaStream_t st) {
-    B2_CHECK_ARG((bn == 64 || bn == 128) && (S == 2 || S == 4) && S <= (g.K + KS_BK - 1) / KS_BK && g.act != ACT_SWIGLU && g.act != ACT_ROPE_QKV && g.tile_group == nullptr,
-                 "gemm(split K): bad plan bn=%d S=%d K=%d", bn, S, g.K);
+    B2_CHECK_ARG((bn == 64 || bn == 128) && (S == 2 || S == 4) && S <= (g.K + KS_BK - 1) / KS_BK && g.tile_group == nullptr, "gemm(split K): bad plan bn=%d S=%d K=%d", bn, S, g.K);
+    // (a gated unit's output has half the product's columns: without its epilogue here, the plain one would write past every row)
+    B2_CHECK_ARG(g.act == ACT_NONE || g.act == ACT_QUICK_GELU || g.act == ACT_GELU_ERF, "gemm(split K): activation %d has no epilogue here", g.act);
     KsEpi ep;
     ep.a_bytes = gemm_a_rows(g.M) * KS_BK * 2;
     ep.bias = reinterpret_cast<const __nv_bfloat16*>(g.bias); ep.residual = reinterpret_cast<const __nv_bfloat16*>(g.residual);

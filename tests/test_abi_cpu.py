@@ -76,3 +76,14 @@ def test_stream_k_plan_helpers_are_host_only():
     assert lib.b2_op_gemm_skinny_workspace_bytes(0, 128, 64) == -1
     assert lib.b2_op_gemm_skinny_workspace_bytes(129, 128, 64) == -1
     assert lib.b2_op_gemm_skinny_counter_bytes(0) == -1
+
+
+@pytest.mark.parametrize("plan", [2064, 2128, 4064, 4128])
+def test_gated_unit_refuses_plans_that_cut_k(plan):
+    """The kernel that cuts K over a cluster has no gated epilogue: the plain one would write 2 ff columns into rows of ff. The host
+    refuses the plan before it looks at any of the operands (no GPU, and the addresses below are never read)."""
+    from llava import _b2
+
+    lib, at = _b2.load_library(), 1 << 20
+    r = lib.b2_op_gemm_glu(at, 512, at, 512, at, 64, 32, 64, 512, 1.0, 0.0, 0.0, 0, None, 1, plan, None)
+    assert r == -1 and "no epilogue" in _b2.last_error()
