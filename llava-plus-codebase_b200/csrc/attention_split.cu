@@ -135,7 +135,6 @@ __device__ __noinline__ float sigmoid_times(float gate, float v) { return v / (1
 template <int DKS, int DVS, int KT, bool EXTRA>   // EXTRA: soft-cap or distance bias
 __global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                                                                    const __grid_constant__ SplitParams p) {
-    pdl_enter();
     using Cfg = SplitCfg<DKS, DVS, KT>;
     constexpr int KH = KT / 2, CH = 32 * DVS;   // keys of a tile and value columns per softmax thread
     extern __shared__ uint8_t sp_raw[];
@@ -150,17 +149,6 @@ __global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_
 
     const BiasAttnArgs& a = p.a;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, HG = p.HG;
-    // the query tiles with the most keys go first
-    const int nq = (a.rows + p.QT - 1) / p.QT, qt = nq - 1 - (int)(blockIdx.x / a.G), g = blockIdx.x % a.G;
-    const int gv = a.Gv > 0 ? g % a.Gv : g;
-    const int r0 = qt * p.QT, nrows = min(p.QT, a.rows - r0), P = nrows * HG;
-    const int minpos = a.row_pos[r0], maxpos = a.row_pos[r0 + nrows - 1];   // consecutive positions of one slot
-    const int first = split_first(minpos, a.mask_kind, a.mask_size), maxfirst = split_first(maxpos, a.mask_kind, a.mask_size);
-    const int keep = a.mask_kind == MASK_WINDOW ? a.mask_keep : 0;
-    // visible keys: [0, nA) (kept first positions in front of the earliest window) and [first, maxpos], in tiles of KT
-    const int nA = min(keep, first), tilesA = (nA + KT - 1) / KT, T = tilesA + (maxpos + 1 - first + KT - 1) / KT;
-    auto tile_start = [&](int t) { return t < tilesA ? t * KT : first + (t - tilesA) * KT; };
-
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tm_k);
         tma_prefetch_desc(&tm_v);
@@ -172,6 +160,19 @@ __global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_
     __syncthreads();
     tc_fence_after();
     const uint32_t tm = *tmem_slot;
+    pdl_trigger_small();   // (behind the allocation: see tmem_alloc)
+    pdl_wait();
+
+    // the query tiles with the most keys go first
+    const int nq = (a.rows + p.QT - 1) / p.QT, qt = nq - 1 - (int)(blockIdx.x / a.G), g = blockIdx.x % a.G;
+    const int gv = a.Gv > 0 ? g % a.Gv : g;
+    const int r0 = qt * p.QT, nrows = min(p.QT, a.rows - r0), P = nrows * HG;
+    const int minpos = a.row_pos[r0], maxpos = a.row_pos[r0 + nrows - 1];   // consecutive positions of one slot
+    const int first = split_first(minpos, a.mask_kind, a.mask_size), maxfirst = split_first(maxpos, a.mask_kind, a.mask_size);
+    const int keep = a.mask_kind == MASK_WINDOW ? a.mask_keep : 0;
+    // visible keys: [0, nA) (kept first positions in front of the earliest window) and [first, maxpos], in tiles of KT
+    const int nA = min(keep, first), tilesA = (nA + KT - 1) / KT, T = tilesA + (maxpos + 1 - first + KT - 1) / KT;
+    auto tile_start = [&](int t) { return t < tilesA ? t * KT : first + (t - tilesA) * KT; };
 
     auto load_tile = [&](const CUtensorMap* map, uint8_t* dst, uint64_t* bar, int t, int head, int slabs, int bytes) {
         const int j0 = tile_start(t), i0 = j0 < p.nA0 ? j0 : j0 - p.first0 + p.nA0;

@@ -118,7 +118,6 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // causal: the query tiles with the most keys go first
     const int q0 = (CAUSAL ? (int)(gridDim.z - 1 - blockIdx.z) : (int)blockIdx.z) * TC_BM;
     const int head = blockIdx.x, b = blockIdx.y;
-    pdl_trigger();
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tm_q);
         tma_prefetch_desc(&tm_k);
@@ -141,6 +140,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const uint32_t tm = *tmem_slot;
+    pdl_trigger();  // (behind the allocation: see tmem_alloc)
     pdl_wait();  // q/k/v (and seq_lens) are outputs of upstream kernels (programmatic dependent launch)
     const int len = p.seq_lens != nullptr ? p.seq_lens[b] : p.S;
     const int kv_end = CAUSAL ? min(len, q0 + TC_BM) : len;

@@ -246,6 +246,8 @@ constexpr uint64_t kEvictLast = 0x14F0000000000000ull;
 // ----------------------------------------------------------------------------------------------
 // tcgen05 / TMEM
 // ----------------------------------------------------------------------------------------------
+// A kernel that allocates TMEM lets its dependents start (pdl_trigger) only behind the allocation and the barrier after it. A dependent that
+// has TMEM of its own holds it until this kernel is done; if it could be resident before this kernel's CTAs have theirs, each would wait for the other.
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_dst, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(smem_dst)),

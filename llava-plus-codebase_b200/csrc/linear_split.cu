@@ -52,7 +52,6 @@ __device__ __noinline__ float lx_act(float v, int act) { return epi_post_act(v, 
 
 template <int BN>
 __global__ void __launch_bounds__(LX_THREADS, 1) linear_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w, LinearArgs a) {
-    pdl_enter();
     using Cfg = LxCfg<BN>;
     constexpr int CH = BN / 2;   // columns per epilogue thread
     extern __shared__ uint8_t lx_raw[];
@@ -76,6 +75,8 @@ __global__ void __launch_bounds__(LX_THREADS, 1) linear_split_kernel(const __gri
     __syncthreads();
     tc_fence_after();
     const uint32_t tm = *tmem_slot;
+    pdl_trigger_small();   // (behind the allocation: see tmem_alloc)
+    pdl_wait();
 
     if (warp == 0) {
         if (lane == 0) {
