@@ -144,7 +144,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     pdl_wait();  // q/k/v (and seq_lens) are outputs of upstream kernels (programmatic dependent launch)
     const int len = p.seq_lens != nullptr ? p.seq_lens[b] : p.S;
     const int kv_end = CAUSAL ? min(len, q0 + TC_BM) : len;
-    const int T = (kv_end + TC_BN - 1) / TC_BN;  // >= 1 (len >= 1)
+    const int T = (max(kv_end, 0) + TC_BN - 1) / TC_BN;  // 0: a request without keys, whose rows are zeros
 
     if (warp == 0) {
         if (lane == 0) {
@@ -274,8 +274,8 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             __syncwarp();
             if (lane == 0) mbar_arrive(&p_full[t & 1]);
         }
-        // ---- epilogue: O / l ----
-        mbar_wait(o_last, 0);
+        // ---- epilogue: O / l (no key: no product to wait for, and nothing of O to read) ----
+        if (T > 0) mbar_wait(o_last, 0);
         tc_fence_after();
         const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
         __nv_bfloat16* orow = p.o + b * p.o_bs + (int64_t)qrow * p.o_ts + head * p.o_hs;
@@ -285,6 +285,10 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             __syncwarp();
             tmem_ld_32x32(lanes + TM_O + c * 32, v);
             tmem_ld_wait();
+            if (T == 0) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) v[i] = 0u;
+            }
             if (qrow < p.S) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {

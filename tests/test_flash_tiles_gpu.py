@@ -47,6 +47,28 @@ def test_tile_edges(S, D, causal, growing):
             assert float((o[b, :n].double() - ref[b, :n]).abs().max()) <= tol
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [0, 1])
+def test_requests_without_keys(D, causal):
+    """A length of 0 (or below) leaves its rows zeros and the other requests of the call as they are."""
+    from llava import _b2
+
+    lib, P = _b2.init(0), _b2.ptr
+    B, S, H = 5, 130, 2
+    g = torch.Generator(device="cuda").manual_seed(D)
+    q, k, v = (torch.randn(B, S, H, D, device="cuda", generator=g).bfloat16() for _ in range(3))
+    lens = torch.tensor([70, 0, 130, -3, 1], dtype=torch.int32, device="cuda")
+    o = torch.full_like(q, 7.0)
+    _b2.check(lib.b2_op_flash_attn(P(q), P(k), P(v), P(o), P(lens), B, S, H, D, causal, 1 / math.sqrt(D), _b2.stream_ptr()))
+    for b, n in enumerate(lens.tolist()):
+        if n <= 0:
+            assert bool((o[b] == 0).all())
+        else:
+            ref = attend(q[b:b + 1], k[b:b + 1], v[b:b + 1], lens[b:b + 1], causal, 1 / math.sqrt(D))[0]
+            rows = n if causal else S
+            assert float((o[b, :rows].double() - ref[:rows]).abs().max()) <= 2 ** -8 * float(v[b].abs().max()) + 2 ** -8
+
+
 @pytest.mark.parametrize("D,causal,S,B,H", [(128, 1, 704, 8, 32), (128, 0, 321, 8, 32), (64, 0, 577, 16, 16), (64, 1, 704, 8, 32), (128, 1, 128, 64, 32)])
 def test_full_grids(D, causal, S, B, H):
     """Several waves of blocks, two on each multiprocessor: products are slow enough here for the softmax of the last tile to end before the product
