@@ -79,6 +79,7 @@ struct SeqModel {
     DevBuf x, proj, act, y, gated, mixout, mixes, rp, wl1, wlog, ff, xn, tok, want;
     DevBuf lin_parts;                  // fp32 compute: bf16 parts of a product's operands (linear_split.cu)
     DevBuf scan_chunks;                // chunk states of a long prompt's recurrences (recurrent.cu)
+    DevBuf attn_parts;                 // bf16 parts of the keys and values that a prompt portion sees (attention_split.cu); grows with the longest cache
     DevBuf a16;                        // bf16 copy of a GEMM's A operand (tensor-core path of the bf16 compute mode)
     int a16_w = 0;
     DevBuf segs, row_slot, row_pos;
@@ -100,7 +101,6 @@ struct SeqState {
     DevBuf last_tok;                   // int32 [slots]: the token in front of the next one (hashed bigram embedding)
     DevBuf kmat, vmat;                 // latent attention, long prompt portions: per-head keys / values of one slot's positions [Smax][heads*size]
     int kmat_ld = 0, vmat_ld = 0;
-    DevBuf parts;                      // bf16 parts of the keys and values that a prompt portion sees (attention_split.cu)
     DevBuf attn_partial;
     int nsplit_max = 1;
 };
@@ -110,9 +110,21 @@ namespace {
 const size_t F4 = sizeof(float);
 size_t esz(int dt) { return dt == DT_F32 ? 4 : 2; }
 
-// scratch that a faster path wants and that nothing depends on: a device without room for it runs the other path
+// Scratch that a faster path wants and that nothing depends on: a device without room for it runs the other path. It is taken behind everything
+// that a model or a cache cannot do without, once per model (never per cache), and only where it leaves the device SPARE_RESERVE for what is created
+// after it. A buffer that is too small is kept if there is no room for a larger one.
+constexpr size_t SPARE_RESERVE = (size_t)1 << 30;
 void alloc_spare(DevBuf& b, size_t bytes) {
-    if (b.alloc(bytes) != 0) cudaGetLastError();
+    size_t free_bytes = 0, total = 0;
+    if (bytes <= b.bytes) return;
+    DevBuf n;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || free_bytes < bytes + SPARE_RESERVE || n.alloc(bytes) != 0) {
+        cudaGetLastError();
+        return;
+    }
+    if (b.p != nullptr) cudaDeviceSynchronize();   // calls in flight may use the old one
+    b.free();
+    b = n;
 }
 
 int64_t numel(const int64_t* shape, int ndim) {
@@ -261,10 +273,10 @@ static void mask_of(const b2_seq_layer_desc& d, BiasAttnArgs& aa) {
 }
 
 // a prompt portion (nseg == 1): where it lies, and the scratch with which its attention runs on the tensor cores
-static void portion_of(const SeqState& state, int nseg, int slot, int ctx_end, BiasAttnArgs& aa) {
+static void portion_of(const SeqModel& s, int nseg, int slot, int ctx_end, BiasAttnArgs& aa) {
     if (nseg != 1 || ctx_end < aa.rows) return;
     aa.slot = slot; aa.key_end = ctx_end;
-    aa.parts = state.parts.p; aa.parts_bytes = state.parts.bytes;
+    aa.parts = s.attn_parts.p; aa.parts_bytes = s.attn_parts.bytes;
 }
 
 // Attention over a low-rank latent. S: the run's own state (rotation table); KS: the state whose cache rows it reads (its own,
@@ -331,7 +343,7 @@ static int latent_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeight
         aa.kv_row_stride = state.kmat_ld; aa.kv_row_stride_v = state.vmat_ld;
         aa.out = y; aa.ldo = L.pv;
         aa.G = H; aa.dk = qh; aa.dv = dv; aa.nsplit = 1;
-        portion_of(state, nseg, slot, ctx_end, aa);
+        portion_of(s, nseg, slot, ctx_end, aa);
         B2_TRY(attn_bias_f32(aa, st));
     } else {
         // absorbed form: q_h -> W_uk_h^T q_h lives in the latent space (the rotated part rides behind it), so scores and values
@@ -435,7 +447,7 @@ static int gqa_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeights& 
     if (chan_in_attn) { aa.chan_gate = gates; aa.ldg = L.lproj_ld; }
     const bool out16 = maps == 1 && !d.ga_rot_values && lin.tensor_cores(width, L.ng, target, width, R);
     if (out16) aa.out16 = s.a16.p;
-    portion_of(state, nseg, slot, ctx_end, aa);
+    portion_of(s, nseg, slot, ctx_end, aa);
     B2_TRY(attn_bias_f32(aa, st));
     if (out16) return lin(nullptr, 0, W.o_w, width, L.ng, target, width, R, LIN_NONE, alpha, accumulate, nullptr, 0, nullptr, s.a16.p);
     const float* yo = s.y.as<float>();
@@ -983,7 +995,7 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
             aa.tile_rows = max_n;
             if (aa.nsplit > state.nsplit_max) aa.nsplit = state.nsplit_max;
             aa.partial = state.attn_partial.as<float>();
-            portion_of(state, nseg, slot, ctx_end, aa);
+            portion_of(s, nseg, slot, ctx_end, aa);
             B2_TRY(attn_prepare_f32(aa, st));
             B2_TRY(attn_bias_f32(aa, st));
             B2_TRY(sigmoid_gate_f32(s.y.as<float>(), L.ng, proj + L.nq + L.nk + L.nv, L.lproj_ld, s.gated.as<float>(), L.ng, R, L.ng, st));
@@ -1565,15 +1577,6 @@ int seq_finalize(b2_model* m) {
     if (s.d.loop_mix) B2_TRY(s.cat.alloc(R * 2 * width * F4));
     if (s.d.block == B2_BLOCK_PARALLEL2) B2_TRY(s.h2.alloc(R * width * F4));
     if (den_w > 0) B2_TRY(s.den.alloc(R * den_w * F4));
-    size_t chunk_floats = 0;
-    for (const SeqLayerInfo& L : s.layers) {
-        const b2_seq_layer_desc& d = L.d;
-        if (d.type == B2_MIXER_MAMBA2) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.m_heads, d.m_state, d.m_vdim));
-        else if (d.type == B2_MIXER_PARALLEL) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.r_heads, d.r_dim, d.r_dim));
-        else if (d.type == B2_MIXER_HGRN2) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.g_heads, d.g_dim, d.g_vdim));
-        else if (d.type == B2_MIXER_GLA) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.gl_heads, d.gl_dim, d.gl_vdim));
-    }
-    alloc_spare(s.scan_chunks, chunk_floats * F4);
     if (s.d.compute == B2_COMPUTE_BF16) {
         if (dyt || s.d.block == B2_BLOCK_PARALLEL_RMS || s.d.block == B2_BLOCK_PARALLEL2) B2_TRY(s.h1_16.alloc(R * width * 2));
         if (dyt) B2_TRY(s.h2_16.alloc(R * width * 2));
@@ -1614,7 +1617,6 @@ int seq_finalize(b2_model* m) {
             kmax = std::max(kmax, std::max(std::max(std::max(L.inner, L.ng), std::max(L.rn, L.d.ff)), std::max(std::max(L.pv, std::max(L.lrow, L.d.la_q_rank)), std::max(L.d.la_dim, L.d.moe_shared_ff))));
         s.a16_w = (kmax + 7) / 8 * 8;
         if (s.d.compute == B2_COMPUTE_BF16) B2_TRY(s.a16.alloc(R * s.a16_w * 2));
-        else alloc_spare(s.lin_parts, linear_split_bytes((int)R, kmax) + ((size_t)64 << 20));   // (with room for the weights in blocks of rows)
     }
     B2_TRY(s.tok.alloc(R * 4));
     B2_TRY(s.want.alloc(R * 4));
@@ -1622,6 +1624,17 @@ int seq_finalize(b2_model* m) {
     B2_TRY(s.row_slot.alloc(R * 4));
     B2_TRY(s.row_pos.alloc(R * 4));
     B2_TRY(m->logits.alloc((size_t)s.d.max_batch * s.d.vocab * 4));
+    // (nothing that the model needs is allocated behind these)
+    size_t chunk_floats = 0;
+    for (const SeqLayerInfo& L : s.layers) {
+        const b2_seq_layer_desc& d = L.d;
+        if (d.type == B2_MIXER_MAMBA2) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.m_heads, d.m_state, d.m_vdim));
+        else if (d.type == B2_MIXER_PARALLEL) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.r_heads, d.r_dim, d.r_dim));
+        else if (d.type == B2_MIXER_HGRN2) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.g_heads, d.g_dim, d.g_vdim));
+        else if (d.type == B2_MIXER_GLA) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.gl_heads, d.gl_dim, d.gl_vdim));
+    }
+    alloc_spare(s.scan_chunks, chunk_floats * F4);
+    if (s.d.compute != B2_COMPUTE_BF16) alloc_spare(s.lin_parts, linear_split_bytes((int)R, s.a16_w) + ((size_t)64 << 20));   // (with room for the weights in blocks of rows)
     return 0;
 }
 
@@ -1640,7 +1653,7 @@ void seq_model_free(b2_model* m) {
     DevBuf* bs[] = {&s.embed, &s.head, &s.final_w, &s.final_b, &s.x, &s.proj, &s.act, &s.y, &s.gated, &s.mixout, &s.mixes, &s.rp, &s.wl1, &s.wlog,
                     &s.ff, &s.xn, &s.tok, &s.want, &s.segs, &s.row_slot, &s.row_pos, &s.a16, &s.bigram, &s.loop_step, &s.x0, &s.qabs, &s.olat, &s.ffa,
                     &s.rlogit, &s.moe_idx, &s.moe_w, &s.moe_pos, &s.moe_src, &s.moe_tile, &s.moe_h, &s.moe_a, &s.moe_y, &s.moe_a16, &s.zero_idx, &s.hin, &s.final_a, &s.loop_in, &s.cat,
-                    &s.h2, &s.h1_16, &s.h2_16, &s.f16, &s.den, &s.embed_nw, &s.scan_chunks, &s.lin_parts};
+                    &s.h2, &s.h1_16, &s.h2_16, &s.f16, &s.den, &s.embed_nw, &s.scan_chunks, &s.lin_parts, &s.attn_parts};
     for (DevBuf* b : bs) b->free();
     delete m->seq;
     m->seq = nullptr;
@@ -1778,7 +1791,9 @@ int seq_kv_alloc(b2_kv* kv) {
         B2_TRY(kv->seq->kmat.alloc(Smax * kw * F4));
         B2_TRY(kv->seq->vmat.alloc(Smax * vw * F4));
     }
-    {   // bf16 parts of what a prompt portion sees, at most PARTS_MAX: a portion that sees more keys stays on the fp32 pipe
+    kv->seq->nsplit_max = 64;
+    B2_TRY(kv->seq->attn_partial.alloc((size_t)8 * maxH * kv->seq->nsplit_max * (maxdv + 2) * F4));
+    if (Smax >= (size_t)ATTN_SPLIT_MIN_KEYS) {   // parts of what a prompt portion sees, at most PARTS_MAX: a portion that sees more keys stays on the fp32 pipe
         size_t per_key = 0;
         for (const SeqLayerInfo& L : s.layers) {
             const b2_seq_layer_desc& d = L.d;
@@ -1787,10 +1802,8 @@ int seq_kv_alloc(b2_kv* kv) {
             else if (d.type == B2_MIXER_PARALLEL) per_key = std::max(per_key, attn_split_bytes_per_key(d.a_kv_heads, d.a_kv_heads, d.a_dim, d.a_vdim));
         }
         const size_t PARTS_MAX = (size_t)256 << 20;
-        alloc_spare(kv->seq->parts, std::min(Smax * per_key, PARTS_MAX));
+        alloc_spare(m->seq->attn_parts, std::min(Smax * per_key, PARTS_MAX));
     }
-    kv->seq->nsplit_max = 64;
-    B2_TRY(kv->seq->attn_partial.alloc((size_t)8 * maxH * kv->seq->nsplit_max * (maxdv + 2) * F4));
     return 0;
 }
 
@@ -1803,7 +1816,6 @@ void seq_kv_free(b2_kv* kv) {
     kv->seq->last_tok.free();
     kv->seq->kmat.free();
     kv->seq->vmat.free();
-    kv->seq->parts.free();
     kv->seq->attn_partial.free();
     delete kv->seq;
     kv->seq = nullptr;
