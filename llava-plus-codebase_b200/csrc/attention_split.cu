@@ -1,7 +1,8 @@
 // fp32 attention of a prompt portion on the tensor cores (sm_100a): the same softmax attention over an fp32 cache as
 // attn_tile_kernel (attention_bias.cu) with every fp32 operand carried as THREE bf16 parts.
 //
-// x = hi + mid + lo (bf16 each, round to nearest: 24 significant bits, fp32's exponent range, so no scaling and no loss), and a product
+// x = hi + mid + lo (bf16 each, round to nearest: 24 significant bits, fp32's exponent range, so no scaling and no loss; what has no parts is
+// done over in plain fp32, attn_plain below), and a product
 // of two such operands is the six products hi*hi, hi*mid, mid*hi, hi*lo, lo*hi, mid*mid on tcgen05 (kind::f16) with fp32 accumulation;
 // the three that are left out lie below 2^-25 of |q| |k|. The tensor core TRUNCATES its fp32 sum after every step of 16 (measured: sums of K
 // bf16 products of random sign are off by 1.2e-7 of the result at K = 128 and 1.0e-6 at K = 1024, a serial fp32 chain by 0.7e-7 and
@@ -131,6 +132,65 @@ struct SplitCfg {
 // instructions: 220 us against 129 us for 2048 rows of 16 heads of 128 with a window of 1024
 __device__ __noinline__ float soft_cap(float v, float cap) { return cap * tanhf(v / cap); }
 __device__ __noinline__ float sigmoid_times(float gate, float v) { return v / (1.f + expf(-gate)); }
+
+__device__ __forceinline__ float plain_score(const BiasAttnArgs& a, const float* q, const float* k, int head, int dist) {
+    float s = 0.f;
+    for (int d = 0; d < a.dk; ++d) s = fmaf(q[d], k[d], s);
+    s *= a.scale;
+    if (a.softcap > 0.f) s = a.softcap * tanhf(s / a.softcap);
+    if (a.rel != nullptr) s += a.rel[(size_t)a.bucket_of[dist] * a.H + head];
+    return s;
+}
+// Value columns [d0, d1) of one (row, head) in plain fp32, for a row that saw an operand without parts (split.cuh): maximum, denominator, then 16
+// columns at a time. Keys that the row does not see have no part in it. Once the denominator, or all 16 columns, are NaN they stay so.
+__device__ __noinline__ void attn_plain(const SplitParams& p, int row, int head, int pos, int d0, int d1) {
+    const BiasAttnArgs& a = p.a;
+    const int g = head / p.HG, Gv = a.Gv > 0 ? a.Gv : a.G, gv = g % Gv;
+    const bool mat = a.kv_row_stride > 0;
+    const float* K = mat ? a.kcache + (size_t)g * a.dk : a.kcache + ((size_t)a.slot * a.G + g) * a.Smax * a.dk;
+    const float* V = mat ? a.vcache + (size_t)gv * a.dv : a.vcache + ((size_t)a.slot * Gv + gv) * a.Smax * a.dv;
+    const size_t ks = mat ? (size_t)a.kv_row_stride : (size_t)a.dk, vs = mat ? (size_t)a.kv_row_stride_v : (size_t)a.dv;
+    const float* q = a.q + (size_t)row * a.ldq + (size_t)head * a.dk;
+    const int first = split_first(pos, a.mask_kind, a.mask_size), kept = min(a.mask_kind == MASK_WINDOW ? a.mask_keep : 0, first);
+    auto next = [&](int j) { return j + 1 == kept ? first : j + 1; };   // visible keys: [0, kept) and [first, pos]
+    const int start = kept > 0 ? 0 : first;
+    float m = -INFINITY, l = 0.f;
+    for (int j = start; j <= pos; j = next(j)) m = fmaxf(m, plain_score(a, q, K + j * ks, head, pos - j));
+    const float m_use = m == -INFINITY ? 0.f : m;
+    for (int j = start; j <= pos && l == l; j = next(j)) l += expf(plain_score(a, q, K + j * ks, head, pos - j) - m_use);
+    float inv = 1.f / l;
+    if (a.sink != nullptr || a.sink_fixed) {
+        const float sk = a.sink != nullptr ? a.sink[head] : a.sink_value, mf = fmaxf(m, sk), c0 = expf(m - mf);
+        inv = c0 / fmaf(l, c0, expf(sk - mf));
+    }
+    if (a.head_gate != nullptr) inv /= 1.f + expf(-a.head_gate[(size_t)row * a.ldg + head]);
+    const float* cg = a.chan_gate != nullptr ? a.chan_gate + (size_t)row * a.ldg + (size_t)head * a.dv : nullptr;
+    const size_t at = (size_t)row * a.ldo + (size_t)head * a.dv;
+    for (int d = d0; d < d1; d += 16) {
+        float o[16];
+#pragma unroll
+        for (int c = 0; c < 16; ++c) o[c] = 0.f;
+        bool live = inv == inv;
+        for (int j = start; j <= pos && live; j = next(j)) {
+            const float w = expf(plain_score(a, q, K + j * ks, head, pos - j) - m_use);
+            live = false;
+#pragma unroll
+            for (int c = 0; c < 16; ++c)
+                if (d + c < d1) {
+                    o[c] = fmaf(w, V[j * vs + d + c], o[c]);
+                    live |= o[c] == o[c];
+                }
+        }
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+            if (d + c >= d1) continue;
+            float y = o[c] * inv;
+            if (cg != nullptr) y = sigmoid_times(cg[d + c], y);
+            if (a.out16 != nullptr) reinterpret_cast<__nv_bfloat16*>(a.out16)[at + d + c] = __float2bfloat16_rn(y);
+            else a.out[at + d + c] = y;
+        }
+    }
+}
 
 template <int DKS, int DVS, int KT, bool EXTRA>   // EXTRA: soft-cap or distance bias
 __global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -364,7 +424,12 @@ __global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_
         red[half * SP_M + pair] = l;
         softmax_sync();
         l += red[(half ^ 1) * SP_M + pair];
-        if (live) {
+        bool plain = l != l;
+#pragma unroll
+        for (int c = 0; c < CH; ++c) plain |= o[c] != o[c];
+        if (live && plain) {
+            attn_plain(p, row, head, pos, half * CH, min((half + 1) * CH, a.dv));
+        } else if (live) {
             float inv = 1.f / l;
             if (a.sink != nullptr || a.sink_fixed) {   // the sink joins the denominator once, under the common maximum
                 const float sk = a.sink != nullptr ? a.sink[head] : a.sink_value, mf = fmaxf(m, sk), c0 = expf(m - mf);

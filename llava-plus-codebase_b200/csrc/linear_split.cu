@@ -50,8 +50,20 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
 
 __device__ __noinline__ float lx_act(float v, int act) { return epi_post_act(v, act); }
 
+// cols outputs of row m from column c0 on in plain fp32, for a row with an operand that has no parts (split.cuh). A sum that has become NaN stays one.
+__device__ __noinline__ void lx_plain(const LinearArgs& a, int m, int c0, int cols) {
+    const float* x = a.A + (size_t)m * a.lda;
+    for (int n = c0; n < min(c0 + cols, a.N); ++n) {
+        const float* w = reinterpret_cast<const float*>(a.W) + (size_t)n * a.ldw;
+        float acc = 0.f;
+        for (int k = 0; k < a.K && acc == acc; ++k) acc = fmaf(x[k], w[k], acc);
+        linear_store(a.out + (size_t)m * a.ld_out + n, acc, a.bias, n, a.act, a.alpha, a.accumulate);
+    }
+}
+
 template <int BN>
-__global__ void __launch_bounds__(LX_THREADS, 1) linear_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w, LinearArgs a) {
+__global__ void __launch_bounds__(LX_THREADS, 1) linear_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
+                                                                      const __grid_constant__ LinearArgs a) {
     using Cfg = LxCfg<BN>;
     constexpr int CH = BN / 2;   // columns per epilogue thread
     extern __shared__ uint8_t lx_raw[];
@@ -135,7 +147,12 @@ __global__ void __launch_bounds__(LX_THREADS, 1) linear_split_kernel(const __gri
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[b & 1]);
         }
-        if (m < a.M) {
+        bool plain = false;
+#pragma unroll
+        for (int i = 0; i < CH; ++i) plain |= acc[i] != acc[i];
+        if (m < a.M && plain) {
+            lx_plain(a, m, n0 + half * CH, CH);
+        } else if (m < a.M) {
             const int c0 = n0 + half * CH;
             float* o = a.out + (size_t)m * a.ld_out + c0;
             const bool vec = a.ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
@@ -209,7 +226,8 @@ int linear_split_f32(const LinearArgs& a, cudaStream_t st) {
         b.N = std::min(step, a.N - n0);
         b.out = a.out + n0;
         if (a.bias != nullptr) b.bias = a.bias + n0;
-        B2_TRY(split_rows(reinterpret_cast<const float*>(a.W) + (size_t)n0 * a.ldw, a.ldw, b.N, a.K, pitch, pw, st));
+        b.W = reinterpret_cast<const float*>(a.W) + (size_t)n0 * a.ldw;
+        B2_TRY(split_rows(reinterpret_cast<const float*>(b.W), a.ldw, b.N, a.K, pitch, pw, st));
         const int num_m = (b.M + LX_M - 1) / LX_M;
         // tiles of 128 columns read A half as often; narrower ones where they would leave SMs idle
         const bool wide = num_m * ((b.N + 127) / 128) > num_sms() / 2;

@@ -5,7 +5,11 @@
 
 namespace b2 {
 
-// two values -> their three bf16 parts, packed (first value in the low half)
+// two values -> their three bf16 parts, packed (first value in the low half). A value that bf16 does not hold (an infinity, a NaN, a magnitude of
+// 2^128 (1 - 2^-9) and more, which rounds to infinity) has NaN among its parts, and NaN is then what every sum of products that it enters comes
+// to, whatever the other operand. So the kernels take a sum that is NaN for one they cannot do, and do it over in plain fp32 from the
+// operands themselves (linear_split.cu, attention_split.cu): infinite results, scores of -inf and large finite values come out as they
+// would from fp32 products.
 __device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
     hi = pack_bf16(a, b);
     const float a1 = a - bf16_lo(hi), b1 = b - bf16_hi(hi);
