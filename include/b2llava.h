@@ -390,7 +390,10 @@ int b2_op_gemm_glu(const void* A, int lda, const void* W, int ldw, void* out, in
 int b2_op_gemv(const void* x, int64_t ldx, const void* W, int ldw, const void* norm_gamma, float eps,
                const void* residual, int ld_res, void* out, int ld_out, int out_fp32, int B, int N, int K, int act,
                void* stream);
-/* decode Linear at batch 9..128 (swap-AB stream-K tcgen05 GEMM, csrc/gemm_skinny.cu): out[B,N] = x[B,K]·W[N,K]^T
+/* 1 where a bf16 decode step of `batch` requests (7..128) of a LLaMA of these widths runs its Linears on the stream-K GEMM below, 0: on the
+ * tile GEMMs. Host arithmetic only. */
+int b2_op_decode_stream_k(int hidden, int inter, int batch);
+/* decode Linear at batch 7..128 (swap-AB stream-K tcgen05 GEMM, csrc/gemm_skinny.cu): out[B,N] = x[B,K]·W[N,K]^T
  * (+ residual); act = B2_ACT_NONE | B2_ACT_SWIGLU (out [B,N/2], W rows block-64 interleaved). `workspace` (fp32,
  * >= b2_op_gemm_skinny_workspace_bytes) and `counters` (int32, >= b2_op_gemm_skinny_counter_bytes, zero-filled once
  * by the caller; the kernel leaves them zero) are caller-owned scratch. */

@@ -114,7 +114,7 @@ struct b2_kv {
     int max_batch = 0, max_seq = 0;
     DevBuf k, v;  // [L][B][H][Smax][D]
     DevBuf len_dev, tok, step_counter, out_tokens, attn_partial, attn_counters;
-    DevBuf sk_partial, sk_counters;  // stream-K workspace of the skinny decode GEMM (batch 9..128)
+    DevBuf sk_partial, sk_counters;  // stream-K workspace of the skinny decode GEMM (batch 7..128: fp8 steps, bf16 steps of wide models)
     std::vector<int32_t> len_host;
     int out_capacity = 0;  // steps
     // cached decode-step graph

@@ -1,4 +1,4 @@
-// Weight-streaming "skinny" GEMM for decode at batch 9..128 on sm_100a (swap-AB + stream-K):
+// Weight-streaming "skinny" GEMM for decode at batch 7..128 on sm_100a (swap-AB + stream-K), for fp8 weights and for wide bf16 models:
 //
 //     out[b, n] = sum_k x[b, k] * W[n, k]   (+ residual[b, n])          b < B <= 128,  n < N
 //     out[b, c] = silu(gate_c . x_b) * (up_c . x_b)                     (ACT_SWIGLU, W rows block-64 interleaved)

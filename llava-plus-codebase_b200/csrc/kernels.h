@@ -67,7 +67,7 @@ int gemm_bf16_2cta(const GemmArgs& g, cudaStream_t stream);
 // K cut over clusters of S CTAs, tiles of 128 x bn (gemm_splitk.cu; chosen by gemm_bf16, or bn_override == 1000 * S + bn)
 int gemm_bf16_splitk(const GemmArgs& g, int bn, int S, cudaStream_t stream);
 
-// ---- swap-AB stream-K GEMM for decode at batch 9..128 (gemm_skinny.cu) ------------------------------------
+// ---- swap-AB stream-K GEMM for decode at batch 7..128 (gemm_skinny.cu): fp8 steps, and bf16 steps of wide models (stream_k_step, model.cu) ----
 // out[B, N] = x[B,K] · W[N,K]^T (+ residual); ACT_SWIGLU: out[B, N/2] (W rows block-64 interleaved).
 struct SkinnyArgs {
     const void* x = nullptr; int ldx = 0;        // bf16 [B, K]

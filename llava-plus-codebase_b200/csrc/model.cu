@@ -111,14 +111,25 @@ int gemv(const void* x, int64_t ldx, const void* W, int ldw, const void* gamma, 
     return gemv_bf16(g, st);
 }
 
-// Decode Linear at batch 7..128: the tile GEMMs (a tile loads the rows of x that there are; K cut over clusters where few tiles would be left).
-// Measured against the stream-K GEMM over the kv-owned workspace, whose shared tiles cost it 8 us of fix-up (h = 4096, weights from memory; B = 9 /
-// 32 / 128): [B, 12288] 26.6 -> 22.9, 27.3 -> 22.8, 39.5 -> 24.1 us; [B, 4096] 14.6 -> 10.5, 15.4 -> 10.9, 35.3 -> 12.2; gate/up 36.5 -> 36.1, 37.6 ->
-// 36.6, 57.7 -> 37.7; down 22.3 -> 20.1, 23.2 -> 20.4, 43.2 -> 22.2; 32000 columns 51.4 -> 46.6, 52.3 -> 46.9, 76.9 -> 50.7. It stays for sizes that
-// the tile GEMMs refuse, and for fp8 weights.
+// The bf16 Linears of a decode step of 7..128 requests run on one of two kernels, all of a step on the same (launches of one kind start earlier
+// behind one another than a mix). The tile GEMMs load the rows of x that there are and cut K over clusters where few tiles would be left, but
+// multiply 128 rows whatever B is: their heat costs clock where a step is a long stream of weights (1650..1780 MHz under the power limit at widths of 5120
+// and more, against 1850..1965). The stream-K GEMM over the kv-owned workspace multiplies 32 / 64 / 128, spreads every matrix over all SMs, and pays
+// ~8 us of fix-up per launch. ms per step, tile GEMMs / stream-K, ~740 cached positions (width, weights of a layer, layers):
+//   4096, 405 MB, 32: B = 7 3.71 / 3.99, 16 4.41 / 4.66, 32 5.51 / 5.87, 64 7.74 / 9.20, 128 12.7 / 15.6     (2048, 3072: 15..31 % at B = 7..32)
+//   4608, 510 MB, 16: B = 7 2.25 / 2.28, 16 2.63 / 2.67, 32 3.30 / 3.33, 64 4.61 / 5.20
+//   5120, 634 MB, 40: B = 7 6.49 / 6.38, 16 7.81 / 7.70, 20 8.35 / 7.98, 32 9.78 / 9.46, 33 9.90 / 11.05, 64 13.0 / 14.3, 128 20.8 / 24.2
+//   6656, 1.07 GB, 12: B = 7 2.96 / 2.88, 32 4.09 / 3.95, 33 4.08 / 4.29, 64 5.47 / 5.65, 128 8.39 / 9.72
+//   8192, 1.62 GB, 12: B = 7 4.30 / 3.89, 32 5.72 / 5.27, 40 6.13 / 6.01, 64 7.53 / 7.37, 128 11.2 / 12.3
+// so up to 32 requests (x tiles of 32) the line lies between 510 and 634 MB, up to 64 between 1.07 and 1.62 GB.
+bool stream_k_step(int hidden, int inter, int B) {
+    const double mb = 2e-6 * hidden * (4.0 * hidden + 3.0 * inter);
+    return (B <= 32 && mb >= 570) || (B <= 64 && mb >= 1350);
+}
+// (stream_k: see above. Sizes that the tile GEMMs refuse, a vocabulary that is no multiple of 8, take the stream-K GEMM in any case.)
 int skinny(b2_kv* kv, const void* x, int ldx, const void* W, int ldw, const void* res, int ld_res, void* out, int ld_out,
-           int out_fp32, int B, int N, int K, int act, cudaStream_t st) {
-    if (N % 8 == 0 && ld_out % 8 == 0 && (res == nullptr || ld_res % 8 == 0)) return gemm(x, ldx, W, ldw, nullptr, res, ld_res, out, ld_out, out_fp32, B, N, K, act, st);
+           int out_fp32, int B, int N, int K, int act, bool stream_k, cudaStream_t st) {
+    if (!stream_k && N % 8 == 0 && ld_out % 8 == 0 && (res == nullptr || ld_res % 8 == 0)) return gemm(x, ldx, W, ldw, nullptr, res, ld_res, out, ld_out, out_fp32, B, N, K, act, st);
     SkinnyArgs g;
     g.x = x; g.ldx = ldx; g.W = W; g.ldw = ldw; g.residual = res; g.ld_res = ld_res;
     g.out = out; g.ld_out = ld_out; g.out_fp32 = out_fp32; g.B = B; g.N = N; g.K = K; g.act = act;
@@ -126,11 +137,6 @@ int skinny(b2_kv* kv, const void* x, int ldx, const void* W, int ldw, const void
     g.counters = kv->sk_counters.as<int>();
     return gemm_skinny_bf16(g, st);
 }
-// Batch 7..128. Measured ladder (7B, ms/step, profiles/r1e_config_sweep_*.jsonl): the stream-K GEMM path costs 4.13-4.19 for
-// every B <= 8 (7 kernels/layer, ~8 us of fixed cost per GEMM launch: profiles/r1e_decode_launch_shares_b4.txt), the GEMV
-// path (5 kernels/layer, RMSNorm fused) 3.63 at B=4 and 4.51 at B=8 -> crossover between 6 and 7. B2_DECODE_SKINNY=0
-// restores the earlier paths for A/B runs (GEMV kernels for B <= 8, tile GEMM with the batch padded to M=128 above),
-// B2_DECODE_SKINNY=3 lowers the threshold to 3.
 // fp8 variant: xq8 / xscale hold the quantised activations of this GEMM
 int skinny8(b2_model* m, b2_kv* kv, const void* W8, const float* w_scale, const void* res, int ld_res, void* out, int ld_out,
             int out_fp32, int B, int N, int K, int act, cudaStream_t st) {
@@ -142,6 +148,10 @@ int skinny8(b2_model* m, b2_kv* kv, const void* W8, const float* w_scale, const 
     g.w_scale = w_scale; g.x_scale = m->xscale.as<float>();
     return gemm_skinny_fp8(g, st);
 }
+// From 7 requests on (5 kernels a layer with RMSNorm fused below, on the GEMV kernels, 7 above). The line was drawn against the stream-K GEMM; the tile
+// GEMMs would pass the GEMV kernels from 3 on (width 4096, ms per step, GEMV / tiles: B = 3 3.64 / 3.34, 4 3.80 / 3.48, 6 4.15 / 3.60; width 5120:
+// B = 3 6.58 / 6.00, 4 6.65 / 6.09, and from 5 on the activations exceed what the GEMV kernels stage). B2_DECODE_SKINNY=3 draws it there,
+// B2_DECODE_SKINNY=0 takes the paths without a workspace at every batch (GEMV kernels up to 8, tile GEMMs above).
 bool use_skinny(const b2_kv* kv, int B) {
     const char* e0 = getenv("B2_DECODE_SKINNY");
     const int lo = (e0 != nullptr && e0[0] == '3') ? 3 : 7;
@@ -393,10 +403,9 @@ int decode_step_launch(b2_model* m, b2_kv* kv, int B, cudaStream_t st) {
     const int h = d.hidden, I = d.inter, H = d.heads, V = d.vocab;
     const int nsplit = decode_nsplit(B, H, kv->max_seq);
     B2_TRY(embed_tokens(kv->tok.as<int32_t>(), m->embed.p, m->x.p, B, h, V, m->err_dev, st));
-    // batch <= 8: tensor-core GEMV kernels (falls back to the skinny-M tcgen05 GEMM when the activations do not fit smem)
-    // batch 7..128: swap-AB stream-K GEMM (weights streamed once, all SMs busy); otherwise GEMV kernels (B <= 8) or
-    // the tile GEMM
-    const bool sk = use_skinny(kv, B);
+    // 7..128 requests: tile GEMMs or the stream-K GEMM (stream_k_step); fewer: tensor-core GEMV kernels, or the tile GEMMs where the activations do
+    // not fit their shared memory
+    const bool sk = use_skinny(kv, B), stream_k = sk && stream_k_step(h, I, B);
     const bool small = !sk && B <= 8 && gemv_fits(B, h, I, ACT_NONE) && gemv_fits(B, 2 * I, h, ACT_SWIGLU) &&
                        gemv_fits(B, 3 * h, h, ACT_NONE) && gemv_fits(B, V, h, ACT_NONE);
     const bool f8 = sk && m->fp8_decode;  // e4m3 weights x e4m3 activations through the same stream-K GEMM
@@ -410,7 +419,7 @@ int decode_step_launch(b2_model* m, b2_kv* kv, int B, cudaStream_t st) {
                         ACT_NONE, st));
         } else if (sk) {
             B2_TRY(rmsnorm_bf16(m->x.p, h, L.ln1.p, m->xn.p, B, h, d.rms_eps, st));
-            B2_TRY(skinny(kv, m->xn.p, h, L.wqkv.p, h, nullptr, 0, m->qkv.p, 3 * h, 0, B, 3 * h, h, ACT_NONE, st));
+            B2_TRY(skinny(kv, m->xn.p, h, L.wqkv.p, h, nullptr, 0, m->qkv.p, 3 * h, 0, B, 3 * h, h, ACT_NONE, stream_k, st));
         } else {
             B2_TRY(rmsnorm_bf16(m->x.p, h, L.ln1.p, m->xn.p, B, h, d.rms_eps, st));
             B2_TRY(gemm(m->xn.p, h, L.wqkv.p, h, nullptr, nullptr, 0, m->qkv.p, 3 * h, 0, B, 3 * h, h, ACT_NONE, st));
@@ -440,10 +449,10 @@ int decode_step_launch(b2_model* m, b2_kv* kv, int B, cudaStream_t st) {
                         ACT_SWIGLU, st));
             B2_TRY(gemv(m->act.p, I, L.wd.p, I, nullptr, 0.f, m->x.p, h, m->x.p, h, 0, B, h, I, ACT_NONE, st));
         } else if (sk) {
-            B2_TRY(skinny(kv, m->attn.p, h, L.wo.p, h, m->x.p, h, m->x.p, h, 0, B, h, h, ACT_NONE, st));
+            B2_TRY(skinny(kv, m->attn.p, h, L.wo.p, h, m->x.p, h, m->x.p, h, 0, B, h, h, ACT_NONE, stream_k, st));
             B2_TRY(rmsnorm_bf16(m->x.p, h, L.ln2.p, m->xn.p, B, h, d.rms_eps, st));
-            B2_TRY(skinny(kv, m->xn.p, h, L.wgu.p, h, nullptr, 0, m->act.p, I, 0, B, 2 * I, h, ACT_SWIGLU, st));
-            B2_TRY(skinny(kv, m->act.p, I, L.wd.p, I, m->x.p, h, m->x.p, h, 0, B, h, I, ACT_NONE, st));
+            B2_TRY(skinny(kv, m->xn.p, h, L.wgu.p, h, nullptr, 0, m->act.p, I, 0, B, 2 * I, h, ACT_SWIGLU, stream_k, st));
+            B2_TRY(skinny(kv, m->act.p, I, L.wd.p, I, m->x.p, h, m->x.p, h, 0, B, h, I, ACT_NONE, stream_k, st));
         } else {
             B2_TRY(gemm(m->attn.p, h, L.wo.p, h, nullptr, m->x.p, h, m->x.p, h, 0, B, h, h, ACT_NONE, st));
             B2_TRY(rmsnorm_bf16(m->x.p, h, L.ln2.p, m->xn.p, B, h, d.rms_eps, st));
@@ -459,7 +468,7 @@ int decode_step_launch(b2_model* m, b2_kv* kv, int B, cudaStream_t st) {
                     ACT_NONE, st));
     } else if (sk) {
         B2_TRY(rmsnorm_bf16(m->x.p, h, m->final_norm.p, m->xn.p, B, h, d.rms_eps, st));
-        B2_TRY(skinny(kv, m->xn.p, h, m->lm_head.p, h, nullptr, 0, m->logits.p, V, 1, B, V, h, ACT_NONE, st));
+        B2_TRY(skinny(kv, m->xn.p, h, m->lm_head.p, h, nullptr, 0, m->logits.p, V, 1, B, V, h, ACT_NONE, stream_k, st));
     } else {
         B2_TRY(rmsnorm_bf16(m->x.p, h, m->final_norm.p, m->xn.p, B, h, d.rms_eps, st));
         B2_TRY(gemm(m->xn.p, h, m->lm_head.p, h, nullptr, nullptr, 0, m->logits.p, V, 1, B, V, h, ACT_NONE, st));
@@ -1533,6 +1542,8 @@ int b2_op_gemv(const void* x, int64_t ldx, const void* W, int ldw, const void* n
     return gemv(x, ldx, W, ldw, norm_gamma, eps, residual, ld_res, out, ld_out, out_fp32, B, N, K, act,
                 reinterpret_cast<cudaStream_t>(stream));
 }
+
+int b2_op_decode_stream_k(int hidden, int inter, int batch) { return stream_k_step(hidden, inter, batch) ? 1 : 0; }
 
 int b2_op_gemm_skinny(const void* x, int ldx, const void* W, int ldw, const void* residual, int ld_res, void* out,
                       int ld_out, int out_fp32, int B, int N, int K, int act, void* workspace, int64_t workspace_bytes,

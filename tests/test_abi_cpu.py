@@ -87,3 +87,14 @@ def test_gated_unit_refuses_plans_that_cut_k(plan):
     lib, at = _b2.load_library(), 1 << 20
     r = lib.b2_op_gemm_glu(at, 512, at, 512, at, 64, 32, 64, 512, 1.0, 0.0, 0.0, 0, None, 1, plan, None)
     assert r == -1 and "no epilogue" in _b2.last_error()
+
+
+def test_route_of_batched_decode_steps():
+    """Which kernel a bf16 step of several requests runs its Linears on, at the widths and batches where both were timed: the tile GEMMs up to a
+    width of 4608, the stream-K GEMM above it for as many requests as it does not pad (32, and 64 at a width of 8192)."""
+    from llava import _b2
+
+    route = _b2.load_library().b2_op_decode_stream_k
+    for h, inter, most in [(2048, 5632, 0), (3072, 8192, 0), (4096, 11008, 0), (4608, 12288, 0), (5120, 13824, 32), (6656, 17920, 32), (8192, 22016, 64)]:
+        for B in (7, 8, 16, 32, 33, 40, 64, 65, 128):
+            assert route(h, inter, B) == int(B <= most), (h, B)

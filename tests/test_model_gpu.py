@@ -308,11 +308,11 @@ def test_13b_layer_shapes_decode_equals_prefill_recompute(B):
     eng.close()
 
 
-@pytest.mark.parametrize("B,dims", [(12, (4096, 11008, 32)), (32, (4096, 11008, 32)), (32, (5120, 13824, 40))])
+@pytest.mark.parametrize("B,dims", [(12, (4096, 11008, 32)), (32, (4096, 11008, 32)), (7, (5120, 13824, 40)), (32, (5120, 13824, 40)), (33, (5120, 13824, 40))])
 def test_batched_decode_skinny_gemm_equals_prefill_recompute(B, dims):
-    """BASELINE bs=32 decode at LLaVA-1.5-7B / 13B layer shapes (2 layers): every Linear of the step runs through the
-    swap-AB stream-K tcgen05 GEMM (csrc/gemm_skinny.cu: stream-K splits, SwiGLU epilogue, fp32 logits) replayed from a
-    CUDA graph; its logits must equal a prefill (tile GEMM + flash attention) over the extended sequence."""
+    """BASELINE bs=32 decode at LLaVA-1.5-7B / 13B layer shapes (2 layers): every Linear of the step runs on the tile
+    GEMMs (7B, and 13B above 32 requests) or on the swap-AB stream-K tcgen05 GEMM (13B up to 32; csrc/gemm_skinny.cu: stream-K
+    splits, SwiGLU epilogue, fp32 logits), replayed from a CUDA graph; its logits must equal a prefill (tile GEMM + flash attention) over the extended sequence."""
     h, I, H = dims
     cfg = O.make_config(hidden=h, inter=I, layers=2, heads=H, vit_layers=2)
     w = O.make_weights(cfg, seed=11)
@@ -338,7 +338,7 @@ def test_batched_decode_skinny_gemm_equals_prefill_recompute(B, dims):
 
 
 def test_decode_batch_above_8_uses_gemm_path_and_matches_oracle():
-    """B > 8 decode runs the swap-AB stream-K tcgen05 GEMM path (+ CUDA-graph replay); B <= 8 the GEMV kernels / the
+    """Decode of 7 and more requests runs the tile GEMMs at these widths (+ CUDA-graph replay); fewer the GEMV kernels / the
     persistent megakernel (B <= 2).
     Both must agree with the oracle and with each other on the shared samples."""
     cfg = O.CONFIGS["tiny"]
