@@ -174,16 +174,18 @@ int want_shape(const char* key, const int64_t* shape, int ndim, int64_t a, int64
     return 0;
 }
 
-bool tc_enabled() {  // B2_SEQ_TC=0: every Linear on the FMA kernels (A/B runs, tests of the two paths against each other)
+bool tc_enabled() {  // B2_SEQ_TC=0: every Linear, of one row too, on the FMA kernels of linear_generic.cu (A/B runs, tests of the two paths against each other)
     const char* e = getenv("B2_SEQ_TC");
     return !(e != nullptr && e[0] == '0');
 }
 
-int tc_min_rows() {  // fewest rows that take the tensor-core GEMM (below: the weight-streaming FMA kernels)
+// Fewest rows whose products count as tensor-core ones: the kernel in front then writes the bf16 rows that the product reads, and a dynamic-tanh norm
+// is a launch of its own. The products themselves stream their weights up to LINEAR_STREAM_MAX rows (linear_stream.cu) and are tile GEMMs above.
+int tc_min_rows() {
     const char* e = getenv("B2_SEQ_TC_MIN_ROWS");
     const int v = e != nullptr ? atoi(e) : 0;
-    // measured at widths 2048 / 4096 (decode step, ms): 4 rows 0.76 / 1.38 on the tile GEMM vs 0.78 / 1.48 on the FMA kernel,
-    // 8 rows 0.87 / 1.59 vs 1.14 / 3.45; 2 rows 0.71 / 1.28 vs 0.62 / 1.10
+    // (drawn when 4 and more rows ran on the tile GEMM, decode steps at widths 2048 / 4096 in ms: 4 rows 0.76 / 1.38 vs 0.78 / 1.48 on the FMA kernel, 2
+    // rows 0.71 / 1.28 vs 0.62 / 1.10; the streamed products take fp32 and bf16 rows alike)
     return v >= 1 ? v : 4;
 }
 
@@ -214,7 +216,7 @@ struct Lin {  // one Linear call on the model's compute dtype
         a.A16 = a16;
         a.parts = s.lin_parts.p; a.parts_bytes = s.lin_parts.bytes;
         if (tc_enabled() && linear_splits(a)) return linear_split_f32(a, st);
-        if ((M == 1 || tc_enabled()) && linear_streams(a)) return linear_stream_f32(a, st);
+        if (tc_enabled() && linear_streams(a)) return linear_stream_f32(a, st);
         // bf16 compute, a portion of a prompt: the tcgen05 GEMM on a bf16 copy of A (weights are stored with their rows
         // padded to a multiple of 8, zero-filled, so N rounds up; the pitch of every projection buffer is a multiple of 8)
         const int Np = (N + 7) / 8 * 8;
@@ -725,7 +727,7 @@ static int seq_feed_forward(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, c
         LinearArgs up;   // a handful of rows: both products and the unit in one stream of the weights
         up.A = h; up.lda = width; up.A16 = in.h16; up.W = W.up_w.p; up.ldw = width; up.w_dtype = s.w_dtype; up.out = s.ffa.as<float>(); up.ld_out = ff;
         up.M = R; up.N = ff; up.K = width; up.round_a = s.d.compute == B2_COMPUTE_BF16; up.gated = 1; up.glu = act;
-        if ((R == 1 || tc_enabled()) && linear_streams(up)) {
+        if (tc_enabled() && linear_streams(up)) {
             if (R > 1 && lin.tensor_cores(width, ff, target, width, R)) up.out16 = s.ff.p;   // bf16 rows for the second product
             B2_TRY(linear_stream_f32(up, st));
             return lin(up.out16 != nullptr ? nullptr : s.ffa.as<float>(), ff, W.down_w, width, ff, target, width, R, LIN_NONE, alpha, accumulate, nullptr, 0, nullptr,
