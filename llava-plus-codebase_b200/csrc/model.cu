@@ -564,7 +564,7 @@ int decode_step_mega(b2_model* m, b2_kv* kv, int B, cudaStream_t st) {
     static int trace_mode = -1;
     if (trace_mode < 0) { const char* e = getenv("B2_MEGA_TRACE"); trace_mode = (e && e[0] == '1') ? 1 : 0; }
     if (trace_mode == 1) {
-        // debug: per-phase SM-clock timestamps of CTA 0 for one step, dumped to gpurun_out/mega_trace.txt
+        // debug: per-phase SM-clock timestamps of CTA 0 for one step, written to mega_trace.txt in the working directory
         static int steps_seen = 0;
         if (++steps_seen == 40) {
             const int n = (5 * d.layers + 2) * 4;
@@ -576,7 +576,7 @@ int decode_step_mega(b2_model* m, b2_kv* kv, int B, cudaStream_t st) {
             cudaStreamSynchronize(st);
             std::vector<long long> host(n);
             cudaMemcpy(host.data(), tb.p, (size_t)n * 8, cudaMemcpyDeviceToHost);
-            FILE* f = fopen("gpurun_out/mega_trace.txt", "w");
+            FILE* f = fopen("mega_trace.txt", "w");
             if (f) {
                 for (int ph = 0; ph <= 5 * d.layers; ++ph)
                     fprintf(f, "%d %lld %lld %lld %lld %lld\n", ph, host[ph * 4], host[ph * 4 + 1], host[ph * 4 + 2],

@@ -1,6 +1,6 @@
 """Sweep of the BASELINE.json configurations that are not bench.py's headline line (configs[2], [3] and the
 batch ladder of configs[1]): device-resident timings with CUDA events on the launching stream, one model build
-per size. Writes one JSON object per measurement to stdout (and to gpurun_out/config_sweep.jsonl).
+per size. Writes one JSON object per measurement to stdout (and to --out).
 
     python scripts/config_sweep.py --model 7b --vit 1,16,64,256 --prefill 1,8,32 --decode 1,2,4,8,16,32
 """
@@ -39,7 +39,7 @@ def main():
     ap.add_argument("--prompt", type=int, default=128)
     ap.add_argument("--new", type=int, default=64)
     ap.add_argument("--max-images", type=int, default=32)
-    ap.add_argument("--out", default="gpurun_out/config_sweep.jsonl")
+    ap.add_argument("--out", default="./config_sweep.jsonl")
     a = ap.parse_args()
     from llava import _b2
     from llava.model.llava_arch import build_source_index

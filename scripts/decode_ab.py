@@ -26,7 +26,7 @@ def main():
     ap.add_argument("--batches", default="8,32")
     ap.add_argument("--new", type=int, default=64)
     ap.add_argument("--variants", default="default;B2_SAMPLE_LEGACY=1")
-    ap.add_argument("--out", default="gpurun_out/decode_ab.jsonl")
+    ap.add_argument("--out", default="./decode_ab.jsonl")
     a = ap.parse_args()
     from llava import _b2
     from llava.model.llava_arch import build_source_index

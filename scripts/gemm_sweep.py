@@ -67,5 +67,4 @@ for name, M, N, K, act in SHAPES:
     row["cublas_tflops"] = round(2.0 * M * N * K / (e0.elapsed_time(e1) / 20 * 1e-3) / 1e12, 1)
     res.append(row)
     print(json.dumps(row), flush=True)
-os.makedirs(os.path.join(ROOT, "gpurun_out"), exist_ok=True)
-json.dump(res, open(os.path.join(ROOT, "gpurun_out", "gemm_sweep.json"), "w"), indent=1)
+json.dump(res, open("gemm_sweep.json", "w"), indent=1)

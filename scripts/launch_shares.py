@@ -1,5 +1,5 @@
 """Aggregate an `ncu --metrics gpu__time_duration.sum --csv` log by kernel name: launches, total and average time.
-   python scripts/launch_shares.py gpurun_out/launches_b4.csv [name-regex-to-keep]"""
+   python scripts/launch_shares.py launches_b4.csv [name-regex-to-keep]"""
 import collections
 import csv
 import re

@@ -26,7 +26,7 @@ def main():
     ap.add_argument("--reps", type=int, default=3)
     ap.add_argument("--configs", default="0,1,0;0,1,1;4,1,0;8,1,0;12,1,0;16,1,0;8,2,0;8,1,1;12,1,1")
     ap.add_argument("--batches", default="", help="after the knob sweep: decode at these batch sizes with the skinny GEMM on/off")
-    ap.add_argument("--out", default="gpurun_out/mega_sweep.jsonl")
+    ap.add_argument("--out", default="./mega_sweep.jsonl")
     a = ap.parse_args()
     from llava import _b2
     from llava.model.llava_arch import build_source_index

@@ -39,7 +39,7 @@ def main():
     ap.add_argument("--model", default="7b")
     ap.add_argument("--batch", default="32")
     ap.add_argument("--ctx", type=int, default=736)
-    ap.add_argument("--out", default="gpurun_out/op_bench.jsonl")
+    ap.add_argument("--out", default="./op_bench.jsonl")
     a = ap.parse_args()
     _b2.init(0)
     lib = _b2.load_library()

@@ -7,8 +7,8 @@ for the launches of the LAST decode step in the file, where each launch's time g
     tail      publish -> exit (finalisers: re-read partials, epilogue, stores); fx_wait / fx_epi / fx_exit split a staged fix-up into
               partials landed in shared memory / sums + stores issued / exit
 
-    B2_SKINNY_TRACE=gpurun_out/sk_trace.txt python scripts/decode_ab.py --batches 32 --variants REPS=2 ...
-    python scripts/skinny_trace.py gpurun_out/sk_trace.txt [launches_per_step]
+    B2_SKINNY_TRACE=sk_trace.txt python scripts/decode_ab.py --batches 32 --variants REPS=2 ...
+    python scripts/skinny_trace.py sk_trace.txt [launches_per_step]
 """
 import statistics
 import sys

@@ -1,9 +1,8 @@
-"""Turn gpurun_out/ ncu artefacts into the tracked summaries under profiles/ (run in the build container).
-   python scripts/summarize_profiles.py <tag>      e.g. r1a
+"""Text summaries of ncu output (launch lists, .ncu-rep reports).
+   python scripts/summarize_profiles.py <tag> <folder with the profiler's output> [folder for the summaries, profiles/ by default]
 """
 import collections
 import csv
-import gzip
 import os
 import re
 import shutil
@@ -11,7 +10,7 @@ import subprocess
 import sys
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-OUT = os.path.join(ROOT, "gpurun_out")
+OUT = "."
 PROF = os.path.join(ROOT, "profiles")
 KEYS = ["gpu__time_duration.sum", "dram__bytes_read.sum", "dram__bytes_write.sum",
         "gpu__dram_throughput.avg.pct_of_peak_sustained_elapsed", "dram__bytes_read.sum.per_second",
@@ -42,12 +41,10 @@ def launches(tag, name="launches.csv"):
     tot = sum(v[1] for v in agg.values())
     with open(os.path.join(PROF, f"{tag}_launches_summary.txt"), "w") as f:
         f.write(f"# ncu --metrics gpu__time_duration.sum --clock-control none (serialised, cold-cache): compare SHARES\n")
-        f.write(f"# source: gpurun_out/{name} ({sum(v[0] for v in agg.values())} launches, {tot/1e6:.1f} ms of kernel time)\n")
+        f.write(f"# source: {name} ({sum(v[0] for v in agg.values())} launches, {tot/1e6:.1f} ms of kernel time)\n")
         f.write(f"{'share':>8} {'launches':>9} {'avg_us':>10}  kernel\n")
         for k, v in sorted(agg.items(), key=lambda x: -x[1][1]):
             f.write(f"{v[1]/tot*100:7.2f}% {v[0]:9d} {v[1]/v[0]/1e3:10.2f}  {k}\n")
-    with open(path, "rb") as fi, gzip.open(os.path.join(PROF, f"{tag}_launches.csv.gz"), "wb") as fo:
-        shutil.copyfileobj(fi, fo)
 
 
 def full(tag, rep):
@@ -58,7 +55,7 @@ def full(tag, rep):
     rows = list(csv.reader(raw.splitlines()))
     hdr, units = rows[0], rows[1]
     with open(os.path.join(PROF, f"{tag}_{rep}_ncu_full.txt"), "w") as f:
-        f.write(f"# ncu --set full --clock-control none --import-source on; source gpurun_out/{rep}.ncu-rep\n")
+        f.write(f"# ncu --set full --clock-control none --import-source on; source {rep}.ncu-rep\n")
         for n, row in enumerate(rows[2:]):
             f.write(f"\n## launch {n}: {row[hdr.index('Kernel Name')][:110]}\n")
             for k in KEYS:
@@ -74,8 +71,8 @@ def full(tag, rep):
 
 if __name__ == "__main__":
     tag = sys.argv[1] if len(sys.argv) > 1 else "r1"
-    if len(sys.argv) > 2:   # on the GPU box: write the text summaries next to the reports (only gpurun_out/ travels back,
-        PROF = sys.argv[2]  # and it is capped at 64 MiB: the .ncu-rep files themselves are deleted by the calling script)
+    OUT = sys.argv[2] if len(sys.argv) > 2 else OUT
+    PROF = sys.argv[3] if len(sys.argv) > 3 else PROF
     os.makedirs(PROF, exist_ok=True)
     launches(tag)
     import glob
