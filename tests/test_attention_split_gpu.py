@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 import torch
 
+import test_katadra_gpu as K
 from oracle import sofopel_oracle as O
 from test_sofopel_gpu import build, config, diff, tokens_for, win
 
@@ -36,6 +37,42 @@ def check(mixer, portions, seed=0):
 @pytest.mark.parametrize("n", [15, 16, 31, 33, 63, 64, 65, 128, 129])
 def test_edges_of_key_and_query_tiles(n):
     check(win(4, 1, 128, 128, None, None, 64), [n])
+
+
+@pytest.mark.parametrize("n", [40, 63, 64, 65, 96, 97])
+@pytest.mark.parametrize("vdim", [64, 128])
+def test_edges_of_the_key_tiles_of_wide_keys(n, vdim):
+    check(win(3, 1, 192, vdim, None, None, 64), [n])
+
+
+# as BOUND, with the soft-cap, the query's temperature and the layer norm behind the three sums
+BOUND_EXTRA = 5e-6
+
+
+@pytest.mark.parametrize("dim,vdim", [(40, 64), (64, 128), (128, 64), (128, 128), (192, 64), (192, 128)])
+@pytest.mark.parametrize("extra", ["cap", "bias", "both"])
+@pytest.mark.parametrize("portions", [[40], [63], [64], [65], [129], [45, 20, 64]])
+def test_soft_cap_and_distance_bias(dim, vdim, extra, portions):
+    left = {"heads": 4, "kv_heads": 2, "dim": dim, "vdim": vdim, "bias_max": 50, "scale": dim ** -0.5, "softcap": 1e4 if extra == "bias" else 1.5,
+            "q_temp": {"coef": 0.3, "every": 16}, "rel_rows": 12}
+    cfg = K.config([{"type": "parallel", "mlp": None, "mixer": {"left": left, "right": {"heads": 1, "dim": 8, "decay_rank": 2}, "left_scale": 1.0, "right_scale": 0.0}}],
+                   width=64, vocab=90)
+    w = K.O.random_weights(cfg, seed=2)
+    rel = next(k for k in w if k.endswith("left.rel"))
+    w[rel] = w[rel] * 0 if extra == "cap" else (w[rel] / w[rel].std()).bfloat16().to(w[rel].dtype)
+    n = sum(portions)
+    model, _ = K.build(cfg, torch.float32, weights=w, max_batch=2, max_seq=n + 3, max_rows=max(portions))
+    toks = K.tokens_for(cfg, n)
+    eng = model._ensure_engine()
+    kv, got, at = eng.new_kv(2, n + 3), [], 0
+    for p in portions:
+        got.append(eng.append_tokens(kv, 1, toks[at:at + p], restart=at == 0, residuals=True)[1][0])
+        at += p
+    got = torch.cat(got).double().cpu()
+    model.invalidate_engine()
+    ref = K.O.forward(cfg, w, toks, return_layers=True)[1][0].double()
+    add = ref - w["embed"].double()[torch.tensor(toks)]
+    assert float((got - ref).norm() / add.norm()) <= BOUND_EXTRA
 
 
 @pytest.mark.parametrize("heads,kv,dim,vdim", [(1, 1, 64, 64), (2, 2, 65, 65), (3, 1, 192, 128), (5, 5, 8, 4), (6, 2, 129, 61), (7, 1, 30, 127), (2, 1, 193, 128), (2, 1, 128, 129)])
