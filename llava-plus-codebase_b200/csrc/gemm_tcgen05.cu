@@ -711,11 +711,7 @@ int gemm_bf16(const GemmArgs& g, cudaStream_t stream) {
     const bool grouped = g.tile_group != nullptr, glu = g.act == ACT_SWIGLU || g.act == ACT_GLU;
     B2_CHECK_ARG(!grouped || (g.groups >= 1 && (g.act == ACT_NONE || g.act == ACT_GLU) && g.bias == nullptr && g.residual == nullptr && g.M % BM == 0),
                  "gemm: a grouped product takes whole tiles of %d rows, no bias, residual or fused activation but the gated unit", BM);
-    // An explicit plan that cuts K over a cluster. Calls that it cannot take but that ignored such a number before the plan existed (fused SwiGLU and
-    // rotation, fewer k-blocks than CTAs) still ignore it; the gated unit is refused inside.
-    const int plan_s = g.bn_override / 1000, plan_bn = g.bn_override % 1000;
-    if ((plan_s == 2 || plan_s == 4) && (plan_bn == 64 || plan_bn == 128) && !grouped && g.act != ACT_SWIGLU && g.act != ACT_ROPE_QKV && plan_s <= (g.K + BK - 1) / BK)
-        return gemm_bf16_splitk(g, plan_bn, plan_s, stream);
+    if (g.bn_override >= 1000 && !grouped) return gemm_bf16_splitk(g, g.bn_override % 1000, g.bn_override / 1000, stream);
     if (g.bn_override == 2 && !grouped) return gemm_bf16_2cta(g, stream);  // CTA-pair kernel (cta_group::2, 256x256 pair tiles)
 
     // Tile-N choice. Cost model fitted to profiles/r1b_gemm_sweep.json: a tile costs ~BN / rel(BN) (rel = tensor-pipe
