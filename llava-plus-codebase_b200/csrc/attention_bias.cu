@@ -49,7 +49,7 @@ __device__ __forceinline__ void store_out(const BiasAttnArgs& a, int row, int he
 
 // unit = q head (normalise, temperature, in place) | k head (normalise, append) | v head (append)
 __global__ void attn_prepare_kernel(BiasAttnArgs a) {
-    pdl_enter();
+    pdl_enter_late();
     const int units = a.H + 2 * a.G;
     const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (w >= a.rows * units) return;
@@ -83,7 +83,7 @@ constexpr int AT_WARPS = 4, AT_MAXC = 8;  // dv <= 32 * AT_MAXC
 
 template <bool VEC>
 __global__ void __launch_bounds__(AT_WARPS * 32) attn_bias_kernel(BiasAttnArgs a) {
-    pdl_enter();
+    pdl_enter_late();
     extern __shared__ float sq[];  // [AT_WARPS][dk]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int w = blockIdx.x * AT_WARPS + warp;
@@ -210,7 +210,7 @@ __device__ __forceinline__ void copy_rows_f4(float* __restrict__ dst, int dpitch
 
 template <bool VEC, int MAXC>
 __global__ void __launch_bounds__(TL_WARPS * 32, MAXC == 16 ? 1 : 2) attn_tile_kernel(BiasAttnArgs a, int QT, int HC) {
-    pdl_enter();
+    pdl_enter_late();
     extern __shared__ float sm[];
     const int HGall = a.H / a.G, chunks = (HGall + HC - 1) / HC;
     const int g = blockIdx.y / chunks, h0 = g * HGall + (blockIdx.y % chunks) * HC, HG = min(HC, g * HGall + HGall - h0);
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(TL_WARPS * 32, MAXC == 16 ? 1 : 2) attn_tile_k
 // one block per (row, head): every thread turns the splits' (max, sum) into weights (nsplit <= 64 values from L1) and combines
 // its value columns in split order
 __global__ void __launch_bounds__(512) attn_merge_kernel(BiasAttnArgs a) {
-    pdl_enter();
+    pdl_enter_late();
     const int w = blockIdx.x;
     const int r = w / a.H, h = w % a.H;
     if (a.row_pos[r] < 0) return;

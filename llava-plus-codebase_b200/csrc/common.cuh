@@ -66,9 +66,18 @@ __device__ __forceinline__ void pdl_trigger_small() {
 // First statement of a kernel of the layer-list path: it is launched while its predecessor drains, and its own successor while it does. A step
 // or a prompt is a chain of 30..60 kernels of 2..30 us; launched one after the other's end they stood 2.2 us apart in a prompt and ~0.4 us in a
 // captured step: prompts 500 -> 457 us (latent attention with experts, 1536 rows), 419 -> 366 (41 rows of a four-layer model), a step 276 -> 270.
+// pdl_enter lets the successor in before the kernel may start itself. A chain of such kernels piles up: each lets in the next, and their waiting
+// blocks take slots from the one that works. So some kernels of every layer (attention against the cache, rotation, routing of experts, sandwich
+// norms) break the chain with pdl_enter_late. Where the products follow their weights can travel early, and those keep pdl_enter. One token (us; all
+// early / all late / as it is; the plain launches before): latent attention with experts, width 1024 298 / 268 / 267 (298), in fp32 327 / 309 / 304
+// (312); window and gated linear attention 150 / 145 / 144 (172). A prompt of 41 rows, width 2048: 346 / 355 / 331 (498).
 __device__ __forceinline__ void pdl_enter() {
     pdl_trigger_small();
     pdl_wait();
+}
+__device__ __forceinline__ void pdl_enter_late() {
+    pdl_wait();
+    pdl_trigger_small();
 }
 
 bool pdl_enabled();  // B2_PDL=0 turns the launch attribute off (A/B runs)

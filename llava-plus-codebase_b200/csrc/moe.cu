@@ -24,7 +24,7 @@ __device__ __forceinline__ void warp_argmax(float& v, int& i) {
 
 // One warp per row. Shared memory per warp: E scores, G group scores (later: group alive flags), E taken flags, E choice scores.
 __global__ void moe_route_kernel(MoeRouteArgs a) {
-    pdl_enter();
+    pdl_enter_late();
     extern __shared__ float sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = blockIdx.x * (blockDim.x >> 5) + warp;
@@ -107,7 +107,7 @@ __global__ void moe_route_kernel(MoeRouteArgs a) {
 __global__ void __launch_bounds__(1024) moe_plan_kernel(const int32_t* __restrict__ idx, int pairs, int top, int experts, int tile, int max_tiles,
                                                         int32_t* __restrict__ pair_pos, int32_t* __restrict__ src_row,
                                                         int32_t* __restrict__ tile_group) {
-    pdl_enter();
+    pdl_enter_late();
     extern __shared__ int cnt[];   // [experts] counts, then [experts] offsets
     int* off = cnt + experts;
     for (int e = threadIdx.x; e < experts; e += blockDim.x) cnt[e] = 0;
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int32_t* __restric
 // out[r, c] = act(in[r, c], in[r, ff + c]): the gated unit (SiLU(g) u, or its bounded and shifted form)
 __global__ void glu_rows_kernel(const float* __restrict__ in, int64_t ld_in, float* __restrict__ out, int64_t ld_out, int ff,
                                 __nv_bfloat16* __restrict__ out16, int64_t ld_out16, GluAct act) {
-    pdl_enter();
+    pdl_enter_late();
     const size_t r = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < ff) {
@@ -147,7 +147,7 @@ __global__ void glu_rows_kernel(const float* __restrict__ in, int64_t ld_in, flo
 
 __global__ void gather_rows_bf16_kernel(const float* __restrict__ A, int64_t lda, const int32_t* __restrict__ src_row, __nv_bfloat16* __restrict__ out,
                                         int64_t ld_out, int K) {
-    pdl_enter();
+    pdl_enter_late();
     const size_t p = blockIdx.y;
     const int src = src_row[p];
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) * 2;
@@ -162,7 +162,7 @@ __global__ void gather_rows_bf16_kernel(const float* __restrict__ A, int64_t lda
 // x[r] += alpha * sum_k w[r, k] * y[pair_pos[r * top + k]] (a negative position: h[r] in y's place)
 __global__ void moe_combine_kernel(float* __restrict__ x, const float* __restrict__ y, int64_t ldy, const int32_t* __restrict__ pair_pos,
                                    const float* __restrict__ w, int top, int cols, float alpha, const float* __restrict__ h, int64_t ldh) {
-    pdl_enter();
+    pdl_enter_late();
     const size_t r = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= cols) return;

@@ -430,7 +430,7 @@ int launch_embed_norm(const int32_t* tokens, const TT* table, float* x, int rows
 
 // post-norm add of one sublayer, pre-norm of the next, and (decode steps) the input convolution with its carried inputs
 __global__ void sandwich_norm_kernel(SandwichNormArgs a) {
-    pdl_enter();
+    pdl_enter_late();
     __shared__ float red[33];
     const size_t r = blockIdx.x;
     const int cols = a.cols;
@@ -486,7 +486,7 @@ __global__ void sandwich_norm_kernel(SandwichNormArgs a) {
 // row and is bound by round trips, not by bandwidth).
 template <int V, int TP>
 __global__ void __launch_bounds__(512) sandwich_norm_reg_kernel(SandwichNormArgs a) {
-    pdl_enter();
+    pdl_enter_late();
     __shared__ float red[33];
     const size_t r = blockIdx.x;
     const int cols = a.cols, tid = threadIdx.x, nt = blockDim.x;

@@ -23,11 +23,11 @@ namespace {
 struct RotateParts { RotateArgs p[3]; };
 __device__ __forceinline__ void rotate_rows_body(const RotateArgs& a);
 __global__ void __launch_bounds__(256) rotate_rows_kernel(RotateArgs a) {
-    pdl_enter();
+    pdl_enter_late();
     rotate_rows_body(a);
 }
 __global__ void __launch_bounds__(256) rotate_rows_multi_kernel(RotateParts ps) {
-    pdl_enter();
+    pdl_enter_late();
     rotate_rows_body(ps.p[blockIdx.z]);
 }
 __device__ __forceinline__ void rotate_rows_body(const RotateArgs& a) {
@@ -68,7 +68,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 // everything it writes before it writes (its own pairs and single entries), and the sum of squares is complete before any lane writes,
 // so the call may run in place.
 __global__ void __launch_bounds__(256) rotate_rows_warp_kernel(RotateParts ps, int n_parts) {
-    pdl_enter();
+    pdl_enter_late();
     const int r = blockIdx.y, lane = threadIdx.x & 31;
     int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     int pi = 0;
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(256) rotate_rows_warp_kernel(RotateParts ps, i
 // then every head's pairs turn. Parts may read the same input (values that are the raw keys), so a part writes in place only what no
 // other part reads.
 __global__ void __launch_bounds__(256) rotate_rows_block_kernel(RotateParts ps) {
-    pdl_enter();
+    pdl_enter_late();
     __shared__ float red[8];
     const RotateArgs& a = ps.p[blockIdx.y];
     const int r = blockIdx.x, tid = threadIdx.x;
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(128) latent_rot_append_kernel(const float* __r
                                                                 float* __restrict__ cache, const int32_t* __restrict__ row_slot,
                                                                 const int32_t* __restrict__ row_pos, int rank, int rot, int pairs,
                                                                 const float2* __restrict__ table, int Smax, float eps) {
-    pdl_enter();
+    pdl_enter_late();
     __shared__ float red[4];
     const size_t r = blockIdx.x;
     const int pos = row_pos[r];
