@@ -113,8 +113,8 @@ int gemv(const void* x, int64_t ldx, const void* W, int ldw, const void* gamma, 
 
 // The bf16 Linears of a decode step of 7..128 requests run on one of two kernels, all of a step on the same (launches of one kind start earlier
 // behind one another than a mix). The tile GEMMs load the rows of x that there are and cut K over clusters where few tiles would be left, but
-// multiply 128 rows whatever B is: their heat costs clock where a step is a long stream of weights (1650..1780 MHz under the power limit at widths of 5120
-// and more, against 1850..1965). The stream-K GEMM over the kv-owned workspace multiplies 32 / 64 / 128, spreads every matrix over all SMs, and pays
+// multiply 128 rows whatever B is: their heat costs clock where a step is a long stream of weights (under the power limit 1610..1840 MHz at widths of
+// 5120 and more, against 1755..1965). The stream-K GEMM over the kv-owned workspace multiplies 32 / 64 / 128, spreads every matrix over all SMs, and pays
 // ~8 us of fix-up per launch. ms per step, tile GEMMs / stream-K, ~740 cached positions (width, weights of a layer, layers):
 //   4096, 405 MB, 32: B = 7 3.71 / 3.99, 16 4.41 / 4.66, 32 5.51 / 5.87, 64 7.74 / 9.20, 128 12.7 / 15.6     (2048, 3072: 15..31 % at B = 7..32)
 //   4608, 510 MB, 16: B = 7 2.25 / 2.28, 16 2.63 / 2.67, 32 3.30 / 3.33, 64 4.61 / 5.20

@@ -146,8 +146,8 @@ __global__ void __launch_bounds__(128) token_shift_carry_kernel(const float* __r
 // chunk's final state and the product of its decays per key; a second launch starts each further chunk from what those fold to, S_c = P_c S_(c-1)
 // + L_c, and writes its outputs. The chain is then 2 / C of the tokens for 5/3 of the arithmetic.
 // 1900 tokens, 8 heads of 128 x 256 (gated linear attention): 625 -> 191 us (two walks of 90 us, 11 us for the gates beforehand; before, 8 keys x
-// one column per thread and one chain). Issue slots bound a walk (65 % with the gates' arithmetic in it: 291 us for both, hence
-// scan_prepare_kernel), then the multiply-add pipe. 600 tokens, 32 heads of 128 x 64 (state space): 152 -> 84 us, 16 heads of 64 x 64 (RWKV) 128 -> 58.
+// one column per thread and one chain). Issue slots bound a walk (74 % of them taken in the first, 58 % in the one that
+// writes; with the gates' arithmetic in it 291 us for both, hence scan_prepare_kernel), then the multiply-add pipe. 600 tokens, 32 heads of 128 x 64 (state space): 152 -> 84 us, 16 heads of 64 x 64 (RWKV) 128 -> 58.
 constexpr int SC_TT = 16, SC_COLS = 64, SC_MAX_CHUNKS = 10;
 
 struct ScanPlan {
