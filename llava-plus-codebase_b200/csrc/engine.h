@@ -23,6 +23,7 @@ struct DevBuf {
         cudaError_t e = cudaMalloc(&p, n);
         if (e != cudaSuccess) {
             p = nullptr;
+            cudaGetLastError();  // a refusal, not a fault: the next launch must not report it as its own
             set_error("cudaMalloc(%zu bytes) failed: %s", n, cudaGetErrorString(e));
             return -2;
         }

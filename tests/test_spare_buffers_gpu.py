@@ -23,7 +23,6 @@ def device_with(free):
     try:
         yield
     finally:
-        torch.cuda.synchronize()
         del held
         torch.cuda.empty_cache()
 
@@ -41,11 +40,16 @@ def test_a_cache_fits_where_its_own_memory_does():
     ref = prompt(eng, first, toks)
     own = kv_heads * seq * (dim + vdim) * 4 + 8 * heads * 64 * (vdim + 2) * 4   # keys and values, partial sums of a step's key splits
     spare = 6 * kv_heads * (dim + vdim) * seq                                   # bf16 parts of its keys and values: as large as the partial sums
-    assert spare > 40 * MB
-    with device_with(own + 30 * MB):
+    assert spare > 60 * MB
+    again = eng.new_kv(1, 64)
+    assert torch.equal(prompt(eng, again, toks), ref)   # every kernel of the lines below is loaded by now
+    again.close()
+    with device_with(own + 50 * MB):
         kv = eng.new_kv(1, seq)
-        assert torch.equal(prompt(eng, kv, toks), ref)
+        got = prompt(eng, kv, toks)
+        torch.cuda.synchronize()
         kv.close()
+    assert torch.equal(got, ref)
     first.close()
     model.invalidate_engine()
 
@@ -76,3 +80,15 @@ def test_engines_without_spare_scratch(name):
     for got in (with_scratch, without):
         assert mod.err(got, ref) <= 2e-4     # the bound of the engines' own tests in true fp32
     assert not torch.equal(with_scratch, without)   # the two did take different paths
+
+
+def test_a_refused_cache_leaves_the_calls_behind_it_alone():
+    cfg = S.config([dict(S.win(8, 8, 128, 16, None, None, 0), mlp=None)], width=64)
+    model, _ = S.build(cfg, torch.float32, max_batch=1, max_seq=64, max_rows=64)
+    eng, toks = model._ensure_engine(), S.tokens_for(cfg, 50)
+    kv = eng.new_kv(1, 64)
+    ref = prompt(eng, kv, toks)
+    with pytest.raises(RuntimeError, match="cudaMalloc"):
+        eng.new_kv(1, 60_000_000)      # 245 GB of keys
+    assert torch.equal(prompt(eng, kv, toks), ref)
+    model.invalidate_engine()
