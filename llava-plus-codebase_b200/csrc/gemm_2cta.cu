@@ -24,6 +24,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "tile_store.cuh"
 
 namespace b2 {
 
@@ -41,7 +42,10 @@ constexpr int P_TILE_BYTES = P_BM * P_BK * 2;      // 16 KB
 constexpr int P_STAGE_BYTES = 2 * P_TILE_BYTES;    // A half + B half per CTA
 constexpr int P_STAGES = 6;
 constexpr int P_TMEM_COLS = 512;                   // two 256-column accumulator stages
-constexpr int P_SMEM = P_STAGES * P_STAGE_BYTES + 1024 + 256;
+constexpr int P_BOX = 128;                         // bytes of a row of an epilogue warp's box (tile_store.cuh)
+constexpr int P_BOX_BYTES = P_EPI_WARPS * 32 * P_BOX;
+constexpr int P_SMEM = P_STAGES * P_STAGE_BYTES + P_BOX_BYTES + 1024 + 256;
+static_assert(P_SMEM <= 227 * 1024, "shared memory of one CTA");
 
 struct PairEpi {
     const __nv_bfloat16* bias;
@@ -112,21 +116,20 @@ __device__ __forceinline__ void umma_commit_2sm(uint64_t* bar) {
                  : "memory");
 }
 
-__device__ __forceinline__ float p_quick_gelu(float x) { return __fdividef(x, 1.0f + __expf(-1.702f * x)); }
-__device__ __forceinline__ float p_gelu_erf(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752440f)); }
 __device__ __forceinline__ float p_silu(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
 // q*cos + rotate_half(q)*sin with bf16 rounding of each product and of the sum (attention.cu rope_apply: same expression)
 __device__ __forceinline__ float p_rope(float x, float partner_signed, float c, float s) {
     return round_bf16(round_bf16(x * c) + round_bf16(partner_signed * s));
 }
 
-template <int ACT>
+template <int ACT, bool F32>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1)
-gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, int M, int N, int K,
-                      PairEpi ep) {
+gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                      const __grid_constant__ CUtensorMap tmap_out, int M, int N, int K, PairEpi ep) {
     extern __shared__ uint8_t p_smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p_smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + P_STAGES * P_STAGE_BYTES);
+    uint8_t* boxes = smem + P_STAGES * P_STAGE_BYTES;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(boxes + P_BOX_BYTES);
     uint64_t* full_bar = bars;                        // [P_STAGES]   used in the leader
     uint64_t* empty_bar = bars + P_STAGES;            // [P_STAGES]   one per CTA
     uint64_t* tmem_full = bars + 2 * P_STAGES;        // [2]          one per CTA
@@ -156,6 +159,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tmap_a);
         tma_prefetch_desc(&tmap_b);
+        if constexpr (ACT != ACT_ROPE_QKV && !F32) tma_prefetch_desc(&tmap_out);
         for (int s = 0; s < P_STAGES; ++s) {
             mbar_init(&full_bar[s], 1);    // the leader producer's arrive.expect_tx (+ the TMA bytes of both CTAs)
             mbar_init(&empty_bar[s], 1);   // one multicast tcgen05.commit per use
@@ -171,31 +175,46 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     cluster_sync_all();  // barriers initialised and TMEM allocated in both CTAs before anyone signals across
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    pdl_trigger();
-    pdl_wait();  // set-up above overlapped the upstream kernel's tail (programmatic dependent launch); A / residual are its outputs
+    pdl_trigger();   // the set-up above and the first weights below overlap the upstream kernel's tail; A / residual are its outputs
 
     if (warp == 0) {
         if (lane == 0) {
             // ===================== TMA producer (both CTAs) =====================
-            int stage = 0;
+            // b_row: this CTA's 128 rows of W (half of the N tile; ACT_GLU: 64 of gate, 64 of up)
+            auto load_b = [&](uint8_t* sb, uint32_t leader_full, int kb, int b_row) {
+                if constexpr (ACT == ACT_GLU) {
+                    tma_load_2d_2sm(sb, &tmap_b, leader_full, kb * P_BK, b_row / 2, kEvictNormal);
+                    tma_load_2d_2sm(sb + P_TILE_BYTES / 2, &tmap_b, leader_full, kb * P_BK, N / 2 + b_row / 2, kEvictNormal);
+                } else {
+                    tma_load_2d_2sm(sb, &tmap_b, leader_full, kb * P_BK, b_row, kEvictNormal);
+                }
+            };
+            // the weight halves of the first stages travel in front of the programmatic-dependent-launch wait, A follows behind it
+            int pre = 0;
+            if (pair < num_tiles) {
+                int m_blk, n_blk;
+                tile_coords(pair, m_blk, n_blk);
+                for (; pre < num_kb && pre < P_STAGES; ++pre) {
+                    if (leader) mbar_arrive_expect_tx(&full_bar[pre], 2 * P_STAGE_BYTES);
+                    load_b(smem + pre * P_STAGE_BYTES + P_TILE_BYTES, mapa_rank(smem_u32(&full_bar[pre]), 0), pre, n_blk * P_TN + (int)rank * P_BM);
+                }
+            }
+            pdl_wait();
+            int stage = 0, seen = 0;
             uint32_t phase = 0;
             for (int t = pair; t < num_tiles; t += num_pairs) {
                 int m_blk, n_blk;
                 tile_coords(t, m_blk, n_blk);
                 const int a_row = m_blk * P_TM + (int)rank * P_BM;  // this CTA's 128 rows of A
-                const int b_row = n_blk * P_TN + (int)rank * P_BM;  // this CTA's 128 rows of W (half of the N tile; ACT_GLU: 64 of gate, 64 of up)
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    mbar_wait(&empty_bar[stage], phase ^ 1);
+                for (int kb = 0; kb < num_kb; ++kb, ++seen) {
                     uint8_t* sa = smem + stage * P_STAGE_BYTES;
                     const uint32_t leader_full = mapa_rank(smem_u32(&full_bar[stage]), 0);
-                    if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * P_STAGE_BYTES);
-                    tma_load_2d_2sm(sa, &tmap_a, leader_full, kb * P_BK, a_row, kEvictNormal);
-                    if constexpr (ACT == ACT_GLU) {
-                        tma_load_2d_2sm(sa + P_TILE_BYTES, &tmap_b, leader_full, kb * P_BK, b_row / 2, kEvictNormal);
-                        tma_load_2d_2sm(sa + P_TILE_BYTES + P_TILE_BYTES / 2, &tmap_b, leader_full, kb * P_BK, N / 2 + b_row / 2, kEvictNormal);
-                    } else {
-                        tma_load_2d_2sm(sa + P_TILE_BYTES, &tmap_b, leader_full, kb * P_BK, b_row, kEvictNormal);
+                    if (seen >= pre) {
+                        mbar_wait(&empty_bar[stage], phase ^ 1);
+                        if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * P_STAGE_BYTES);
+                        load_b(sa + P_TILE_BYTES, leader_full, kb, n_blk * P_TN + (int)rank * P_BM);
                     }
+                    tma_load_2d_2sm(sa, &tmap_a, leader_full, kb * P_BK, a_row, kEvictNormal);
                     if (++stage == P_STAGES) { stage = 0; phase ^= 1; }
                 }
             }
@@ -229,6 +248,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         }
     } else {
         // ===================== epilogue warps 2..9 (both CTAs: own 128 rows of the pair tile) =====================
+        pdl_wait();   // residual / out may be read or written by the upstream kernel
         const int q = warp & 3;
         const int half = (warp - 2) >> 2;
         int local = 0;
@@ -236,134 +256,85 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             int m_blk, n_blk;
             tile_coords(t, m_blk, n_blk);
             const int as = local & 1;
-            mbar_wait(&tmem_full[as], (local >> 1) & 1);
-            tc_fence_after();
-            const int row = m_blk * P_TM + (int)rank * P_BM + q * 32 + lane;
-            const bool row_ok = row < M;
-            const uint32_t taddr_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + as * P_TN;
+            const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + as * P_TN + half * 128;
+            const int row0 = m_blk * P_TM + (int)rank * P_BM + q * 32;
+            uint8_t* buf = boxes + (warp - 2) * 32 * P_BOX;
+            auto ready = [&] { mbar_wait(&tmem_full[as], (local >> 1) & 1); tc_fence_after(); };
+            auto drained = [&] {   // this warp has read its part of accumulator stage `as`: tell the leader's MMA issuer
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(mapa_rank(smem_u32(&tmem_empty[as]), 0));
+            };
             if constexpr (ACT == ACT_SWIGLU || ACT == ACT_GLU) {   // 64 gate columns, then 64 up columns of the same outputs
-#pragma unroll 1
-                for (int it = half * (P_TN / 128); it < (half + 1) * (P_TN / 128); ++it) {
-                    const int g = it >> 1, j = it & 1;
-                    uint32_t vg[32], vu[32];
-                    __syncwarp();
-                    tmem_ld_32x32(taddr_row + g * 128 + j * 32, vg);
-                    tmem_ld_32x32(taddr_row + g * 128 + 64 + j * 32, vu);
-                    tmem_ld_wait();
-                    const int ocol0 = (n_blk * P_TN) / 2 + g * 64 + j * 32;
-                    if (row_ok && ocol0 < N / 2) {
-                        __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(ep.out) + (size_t)row * ep.ld_out + ocol0;
-#pragma unroll
-                        for (int v8 = 0; v8 < 4; ++v8) {
-                            uint32_t pk[4];
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const float g0 = __uint_as_float(vg[v8 * 8 + 2 * e]), g1 = __uint_as_float(vg[v8 * 8 + 2 * e + 1]);
-                                const float u0 = __uint_as_float(vu[v8 * 8 + 2 * e]), u1 = __uint_as_float(vu[v8 * 8 + 2 * e + 1]);
-                                if constexpr (ACT == ACT_GLU) pk[e] = pack_bf16(glu_act(g0, u0, ep.glu), glu_act(g1, u1, ep.glu));
-                                else pk[e] = pack_bf16(p_silu(g0) * u0, p_silu(g1) * u1);
-                            }
-                            if (ACT == ACT_SWIGLU || ocol0 + v8 * 8 < N / 2) *reinterpret_cast<uint4*>(op + v8 * 8) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                        }
-                    }
-                }
+                const TileBox<P_BOX> box{&tmap_out, buf, lane, row0, M, N / 2};
+                store_glu_tile<P_BOX, 64, ACT == ACT_GLU ? 8 : 32>(box, taddr, n_blk * (P_TN / 2) + half * 64, ready, drained, [&](float g, float u) {
+                    if constexpr (ACT == ACT_GLU) return glu_act(g, u, ep.glu);
+                    else return p_silu(g) * u;
+                });
             } else if constexpr (ACT == ACT_ROPE_QKV) {
                 // This warp's half of the pair tile is the 128 columns of ONE head of q, k or v (hidden % 256 == 0, head_dim 128).
-                // Element i of the head rotates with element i + 64: the two 32-column chunks j and j + 2 are read together.
+                // Element i of the head rotates with element i + 64: columns j.. and 64 + j.. are read together, 8 at a time.
+                // Rows of q and rows of the caches lie at pitches of their own (and a tile may hold rows of two prompts), so the box leaves by
+                // ordinary stores: four lanes on 64 bytes of a row.
+                const int row = row0 + lane;
                 const int col_base = n_blk * P_TN + half * 128;
                 const int hdim = ep.rope_H * 128;
                 const int part = col_base / hdim;  // 0 = q, 1 = k, 2 = v
                 const int head = (col_base - part * hdim) >> 7;
-                const int b = row / ep.rope_S, tpos = row - b * ep.rope_S;
+                const uint4* tab = reinterpret_cast<const uint4*>(ep.rope_tab + (size_t)(row % ep.rope_S) * 64);  // 16 x 16 B: 64 (cos, sin) pairs
+                ready();
 #pragma unroll 1
-                for (int j = 0; j < 2; ++j) {
-                    uint32_t lo[32], hi[32];
+                for (int j = 0; j < 8; ++j) {
+                    uint32_t lo[8], hi[8];
                     __syncwarp();
-                    tmem_ld_32x32(taddr_row + half * 128 + j * 32, lo);
-                    tmem_ld_32x32(taddr_row + half * 128 + 64 + j * 32, hi);
+                    tmem_ld_cols(taddr + j * 8, lo);
+                    tmem_ld_cols(taddr + 64 + j * 8, hi);
                     tmem_ld_wait();
-                    if (!(row_ok && col_base < N)) continue;
-                    __nv_bfloat16* dst;
-                    if (part == 0) dst = reinterpret_cast<__nv_bfloat16*>(ep.out) + (size_t)row * ep.ld_out + col_base + j * 32;
-                    else dst = (part == 1 ? ep.kcache : ep.vcache) + (((size_t)b * ep.rope_H + head) * ep.rope_Smax + tpos) * 128 + j * 32;
-                    const uint4* tab = reinterpret_cast<const uint4*>(ep.rope_tab + (size_t)tpos * 64 + j * 32);  // 8 x 16 B: 32 (cos, sin) pairs
+                    if (j == 7) drained();
+                    float ol[8], oh[8];
+                    uint32_t csw[8];
+                    if (part < 2) {
+                        const uint4 t0 = __ldg(tab + j * 2), t1 = __ldg(tab + j * 2 + 1);
+                        csw[0] = t0.x; csw[1] = t0.y; csw[2] = t0.z; csw[3] = t0.w;
+                        csw[4] = t1.x; csw[5] = t1.y; csw[6] = t1.z; csw[7] = t1.w;
+                    }
 #pragma unroll
-                    for (int v8 = 0; v8 < 4; ++v8) {
-                        float ol[8], oh[8];
-                        uint32_t csw[8];
+                    for (int e = 0; e < 8; ++e) {
+                        const float xl = round_bf16(__uint_as_float(lo[e]));  // the projection as bf16, like the unfused path
+                        const float xh = round_bf16(__uint_as_float(hi[e]));
                         if (part < 2) {
-                            const uint4 t0 = __ldg(tab + v8 * 2), t1 = __ldg(tab + v8 * 2 + 1);
-                            csw[0] = t0.x; csw[1] = t0.y; csw[2] = t0.z; csw[3] = t0.w;
-                            csw[4] = t1.x; csw[5] = t1.y; csw[6] = t1.z; csw[7] = t1.w;
+                            const float cs_c = bf16_lo(csw[e]), cs_s = bf16_hi(csw[e]);
+                            ol[e] = p_rope(xl, -xh, cs_c, cs_s);
+                            oh[e] = p_rope(xh, xl, cs_c, cs_s);
+                        } else {
+                            ol[e] = xl; oh[e] = xh;
                         }
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            const float xl = round_bf16(__uint_as_float(lo[v8 * 8 + e]));  // the projection as bf16, like the unfused path
-                            const float xh = round_bf16(__uint_as_float(hi[v8 * 8 + e]));
-                            if (part < 2) {
-                                const float cs_c = bf16_lo(csw[e]), cs_s = bf16_hi(csw[e]);
-                                ol[e] = p_rope(xl, -xh, cs_c, cs_s);
-                                oh[e] = p_rope(xh, xl, cs_c, cs_s);
-                            } else {
-                                ol[e] = xl; oh[e] = xh;
-                            }
+                    }
+                    *box_slot<P_BOX>(buf, lane, j & 3) = make_uint4(pack_bf16(ol[0], ol[1]), pack_bf16(ol[2], ol[3]), pack_bf16(ol[4], ol[5]), pack_bf16(ol[6], ol[7]));
+                    *box_slot<P_BOX>(buf, lane, 4 + (j & 3)) = make_uint4(pack_bf16(oh[0], oh[1]), pack_bf16(oh[2], oh[3]), pack_bf16(oh[4], oh[5]), pack_bf16(oh[6], oh[7]));
+                    if ((j & 3) != 3) continue;
+                    __syncwarp();
+                    const int piece = lane & 7, at = (piece < 4 ? 0 : 64) + (j >> 2) * 32 + (piece & 3) * 8;
+#pragma unroll 4
+                    for (int i = 0; i < 8; ++i) {
+                        const int r = i * 4 + (lane >> 3), orow = row0 + r;
+                        if (!(orow < M && col_base < N)) continue;
+                        __nv_bfloat16* dst;
+                        if (part == 0) {
+                            dst = reinterpret_cast<__nv_bfloat16*>(ep.out) + (size_t)orow * ep.ld_out + col_base;
+                        } else {
+                            const int b = orow / ep.rope_S, t2 = orow - b * ep.rope_S;
+                            dst = (part == 1 ? ep.kcache : ep.vcache) + (((size_t)b * ep.rope_H + head) * ep.rope_Smax + t2) * 128;
                         }
-                        *reinterpret_cast<uint4*>(dst + v8 * 8) =
-                            make_uint4(pack_bf16(ol[0], ol[1]), pack_bf16(ol[2], ol[3]), pack_bf16(ol[4], ol[5]), pack_bf16(ol[6], ol[7]));
-                        *reinterpret_cast<uint4*>(dst + 64 + v8 * 8) =
-                            make_uint4(pack_bf16(oh[0], oh[1]), pack_bf16(oh[2], oh[3]), pack_bf16(oh[4], oh[5]), pack_bf16(oh[6], oh[7]));
+                        *reinterpret_cast<uint4*>(dst + at) = *box_slot<P_BOX>(buf, r, piece);
                     }
                 }
             } else {
-#pragma unroll 1
-                for (int c = half * (P_TN / 64); c < (half + 1) * (P_TN / 64); ++c) {
-                    uint32_t v[32];
-                    __syncwarp();
-                    tmem_ld_32x32(taddr_row + c * 32, v);
-                    tmem_ld_wait();
-                    const int col0 = n_blk * P_TN + c * 32;
-#pragma unroll
-                    for (int v8 = 0; v8 < 4; ++v8) {
-                        const int col = col0 + v8 * 8;
-                        if (!(row_ok && col < N)) continue;
-                        float x[8];
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) x[e] = __uint_as_float(v[v8 * 8 + e]);
-                        if (ep.bias != nullptr) {
-                            const uint4 b = *reinterpret_cast<const uint4*>(ep.bias + col);
-                            x[0] += bf16_lo(b.x); x[1] += bf16_hi(b.x); x[2] += bf16_lo(b.y); x[3] += bf16_hi(b.y);
-                            x[4] += bf16_lo(b.z); x[5] += bf16_hi(b.z); x[6] += bf16_lo(b.w); x[7] += bf16_hi(b.w);
-                        }
-                        if constexpr (ACT == ACT_QUICK_GELU) {
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) x[e] = p_quick_gelu(x[e]);
-                        } else if constexpr (ACT == ACT_GELU_ERF) {
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) x[e] = p_gelu_erf(x[e]);
-                        }
-                        if (ep.residual != nullptr) {
-                            const uint4 r = *reinterpret_cast<const uint4*>(ep.residual + (size_t)row * ep.ld_res + col);
-                            x[0] += bf16_lo(r.x); x[1] += bf16_hi(r.x); x[2] += bf16_lo(r.y); x[3] += bf16_hi(r.y);
-                            x[4] += bf16_lo(r.z); x[5] += bf16_hi(r.z); x[6] += bf16_lo(r.w); x[7] += bf16_hi(r.w);
-                        }
-                        if (ep.out_fp32) {
-                            float* op = reinterpret_cast<float*>(ep.out) + (size_t)row * ep.ld_out + col;
-                            if (ep.post != 0 || ep.accumulate != 0 || ep.alpha != 1.f) epi_post8(x, op, ep.post, ep.alpha, ep.accumulate);
-                            *reinterpret_cast<float4*>(op) = make_float4(x[0], x[1], x[2], x[3]);
-                            *reinterpret_cast<float4*>(op + 4) = make_float4(x[4], x[5], x[6], x[7]);
-                        } else {
-                            __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(ep.out) + (size_t)row * ep.ld_out + col;
-                            *reinterpret_cast<uint4*>(op) = make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]),
-                                                                       pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
-                        }
-                    }
-                }
+                const TileBox<P_BOX> box{&tmap_out, buf, lane, row0, M, N};
+                store_tile<ACT, P_BOX, 128, F32>(box, taddr, n_blk * P_TN + half * 128, ep, ready, drained);
             }
-            // this warp has read its part of accumulator stage `as`: tell the leader's MMA issuer
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(mapa_rank(smem_u32(&tmem_empty[as]), 0));
         }
+        if (lane == 0) bulk_wait_all();
     }
 
     __syncwarp();  // lanes 1..31 of the producer / MMA warps waited here: the cluster barrier below is .aligned
@@ -375,18 +346,20 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     }
 }
 
-template <int ACT>
+template <int ACT, bool F32 = false>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int K, const PairEpi& ep, cudaStream_t stream) {
     static bool attr_set = false;
-    auto kern = gemm_bf16_2cta_kernel<ACT>;
+    auto kern = gemm_bf16_2cta_kernel<ACT, F32>;
     if (!attr_set) {
         B2_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM));
         attr_set = true;
     }
+    CUtensorMap to = {};
+    if (ACT != ACT_ROPE_QKV && !F32) B2_TRY(make_tmap_out(&to, ep.out, M, ACT == ACT_SWIGLU || ACT == ACT_GLU ? N / 2 : N, ep.ld_out, P_BOX));
     const int tiles = ((M + P_TM - 1) / P_TM) * ((N + P_TN - 1) / P_TN);
     const int max_pairs = num_sms() / 2;
     const int pairs = tiles < max_pairs ? tiles : max_pairs;
-    B2_CUDA_CHECK(launch_pdl(kern, dim3(2 * pairs), dim3(P_THREADS), (size_t)P_SMEM, stream, ta, tb, M, N, K, ep));  // cluster dims (2,1,1) are a kernel attribute
+    B2_CUDA_CHECK(launch_pdl(kern, dim3(2 * pairs), dim3(P_THREADS), (size_t)P_SMEM, stream, ta, tb, to, M, N, K, ep));  // cluster dims (2,1,1) are a kernel attribute
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -424,9 +397,9 @@ int gemm_bf16_2cta(const GemmArgs& g, cudaStream_t stream) {
                      "gemm_2cta(rope_qkv): needs N = 3*H*128 with H*128 %% 256 == 0, M = B*S, bf16 output, no bias/residual");
     }
     switch (g.act) {
-        case ACT_NONE: return launch_pair<ACT_NONE>(ta, tb, g.M, g.N, g.K, ep, stream);
-        case ACT_QUICK_GELU: return launch_pair<ACT_QUICK_GELU>(ta, tb, g.M, g.N, g.K, ep, stream);
-        case ACT_GELU_ERF: return launch_pair<ACT_GELU_ERF>(ta, tb, g.M, g.N, g.K, ep, stream);
+        case ACT_NONE: return ep.out_fp32 ? launch_pair<ACT_NONE, true>(ta, tb, g.M, g.N, g.K, ep, stream) : launch_pair<ACT_NONE>(ta, tb, g.M, g.N, g.K, ep, stream);
+        case ACT_QUICK_GELU: return ep.out_fp32 ? launch_pair<ACT_QUICK_GELU, true>(ta, tb, g.M, g.N, g.K, ep, stream) : launch_pair<ACT_QUICK_GELU>(ta, tb, g.M, g.N, g.K, ep, stream);
+        case ACT_GELU_ERF: return ep.out_fp32 ? launch_pair<ACT_GELU_ERF, true>(ta, tb, g.M, g.N, g.K, ep, stream) : launch_pair<ACT_GELU_ERF>(ta, tb, g.M, g.N, g.K, ep, stream);
         case ACT_SWIGLU: return launch_pair<ACT_SWIGLU>(ta, tb, g.M, g.N, g.K, ep, stream);
         case ACT_GLU: return launch_pair<ACT_GLU>(ta, tb, g.M, g.N, g.K, ep, stream);
         case ACT_ROPE_QKV: return launch_pair<ACT_ROPE_QKV>(ta, tb, g.M, g.N, g.K, ep, stream);

@@ -15,6 +15,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "tile_store.cuh"
 
 namespace b2 {
 
@@ -73,6 +74,26 @@ int make_tmap_bf16(CUtensorMap* map, const void* ptr, int64_t rows, int64_t cols
     return 0;
 }
 
+int make_tmap_out(CUtensorMap* map, const void* ptr, int64_t rows, int64_t cols, int64_t ld, int box_bytes) {
+    PFN_encodeTiled fn = get_encode_fn();
+    if (fn == nullptr) {
+        set_error("cuTensorMapEncodeTiled entry point unavailable");
+        return -2;
+    }
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)(ld * 2)};
+    cuuint32_t box[2] = {(cuuint32_t)(box_bytes / 2), 32u};
+    cuuint32_t estr[2] = {1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, box_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                    CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        set_error("cuTensorMapEncodeTiled(output) failed (%d) rows=%lld cols=%lld ld=%lld", (int)r, (long long)rows, (long long)cols, (long long)ld);
+        return -2;
+    }
+    return 0;
+}
+
 // 2D byte tensor (fp8 operands) row-major [rows, cols] with row pitch ld bytes; box = [box_rows, 128 B]. gemm_skinny.cu.
 int make_tmap_u8(CUtensorMap* map, const void* ptr, int64_t rows, int64_t cols, int64_t ld, int box_rows) {
     PFN_encodeTiled fn = get_encode_fn();
@@ -111,10 +132,14 @@ template <int BN>
 struct GemmCfg {
     static constexpr int B_TILE_BYTES = BN * BK * 2;
     static constexpr int STAGE_BYTES = A_TILE_BYTES + B_TILE_BYTES;
-    static constexpr int STAGES = (BN == 256) ? 4 : (BN == 192 ? 5 : (BN == 128 ? 7 : 9));
+    static constexpr int STAGES = (BN == 256) ? 4 : (BN == 192 ? 5 : (BN == 128 ? 6 : 8));
     static constexpr int ACC_STRIDE = (BN == 192) ? 256 : BN;      // TMEM columns between the two accumulator stages
     static constexpr int TMEM_COLS = 2 * ACC_STRIDE;               // power of two (128 / 256 / 512)
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
+    // Bytes of a row of an epilogue warp's box (tile_store.cuh): its half of the tile is whole boxes of 64 bf16 columns, or of 32
+    static constexpr int BOX = BN % 128 == 0 ? 128 : 64, BOX_GLU = BN == 256 ? 128 : 64;
+    static constexpr int BOX_BYTES = kNumEpiWarps * 32 * BOX;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + BOX_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
+    static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of one CTA");
 };
 
 struct EpiParams {
@@ -135,16 +160,15 @@ struct EpiParams {
     int a_bytes = BM * BK * 2;   // of A per k-block: gemm_a_rows(M) rows
 };
 
-__device__ __forceinline__ float act_quick_gelu(float x) { return __fdividef(x, 1.0f + __expf(-1.702f * x)); }
 __device__ __forceinline__ float act_gelu_erf(float x) {
     return 0.5f * x * (1.0f + erff(x * 0.70710678118654752440f));
 }
 __device__ __forceinline__ float act_silu(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
 
-template <int BN, int ACT>
+template <int BN, int ACT, bool F32>
 __global__ void __launch_bounds__(kNumThreads, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                         const __grid_constant__ CUtensorMap tmap_b, int M, int N, int K,
+                         const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_out, int M, int N, int K,
                          EpiParams ep) {
     using Cfg = GemmCfg<BN>;
     constexpr int STAGES = Cfg::STAGES;
@@ -153,7 +177,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     // SWIZZLE_128B tiles need 1024-byte alignment
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES);
+    uint8_t* boxes = smem + STAGES * Cfg::STAGE_BYTES;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(boxes + Cfg::BOX_BYTES);
     uint64_t* full_bar = bars;                    // [STAGES]
     uint64_t* empty_bar = bars + STAGES;          // [STAGES]
     uint64_t* tmem_full = bars + 2 * STAGES;      // [2]
@@ -182,6 +207,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tmap_a);
         tma_prefetch_desc(&tmap_b);
+        if constexpr (!F32) tma_prefetch_desc(&tmap_out);
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&full_bar[s], 1);
             mbar_init(&empty_bar[s], 1);
@@ -309,106 +335,32 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
             const int as = local & 1;
             const uint32_t aphase = (local >> 1) & 1;
             ++local;
-            mbar_wait(&tmem_full[as], aphase);
-            tc_fence_after();
-            const int row = m_blk * BM + q * 32 + lane;
-            const bool row_ok = row < M;
-            const uint32_t taddr_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + as * Cfg::ACC_STRIDE;
-
+            const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + as * Cfg::ACC_STRIDE;
+            const int row0 = m_blk * BM + q * 32;
+            uint8_t* buf = boxes + (warp - 2) * 32 * Cfg::BOX;
+            auto ready = [&] { mbar_wait(&tmem_full[as], aphase); tc_fence_after(); };
+            auto drained = [&] {   // this warp's reads of the accumulator stage are complete: hand it back
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&tmem_empty[as]);
+            };
             if constexpr (ACT == ACT_SWIGLU || ACT == ACT_GLU) {
                 // W rows are block-interleaved (ACT_GLU: by the loads): within each 128-col group, cols [0,64) = gate, [64,128) = up
                 // for the same 64 output channels. out is [M, N/2].
                 static_assert(BN % 128 == 0, "swiglu needs BN multiple of 128");
-#pragma unroll 1
-                for (int it = half * (BN / 128); it < (half + 1) * (BN / 128); ++it) {
-                    {
-                        const int g = it >> 1, j = it & 1;
-                        uint32_t vg[32], vu[32];
-                        __syncwarp();
-                        tmem_ld_32x32(taddr_row + g * 128 + j * 32, vg);
-                        tmem_ld_32x32(taddr_row + g * 128 + 64 + j * 32, vu);
-                        tmem_ld_wait();
-                        const int ocol0 = (n_blk * BN) / 2 + g * 64 + j * 32;
-                        if (row_ok && ocol0 < N / 2) {
-                            __nv_bfloat16* op =
-                                reinterpret_cast<__nv_bfloat16*>(ep.out) + (size_t)row * ep.ld_out + ocol0;
-#pragma unroll
-                            for (int v8 = 0; v8 < 4; ++v8) {
-                                uint32_t pk[4];
-#pragma unroll
-                                for (int e = 0; e < 4; ++e) {
-                                    float g0 = __uint_as_float(vg[v8 * 8 + 2 * e]);
-                                    float g1 = __uint_as_float(vg[v8 * 8 + 2 * e + 1]);
-                                    float u0 = __uint_as_float(vu[v8 * 8 + 2 * e]);
-                                    float u1 = __uint_as_float(vu[v8 * 8 + 2 * e + 1]);
-                                    if constexpr (ACT == ACT_GLU) pk[e] = pack_bf16(glu_act(g0, u0, ep.glu), glu_act(g1, u1, ep.glu));
-                                    else pk[e] = pack_bf16(act_silu(g0) * u0, act_silu(g1) * u1);
-                                }
-                                if (ACT == ACT_SWIGLU || ocol0 + v8 * 8 < N / 2)
-                                    *reinterpret_cast<uint4*>(op + v8 * 8) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                            }
-                        }
-                    }
-                }
+                constexpr int COLS = BN / 4;       // BN 256: a warp takes one group, BN 128: half of it
+                const int c = half * COLS;
+                const TileBox<Cfg::BOX_GLU> box{&tmap_out, buf, lane, row0, M, N / 2};
+                store_glu_tile<Cfg::BOX_GLU, COLS, ACT == ACT_GLU ? 8 : 32>(box, taddr + (c >> 6) * 128 + (c & 63), n_blk * (BN / 2) + c, ready, drained, [&](float g, float u) {
+                    if constexpr (ACT == ACT_GLU) return glu_act(g, u, ep.glu);
+                    else return act_silu(g) * u;
+                });
             } else {
-#pragma unroll 1
-                for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
-                    uint32_t v[32];
-                    __syncwarp();
-                    tmem_ld_32x32(taddr_row + c * 32, v);
-                    tmem_ld_wait();
-                    const int col0 = n_blk * BN + c * 32;
-#pragma unroll
-                    for (int v8 = 0; v8 < 4; ++v8) {
-                        const int col = col0 + v8 * 8;
-                        // N % 8 == 0 is enforced on the host; no early-outs here: the tcgen05.ld above is
-                        // .sync.aligned, so the warp must stay converged across loop iterations
-                        if (!(row_ok && col < N)) continue;
-                        float x[8];
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) x[e] = __uint_as_float(v[v8 * 8 + e]);
-                        if (ep.bias != nullptr) {
-                            const uint4 b = *reinterpret_cast<const uint4*>(ep.bias + col);
-                            x[0] += bf16_lo(b.x); x[1] += bf16_hi(b.x);
-                            x[2] += bf16_lo(b.y); x[3] += bf16_hi(b.y);
-                            x[4] += bf16_lo(b.z); x[5] += bf16_hi(b.z);
-                            x[6] += bf16_lo(b.w); x[7] += bf16_hi(b.w);
-                        }
-                        if constexpr (ACT == ACT_QUICK_GELU) {
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) x[e] = act_quick_gelu(x[e]);
-                        } else if constexpr (ACT == ACT_GELU_ERF) {
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) x[e] = act_gelu_erf(x[e]);
-                        }
-                        if (ep.residual != nullptr) {
-                            const uint4 r = *reinterpret_cast<const uint4*>(
-                                ep.residual + (size_t)row * ep.ld_res + col);
-                            x[0] += bf16_lo(r.x); x[1] += bf16_hi(r.x);
-                            x[2] += bf16_lo(r.y); x[3] += bf16_hi(r.y);
-                            x[4] += bf16_lo(r.z); x[5] += bf16_hi(r.z);
-                            x[6] += bf16_lo(r.w); x[7] += bf16_hi(r.w);
-                        }
-                        if (ep.out_fp32) {
-                            float* op = reinterpret_cast<float*>(ep.out) + (size_t)row * ep.ld_out + col;
-                            if (ep.post != 0 || ep.accumulate != 0 || ep.alpha != 1.f) epi_post8(x, op, ep.post, ep.alpha, ep.accumulate);
-                            *reinterpret_cast<float4*>(op) = make_float4(x[0], x[1], x[2], x[3]);
-                            *reinterpret_cast<float4*>(op + 4) = make_float4(x[4], x[5], x[6], x[7]);
-                        } else {
-                            __nv_bfloat16* op =
-                                reinterpret_cast<__nv_bfloat16*>(ep.out) + (size_t)row * ep.ld_out + col;
-                            *reinterpret_cast<uint4*>(op) =
-                                make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]),
-                                           pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
-                        }
-                    }
-                }
+                const TileBox<Cfg::BOX> box{&tmap_out, buf, lane, row0, M, N};
+                store_tile<ACT, Cfg::BOX, BN / 2, F32>(box, taddr + half * (BN / 2), n_blk * BN + half * (BN / 2), ep, ready, drained);
             }
-            // all TMEM reads of this accumulator stage are complete (wait::ld above): hand it back
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tmem_empty[as]);
         }
+        if (lane == 0) bulk_wait_all();
     }
 
     tc_fence_before();
@@ -616,19 +568,22 @@ projector_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
 // ---------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------
-template <int BN, int ACT>
+template <int BN, int ACT, bool F32 = false>
 int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int K, const EpiParams& ep,
                 cudaStream_t stream) {
     using Cfg = GemmCfg<BN>;
+    constexpr bool GLU = ACT == ACT_SWIGLU || ACT == ACT_GLU;
+    CUtensorMap to = {};
+    if (!F32) B2_TRY(make_tmap_out(&to, ep.out, M, GLU ? N / 2 : N, ep.ld_out, GLU ? Cfg::BOX_GLU : Cfg::BOX));
     static bool attr_set = false;
-    auto kern = gemm_bf16_tcgen05_kernel<BN, ACT>;
+    auto kern = gemm_bf16_tcgen05_kernel<BN, ACT, F32>;
     if (!attr_set) {
         B2_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
         attr_set = true;
     }
     const int num_tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
     const int grid = num_tiles < num_sms() ? num_tiles : num_sms();
-    B2_CUDA_CHECK(launch_pdl(kern, dim3(grid), dim3(kNumThreads), (size_t)Cfg::SMEM_BYTES, stream, ta, tb, M, N, K, ep));
+    B2_CUDA_CHECK(launch_pdl(kern, dim3(grid), dim3(kNumThreads), (size_t)Cfg::SMEM_BYTES, stream, ta, tb, to, M, N, K, ep));
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -637,9 +592,9 @@ template <int BN>
 int dispatch_act(int act, const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int K,
                  const EpiParams& ep, cudaStream_t stream) {
     switch (act) {
-        case ACT_NONE: return launch_gemm<BN, ACT_NONE>(ta, tb, M, N, K, ep, stream);
-        case ACT_QUICK_GELU: return launch_gemm<BN, ACT_QUICK_GELU>(ta, tb, M, N, K, ep, stream);
-        case ACT_GELU_ERF: return launch_gemm<BN, ACT_GELU_ERF>(ta, tb, M, N, K, ep, stream);
+        case ACT_NONE: return ep.out_fp32 ? launch_gemm<BN, ACT_NONE, true>(ta, tb, M, N, K, ep, stream) : launch_gemm<BN, ACT_NONE>(ta, tb, M, N, K, ep, stream);
+        case ACT_QUICK_GELU: return ep.out_fp32 ? launch_gemm<BN, ACT_QUICK_GELU, true>(ta, tb, M, N, K, ep, stream) : launch_gemm<BN, ACT_QUICK_GELU>(ta, tb, M, N, K, ep, stream);
+        case ACT_GELU_ERF: return ep.out_fp32 ? launch_gemm<BN, ACT_GELU_ERF, true>(ta, tb, M, N, K, ep, stream) : launch_gemm<BN, ACT_GELU_ERF>(ta, tb, M, N, K, ep, stream);
         default: break;
     }
     set_error("gemm: unsupported activation %d", act);
