@@ -13,8 +13,11 @@
 // window may keep the sequence's first positions visible (mask_keep): the visible keys are then two ranges, [0, keep) and the
 // window, and the tiles of the gap between them are never staged. Value heads may be fewer than key heads (Gv < G: key head g
 // reads value head g mod Gv), which is how the two maps of differential attention share one set of values.
-// Prompt portions whose sizes allow it leave for attention_split.cu; decode steps, short portions and wide heads stay here.
+// Prompt portions whose sizes allow it leave for attention_split.cu; decode steps (attn_step_kernel, or the tiled kernel with its keys cut up), short
+// portions and wide heads stay here.
 #include <math.h>
+
+#include <algorithm>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -433,6 +436,161 @@ __global__ void __launch_bounds__(512) attn_merge_kernel(BiasAttnArgs a) {
     }
 }
 
+// ---- one row per slot (a decode step): the keys of a (row, key/value head) are shared out over a cluster of C CTAs and, inside them, over 16
+// warps; partial results meet in shared memory, then in the cluster's, and leave in the same launch. A warp takes 8 keys at a time: the loads of
+// their key and value rows (16 bytes a lane) all start before the first product, four keys side by side with eight lanes each for the scores.
+// What bounds it is latency: the chain launch - position - key rows - exponentials - two meetings. The tiled kernel with its key splits staged 32 keys
+// at a time (load, barrier, products, barrier) and met in a second launch. A step of one layer of width 1024 (us, before -> now; keys, slots):
+// 8 key/value heads 41.1 -> 33.0 (500, 1), 86 -> 45 (8000, 1), 68 -> 37 (500, 8), 276 -> 77 (4000, 8); 2 of them 41.1 -> 35.2 (500, 1).
+constexpr int ST_WARPS = 16, ST_KEYS = 8, ST_DK = 128, ST_DV = 128;
+
+__device__ __forceinline__ void st_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float st_ld_remote(const float* p, int rank) {
+    uint32_t at;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+    return v;
+}
+
+// grid (C, G * chunks, rows), clusters along x; NH >= query heads of a chunk
+template <int NH>
+__global__ void __launch_bounds__(ST_WARPS * 32, 1) attn_step_kernel(BiasAttnArgs a, int C) {
+    pdl_enter_late();
+    __shared__ __align__(16) float sq[NH * ST_DK];
+    __shared__ __align__(16) float so[ST_WARPS][NH][ST_DV];
+    __shared__ float sm[ST_WARPS][NH], sl[ST_WARPS][NH];
+    __shared__ float po[NH][ST_DV], pm[NH], pl[NH];     // this CTA's share, read by the cluster
+    const int rank = blockIdx.x, r = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int HGall = a.H / a.G, chunks = (HGall + NH - 1) / NH;
+    const int g = blockIdx.y / chunks, h0 = g * HGall + (blockIdx.y % chunks) * NH, HG = min(NH, g * HGall + HGall - h0);
+    const int dk = a.dk, dv = a.dv;
+    const int pos = a.row_pos[r], slot = a.row_slot[r];
+    if (pos < 0) return;                                // (the whole cluster)
+    for (int e = threadIdx.x; e < NH * dk / 4; e += ST_WARPS * 32)
+        reinterpret_cast<float4*>(sq)[e] = e < HG * dk / 4 ? reinterpret_cast<const float4*>(a.q + (size_t)r * a.ldq + (size_t)h0 * dk)[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+    // visible keys: [0, nA), the kept first positions in front of the window, then [first, pos]; numbered through, this CTA's are [k0, k1)
+    const int first = mask_first(pos, a.mask_kind, a.mask_size), nA = a.mask_kind == MASK_WINDOW ? min(a.mask_keep, first) : 0;
+    const int n = nA + pos + 1 - first, per = (n + C - 1) / C, k0 = min(n, rank * per), k1 = min(n, k0 + per);
+    const int Gv = a.Gv > 0 ? a.Gv : a.G;
+    const float* K = a.kcache + ((size_t)slot * a.G + g) * a.Smax * dk;
+    const float* V = a.vcache + ((size_t)slot * Gv + g % Gv) * a.Smax * dv;
+    const int kg = lane >> 3, kl = (lane & 7) * 4;
+    float m[NH], l[NH];
+    float4 o[NH];
+#pragma unroll
+    for (int h = 0; h < NH; ++h) { m[h] = -INFINITY; l[h] = 0.f; o[h] = make_float4(0.f, 0.f, 0.f, 0.f); }
+    __syncthreads();
+#pragma unroll 1
+    for (int b = k0 + warp * ST_KEYS; b < k1; b += ST_WARPS * ST_KEYS) {
+        float4 kf[2][ST_DK / 32], vf[ST_KEYS];
+        int at[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int i = min(b + j * 4 + kg, k1 - 1);   // (a key that is not there: the last one, its probability is 0)
+            at[j] = i < nA ? i : first + i - nA;
+#pragma unroll
+            for (int c = 0; c < ST_DK / 32; ++c)
+                kf[j][c] = c * 32 < dk ? *reinterpret_cast<const float4*>(K + (size_t)at[j] * dk + c * 32 + kl) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int e = 0; e < ST_KEYS; ++e) {
+            const int i = min(b + e, k1 - 1), v = i < nA ? i : first + i - nA;
+            vf[e] = lane * 4 < dv && b + e < k1 ? *reinterpret_cast<const float4*>(V + (size_t)v * dv + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int h = 0; h < NH; ++h) {
+            float s[2], p[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                float acc = 0.f;
+#pragma unroll
+                for (int c = 0; c < ST_DK / 32; ++c) {
+                    if (c * 32 >= dk) continue;
+                    const float4 q = *reinterpret_cast<const float4*>(sq + h * dk + c * 32 + kl);
+                    acc = fmaf(q.x, kf[j][c].x, acc); acc = fmaf(q.y, kf[j][c].y, acc); acc = fmaf(q.z, kf[j][c].z, acc); acc = fmaf(q.w, kf[j][c].w, acc);
+                }
+#pragma unroll
+                for (int x = 1; x < 8; x <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, x);
+                acc *= a.scale;
+                if (a.softcap > 0.f) acc = a.softcap * tanhf(acc / a.softcap);
+                if (a.rel != nullptr && h < HG) acc += a.rel[(size_t)a.bucket_of[pos - at[j]] * a.H + h0 + h];
+                s[j] = b + j * 4 + kg < k1 ? acc : -INFINITY;
+            }
+            float mx = fmaxf(s[0], s[1]);
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+            mx = fmaxf(m[h], mx);
+            const float ref = mx == -INFINITY ? 0.f : mx;   // (only scores of minus infinity so far: they weigh nothing)
+            const float corr = expf(m[h] - ref);
+            m[h] = mx;
+            p[0] = expf(s[0] - ref);
+            p[1] = expf(s[1] - ref);
+            float sum = p[0] + p[1];
+            sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+            l[h] = fmaf(l[h], corr, sum);
+            o[h].x *= corr; o[h].y *= corr; o[h].z *= corr; o[h].w *= corr;
+#pragma unroll
+            for (int e = 0; e < ST_KEYS; ++e) {
+                const float pe = __shfl_sync(0xffffffffu, p[e >> 2], (e & 3) * 8);
+                o[h].x = fmaf(pe, vf[e].x, o[h].x); o[h].y = fmaf(pe, vf[e].y, o[h].y); o[h].z = fmaf(pe, vf[e].z, o[h].z); o[h].w = fmaf(pe, vf[e].w, o[h].w);
+            }
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < NH; ++h) {
+        if (lane * 4 < dv) *reinterpret_cast<float4*>(&so[warp][h][lane * 4]) = o[h];
+        if (lane == 0) { sm[warp][h] = m[h]; sl[warp][h] = l[h]; }
+    }
+    __syncthreads();
+    if (warp < NH) {   // the warps' weights, and the CTA's maximum and sum
+        const float mw = lane < ST_WARPS ? sm[lane][warp] : -INFINITY, lw = lane < ST_WARPS ? sl[lane][warp] : 0.f;
+        const float mx = warp_max(lw != 0.f ? mw : -INFINITY);
+        const float w = lw != 0.f ? expf(mw - mx) : 0.f, sum = warp_sum(lw * w);
+        if (lane < ST_WARPS) sm[lane][warp] = w;
+        if (lane == 0) { pm[warp] = mx; pl[warp] = sum; }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < NH * dv; e += ST_WARPS * 32) {
+        const int h = e / dv, d = e - h * dv;
+        float acc = 0.f;
+#pragma unroll
+        for (int w = 0; w < ST_WARPS; ++w) acc = fmaf(so[w][h][d], sm[w][h], acc);
+        po[h][d] = acc;
+    }
+    st_cluster_sync();
+    const int share = (HG * dv + C - 1) / C;
+    for (int e = rank * share + threadIdx.x; e < min(HG * dv, (rank + 1) * share); e += ST_WARPS * 32) {
+        const int h = e / dv, d = e - h * dv, head = h0 + h;
+        float mc[8], lc[8], oc[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const int from = c < C ? c : rank;
+            mc[c] = st_ld_remote(&pm[h], from); lc[c] = st_ld_remote(&pl[h], from); oc[c] = st_ld_remote(&po[h][d], from);
+            if (c >= C) lc[c] = 0.f;
+        }
+        const bool has_sink = a.sink != nullptr || a.sink_fixed;
+        float mx = a.sink != nullptr ? a.sink[head] : (a.sink_fixed ? a.sink_value : -INFINITY);
+        const float sk = mx;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) mx = lc[c] != 0.f ? fmaxf(mx, mc[c]) : mx;
+        float sum = has_sink ? expf(sk - mx) : 0.f, acc = 0.f;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const float w = lc[c] != 0.f ? expf(mc[c] - mx) : 0.f;   // (a share without keys, or a sum that is NaN: NaN != 0)
+            sum = fmaf(lc[c], w, sum);
+            acc = lc[c] != 0.f ? fmaf(oc[c], w, acc) : acc;
+        }
+        const float inv = a.head_gate != nullptr ? 1.f / (sum * (1.f + expf(-a.head_gate[(size_t)r * a.ldg + head]))) : 1.f / sum;
+        store_out(a, r, head, d, acc * inv);
+    }
+    st_cluster_sync();   // no share goes away while another CTA reads it
+}
+
 int check_args(const BiasAttnArgs& a, const char* who) {
     B2_CHECK_ARG(a.q && a.kcache && a.vcache && a.row_slot && a.row_pos && a.rows > 0, "%s: null argument", who);
     B2_CHECK_ARG(a.H > 0 && a.G > 0 && a.H % a.G == 0, "%s: %d query heads cannot share %d key/value heads", who, a.H, a.G);
@@ -467,11 +625,49 @@ int launch_tile(const BiasAttnArgs& a, int QT, int HC, dim3 grid, size_t smem, c
     return 0;
 }
 
+// CTAs a cluster of attn_step_kernel: as many as the SMs hold at once
+static int step_cluster(const BiasAttnArgs& a, int units) {
+    int C = 8;
+    while (C > 1 && (long long)a.rows * units * C > num_sms()) C /= 2;
+    return C;
+}
+// One row per slot, caches of heads that 16-byte loads of 32 lanes cover. Few key/value heads fill few SMs: from some thousand keys a CTA on
+// the tiled kernel's key splits (up to 64) read them faster. One slot, 2 key/value heads, 16 CTAs: 8000 keys 61.9 us tiled, 59.3 here; 16000
+// 86.1 / 84.4; 32000 133 / 141.
+static bool attn_step_fits(const BiasAttnArgs& a) {
+    const int heads = a.H / a.G, units = a.G * ((heads + 3) / 4);
+    const long long keys = a.mask_kind == MASK_WINDOW ? (long long)a.mask_size + a.mask_keep : a.mask_kind == MASK_CHUNK ? a.mask_size : a.Smax;
+    if (std::min<long long>(keys, a.Smax) > 1024ll * a.rows * units * step_cluster(a, units)) return false;
+    const auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+    return a.tile_rows == 1 && a.vcache != a.kcache && a.kv_row_stride == 0 && a.dk % 32 == 0 && a.dk <= ST_DK && a.dv % 4 == 0 && a.dv <= ST_DV &&
+           a.ldq % 4 == 0 && aligned(a.q) && aligned(a.kcache) && aligned(a.vcache);
+}
+template <int NH>
+int launch_step(const BiasAttnArgs& a, cudaStream_t st) {
+    const int HG = a.H / a.G, units = a.G * ((HG + NH - 1) / NH);
+    const int C = step_cluster(a, units);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(C, units, a.rows); cfg.blockDim = dim3(ST_WARPS * 32); cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C; attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    cfg.attrs = attr; cfg.numAttrs = 2;
+    B2_CUDA_CHECK(cudaLaunchKernelEx(&cfg, attn_step_kernel<NH>, a, C));
+    B2_LAUNCH_CHECK();
+    return 0;
+}
+
 int attn_bias_f32(const BiasAttnArgs& a, cudaStream_t st) {
     B2_TRY(check_args(a, "attn_bias"));
     B2_CHECK_ARG((a.out || a.out16) && (a.rel == nullptr || a.bucket_of != nullptr), "attn_bias: null argument");
     B2_CHECK_ARG(a.nsplit >= 1 && a.nsplit <= 64 && (a.nsplit == 1 || a.partial != nullptr), "attn_bias: 1..64 key splits, with scratch");
     if (attn_split_fits(a)) return attn_split_f32(a, st);
+    if (attn_step_fits(a)) {
+        const int heads = a.H / a.G;
+        return heads == 1 ? launch_step<1>(a, st) : heads == 2 ? launch_step<2>(a, st) : launch_step<4>(a, st);
+    }
     const int warps = a.rows * a.H;
     const bool vec = a.dk % 4 == 0 && (reinterpret_cast<uintptr_t>(a.kcache) & 15) == 0;
     const int HG = a.H / a.G;
