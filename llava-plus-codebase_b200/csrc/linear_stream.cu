@@ -1,6 +1,6 @@
 // Linears of a handful of rows (decode steps of 1..16 slots, tails of prompts) on bf16 weights: out[M, N] = A[M, K] W[N, K]^T with the fp32
 // epilogue of linear_f32. A weight is used M times at most, so the kernel is a stream of weights and everything else stays out of its way:
-//   * a CTA of 8 warps owns tiles of 16 output columns; its warps share a tile's K in units of 128, so that even the smallest matrix of a
+//   * a CTA of 8 or 16 warps owns tiles of 16 output columns; its warps share a tile's K in units of 128, so that even the smallest matrix of a
 //     model is spread over all SMs with its whole stream in flight, and the partial sums meet in shared memory in a fixed order;
 //   * weights go from global memory straight into registers, 16 bytes per lane, in the order in which the tensor-core fragment wants them: the
 //     sum over k may be taken in any order, so a lane's 8 consecutive k (of 32) are the fragment's k of two steps of 16 for A and B alike;
@@ -19,7 +19,7 @@
 namespace b2 {
 namespace {
 
-constexpr int LS_WARPS = 8, LS_UNIT = 128, LS_N = 16;
+constexpr int LS_UNIT = 128, LS_N = 16;
 
 __device__ __forceinline__ void mma_16x8x16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -27,9 +27,9 @@ __device__ __forceinline__ void mma_16x8x16(float (&c)[4], uint32_t a0, uint32_t
 }
 
 // NT: column tiles of 8 rows of A (0: one row on the FMA pipe). A16: A lies there as bf16 rows of pitch K. GLU: a tile is 8 outputs of a gated unit,
-// rows 0..7 their gate weights and 8..15 their up weights.
-template <int NT, bool A16, bool GLU>
-__global__ void __launch_bounds__(LS_WARPS * 32, 2) linear_stream_kernel(LinearArgs a) {
+// rows 0..7 their gate weights and 8..15 their up weights. An SM holds 16 warps: one CTA of 16, or two of 8.
+template <int NT, bool A16, bool GLU, int LS_WARPS>
+__global__ void __launch_bounds__(LS_WARPS * 32, 16 / LS_WARPS) linear_stream_kernel(LinearArgs a) {
     constexpr int COLS = NT == 0 ? 1 : 8 * NT, OUTS = GLU ? LS_N / 2 : LS_N;   // outputs per tile
     __shared__ float red[LS_WARPS][LS_N][COLS + (NT == 0 ? 0 : 1)];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = lane >> 2, kq = (lane & 3) * 8;
@@ -163,8 +163,13 @@ __global__ void __launch_bounds__(LS_WARPS * 32, 2) linear_stream_kernel(LinearA
 
 template <int NT, bool A16, bool GLU>
 int launch_stream(const LinearArgs& a, cudaStream_t st) {
-    const int tiles = GLU ? (a.N + LS_N / 2 - 1) / (LS_N / 2) : (a.N + LS_N - 1) / LS_N;
-    B2_CUDA_CHECK(launch_pdl(linear_stream_kernel<NT, A16, GLU>, dim3(std::min(tiles, 2 * num_sms())), dim3(LS_WARPS * 32), 0, st, a));
+    const int outs = GLU ? LS_N / 2 : LS_N, tiles = (a.N + outs - 1) / outs, units = (a.K + LS_UNIT - 1) / LS_UNIT;
+    // The longest chain of units that a warp walks, with two CTAs of 8 warps on an SM and with one of 16: the shorter one. (48 steps of the
+    // four-layer model above, one slot: gate and up of 5120 x 2048 6 / 5 units, down 5 / 3, the rest 2 / 2 and 2 / 1: 10.32 -> 9.87 ms;
+    // eight slots 12.74 -> 12.55.)
+    const int chain8 = ((tiles + 2 * num_sms() - 1) / (2 * num_sms())) * ((units + 7) / 8), chain16 = ((tiles + num_sms() - 1) / num_sms()) * ((units + 15) / 16);
+    if (chain16 <= chain8) B2_CUDA_CHECK(launch_pdl(linear_stream_kernel<NT, A16, GLU, 16>, dim3(std::min(tiles, num_sms())), dim3(512), 0, st, a));
+    else B2_CUDA_CHECK(launch_pdl(linear_stream_kernel<NT, A16, GLU, 8>, dim3(std::min(tiles, 2 * num_sms())), dim3(256), 0, st, a));
     B2_LAUNCH_CHECK();
     return 0;
 }
