@@ -10,14 +10,15 @@
 // have an accumulator of their own, and the weighted sum of values leaves TMEM after every key tile and is added up in fp32 registers. Scores, bias, soft-cap, mask, maximum, exponential, denominator: fp32 on the
 // CUDA cores, as before.
 //
-// What bounds it: the tensor pipe (12 products of a tile where bf16 attention has 2; 38 % active) and, beside it, the chain of a tile through
-// the softmax warps. 2048 rows, 16 heads of 128 on 4 key/value heads: window of 1024 + 4 kept positions 1061 -> 129 us (attn_tile_kernel -> this,
-// 100 TFLOP/s of fp32 arithmetic), no window, 1536 rows on 16 key/value heads 947 -> 103 us; cutting the keys and values: 4 us of that call.
+// What bounds it: the products (12 of a tile where bf16 attention has 2), as fast as they are issued: walked by one lane an instruction took 80-107 clk
+// for 48-64 of work, by the whole warp with an elected lane less (window 129 -> 106 us). Then the chain of a tile through the softmax warps. 2048
+// rows, 16 heads of 128 on 4 key/value heads: window of 1024 + 4 kept positions 1061 -> 106 us (attn_tile_kernel -> this), no window, 1536 rows on
+// 16 key/value heads 947 -> 84 us; cutting the keys and values: 4 us of that call.
 // Error of one fp32 layer against 64 bits, old -> new: 5.0e-7 -> 4.7e-7 at 17 rows, 7.1e-7 -> 5.9e-7 at 333, 8.6e-7 -> 6.5e-7 at 2048.
 //   1. attn_split_kv_kernel cuts the visible keys and values of the call into parts once (they are read by every query tile);
 //   2. attn_split_kernel: CTA = 128 (row, head) pairs of ONE key/value head (rows x the group's query heads, so that a key tile serves
-//      all of them), warp 0 TMA producer, warp 1 MMA issuer, warps 2..9 softmax: two threads per pair, each half of a tile's keys and half
-//      of the value columns. S is double-buffered in TMEM: S(t+1) runs while softmax(t) does, O(t) while softmax(t+1) does. P goes to TMEM
+//      all of them), warp 0 TMA producer, warp 1 MMA issuer, warps 2.. softmax: two or four threads per pair, each its share of a tile's
+//      keys and of the value columns. S is double-buffered in TMEM: S(t+1) runs while softmax(t) does, O(t) while softmax(t+1) does. P goes to TMEM
 //      as the A operand of the second product.
 // Key tiles of 64 for key sizes up to 128; the 192 sizes (latent attention with a rotated part) leave room for 32.
 #include <cuda.h>
@@ -49,7 +50,7 @@ int make_tmap_parts(CUtensorMap* map, const void* ptr, int pitch, int64_t nkeys,
 
 namespace {
 
-constexpr int SP_M = 128, SP_THREADS = 320, SP_SLAB_Q = SP_M * 128;
+constexpr int SP_M = 128, SP_SLAB_Q = SP_M * 128, FEW_KEYS = 256;
 
 __device__ __forceinline__ int split_first(int pos, int kind, int size) {   // first position a row at `pos` sees (kept first positions aside)
     if (kind == MASK_WINDOW) return max(0, pos - size + 1);
@@ -93,21 +94,16 @@ __device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint64_t b, uint
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
         ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t t, float* v) {
-    uint32_t u[16];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]), "=r"(u[9]),
-                   "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
-                 : "r"(t) : "memory");
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(u[i]);
-}
 __device__ __forceinline__ void tmem_st8(uint32_t t, const uint32_t* v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                  ::"r"(t), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
+__device__ __forceinline__ void tmem_st4(uint32_t t, const uint32_t* v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(t), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
 __device__ __forceinline__ void tmem_st_done() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void softmax_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+template <int SOFT>
+__device__ __forceinline__ void softmax_sync() { asm volatile("bar.sync 1, %0;" ::"n"(32 * SOFT) : "memory"); }
 
 // MN-major operand of 128-byte rows (64 entries of the row per slab), SWIZZLE_128B; lbo: bytes between the slabs
 __device__ __forceinline__ uint64_t make_mn_desc(uint32_t addr, uint32_t lbo) {
@@ -123,7 +119,7 @@ struct SplitParams {
 template <int DKS, int DVS, int KT>
 struct SplitCfg {
     static constexpr int Q_BYTES = 3 * DKS * SP_SLAB_Q, K_BYTES = 3 * DKS * KT * 128, V_BYTES = 3 * DVS * KT * 128;
-    static constexpr int SMEM = Q_BYTES + K_BYTES + V_BYTES + 4 * SP_M * 4 + 128 + 1024;
+    static constexpr int SMEM = Q_BYTES + K_BYTES + V_BYTES + 8 * SP_M * 4 + 128 + 1024;
     static constexpr int TM_P = 2 * DKS * KT, TM_O = TM_P + 3 * KT / 2;   // TMEM columns: S [2][DKS][KT], P [3][KT / 2], O
     static_assert(TM_O + 64 * DVS <= 512, "TMEM");
 };
@@ -192,18 +188,19 @@ __device__ __noinline__ void attn_plain(const SplitParams& p, int row, int head,
     }
 }
 
-template <int DKS, int DVS, int KT, bool EXTRA>   // EXTRA: soft-cap or distance bias
-__global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
+template <int DKS, int DVS, int KT, bool EXTRA, int SOFT>   // EXTRA: soft-cap or distance bias; SOFT: softmax warps, 8 or 16
+__global__ void __launch_bounds__(64 + 32 * SOFT, 1) attn_split_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                                                                    const __grid_constant__ SplitParams p) {
     using Cfg = SplitCfg<DKS, DVS, KT>;
-    constexpr int KH = KT / 2, CH = 32 * DVS;   // keys of a tile and value columns per softmax thread
+    constexpr int SP_THREADS = 64 + 32 * SOFT, SHARES = SOFT / 4;             // softmax threads of a pair
+    constexpr int KH = KT / 2, KQ = KT / SHARES, CQ = 64 * DVS / SHARES;       // TMEM columns of a part of P; keys of a tile and value columns of one of them
     extern __shared__ uint8_t sp_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(sp_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint8_t* sQ = smem;                          // [part][slab][128 pairs][128 B]
     uint8_t* sK = sQ + Cfg::Q_BYTES;             // [part][slab][KT keys][128 B]
     uint8_t* sV = sK + Cfg::K_BYTES;             // [part][slab][KT keys][128 B]
-    float* s_red = reinterpret_cast<float*>(sV + Cfg::V_BYTES);   // [tile parity][half][128]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(s_red + 4 * SP_M);
+    float* s_red = reinterpret_cast<float*>(sV + Cfg::V_BYTES);   // [tile parity][share][128]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(s_red + 8 * SP_M);
     uint64_t *k_full = bars, *k_empty = bars + 1, *v_full = bars + 2, *v_empty = bars + 3, *s_full = bars + 4 /*[2]*/, *p_full = bars + 6, *o_full = bars + 7;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
 
@@ -212,7 +209,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tm_k);
         tma_prefetch_desc(&tm_v);
-        for (int i = 0; i < 8; ++i) mbar_init(&bars[i], i == 6 ? 8 : 1);   // p_full: one arrive per softmax warp
+        for (int i = 0; i < 8; ++i) mbar_init(&bars[i], i == 6 ? SOFT : 1);   // p_full: one arrive per softmax warp
         fence_barrier_init();
     }
     if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
@@ -246,7 +243,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_
     }
     {   // queries: pair = row * HG + head; parts into the swizzled K-major operand tiles, idle pairs and entries past dk as zeros
         const bool vec = a.dk % 4 == 0 && a.ldq % 4 == 0 && (reinterpret_cast<uintptr_t>(a.q) & 15) == 0;
-        constexpr int U = 4, TASKS = SP_M * DKS * 8;   // a task is 8 entries of a pair; a thread has the loads of four in flight
+        constexpr int U = SOFT == 8 ? 4 : 2, TASKS = SP_M * DKS * 8;   // a task is 8 entries of a pair; a thread has the loads of U in flight
         for (int e0 = threadIdx.x; e0 < TASKS; e0 += SP_THREADS * U) {
             float x[U][8];
 #pragma unroll
@@ -288,8 +285,9 @@ __global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // (the loops stay rolled: the kernel's roles share the instruction cache)
+        {
+            // walked by the whole warp, an elected lane issues (elect_one, common.cuh); the loops stay rolled: the kernel's roles share the instruction cache
+            const bool leader = elect_one();
             constexpr uint32_t idesc_s = make_idesc_bf16_f32(SP_M, KT), idesc_o = make_idesc_bf16_f32(SP_M, 64 * DVS) | (1u << 16);
             const uint64_t q_desc = make_sw128_kmajor_desc(smem_u32(sQ)), k_desc = make_sw128_kmajor_desc(smem_u32(sK)), v_desc = make_mn_desc(smem_u32(sV), KT * 128);
 #pragma unroll 1
@@ -301,6 +299,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_
 #pragma unroll 1
                     for (int i = 0; i < 6; ++i) {
                         const uint32_t pa = (SPLIT_A >> (2 * i)) & 3u, pb = (SPLIT_B >> (2 * i)) & 3u;
+                        if (leader)
 #pragma unroll
                         for (int s = 0; s < DKS; ++s)   // a slab of 64 entries of the head has an accumulator of its own
 #pragma unroll
@@ -308,8 +307,11 @@ __global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_
                                 umma_bf16(d0 + s * KT, q_desc + ((pa * DKS + s) * (SP_SLAB_Q >> 4) + 2 * k), k_desc + ((pb * DKS + s) * (KT * 8) + 2 * k), idesc_s,
                                           (i | k) != 0 ? 1u : 0u);
                     }
-                    umma_commit(k_empty);
-                    umma_commit(&s_full[(t + 1) & 1]);
+                    if (leader) {
+                        umma_commit(k_empty);
+                        umma_commit(&s_full[(t + 1) & 1]);
+                    }
+                    __syncwarp();
                 }
                 if (t >= 0) {   // O(t)
                     mbar_wait(v_full, t & 1);
@@ -318,90 +320,92 @@ __global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_
 #pragma unroll 1
                     for (int i = 0; i < 6; ++i) {
                         const uint32_t pa = (SPLIT_A >> (2 * i)) & 3u, pb = (SPLIT_B >> (2 * i)) & 3u;
+                        if (leader)
 #pragma unroll
                         for (int k = 0; k < KT / 16; ++k)
                             umma_ts(tm + Cfg::TM_O, tm + Cfg::TM_P + pa * KH + k * 8, v_desc + (pb * (DVS * KT * 8) + k * 128), idesc_o, (i | k) != 0 ? 1u : 0u);
                     }
-                    umma_commit(v_empty);
-                    umma_commit(o_full);
+                    if (leader) {
+                        umma_commit(v_empty);
+                        umma_commit(o_full);
+                    }
+                    __syncwarp();
                 }
             }
         }
     } else {
-        const int quad = warp & 3, half = (warp - 2) >> 2, pair = quad * 32 + lane;
+        const int quad = warp & 3, share = (warp - 2) >> 2, pair = quad * 32 + lane;
         const uint32_t lanes = tm + (static_cast<uint32_t>(quad * 32) << 16);
         const bool live = pair < P;
         const int row = r0 + (live ? pair / HG : 0), head = g * HG + (live ? pair % HG : 0);
         const int pos = live ? minpos + pair / HG : -1, pfirst = split_first(max(pos, 0), a.mask_kind, a.mask_size);
-        float m = -INFINITY, l = 0.f, corr = 1.f, o[CH];
+        float m = -INFINITY, l = 0.f, corr = 1.f, o[CQ];
 #pragma unroll
-        for (int c = 0; c < CH; ++c) o[c] = 0.f;
+        for (int c = 0; c < CQ; ++c) o[c] = 0.f;
         auto join = [&](int t) {   // O(t), in the measure of the maximum that P(t) had
             mbar_wait(o_full, t & 1);
             tc_fence_after();
+            constexpr int W = CQ < 32 ? CQ : 32;
 #pragma unroll
-            for (int c = 0; c < CH / 32; ++c) {
-                uint32_t v[32];
+            for (int c = 0; c < CQ; c += W) {
+                uint32_t v[W];
                 __syncwarp();
-                tmem_ld_32x32(lanes + Cfg::TM_O + half * CH + c * 32, v);
+                tmem_ld_cols(lanes + Cfg::TM_O + share * CQ + c, v);
                 tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 32; ++i) o[c * 32 + i] = fmaf(o[c * 32 + i], corr, __uint_as_float(v[i]));
+                for (int i = 0; i < W; ++i) o[c + i] = fmaf(o[c + i], corr, __uint_as_float(v[i]));
             }
             tc_fence_before();
         };
         for (int t = 0; t < T; ++t) {
-            const int j0 = tile_start(t), jh = j0 + half * KH;
+            const int j0 = tile_start(t), jh = j0 + share * KQ;
             const int nk = min(KT, (t < tilesA ? nA : maxpos + 1) - j0);
             const bool full = nk == KT && j0 + KT <= minpos + 1 && (t < tilesA || j0 >= maxfirst);   // every pair sees every key of the tile
-            float s[KH];
+            float s[KQ];
             mbar_wait(&s_full[t & 1], (t >> 1) & 1);
             tc_fence_after();
             __syncwarp();
 #pragma unroll
-            for (int c = 0; c < KH / 16; ++c) tmem_ld16(lanes + (t & 1) * DKS * KT + half * KH + c * 16, s + c * 16);
-            tmem_ld_wait();
-#pragma unroll
-            for (int sl = 1; sl < DKS; ++sl) {
-                float u[KH];
-#pragma unroll
-                for (int c = 0; c < KH / 16; ++c) tmem_ld16(lanes + ((t & 1) * DKS + sl) * KT + half * KH + c * 16, u + c * 16);
+            for (int sl = 0; sl < DKS; ++sl) {
+                uint32_t u[KQ];
+                tmem_ld_cols(lanes + ((t & 1) * DKS + sl) * KT + share * KQ, u);
                 tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < KH; ++i) s[i] += u[i];
+                for (int i = 0; i < KQ; ++i) s[i] = sl == 0 ? __uint_as_float(u[i]) : s[i] + __uint_as_float(u[i]);
             }
             tc_fence_before();
             float mx = -INFINITY;
 #pragma unroll
-            for (int i = 0; i < KH; ++i) {
+            for (int i = 0; i < KQ; ++i) {
                 s[i] *= a.scale;
                 if (EXTRA && a.softcap > 0.f) s[i] = soft_cap(s[i], a.softcap);
             }
             if (EXTRA && a.rel != nullptr) {   // all of the tile's rows of the bias table, then all of its entries
-                int b[KH];
+                int b[KQ];
 #pragma unroll
-                for (int i = 0; i < KH; ++i) b[i] = a.bucket_of[max(pos - jh - i, 0)];
+                for (int i = 0; i < KQ; ++i) b[i] = a.bucket_of[max(pos - jh - i, 0)];
 #pragma unroll
-                for (int i = 0; i < KH; ++i) s[i] += a.rel[(size_t)b[i] * a.H + head];
+                for (int i = 0; i < KQ; ++i) s[i] += a.rel[(size_t)b[i] * a.H + head];
             }
             if (!full) {
                 const int hi = min(pos, j0 + nk - 1) - jh, lo = pfirst - jh, kept = keep - jh;
 #pragma unroll
-                for (int i = 0; i < KH; ++i)
+                for (int i = 0; i < KQ; ++i)
                     if (!(i <= hi && (i >= lo || i < kept))) s[i] = -INFINITY;
             }
 #pragma unroll
-            for (int i = 0; i < KH; ++i) mx = fmaxf(mx, s[i]);
-            float* red = s_red + (t & 1) * 2 * SP_M;
-            red[half * SP_M + pair] = mx;
-            softmax_sync();
-            mx = fmaxf(mx, red[(half ^ 1) * SP_M + pair]);
+            for (int i = 0; i < KQ; ++i) mx = fmaxf(mx, s[i]);
+            float* red = s_red + (t & 1) * 4 * SP_M;
+            red[share * SP_M + pair] = mx;
+            softmax_sync<SOFT>();
+#pragma unroll
+            for (int i = 0; i < SHARES; ++i) mx = fmaxf(mx, red[i * SP_M + pair]);
             const float m_new = fmaxf(m, mx), m_use = m_new == -INFINITY ? 0.f : m_new, c_new = expf(m - m_use);   // (m = -inf: 0)
             m = m_new;
             float sum = 0.f;
-            uint32_t part[3][KH / 2];
+            uint32_t part[3][KQ / 2];
 #pragma unroll
-            for (int i = 0; i < KH; i += 2) {
+            for (int i = 0; i < KQ; i += 2) {
                 const float p0 = expf(s[i] - m_use), p1 = expf(s[i + 1] - m_use);
                 sum += p0 + p1;
                 split3(p0, p1, part[0][i / 2], part[1][i / 2], part[2][i / 2]);
@@ -411,24 +415,27 @@ __global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_
             corr = c_new;
             __syncwarp();
 #pragma unroll
-            for (int q = 0; q < 3; ++q)
+            for (int q = 0; q < 3; ++q) {
+                if constexpr (KQ == 8) tmem_st4(lanes + Cfg::TM_P + q * KH + share * (KQ / 2), part[q]);
 #pragma unroll
-                for (int c = 0; c < KH / 16; ++c) tmem_st8(lanes + Cfg::TM_P + q * KH + half * (KH / 2) + c * 8, &part[q][c * 8]);
+                for (int c = 0; c < KQ / 16; ++c) tmem_st8(lanes + Cfg::TM_P + q * KH + share * (KQ / 2) + c * 8, &part[q][c * 8]);
+            }
             tmem_st_done();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(p_full);
         }
         join(T - 1);
-        float* red = s_red + (T & 1) * 2 * SP_M;
-        red[half * SP_M + pair] = l;
-        softmax_sync();
-        l += red[(half ^ 1) * SP_M + pair];
+        float* red = s_red + (T & 1) * 4 * SP_M;
+        red[share * SP_M + pair] = l;
+        softmax_sync<SOFT>();
+        l = red[pair] + red[SP_M + pair];
+        if constexpr (SHARES == 4) l += red[2 * SP_M + pair] + red[3 * SP_M + pair];
         bool plain = l != l;
 #pragma unroll
-        for (int c = 0; c < CH; ++c) plain |= o[c] != o[c];
+        for (int c = 0; c < CQ; ++c) plain |= o[c] != o[c];
         if (live && plain) {
-            attn_plain(p, row, head, pos, half * CH, min((half + 1) * CH, a.dv));
+            attn_plain(p, row, head, pos, share * CQ, min((share + 1) * CQ, a.dv));
         } else if (live) {
             float inv = 1.f / l;
             if (a.sink != nullptr || a.sink_fixed) {   // the sink joins the denominator once, under the common maximum
@@ -436,13 +443,13 @@ __global__ void __launch_bounds__(SP_THREADS, 1) attn_split_kernel(const __grid_
                 inv = c0 / fmaf(l, c0, expf(sk - mf));
             }
             if (a.head_gate != nullptr) inv /= 1.f + expf(-a.head_gate[(size_t)row * a.ldg + head]);
-            const int d0 = half * CH;
+            const int d0 = share * CQ;
             const float* cg = a.chan_gate != nullptr ? a.chan_gate + (size_t)row * a.ldg + (size_t)head * a.dv : nullptr;
             const size_t at = (size_t)row * a.ldo + (size_t)head * a.dv;
             const bool vec = a.dv % 4 == 0 && a.ldo % 4 == 0 &&
                              (a.out16 != nullptr ? (reinterpret_cast<uintptr_t>(a.out16) & 7) == 0 : (reinterpret_cast<uintptr_t>(a.out) & 15) == 0);
 #pragma unroll
-            for (int c = 0; c < CH; c += 4) {
+            for (int c = 0; c < CQ; c += 4) {
                 float y[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -475,9 +482,13 @@ int launch_split(const SplitParams& p, const SplitSrc& k, const SplitSrc& v, int
     CUtensorMap tk, tv;
     B2_TRY(make_tmap_parts(&tk, k.out, k.pitch, nkeys, 3 * k.heads, KT));
     B2_TRY(make_tmap_parts(&tv, v.out, v.pitch, nkeys, 3 * v.heads, KT));
-    auto kernel = p.a.softcap > 0.f || p.a.rel != nullptr ? attn_split_kernel<DKS, DVS, KT, true> : attn_split_kernel<DKS, DVS, KT, false>;
+    // Four threads a pair where a tile is a long chain (soft-cap, bias: 600 rows of a fp32 layer 850 -> 816 us a pass) and for few keys, where the
+    // time goes into queries, first use and last write (a pass of 41 rows through four layers 339 -> 329, 200 rows through one 126.9 -> 123.9); from
+    // there on two, whose exchanges are fewer (260 rows 241.0 / 240.2, 1000 rows 324.8 / 321.0, 2048 rows 336 / 332).
+    const bool extra = p.a.softcap > 0.f || p.a.rel != nullptr, wide = extra || nkeys <= FEW_KEYS;
+    auto kernel = extra ? attn_split_kernel<DKS, DVS, KT, true, 16> : wide ? attn_split_kernel<DKS, DVS, KT, false, 16> : attn_split_kernel<DKS, DVS, KT, false, 8>;
     B2_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));
-    launch_pdl(kernel, dim3(((p.a.rows + p.QT - 1) / p.QT) * p.a.G), dim3(SP_THREADS), Cfg::SMEM, st, tk, tv, p);
+    launch_pdl(kernel, dim3(((p.a.rows + p.QT - 1) / p.QT) * p.a.G), dim3(64 + 32 * (wide ? 16 : 8)), Cfg::SMEM, st, tk, tv, p);
     B2_LAUNCH_CHECK();
     return 0;
 }
