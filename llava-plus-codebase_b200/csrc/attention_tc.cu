@@ -8,7 +8,7 @@
 //   warp 0 / lane 0 : TMA producer — Q once, then K_t / V_t tiles of 64 keys into rings (4-D tensor maps over the strided [b, t, h, d]
 //                     views: the same kernel reads the fused qkv activation buffer of the ViT and the [B, H, Smax, 128] KV cache
 //                     of the decoder)
-//   warp 1 / lane 0 : MMA issuer — S_t = Q K_t^T  (UMMA 128x64xD, both operands K-major, SWIZZLE_128B), into one of two TMEM buffers
+//   warp 1          : MMA issuer — S_t = Q K_t^T  (UMMA 128x64xD, both operands K-major, SWIZZLE_128B), into one of two TMEM buffers
 //                                  O += P_t V_t (UMMA 128xDx64; P from TMEM, V straight from its [keys, d] tile as an MN-major operand)
 //   warps 2..5      : softmax — thread r owns query row r: tcgen05.ld the S row, scale/mask, running max / sum, P = exp2(s - m) as bf16
 //                     back into TMEM over the score row it came from; O in TMEM is rescaled only when a row's max grew by more
@@ -170,8 +170,9 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // ---------------- MMA issuer ----------------
+        {
+            // ---------------- MMA issuer: walked by the whole warp, an elected lane issues (elect_one, common.cuh) ----------------
+            const bool leader = elect_one();
             constexpr uint32_t idesc_s = make_idesc(TC_BM, TC_BN, 0), idesc_o = make_idesc(TC_BM, D, 1);
             const uint64_t q_desc = make_sw128_kmajor_desc(smem_u32(sQ));
             auto scores = [&](int t) {   // S_t: K-loop over the head dim in steps of 16 (32 B inside a 128 B swizzle row; slabs of 64)
@@ -179,12 +180,16 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 mbar_wait(&k_full[s], (t / STAGES) & 1);
                 tc_fence_after();
                 const uint64_t k_desc = make_sw128_kmajor_desc(smem_u32(sK + s * Cfg::TILE));
+                if (leader)
 #pragma unroll
                 for (int k = 0; k < D / 16; ++k)
                     umma_bf16(tm + (t & 1) * TC_BN, q_desc + ((k >> 2) * (Q_SLAB >> 4) + (k & 3) * 2), k_desc + ((k >> 2) * (KV_SLAB >> 4) + (k & 3) * 2), idesc_s,
                               k != 0 ? 1u : 0u);
-                umma_commit(&k_empty[s]);
-                umma_commit(&s_full[t & 1]);
+                if (leader) {
+                    umma_commit(&k_empty[s]);
+                    umma_commit(&s_full[t & 1]);
+                }
+                __syncwarp();
             };
             mbar_wait(q_full, 0);
 #pragma unroll 1
@@ -195,13 +200,15 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                     mbar_wait(&p_full[t & 1], (t >> 1) & 1);
                     tc_fence_after();
                     const uint64_t v_desc = make_sw128_mnmajor_desc(smem_u32(sV + s * Cfg::TILE), KV_SLAB);
+                    if (leader)
 #pragma unroll
                     for (int k = 0; k < TC_BN / 16; ++k)
                         umma_ts(tm + TM_O, tm + (t & 1) * TC_BN + k * 8, v_desc + k * 128, idesc_o, (t | k) != 0 ? 1u : 0u);   // 16 key rows of 128 B per step
-                    umma_commit(&v_empty[s]);
+                    if (leader) umma_commit(&v_empty[s]);
                     // the last product has a barrier of its own: its waiters may come while the one before is still under way, and would
                     // take the parity of the one before that for theirs
-                    umma_commit(t + 1 < T ? o_done : o_last);
+                    if (leader) umma_commit(t + 1 < T ? o_done : o_last);
+                    __syncwarp();
                     if (t + 2 < T) mbar_wait(o_done, t & 1);   // S_(t+2) takes the buffer that P_t was read from
                 }
                 if (t + 2 < T) scores(t + 2);
