@@ -379,7 +379,8 @@ int b2_kv_free_slot(b2_kv* kv, int slot, void* stream);
 /* Bytes of device memory one cache of (max_batch, max_seq) takes for this model (state + key/value slabs). */
 int64_t b2_kv_bytes(b2_model* m, int max_batch, int max_seq);
 
-/* ---- single-kernel entry points (unit-level parity tests; same kernels the hot path launches) ----------- */
+/* ---- single-kernel entry points (unit-level parity tests; same kernels the hot path launches) -----------
+ * Every operand, W too, may be what an earlier call on the same stream writes. */
 int b2_op_gemm(const void* A, int lda, const void* W, int ldw, const void* bias, const void* residual, int ld_res,
                void* out, int ld_out, int out_fp32, int M, int N, int K, int act, int bn_override, void* stream);
 // out[M, ff] = bf16(a(gate) (up + up_shift)), [gate | up] = A[M,K] W[2 ff, K]^T: the products and their gated unit in one launch; ff % 8 == 0.

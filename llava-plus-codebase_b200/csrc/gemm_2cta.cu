@@ -61,6 +61,7 @@ struct PairEpi {
     __nv_bfloat16* vcache;
     int rope_S, rope_H, rope_Smax;
     GluAct glu;            // ACT_GLU
+    int w_early;           // GemmArgs
 };
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -175,7 +176,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     cluster_sync_all();  // barriers initialised and TMEM allocated in both CTAs before anyone signals across
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    pdl_trigger();   // the set-up above and the first weights below overlap the upstream kernel's tail; A / residual are its outputs
+    pdl_trigger();   // the set-up above and (w_early) the first weights below overlap the upstream kernel's tail; A / residual are its outputs
 
     if (warp == 0) {
         if (lane == 0) {
@@ -189,9 +190,10 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                     tma_load_2d_2sm(sb, &tmap_b, leader_full, kb * P_BK, b_row, kEvictNormal);
                 }
             };
-            // the weight halves of the first stages travel in front of the programmatic-dependent-launch wait, A follows behind it
+            // the weight halves of the first stages travel in front of the programmatic-dependent-launch wait (unless the kernel in front may be
+            // writing W: w_early), A follows behind it
             int pre = 0;
-            if (pair < num_tiles) {
+            if (ep.w_early != 0 && pair < num_tiles) {
                 int m_blk, n_blk;
                 tile_coords(pair, m_blk, n_blk);
                 for (; pre < num_kb && pre < P_STAGES; ++pre) {
@@ -389,6 +391,7 @@ int gemm_bf16_2cta(const GemmArgs& g, cudaStream_t stream) {
     ep.kcache = reinterpret_cast<__nv_bfloat16*>(g.rope.kcache); ep.vcache = reinterpret_cast<__nv_bfloat16*>(g.rope.vcache);
     ep.rope_S = g.rope.S; ep.rope_H = g.rope.H; ep.rope_Smax = g.rope.Smax;
     ep.glu = g.glu;
+    ep.w_early = g.w_early;
     if (g.act == ACT_ROPE_QKV) {
         B2_CHECK_ARG(g.rope.table && g.rope.kcache && g.rope.vcache && g.rope.S > 0 && g.rope.H > 0 && g.rope.Smax >= g.rope.S,
                      "gemm_2cta(rope_qkv): rope arguments missing");

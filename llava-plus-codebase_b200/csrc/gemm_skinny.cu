@@ -65,6 +65,7 @@ struct SkEpi {
     int ld_out, ld_res, out_fp32, maxseg;
     const float* w_scale;           // fp8 only: [N] per weight row (physical row order of W)
     const float* x_scale;           // fp8 only: [B] per token
+    int w_early;                    // SkinnyArgs
     int stages;                     // ring depth actually used (<= SkCfg::STAGES); B2_SKINNY_STAGES
     unsigned long long* trace;      // debug (B2_SKINNY_TRACE=<file>): 16 slots (8 %globaltimer stamps + tiles finalised) per CTA of this launch, else nullptr
 };
@@ -156,7 +157,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     if (warp == 0) {
         if (lane == 0) {  // ===== TMA producer: weights are read exactly once -> evict-first; activations stay in L2 =====
             // Programmatic dependent launch: this CTA may be running while the kernel that PRODUCES x is still finishing.
-            // Weights depend on nothing, so the first ring-full of W tiles is requested right away; the activation half of
+            // A model's weights depend on nothing (w_early), so the first ring-full of W tiles is requested right away; the activation half of
             // those stages follows once the upstream grid has completed (pdl_wait), everything after that runs as usual.
             int stage = 0; uint32_t phase = 0;
             int pre_n = 0;                      // stages whose W half is already in flight
@@ -164,7 +165,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                 int t = t_first;
                 int kb = (int)(u0 - (long long)t * nkb);
                 long long u = u0;
-                while (u < u1 && pre_n < STAGES) {
+                while (ep.w_early != 0 && u < u1 && pre_n < STAGES) {
                     uint8_t* sw = smem + pre_n * Cfg::STAGE;
                     mbar_arrive_expect_tx(&full_bar[pre_n], Cfg::STAGE);
                     tma_load_2d(sw, &tmap_w, &full_bar[pre_n], kb * BKE, t * SK_BM, kEvictFirst);
@@ -505,7 +506,7 @@ static int gemm_skinny_any(const SkinnyArgs& g, cudaStream_t stream) {
     ep.residual = reinterpret_cast<const __nv_bfloat16*>(g.residual);
     ep.out = g.out; ep.partial = g.partial; ep.counters = g.counters;
     ep.ld_out = g.ld_out; ep.ld_res = g.ld_res; ep.out_fp32 = g.out_fp32; ep.maxseg = pl.maxseg;
-    ep.w_scale = g.w_scale; ep.x_scale = g.x_scale;
+    ep.w_scale = g.w_scale; ep.x_scale = g.x_scale; ep.w_early = g.w_early;
     {   // ring depth: the full ring by default; a shallower ring (<= half of the SM's shared memory) lets the CTAs of two
         // consecutive launches share an SM under programmatic dependent launch. Re-read per launch (A/B inside one process).
         const int full = pl.bn == 32 ? SkCfg<32>::STAGES : (pl.bn == 64 ? SkCfg<64>::STAGES : SkCfg<128>::STAGES);

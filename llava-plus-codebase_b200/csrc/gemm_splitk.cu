@@ -29,6 +29,7 @@ struct KsEpi {
     int ld_out, ld_res, out_fp32, post, accumulate;
     float alpha;
     int a_bytes;           // of A per k-block: gemm_a_rows(M) rows
+    int w_early;           // GemmArgs
 };
 
 __device__ __forceinline__ uint32_t ks_rank() {
@@ -78,8 +79,9 @@ __global__ void __launch_bounds__(KS_THREADS, 1) gemm_splitk_kernel(const __grid
     pdl_trigger();
     if (warp == 0) {
         if (lane == 0) {
-            // the weight halves of the first stages travel in front of the programmatic-dependent-launch wait, A follows behind it
-            const int pre = kb1 - kb0 < STAGES ? kb1 - kb0 : STAGES;
+            // the weight halves of the first stages travel in front of the programmatic-dependent-launch wait (unless the kernel in front may be
+            // writing W: w_early), A follows behind it
+            const int pre = ep.w_early == 0 ? 0 : kb1 - kb0 < STAGES ? kb1 - kb0 : STAGES;
             for (int i = 0; i < pre; ++i) {
                 mbar_arrive_expect_tx(&full[i], ep.a_bytes + BN * KS_BK * 2);
                 tma_load_2d(smem + i * Cfg::STAGE + KS_A, &tmap_b, &full[i], (kb0 + i) * KS_BK, n0, kEvictNormal);
@@ -217,6 +219,7 @@ int gemm_bf16_splitk(const GemmArgs& g, int bn, int S, cudaStream_t st) {
     B2_CHECK_ARG(g.act == ACT_NONE || g.act == ACT_QUICK_GELU || g.act == ACT_GELU_ERF, "gemm(split K): activation %d has no epilogue here", g.act);
     KsEpi ep;
     ep.a_bytes = gemm_a_rows(g.M) * KS_BK * 2;
+    ep.w_early = g.w_early;
     ep.bias = reinterpret_cast<const __nv_bfloat16*>(g.bias); ep.residual = reinterpret_cast<const __nv_bfloat16*>(g.residual);
     ep.out = g.out; ep.ld_out = g.ld_out; ep.ld_res = g.ld_res; ep.out_fp32 = g.out_fp32;
     ep.post = g.out_fp32 ? g.post : 0; ep.alpha = g.out_fp32 ? g.alpha : 1.f; ep.accumulate = g.out_fp32 ? g.accumulate : 0;

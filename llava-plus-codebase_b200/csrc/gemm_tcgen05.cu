@@ -158,6 +158,7 @@ struct EpiParams {
     int group_rows = 0;
     GluAct glu;            // ACT_GLU
     int a_bytes = BM * BK * 2;   // of A per k-block: gemm_a_rows(M) rows
+    int w_early = 0;             // GemmArgs
 };
 
 __device__ __forceinline__ float act_gelu_erf(float x) {
@@ -232,7 +233,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
         // ===================== TMA producer (one thread) =====================
         if (lane == 0) {
             // Programmatic dependent launch: the WEIGHT halves of the first ring-full of stages are requested before the
-            // upstream kernel (which produces A) is known to have finished; the A halves follow after pdl_wait().
+            // upstream kernel (which produces A) is known to have finished, where that kernel cannot be writing W (w_early); the A
+            // halves follow after pdl_wait().
             auto load_b = [&](uint8_t* sb, uint64_t* bar, int kb, int w_row0, int n_blk) {
                 if constexpr (ACT == ACT_GLU) {   // 64 rows of gate, then the 64 rows of up of the same outputs
 #pragma unroll
@@ -245,7 +247,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
             int stage = 0;
             uint32_t phase = 0;
             int pre_n = 0;
-            if ((int)blockIdx.x < num_tiles && ep.tile_group == nullptr) {   // (the group table is made by the upstream kernel)
+            if (ep.w_early != 0 && (int)blockIdx.x < num_tiles && ep.tile_group == nullptr) {   // (the group table is made by the upstream kernel)
                 int m_blk, n_blk;
                 tile_coords(blockIdx.x, m_blk, n_blk);
                 for (int kb = 0; kb < num_kb && pre_n < STAGES; ++kb, ++pre_n) {
@@ -725,6 +727,7 @@ int gemm_bf16(const GemmArgs& g, cudaStream_t stream) {
     EpiParams ep;
     ep.glu = g.glu;
     ep.a_bytes = gemm_a_rows(g.M) * BK * 2;
+    ep.w_early = g.w_early;
     ep.tile_group = g.tile_group; ep.group_rows = g.N;
     ep.bias = reinterpret_cast<const __nv_bfloat16*>(g.bias);
     ep.residual = reinterpret_cast<const __nv_bfloat16*>(g.residual);

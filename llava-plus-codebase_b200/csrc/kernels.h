@@ -53,6 +53,9 @@ struct GemmArgs {
     // grouped product (mixture of experts; single-CTA kernels only): M is a multiple of 128, tile t of 128 rows multiplies with
     // W rows [g * N, (g + 1) * N), g = tile_group[t] (device; negative: the tile is skipped); W holds `groups` matrices of N rows
     const int* tile_group = nullptr; int groups = 1;
+    // W was complete before the kernel in front of this one on the stream was launched (weights of a model): its first tiles may be loaded while
+    // that kernel still runs. Not so for an operand of a caller, which that kernel may be writing.
+    int w_early = 0;
 };
 int gemm_bf16(const GemmArgs& g, cudaStream_t stream);
 // Rows of A that a tile of 128 rows loads per k-block: with fewer rows in all, the rest of the tile is left as it lies in shared memory (a row of
@@ -80,6 +83,7 @@ struct SkinnyArgs {
     int* counters = nullptr;                     // >= gemm_skinny_counter_bytes(N), zero-initialised once
     const float* w_scale = nullptr;              // fp8 variant: [N] per weight row; x / W then hold e4m3 bytes
     const float* x_scale = nullptr;              // fp8 variant: [B] per token
+    int w_early = 0;                             // as in GemmArgs
 };
 int gemm_skinny_bf16(const SkinnyArgs& g, cudaStream_t stream);
 int gemm_skinny_fp8(const SkinnyArgs& g, cudaStream_t stream);

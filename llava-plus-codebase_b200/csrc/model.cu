@@ -99,6 +99,7 @@ int gemm(const void* A, int lda, const void* W, int ldw, const void* bias, const
     GemmArgs g;
     g.A = A; g.lda = lda; g.W = W; g.ldw = ldw; g.bias = bias; g.residual = res; g.ld_res = ld_res;
     g.out = out; g.ld_out = ld_out; g.out_fp32 = out_fp32; g.M = M; g.N = N; g.K = K; g.act = act;
+    g.w_early = 1;   // W: a weight of the model, in all that follows
     return gemm_bf16(g, st);
 }
 
@@ -135,6 +136,7 @@ int skinny(b2_kv* kv, const void* x, int ldx, const void* W, int ldw, const void
     g.out = out; g.ld_out = ld_out; g.out_fp32 = out_fp32; g.B = B; g.N = N; g.K = K; g.act = act;
     g.partial = kv->sk_partial.as<float>(); g.partial_bytes = kv->sk_partial.bytes;
     g.counters = kv->sk_counters.as<int>();
+    g.w_early = 1;
     return gemm_skinny_bf16(g, st);
 }
 // fp8 variant: xq8 / xscale hold the quantised activations of this GEMM
@@ -146,6 +148,7 @@ int skinny8(b2_model* m, b2_kv* kv, const void* W8, const float* w_scale, const 
     g.partial = kv->sk_partial.as<float>(); g.partial_bytes = kv->sk_partial.bytes;
     g.counters = kv->sk_counters.as<int>();
     g.w_scale = w_scale; g.x_scale = m->xscale.as<float>();
+    g.w_early = 1;
     return gemm_skinny_fp8(g, st);
 }
 // From 7 requests on (5 kernels a layer with RMSNorm fused below, on the GEMV kernels, 7 above). The line was drawn against the stream-K GEMM; the tile
@@ -1190,7 +1193,7 @@ int b2_prefill_slots(b2_model* m, b2_kv* kv, const void* embeds, const int32_t* 
             // QKV projection with RoPE and the cache write in its epilogue (CTA-pair kernel): q -> qkv buffer, k / v -> cache
             GemmArgs g;
             g.A = m->xn.p; g.lda = h; g.W = L.wqkv.p; g.ldw = h; g.out = m->qkv.p; g.ld_out = 3 * h;
-            g.M = T; g.N = 3 * h; g.K = h; g.act = ACT_ROPE_QKV;
+            g.M = T; g.N = 3 * h; g.K = h; g.act = ACT_ROPE_QKV; g.w_early = 1;
             g.rope.table = kv->rope_tab.p; g.rope.kcache = kc; g.rope.vcache = vc; g.rope.S = S; g.rope.H = H; g.rope.Smax = kv->max_seq;
             B2_TRY(gemm_bf16_2cta(g, st));
         } else {

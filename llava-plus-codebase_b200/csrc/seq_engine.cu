@@ -226,7 +226,7 @@ struct Lin {  // one Linear call on the model's compute dtype
             if (a16 == nullptr) B2_TRY(cast_rows_bf16(A, lda, s.a16.p, K, M, K, st));
             GemmArgs g;
             g.A = a16 != nullptr ? a16 : s.a16.p; g.lda = K; g.W = a.W; g.ldw = K; g.out = out; g.ld_out = (int)ldo; g.out_fp32 = 1; g.bias = bias16;
-            g.M = M; g.N = Np; g.K = K; g.act = ACT_NONE; g.post = act; g.alpha = alpha; g.accumulate = accumulate;
+            g.M = M; g.N = Np; g.K = K; g.act = ACT_NONE; g.post = act; g.alpha = alpha; g.accumulate = accumulate; g.w_early = 1;
             return gemm_bf16(g, st);
         }
         return linear_f32(a, st);
@@ -588,7 +588,7 @@ static int gelu_up(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, const SubI
         if (in.h16 == nullptr) B2_TRY(cast_rows_bf16(in.h, width, s.a16.p, width, R, width, st));
         GemmArgs g;
         g.A = in.h16 != nullptr ? in.h16 : s.a16.p; g.lda = width; g.W = W.up_w.p; g.ldw = width; g.out = s.f16.p; g.ld_out = ff;
-        g.M = R; g.N = ff; g.K = width; g.act = ACT_GELU_ERF;
+        g.M = R; g.N = ff; g.K = width; g.act = ACT_GELU_ERF; g.w_early = 1;
         return gemm_bf16(g, st);
     }
     return lin(in.h, width, W.up_w, ff, width, s.ff.as<float>(), (ff + 7) / 8 * 8, R, LIN_GELU, 1.f, 0, nullptr, 0, nullptr, in.h16, in.norm);
@@ -701,7 +701,7 @@ static int glu_product(const Lin& lin, const SubIn& in, const DevBuf& W, int ff,
     if (in.h16 == nullptr) B2_TRY(cast_rows_bf16(in.h, width, s.a16.p, width, R, width, lin.st));
     GemmArgs g;
     g.A = in.h16 != nullptr ? in.h16 : s.a16.p; g.lda = width; g.W = W.p; g.ldw = width; g.out = s.ff.p; g.ld_out = ff;
-    g.M = R; g.N = 2 * ff; g.K = width; g.act = ACT_GLU; g.glu = act;
+    g.M = R; g.N = 2 * ff; g.K = width; g.act = ACT_GLU; g.glu = act; g.w_early = 1;
     return gemm_bf16(g, lin.st);
 }
 
