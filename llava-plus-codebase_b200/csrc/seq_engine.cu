@@ -237,13 +237,27 @@ bool is_glu(int ff_kind) { return ff_kind == B2_FF_CLAMP_GLU || ff_kind == B2_FF
 
 int router_rows(int experts) { return std::max(32, (experts + 7) / 8 * 8); }   // rows of the (zero-padded) router matrix
 
-// Prompt portions of at least this many rows make per-head keys / values of the positions they see instead of absorbing W_uk / W_uv. Absorbing takes
-// two launches a head from 9 rows on (up to 8 rows share one) and attends with the latent's width. 16 heads of 128 over a latent of 512, us a call,
-// absorbed / per head: 9 rows 652 / 489, behind 8000 positions 5047 / 3004; 40 rows 763 / 556, behind 2000 1906 / 672, behind 8000 5336 / 998.
-int latent_materialise_rows() {
+// Whether a prompt portion makes per-head keys / values of `keys` positions (a: its attention over them) instead of absorbing W_uk / W_uv.
+// Absorbing takes two launches a head from 9 rows on (up to 8 rows share one) and attends on the fp32 pipe with the widths of the latent (`wide`, keys
+// and values together); per head, two products go over all positions, in pieces of at most `piece` rows. us a call of one layer, absorbed / per head:
+//   on the tensor cores (16 rows and more): 2 heads of 32 over rank 64, 16 rows behind 4000 positions 800 / 224, in pieces of 512 798 / 291, of 64
+//     803 / 984; 16 heads of 128 over 512, 63 rows behind 4000 3557 / 478; a rank of 32 under heads of 128, 16 rows behind 4000 698 / 287;
+//   nothing behind them: 9 rows, 2 heads 73 / 65, 16 heads 233 / 86, 8 heads of 256 134 / 84; one head 65 / 66, 24 rows of it 82 / 84;
+//   else the widths decide: 9 rows behind 4000, rank 512 under 16 heads of 128 2464 / 1050, 128 under 64 975 / 742, 64 under 32 679 / 614 (true
+//     fp32, pieces of 1024 711 / 660, of 512 712 / 728), but 128 under 128 behind 12000 2843 / 3011, 64 under 128 761 / 985, and under
+//     heads of 256 a rank of 128 1026 / 2472, of 512 2385 / 2514 (63 rows 3507 / 5201).
+// A window that keeps first positions sees `seen` of them; those in between would be made too. From 64 rows on it makes them in any case;
+// B2_LATENT_MATERIALISE_ROWS=n: from n rows on.
+bool latent_per_head(const BiasAttnArgs& a, int keys, int seen, int wide, int piece) {
     const char* e = getenv("B2_LATENT_MATERIALISE_ROWS");
     const int v = e != nullptr ? atoi(e) : 0;
-    return v >= 1 ? v : 9;
+    if (v >= 1) return a.rows >= v;
+    if (a.rows < 9 || a.rows >= 64) return a.rows >= 64;
+    if (keys / 2 > seen) return false;
+    if (attn_split_fits(a)) return keys <= piece || piece >= 512;
+    if (a.G < 2) return false;
+    if (keys <= 64) return keys <= piece;
+    return a.dk <= 192 && a.dv <= 128 && wide >= 2 * (a.dk + a.dv) && (keys <= piece || piece >= 1024);
 }
 
 int attn_nsplit(int rows, int G, int max_seq) {
@@ -324,7 +338,17 @@ static int latent_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeight
     aa.partial = state.attn_partial.as<float>();
     mask_of(d, aa);
     float* y = s.y.as<float>();
-    if (nseg == 1 && R >= latent_materialise_rows() && ctx_end > 0) {
+    const int first = d.mask_kind == B2_MASK_WINDOW ? (d.mask_keep > 0 ? 0 : std::max(0, ctx_end - R - d.mask_size + 1))
+                    : d.mask_kind == B2_MASK_CHUNK ? (ctx_end - R) / d.mask_size * d.mask_size : 0;
+    const int keys = ctx_end - first, seen = d.mask_keep > 0 ? (int)std::min<int64_t>(keys, (int64_t)R + d.mask_size + d.mask_keep) : keys;
+    BiasAttnArgs ah = aa;   // over per-head keys and values
+    ah.q = q; ah.ldq = ldq;
+    ah.kcache = state.kmat.as<float>(); ah.vcache = state.vmat.as<float>();
+    ah.kv_row_stride = state.kmat_ld; ah.kv_row_stride_v = state.vmat_ld;
+    ah.out = y; ah.ldo = L.pv;
+    ah.G = H; ah.dk = qh; ah.dv = dv; ah.nsplit = 1;
+    portion_of(s, nseg, slot, ctx_end, ah);
+    if (nseg == 1 && ctx_end > 0 && latent_per_head(ah, keys, seen, lrow + rank, s.rows)) {
         // a long portion: per-head keys and values of every visible position of the slot so far are made from the cached rows
         // with two products (the key product carries the rotated part through an identity block), and the attention runs over
         // them with the heads' own sizes
@@ -335,21 +359,13 @@ static int latent_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeight
             B2_TRY(rotate_rows_f32(ra, st));
         }
         const float* lat = lat_cache + (size_t)slot * kv->max_seq * lrow;
-        const int first = d.mask_kind == B2_MASK_WINDOW ? (d.mask_keep > 0 ? 0 : std::max(0, ctx_end - R - d.mask_size + 1))
-                        : d.mask_kind == B2_MASK_CHUNK ? (ctx_end - R) / d.mask_size * d.mask_size : 0;
         const DevBuf& wk = rd > 0 ? W.ukx_w : W.uk_w;
         for (int m0 = first; m0 < ctx_end; m0 += s.rows) {
             const int mc = std::min(s.rows, ctx_end - m0);
             B2_TRY(lin(lat + (size_t)m0 * lrow, lrow, wk, L.lqw, lrow, state.kmat.as<float>() + (size_t)m0 * state.kmat_ld, state.kmat_ld, mc));
             B2_TRY(lin(lat + (size_t)m0 * lrow, lrow, W.uv_w, L.pv, rank, state.vmat.as<float>() + (size_t)m0 * state.vmat_ld, state.vmat_ld, mc));
         }
-        aa.q = q; aa.ldq = ldq;
-        aa.kcache = state.kmat.as<float>(); aa.vcache = state.vmat.as<float>();
-        aa.kv_row_stride = state.kmat_ld; aa.kv_row_stride_v = state.vmat_ld;
-        aa.out = y; aa.ldo = L.pv;
-        aa.G = H; aa.dk = qh; aa.dv = dv; aa.nsplit = 1;
-        portion_of(s, nseg, slot, ctx_end, aa);
-        B2_TRY(attn_bias_f32(aa, st));
+        B2_TRY(attn_bias_f32(ah, st));
     } else {
         // absorbed form: q_h -> W_uk_h^T q_h lives in the latent space (the rotated part rides behind it), so scores and values
         // read the cached rows directly, and W_uv_h carries the latent-space output to the head's values
