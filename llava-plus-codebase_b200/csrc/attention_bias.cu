@@ -444,10 +444,6 @@ __global__ void __launch_bounds__(512) attn_merge_kernel(BiasAttnArgs a) {
 // 8 key/value heads 41.1 -> 33.0 (500, 1), 86 -> 45 (8000, 1), 68 -> 37 (500, 8), 276 -> 77 (4000, 8); 2 of them 41.1 -> 35.2 (500, 1).
 constexpr int ST_WARPS = 16, ST_KEYS = 8, ST_DK = 128, ST_DV = 128;
 
-__device__ __forceinline__ void st_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ float st_ld_remote(const float* p, int rank) {
     uint32_t at;
     float v;
@@ -562,7 +558,7 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 1) attn_step_kernel(BiasAttnArg
         for (int w = 0; w < ST_WARPS; ++w) acc = fmaf(so[w][h][d], sm[w][h], acc);
         po[h][d] = acc;
     }
-    st_cluster_sync();
+    cluster_sync();
     const int share = (HG * dv + C - 1) / C;
     for (int e = rank * share + threadIdx.x; e < min(HG * dv, (rank + 1) * share); e += ST_WARPS * 32) {
         const int h = e / dv, d = e - h * dv, head = h0 + h;
@@ -588,7 +584,7 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 1) attn_step_kernel(BiasAttnArg
         const float inv = a.head_gate != nullptr ? 1.f / (sum * (1.f + expf(-a.head_gate[(size_t)r * a.ldg + head]))) : 1.f / sum;
         store_out(a, r, head, d, acc * inv);
     }
-    st_cluster_sync();   // no share goes away while another CTA reads it
+    cluster_sync();   // no share goes away while another CTA reads it
 }
 
 int check_args(const BiasAttnArgs& a, const char* who) {

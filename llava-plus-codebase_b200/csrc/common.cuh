@@ -255,6 +255,13 @@ constexpr uint64_t kEvictLast = 0x14F0000000000000ull;
 // ----------------------------------------------------------------------------------------------
 // tcgen05 / TMEM
 // ----------------------------------------------------------------------------------------------
+// All threads of a cluster. The barrier's aligned form takes whole warps: lanes that left a loop or a branch at different turns meet in front of it.
+__device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // A kernel that allocates TMEM lets its dependents start (pdl_trigger) only behind the allocation and the barrier after it. A dependent that
 // has TMEM of its own holds it until this kernel is done; if it could be resident before this kernel's CTAs have theirs, each would wait for the other.
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_dst, uint32_t ncols) {

@@ -69,10 +69,6 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // shared::cluster address of `local_smem_addr` (a shared::cta address of THIS CTA) in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t mapa_rank(uint32_t local_smem_addr, uint32_t rank) {
     uint32_t r;
@@ -173,7 +169,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     }
     if (warp == 1) tmem_alloc_2sm(tmem_slot, P_TMEM_COLS);  // collective over the pair: one warp in each CTA
     tc_fence_before();
-    cluster_sync_all();  // barriers initialised and TMEM allocated in both CTAs before anyone signals across
+    cluster_sync();  // barriers initialised and TMEM allocated in both CTAs before anyone signals across
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_trigger();   // the set-up above and (w_early) the first weights below overlap the upstream kernel's tail; A / residual are its outputs
@@ -339,9 +335,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         if (lane == 0) bulk_wait_all();
     }
 
-    __syncwarp();  // lanes 1..31 of the producer / MMA warps waited here: the cluster barrier below is .aligned
     tc_fence_before();
-    cluster_sync_all();  // no CTA may free TMEM / exit while its partner can still signal into its shared memory
+    cluster_sync();  // no CTA may free TMEM / exit while its partner can still signal into its shared memory
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc_2sm(tmem_base, P_TMEM_COLS);

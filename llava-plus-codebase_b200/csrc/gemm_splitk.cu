@@ -37,10 +37,6 @@ __device__ __forceinline__ uint32_t ks_rank() {
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
-__device__ __forceinline__ void ks_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ float4 ks_ld_remote(uint32_t addr, uint32_t rank) {
     uint32_t a;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
@@ -141,7 +137,7 @@ __global__ void __launch_bounds__(KS_THREADS, 1) gemm_splitk_kernel(const __grid
         }
         tc_fence_before();
     }
-    ks_cluster_sync();
+    cluster_sync();
     if (warp >= 2) {
         pdl_wait();   // residual and output may be written by the kernels in front
         const int t = threadIdx.x - 64, row = t & 127, per = BN / S / 8;   // 8-column groups of this CTA's share
@@ -181,8 +177,7 @@ __global__ void __launch_bounds__(KS_THREADS, 1) gemm_splitk_kernel(const __grid
             }
         }
     }
-    __syncwarp();
-    ks_cluster_sync();   // no ring goes away while another CTA reads it
+    cluster_sync();   // no ring goes away while another CTA reads it
     if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, BN); }
 }
 

@@ -32,3 +32,15 @@ def test_dependents_start_behind_the_allocation_of_tensor_memory(repo_root):
                 between = body[alloc.end():min(starts)] if min(starts) > alloc.start() else ""
                 assert re.search(r"__syncthreads\(\)|cluster_sync\w*\(", between), f"{os.path.basename(path)}: {name} lets dependents start before its allocation"
     assert seen >= 8
+
+
+def test_cluster_barriers_take_whole_warps(repo_root):
+    """barrier.cluster in its aligned form needs every lane of a warp at the same instruction; behind a loop whose lanes leave at different turns only
+    __syncwarp brings them there. So there is one function with the barrier, and it begins with that."""
+    seen = 0
+    for path in glob.glob(os.path.join(repo_root, "llava-plus-codebase_b200", "csrc", "*.cu*")):
+        src = re.sub(r"//[^\n]*|/\*.*?\*/", "", open(path).read(), flags=re.S)
+        for m in re.finditer(r"barrier\.cluster\.arrive[\w.]*aligned", src):
+            seen += 1
+            assert re.search(r"__syncwarp\(\);\s*asm volatile\(\"$", src[:m.start()]), os.path.basename(path)
+    assert seen >= 1
