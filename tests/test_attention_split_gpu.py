@@ -90,3 +90,26 @@ def test_windows_and_kept_positions(size, keep, portions):
 @pytest.mark.parametrize("portions", [[150], [20, 60, 16, 41]])
 def test_two_maps_in_chunks(chunk, portions):
     check(diff(4, 2, 64, 72, 3, chunk, 32), portions)
+
+
+# Without soft-cap and bias, calls that see more than 256 keys run with two softmax threads a pair, the others with four
+SIZES = [(64, 64), (64, 128), (128, 64), (128, 128), (192, 64), (192, 128)]
+
+
+@pytest.mark.parametrize("dim,vdim", SIZES)
+@pytest.mark.parametrize("portions", [[255], [256], [257], [330], [200, 65, 64]])
+def test_around_the_line_between_two_and_four_softmax_threads(dim, vdim, portions):
+    check(win(4, 2, dim, vdim, None, None, dim // 2), portions)
+
+
+@pytest.mark.parametrize("dim,vdim", SIZES)
+@pytest.mark.parametrize("size,keep", [(300, 5), (70, 64), (260, 0)])
+def test_windows_over_many_keys(dim, vdim, size, keep):
+    check(win(3, 1, dim, vdim, size, keep, 8), [400])
+
+
+@pytest.mark.parametrize("dim,vdim", [(64, 64), (128, 128), (192, 128)])
+@pytest.mark.parametrize("chunk", [50, 280])
+@pytest.mark.parametrize("portions", [[400], [290, 110]])
+def test_two_maps_in_chunks_over_many_keys(dim, vdim, chunk, portions):
+    check(diff(2, 1, dim, vdim, 3, chunk, 32), portions)
