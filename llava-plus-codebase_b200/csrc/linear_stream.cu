@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(LS_WARPS * 32, 16 / LS_WARPS) linear_stream_ke
     const __nv_bfloat16* W = reinterpret_cast<const __nv_bfloat16*>(a.W);
 
     uint4 w[2][4][2];
-    auto load_w = [&](int s, uint4 (&u)[4][2]) {   // step s: tile s / upw of this CTA, unit (s % upw) * 8 + warp
+    auto load_w = [&](int s, uint4 (&u)[4][2]) {   // step s: tile s / upw of this CTA, unit (s % upw) * LS_WARPS + warp
         const int n0 = ((int)blockIdx.x + (s / upw) * (int)gridDim.x) * OUTS, k0 = ((s % upw) * LS_WARPS + warp) * LS_UNIT + kq;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {

@@ -105,3 +105,16 @@ def test_units_biases_and_slots(name, n, slots, monkeypatch):
         return outputs(model, toks, n, slots)
 
     both_ways(run, monkeypatch, bound(104, 136, 4 * 24))
+
+
+# One CTA of 16 warps an SM or two of 8, whichever has the shorter longest chain: tiles that fill both forms' CTAs once, twice and a little more
+@pytest.mark.parametrize("width,vocab", [(72, 2376), (264, 2600), (1024, 3001), (1024, 4736), (1032, 4745), (520, 9500), (2048, 2377), (2056, 2600), (4096, 5003)])
+@pytest.mark.parametrize("n", [1, 8, 9, 16])
+def test_several_tiles_a_block(width, vocab, n):
+    test_head_against_64_bits(width, vocab, n)
+
+
+@pytest.mark.parametrize("width,ff", [(136, 2376), (264, 2504), (1024, 2400), (2048, 1200)])
+@pytest.mark.parametrize("n", [1, 8, 9, 16])
+def test_several_gated_tiles_a_block(width, ff, n, monkeypatch):
+    test_streamed_weights_equal_the_fma_kernels(width, ff, n, monkeypatch)
