@@ -79,6 +79,11 @@ __device__ __forceinline__ void add_bf16x8(float* x, const uint4& b) {
     x[4] += bf16_lo(b.z); x[5] += bf16_hi(b.z); x[6] += bf16_lo(b.w); x[7] += bf16_hi(b.w);
 }
 
+// fp32 outputs of a few rows leave straight from the registers: there are few lines to open, and the way through the box is the longer chain behind a
+// launch's products. us, straight / boxes: 8 rows N = 12288, K = 4096 23.7 / 25.0, N = 32000, K = 2048 25.2 / 27.3; 33 rows 24.5 / 25.6, 26.7 / 28.0; 64 rows
+// 26.0 / 26.2, 29.7 / 29.1; 128 rows 29.3 / 27.1, 34.9 / 30.8.
+constexpr int FEW_ROWS = 48;
+
 // out = act(acc + bias) + residual, bf16, or (F32) fp32 with post activation, scale and accumulation, for a warp's COLS columns: accumulator columns
 // from taddr on are output columns from col0 on. EP: bias, residual, ld_res, out, ld_out, post, alpha, accumulate. `ready` is called in front of the
 // first read of the accumulator (behind the first requests to global memory), `drained` behind the last one.
@@ -94,6 +99,7 @@ __device__ __forceinline__ void store_tile(const TileBox<CH>& box, uint32_t tadd
         return;
     }
     const bool in = box.row0 + box.lane < box.M;
+    const bool few = F32 && box.M <= FEW_ROWS && ep.post == 0 && ep.accumulate == 0;
     const bool has_old = F32 ? ep.accumulate != 0 : ep.residual != nullptr;
     RowBox<CH> old;                                 // what the next box is added to: the residual (bf16), or what the output holds (fp32)
     auto load_old = [&](int col) {
@@ -143,6 +149,14 @@ __device__ __forceinline__ void store_tile(const TileBox<CH>& box, uint32_t tadd
 #pragma unroll
                 for (int i = 0; i < 2; ++i)
                     if (col + i * 8 < box.N) add_bf16x8(x + i * 8, *reinterpret_cast<const uint4*>(ep.residual + (size_t)(box.row0 + box.lane) * ep.ld_res + col + i * 8));
+            }
+            if (few) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (in && col + 4 * i < box.N)
+                        *reinterpret_cast<float4*>(static_cast<float*>(ep.out) + (size_t)(box.row0 + box.lane) * ep.ld_out + col + 4 * i) =
+                            make_float4(ep.alpha * x[4 * i], ep.alpha * x[4 * i + 1], ep.alpha * x[4 * i + 2], ep.alpha * x[4 * i + 3]);
+                continue;
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i)

@@ -40,3 +40,10 @@ def test_rows_and_columns_at_the_edges(M, N, K, act, f32, bias, residual, plan):
     err = (out[:M, :N].double() - ref).abs()
     assert bool((err <= tol).all()), float((err - tol).max())
     assert bool((out[M:] == 7.0).all()) and bool((out[:, N:] == 7.0).all())
+
+
+@pytest.mark.parametrize("plan", [64, 128, 192, 256, 2])
+@pytest.mark.parametrize("M", [1, 8, 31, 33, 48, 49])
+@pytest.mark.parametrize("N,act,bias,residual", [(8, 0, 0, 0), (264, 1, 1, 0), (1000, 0, 0, 1)])
+def test_fp32_outputs_of_a_few_rows(M, N, act, bias, residual, plan):
+    test_rows_and_columns_at_the_edges(M, N, 136, act, 1, bias, residual, plan)
