@@ -164,11 +164,12 @@ __global__ void __launch_bounds__(LS_WARPS * 32, 16 / LS_WARPS) linear_stream_ke
 template <int NT, bool A16, bool GLU>
 int launch_stream(const LinearArgs& a, cudaStream_t st) {
     const int outs = GLU ? LS_N / 2 : LS_N, tiles = (a.N + outs - 1) / outs, units = (a.K + LS_UNIT - 1) / LS_UNIT;
-    // The longest chain of units that a warp walks, with two CTAs of 8 warps on an SM and with one of 16: the shorter one. (48 steps of the
-    // four-layer model above, one slot: gate and up of 5120 x 2048 6 / 5 units, down 5 / 3, the rest 2 / 2 and 2 / 1: 10.32 -> 9.87 ms;
-    // eight slots 12.74 -> 12.55.)
-    const int chain8 = ((tiles + 2 * num_sms() - 1) / (2 * num_sms())) * ((units + 7) / 8), chain16 = ((tiles + num_sms() - 1) / num_sms()) * ((units + 15) / 16);
-    if (chain16 <= chain8) B2_CUDA_CHECK(launch_pdl(linear_stream_kernel<NT, A16, GLU, 16>, dim3(std::min(tiles, num_sms())), dim3(512), 0, st, a));
+    // Two CTAs of 8 warps on an SM, or one of 16: the shorter one of the longest chains that a warp walks, in half units of weights. The end of a tile
+    // (two barriers, the warps' sums) takes about half a unit's time, with more than 8 rows a whole one's. us a step, always 8 / shorter chain of
+    // units alone / this: four mixed layers of width 2048, one slot 197 / 192 / 188, 16 slots 262 / 255 / 251; of 1280 166 / 150 / 150; of 3072 291 / 298 /
+    // 292; one layer of window attention of 4096, 16 slots 202 / 212 / 200; of gated linear attention of 4096 267 / 280 / 267.
+    const auto chain = [&](int ctas, int warps) { return ((tiles + ctas - 1) / ctas) * (2 * ((units + warps - 1) / warps) + (NT == 2 ? 2 : 1)); };
+    if (chain(num_sms(), 16) <= chain(2 * num_sms(), 8)) B2_CUDA_CHECK(launch_pdl(linear_stream_kernel<NT, A16, GLU, 16>, dim3(std::min(tiles, num_sms())), dim3(512), 0, st, a));
     else B2_CUDA_CHECK(launch_pdl(linear_stream_kernel<NT, A16, GLU, 8>, dim3(std::min(tiles, 2 * num_sms())), dim3(256), 0, st, a));
     B2_LAUNCH_CHECK();
     return 0;
