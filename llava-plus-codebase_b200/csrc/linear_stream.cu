@@ -165,10 +165,13 @@ template <int NT, bool A16, bool GLU>
 int launch_stream(const LinearArgs& a, cudaStream_t st) {
     const int outs = GLU ? LS_N / 2 : LS_N, tiles = (a.N + outs - 1) / outs, units = (a.K + LS_UNIT - 1) / LS_UNIT;
     // Two CTAs of 8 warps on an SM, or one of 16: the shorter one of the longest chains that a warp walks, in half units of weights. The end of a tile
-    // (two barriers, the warps' sums) takes about half a unit's time, with more than 8 rows a whole one's. us a step, always 8 / shorter chain of
-    // units alone / this: four mixed layers of width 2048, one slot 197 / 192 / 188, 16 slots 262 / 255 / 251; of 1280 166 / 150 / 150; of 3072 291 / 298 /
-    // 292; one layer of window attention of 4096, 16 slots 202 / 212 / 200; of gated linear attention of 4096 267 / 280 / 267.
-    const auto chain = [&](int ctas, int warps) { return ((tiles + ctas - 1) / ctas) * (2 * ((units + warps - 1) / warps) + (NT == 2 ? 2 : 1)); };
+    // (two barriers, the warps' sums) takes about half a unit's time, with more than 8 rows a whole one's; in a long stream of tiles whose last units
+    // leave some of 8 warps idle (a head of 32000 outputs, K = 1536: 12 units), 16 warps were the faster form all the same. us a step, always 8 warps /
+    // the shorter chain of units alone / this: four mixed layers of width 2048, one slot 205 / 197 / 194, 16 slots 271 / 265 / 258; of 1280, one slot 170 / 156 /
+    // 154; of 3072, 8 slots 303 / 310 / 303; gated linear attention of 1536, 3 slots 80 / 73 / 71, 16 slots 121 / 125 / 116; window attention of 4096, 16 slots
+    // 202 / 212 / 200.
+    const int end = NT == 2 ? 2 : tiles >= 8 * num_sms() && units % 8 != 0 ? 0 : 1;
+    const auto chain = [&](int ctas, int warps) { return ((tiles + ctas - 1) / ctas) * (2 * ((units + warps - 1) / warps) + end); };
     if (chain(num_sms(), 16) <= chain(2 * num_sms(), 8)) B2_CUDA_CHECK(launch_pdl(linear_stream_kernel<NT, A16, GLU, 16>, dim3(std::min(tiles, num_sms())), dim3(512), 0, st, a));
     else B2_CUDA_CHECK(launch_pdl(linear_stream_kernel<NT, A16, GLU, 8>, dim3(std::min(tiles, 2 * num_sms())), dim3(256), 0, st, a));
     B2_LAUNCH_CHECK();
