@@ -629,7 +629,9 @@ static int step_cluster(const BiasAttnArgs& a, int units) {
 }
 // One row per slot, caches of heads that 16-byte loads of 32 lanes cover. Few key/value heads fill few SMs: from some thousand keys a CTA on
 // the tiled kernel's key splits (up to 64) read them faster. One slot, 2 key/value heads, 16 CTAs: 8000 keys 61.9 us tiled, 59.3 here; 16000
-// 86.1 / 84.4; 32000 133 / 141.
+// 86.1 / 84.4; 32000 133 / 141. Where the heads fill many SMs, the keys of one may be any number: also with half the SMs idle (75 to 147 units: one CTA each)
+// the tiled kernel is slower, whose splits end at 8 rows. Keys and values of 128, us a step, tiled / here: 5 slots of 16 heads 500 keys 77 / 42, 8000 655 /
+// 149; 10 slots of 8 heads 8000 keys 1689 / 152; 18 slots of 8 2000 keys 512 / 89; 3 slots of 8, 24000 keys 504 / 128.
 static bool attn_step_fits(const BiasAttnArgs& a) {
     const int heads = a.H / a.G, units = a.G * ((heads + 3) / 4);
     const long long keys = a.mask_kind == MASK_WINDOW ? (long long)a.mask_size + a.mask_keep : a.mask_kind == MASK_CHUNK ? a.mask_size : a.Smax;

@@ -10,10 +10,11 @@
 // have an accumulator of their own, and the weighted sum of values leaves TMEM after every key tile and is added up in fp32 registers. Scores, bias, soft-cap, mask, maximum, exponential, denominator: fp32 on the
 // CUDA cores, as before.
 //
-// What bounds it: the products (12 of a tile where bf16 attention has 2), as fast as they are issued: walked by one lane an instruction took 80-107 clk
-// for 48-64 of work, by the whole warp with an elected lane less (window 129 -> 106 us). Then the chain of a tile through the softmax warps. 2048
-// rows, 16 heads of 128 on 4 key/value heads: window of 1024 + 4 kept positions 1061 -> 106 us (attn_tile_kernel -> this), no window, 1536 rows on
-// 16 key/value heads 947 -> 84 us; cutting the keys and values: 4 us of that call.
+// What bounds it: the products (12 of a tile where bf16 attention has 2) and their issue; with them issued by an elected lane of the whole warp instead of by
+// one lane's loop, window 129 -> 106 us, tensor pipe active 38.7 -> 48.4 % (profiles/split_attention_scan_ncu.txt). Then the chain of a tile through the
+// softmax warps, and CTAs whose rows see few keys beside CTAs whose rows see many. 2048 rows, 16 heads of 128 on 4 key/value heads: window of 1024 + 4
+// kept positions 1061 -> 104 us (attn_tile_kernel -> this), no window, 1536 rows on 16 key/value heads 947 -> 80 us; cutting the keys and values: 4 us of
+// that call.
 // Error of one fp32 layer against 64 bits, old -> new: 5.0e-7 -> 4.7e-7 at 17 rows, 7.1e-7 -> 5.9e-7 at 333, 8.6e-7 -> 6.5e-7 at 2048.
 //   1. attn_split_kv_kernel cuts the visible keys and values of the call into parts once (they are read by every query tile);
 //   2. attn_split_kernel: CTA = 128 (row, head) pairs of ONE key/value head (rows x the group's query heads, so that a key tile serves
@@ -484,7 +485,8 @@ int launch_split(const SplitParams& p, const SplitSrc& k, const SplitSrc& v, int
     B2_TRY(make_tmap_parts(&tv, v.out, v.pitch, nkeys, 3 * v.heads, KT));
     // Four threads a pair where a tile is a long chain (soft-cap, bias: 600 rows of a fp32 layer 850 -> 816 us a pass) and for few keys, where the
     // time goes into queries, first use and last write (a pass of 41 rows through four layers 339 -> 329, 200 rows through one 126.9 -> 123.9); from
-    // there on two, whose exchanges are fewer (260 rows 241.0 / 240.2, 1000 rows 324.8 / 321.0, 2048 rows 336 / 332).
+    // there on two, whose exchanges are fewer (260 rows 241.0 / 240.2, 1000 rows 324.8 / 321.0, 2048 rows 336 / 332). 18 warps leave a thread 96 registers:
+    // with value heads of 128 the four-thread form spills (208 / 148 bytes stored / loaded at <2, 2, 64, true, 16>, 132 / 140 without cap and bias).
     const bool extra = p.a.softcap > 0.f || p.a.rel != nullptr, wide = extra || nkeys <= FEW_KEYS;
     auto kernel = extra ? attn_split_kernel<DKS, DVS, KT, true, 16> : wide ? attn_split_kernel<DKS, DVS, KT, false, 16> : attn_split_kernel<DKS, DVS, KT, false, 8>;
     B2_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));

@@ -260,7 +260,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                 // Fix-up through shared memory: when the tile being finalised is this CTA's LAST one, the ring is drained (every
                 // load consumed, every MMA complete), so the nseg partials are fetched with ONE round of 1-D bulk copies into it
                 // instead of nseg x 32 L2 loads per thread in dependent rounds (~2 us each while the next kernel's weight
-                // prefetch keeps the memory system busy: profiles/r2l_sk_trace_b32_summary.txt).
+                // prefetch keeps the memory system busy).
                 staged = finalize && t == t_last && (size_t)nseg * (BN * SK_BM * 4) <= (size_t)STAGES * Cfg::STAGE;
                 if (staged && et == 0) {
                     asm volatile("fence.proxy.async;" ::: "memory");  // other CTAs' generic-proxy stores -> async-proxy reads

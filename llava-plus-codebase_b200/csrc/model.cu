@@ -525,7 +525,7 @@ bool use_mega(const b2_model* m, int B) {
     return flag == 1;
 }
 
-// defaults of the megakernel knobs (measured on B200: profiles/r1e_mega_sweep.txt)
+// defaults of the megakernel knobs (measured on B200: profiles/r1e_mega_knob_sweep.jsonl)
 constexpr int kMegaL2AheadDefault = 0;
 constexpr int kMegaFastPrologueDefault = 0;
 
