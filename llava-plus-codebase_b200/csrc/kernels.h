@@ -328,6 +328,9 @@ int linear_split_f32(const LinearArgs& a, cudaStream_t stream);
 constexpr int LINEAR_STREAM_MAX = 16;
 bool linear_streams(const LinearArgs& a);
 int linear_stream_f32(const LinearArgs& a, cudaStream_t stream);
+// Two such products in one launch: a beside a gated unit b of the same rows; a + b on the outputs of a (its epilogue: b's output is not looked at)
+int linear_stream_side_f32(const LinearArgs& a, const LinearArgs& b, cudaStream_t stream);
+int linear_stream_sum_f32(const LinearArgs& a, const LinearArgs& b, cudaStream_t stream);
 // whether a call of these sizes can norm A on its way in: a handful of rows with K % 8 == 0 (the weight-streaming kernel)
 bool linear_fuses_norm(int M, int K);
 int linear_f32(const LinearArgs& a, cudaStream_t stream);

@@ -26,27 +26,42 @@ __device__ __forceinline__ void mma_16x8x16(float (&c)[4], uint32_t a0, uint32_t
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// NT: column tiles of 8 rows of A (0: one row on the FMA pipe). A16: A lies there as bf16 rows of pitch K. GLU: a tile is 8 outputs of a gated unit,
-// rows 0..7 their gate weights and 8..15 their up weights. An SM holds 16 warps: one CTA of 16, or two of 8.
-template <int NT, bool A16, bool GLU, int LS_WARPS>
-__global__ void __launch_bounds__(LS_WARPS * 32, 16 / LS_WARPS) linear_stream_kernel(LinearArgs a) {
-    constexpr int COLS = NT == 0 ? 1 : 8 * NT, OUTS = GLU ? LS_N / 2 : LS_N;   // outputs per tile
+// What a launch computes: a product; a gated unit (a tile is 8 outputs, rows 0..7 their gate weights and 8..15 their up weights); a product `a` and a gated
+// unit `b` of the same rows of A, side by side (the tiles of a, then those of b); the sum of two products on the same outputs (the units of a, then
+// those of b; a's epilogue).
+enum { LS_ONE = 0, LS_GLU = 1, LS_SIDE = 2, LS_SUM = 3 };
+
+// NT: column tiles of 8 rows of A (0: one row on the FMA pipe). A16: A lies there as bf16 rows of pitch K (LS_SUM: looked up for each product).
+// An SM holds 16 warps: one CTA of 16, or two of 8.
+template <int NT, bool A16, int FORM, int LS_WARPS>
+__device__ __forceinline__ void linear_stream_body(const LinearArgs& a, const LinearArgs& b) {
+    constexpr int COLS = NT == 0 ? 1 : 8 * NT;
     __shared__ float red[LS_WARPS][LS_N][COLS + (NT == 0 ? 0 : 1)];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = lane >> 2, kq = (lane & 3) * 8;
-    const int units = (a.K + LS_UNIT - 1) / LS_UNIT, upw = (units + LS_WARPS - 1) / LS_WARPS;   // units per warp and tile
-    const int tiles = (a.N + OUTS - 1) / OUTS, mine = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int units0 = (a.K + LS_UNIT - 1) / LS_UNIT, units = units0 + (FORM == LS_SUM ? (b.K + LS_UNIT - 1) / LS_UNIT : 0);
+    const int upw = (units + LS_WARPS - 1) / LS_WARPS;   // units per warp and tile
+    constexpr int OUTS = FORM == LS_GLU ? LS_N / 2 : LS_N;   // outputs per tile of a
+    const int tiles0 = (a.N + OUTS - 1) / OUTS, tiles = tiles0 + (FORM == LS_SIDE ? (b.N + LS_N / 2 - 1) / (LS_N / 2) : 0);
+    const int mine = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
     const int steps = mine * upw;
-    const __nv_bfloat16* W = reinterpret_cast<const __nv_bfloat16*>(a.W);
 
     uint4 w[2][4][2];
     auto load_w = [&](int s, uint4 (&u)[4][2]) {   // step s: tile s / upw of this CTA, unit (s % upw) * LS_WARPS + warp
-        const int n0 = ((int)blockIdx.x + (s / upw) * (int)gridDim.x) * OUTS, k0 = ((s % upw) * LS_WARPS + warp) * LS_UNIT + kq;
+        int tile = (int)blockIdx.x + (s / upw) * (int)gridDim.x, unit = (s % upw) * LS_WARPS + warp;
+        const bool second = FORM == LS_SIDE ? tile >= tiles0 : FORM == LS_SUM && unit >= units0;
+        const bool pairs = FORM == LS_GLU || (FORM == LS_SIDE && second);
+        if (FORM == LS_SIDE && second) tile -= tiles0;
+        if (FORM == LS_SUM && second) unit -= units0;
+        const LinearArgs& p = second ? b : a;
+        const int N = p.N, K = p.K, n0 = tile * (pairs ? LS_N / 2 : LS_N), k0 = unit * LS_UNIT + kq;
+        const int64_t ldw = p.ldw;
+        const __nv_bfloat16* W = reinterpret_cast<const __nv_bfloat16*>(p.W);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int n = n0 + row + (GLU ? 0 : 8 * h);
-            const __nv_bfloat16* p = W + (size_t)(n < a.N ? n + (GLU ? h * a.N : 0) : 0) * a.ldw + k0;
+            const int n = n0 + row + (pairs ? 0 : 8 * h);
+            const __nv_bfloat16* q = W + (size_t)(n < N ? n + (pairs ? h * N : 0) : 0) * ldw + k0;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) u[c][h] = s < steps && n < a.N && k0 + 32 * c < a.K ? ld_stream_16(p + 32 * c) : make_uint4(0, 0, 0, 0);
+            for (int c = 0; c < 4; ++c) u[c][h] = s < steps && n < N && k0 + 32 * c < K ? ld_stream_16(q + 32 * c) : make_uint4(0, 0, 0, 0);
         }
     };
     load_w(0, w[0]);
@@ -60,15 +75,20 @@ __global__ void __launch_bounds__(LS_WARPS * 32, 16 / LS_WARPS) linear_stream_ke
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[t][i] = 0.f;
     auto step = [&](int s, const uint4 (&u)[4][2]) {
-        const int k0 = ((s % upw) * LS_WARPS + warp) * LS_UNIT + kq;
+        int unit = (s % upw) * LS_WARPS + warp;
+        const bool second = FORM == LS_SUM && unit >= units0;
+        if (second) unit -= units0;
+        const LinearArgs& p = second ? b : a;
+        const int k0 = unit * LS_UNIT + kq, K = p.K;
+        const float* A = p.A;
         if (NT == 0) {
             float x[4][8];
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                const bool in = k0 + 32 * c < a.K;
-                const float4 p = in ? *reinterpret_cast<const float4*>(a.A + k0 + 32 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
-                const float4 q = in ? *reinterpret_cast<const float4*>(a.A + k0 + 32 * c + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-                x[c][0] = p.x; x[c][1] = p.y; x[c][2] = p.z; x[c][3] = p.w; x[c][4] = q.x; x[c][5] = q.y; x[c][6] = q.z; x[c][7] = q.w;
+                const bool in = k0 + 32 * c < K;
+                const float4 f = in ? *reinterpret_cast<const float4*>(A + k0 + 32 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 g = in ? *reinterpret_cast<const float4*>(A + k0 + 32 * c + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+                x[c][0] = f.x; x[c][1] = f.y; x[c][2] = f.z; x[c][3] = f.w; x[c][4] = g.x; x[c][5] = g.y; x[c][6] = g.z; x[c][7] = g.w;
             }
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
@@ -87,6 +107,7 @@ __global__ void __launch_bounds__(LS_WARPS * 32, 16 / LS_WARPS) linear_stream_ke
                 }
             }
         } else {
+            const bool as16 = FORM == LS_SUM ? p.A16 != nullptr : A16;
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
                 const int m = t * 8 + row;
@@ -94,12 +115,12 @@ __global__ void __launch_bounds__(LS_WARPS * 32, 16 / LS_WARPS) linear_stream_ke
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     x[c] = make_uint4(0, 0, 0, 0);
-                    if (m < a.M && k0 + 32 * c < a.K) {
-                        if (A16) {
-                            x[c] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.A16) + (size_t)m * a.K + k0 + 32 * c);
+                    if (m < a.M && k0 + 32 * c < K) {
+                        if (as16) {
+                            x[c] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.A16) + (size_t)m * K + k0 + 32 * c);
                         } else {
-                            const float* p = a.A + (size_t)m * a.lda + k0 + 32 * c;
-                            const float4 f = *reinterpret_cast<const float4*>(p), g = *reinterpret_cast<const float4*>(p + 4);
+                            const float* r = A + (size_t)m * p.lda + k0 + 32 * c;
+                            const float4 f = *reinterpret_cast<const float4*>(r), g = *reinterpret_cast<const float4*>(r + 4);
                             x[c] = make_uint4(pack_bf16(f.x, f.y), pack_bf16(f.z, f.w), pack_bf16(g.x, g.y), pack_bf16(g.z, g.w));
                         }
                     }
@@ -114,7 +135,7 @@ __global__ void __launch_bounds__(LS_WARPS * 32, 16 / LS_WARPS) linear_stream_ke
     };
     auto finish = [&](int s) {   // the last unit of a tile: the warps' sums meet, every thread writes some outputs
         if (s % upw != upw - 1) return;
-        const int n0 = ((int)blockIdx.x + (s / upw) * (int)gridDim.x) * OUTS;
+        const int tile = (int)blockIdx.x + (s / upw) * (int)gridDim.x;
         __syncthreads();   // the previous tile's sums have been read
         if (NT == 0) {
             float v0 = acc[0][0] + acc[0][1], v1 = acc[0][2] + acc[0][3];
@@ -134,19 +155,29 @@ __global__ void __launch_bounds__(LS_WARPS * 32, 16 / LS_WARPS) linear_stream_ke
 #pragma unroll
             for (int i = 0; i < 4; ++i) acc[t][i] = 0.f;
         __syncthreads();
-        const int i = threadIdx.x % OUTS, m = threadIdx.x / OUTS, n = n0 + i;
-        if (m < a.M && m < COLS && n < a.N) {
-            float v = 0.f;
+        const bool pairs = FORM == LS_GLU || (FORM == LS_SIDE && tile >= tiles0);
+        if (pairs) {
+            const LinearArgs& p = FORM == LS_SIDE ? b : a;
+            constexpr int H = LS_N / 2;
+            const int i = threadIdx.x % H, m = threadIdx.x / H, n = (FORM == LS_SIDE ? tile - tiles0 : tile) * H + i;
+            if (m < p.M && m < COLS && n < p.N) {
+                float v = 0.f, u = 0.f;
 #pragma unroll
-            for (int q = 0; q < LS_WARPS; ++q) v += red[q][i][m];
-            if constexpr (GLU) {
-                float u = 0.f;
+                for (int q = 0; q < LS_WARPS; ++q) v += red[q][i][m];
 #pragma unroll
-                for (int q = 0; q < LS_WARPS; ++q) u += red[q][i + OUTS][m];
-                v = glu_act(v, u, a.glu);
-                if (a.out16 != nullptr) reinterpret_cast<__nv_bfloat16*>(a.out16)[(size_t)m * a.ld_out + n] = __float2bfloat16_rn(v);
-                else a.out[(size_t)m * a.ld_out + n] = v;
-            } else linear_store(a.out + (size_t)m * a.ld_out + n, v, a.bias, n, a.act, a.alpha, a.accumulate);
+                for (int q = 0; q < LS_WARPS; ++q) u += red[q][i + H][m];
+                v = glu_act(v, u, p.glu);
+                if (p.out16 != nullptr) reinterpret_cast<__nv_bfloat16*>(p.out16)[(size_t)m * p.ld_out + n] = __float2bfloat16_rn(v);
+                else p.out[(size_t)m * p.ld_out + n] = v;
+            }
+        } else {
+            const int i = threadIdx.x % LS_N, m = threadIdx.x / LS_N, n = tile * LS_N + i;
+            if (m < a.M && m < COLS && n < a.N) {
+                float v = 0.f;
+#pragma unroll
+                for (int q = 0; q < LS_WARPS; ++q) v += red[q][i][m];
+                linear_store(a.out + (size_t)m * a.ld_out + n, v, a.bias, n, a.act, a.alpha, a.accumulate);
+            }
         }
     };
     for (int s = 0; s < steps; s += 2) {
@@ -161,9 +192,18 @@ __global__ void __launch_bounds__(LS_WARPS * 32, 16 / LS_WARPS) linear_stream_ke
     }
 }
 
-template <int NT, bool A16, bool GLU>
-int launch_stream(const LinearArgs& a, cudaStream_t st) {
-    const int outs = GLU ? LS_N / 2 : LS_N, tiles = (a.N + outs - 1) / outs, units = (a.K + LS_UNIT - 1) / LS_UNIT;
+template <int NT, bool A16, bool GLU, int LS_WARPS>
+__global__ void __launch_bounds__(LS_WARPS * 32, 16 / LS_WARPS) linear_stream_kernel(LinearArgs a) {
+    linear_stream_body<NT, A16, GLU ? LS_GLU : LS_ONE, LS_WARPS>(a, a);
+}
+template <int NT, bool A16, int FORM, int LS_WARPS>
+__global__ void __launch_bounds__(LS_WARPS * 32, 16 / LS_WARPS) linear_stream_two_kernel(LinearArgs a, LinearArgs b) {
+    linear_stream_body<NT, A16, FORM, LS_WARPS>(a, b);
+}
+
+// Whether a launch of `tiles` tiles of `units` units runs as one CTA of 16 warps an SM, not two of 8
+template <int NT>
+bool wide_ctas(int tiles, int units) {
     // Two CTAs of 8 warps on an SM, or one of 16: the shorter one of the longest chains that a warp walks, in half units of weights. The end of a tile
     // (two barriers, the warps' sums) takes about half a unit's time, with more than 8 rows a whole one's; in a long stream of tiles whose last units
     // leave some of 8 warps idle (a head of 32000 outputs, K = 1536: 12 units), 16 warps were the faster form all the same. us a step, always 8 warps /
@@ -172,8 +212,23 @@ int launch_stream(const LinearArgs& a, cudaStream_t st) {
     // 202 / 212 / 200.
     const int end = NT == 2 ? 2 : tiles >= 8 * num_sms() && units % 8 != 0 ? 0 : 1;
     const auto chain = [&](int ctas, int warps) { return ((tiles + ctas - 1) / ctas) * (2 * ((units + warps - 1) / warps) + end); };
-    if (chain(num_sms(), 16) <= chain(2 * num_sms(), 8)) B2_CUDA_CHECK(launch_pdl(linear_stream_kernel<NT, A16, GLU, 16>, dim3(std::min(tiles, num_sms())), dim3(512), 0, st, a));
+    return chain(num_sms(), 16) <= chain(2 * num_sms(), 8);
+}
+
+template <int NT, bool A16, bool GLU>
+int launch_stream(const LinearArgs& a, cudaStream_t st) {
+    const int outs = GLU ? LS_N / 2 : LS_N, tiles = (a.N + outs - 1) / outs;
+    if (wide_ctas<NT>(tiles, (a.K + LS_UNIT - 1) / LS_UNIT)) B2_CUDA_CHECK(launch_pdl(linear_stream_kernel<NT, A16, GLU, 16>, dim3(std::min(tiles, num_sms())), dim3(512), 0, st, a));
     else B2_CUDA_CHECK(launch_pdl(linear_stream_kernel<NT, A16, GLU, 8>, dim3(std::min(tiles, 2 * num_sms())), dim3(256), 0, st, a));
+    B2_LAUNCH_CHECK();
+    return 0;
+}
+template <int NT, bool A16, int FORM>
+int launch_two(const LinearArgs& a, const LinearArgs& b, cudaStream_t st) {
+    const int tiles = (a.N + LS_N - 1) / LS_N + (FORM == LS_SIDE ? (b.N + LS_N / 2 - 1) / (LS_N / 2) : 0);
+    const int units = (a.K + LS_UNIT - 1) / LS_UNIT + (FORM == LS_SUM ? (b.K + LS_UNIT - 1) / LS_UNIT : 0);
+    if (wide_ctas<NT>(tiles, units)) B2_CUDA_CHECK(launch_pdl(linear_stream_two_kernel<NT, A16, FORM, 16>, dim3(std::min(tiles, num_sms())), dim3(512), 0, st, a, b));
+    else B2_CUDA_CHECK(launch_pdl(linear_stream_two_kernel<NT, A16, FORM, 8>, dim3(std::min(tiles, 2 * num_sms())), dim3(256), 0, st, a, b));
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -190,6 +245,20 @@ static int stream_rows(const LinearArgs& a, cudaStream_t st) {
     if (a.M == 1) return launch_stream<0, false, GLU>(a, st);
     if (a.M <= 8) return a.A16 != nullptr ? launch_stream<1, true, GLU>(a, st) : launch_stream<1, false, GLU>(a, st);
     return a.A16 != nullptr ? launch_stream<2, true, GLU>(a, st) : launch_stream<2, false, GLU>(a, st);
+}
+
+int linear_stream_side_f32(const LinearArgs& a, const LinearArgs& b, cudaStream_t st) {
+    B2_CHECK_ARG(linear_streams(a) && linear_streams(b) && !a.gated && b.gated && a.M == b.M && a.K == b.K && a.A == b.A && a.A16 == b.A16 && a.lda == b.lda && a.round_a == b.round_a,
+                 "linear_stream_side: two products that do not share their rows");
+    if (a.M == 1) return launch_two<0, false, LS_SIDE>(a, b, st);
+    if (a.M <= 8) return a.A16 != nullptr ? launch_two<1, true, LS_SIDE>(a, b, st) : launch_two<1, false, LS_SIDE>(a, b, st);
+    return a.A16 != nullptr ? launch_two<2, true, LS_SIDE>(a, b, st) : launch_two<2, false, LS_SIDE>(a, b, st);
+}
+
+int linear_stream_sum_f32(const LinearArgs& a, const LinearArgs& b, cudaStream_t st) {
+    B2_CHECK_ARG(linear_streams(a) && linear_streams(b) && !a.gated && !b.gated && a.M == b.M && a.N == b.N && a.round_a == b.round_a, "linear_stream_sum: two products of other sizes");
+    if (a.M == 1) return launch_two<0, false, LS_SUM>(a, b, st);
+    return a.M <= 8 ? launch_two<1, false, LS_SUM>(a, b, st) : launch_two<2, false, LS_SUM>(a, b, st);
 }
 
 int linear_stream_f32(const LinearArgs& a, cudaStream_t st) { return a.gated ? stream_rows<true>(a, st) : stream_rows<false>(a, st); }

@@ -203,9 +203,9 @@ struct Lin {  // one Linear call on the model's compute dtype
     // whether a product of these sizes can take its input through a dynamic-tanh norm on the way in (a decode step's weight-streaming kernel)
     bool fuses_norm(int K, int M) const { return linear_fuses_norm(M, K) && (m->seq->d.compute == B2_COMPUTE_F32 || M < tc_min_rows() || !tc_enabled()); }
     // a16: A is already there as bf16 rows of pitch K (the producing kernel wrote them): no cast. norm: A passes it on the way in (fuses_norm)
-    int operator()(const float* A, int64_t lda, const DevBuf& W, int N, int K, float* out, int64_t ldo, int M, int act = LIN_NONE,
-                   float alpha = 1.f, int accumulate = 0, const float* bias = nullptr, size_t w_row0 = 0, const void* bias16 = nullptr,
-                   const void* a16 = nullptr, const DytNorm* norm = nullptr) const {
+    LinearArgs args(const float* A, int64_t lda, const DevBuf& W, int N, int K, float* out, int64_t ldo, int M, int act = LIN_NONE,
+                    float alpha = 1.f, int accumulate = 0, const float* bias = nullptr, size_t w_row0 = 0, const void* a16 = nullptr,
+                    const DytNorm* norm = nullptr) const {
         LinearArgs a;
         const SeqModel& s = *m->seq;
         a.A = A; a.lda = lda; a.ldw = K; a.w_dtype = s.w_dtype;
@@ -215,6 +215,13 @@ struct Lin {  // one Linear call on the model's compute dtype
         if (norm != nullptr) a.norm = *norm;
         a.A16 = a16;
         a.parts = s.lin_parts.p; a.parts_bytes = s.lin_parts.bytes;
+        return a;
+    }
+    int operator()(const float* A, int64_t lda, const DevBuf& W, int N, int K, float* out, int64_t ldo, int M, int act = LIN_NONE,
+                   float alpha = 1.f, int accumulate = 0, const float* bias = nullptr, size_t w_row0 = 0, const void* bias16 = nullptr,
+                   const void* a16 = nullptr, const DytNorm* norm = nullptr) const {
+        const SeqModel& s = *m->seq;
+        const LinearArgs a = args(A, lda, W, N, K, out, ldo, M, act, alpha, accumulate, bias, w_row0, a16, norm);
         if (tc_enabled() && linear_splits(a)) return linear_split_f32(a, st);
         if (tc_enabled() && linear_streams(a)) return linear_stream_f32(a, st);
         // bf16 compute, a portion of a prompt: the tcgen05 GEMM on a bf16 copy of A (weights are stored with their rows
@@ -407,12 +414,56 @@ static int latent_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeight
     return lin(y, L.pv, W.o_w, width, L.pv, target, width, R, LIN_NONE, alpha, accumulate);
 }
 
+// The gated unit of a dense feed-forward: the bounded one a(g) (u + 1), or gelu(g) u
+static GluAct glu_of(const b2_seq_layer_desc& d) {
+    if (d.ff_kind != B2_FF_GELU_GLU) return GluAct{d.ff_act_slope, d.ff_limit, 1.f};
+    GluAct act;
+    act.kind = GLU_GELU_TANH;
+    return act;
+}
+// its first product for a handful of rows, the unit inside; bf16 rows out where the second product (onto `target`) reads those
+static LinearArgs glu_rows_args(const Lin& lin, const SeqLayerInfo& L, SeqWeights& W, const SubIn& in, float* target, int R) {
+    const SeqModel& s = *lin.m->seq;
+    LinearArgs up = lin.args(in.h, s.d.width, W.up_w, L.d.ff, s.d.width, s.ffa.as<float>(), L.d.ff, R, LIN_NONE, 1.f, 0, nullptr, 0, in.h16);
+    up.gated = 1; up.glu = glu_of(L.d);
+    if (R > 1 && lin.tensor_cores(s.d.width, L.d.ff, target, s.d.width, R)) up.out16 = s.ff.p;
+    return up;
+}
+
+// A handful of rows through a parallel block: mixer and feed-forward read the same rows and add onto the same ones, so the feed-forward's two
+// products ride in the launches of the mixer's first and last (linear_stream.cu): two launches a layer fewer, each 1.5 to 3 us of start, ragged last
+// tiles and end. 48 steps of four mixed layers, width 2048 (us, before -> now): one slot 9773 -> 9436, 8 slots 12293 -> 12106.
+struct RowFeedForward { LinearArgs up, down; };
+static LinearArgs gqa_first(const Lin& lin, const SeqLayerInfo& L, SeqWeights& W, const SubIn& in, int R) {
+    const SeqModel& s = *lin.m->seq;
+    return lin.args(in.h, s.d.width, W.lproj_w, L.lproj, s.d.width, s.proj.as<float>(), L.lproj_ld, R, LIN_NONE, 1.f, 0, W.qkv_b.as<float>(), 0, in.h16, in.norm);
+}
+static LinearArgs gla_first(const Lin& lin, const SeqLayerInfo& L, SeqWeights& W, const float* h, int R) {
+    const SeqModel& s = *lin.m->seq;
+    return lin.args(h, s.d.width, W.gla_w, L.pproj, s.d.width, s.proj.as<float>(), L.pproj_ld, R);
+}
+// its arguments, where every one of the four products streams its weights
+static bool row_feed_forward(const Lin& lin, const SeqLayerInfo& L, SeqWeights& W, const SubIn& in, float* target, float alpha, int R, RowFeedForward& f) {
+    const SeqModel& s = *lin.m->seq;
+    const b2_seq_layer_desc& d = L.d;
+    const int width = s.d.width, ff = d.ff;
+    if (ff <= 0 || !is_glu(d.ff_kind) || in.norm != nullptr || !tc_enabled() || (d.type != B2_MIXER_GQA_ATTN && d.type != B2_MIXER_GLA)) return false;
+    f.up = glu_rows_args(lin, L, W, in, target, R);
+    const float* fa = f.up.out16 != nullptr ? nullptr : f.up.out;
+    f.down = lin.args(fa, ff, W.down_w, width, ff, target, width, R, LIN_NONE, alpha, 1, nullptr, 0, f.up.out16);
+    const bool gqa = d.type == B2_MIXER_GQA_ATTN;
+    const int inner = gqa ? L.ng : L.pv;
+    const LinearArgs first = gqa ? gqa_first(lin, L, W, in, R) : gla_first(lin, L, W, in.h, R);
+    return first.A16 == f.up.A16 && linear_streams(first) && linear_streams(f.up) && linear_streams(f.down) &&
+           linear_streams(lin.args(s.gated.as<float>(), inner, W.o_w, width, inner, target, width, R, LIN_NONE, alpha, 1));
+}
+
 // Attention with grouped key/value heads, biases on q / k / v, a short convolution on q / k / v, an optional weighted norm of the q / k heads, rotary q / k in
 // either pair layout, optionally rotated values, a masked softmax with an optional fixed sink, and a sigmoid output gate per channel or
 // per head. With two maps (differential attention) the projection rows were ordered [map][head][dim] when the tensors were set, so the
 // maps are simply twice the query and key heads over the same value heads, and a head's two outputs are joined after the softmax.
 static int gqa_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeights& W, SeqLayerState& S, const SubIn& in, float* target, float alpha,
-                     int accumulate, int R, int nseg, int slot, int ctx_end, cudaStream_t st) {
+                     int accumulate, int R, int nseg, int slot, int ctx_end, cudaStream_t st, const RowFeedForward* ff = nullptr) {
     SeqModel& s = *m->seq;
     SeqState& state = *kv->seq;
     const b2_seq_layer_desc& d = L.d;
@@ -424,7 +475,8 @@ static int gqa_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeights& 
     const int32_t* row_slot = s.row_slot.as<int32_t>();
     const int32_t* row_pos = s.row_pos.as<int32_t>();
     float* proj = s.proj.as<float>();  // [R, nq | nk | nv | gate]
-    B2_TRY(lin(in.h, width, W.lproj_w, L.lproj, width, proj, L.lproj_ld, R, LIN_NONE, 1.f, 0, W.qkv_b.as<float>(), 0, W.qkv_b16.p, in.h16, in.norm));
+    if (ff != nullptr) B2_TRY(linear_stream_side_f32(gqa_first(lin, L, W, in, R), ff->up, st));
+    else B2_TRY(lin(in.h, width, W.lproj_w, L.lproj, width, proj, L.lproj_ld, R, LIN_NONE, 1.f, 0, W.qkv_b.as<float>(), 0, W.qkv_b16.p, in.h16, in.norm));
     float* qkv = proj;
     int64_t ldc = L.lproj_ld;
     if (d.ga_conv >= 1) {
@@ -470,6 +522,7 @@ static int gqa_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeights& 
     if (out16) aa.out16 = s.a16.p;
     portion_of(s, nseg, slot, ctx_end, aa);
     B2_TRY(attn_bias_f32(aa, st));
+    if (out16 && ff != nullptr) return linear_stream_sum_f32(ff->down, lin.args(nullptr, 0, W.o_w, width, L.ng, target, width, R, LIN_NONE, alpha, accumulate, nullptr, 0, s.a16.p), st);
     if (out16) return lin(nullptr, 0, W.o_w, width, L.ng, target, width, R, LIN_NONE, alpha, accumulate, nullptr, 0, nullptr, s.a16.p);
     const float* yo = s.y.as<float>();
     float* gated = s.gated.as<float>();
@@ -491,19 +544,21 @@ static int gqa_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeights& 
         B2_TRY(head_gate_f32(yo, L.ng, gates, L.lproj_ld, gated, L.ng, R, H, dv, st));
         yo = gated;
     }
+    if (ff != nullptr) return linear_stream_sum_f32(ff->down, lin.args(yo, L.ng, W.o_w, width, L.ng, target, width, R, LIN_NONE, alpha, accumulate), st);
     return lin(yo, L.ng, W.o_w, width, L.ng, target, width, R, LIN_NONE, alpha, accumulate);
 }
 
 // Gated linear attention: one fused projection [q | k | v | g | a1], the decay logits through the second low-rank matrix, the
 // recurrence (decay, scaled query and state in fp32), per-head RMS norm with the gate, out-projection.
 static int gla_mixer(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, SeqLayerState& S, const float* h, float* target, float alpha, int accumulate,
-                     int R, int nseg, cudaStream_t st) {
+                     int R, int nseg, cudaStream_t st, const RowFeedForward* ff = nullptr) {
     SeqModel& s = *m->seq;
     const b2_seq_layer_desc& d = L.d;
     const Lin lin{m, st};
     const int width = s.d.width, H = d.gl_heads, dk = d.gl_dim, dv = d.gl_vdim;
     float* proj = s.proj.as<float>();
-    B2_TRY(lin(h, width, W.gla_w, L.pproj, width, proj, L.pproj_ld, R));
+    if (ff != nullptr) B2_TRY(linear_stream_side_f32(gla_first(lin, L, W, h, R), ff->up, st));
+    else B2_TRY(lin(h, width, W.gla_w, L.pproj, width, proj, L.pproj_ld, R));
     float* z = s.wlog.as<float>();   // [R, heads * dim] decay logits without their bias (the recurrence adds it in fp32)
     B2_TRY(lin(proj + 2 * L.pq + 2 * L.pv, L.pproj_ld, W.a2_w, L.pq, d.gl_rank, z, L.pq, R));
     ScanArgs sa;
@@ -522,6 +577,7 @@ static int gla_mixer(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, SeqLayer
     B2_TRY(linear_scan_f32(sa, st));
     B2_TRY(gated_group_rmsnorm_f32(s.y.as<float>(), L.pv, proj + 2 * L.pq + L.pv, L.pproj_ld, W.gnorm.as<float>(), s.gated.as<float>(), L.pv, R, L.pv, dv,
                                    0, s.d.norm_eps, st, 1));
+    if (ff != nullptr) return linear_stream_sum_f32(ff->down, lin.args(s.gated.as<float>(), L.pv, W.o_w, width, L.pv, target, width, R, LIN_NONE, alpha, accumulate), st);
     return lin(s.gated.as<float>(), L.pv, W.o_w, width, L.pv, target, width, R, LIN_NONE, alpha, accumulate);
 }
 
@@ -736,18 +792,13 @@ static int seq_feed_forward(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, c
         B2_TRY(polynorm_f32(s.ff.as<float>(), ffl, W.up_b.as<float>(), W.act_coef.as<float>(), s.ffa.as<float>(), d.ff, R, d.ff, eps, st));
         return lin(s.ffa.as<float>(), d.ff, W.down_w, width, d.ff, target, width, R, LIN_NONE, alpha, accumulate, W.down_b.as<float>(), 0, W.down_b16.p);
     }
-    const GluAct clamp_glu{d.ff_act_slope, d.ff_limit, 1.f};   // the bounded gated unit a(g) (u + 1)
     if (is_glu(d.ff_kind)) {
         // [gate | up] in one matrix, then the gated unit; a decode step of one row takes product and unit in one launch (more rows would
         // stream the matrix once per row there)
         const int ff = d.ff, ffl = (2 * ff + 7) / 8 * 8;
-        GluAct act = clamp_glu;
-        if (d.ff_kind == B2_FF_GELU_GLU) { act = GluAct{}; act.kind = GLU_GELU_TANH; }
-        LinearArgs up;   // a handful of rows: both products and the unit in one stream of the weights
-        up.A = h; up.lda = width; up.A16 = in.h16; up.W = W.up_w.p; up.ldw = width; up.w_dtype = s.w_dtype; up.out = s.ffa.as<float>(); up.ld_out = ff;
-        up.M = R; up.N = ff; up.K = width; up.round_a = s.d.compute == B2_COMPUTE_BF16; up.gated = 1; up.glu = act;
+        const GluAct act = glu_of(d);
+        const LinearArgs up = glu_rows_args(lin, L, W, in, target, R);   // a handful of rows: both products and the unit in one stream of the weights
         if (tc_enabled() && linear_streams(up)) {
-            if (R > 1 && lin.tensor_cores(width, ff, target, width, R)) up.out16 = s.ff.p;   // bf16 rows for the second product
             B2_TRY(linear_stream_f32(up, st));
             return lin(up.out16 != nullptr ? nullptr : s.ffa.as<float>(), ff, W.down_w, width, ff, target, width, R, LIN_NONE, alpha, accumulate, nullptr, 0, nullptr,
                        up.out16);
@@ -782,7 +833,7 @@ static int seq_feed_forward(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, c
     }
     const int E = d.moe_experts, top = d.moe_top, ff = d.ff;
     const bool gated = d.moe_act != B2_MOE_ACT_RELU_SQ;
-    const GluAct act = d.moe_act == B2_MOE_ACT_CLAMP_GLU ? clamp_glu : GluAct{};   // the experts' gated unit
+    const GluAct act = d.moe_act == B2_MOE_ACT_CLAMP_GLU ? GluAct{d.ff_act_slope, d.ff_limit, 1.f} : GluAct{};   // the experts' gated unit
     const int un = gated ? 2 * ff : ff;   // rows of an expert's first matrix: [gate | up], or up alone
     const int round_a = s.d.compute == B2_COMPUTE_BF16;
     const int choices = E + d.moe_identity;   // rows of the router: the experts, then the identity experts
@@ -925,21 +976,23 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
                 DytNorm n1, n2;
                 SubIn in1, in2;
                 B2_TRY(parallel_inputs(m, L, W, x, R, two, L.lproj > 0 ? L.lproj : L.pproj, x, n1, n2, in1, in2, st));
+                RowFeedForward rf;
+                const RowFeedForward* ride = !two && row_feed_forward(lin, L, W, in1, x, rm, R, rf) ? &rf : nullptr;
                 if (early) B2_TRY(gelu_up(m, L, W, in2, x, R, st));   // reads x (through its norm) before the mixer's output joins it
                 if (d.type == B2_MIXER_LATENT_ATTN) {
                     SeqLayerState& KS = d.la_kv_from > 0 ? state.layer[s.runs[ri].kv_run] : S;
                     B2_TRY(latent_mixer(m, kv, L, W, S, KS, in1.h, x, rm, 1, R, nseg, slot, ctx_end, st));
                 } else if (d.type == B2_MIXER_GQA_ATTN) {
-                    B2_TRY(gqa_mixer(m, kv, L, W, S, in1, x, rm, 1, R, nseg, slot, ctx_end, st));
+                    B2_TRY(gqa_mixer(m, kv, L, W, S, in1, x, rm, 1, R, nseg, slot, ctx_end, st, ride));
                 } else if (d.type == B2_MIXER_MLSTM || d.type == B2_MIXER_DELTA) {
                     B2_TRY(memory_mixer(m, L, W, S, in1, x, rm, 1, R, nseg, st));
                 } else if (d.type == B2_MIXER_GLA) {
-                    B2_TRY(gla_mixer(m, L, W, S, in1.h, x, rm, 1, R, nseg, st));
+                    B2_TRY(gla_mixer(m, L, W, S, in1.h, x, rm, 1, R, nseg, st, ride));
                 } else {
                     B2_TRY(hgrn2_mixer(m, L, W, S, in1.h, x, rm, 1, R, nseg, st));
                 }
                 if (early) B2_TRY(gelu_down(m, L, W, x, rm, 1, R, st));
-                else if (d.ff > 0) B2_TRY(seq_feed_forward(m, L, W, in2, x, rm, 1, R, st));
+                else if (d.ff > 0 && ride == nullptr) B2_TRY(seq_feed_forward(m, L, W, in2, x, rm, 1, R, st));
                 if (resid_out != nullptr)
                     B2_CUDA_CHECK(cudaMemcpyAsync(resid_out + ri * (size_t)R * width, x, (size_t)R * width * F4, cudaMemcpyDeviceToDevice, st));
                 continue;

@@ -8,7 +8,7 @@ import torch
 import test_kuvelix_gpu as KV
 import test_ramosun_gpu as RA
 from oracle import sofopel_oracle as O
-from test_sofopel_gpu import config, tokens_for, win
+from test_sofopel_gpu import config, diff, gla, tokens_for, win
 
 pytestmark = pytest.mark.gpu
 
@@ -118,3 +118,14 @@ def test_several_tiles_a_block(width, vocab, n):
 @pytest.mark.parametrize("n", [1, 8, 9, 16])
 def test_several_gated_tiles_a_block(width, ff, n, monkeypatch):
     test_streamed_weights_equal_the_fma_kernels(width, ff, n, monkeypatch)
+
+
+# A feed-forward whose products run in the launches of the mixer's first and last: tiles of both kinds in a launch, units of two products in a sum
+@pytest.mark.parametrize("mixer", ["gla", "diff", "win"])
+@pytest.mark.parametrize("width,ff", [(136, 72), (264, 1048), (1160, 272), (2048, 136)])
+@pytest.mark.parametrize("n", [1, 3, 4, 8, 9, 16])
+def test_products_that_share_a_launch(mixer, width, ff, n, monkeypatch):
+    mix = {"gla": gla(3, 16, 40), "diff": diff(4, 2, 16, 24, 3, 13, 8), "win": win(5, 1, 24, 40, 11, 3, 8)}[mixer]
+    cfg = config([dict(mix, mlp={"kind": "dense", "ff": ff, "limit": 7.0})], width=width, vocab=101)
+    w = O.random_weights(cfg, seed=5)
+    both_ways(lambda: residuals(cfg, w, n, 2), monkeypatch, bound(width, ff, 3 * 40, 4 * 24))
