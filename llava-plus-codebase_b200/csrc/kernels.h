@@ -313,17 +313,21 @@ struct LinearArgs {
     int round_a = 0;                             // round A to bf16 first (bf16 compute: the product is bf16 x bf16 -> fp32)
     DytNorm norm;                                // norm.alpha non-null: A passes this norm while it is staged (linear_fuses_norm calls only)
     void* parts = nullptr; size_t parts_bytes = 0;   // scratch of linear_split_f32
+    const void* W16 = nullptr;                   // fp32 W whose values all are bf16 ones: the same as bf16, pitch K (K % 8 == 0), for linear_split_f32
     int gated = 0; GluAct glu;                   // linear_stream_f32 only: W = [gate | up] of N rows each, out = glu_act(gate, up); no act, bias, alpha
     void* out16 = nullptr;                       // with gated: bf16 rows of pitch ld_out in place of out
     const void* A16 = nullptr;                   // the same rows already rounded to bf16, pitch K (linear_stream_f32 reads these when there are 2 or more)
 };
-// True fp32, a portion of a prompt (linear_split.cu): whether a call runs on the tensor cores as products of bf16 parts. Scratch: the parts of A and
-// of at least 128 rows of W, linear_split_bytes each. Up to 8 rows the weight-streaming kernel is the faster one; the tiled FMA kernel never was (a
+// True fp32, a portion of a prompt (linear_split.cu): whether a call runs on the tensor cores as products of bf16 parts. Scratch: the parts of A
+// and, without W16, of at least 128 rows of W, linear_split_bytes each. Up to 8 rows the weight-streaming kernel is the faster one; the tiled FMA kernel never was (a
 // fp32 layer of width 1024 with everything on it / on the tensor cores: 24 rows 952 / 243 us, 100 rows 928 / 251 us).
 constexpr int LINEAR_SPLIT_MIN_ROWS = 9;
 bool linear_splits(const LinearArgs& a);
 size_t linear_split_bytes(int rows, int K);
 int linear_split_f32(const LinearArgs& a, cudaStream_t stream);
+// *other := 1 if a value of w is not a bf16 one (n % 4 == 0; other is not cleared); the high halves of fp32 values, which are the values then
+int bf16_values(const float* w, int64_t n, int* other, cudaStream_t stream);
+int high_halves(const float* w, int64_t n, void* out, cudaStream_t stream);
 // A handful of rows on bf16 weights (linear_stream.cu): whether a call is one of those that stream their weights through registers
 constexpr int LINEAR_STREAM_MAX = 16;
 bool linear_streams(const LinearArgs& a);

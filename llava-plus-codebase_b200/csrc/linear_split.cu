@@ -1,16 +1,21 @@
 // Linears in true fp32 for portions of a prompt, on the tensor cores: out[M, N] = alpha act(A[M, K] W[N, K]^T + bias) (+ out), all fp32, with both
-// operands as three bf16 parts and six products of each pair (split.cuh). The tensor core cuts its fp32 sums off after every step of 16, so an
-// accumulator spans one block of 64 of K only; the blocks are added up in fp32 registers.
-//   1. split_rows_kernel writes the parts of A and of W (per call: the weights stay fp32 in memory, and a pass over them is short beside the product);
-//      a W whose parts exceed the scratch goes in blocks of rows;
-//   2. linear_split_kernel: one tile of 128 x BN per CTA, warp 0 TMA producer (a stage: the three parts of 64 columns of A and W), warp 1 MMA
-//      issuer, warps 2..9 take every block's accumulator out of TMEM (two of them, so that the next block's products run meanwhile).
-// What bounds it: the stream of parts into the SM (96 KB per block at BN = 128 against 1536 clk of products), then too few tiles at small N.
-// 600 rows, 13 products of a state-space + RWKV pair of width 1024 (33 GFLOP): 2512 us on linear_tiled_kernel -> 413 us and 86 us of cutting; the
-// pair's error against 64 bits falls from 1.4e-6 to 3.6e-7.
+// operands as bf16 parts (split.cuh): A in three, W in three and six products of each pair, or, where every value of W is a bf16 one (the weights of a
+// bf16 checkpoint, looked at when the model is finalized), W as it is and the three products that are not zero: the same sums. The tensor core cuts
+// its fp32 sums off after every step of 16, so an accumulator spans one block of 64 of K only; the blocks are added up in fp32 registers.
+//   1. split_rows_kernel writes the parts of A, and of a W of three parts, per call: a W whose parts exceed the scratch goes in blocks of rows;
+//   2. linear_split_kernel: one tile of 128 x BN per CTA, or per cluster whose CTAs share out K; warp 0 TMA producer (a stage: the parts of 64 columns of
+//      A and W), warp 1 MMA issuer, warps 2..9 take every block's accumulator out of TMEM (four of them, two at BN = 256). The sums pass through
+//      shared memory, the cluster's meet there, and leave in whole rows.
+// What bounds it: the stream of parts into the SM, some 40 B a clock (64 KB a block at BN = 128 with W in one part, 768 clk of products). Splitting A
+// inside the kernel (32 KB a block) was slower: 8 warps convert a block of 128 x 64 in 1300 clk (600 x 1024 x 4096: 60 us, the parts by TMA 41, K over
+// a cluster 24).
+// 600 rows, 13 products of a state-space + RWKV pair of width 1024 (33 GFLOP): 2512 us on linear_tiled_kernel -> 413 us and 86 us of cutting on tiles of
+// 64 and 128 columns, six products and one CTA a tile; the whole call 764 -> 576 us with W in one part, tiles of up to 256 columns and clusters. The pair's
+// error against 64 bits: 1.4e-6, 3.6e-7 on the tensor cores.
 #include <cuda.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "kernels.h"
 #include "split.cuh"
@@ -21,12 +26,16 @@ int make_tmap_parts(CUtensorMap* map, const void* ptr, int pitch, int64_t rows, 
 
 namespace {
 
-constexpr int LX_M = 128, LX_K = 64, LX_THREADS = 320;
+constexpr int LX_M = 128, LX_K = 64, LX_THREADS = 320, LX_MAX_CLUSTER = 8;
 
-template <int BN>
+// WP: parts of W (3, or 1: W holds bf16 values)
+template <int BN, int WP>
 struct LxCfg {
-    static constexpr int A_BYTES = 3 * LX_M * 128, B_BYTES = 3 * BN * 128, STAGE = A_BYTES + B_BYTES, STAGES = BN == 128 ? 2 : 3;
-    static constexpr int SMEM = STAGES * STAGE + 1024 + 128;
+    static constexpr int A_BYTES = 3 * LX_M * 128, B_BYTES = WP * BN * 128, STAGE = A_BYTES + B_BYTES, STAGES = STAGE > 72 * 1024 ? 2 : STAGE > 56 * 1024 ? 3 : 4;
+    static constexpr int ACCS = BN == 256 ? 2 : 4;                     // accumulators in TMEM
+    static constexpr int PITCH = BN + 4;                               // floats between rows of the tile of sums, which takes the ring's place
+    static constexpr int SMEM = STAGES * STAGE + 1024 + 256;
+    static_assert(LX_M * PITCH * 4 <= STAGES * STAGE, "the sums fit into the ring");
 };
 
 // rows of fp32 -> [part][rows][pitch] bf16, entries past K zero
@@ -61,27 +70,36 @@ __device__ __noinline__ void lx_plain(const float* x, const float* w, int64_t ld
     }
 }
 
-template <int BN>
-__global__ void __launch_bounds__(LX_THREADS, 1) linear_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w, LinearArgs a) {
-    using Cfg = LxCfg<BN>;
+__device__ __forceinline__ float4 lx_ld_remote4(const float* p, int rank) {
+    uint32_t at;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+    return v;
+}
+
+// grid: tiles x S, clusters of S CTAs that share out the blocks of K, `per` each
+template <int BN, int WP>
+__global__ void __launch_bounds__(LX_THREADS, 1) linear_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w, LinearArgs a, int S, int per) {
+    using Cfg = LxCfg<BN, WP>;
     constexpr int CH = BN / 2;   // columns per epilogue thread
     extern __shared__ uint8_t lx_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(lx_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::STAGES * Cfg::STAGE);
-    uint64_t *full = bars, *empty = bars + Cfg::STAGES, *acc_full = bars + 2 * Cfg::STAGES /*[2]*/, *acc_empty = acc_full + 2 /*[2]*/;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int num_m = (a.M + LX_M - 1) / LX_M, m0 = (int)(blockIdx.x % num_m) * LX_M, n0 = (int)(blockIdx.x / num_m) * BN;
-    const int blocks = (a.K + LX_K - 1) / LX_K;
+    uint64_t *full = bars, *empty = bars + Cfg::STAGES, *acc_full = bars + 2 * Cfg::STAGES, *acc_empty = acc_full + Cfg::ACCS;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + Cfg::ACCS);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)blockIdx.x % S, tile = (int)blockIdx.x / S;
+    const int num_m = (a.M + LX_M - 1) / LX_M, m0 = tile % num_m * LX_M, n0 = tile / num_m * BN;
+    const int k_blocks = (a.K + LX_K - 1) / LX_K, b0 = rank * per, blocks = min(per, k_blocks - b0);
 
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tm_a);
         tma_prefetch_desc(&tm_w);
         for (int s = 0; s < Cfg::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); }
+        for (int i = 0; i < Cfg::ACCS; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); }
         fence_barrier_init();
     }
-    if (warp == 1) { tmem_alloc(tmem_slot, 2 * BN); tmem_relinquish(); }
+    if (warp == 1) { tmem_alloc(tmem_slot, Cfg::ACCS * BN); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -97,8 +115,8 @@ __global__ void __launch_bounds__(LX_THREADS, 1) linear_split_kernel(const __gri
                 mbar_wait(&empty[stage], phase ^ 1);
                 uint8_t* d = smem + stage * Cfg::STAGE;
                 mbar_arrive_expect_tx(&full[stage], Cfg::STAGE);
-                for (int p = 0; p < 3; ++p) tma_load_3d(d + p * LX_M * 128, &tm_a, &full[stage], b * LX_K, m0, p);
-                for (int p = 0; p < 3; ++p) tma_load_3d(d + Cfg::A_BYTES + p * BN * 128, &tm_w, &full[stage], b * LX_K, n0, p);
+                for (int p = 0; p < 3; ++p) tma_load_3d(d + p * LX_M * 128, &tm_a, &full[stage], (b0 + b) * LX_K, m0, p);
+                for (int p = 0; p < WP; ++p) tma_load_3d(d + Cfg::A_BYTES + p * BN * 128, &tm_w, &full[stage], (b0 + b) * LX_K, n0, p);
                 if (++stage == Cfg::STAGES) { stage = 0; phase ^= 1; }
             }
         }
@@ -110,83 +128,97 @@ __global__ void __launch_bounds__(LX_THREADS, 1) linear_split_kernel(const __gri
         int stage = 0;
         uint32_t phase = 0;
         for (int b = 0; b < blocks; ++b) {
-            mbar_wait(&acc_empty[b & 1], ((b >> 1) & 1) ^ 1);
+            const int ac = b % Cfg::ACCS;
+            mbar_wait(&acc_empty[ac], ((b / Cfg::ACCS) & 1) ^ 1);
             mbar_wait(&full[stage], phase);
             tc_fence_after();
             const uint32_t s = smem_u32(smem + stage * Cfg::STAGE);
             const uint64_t da = make_sw128_kmajor_desc(s), db = make_sw128_kmajor_desc(s + Cfg::A_BYTES);
-#pragma unroll 1
-            for (int i = 0; i < 6; ++i) {
-                const uint32_t pa = (SPLIT_A >> (2 * i)) & 3u, pb = (SPLIT_B >> (2 * i)) & 3u;
-                if (leader)
+            if (leader) {
+#pragma unroll
+                for (int i = 0; i < (WP == 1 ? 3 : 6); ++i) {   // (W's one part: lo, mid, hi of A in turn)
+                    const uint32_t pa = WP == 1 ? 2 - i : (SPLIT_A >> (2 * i)) & 3u, pb = WP == 1 ? 0 : (SPLIT_B >> (2 * i)) & 3u;
 #pragma unroll
                     for (int k = 0; k < LX_K / 16; ++k)
-                        umma_bf16(tm + (b & 1) * BN, da + (pa * (LX_M * 8) + 2 * k), db + (pb * (BN * 8) + 2 * k), idesc, (i | k) != 0 ? 1u : 0u);
-            }
-            if (leader) {
+                        umma_bf16(tm + ac * BN, da + (pa * (LX_M * 8) + 2 * k), db + (pb * (BN * 8) + 2 * k), idesc, (i | k) != 0 ? 1u : 0u);
+                }
                 umma_commit(&empty[stage]);
-                umma_commit(&acc_full[b & 1]);
+                umma_commit(&acc_full[ac]);
             }
             __syncwarp();
             if (++stage == Cfg::STAGES) { stage = 0; phase ^= 1; }
         }
     } else {
-        const int q = warp & 3, half = (warp - 2) >> 2, m = m0 + q * 32 + lane;
+        const int q = warp & 3, half = (warp - 2) >> 2;
         float acc[CH];
 #pragma unroll
         for (int i = 0; i < CH; ++i) acc[i] = 0.f;
         for (int b = 0; b < blocks; ++b) {
-            mbar_wait(&acc_full[b & 1], (b >> 1) & 1);
+            const int ac = b % Cfg::ACCS;
+            mbar_wait(&acc_full[ac], (b / Cfg::ACCS) & 1);
             tc_fence_after();
 #pragma unroll
             for (int c = 0; c < CH / 32; ++c) {
                 uint32_t v[32];
                 __syncwarp();
-                tmem_ld_32x32(tm + (static_cast<uint32_t>(q * 32) << 16) + (b & 1) * BN + half * CH + c * 32, v);
+                tmem_ld_32x32(tm + (static_cast<uint32_t>(q * 32) << 16) + ac * BN + half * CH + c * 32, v);
                 tmem_ld_wait();
 #pragma unroll
                 for (int i = 0; i < 32; ++i) acc[c * 32 + i] += __uint_as_float(v[i]);
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[b & 1]);
+            if (lane == 0) mbar_arrive(&acc_empty[ac]);
         }
-        bool plain = false;
+        // (the last products are done, so nothing reads the ring any more and no copy is on its way)
+        float* row = reinterpret_cast<float*>(smem) + (q * 32 + lane) * Cfg::PITCH + half * CH;
 #pragma unroll
-        for (int i = 0; i < CH; ++i) plain |= acc[i] != acc[i];
-        if (m < a.M && plain) {
-            lx_plain(a.A + (size_t)m * a.lda, reinterpret_cast<const float*>(a.W), a.ldw, a.K, a.out + (size_t)m * a.ld_out, a.bias, n0 + half * CH, min(n0 + (half + 1) * CH, a.N), a.act, a.alpha,
-                     a.accumulate);
-        } else if (m < a.M) {
-            const int c0 = n0 + half * CH;
-            float* o = a.out + (size_t)m * a.ld_out + c0;
-            const bool vec = a.ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
-#pragma unroll
-            for (int c = 0; c < CH; c += 4) {
-                float y[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    y[i] = acc[c + i] + (a.bias != nullptr && c0 + c + i < a.N ? a.bias[c0 + c + i] : 0.f);
-                    if (a.act != 0) y[i] = lx_act(y[i], a.act);
-                    y[i] *= a.alpha;
-                }
-                if (vec && c0 + c + 4 <= a.N) {
-                    if (a.accumulate) {
-                        const float4 p = *reinterpret_cast<const float4*>(o + c);
-                        y[0] += p.x; y[1] += p.y; y[2] += p.z; y[3] += p.w;
-                    }
-                    *reinterpret_cast<float4*>(o + c) = make_float4(y[0], y[1], y[2], y[3]);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (c0 + c + i < a.N) o[c + i] = a.accumulate ? o[c + i] + y[i] : y[i];
-                }
-            }
-        }
+        for (int i = 0; i < CH; i += 4) *reinterpret_cast<float4*>(row + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
     }
     tc_fence_before();
-    __syncthreads();
-    if (warp == 1) { tc_fence_after(); tmem_dealloc(tm, 2 * BN); }
+    if (S > 1) cluster_sync();
+    else __syncthreads();
+    if (warp == 1) { tc_fence_after(); tmem_dealloc(tm, Cfg::ACCS * BN); }
+    // The sums of the cluster, in the order of K, leave in whole rows: rows rank, rank + S, ... are this CTA's
+    const bool vec = a.ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
+    const float* sums = reinterpret_cast<const float*>(smem);
+    for (int e = threadIdx.x; e < (LX_M - rank + S - 1) / S * (BN / 4); e += LX_THREADS) {
+        const int r = rank + e / (BN / 4) * S, c = e % (BN / 4) * 4, m = m0 + r, n = n0 + c;
+        if (m >= a.M || n >= a.N) continue;
+        float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (S == 1) {
+            f = *reinterpret_cast<const float4*>(sums + r * Cfg::PITCH + c);
+        } else {
+            for (int s = 0; s < S; ++s) {
+                const float4 g = lx_ld_remote4(sums + r * Cfg::PITCH + c, s);
+                f.x += g.x; f.y += g.y; f.z += g.z; f.w += g.w;
+            }
+        }
+        float* o = a.out + (size_t)m * a.ld_out + n;
+        float y[4] = {f.x, f.y, f.z, f.w};
+        if (f.x != f.x || f.y != f.y || f.z != f.z || f.w != f.w) {
+            lx_plain(a.A + (size_t)m * a.lda, reinterpret_cast<const float*>(a.W), a.ldw, a.K, a.out + (size_t)m * a.ld_out, a.bias, n, min(n + 4, a.N), a.act, a.alpha, a.accumulate);
+            continue;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            y[i] += a.bias != nullptr && n + i < a.N ? a.bias[n + i] : 0.f;
+            if (a.act != 0) y[i] = lx_act(y[i], a.act);
+            y[i] *= a.alpha;
+        }
+        if (vec && n + 4 <= a.N) {
+            if (a.accumulate) {
+                const float4 p = *reinterpret_cast<const float4*>(o);
+                y[0] += p.x; y[1] += p.y; y[2] += p.z; y[3] += p.w;
+            }
+            *reinterpret_cast<float4*>(o) = make_float4(y[0], y[1], y[2], y[3]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (n + i < a.N) o[i] = a.accumulate ? o[i] + y[i] : y[i];
+        }
+    }
+    if (S > 1) cluster_sync();   // no tile goes away while another CTA reads it
 }
 
 int split_rows(const float* in, int64_t ld, int rows, int K, int pitch, __nv_bfloat16* out, cudaStream_t st) {
@@ -197,25 +229,96 @@ int split_rows(const float* in, int64_t ld, int rows, int K, int pitch, __nv_bfl
     return 0;
 }
 
-template <int BN>
-int launch_split_linear(const LinearArgs& a, const __nv_bfloat16* pa, const __nv_bfloat16* pw, int pitch, cudaStream_t st) {
+template <int BN, int WP>
+int launch_split_linear(const LinearArgs& a, const __nv_bfloat16* pa, const __nv_bfloat16* w, int pitch, int pitch_w, int S, cudaStream_t st) {
     CUtensorMap ta, tw;
     B2_TRY(make_tmap_parts(&ta, pa, pitch, a.M, 3, LX_M));
-    B2_TRY(make_tmap_parts(&tw, pw, pitch, a.N, 3, BN));
-    B2_CUDA_CHECK(cudaFuncSetAttribute(linear_split_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, LxCfg<BN>::SMEM));
-    launch_pdl(linear_split_kernel<BN>, dim3(((a.M + LX_M - 1) / LX_M) * ((a.N + BN - 1) / BN)), dim3(LX_THREADS), LxCfg<BN>::SMEM, st, ta, tw, a);
+    B2_TRY(make_tmap_parts(&tw, w, pitch_w, a.N, WP, BN));
+    B2_CUDA_CHECK(cudaFuncSetAttribute(linear_split_kernel<BN, WP>, cudaFuncAttributeMaxDynamicSharedMemorySize, LxCfg<BN, WP>::SMEM));
+    const int blocks = (a.K + LX_K - 1) / LX_K, per = (blocks + S - 1) / S;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(((a.M + LX_M - 1) / LX_M) * ((a.N + BN - 1) / BN) * S); cfg.blockDim = dim3(LX_THREADS); cfg.dynamicSmemBytes = LxCfg<BN, WP>::SMEM; cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = S; attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = S > 1 ? 2 : 1;
+    B2_CUDA_CHECK(cudaLaunchKernelEx(&cfg, linear_split_kernel<BN, WP>, ta, tw, a, S, per));
     B2_LAUNCH_CHECK();
     return 0;
 }
+// Clusters of S CTAs, one CTA an SM, that the device holds at once: what its GPCs' sizes leave
+int clusters_held(int S) {
+    static std::atomic<int> held[16][LX_MAX_CLUSTER + 1];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= 16) return std::max(1, num_sms() / (2 * S));
+    n = held[dev][S].load(std::memory_order_relaxed);
+    if (n > 0) return n;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(S); cfg.blockDim = dim3(LX_THREADS); cfg.dynamicSmemBytes = LxCfg<128, 1>::SMEM;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = S; attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(linear_split_kernel<128, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, LxCfg<128, 1>::SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, linear_split_kernel<128, 1>, &cfg) != cudaSuccess || n < 1) {
+        cudaGetLastError();
+        n = std::max(1, num_sms() / (2 * S));
+    }
+    held[dev][S].store(n, std::memory_order_relaxed);
+    return n;
+}
+
+// Tiles of 64, 128 or (W in one part) 256 columns, K in one piece or shared out over a cluster of up to 8 CTAs: whichever is done first. Clocks of a CTA: a
+// block of K is bound by its bytes, some 40 a clock (56 KB at 64 columns with W in one part: 1216 measured, 64 KB at 128: 1500, 80 KB at 256: 2025) or by
+// its products (48, 64, 128 clk each); what a tile costs beside them grows with its columns, a cluster adds its barriers and the reads of its tiles. Wide
+// tiles read A less often, a cut K fills the SMs. us with the parts of A made, rows x outputs x K, W in one part, 64 columns uncut / the rule's / the best
+// of all 24 forms: 600 x 1024 x 1024 15.2 / 14.1 / 14.1; x 4096 41.0 / 23.8 / 23.8; 600 x 4096 x 1024 38.0 / 27.1 / 27.1; 600 x 6176 x 1024 50.2 / 27.9 /
+// 27.9; 600 x 64 x 1024 14.5 / 8.3 / 8.3; 64 x 1024 x 1024 13.5 / 7.9 / 7.9; 300 x 1536 x 1536 18.8 / 14.9 / 14.7; 1200 x 2048 x 2048 64.4 / 41.3 / 41.3;
+// 40 x 4096 x 1024 13.2 / 9.8 / 9.0. W in three parts: 600 x 1024 x 4096 66.5 / 39.9 / 39.9.
+template <int WP>
+int launch_tiles(const LinearArgs& a, const __nv_bfloat16* pa, const __nv_bfloat16* w, int pitch, int pitch_w, cudaStream_t st) {
+    const int num_m = (a.M + LX_M - 1) / LX_M, blocks = (a.K + LX_K - 1) / LX_K;
+    int best_bn = 64, best_s = 1;
+    int64_t best = INT64_MAX;
+    for (int bn = 64; bn <= (WP == 1 ? 256 : 128); bn *= 2) {
+        const int tiles = num_m * ((a.N + bn - 1) / bn);
+        const int block = std::max((WP == 1 ? 12 : 24) * std::max(48, bn / 2), (3 * LX_M + WP * bn) * 128 / 40);
+        for (int S = 1; S <= LX_MAX_CLUSTER && S <= blocks; ++S) {
+            const int per = (blocks + S - 1) / S, held = S == 1 ? num_sms() : clusters_held(S);
+            if ((S - 1) * per >= blocks) continue;   // (a CTA without blocks)
+            const int64_t clk = (int64_t)((tiles + held - 1) / held) * ((int64_t)per * block + 2500 + 36 * bn + (S > 1 ? 1500 + 30 * std::min(bn, 128) + 300 * S : 0));
+            if (clk < best) { best = clk; best_bn = bn; best_s = S; }
+        }
+    }
+    if (WP == 1 && best_bn == 256) return launch_split_linear<WP == 1 ? 256 : 128, WP>(a, pa, w, pitch, pitch_w, best_s, st);
+    return best_bn == 128 ? launch_split_linear<128, WP>(a, pa, w, pitch, pitch_w, best_s, st) : launch_split_linear<64, WP>(a, pa, w, pitch, pitch_w, best_s, st);
+}
 
 int pitch_of(int K) { return (K + 7) / 8 * 8; }
+
+__global__ void __launch_bounds__(256) bf16_values_kernel(const uint4* __restrict__ w, int64_t n4, int* __restrict__ other) {
+    int bad = 0;
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (int64_t)gridDim.x * 256) {
+        const uint4 v = w[i];
+        bad |= ((v.x | v.y | v.z | v.w) & 0xffffu) != 0;
+    }
+    if (__syncthreads_or(bad) && threadIdx.x == 0) *other = 1;
+}
+__global__ void __launch_bounds__(256) high_halves_kernel(const uint4* __restrict__ w, int64_t n4, uint2* __restrict__ out) {
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (int64_t)gridDim.x * 256) {
+        const uint4 v = w[i];
+        out[i] = make_uint2(v.x >> 16 | (v.y & 0xffff0000u), v.z >> 16 | (v.w & 0xffff0000u));
+    }
+}
 }  // namespace
 
 size_t linear_split_bytes(int rows, int K) { return (size_t)6 * rows * pitch_of(K); }
 
 bool linear_splits(const LinearArgs& a) {
     return a.w_dtype == DT_F32 && !a.round_a && a.norm.alpha == nullptr && a.parts != nullptr && a.M >= LINEAR_SPLIT_MIN_ROWS &&
-           linear_split_bytes(a.M, a.K) + linear_split_bytes(std::min(a.N, 128), a.K) <= a.parts_bytes;
+           linear_split_bytes(a.M, a.K) + (a.W16 != nullptr ? 0 : linear_split_bytes(std::min(a.N, 128), a.K)) <= a.parts_bytes;
 }
 
 int linear_split_f32(const LinearArgs& a, cudaStream_t st) {
@@ -223,6 +326,7 @@ int linear_split_f32(const LinearArgs& a, cudaStream_t st) {
     __nv_bfloat16* pa = reinterpret_cast<__nv_bfloat16*>(a.parts);
     __nv_bfloat16* pw = pa + (size_t)3 * a.M * pitch;
     B2_TRY(split_rows(a.A, a.lda, a.M, a.K, pitch, pa, st));
+    if (a.W16 != nullptr) return launch_tiles<1>(a, pa, reinterpret_cast<const __nv_bfloat16*>(a.W16), pitch, a.K, st);
     // as many rows of W at a time as the scratch holds, in whole tiles
     const int64_t fit = (int64_t)((a.parts_bytes - linear_split_bytes(a.M, a.K)) / linear_split_bytes(1, a.K));
     const int step = fit >= a.N ? a.N : (int)(fit / 128 * 128);
@@ -233,11 +337,21 @@ int linear_split_f32(const LinearArgs& a, cudaStream_t st) {
         if (a.bias != nullptr) b.bias = a.bias + n0;
         b.W = reinterpret_cast<const float*>(a.W) + (size_t)n0 * a.ldw;
         B2_TRY(split_rows(reinterpret_cast<const float*>(b.W), a.ldw, b.N, a.K, pitch, pw, st));
-        const int num_m = (b.M + LX_M - 1) / LX_M;
-        // tiles of 128 columns read A half as often; narrower ones where they would leave SMs idle
-        const bool wide = num_m * ((b.N + 127) / 128) > num_sms() / 2;
-        B2_TRY(wide ? launch_split_linear<128>(b, pa, pw, pitch, st) : launch_split_linear<64>(b, pa, pw, pitch, st));
+        B2_TRY(launch_tiles<3>(b, pa, pw, pitch, pitch, st));
     }
+    return 0;
+}
+
+int bf16_values(const float* w, int64_t n, int* other, cudaStream_t st) {
+    B2_CHECK_ARG(n % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0, "bf16_values: whole fours on 16 bytes");
+    bf16_values_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((n / 4 + 255) / 256, 8 * num_sms())), 256, 0, st>>>(reinterpret_cast<const uint4*>(w), n / 4, other);
+    B2_LAUNCH_CHECK();
+    return 0;
+}
+int high_halves(const float* w, int64_t n, void* out, cudaStream_t st) {
+    B2_CHECK_ARG(n % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0, "high_halves: whole fours on 16 bytes");
+    high_halves_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((n / 4 + 255) / 256, 8 * num_sms())), 256, 0, st>>>(reinterpret_cast<const uint4*>(w), n / 4, reinterpret_cast<uint2*>(out));
+    B2_LAUNCH_CHECK();
     return 0;
 }
 

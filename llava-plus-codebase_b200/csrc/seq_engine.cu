@@ -78,6 +78,11 @@ struct SeqModel {
     // workspaces (fp32 unless noted)
     DevBuf x, proj, act, y, gated, mixout, mixes, rp, wl1, wlog, ff, xn, tok, want;
     DevBuf lin_parts;                  // fp32 compute: bf16 parts of a product's operands (linear_split.cu)
+    // fp32 compute: the matrices whose values all are bf16 ones (a bf16 checkpoint), as bf16 beside the fp32 ones: their products take half as many
+    // steps and no parts are made of them. Read by prompt portions only, and not from when a weight is set until the model is finalized again: the
+    // graph of a decode step goes on reading the fp32 matrices, which are set in place.
+    std::map<const void*, DevBuf> w16;
+    bool w16_valid = false, portion = false;
     DevBuf scan_chunks;                // chunk states of a long prompt's recurrences (recurrent.cu)
     DevBuf attn_parts;                 // bf16 parts of the keys and values that a prompt portion sees (attention_split.cu); grows with the longest cache
     DevBuf a16;                        // bf16 copy of a GEMM's A operand (tensor-core path of the bf16 compute mode)
@@ -215,6 +220,10 @@ struct Lin {  // one Linear call on the model's compute dtype
         if (norm != nullptr) a.norm = *norm;
         a.A16 = a16;
         a.parts = s.lin_parts.p; a.parts_bytes = s.lin_parts.bytes;
+        if (s.portion && s.w16_valid && K % 8 == 0) {
+            const auto it = s.w16.find(W.p);
+            if (it != s.w16.end()) a.W16 = it->second.as<__nv_bfloat16>() + w_row0 * (size_t)K;
+        }
         return a;
     }
     int operator()(const float* A, int64_t lda, const DevBuf& W, int N, int K, float* out, int64_t ldo, int M, int act = LIN_NONE,
@@ -1163,6 +1172,7 @@ static int seq_head(b2_model* m, const int32_t* index, int n, float* logits, int
 // one decode step over the slots [slot0, slot0 + B): kv->tok -> logits (m->logits) -> token selection, lengths += 1
 int seq_decode_launch(b2_model* m, b2_kv* kv, int B, int slot0, cudaStream_t st) {
     SeqModel& s = *m->seq;
+    s.portion = false;
     RowMap rm{s.segs.as<SeqSeg>(), s.row_slot.as<int32_t>(), s.row_pos.as<int32_t>()};
     B2_TRY(rowmap_decode(rm, kv->len_dev.as<int32_t>(), kv->sstate.as<SampleState>(), kv->rows_dev.as<RowState>(), slot0, B, st));
     B2_TRY(seq_embed(m, kv, kv->tok.as<int32_t>() + slot0, B, B, st));
@@ -1179,6 +1189,7 @@ int seq_decode_launch(b2_model* m, b2_kv* kv, int B, int slot0, cudaStream_t st)
 // ------------------------------------------------------------------------------------------------------------------
 int seq_set_weight(b2_model* m, const char* key, const void* ptr, const int64_t* shape, int ndim, int dt) {
     SeqModel& s = *m->seq;
+    s.w16_valid = false;
     const int width = s.d.width, V = s.d.vocab, WD = s.w_dtype;
     const std::string k(key);
     if (k == "embed") { B2_TRY(want_shape(key, shape, ndim, V, width)); s.got[k] = 1; return put_tensor(s.embed, WD, (size_t)((V + 7) / 8 * 8) * width, 0, ptr, dt, (int64_t)V * width); }
@@ -1562,6 +1573,42 @@ static std::vector<std::string> required_of(const SeqLayerInfo& L, const b2_seq_
     return v;
 }
 
+// The fp32 matrices that prompt portions multiply with, where all their values are bf16 ones, once more as bf16
+static int copy_bf16_weights(SeqModel& s) {
+    if (!s.w16.empty()) cudaDeviceSynchronize();   // calls in flight may use the old ones
+    for (auto& e : s.w16) e.second.free();
+    s.w16.clear();
+    std::vector<const DevBuf*> mats;
+    for (const SeqWeights& W : s.w)
+        for (const DevBuf* b : {&W.in_w, &W.o_w, &W.lproj_w, &W.lo_w, &W.r_w, &W.k_w, &W.v_w, &W.g_w, &W.w1, &W.w2, &W.ro_w, &W.up_w, &W.down_w, &W.qdg_w, &W.uk_w, &W.uv_w,
+                                &W.qfv_w, &W.router_w, &W.sgu_w, &W.sd_w, &W.uq_w, &W.ukx_w, &W.gla_w, &W.a2_w, &W.mem_w})
+            if (b->p != nullptr && b->bytes % 16 == 0) mats.push_back(b);
+    for (const DevBuf* b : {s.d.tied_head ? &s.embed : &s.head, &s.loop_in})
+        if (b->p != nullptr && b->bytes % 16 == 0) mats.push_back(b);
+    if (mats.empty()) return 0;
+    std::vector<int> other(mats.size(), 0);
+    DevBuf flags;
+    B2_TRY(flags.alloc(other.size() * 4));
+    cudaError_t e = cudaMemset(flags.p, 0, other.size() * 4);
+    int r = 0;
+    for (size_t i = 0; i < mats.size() && r == 0; ++i) r = bf16_values(mats[i]->as<float>(), (int64_t)(mats[i]->bytes / F4), flags.as<int>() + i, 0);
+    if (e == cudaSuccess) e = cudaMemcpy(other.data(), flags.p, other.size() * 4, cudaMemcpyDeviceToHost);
+    flags.free();
+    B2_TRY(r);
+    B2_CUDA_CHECK(e);
+    for (size_t i = 0; i < mats.size(); ++i) {
+        if (other[i] != 0) continue;
+        DevBuf c;
+        alloc_spare(c, mats[i]->bytes / 2);
+        if (c.p == nullptr) continue;
+        s.w16[mats[i]->p] = c;
+        B2_TRY(high_halves(mats[i]->as<float>(), (int64_t)(mats[i]->bytes / F4), c.p, 0));
+    }
+    B2_CUDA_CHECK(cudaStreamSynchronize(0));
+    s.w16_valid = true;
+    return 0;
+}
+
 int seq_finalize(b2_model* m) {
     SeqModel& s = *m->seq;
     std::string missing;
@@ -1708,7 +1755,10 @@ int seq_finalize(b2_model* m) {
         else if (d.type == B2_MIXER_GLA) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.gl_heads, d.gl_dim, d.gl_vdim));
     }
     alloc_spare(s.scan_chunks, chunk_floats * F4);
-    if (s.d.compute != B2_COMPUTE_BF16) alloc_spare(s.lin_parts, linear_split_bytes((int)R, s.a16_w) + ((size_t)64 << 20));   // (with room for the weights in blocks of rows)
+    if (s.d.compute != B2_COMPUTE_BF16) {
+        alloc_spare(s.lin_parts, linear_split_bytes((int)R, s.a16_w) + ((size_t)64 << 20));   // (with room for the weights in blocks of rows)
+        B2_TRY(copy_bf16_weights(s));
+    }
     return 0;
 }
 
@@ -1729,6 +1779,7 @@ void seq_model_free(b2_model* m) {
                     &s.rlogit, &s.moe_idx, &s.moe_w, &s.moe_pos, &s.moe_src, &s.moe_tile, &s.moe_h, &s.moe_a, &s.moe_y, &s.moe_a16, &s.zero_idx, &s.hin, &s.final_a, &s.loop_in, &s.cat,
                     &s.h2, &s.h1_16, &s.h2_16, &s.f16, &s.den, &s.embed_nw, &s.scan_chunks, &s.lin_parts, &s.attn_parts};
     for (DevBuf* b : bs) b->free();
+    for (auto& e : s.w16) e.second.free();
     delete m->seq;
     m->seq = nullptr;
 }
@@ -2128,6 +2179,7 @@ int b2_append_tokens(b2_model* m, b2_kv* kv, int slot, const int32_t* tokens_hos
     for (int i = 0; i < n_want; ++i) B2_CHECK_ARG(want_host[i] >= 0 && want_host[i] < n, "b2_append_tokens: wanted index %d outside the %d tokens", want_host[i], n);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     B2_TRY(ws_enter(m, st));
+    s.portion = true;
     B2_CUDA_CHECK(cudaMemcpyAsync(s.tok.p, tokens_host, (size_t)n * 4, cudaMemcpyHostToDevice, st));
     RowMap rm{s.segs.as<SeqSeg>(), s.row_slot.as<int32_t>(), s.row_pos.as<int32_t>()};
     // a slot that starts over begins from position 0 whatever its device-side length says
