@@ -565,7 +565,7 @@ struct ScanArgs {
     int rows = 0;                                                         // tokens of the one segment (nseg == 1); with the scratch (floats, see below) a long
     float* chunk_scratch = nullptr; size_t chunk_floats = 0;              // prompt is walked in chunks side by side
 };
-size_t linear_scan_scratch_floats(int heads, int dk, int dv);
+size_t linear_scan_scratch_floats(int mode, int heads, int dk, int dv, int rows);
 int linear_scan_f32(const ScanArgs& a, cudaStream_t stream);
 
 // ---- matrix memories with one decay per head (matrix_memory.cu) ------------------------------------------------------------------

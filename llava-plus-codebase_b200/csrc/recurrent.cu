@@ -5,14 +5,10 @@
 // state whatever its slot held before, so a slot that is handed to a new request needs no clearing.
 #include <algorithm>
 
-#include "common.cuh"
-#include "kernels.h"
+#include "scan.cuh"
 
 namespace b2 {
 namespace {
-
-__device__ __forceinline__ float silu_f(float v) { return v / (1.f + expf(-v)); }
-__device__ __forceinline__ float softplus_f(float v) { return v > 20.f ? v : log1pf(expf(v)); }
 
 // ---- causal depthwise convolution + SiLU -----------------------------------------------------------------------------------
 // One thread per (channel, tile of CONV_TILE tokens): it primes its window from the inputs in front of the tile (rows of this
@@ -145,6 +141,7 @@ __global__ void __launch_bounds__(128) token_shift_carry_kernel(const float* __r
 // divided by): a first launch walks every chunk from an empty state (the first one from the slot's state, with its outputs) and leaves the
 // chunk's final state and the product of its decays per key; a second launch starts each further chunk from what those fold to, S_c = P_c S_(c-1)
 // + L_c, and writes its outputs. The chain is then 2 / C of the tokens for 5/3 of the arithmetic.
+// Long prompts with a decay per key run in blocks on the tensor cores instead (scan_blocks.cu).
 // 1900 tokens, 8 heads of 128 x 256 (gated linear attention): 625 -> 191 us (two walks of 90 us, 11 us for the gates beforehand; before, 8 keys x
 // one column per thread and one chain). Issue slots bound a walk (74 % of them taken in the first, 58 % in the one that
 // writes; with the gates' arithmetic in it 291 us for both, hence scan_prepare_kernel), then the multiply-add pipe. 600 tokens, 32 heads of 128 x 64 (state space): 152 -> 84 us, 16 heads of 64 x 64 (RWKV) 128 -> 58.
@@ -165,24 +162,7 @@ __device__ __forceinline__ void scan_cp4(void* dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 
-// The gates' arithmetic, on a query and a raw decay entry of key `key` of head h (SSD, one decay per token, has its own): the forget gate bounded
-// below f = l + (1 - l) sigmoid(z + b) (HGRN2: what is forgotten, 1 - f, is what is written), sigmoid(z + b)^(1 / tau) = exp(log_sigmoid(z + b) /
-// tau) with log_sigmoid(u) = min(u, 0) - log1p(exp(-|u|)) (GLA), exp(-exp(z)) (RWKV).
-template <int MODE>
-__device__ __forceinline__ float scan_decay(const ScanArgs& a, int at, float z) {   // at = h * dk + key
-    if (MODE == SCAN_HGRN2) {
-        const float low = a.gate_lower[at];
-        return fmaf(1.f - low, 1.f / (1.f + expf(-(z + a.gate_bias[at]))), low);
-    }
-    if (MODE == SCAN_GLA) {
-        const float u = z + a.gate_bias[at];
-        return expf((fminf(u, 0.f) - log1pf(expf(-fabsf(u)))) / a.tau);
-    }
-    return expf(-expf(z));
-}
-template <int MODE>
-__device__ __forceinline__ float scan_query(const ScanArgs& a, float q) { return MODE == SCAN_HGRN2 ? silu_f(q) : MODE == SCAN_GLA ? q * a.q_scale : q; }
-// ... in place over a long prompt's rows (workspaces of the call), where every column block of both launches would redo it
+// The gates' arithmetic in place over a long prompt's rows (workspaces of the call), where every column block of both launches would redo it
 template <int MODE>
 __global__ void __launch_bounds__(256) scan_prepare_kernel(ScanArgs a) {
     pdl_enter();
@@ -197,9 +177,10 @@ __global__ void __launch_bounds__(256) scan_prepare_kernel(ScanArgs a) {
     }
 }
 
-// KW: warps over the keys (64 each); V16: every operand row is 16-byte aligned with sizes in whole fours
-template <int MODE, int KW, bool V16>
-__global__ void __launch_bounds__(KW * 128, KW == 4 ? 1 : 2) linear_scan_kernel(ScanArgs a, ScanPlan p) {
+// KW: warps over the keys (64 each); V16: every operand row is 16-byte aligned with sizes in whole fours. AFTER: behind scan_blocks_f32, whose tokens
+// are walked only for heads that the products could not do; the other heads' state is put in its place.
+template <int MODE, int KW, bool V16, bool AFTER>
+__device__ __forceinline__ void linear_scan_body(const ScanArgs& a, const ScanPlan& p, const BlockScan& bs) {
     pdl_enter();
     constexpr int DKP = KW * 64, NTHR = KW * 128;
     constexpr bool PER_KEY = MODE != SCAN_SSD, HAS_K = MODE != SCAN_HGRN2;
@@ -211,7 +192,8 @@ __global__ void __launch_bounds__(KW * 128, KW == 4 ? 1 : 2) linear_scan_kernel(
     float* sY = sV + 2 * SC_TT * SC_COLS;            // [KW][TT][COLS]
     const int chunk = p.chunks > 1 ? p.z0 + (int)blockIdx.z : 0;
     const SeqSeg sg = a.segs[p.chunks > 1 ? 0 : blockIdx.z];
-    const int t_lo = chunk * p.len, t_hi = p.chunks > 1 && chunk + 1 < p.chunks ? min(sg.n, t_lo + p.len) : sg.n;
+    const int t_end = AFTER ? bs.t0 + bs.n : sg.n;
+    const int t_lo = AFTER ? bs.t0 : chunk * p.len, t_hi = p.chunks > 1 && chunk + 1 < p.chunks ? min(sg.n, t_lo + p.len) : t_end;
     if (t_lo >= t_hi) return;
     const bool outputs = p.chunks == 1 || p.second != 0 || chunk == 0;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, kw = warp % KW, cw = warp / KW, kg = lane & 7, cg = lane >> 3;
@@ -226,6 +208,22 @@ __global__ void __launch_bounds__(KW * 128, KW == 4 ? 1 : 2) linear_scan_kernel(
     const float* vg = a.v + (size_t)sg.row0 * a.ldv + (size_t)h * dv + col0;
     const int ncol = min(SC_COLS, dv - col0);
     const size_t head_state = ((size_t)h * dk) * dv, all_state = (size_t)a.heads * dk * dv;
+    if (AFTER) {
+        int bad = 0;
+        for (int b = tid; b < bs.blocks; b += NTHR) {
+            const size_t bh = (size_t)b * a.heads + h;
+            bad |= bs.bad_in[bh];
+            for (int c = 0; c < bs.col_tiles; ++c) bad |= bs.bad_v[bh * bs.col_tiles + c] | bs.bad_out[bh * bs.col_tiles + c];
+        }
+        for (int i = tid; i < bs.fold_ctas; i += NTHR) bad |= bs.bad_state[h * bs.fold_ctas + i];
+        if (!__syncthreads_or(bad)) {   // (whole fours: scan_blocks_fit)
+            for (int e = tid; e < dk * (ncol >> 2); e += NTHR) {
+                const size_t at = head_state + (size_t)(e / (ncol >> 2)) * dv + col0 + e % (ncol >> 2) * 4;
+                *reinterpret_cast<float4*>(a.state + (size_t)sg.slot * all_state + at) = *reinterpret_cast<const float4*>(bs.last + at);
+            }
+            return;
+        }
+    }
 
     float S[8][4], pd[8];
     auto load_state = [&](const float* st, bool fold, const float* dec) {   // S = st, or S = dec S + st
@@ -302,7 +300,7 @@ __global__ void __launch_bounds__(KW * 128, KW == 4 ? 1 : 2) linear_scan_kernel(
     if (p.second != 0) {
         load_state(p.final_state + head_state, false, nullptr);
         for (int c = 1; c < chunk; ++c) load_state(p.final_state + (size_t)c * all_state + head_state, true, p.decays + ((size_t)c * a.heads + h) * dk);
-    } else if (chunk == 0 && sg.pos0 > 0) {
+    } else if (chunk == 0 && (sg.pos0 > 0 || (AFTER && t_lo > 0))) {
         load_state(a.state + (size_t)sg.slot * all_state + head_state, false, nullptr);
     }
     float bon[8];
@@ -438,6 +436,14 @@ __global__ void __launch_bounds__(KW * 128, KW == 4 ? 1 : 2) linear_scan_kernel(
         }
     }
 }
+template <int MODE, int KW, bool V16>
+__global__ void __launch_bounds__(KW * 128, KW == 4 ? 1 : 2) linear_scan_kernel(ScanArgs a, ScanPlan p) {
+    linear_scan_body<MODE, KW, V16, false>(a, p, BlockScan());
+}
+template <int MODE, int KW>
+__global__ void __launch_bounds__(KW * 128, 2) linear_scan_after_kernel(ScanArgs a, BlockScan blocks) {
+    linear_scan_body<MODE, KW, true, true>(a, ScanPlan(), blocks);
+}
 }  // namespace
 
 int causal_conv_silu_f32(const float* in, int64_t ld_in, const float* w, const float* bias, float* tail, float* out, int64_t ld_out, int C,
@@ -488,6 +494,19 @@ int launch_scan(const ScanArgs& a, cudaStream_t st) {
     B2_CUDA_CHECK(cudaFuncSetAttribute(linear_scan_kernel<MODE, KW, V16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int cols = (a.dv + SC_COLS - 1) / SC_COLS, ctas = cols * a.heads;
     ScanPlan p;
+    if constexpr (MODE != SCAN_SSD && V16 && KW <= 2) {
+        if (scan_blocks_fit(a)) {
+            B2_CUDA_CHECK(cudaFuncSetAttribute(linear_scan_after_kernel<MODE, KW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            BlockScan blocks;
+            for (int t0 = 0; t0 < a.rows; t0 += blocks.n) {
+                B2_TRY(scan_blocks_plan(a, t0, &blocks));
+                B2_TRY(scan_blocks_f32(a, blocks, st));
+                launch_pdl(linear_scan_after_kernel<MODE, KW>, dim3(cols, a.heads), dim3(KW * 128), smem, st, a, blocks);
+                B2_LAUNCH_CHECK();
+            }
+            return 0;
+        }
+    }
     // Chunks: enough CTAs for two per SM, of 64 tokens and more; two chunks would walk the whole chain all the same
     // (the last chunk has no part in the first launch, the first one none in the second)
     int chunks = a.nseg == 1 && a.chunk_scratch != nullptr ? 1 + 2 * num_sms() / ctas : 1;
@@ -527,7 +546,14 @@ int scan_of_size(const ScanArgs& a, cudaStream_t st) {
     return v16 ? launch_scan<MODE, 4, true>(a, st) : launch_scan<MODE, 4, false>(a, st);
 }
 
-size_t linear_scan_scratch_floats(int heads, int dk, int dv) { return (size_t)(SC_MAX_CHUNKS - 1) * heads * dk * (dv + 1); }
+// chunk states, or the blocks of a prompt of `rows` tokens, as many as fit into 96 MB but 8 at least (a longer prompt goes in pieces)
+size_t linear_scan_scratch_floats(int mode, int heads, int dk, int dv, int rows) {
+    const size_t chunks = (size_t)(SC_MAX_CHUNKS - 1) * heads * dk * (dv + 1);
+    if (mode == SCAN_SSD || dk > 128) return chunks;
+    int blocks = (rows + SB_TOK - 1) / SB_TOK;
+    while (blocks > SB_MIN_PIECE && scan_blocks_bytes(heads, dk, dv, blocks) > (size_t)96 << 20) --blocks;
+    return std::max(chunks, (scan_blocks_bytes(heads, dk, dv, blocks) + 3) / 4);
+}
 
 int linear_scan_f32(const ScanArgs& a, cudaStream_t st) {
     B2_CHECK_ARG(a.q && (a.k || a.mode == SCAN_HGRN2) && a.v && a.decay_in && a.state && a.y && a.segs && a.nseg > 0, "linear_scan: null argument");

@@ -1749,10 +1749,10 @@ int seq_finalize(b2_model* m) {
     size_t chunk_floats = 0;
     for (const SeqLayerInfo& L : s.layers) {
         const b2_seq_layer_desc& d = L.d;
-        if (d.type == B2_MIXER_MAMBA2) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.m_heads, d.m_state, d.m_vdim));
-        else if (d.type == B2_MIXER_PARALLEL) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.r_heads, d.r_dim, d.r_dim));
-        else if (d.type == B2_MIXER_HGRN2) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.g_heads, d.g_dim, d.g_vdim));
-        else if (d.type == B2_MIXER_GLA) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(d.gl_heads, d.gl_dim, d.gl_vdim));
+        if (d.type == B2_MIXER_MAMBA2) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(SCAN_SSD, d.m_heads, d.m_state, d.m_vdim, s.rows));
+        else if (d.type == B2_MIXER_PARALLEL) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(SCAN_RWKV, d.r_heads, d.r_dim, d.r_dim, s.rows));
+        else if (d.type == B2_MIXER_HGRN2) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(SCAN_HGRN2, d.g_heads, d.g_dim, d.g_vdim, s.rows));
+        else if (d.type == B2_MIXER_GLA) chunk_floats = std::max(chunk_floats, linear_scan_scratch_floats(SCAN_GLA, d.gl_heads, d.gl_dim, d.gl_vdim, s.rows));
     }
     alloc_spare(s.scan_chunks, chunk_floats * F4);
     if (s.d.compute != B2_COMPUTE_BF16) {

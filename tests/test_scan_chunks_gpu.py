@@ -64,3 +64,63 @@ def test_chunks_against_the_oracle(name):
     ref = mod.O.forward(cfg, w, toks) if mod is P else mod.O.forward(cfg, w, toks, return_layers=True)
     ref = torch.as_tensor(np.asarray(ref[1][0])).double()
     assert rel(got, ref) <= 2 ** -21 * n ** 0.5
+
+
+# Blocks of 64 tokens on the tensor cores (csrc/scan_blocks.cu): key sizes of one and two blocks of 64 and parts of one, value sizes around tiles of 128
+# columns, prompts that end inside a block, and one whose blocks exceed the scratch and goes in pieces
+def rwkv(heads, dim):
+    lay = {**RWKV, "mixer": {**RWKV["mixer"], "right": {"heads": heads, "dim": dim, "decay_rank": 5}}}
+    return K, K.config([lay], width=64)
+
+
+def hgrn2(heads, dim, vdim):
+    return P, P.config([P.layer({"type": "hgrn2", "mixer": {"heads": heads, "dim": dim, "vdim": vdim}}, None)], width=64)
+
+
+def gla(heads, dim, vdim):
+    return S, S.config([S.layer(S.gla(heads, dim, vdim), None)], width=64)
+
+
+BLOCKS = {"rwkv_64": rwkv(2, 64), "rwkv_72": rwkv(3, 72), "rwkv_128": rwkv(1, 128), "hgrn2": hgrn2(2, 128, 64), "hgrn2_part": hgrn2(3, 44, 132), "gla_small": gla(3, 16, 24),
+          "gla": gla(2, 128, 256), "gla_part": gla(3, 68, 4)}
+
+
+@pytest.mark.parametrize("name", list(BLOCKS))
+def test_blocks_equal_small_portions(name):
+    mod, cfg = BLOCKS[name]
+    model, _ = mod.build(cfg, torch.float32, max_batch=2, max_seq=700, max_rows=700)
+    eng = model._ensure_engine()
+    kv = eng.new_kv(2, 700)
+    for n in (319, 320, 448, 449, 511, 577, 640):
+        toks = mod.tokens_for(cfg, n, seed=n)
+        one = stream(eng, kv, toks, [100] * (n // 100) + ([n % 100] if n % 100 else []))
+        bound = 2 ** -21 * n ** 0.5
+        assert rel(stream(eng, kv, toks, [n]), one) <= bound, n
+        assert rel(stream(eng, kv, toks, [50, n - 50]), one) <= bound, n
+
+
+def test_blocks_in_pieces():
+    mod, cfg = gla(64, 128, 256)   # 16 MB a block of tokens
+    n = 650
+    model, _ = mod.build(cfg, torch.float32, max_batch=2, max_seq=n, max_rows=n)
+    eng = model._ensure_engine()
+    kv = eng.new_kv(2, n)
+    toks = mod.tokens_for(cfg, n)
+    assert rel(stream(eng, kv, toks, [n]), stream(eng, kv, toks, [50] * 13)) <= 2 ** -21 * n ** 0.5
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.0e38])
+@pytest.mark.parametrize("name", ["rwkv_64", "hgrn2", "gla"])
+def test_a_row_that_is_no_number_reaches_no_earlier_one(name, value):
+    mod, cfg = BLOCKS[name]
+    n, at, tok = 512, 300, 3
+    w = mod.O.random_weights(cfg, seed=1)
+    w["embed"][tok] = value   # (an array, or a tensor)
+    model, _ = mod.build(cfg, torch.float32, weights=w, max_batch=2, max_seq=n, max_rows=n)
+    eng = model._ensure_engine()
+    kv = eng.new_kv(2, n)
+    toks = [t if t != tok else 4 for t in mod.tokens_for(cfg, n)]
+    toks[at] = tok
+    got, ref = stream(eng, kv, toks, [n]), stream(eng, kv, toks, [100] * 5 + [12])
+    assert torch.equal(got.isnan(), ref.isnan()) and not got[:at].isnan().any()
+    assert rel(got[:at], ref[:at]) <= 2 ** -21 * n ** 0.5
