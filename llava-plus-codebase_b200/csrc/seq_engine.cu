@@ -189,9 +189,10 @@ bool tc_enabled() {  // B2_SEQ_TC=0: every Linear, of one row too, on the FMA ke
 int tc_min_rows() {
     const char* e = getenv("B2_SEQ_TC_MIN_ROWS");
     const int v = e != nullptr ? atoi(e) : 0;
-    // (drawn when 4 and more rows ran on the tile GEMM, decode steps at widths 2048 / 4096 in ms: 4 rows 0.76 / 1.38 vs 0.78 / 1.48 on the FMA kernel, 2
-    // rows 0.71 / 1.28 vs 0.62 / 1.10; the streamed products take fp32 and bf16 rows alike)
-    return v >= 1 ? v : 4;
+    // (the streamed products read bf16 rows twice as fast, and a norm on its way in keeps them on the FMA kernels. us a step of four layers, 2 and 3 rows, from
+    // 4 rows on / from 2: mixed layers of width 2048 199 / 182 and 197 / 181; dynamic-tanh norms of 2048 299 / 208 and 328 / 211; parallel experts of 2048 219 /
+    // 209 and 243 / 239; other designs within 1 %)
+    return v >= 1 ? v : 2;
 }
 
 struct Lin {  // one Linear call on the model's compute dtype
@@ -441,7 +442,9 @@ static LinearArgs glu_rows_args(const Lin& lin, const SeqLayerInfo& L, SeqWeight
 
 // A handful of rows through a parallel block: mixer and feed-forward read the same rows and add onto the same ones, so the feed-forward's two
 // products ride in the launches of the mixer's first and last (linear_stream.cu): two launches a layer fewer, each 1.5 to 3 us of start, ragged last
-// tiles and end. 48 steps of four mixed layers, width 2048 (us, before -> now): one slot 9773 -> 9436, 8 slots 12293 -> 12106.
+// tiles and end. 48 steps of four mixed layers, width 2048 (us, before -> now): one slot 9773 -> 9436, 8 slots 12293 -> 12106. Wider layers spend their time
+// on the weights, and a sum's units then fit the SMs no better (a step of four layers, apart / together: width 2560, 4 slots 237 / 239; 3072, 12 slots
+// 377 / 390): one row rides always, more up to 8192 inputs of the sum.
 struct RowFeedForward { LinearArgs up, down; };
 static LinearArgs gqa_first(const Lin& lin, const SeqLayerInfo& L, SeqWeights& W, const SubIn& in, int R) {
     const SeqModel& s = *lin.m->seq;
@@ -463,6 +466,7 @@ static bool row_feed_forward(const Lin& lin, const SeqLayerInfo& L, SeqWeights& 
     const bool gqa = d.type == B2_MIXER_GQA_ATTN;
     const int inner = gqa ? L.ng : L.pv;
     const LinearArgs first = gqa ? gqa_first(lin, L, W, in, R) : gla_first(lin, L, W, in.h, R);
+    if (R > 1 && inner + ff > 8192) return false;
     return first.A16 == f.up.A16 && linear_streams(first) && linear_streams(f.up) && linear_streams(f.down) &&
            linear_streams(lin.args(s.gated.as<float>(), inner, W.o_w, width, inner, target, width, R, LIN_NONE, alpha, 1));
 }
