@@ -442,6 +442,9 @@ __global__ void __launch_bounds__(512) attn_merge_kernel(BiasAttnArgs a) {
 // What bounds it is latency: the chain launch - position - key rows - exponentials - two meetings. The tiled kernel with its key splits staged 32 keys
 // at a time (load, barrier, products, barrier) and met in a second launch. A step of one layer of width 1024 (us, before -> now; keys, slots):
 // 8 key/value heads 41.1 -> 33.0 (500, 1), 86 -> 45 (8000, 1), 68 -> 37 (500, 8), 276 -> 77 (4000, 8); 2 of them 41.1 -> 35.2 (500, 1).
+// APPEND: the launch that normed, turned and appended the rows (3.5 us, with its start and the next one's) is part of this one; the caches are read up to the newest
+// key, which one warp adds from shared memory. 48 steps of four mixed layers of width 2048, with the row map in the embedding's launch and the RMS
+// norms of one row in the first products': one slot 9322 -> 8400 us, 8 slots 12070 -> 11929.
 constexpr int ST_WARPS = 16, ST_KEYS = 8, ST_DK = 128, ST_DV = 128;
 
 __device__ __forceinline__ float st_ld_remote(const float* p, int rank) {
@@ -452,25 +455,60 @@ __device__ __forceinline__ float st_ld_remote(const float* p, int rank) {
     return v;
 }
 
+// One warp: a head's norm and the turn of its pairs, from global into shared memory (rotate_rows_warp_kernel's arithmetic, rotary.cu)
+__device__ __forceinline__ void st_turn(const StepAppend& r, const float* norm_w, const float* src, float* dst, int size, int pos, int lane) {
+    float mul = 1.f;
+    if (norm_w != nullptr) {
+        float q = 0.f;
+        for (int d = lane; d < size; d += 32) q = fmaf(src[d], src[d], q);
+        mul = 1.f / sqrtf(warp_sum(q) / (float)size + r.eps);
+    }
+    const int units = size - r.pairs;
+    for (int u = lane; u < units; u += 32) {
+        if (u < r.pairs) {
+            const int d = r.half ? u : 2 * u, d2 = r.half ? d + r.pairs : d + 1;
+            const float2 cs = r.table[(size_t)pos * r.pairs + u];
+            float x = src[d] * mul, y = src[d2] * mul;
+            if (norm_w != nullptr) { x *= norm_w[d]; y *= norm_w[d2]; }
+            dst[d] = x * cs.x - y * cs.y;
+            dst[d2] = y * cs.x + x * cs.y;
+        } else {
+            const int d = u + r.pairs;
+            float o = src[d] * mul;
+            if (norm_w != nullptr) o *= norm_w[d];
+            dst[d] = o;
+        }
+    }
+}
+
 // grid (C, G * chunks, rows), clusters along x; NH >= query heads of a chunk
-template <int NH>
+template <int NH, bool APPEND>
 __global__ void __launch_bounds__(ST_WARPS * 32, 1) attn_step_kernel(BiasAttnArgs a, int C) {
     pdl_enter_late();
     __shared__ __align__(16) float sq[NH * ST_DK];
     __shared__ __align__(16) float so[ST_WARPS][NH][ST_DV];
     __shared__ float sm[ST_WARPS][NH], sl[ST_WARPS][NH];
     __shared__ float po[NH][ST_DV], pm[NH], pl[NH];     // this CTA's share, read by the cluster
+    __shared__ __align__(16) float sk[APPEND ? ST_DK : 4];   // the newest key
     const int rank = blockIdx.x, r = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int HGall = a.H / a.G, chunks = (HGall + NH - 1) / NH;
     const int g = blockIdx.y / chunks, h0 = g * HGall + (blockIdx.y % chunks) * NH, HG = min(NH, g * HGall + HGall - h0);
     const int dk = a.dk, dv = a.dv;
     const int pos = a.row_pos[r], slot = a.row_slot[r];
     if (pos < 0) return;                                // (the whole cluster)
-    for (int e = threadIdx.x; e < NH * dk / 4; e += ST_WARPS * 32)
-        reinterpret_cast<float4*>(sq)[e] = e < HG * dk / 4 ? reinterpret_cast<const float4*>(a.q + (size_t)r * a.ldq + (size_t)h0 * dk)[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (APPEND) {   // a warp norms and turns a query head, one more the newest key: the last warps, which have the fewest keys
+        const int t = warp - (ST_WARPS - 1 - NH);
+        if (t == NH) st_turn(a.append, a.append.k_norm, a.append.k + (size_t)r * a.ldq + (size_t)g * dk, sk, dk, pos, lane);
+        else if (t >= 0 && t < HG) st_turn(a.append, a.append.q_norm, a.q + (size_t)r * a.ldq + (size_t)(h0 + t) * dk, sq + t * dk, dk, pos, lane);
+        else if (t >= HG) for (int d = lane; d < dk; d += 32) sq[t * dk + d] = 0.f;
+    } else {
+        for (int e = threadIdx.x; e < NH * dk / 4; e += ST_WARPS * 32)
+            reinterpret_cast<float4*>(sq)[e] = e < HG * dk / 4 ? reinterpret_cast<const float4*>(a.q + (size_t)r * a.ldq + (size_t)h0 * dk)[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     // visible keys: [0, nA), the kept first positions in front of the window, then [first, pos]; numbered through, this CTA's are [k0, k1)
     const int first = mask_first(pos, a.mask_kind, a.mask_size), nA = a.mask_kind == MASK_WINDOW ? min(a.mask_keep, first) : 0;
-    const int n = nA + pos + 1 - first, per = (n + C - 1) / C, k0 = min(n, rank * per), k1 = min(n, k0 + per);
+    // (APPEND: those in the caches; the newest one, the row's own, follows)
+    const int n = nA + pos + (APPEND ? 0 : 1) - first, per = (n + C - 1) / C, k0 = min(n, rank * per), k1 = min(n, k0 + per);
     const int Gv = a.Gv > 0 ? a.Gv : a.G;
     const float* K = a.kcache + ((size_t)slot * a.G + g) * a.Smax * dk;
     const float* V = a.vcache + ((size_t)slot * Gv + g % Gv) * a.Smax * dv;
@@ -479,7 +517,7 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 1) attn_step_kernel(BiasAttnArg
     float4 o[NH];
 #pragma unroll
     for (int h = 0; h < NH; ++h) { m[h] = -INFINITY; l[h] = 0.f; o[h] = make_float4(0.f, 0.f, 0.f, 0.f); }
-    __syncthreads();
+    bool met = false;   // the queries are there: met with this warp's first rows on their way
 #pragma unroll 1
     for (int b = k0 + warp * ST_KEYS; b < k1; b += ST_WARPS * ST_KEYS) {
         float4 kf[2][ST_DK / 32], vf[ST_KEYS];
@@ -497,6 +535,7 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 1) attn_step_kernel(BiasAttnArg
             const int i = min(b + e, k1 - 1), v = i < nA ? i : first + i - nA;
             vf[e] = lane * 4 < dv && b + e < k1 ? *reinterpret_cast<const float4*>(V + (size_t)v * dv + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
+        if (!met) { __syncthreads(); met = true; }
 #pragma unroll
         for (int h = 0; h < NH; ++h) {
             float s[2], p[2];
@@ -535,6 +574,32 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 1) attn_step_kernel(BiasAttnArg
                 const float pe = __shfl_sync(0xffffffffu, p[e >> 2], (e & 3) * 8);
                 o[h].x = fmaf(pe, vf[e].x, o[h].x); o[h].y = fmaf(pe, vf[e].y, o[h].y); o[h].z = fmaf(pe, vf[e].z, o[h].z); o[h].w = fmaf(pe, vf[e].w, o[h].w);
             }
+        }
+    }
+    if (!met) __syncthreads();
+    if (APPEND && rank == C - 1) {   // the CTA with the fewest keys: the newest one, by the warp that has had the fewest turns; both rows into the caches
+        const float* vn = a.append.v + (size_t)r * a.ldq + (size_t)(g % Gv) * dv;
+        if (warp == ST_WARPS - 1) {
+            const float4 kf = lane * 4 < dk ? *reinterpret_cast<const float4*>(sk + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 vf = lane * 4 < dv ? make_float4(vn[lane * 4], vn[lane * 4 + 1], vn[lane * 4 + 2], vn[lane * 4 + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int h = 0; h < NH; ++h) {
+                const float4 q = lane * 4 < dk ? *reinterpret_cast<const float4*>(sq + h * dk + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+                float s = q.x * kf.x;
+                s = fmaf(q.y, kf.y, s); s = fmaf(q.z, kf.z, s); s = fmaf(q.w, kf.w, s);
+                s = warp_sum(s) * a.scale;
+                if (a.softcap > 0.f) s = a.softcap * tanhf(s / a.softcap);
+                if (a.rel != nullptr && h < HG) s += a.rel[(size_t)a.bucket_of[0] * a.H + h0 + h];
+                const float mx = fmaxf(m[h], s), ref = mx == -INFINITY ? 0.f : mx, corr = expf(m[h] - ref), p = expf(s - ref);
+                m[h] = mx;
+                l[h] = fmaf(l[h], corr, p);
+                o[h].x = fmaf(p, vf.x, o[h].x * corr); o[h].y = fmaf(p, vf.y, o[h].y * corr); o[h].z = fmaf(p, vf.z, o[h].z * corr); o[h].w = fmaf(p, vf.w, o[h].w * corr);
+            }
+        } else if (warp == 0 && blockIdx.y % chunks == 0) {
+            float* kc = a.kcache + (((size_t)slot * a.G + g) * a.Smax + pos) * dk;
+            for (int d = lane; d < dk; d += 32) kc[d] = sk[d];
+            float* vc = a.vcache + (((size_t)slot * Gv + g % Gv) * a.Smax + pos) * dv;
+            if (g < Gv) for (int d = lane; d < dv; d += 32) vc[d] = vn[d];   // (the maps of a head share its values)
         }
     }
 #pragma unroll
@@ -652,15 +717,18 @@ int launch_step(const BiasAttnArgs& a, cudaStream_t st) {
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
     cfg.attrs = attr; cfg.numAttrs = 2;
-    B2_CUDA_CHECK(cudaLaunchKernelEx(&cfg, attn_step_kernel<NH>, a, C));
+    B2_CUDA_CHECK(a.append.k != nullptr ? cudaLaunchKernelEx(&cfg, attn_step_kernel<NH, true>, a, C) : cudaLaunchKernelEx(&cfg, attn_step_kernel<NH, false>, a, C));
     B2_LAUNCH_CHECK();
     return 0;
 }
+
+bool attn_bias_appends(const BiasAttnArgs& a) { return a.tile_rows == 1 && !attn_split_fits(a) && attn_step_fits(a); }
 
 int attn_bias_f32(const BiasAttnArgs& a, cudaStream_t st) {
     B2_TRY(check_args(a, "attn_bias"));
     B2_CHECK_ARG((a.out || a.out16) && (a.rel == nullptr || a.bucket_of != nullptr), "attn_bias: null argument");
     B2_CHECK_ARG(a.nsplit >= 1 && a.nsplit <= 64 && (a.nsplit == 1 || a.partial != nullptr), "attn_bias: 1..64 key splits, with scratch");
+    B2_CHECK_ARG(a.append.k == nullptr || attn_bias_appends(a), "attn_bias: rows that are not in the caches");
     if (attn_split_fits(a)) return attn_split_f32(a, st);
     if (attn_step_fits(a)) {
         const int heads = a.H / a.G;

@@ -293,8 +293,8 @@ struct RowMap {
 int rowmap_portion(const RowMap& rm, int32_t* len, int slot, int n, int restart, cudaStream_t stream);
 // B segments of one row each for slots slot0 .. slot0+B-1 at positions len[slot]; with sstate->per_row set, slots whose
 // rows_state entry is not active become idle rows
-int rowmap_decode(const RowMap& rm, const int32_t* len, const SampleState* sstate, const RowState* rows_state, int slot0, int B,
-                  cudaStream_t stream);
+struct DecodeRows { RowMap rm; const int32_t* len = nullptr; const SampleState* sstate = nullptr; const RowState* rows_state = nullptr; int slot0 = 0; };
+int rowmap_decode(const DecodeRows& d, int B, cudaStream_t stream);
 
 // ---- generic Linear on fp32 activations (linear_generic.cu): any M, N, K -----------------------------------------------
 enum { LIN_NONE = 0, LIN_SILU = 1, LIN_SIGMOID = 2, LIN_TANH = 3, LIN_RELU_SQ = 4, LIN_GELU = 5 };   // LIN_GELU: the exact (erf) form
@@ -317,6 +317,7 @@ struct LinearArgs {
     int gated = 0; GluAct glu;                   // linear_stream_f32 only: W = [gate | up] of N rows each, out = glu_act(gate, up); no act, bias, alpha
     void* out16 = nullptr;                       // with gated: bf16 rows of pitch ld_out in place of out
     const void* A16 = nullptr;                   // the same rows already rounded to bf16, pitch K (linear_stream_f32 reads these when there are 2 or more)
+    const float* rms_w = nullptr; float rms_eps = 0.f;   // one streamed row of up to LINEAR_RMS_MAX_K (linear_stream_norms): A passes this weighted RMS norm on its way in
 };
 // True fp32, a portion of a prompt (linear_split.cu): whether a call runs on the tensor cores as products of bf16 parts. Scratch: the parts of A
 // and, without W16, of at least 128 rows of W, linear_split_bytes each. Up to 8 rows the weight-streaming kernel is the faster one; the tiled FMA kernel never was (a
@@ -332,6 +333,8 @@ int high_halves(const float* w, int64_t n, void* out, cudaStream_t stream);
 constexpr int LINEAR_STREAM_MAX = 16;
 bool linear_streams(const LinearArgs& a);
 int linear_stream_f32(const LinearArgs& a, cudaStream_t stream);
+constexpr int LINEAR_RMS_MAX_K = 4096;
+bool linear_stream_norms(const LinearArgs& a);
 // Two such products in one launch: a beside a gated unit b of the same rows; a + b on the outputs of a (its epilogue: b's output is not looked at)
 int linear_stream_side_f32(const LinearArgs& a, const LinearArgs& b, cudaStream_t stream);
 int linear_stream_sum_f32(const LinearArgs& a, const LinearArgs& b, cudaStream_t stream);
@@ -453,7 +456,7 @@ int latent_append_f32(const float* in, int64_t ld_in, const float* gamma, float*
 // x[r, :] = table[tokens[r], :] as fp32; ids outside [0, vocab) give a zero row and raise *err_flag (B2_ERR_TOKEN_RANGE)
 int embed_rows_f32(const int32_t* tokens, const void* table, int table_dtype, float* x, int rows, int cols, int vocab, int* err_flag,
                    cudaStream_t stream, float scale = 1.f,    // scale: x = table[token] * scale, in fp32
-                   const float* norm_w = nullptr, float eps = 0.f);   // norm_w (not with scale): the row is divided by sqrt(mean(x^2) + eps) and weighted
+                   const float* norm_w = nullptr, float eps = 0.f, const DecodeRows* rows_map = nullptr);   // rows_map (not with norm_w): rowmap_decode in the same launch; norm_w (not with scale): the row is divided by sqrt(mean(x^2) + eps) and weighted
 // Differential attention, per (row, head): d = a1 - lambda a2 over the head's dv values, out = d / sqrt(mean(d^2) + eps) * out_scale.
 // y holds map 1 of every head, then map 2 of every head: [rows, 2 * heads * dv]
 int diff_combine_f32(const float* y, int64_t ldy, float* out, int64_t ldo, int rows, int heads, int dv, float lambda, float out_scale, float eps,
@@ -596,6 +599,13 @@ int matrix_memory_f32(const MemoryArgs& a, cudaStream_t stream);
 
 // ---- attention with unit-RMS q/k, query temperature, tanh soft-cap and a bucketed distance bias (attention_bias.cu) -----
 enum { MASK_CAUSAL = 0, MASK_WINDOW = 1, MASK_CHUNK = 2 };
+// One row per slot whose queries and newest key are still as the projection left them: the attention norms and turns them itself (as RotateArgs do it), attends
+// to that key and its value and appends both to the caches (attn_bias_appends says where)
+struct StepAppend {
+    const float *k = nullptr, *v = nullptr;       // [rows, G*dk], [rows, Gv*dv], both of pitch ldq; null: they are in the caches
+    const float *q_norm = nullptr, *k_norm = nullptr; float eps = 0.f;   // weights of the heads' norm over dk, or null
+    const float2* table = nullptr; int pairs = 0, half = 0;
+};
 struct BiasAttnArgs {
     float* q = nullptr; int64_t ldq = 0;          // [rows, H*dk]: normalised and scaled in place by attn_prepare
     const float* k = nullptr; int64_t ldk = 0;    // [rows, G*dk] projections of this call's rows
@@ -628,6 +638,7 @@ struct BiasAttnArgs {
     // slot's length behind it, and scratch for the bf16 parts of the keys and values that it sees (null: it stays on the fp32 pipe)
     int slot = 0, key_end = 0;
     void* parts = nullptr; size_t parts_bytes = 0;
+    StepAppend append;
 };
 int attn_prepare_f32(const BiasAttnArgs& a, cudaStream_t stream);  // q/k norms, temperature, cache append
 // Fewer keys take as long on the fp32 pipe, which starts faster (a layer's prompt of n tokens, fp32 pipe -> tensor cores, width 1024: n = 24
@@ -636,6 +647,7 @@ constexpr int ATTN_SPLIT_MIN_ROWS = 16, ATTN_SPLIT_MIN_KEYS = 40;
 bool attn_split_fits(const BiasAttnArgs& a);                       // the call runs on the tensor cores
 size_t attn_split_bytes_per_key(int G, int Gv, int dk, int dv);    // scratch per visible key position
 int attn_split_f32(const BiasAttnArgs& a, cudaStream_t stream);
-int attn_bias_f32(const BiasAttnArgs& a, cudaStream_t stream);     // causal softmax attention of every row against its slot's cache
+int attn_bias_f32(const BiasAttnArgs& a, cudaStream_t stream);
+bool attn_bias_appends(const BiasAttnArgs& a);   // whether a.append is served for a call of these sizes     // causal softmax attention of every row against its slot's cache
 
 }  // namespace b2

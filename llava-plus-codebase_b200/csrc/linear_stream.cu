@@ -33,7 +33,9 @@ enum { LS_ONE = 0, LS_GLU = 1, LS_SIDE = 2, LS_SUM = 3 };
 
 // NT: column tiles of 8 rows of A (0: one row on the FMA pipe). A16: A lies there as bf16 rows of pitch K (LS_SUM: looked up for each product).
 // An SM holds 16 warps: one CTA of 16, or two of 8.
-template <int NT, bool A16, int FORM, int LS_WARPS>
+// RMS (one row): A passes a weighted RMS norm into shared memory on its way in, in every CTA: 8 KB read 148 times, beside weights that are on their way, for
+// a launch of 2 us. (More rows would be 64 KB and more a CTA.)
+template <int NT, bool A16, int FORM, bool RMS, int LS_WARPS>
 __device__ __forceinline__ void linear_stream_body(const LinearArgs& a, const LinearArgs& b) {
     constexpr int COLS = NT == 0 ? 1 : 8 * NT;
     __shared__ float red[LS_WARPS][LS_N][COLS + (NT == 0 ? 0 : 1)];
@@ -69,6 +71,34 @@ __device__ __forceinline__ void linear_stream_body(const LinearArgs& a, const Li
     pdl_trigger();
     pdl_wait();   // A, and the output when it is added to, come from the kernels in front
 
+    __shared__ __align__(16) float normed[RMS ? LINEAR_RMS_MAX_K : 4];
+    if constexpr (RMS) {
+        constexpr int U = LINEAR_RMS_MAX_K / 4 / (LS_WARPS * 32);
+        float4 x[U], g[U];
+        float q = 0.f;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = (threadIdx.x + u * LS_WARPS * 32) * 4;
+            x[u] = c < a.K ? *reinterpret_cast<const float4*>(a.A + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            g[u] = c < a.K ? *reinterpret_cast<const float4*>(a.rms_w + c) : x[u];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) { q = fmaf(x[u].x, x[u].x, q); q = fmaf(x[u].y, x[u].y, q); q = fmaf(x[u].z, x[u].z, q); q = fmaf(x[u].w, x[u].w, q); }
+        q = warp_sum(q);
+        if (lane == 0) red[warp][0][0] = q;
+        __syncthreads();
+        q = warp_sum(lane < LS_WARPS ? red[lane][0][0] : 0.f);
+        const float mul = 1.f / sqrtf(q / (float)a.K + a.rms_eps);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = (threadIdx.x + u * LS_WARPS * 32) * 4;
+            float4 v = make_float4(x[u].x * mul * g[u].x, x[u].y * mul * g[u].y, x[u].z * mul * g[u].z, x[u].w * mul * g[u].w);
+            if (a.round_a) v = make_float4(round_bf16(v.x), round_bf16(v.y), round_bf16(v.z), round_bf16(v.w));
+            if (c < a.K) *reinterpret_cast<float4*>(normed + c) = v;
+        }
+        __syncthreads();
+    }
+
     float acc[NT == 0 ? 1 : NT][4];
 #pragma unroll
     for (int t = 0; t < (NT == 0 ? 1 : NT); ++t)
@@ -80,7 +110,7 @@ __device__ __forceinline__ void linear_stream_body(const LinearArgs& a, const Li
         if (second) unit -= units0;
         const LinearArgs& p = second ? b : a;
         const int k0 = unit * LS_UNIT + kq, K = p.K;
-        const float* A = p.A;
+        const float* A = RMS ? normed : p.A;
         if (NT == 0) {
             float x[4][8];
 #pragma unroll
@@ -92,7 +122,7 @@ __device__ __forceinline__ void linear_stream_body(const LinearArgs& a, const Li
             }
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                if (a.round_a) {
+                if (a.round_a && !RMS) {
 #pragma unroll
                     for (int i = 0; i < 8; ++i) x[c][i] = round_bf16(x[c][i]);
                 }
@@ -192,13 +222,13 @@ __device__ __forceinline__ void linear_stream_body(const LinearArgs& a, const Li
     }
 }
 
-template <int NT, bool A16, bool GLU, int LS_WARPS>
+template <int NT, bool A16, bool GLU, bool RMS, int LS_WARPS>
 __global__ void __launch_bounds__(LS_WARPS * 32, 16 / LS_WARPS) linear_stream_kernel(LinearArgs a) {
-    linear_stream_body<NT, A16, GLU ? LS_GLU : LS_ONE, LS_WARPS>(a, a);
+    linear_stream_body<NT, A16, GLU ? LS_GLU : LS_ONE, RMS, LS_WARPS>(a, a);
 }
-template <int NT, bool A16, int FORM, int LS_WARPS>
+template <int NT, bool A16, int FORM, bool RMS, int LS_WARPS>
 __global__ void __launch_bounds__(LS_WARPS * 32, 16 / LS_WARPS) linear_stream_two_kernel(LinearArgs a, LinearArgs b) {
-    linear_stream_body<NT, A16, FORM, LS_WARPS>(a, b);
+    linear_stream_body<NT, A16, FORM, RMS, LS_WARPS>(a, b);
 }
 
 // Whether a launch of `tiles` tiles of `units` units runs as one CTA of 16 warps an SM, not two of 8
@@ -219,20 +249,20 @@ bool wide_ctas(int tiles, int units, bool side = false) {
     return chain(num_sms(), 16) <= chain(2 * num_sms(), 8);
 }
 
-template <int NT, bool A16, bool GLU>
+template <int NT, bool A16, bool GLU, bool RMS = false>
 int launch_stream(const LinearArgs& a, cudaStream_t st) {
     const int outs = GLU ? LS_N / 2 : LS_N, tiles = (a.N + outs - 1) / outs;
-    if (wide_ctas<NT>(tiles, (a.K + LS_UNIT - 1) / LS_UNIT)) B2_CUDA_CHECK(launch_pdl(linear_stream_kernel<NT, A16, GLU, 16>, dim3(std::min(tiles, num_sms())), dim3(512), 0, st, a));
-    else B2_CUDA_CHECK(launch_pdl(linear_stream_kernel<NT, A16, GLU, 8>, dim3(std::min(tiles, 2 * num_sms())), dim3(256), 0, st, a));
+    if (wide_ctas<NT>(tiles, (a.K + LS_UNIT - 1) / LS_UNIT)) B2_CUDA_CHECK(launch_pdl(linear_stream_kernel<NT, A16, GLU, RMS, 16>, dim3(std::min(tiles, num_sms())), dim3(512), 0, st, a));
+    else B2_CUDA_CHECK(launch_pdl(linear_stream_kernel<NT, A16, GLU, RMS, 8>, dim3(std::min(tiles, 2 * num_sms())), dim3(256), 0, st, a));
     B2_LAUNCH_CHECK();
     return 0;
 }
-template <int NT, bool A16, int FORM>
+template <int NT, bool A16, int FORM, bool RMS = false>
 int launch_two(const LinearArgs& a, const LinearArgs& b, cudaStream_t st) {
     const int tiles = (a.N + LS_N - 1) / LS_N + (FORM == LS_SIDE ? (b.N + LS_N / 2 - 1) / (LS_N / 2) : 0);
     const int units = (a.K + LS_UNIT - 1) / LS_UNIT + (FORM == LS_SUM ? (b.K + LS_UNIT - 1) / LS_UNIT : 0);
-    if (wide_ctas<NT>(tiles, units, FORM == LS_SIDE)) B2_CUDA_CHECK(launch_pdl(linear_stream_two_kernel<NT, A16, FORM, 16>, dim3(std::min(tiles, num_sms())), dim3(512), 0, st, a, b));
-    else B2_CUDA_CHECK(launch_pdl(linear_stream_two_kernel<NT, A16, FORM, 8>, dim3(std::min(tiles, 2 * num_sms())), dim3(256), 0, st, a, b));
+    if (wide_ctas<NT>(tiles, units, FORM == LS_SIDE)) B2_CUDA_CHECK(launch_pdl(linear_stream_two_kernel<NT, A16, FORM, RMS, 16>, dim3(std::min(tiles, num_sms())), dim3(512), 0, st, a, b));
+    else B2_CUDA_CHECK(launch_pdl(linear_stream_two_kernel<NT, A16, FORM, RMS, 8>, dim3(std::min(tiles, 2 * num_sms())), dim3(256), 0, st, a, b));
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -241,6 +271,7 @@ int launch_two(const LinearArgs& a, const LinearArgs& b, cudaStream_t st) {
 bool linear_streams(const LinearArgs& a) {
     return a.w_dtype == DT_BF16 && a.M >= 1 && a.M <= LINEAR_STREAM_MAX && a.K % 8 == 0 && a.ldw % 8 == 0 && (reinterpret_cast<uintptr_t>(a.W) & 15) == 0 &&
            a.norm.alpha == nullptr && (a.M == 1 || a.round_a) &&
+           (a.rms_w == nullptr || (a.M == 1 && a.K <= LINEAR_RMS_MAX_K && (reinterpret_cast<uintptr_t>(a.rms_w) & 15) == 0)) &&
            (a.M > 1 && a.A16 != nullptr ? (reinterpret_cast<uintptr_t>(a.A16) & 15) == 0 : a.A != nullptr && (a.M == 1 || a.lda % 4 == 0) && (reinterpret_cast<uintptr_t>(a.A) & 15) == 0);
 }
 
@@ -251,20 +282,26 @@ static int stream_rows(const LinearArgs& a, cudaStream_t st) {
     return a.A16 != nullptr ? launch_stream<2, true, GLU>(a, st) : launch_stream<2, false, GLU>(a, st);
 }
 
+bool linear_stream_norms(const LinearArgs& a) { return a.rms_w != nullptr && !a.gated && linear_streams(a); }
+
 int linear_stream_side_f32(const LinearArgs& a, const LinearArgs& b, cudaStream_t st) {
-    B2_CHECK_ARG(linear_streams(a) && linear_streams(b) && !a.gated && b.gated && a.M == b.M && a.K == b.K && a.A == b.A && a.A16 == b.A16 && a.lda == b.lda && a.round_a == b.round_a,
+    B2_CHECK_ARG(linear_streams(a) && linear_streams(b) && !a.gated && b.gated && a.M == b.M && a.K == b.K && a.A == b.A && a.A16 == b.A16 && a.lda == b.lda && a.round_a == b.round_a && a.rms_w == b.rms_w,
                  "linear_stream_side: two products that do not share their rows");
-    if (a.M == 1) return launch_two<0, false, LS_SIDE>(a, b, st);
+    if (a.M == 1) return a.rms_w != nullptr ? launch_two<0, false, LS_SIDE, true>(a, b, st) : launch_two<0, false, LS_SIDE>(a, b, st);
     if (a.M <= 8) return a.A16 != nullptr ? launch_two<1, true, LS_SIDE>(a, b, st) : launch_two<1, false, LS_SIDE>(a, b, st);
     return a.A16 != nullptr ? launch_two<2, true, LS_SIDE>(a, b, st) : launch_two<2, false, LS_SIDE>(a, b, st);
 }
 
 int linear_stream_sum_f32(const LinearArgs& a, const LinearArgs& b, cudaStream_t st) {
-    B2_CHECK_ARG(linear_streams(a) && linear_streams(b) && !a.gated && !b.gated && a.M == b.M && a.N == b.N && a.round_a == b.round_a, "linear_stream_sum: two products of other sizes");
+    B2_CHECK_ARG(linear_streams(a) && linear_streams(b) && !a.gated && !b.gated && a.M == b.M && a.N == b.N && a.round_a == b.round_a && a.rms_w == nullptr && b.rms_w == nullptr, "linear_stream_sum: two products of other sizes");
     if (a.M == 1) return launch_two<0, false, LS_SUM>(a, b, st);
     return a.M <= 8 ? launch_two<1, false, LS_SUM>(a, b, st) : launch_two<2, false, LS_SUM>(a, b, st);
 }
 
-int linear_stream_f32(const LinearArgs& a, cudaStream_t st) { return a.gated ? stream_rows<true>(a, st) : stream_rows<false>(a, st); }
+int linear_stream_f32(const LinearArgs& a, cudaStream_t st) {
+    B2_CHECK_ARG(a.rms_w == nullptr || linear_stream_norms(a), "linear_stream: a norm that this product does not take");
+    if (a.rms_w != nullptr) return launch_stream<0, false, false, true>(a, st);
+    return a.gated ? stream_rows<true>(a, st) : stream_rows<false>(a, st);
+}
 
 }  // namespace b2

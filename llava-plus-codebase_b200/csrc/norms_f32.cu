@@ -239,12 +239,22 @@ __device__ __forceinline__ void ld8(const __nv_bfloat16* p, float (&v)[8]) {
     v[0] = bf16_lo(u.x); v[1] = bf16_hi(u.x); v[2] = bf16_lo(u.y); v[3] = bf16_hi(u.y);
     v[4] = bf16_lo(u.z); v[5] = bf16_hi(u.z); v[6] = bf16_lo(u.w); v[7] = bf16_hi(u.w);
 }
+__device__ __forceinline__ void decode_row(const DecodeRows& d, int b) {
+    const int slot = d.slot0 + b;
+    // per-slot mode (continuous batching): a slot that is not armed keeps its state, cache rows and length
+    const bool live = d.sstate == nullptr || d.rows_state == nullptr || d.sstate->per_row == 0 || d.rows_state[slot].active != 0;
+    const int pos = d.len[slot];
+    d.rm.segs[b].slot = slot; d.rm.segs[b].row0 = b; d.rm.segs[b].n = live ? 1 : 0; d.rm.segs[b].pos0 = pos;
+    d.rm.row_slot[b] = slot;
+    d.rm.row_pos[b] = live ? pos : -1;
+}
 // VEC: 8 entries of a row per thread (one entry per thread and step made 16 rounds of loads of a 2048-wide row: 7.4 -> 4.3 us of a step, 1900 rows 11.4 -> 6.4)
 template <typename TT, bool VEC>
 __global__ void embed_rows_kernel(const int32_t* __restrict__ tokens, const TT* __restrict__ table, float* __restrict__ x, int cols, int vocab,
-                                  int* err_flag, float scale) {
+                                  int* err_flag, float scale, DecodeRows map) {
     pdl_enter();
     const size_t r = blockIdx.x;
+    if (map.len != nullptr && threadIdx.x == blockDim.x - 1) decode_row(map, (int)r);   // a decode step: what the row is, for the kernels behind
     const int t = tokens[r];
     const bool ok = t >= 0 && t < vocab;
     if (!ok && threadIdx.x == 0 && err_flag != nullptr) err_flag[0] = 1;  // slot 0 = B2_ERR_TOKEN_RANGE
@@ -694,18 +704,10 @@ __global__ void rowmap_portion_kernel(SeqSeg* segs, int32_t* row_slot, int32_t* 
     }
 }
 
-__global__ void rowmap_decode_kernel(SeqSeg* segs, int32_t* row_slot, int32_t* row_pos, const int32_t* len, const SampleState* sstate,
-                                     const RowState* rows_state, int slot0, int B) {
+__global__ void rowmap_decode_kernel(DecodeRows d, int B) {
     pdl_enter();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    const int slot = slot0 + b;
-    // per-slot mode (continuous batching): a slot that is not armed keeps its state, cache rows and length
-    const bool live = sstate == nullptr || rows_state == nullptr || sstate->per_row == 0 || rows_state[slot].active != 0;
-    const int pos = len[slot];
-    segs[b].slot = slot; segs[b].row0 = b; segs[b].n = live ? 1 : 0; segs[b].pos0 = pos;
-    row_slot[b] = slot;
-    row_pos[b] = live ? pos : -1;
+    if (b < B) decode_row(d, b);
 }
 }  // namespace
 
@@ -748,15 +750,15 @@ int diff_combine_f32(const float* y, int64_t ldy, float* out, int64_t ldo, int r
 }
 
 int embed_rows_f32(const int32_t* tokens, const void* table, int table_dtype, float* x, int rows, int cols, int vocab, int* err_flag,
-                   cudaStream_t st, float scale, const float* norm_w, float eps) {
-    B2_CHECK_ARG(tokens && table && x && rows > 0 && (norm_w == nullptr || scale == 1.f), "embed_rows: bad argument");
+                   cudaStream_t st, float scale, const float* norm_w, float eps, const DecodeRows* rows_map) {
+    B2_CHECK_ARG(tokens && table && x && rows > 0 && (norm_w == nullptr || (scale == 1.f && rows_map == nullptr)), "embed_rows: bad argument");
     if (norm_w != nullptr) {
         if (table_dtype == DT_F32) return launch_embed_norm(tokens, reinterpret_cast<const float*>(table), x, rows, cols, vocab, err_flag, norm_w, eps, st);
         return launch_embed_norm(tokens, reinterpret_cast<const __nv_bfloat16*>(table), x, rows, cols, vocab, err_flag, norm_w, eps, st);
     }
     const bool vec = cols % 8 == 0 && ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
     const dim3 grid(rows), block(vec ? (cols >= 2048 ? 256 : 128) : 128);
-    auto run = [&](auto kernel, auto* tab) { launch_pdl(kernel, grid, block, 0, st, tokens, tab, x, cols, vocab, err_flag, scale); };
+    auto run = [&](auto kernel, auto* tab) { launch_pdl(kernel, grid, block, 0, st, tokens, tab, x, cols, vocab, err_flag, scale, rows_map != nullptr ? *rows_map : DecodeRows()); };
     if (table_dtype == DT_F32) {
         const float* tab = reinterpret_cast<const float*>(table);
         if (vec) run(embed_rows_kernel<float, true>, tab); else run(embed_rows_kernel<float, false>, tab);
@@ -909,9 +911,9 @@ int rowmap_portion(const RowMap& rm, int32_t* len, int slot, int n, int restart,
     return 0;
 }
 
-int rowmap_decode(const RowMap& rm, const int32_t* len, const SampleState* sstate, const RowState* rows_state, int slot0, int B, cudaStream_t st) {
-    B2_CHECK_ARG(rm.segs && rm.row_slot && rm.row_pos && len && B > 0, "rowmap_decode: bad argument");
-    launch_pdl(rowmap_decode_kernel, dim3((B + 127) / 128), dim3(128), 0, st, rm.segs, rm.row_slot, rm.row_pos, len, sstate, rows_state, slot0, B);
+int rowmap_decode(const DecodeRows& d, int B, cudaStream_t st) {
+    B2_CHECK_ARG(d.rm.segs && d.rm.row_slot && d.rm.row_pos && d.len && B > 0, "rowmap_decode: bad argument");
+    launch_pdl(rowmap_decode_kernel, dim3((B + 127) / 128), dim3(128), 0, st, d, B);
     B2_LAUNCH_CHECK();
     return 0;
 }

@@ -294,6 +294,7 @@ int attn_nsplit(int rows, int G, int max_seq) {
 // them; or (norm) the residual stream itself, normed on its way into the product.
 struct SubIn {
     const float* h = nullptr; const void* h16 = nullptr; const DytNorm* norm = nullptr;
+    const float* rms = nullptr;   // with h the residual stream: weight of the RMS norm that it passes on its way into the product (one row, linear_stream.cu)
     SubIn(const float* p) : h(p) {}
     SubIn() {}
 };
@@ -436,6 +437,7 @@ static LinearArgs glu_rows_args(const Lin& lin, const SeqLayerInfo& L, SeqWeight
     const SeqModel& s = *lin.m->seq;
     LinearArgs up = lin.args(in.h, s.d.width, W.up_w, L.d.ff, s.d.width, s.ffa.as<float>(), L.d.ff, R, LIN_NONE, 1.f, 0, nullptr, 0, in.h16);
     up.gated = 1; up.glu = glu_of(L.d);
+    up.rms_w = in.rms; up.rms_eps = s.d.norm_eps;
     if (R > 1 && lin.tensor_cores(s.d.width, L.d.ff, target, s.d.width, R)) up.out16 = s.ff.p;
     return up;
 }
@@ -448,11 +450,15 @@ static LinearArgs glu_rows_args(const Lin& lin, const SeqLayerInfo& L, SeqWeight
 struct RowFeedForward { LinearArgs up, down; };
 static LinearArgs gqa_first(const Lin& lin, const SeqLayerInfo& L, SeqWeights& W, const SubIn& in, int R) {
     const SeqModel& s = *lin.m->seq;
-    return lin.args(in.h, s.d.width, W.lproj_w, L.lproj, s.d.width, s.proj.as<float>(), L.lproj_ld, R, LIN_NONE, 1.f, 0, W.qkv_b.as<float>(), 0, in.h16, in.norm);
+    LinearArgs a = lin.args(in.h, s.d.width, W.lproj_w, L.lproj, s.d.width, s.proj.as<float>(), L.lproj_ld, R, LIN_NONE, 1.f, 0, W.qkv_b.as<float>(), 0, in.h16, in.norm);
+    a.rms_w = in.rms; a.rms_eps = s.d.norm_eps;
+    return a;
 }
-static LinearArgs gla_first(const Lin& lin, const SeqLayerInfo& L, SeqWeights& W, const float* h, int R) {
+static LinearArgs gla_first(const Lin& lin, const SeqLayerInfo& L, SeqWeights& W, const SubIn& in, int R) {
     const SeqModel& s = *lin.m->seq;
-    return lin.args(h, s.d.width, W.gla_w, L.pproj, s.d.width, s.proj.as<float>(), L.pproj_ld, R);
+    LinearArgs a = lin.args(in.h, s.d.width, W.gla_w, L.pproj, s.d.width, s.proj.as<float>(), L.pproj_ld, R);
+    a.rms_w = in.rms; a.rms_eps = s.d.norm_eps;
+    return a;
 }
 // its arguments, where every one of the four products streams its weights
 static bool row_feed_forward(const Lin& lin, const SeqLayerInfo& L, SeqWeights& W, const SubIn& in, float* target, float alpha, int R, RowFeedForward& f) {
@@ -465,7 +471,7 @@ static bool row_feed_forward(const Lin& lin, const SeqLayerInfo& L, SeqWeights& 
     f.down = lin.args(fa, ff, W.down_w, width, ff, target, width, R, LIN_NONE, alpha, 1, nullptr, 0, f.up.out16);
     const bool gqa = d.type == B2_MIXER_GQA_ATTN;
     const int inner = gqa ? L.ng : L.pv;
-    const LinearArgs first = gqa ? gqa_first(lin, L, W, in, R) : gla_first(lin, L, W, in.h, R);
+    const LinearArgs first = gqa ? gqa_first(lin, L, W, in, R) : gla_first(lin, L, W, in, R);
     if (R > 1 && inner + ff > 8192) return false;
     return first.A16 == f.up.A16 && linear_streams(first) && linear_streams(f.up) && linear_streams(f.down) &&
            linear_streams(lin.args(s.gated.as<float>(), inner, W.o_w, width, inner, target, width, R, LIN_NONE, alpha, 1));
@@ -509,7 +515,6 @@ static int gqa_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeights& 
     rq[0].norm_all = rq[1].norm_all = d.ga_qk_norm == B2_QK_NORM_ALL;
     rq[2].in = qkv + L.nq + (d.ga_key_values ? 0 : L.nk); rq[2].hs_in = dv; rq[2].cache = S.vc.as<float>(); rq[2].heads = G; rq[2].size = dv;
     rq[2].table = S.vrot_tab.as<float2>(); rq[2].pairs = d.ga_rot_values ? dv / 2 : 0;
-    B2_TRY(rotate_rows_multi_f32(rq, 3, st));
     BiasAttnArgs aa;
     aa.q = qkv; aa.ldq = ldc;
     aa.kcache = S.kc.as<float>(); aa.vcache = S.vc.as<float>();
@@ -534,6 +539,14 @@ static int gqa_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeights& 
     const bool out16 = maps == 1 && !d.ga_rot_values && lin.tensor_cores(width, L.ng, target, width, R);
     if (out16) aa.out16 = s.a16.p;
     portion_of(s, nseg, slot, ctx_end, aa);
+    // a decode step's attention turns its rows itself where it runs as one launch
+    if (!rq[0].norm_all && rq[2].pairs == 0 && attn_bias_appends(aa)) {
+        aa.append.k = rq[1].in; aa.append.v = rq[2].in;
+        aa.append.q_norm = rq[0].norm_w; aa.append.k_norm = rq[1].norm_w; aa.append.eps = rq[0].eps;
+        aa.append.table = rq[0].table; aa.append.pairs = rq[0].pairs; aa.append.half = rq[0].half;
+    } else {
+        B2_TRY(rotate_rows_multi_f32(rq, 3, st));
+    }
     B2_TRY(attn_bias_f32(aa, st));
     if (out16 && ff != nullptr) return linear_stream_sum_f32(ff->down, lin.args(nullptr, 0, W.o_w, width, L.ng, target, width, R, LIN_NONE, alpha, accumulate, nullptr, 0, s.a16.p), st);
     if (out16) return lin(nullptr, 0, W.o_w, width, L.ng, target, width, R, LIN_NONE, alpha, accumulate, nullptr, 0, nullptr, s.a16.p);
@@ -563,15 +576,15 @@ static int gqa_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeights& 
 
 // Gated linear attention: one fused projection [q | k | v | g | a1], the decay logits through the second low-rank matrix, the
 // recurrence (decay, scaled query and state in fp32), per-head RMS norm with the gate, out-projection.
-static int gla_mixer(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, SeqLayerState& S, const float* h, float* target, float alpha, int accumulate,
+static int gla_mixer(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, SeqLayerState& S, const SubIn& in, float* target, float alpha, int accumulate,
                      int R, int nseg, cudaStream_t st, const RowFeedForward* ff = nullptr) {
     SeqModel& s = *m->seq;
     const b2_seq_layer_desc& d = L.d;
     const Lin lin{m, st};
     const int width = s.d.width, H = d.gl_heads, dk = d.gl_dim, dv = d.gl_vdim;
     float* proj = s.proj.as<float>();
-    if (ff != nullptr) B2_TRY(linear_stream_side_f32(gla_first(lin, L, W, h, R), ff->up, st));
-    else B2_TRY(lin(h, width, W.gla_w, L.pproj, width, proj, L.pproj_ld, R));
+    if (ff != nullptr) B2_TRY(linear_stream_side_f32(gla_first(lin, L, W, in, R), ff->up, st));
+    else B2_TRY(lin(in.h, width, W.gla_w, L.pproj, width, proj, L.pproj_ld, R));
     float* z = s.wlog.as<float>();   // [R, heads * dim] decay logits without their bias (the recurrence adds it in fp32)
     B2_TRY(lin(proj + 2 * L.pq + 2 * L.pv, L.pproj_ld, W.a2_w, L.pq, d.gl_rank, z, L.pq, R));
     ScanArgs sa;
@@ -988,9 +1001,18 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
                 const bool two = s.d.block == B2_BLOCK_PARALLEL2 && d.ff > 0, early = d.ff > 0 && d.ff_kind == B2_FF_GELU;
                 DytNorm n1, n2;
                 SubIn in1, in2;
-                B2_TRY(parallel_inputs(m, L, W, x, R, two, L.lproj > 0 ? L.lproj : L.pproj, x, n1, n2, in1, in2, st));
                 RowFeedForward rf;
-                const RowFeedForward* ride = !two && row_feed_forward(lin, L, W, in1, x, rm, R, rf) ? &rf : nullptr;
+                const RowFeedForward* ride = nullptr;
+                if (R == 1 && !two && s.d.norm_kind != B2_NORM_DYT) {   // one row is normed on its way into the launch of the first products
+                    in1 = SubIn(x);
+                    in1.rms = W.norm1.as<float>();
+                    if (row_feed_forward(lin, L, W, in1, x, rm, R, rf)) ride = &rf;
+                }
+                if (ride == nullptr) {
+                    in1 = SubIn();
+                    B2_TRY(parallel_inputs(m, L, W, x, R, two, L.lproj > 0 ? L.lproj : L.pproj, x, n1, n2, in1, in2, st));
+                    if (!two && row_feed_forward(lin, L, W, in1, x, rm, R, rf)) ride = &rf;
+                }
                 if (early) B2_TRY(gelu_up(m, L, W, in2, x, R, st));   // reads x (through its norm) before the mixer's output joins it
                 if (d.type == B2_MIXER_LATENT_ATTN) {
                     SeqLayerState& KS = d.la_kv_from > 0 ? state.layer[s.runs[ri].kv_run] : S;
@@ -1000,7 +1022,7 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
                 } else if (d.type == B2_MIXER_MLSTM || d.type == B2_MIXER_DELTA) {
                     B2_TRY(memory_mixer(m, L, W, S, in1, x, rm, 1, R, nseg, st));
                 } else if (d.type == B2_MIXER_GLA) {
-                    B2_TRY(gla_mixer(m, L, W, S, in1.h, x, rm, 1, R, nseg, st, ride));
+                    B2_TRY(gla_mixer(m, L, W, S, in1, x, rm, 1, R, nseg, st, ride));
                 } else {
                     B2_TRY(hgrn2_mixer(m, L, W, S, in1.h, x, rm, 1, R, nseg, st));
                 }
@@ -1129,16 +1151,25 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
 }
 
 // token rows -> x (and the kept copy x0 of a looped model); tokens are indexed by row
-static int seq_embed(b2_model* m, b2_kv* kv, const int32_t* tokens, int R, int nseg, cudaStream_t st) {
+static int seq_embed(b2_model* m, b2_kv* kv, const int32_t* tokens, int R, int nseg, cudaStream_t st, const DecodeRows* rows = nullptr) {
     SeqModel& s = *m->seq;
+    if (rows != nullptr && (s.d.bigram_buckets > 0 || s.x0.p != nullptr || s.embed_nw.p != nullptr)) {
+        B2_TRY(rowmap_decode(*rows, R, st));
+        rows = nullptr;
+    }
     if (s.d.bigram_buckets > 0 || s.x0.p != nullptr)
         return embed_bigram_rows_f32(tokens, s.segs.as<SeqSeg>(), nseg, nseg == 1 ? R : 1, s.embed.p, s.bigram.p, s.w_dtype, kv->seq->last_tok.as<int32_t>(),
                                      s.x.as<float>(), s.x0.as<float>(), s.d.width, s.d.vocab, s.d.bigram_buckets, s.d.bigram_mul_prev, s.d.bigram_mul_cur,
                                      m->err_dev, st);
     return embed_rows_f32(tokens, s.embed.p, s.w_dtype, s.x.as<float>(), R, s.d.width, s.d.vocab, m->err_dev, st, s.d.embed_scale != 0.f ? s.d.embed_scale : 1.f,
-                          s.embed_nw.as<float>(), s.d.norm_eps);
+                          s.embed_nw.as<float>(), s.d.norm_eps, rows);
 }
 
+static int seq_cap_logits(const SeqModel& s, float* logits, int n, int64_t ld, cudaStream_t st) {
+    if (!(s.d.logit_softcap > 0.f)) return 0;
+    B2_CHECK_ARG(ld == s.d.vocab, "seq_head: soft-capped logits are contiguous rows");
+    return softcap_f32(logits, (size_t)n * s.d.vocab, s.d.logit_softcap, st);
+}
 // rows `index` (null: all) of x -> final norm -> head -> soft-cap: fp32 logits [n, vocab]
 static int seq_head(b2_model* m, const int32_t* index, int n, float* logits, int64_t ld, cudaStream_t st) {
     SeqModel& s = *m->seq;
@@ -1161,25 +1192,30 @@ static int seq_head(b2_model* m, const int32_t* index, int n, float* logits, int
         }
     } else if (s.d.block == B2_BLOCK_PRE_RMS1)
         B2_TRY(rms_scalar_f32(s.x.as<float>(), index, s.final_w.as<float>(), nullptr, nullptr, s.xn.as<float>(), n, s.d.width, s.d.norm_eps, st));
-    else if (s.d.block == B2_BLOCK_SANDWICH_RMS || s.d.block == B2_BLOCK_PARALLEL_RMS || s.d.block == B2_BLOCK_PARALLEL2)
+    else if (s.d.block == B2_BLOCK_SANDWICH_RMS || s.d.block == B2_BLOCK_PARALLEL_RMS || s.d.block == B2_BLOCK_PARALLEL2) {
+        if (n == 1 && index == nullptr && tc_enabled()) {   // one row is normed on its way into the head
+            LinearArgs a = lin.args(s.x.as<float>(), s.d.width, head, s.d.vocab, s.d.width, logits, ld, 1, LIN_NONE, lscale);
+            a.rms_w = s.final_w.as<float>(); a.rms_eps = s.d.norm_eps;
+            if (linear_stream_norms(a)) {
+                B2_TRY(linear_stream_f32(a, st));
+                return seq_cap_logits(s, logits, n, ld, st);
+            }
+        }
         B2_TRY(rms_weight_f32(s.x.as<float>(), s.d.width, index, s.final_w.as<float>(), s.xn.as<float>(), s.d.width, 0, n, s.d.width, s.d.norm_eps, st));
-    else
+    } else
         B2_TRY(layernorm_gather_f32(s.x.as<float>(), index, s.final_w.as<float>(), s.final_b.as<float>(), s.xn.as<float>(), n, s.d.width, s.d.norm_eps, st));
     B2_TRY(lin(in, s.d.width, head, s.d.vocab, s.d.width, logits, ld, n, LIN_NONE, lscale, 0, nullptr, 0, nullptr, in16, dn.alpha != nullptr ? &dn : nullptr));
-    if (s.d.logit_softcap > 0.f) {
-        B2_CHECK_ARG(ld == s.d.vocab, "seq_head: soft-capped logits are contiguous rows");
-        B2_TRY(softcap_f32(logits, (size_t)n * s.d.vocab, s.d.logit_softcap, st));
-    }
-    return 0;
+    return seq_cap_logits(s, logits, n, ld, st);
 }
 
 // one decode step over the slots [slot0, slot0 + B): kv->tok -> logits (m->logits) -> token selection, lengths += 1
 int seq_decode_launch(b2_model* m, b2_kv* kv, int B, int slot0, cudaStream_t st) {
     SeqModel& s = *m->seq;
     s.portion = false;
-    RowMap rm{s.segs.as<SeqSeg>(), s.row_slot.as<int32_t>(), s.row_pos.as<int32_t>()};
-    B2_TRY(rowmap_decode(rm, kv->len_dev.as<int32_t>(), kv->sstate.as<SampleState>(), kv->rows_dev.as<RowState>(), slot0, B, st));
-    B2_TRY(seq_embed(m, kv, kv->tok.as<int32_t>() + slot0, B, B, st));
+    DecodeRows rows;   // (the row map is made where the rows are embedded: a launch between the graph's first and the next took 4.6 us of a step)
+    rows.rm = RowMap{s.segs.as<SeqSeg>(), s.row_slot.as<int32_t>(), s.row_pos.as<int32_t>()};
+    rows.len = kv->len_dev.as<int32_t>(); rows.sstate = kv->sstate.as<SampleState>(); rows.rows_state = kv->rows_dev.as<RowState>(); rows.slot0 = slot0;
+    B2_TRY(seq_embed(m, kv, kv->tok.as<int32_t>() + slot0, B, B, st, &rows));
     B2_TRY(seq_forward(m, kv, B, B, 0, 0, nullptr, st));
     B2_TRY(seq_head(m, nullptr, B, m->logits.as<float>(), s.d.vocab, st));
     B2_TRY(sample_publish(m->logits.as<float>(), s.d.vocab, B, kv->sstate.as<SampleState>(), kv->rows_dev.as<RowState>() + slot0,

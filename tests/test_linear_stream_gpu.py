@@ -129,3 +129,13 @@ def test_products_that_share_a_launch(mixer, width, ff, n, monkeypatch):
     cfg = config([dict(mix, mlp={"kind": "dense", "ff": ff, "limit": 7.0})], width=width, vocab=101)
     w = O.random_weights(cfg, seed=5)
     both_ways(lambda: residuals(cfg, w, n, 2), monkeypatch, bound(width, ff, 3 * 40, 4 * 24))
+
+
+# One row normed on its way into the launch of the first products, and into the head: widths around one and several turns of a CTA, the widest and one beyond
+@pytest.mark.parametrize("width", [64, 72, 1024, 1032, 2056, 4096, 4104])
+@pytest.mark.parametrize("mixer", ["gla", "win"])
+def test_one_row_normed_on_its_way_in(mixer, width, monkeypatch):
+    mix = {"gla": gla(3, 16, 40), "win": win(2, 1, 32, 40, 11, 3, 8)}[mixer]
+    cfg = config([dict(mix, mlp={"kind": "dense", "ff": 72, "limit": 7.0})], width=width, vocab=1003)
+    w = O.random_weights(cfg, seed=6)
+    both_ways(lambda: residuals(cfg, w, 5, 3), monkeypatch, bound(width, 72, 3 * 40, 2 * 40))
