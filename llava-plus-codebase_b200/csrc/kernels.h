@@ -460,7 +460,7 @@ int embed_rows_f32(const int32_t* tokens, const void* table, int table_dtype, fl
 // Differential attention, per (row, head): d = a1 - lambda a2 over the head's dv values, out = d / sqrt(mean(d^2) + eps) * out_scale.
 // y holds map 1 of every head, then map 2 of every head: [rows, 2 * heads * dv]
 int diff_combine_f32(const float* y, int64_t ldy, float* out, int64_t ldo, int rows, int heads, int dv, float lambda, float out_scale, float eps,
-                     cudaStream_t stream);
+                     cudaStream_t stream, void* out16 = nullptr);   // out16: bf16 rows of pitch ldo in place of out
 // out[r, c] = a[r, c] * sigmoid(g[r, c])
 int sigmoid_gate_f32(const float* a, int64_t lda, const float* g, int64_t ldg, float* out, int64_t ldo, int rows, int cols, cudaStream_t stream);
 

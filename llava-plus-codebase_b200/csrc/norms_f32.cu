@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(256) concat_rows_kernel(const float* __restric
 // differential attention: one warp per (row, head) subtracts lambda times the second map's output from the first map's and brings
 // the difference to unit RMS
 __global__ void diff_combine_kernel(const float* __restrict__ y, int64_t ldy, float* __restrict__ out, int64_t ldo, int rows, int heads, int dv,
-                                    float lambda, float out_scale, float eps) {
+                                    float lambda, float out_scale, float eps, __nv_bfloat16* __restrict__ out16) {
     pdl_enter();
     const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (w >= rows * heads) return;
@@ -226,8 +226,12 @@ __global__ void diff_combine_kernel(const float* __restrict__ y, int64_t ldy, fl
     }
     q = warp_sum(q);
     const float mul = out_scale / sqrtf(q / (float)dv + eps);
-    float* o = out + (size_t)r * ldo + (size_t)h * dv;
-    for (int c = lane; c < dv; c += 32) o[c] = fmaf(-lambda, a2[c], a1[c]) * mul;
+    const size_t o = (size_t)r * ldo + (size_t)h * dv;
+    for (int c = lane; c < dv; c += 32) {
+        const float v = fmaf(-lambda, a2[c], a1[c]) * mul;
+        if (out16 != nullptr) out16[o + c] = __float2bfloat16_rn(v);
+        else out[o + c] = v;
+    }
 }
 
 __device__ __forceinline__ void ld8(const float* p, float (&v)[8]) {
@@ -741,10 +745,10 @@ int group_rmsnorm_f32(const float* y, int64_t ldy, const float* gamma, int gamma
 }
 
 int diff_combine_f32(const float* y, int64_t ldy, float* out, int64_t ldo, int rows, int heads, int dv, float lambda, float out_scale, float eps,
-                     cudaStream_t st) {
-    B2_CHECK_ARG(y && out && y != out && rows > 0 && heads > 0 && dv > 0, "diff_combine: bad argument");
+                     cudaStream_t st, void* out16) {
+    B2_CHECK_ARG(y && (out || out16) && y != out && rows > 0 && heads > 0 && dv > 0, "diff_combine: bad argument");
     const int warps = rows * heads;
-    launch_pdl(diff_combine_kernel, dim3((warps + 7) / 8), dim3(256), 0, st, y, ldy, out, ldo, rows, heads, dv, lambda, out_scale, eps);
+    launch_pdl(diff_combine_kernel, dim3((warps + 7) / 8), dim3(256), 0, st, y, ldy, out, ldo, rows, heads, dv, lambda, out_scale, eps, reinterpret_cast<__nv_bfloat16*>(out16));
     B2_LAUNCH_CHECK();
     return 0;
 }

@@ -456,7 +456,7 @@ static LinearArgs gqa_first(const Lin& lin, const SeqLayerInfo& L, SeqWeights& W
 }
 static LinearArgs gla_first(const Lin& lin, const SeqLayerInfo& L, SeqWeights& W, const SubIn& in, int R) {
     const SeqModel& s = *lin.m->seq;
-    LinearArgs a = lin.args(in.h, s.d.width, W.gla_w, L.pproj, s.d.width, s.proj.as<float>(), L.pproj_ld, R);
+    LinearArgs a = lin.args(in.h, s.d.width, W.gla_w, L.pproj, s.d.width, s.proj.as<float>(), L.pproj_ld, R, LIN_NONE, 1.f, 0, nullptr, 0, in.h16);
     a.rms_w = in.rms; a.rms_eps = s.d.norm_eps;
     return a;
 }
@@ -552,8 +552,10 @@ static int gqa_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeights& 
     if (out16) return lin(nullptr, 0, W.o_w, width, L.ng, target, width, R, LIN_NONE, alpha, accumulate, nullptr, 0, nullptr, s.a16.p);
     const float* yo = s.y.as<float>();
     float* gated = s.gated.as<float>();
+    // two maps without a gate or values to turn back: the joined heads leave as the bf16 operand of W_o too
+    const bool joined16 = maps > 1 && !d.ga_rot_values && d.ga_gate == B2_GATE_NONE && lin.tensor_cores(width, L.ng, target, width, R);
     if (maps > 1) {   // a head's two maps: unit_rms(a1 - lambda a2) * (1 - diff)
-        B2_TRY(diff_combine_f32(yo, (int64_t)maps * L.ng, gated, L.ng, R, H, dv, W.lambda, 1.f - d.ga_diff, s.d.norm_eps, st));
+        B2_TRY(diff_combine_f32(yo, (int64_t)maps * L.ng, gated, L.ng, R, H, dv, W.lambda, 1.f - d.ga_diff, s.d.norm_eps, st, joined16 ? s.a16.p : nullptr));
         yo = gated;
     }
     if (d.ga_rot_values || (d.ga_gate == B2_GATE_CHANNEL && !chan_in_attn)) {
@@ -570,8 +572,9 @@ static int gqa_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeights& 
         B2_TRY(head_gate_f32(yo, L.ng, gates, L.lproj_ld, gated, L.ng, R, H, dv, st));
         yo = gated;
     }
-    if (ff != nullptr) return linear_stream_sum_f32(ff->down, lin.args(yo, L.ng, W.o_w, width, L.ng, target, width, R, LIN_NONE, alpha, accumulate), st);
-    return lin(yo, L.ng, W.o_w, width, L.ng, target, width, R, LIN_NONE, alpha, accumulate);
+    const void* o16 = joined16 ? s.a16.p : nullptr;
+    if (ff != nullptr) return linear_stream_sum_f32(ff->down, lin.args(yo, L.ng, W.o_w, width, L.ng, target, width, R, LIN_NONE, alpha, accumulate, nullptr, 0, o16), st);
+    return lin(yo, L.ng, W.o_w, width, L.ng, target, width, R, LIN_NONE, alpha, accumulate, nullptr, 0, nullptr, o16);
 }
 
 // Gated linear attention: one fused projection [q | k | v | g | a1], the decay logits through the second low-rank matrix, the
@@ -584,7 +587,7 @@ static int gla_mixer(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, SeqLayer
     const int width = s.d.width, H = d.gl_heads, dk = d.gl_dim, dv = d.gl_vdim;
     float* proj = s.proj.as<float>();
     if (ff != nullptr) B2_TRY(linear_stream_side_f32(gla_first(lin, L, W, in, R), ff->up, st));
-    else B2_TRY(lin(in.h, width, W.gla_w, L.pproj, width, proj, L.pproj_ld, R));
+    else B2_TRY(lin(in.h, width, W.gla_w, L.pproj, width, proj, L.pproj_ld, R, LIN_NONE, 1.f, 0, nullptr, 0, nullptr, in.h16));
     float* z = s.wlog.as<float>();   // [R, heads * dim] decay logits without their bias (the recurrence adds it in fp32)
     B2_TRY(lin(proj + 2 * L.pq + 2 * L.pv, L.pproj_ld, W.a2_w, L.pq, d.gl_rank, z, L.pq, R));
     ScanArgs sa;
@@ -601,10 +604,14 @@ static int gla_mixer(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, SeqLayer
     sa.segs = s.segs.as<SeqSeg>(); sa.nseg = nseg;
     sa.rows = R; sa.chunk_scratch = s.scan_chunks.as<float>(); sa.chunk_floats = s.scan_chunks.bytes / F4;
     B2_TRY(linear_scan_f32(sa, st));
-    B2_TRY(gated_group_rmsnorm_f32(s.y.as<float>(), L.pv, proj + 2 * L.pq + L.pv, L.pproj_ld, W.gnorm.as<float>(), s.gated.as<float>(), L.pv, R, L.pv, dv,
-                                   0, s.d.norm_eps, st, 1));
-    if (ff != nullptr) return linear_stream_sum_f32(ff->down, lin.args(s.gated.as<float>(), L.pv, W.o_w, width, L.pv, target, width, R, LIN_NONE, alpha, accumulate), st);
-    return lin(s.gated.as<float>(), L.pv, W.o_w, width, L.pv, target, width, R, LIN_NONE, alpha, accumulate);
+    // (the normed heads leave as the bf16 operand of W_o where that product reads those)
+    const bool tc = lin.tensor_cores(width, L.pv, target, width, R);
+    const void* o16 = tc ? s.a16.p : nullptr;
+    B2_TRY(gated_group_rmsnorm_f32(s.y.as<float>(), L.pv, proj + 2 * L.pq + L.pv, L.pproj_ld, W.gnorm.as<float>(), tc ? nullptr : s.gated.as<float>(), L.pv, R, L.pv, dv,
+                                   0, s.d.norm_eps, st, 1, 0, nullptr, tc ? s.a16.p : nullptr, L.pv));
+    if (ff != nullptr)
+        return linear_stream_sum_f32(ff->down, lin.args(s.gated.as<float>(), L.pv, W.o_w, width, L.pv, target, width, R, LIN_NONE, alpha, accumulate, nullptr, 0, o16), st);
+    return lin(s.gated.as<float>(), L.pv, W.o_w, width, L.pv, target, width, R, LIN_NONE, alpha, accumulate, nullptr, 0, nullptr, o16);
 }
 
 // HGRN2: one fused projection [q | f | v], the recurrence, per-head RMS norm, out-projection.
@@ -726,7 +733,8 @@ static int parallel_inputs(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, fl
     const int Np = (N1 + 7) / 8 * 8;
     if (s.d.norm_kind != B2_NORM_DYT) {
         // a rounded copy beside the fp32 rows where the first product reads bf16 (the other products of both sublayers then read it too)
-        void* h16 = mixer_ok && lin.tensor_cores(N1, width, s.proj.as<float>(), Np, R, W.qkv_b.as<float>(), 0, W.qkv_b16.p) ? s.h1_16.p : nullptr;
+        const bool takes16 = mixer_ok || L.d.type == B2_MIXER_GLA;
+        void* h16 = takes16 && lin.tensor_cores(N1, width, s.proj.as<float>(), Np, R, W.qkv_b.as<float>(), 0, W.qkv_b16.p) ? s.h1_16.p : nullptr;
         B2_TRY(rms_weight_f32(x, width, nullptr, W.norm1.as<float>(), xn, width, 0, R, width, eps, st, h16));
         in1 = SubIn(xn);
         in1.h16 = h16;
@@ -1201,7 +1209,8 @@ static int seq_head(b2_model* m, const int32_t* index, int n, float* logits, int
                 return seq_cap_logits(s, logits, n, ld, st);
             }
         }
-        B2_TRY(rms_weight_f32(s.x.as<float>(), s.d.width, index, s.final_w.as<float>(), s.xn.as<float>(), s.d.width, 0, n, s.d.width, s.d.norm_eps, st));
+        if (s.a16.p != nullptr && lin.tensor_cores(s.d.vocab, s.d.width, logits, ld, n)) in16 = s.a16.p;   // (several rows: as the head reads them)
+        B2_TRY(rms_weight_f32(s.x.as<float>(), s.d.width, index, s.final_w.as<float>(), s.xn.as<float>(), s.d.width, 0, n, s.d.width, s.d.norm_eps, st, const_cast<void*>(in16)));
     } else
         B2_TRY(layernorm_gather_f32(s.x.as<float>(), index, s.final_w.as<float>(), s.final_b.as<float>(), s.xn.as<float>(), n, s.d.width, s.d.norm_eps, st));
     B2_TRY(lin(in, s.d.width, head, s.d.vocab, s.d.width, logits, ld, n, LIN_NONE, lscale, 0, nullptr, 0, nullptr, in16, dn.alpha != nullptr ? &dn : nullptr));
