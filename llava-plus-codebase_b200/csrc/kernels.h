@@ -409,6 +409,8 @@ int glu_rows_f32(const float* in, int64_t ld_in, float* out, int64_t ld_out, int
                  void* out16 = nullptr, int64_t ld_out16 = 0);
 // out[p, :K] = bf16(A[src_row[p], :K]), zeros where src_row[p] < 0: the gathered A operand of a grouped tensor-core product
 int gather_rows_bf16(const float* A, int64_t lda, const int32_t* src_row, void* out, int64_t ld_out, int rows, int K, cudaStream_t stream);
+// the same of rows that are bf16 already, pitches of whole eights on 16 bytes (K % 8 == 0)
+int gather_rows16(const void* A, int64_t lda, const int32_t* src_row, void* out, int64_t ld_out, int rows, int K, cudaStream_t stream);
 // x[r] += alpha * sum_k w[r, k] * y[pair_pos[r * top + k]] (a negative position: an identity expert, h[r] in y's place)
 int moe_combine_f32(float* x, const float* y, int64_t ldy, const int32_t* pair_pos, const float* w, int rows, int top, int cols, float alpha,
                     cudaStream_t stream, const float* h = nullptr, int64_t ldh = 0);
@@ -434,7 +436,7 @@ int group_rmsnorm_f32(const float* y, int64_t ldy, const float* gamma, int gamma
 // One-number RMS norm of pre-norm blocks: out[i] = x[row_index[i]] / sqrt(mean(x^2) + eps) * g[0] (row_index null: row i). With add
 // and/or vec the row is first updated in place, x += add[row] + vec: the opening of a pass of a looped block of layers.
 int rms_scalar_f32(float* x, const int32_t* row_index, const float* g, const float* add, const float* vec, float* out, int rows, int cols,
-                   float eps, cudaStream_t stream);
+                   float eps, cudaStream_t stream, void* out16 = nullptr);   // out16: the rows rounded to bf16 as well
 // dst[b][c][r] = src[b][r][c], elements of 2 or 4 bytes (a stack of matrices transposed one by one)
 int transpose_blocks(const void* src, void* dst, int blocks, int rows, int cols, int elem_size, cudaStream_t stream);
 // PolyNorm: out = c0 N(z) + c1 N(z^2) + c2 N(z^3) + c3, z = in + bias (bias nullable), N(u) = u / sqrt(mean(u^2) + eps) per row; coef on the device

@@ -159,20 +159,55 @@ __global__ void gather_rows_bf16_kernel(const float* __restrict__ A, int64_t lda
     }
 }
 
-// x[r] += alpha * sum_k w[r, k] * y[pair_pos[r * top + k]] (a negative position: h[r] in y's place)
-__global__ void moe_combine_kernel(float* __restrict__ x, const float* __restrict__ y, int64_t ldy, const int32_t* __restrict__ pair_pos,
-                                   const float* __restrict__ w, int top, int cols, float alpha, const float* __restrict__ h, int64_t ldh) {
+// ... rows that are bf16 already: whole 16 bytes (5120 rows of 2048 from 1536: 17.9 us from fp32 rows, 5.6)
+__global__ void __launch_bounds__(256) gather_rows16_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const int32_t* __restrict__ src_row, __nv_bfloat16* __restrict__ out,
+                                                            int64_t ld_out, int rows, int chunks) {
+    pdl_enter_late();
+    const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    const int p = (int)(e / chunks), c = (int)(e - (int64_t)p * chunks) * 8;
+    if (p >= rows) return;
+    const int src = src_row[p];
+    *reinterpret_cast<uint4*>(out + (size_t)p * ld_out + c) = src >= 0 ? *reinterpret_cast<const uint4*>(A + (size_t)src * lda + c) : make_uint4(0, 0, 0, 0);
+}
+
+// x[r] += alpha * sum_k w[r, k] * y[pair_pos[r * top + k]] (a negative position: h[r] in y's place). V: columns per thread; the rows of two choices
+// are on their way at a time
+template <int V>
+__global__ void __launch_bounds__(256) moe_combine_kernel(float* __restrict__ x, const float* __restrict__ y, int64_t ldy, const int32_t* __restrict__ pair_pos,
+                                                          const float* __restrict__ w, int top, int cols, float alpha, const float* __restrict__ h, int64_t ldh) {
     pdl_enter_late();
     const size_t r = blockIdx.y;
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) * V;
     if (c >= cols) return;
-    float acc = 0.f;
-    for (int k = 0; k < top; ++k) {
+    float acc[V], old[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) acc[i] = 0.f;
+    const auto load = [](const float* p, float (&v)[V]) {
+        if constexpr (V == 4) {
+            const float4 f = *reinterpret_cast<const float4*>(p);
+            v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+        } else {
+            v[0] = *p;
+        }
+    };
+    load(x + r * cols + c, old);
+    for (int k = 0; k < top; k += 2) {
         const size_t p = r * top + k;
-        const int pos = pair_pos[p];
-        acc = fmaf(w[p], pos >= 0 ? y[(size_t)pos * ldy + c] : h[r * ldh + c], acc);
+        const int p0 = pair_pos[p], p1 = k + 1 < top ? pair_pos[p + 1] : -1;
+        float a[V], b[V];
+        load(p0 >= 0 ? y + (size_t)p0 * ldy + c : h + r * ldh + c, a);
+        if (k + 1 < top) load(p1 >= 0 ? y + (size_t)p1 * ldy + c : h + r * ldh + c, b);
+        const float w0 = w[p], w1 = k + 1 < top ? w[p + 1] : 0.f;
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            acc[i] = fmaf(w0, a[i], acc[i]);
+            if (k + 1 < top) acc[i] = fmaf(w1, b[i], acc[i]);
+        }
     }
-    x[r * cols + c] += alpha * acc;
+#pragma unroll
+    for (int i = 0; i < V; ++i) old[i] += alpha * acc[i];
+    if constexpr (V == 4) *reinterpret_cast<float4*>(x + r * cols + c) = make_float4(old[0], old[1], old[2], old[3]);
+    else x[r * cols + c] = old[0];
 }
 }  // namespace
 
@@ -216,10 +251,26 @@ int gather_rows_bf16(const float* A, int64_t lda, const int32_t* src_row, void* 
     return 0;
 }
 
+int gather_rows16(const void* A, int64_t lda, const int32_t* src_row, void* out, int64_t ld_out, int rows, int K, cudaStream_t st) {
+    B2_CHECK_ARG(A && src_row && out && rows > 0 && K > 0 && K % 8 == 0 && lda % 8 == 0 && ld_out % 8 == 0 && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(out)) & 15) == 0,
+                 "gather_rows16: bad argument");
+    launch_pdl(gather_rows16_kernel, dim3((unsigned)(((int64_t)rows * (K / 8) + 255) / 256)), dim3(256), 0, st, reinterpret_cast<const __nv_bfloat16*>(A), lda, src_row,
+               reinterpret_cast<__nv_bfloat16*>(out), ld_out, rows, K / 8);
+    B2_LAUNCH_CHECK();
+    return 0;
+}
+
 int moe_combine_f32(float* x, const float* y, int64_t ldy, const int32_t* pair_pos, const float* w, int rows, int top, int cols, float alpha,
                     cudaStream_t st, const float* h, int64_t ldh) {
     B2_CHECK_ARG(x && y && w && pair_pos && rows > 0 && top > 0 && cols > 0, "moe_combine: bad argument");
-    launch_pdl(moe_combine_kernel, dim3((cols + 255) / 256, rows), dim3(256), 0, st, x, y, ldy, pair_pos, w, top, cols, alpha, h, ldh);
+    // whole 16 bytes (1536 rows of 2048, two choices: 20.3 -> 8.7 us)
+    const uintptr_t align = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(h);
+    if (cols % 4 == 0 && ldy % 4 == 0 && ldh % 4 == 0 && (align & 15) == 0) {
+        const int threads = cols / 4 >= 256 ? 256 : 64;
+        launch_pdl(moe_combine_kernel<4>, dim3((cols / 4 + threads - 1) / threads, rows), dim3(threads), 0, st, x, y, ldy, pair_pos, w, top, cols, alpha, h, ldh);
+    } else {
+        launch_pdl(moe_combine_kernel<1>, dim3((cols + 255) / 256, rows), dim3(256), 0, st, x, y, ldy, pair_pos, w, top, cols, alpha, h, ldh);
+    }
     B2_LAUNCH_CHECK();
     return 0;
 }

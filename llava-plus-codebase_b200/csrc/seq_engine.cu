@@ -318,7 +318,7 @@ static void portion_of(const SeqModel& s, int nseg, int slot, int ctx_end, BiasA
 
 // Attention over a low-rank latent. S: the run's own state (rotation table); KS: the state whose cache rows it reads (its own,
 // or an earlier layer's). slot / ctx_end as for seq_forward.
-static int latent_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeights& W, SeqLayerState& S, SeqLayerState& KS, const float* h, float* target,
+static int latent_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeights& W, SeqLayerState& S, SeqLayerState& KS, const SubIn& in, float* target,
                         float alpha, int accumulate, int R, int nseg, int slot, int ctx_end, cudaStream_t st) {
     SeqModel& s = *m->seq;
     SeqState& state = *kv->seq;
@@ -334,7 +334,7 @@ static int latent_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeight
     const int32_t* row_pos = s.row_pos.as<int32_t>();
     const float2* tab = S.rot_tab.as<float2>();
     float* proj = s.proj.as<float>();  // [R, q (or the queries' latent) | dkv | g]
-    B2_TRY(lin(h, width, W.qdg_w, L.pproj, width, proj, L.pproj_ld, R));
+    B2_TRY(lin(in.h, width, W.qdg_w, L.pproj, width, proj, L.pproj_ld, R, LIN_NONE, 1.f, 0, nullptr, 0, nullptr, in.h16));
     float* q = proj;
     int64_t ldq = L.pproj_ld;
     if (d.la_q_rank > 0) {   // queries through their latent: norm in place, then up
@@ -380,10 +380,21 @@ static int latent_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeight
         const DevBuf& wk = rd > 0 ? W.ukx_w : W.uk_w;
         for (int m0 = first; m0 < ctx_end; m0 += s.rows) {
             const int mc = std::min(s.rows, ctx_end - m0);
-            B2_TRY(lin(lat + (size_t)m0 * lrow, lrow, wk, L.lqw, lrow, state.kmat.as<float>() + (size_t)m0 * state.kmat_ld, state.kmat_ld, mc));
-            B2_TRY(lin(lat + (size_t)m0 * lrow, lrow, W.uv_w, L.pv, rank, state.vmat.as<float>() + (size_t)m0 * state.vmat_ld, state.vmat_ld, mc));
+            const float* l0 = lat + (size_t)m0 * lrow;
+            float *km = state.kmat.as<float>() + (size_t)m0 * state.kmat_ld, *vm = state.vmat.as<float>() + (size_t)m0 * state.vmat_ld;
+            // (without a rotated part both products read the same rows: rounded once)
+            const void* l16 = rd == 0 && lin.tensor_cores(L.lqw, lrow, km, state.kmat_ld, mc) && lin.tensor_cores(L.pv, rank, vm, state.vmat_ld, mc) ? s.a16.p : nullptr;
+            if (l16 != nullptr) B2_TRY(cast_rows_bf16(l0, lrow, s.a16.p, lrow, mc, lrow, st));
+            B2_TRY(lin(l0, lrow, wk, L.lqw, lrow, km, state.kmat_ld, mc, LIN_NONE, 1.f, 0, nullptr, 0, nullptr, l16));
+            B2_TRY(lin(l0, lrow, W.uv_w, L.pv, rank, vm, state.vmat_ld, mc, LIN_NONE, 1.f, 0, nullptr, 0, nullptr, l16));
         }
+        // the heads' sigmoid gates ride in the attention's last write, and the output leaves as the bf16 operand of W_o where that product reads those (19 us
+        // of gating and casting before, 1536 rows of 16 heads of 128)
+        if (gate) { ah.head_gate = gates; ah.ldg = L.pproj_ld; }
+        const void* o16 = lin.tensor_cores(width, L.pv, target, width, R) ? s.a16.p : nullptr;
+        if (o16 != nullptr) ah.out16 = s.a16.p;
         B2_TRY(attn_bias_f32(ah, st));
+        return lin(y, L.pv, W.o_w, width, L.pv, target, width, R, LIN_NONE, alpha, accumulate, nullptr, 0, nullptr, o16);
     } else {
         // absorbed form: q_h -> W_uk_h^T q_h lives in the latent space (the rotated part rides behind it), so scores and values
         // read the cached rows directly, and W_uv_h carries the latent-space output to the head's values
@@ -615,14 +626,14 @@ static int gla_mixer(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, SeqLayer
 }
 
 // HGRN2: one fused projection [q | f | v], the recurrence, per-head RMS norm, out-projection.
-static int hgrn2_mixer(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, SeqLayerState& S, const float* h, float* target, float alpha, int accumulate,
+static int hgrn2_mixer(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, SeqLayerState& S, const SubIn& in, float* target, float alpha, int accumulate,
                        int R, int nseg, cudaStream_t st) {
     SeqModel& s = *m->seq;
     const b2_seq_layer_desc& d = L.d;
     const Lin lin{m, st};
     const int width = s.d.width, H = d.g_heads, dk = d.g_dim, dv = d.g_vdim;
     float* proj = s.proj.as<float>();  // [R, q | f | v]
-    B2_TRY(lin(h, width, W.qfv_w, L.pproj, width, proj, L.pproj_ld, R));
+    B2_TRY(lin(in.h, width, W.qfv_w, L.pproj, width, proj, L.pproj_ld, R, LIN_NONE, 1.f, 0, nullptr, 0, nullptr, in.h16));
     ScanArgs sa;
     sa.mode = SCAN_HGRN2;
     sa.q = proj; sa.ldq = L.pproj_ld;
@@ -939,7 +950,8 @@ static int seq_feed_forward(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, c
         // expert's rows of the stacked weight matrices in ONE launch per product
         __nv_bfloat16* a16 = s.moe_a16.as<__nv_bfloat16>();
         __nv_bfloat16* h16 = a16 + (size_t)s.moe_rows * width;
-        B2_TRY(gather_rows_bf16(h, width, s.moe_src.as<int32_t>(), a16, width, P, width, st));
+        if (in.h16 != nullptr) B2_TRY(gather_rows16(in.h16, width, s.moe_src.as<int32_t>(), a16, width, P, width, st));
+        else B2_TRY(gather_rows_bf16(h, width, s.moe_src.as<int32_t>(), a16, width, P, width, st));
         GemmArgs g1;
         g1.A = a16; g1.lda = width; g1.W = W.egu_w.p; g1.ldw = width; g1.out = s.moe_h.p; g1.ld_out = un; g1.out_fp32 = 1;
         g1.M = P; g1.N = un; g1.K = width; g1.tile_group = s.moe_tile.as<int32_t>(); g1.groups = E;
@@ -1024,7 +1036,7 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
                 if (early) B2_TRY(gelu_up(m, L, W, in2, x, R, st));   // reads x (through its norm) before the mixer's output joins it
                 if (d.type == B2_MIXER_LATENT_ATTN) {
                     SeqLayerState& KS = d.la_kv_from > 0 ? state.layer[s.runs[ri].kv_run] : S;
-                    B2_TRY(latent_mixer(m, kv, L, W, S, KS, in1.h, x, rm, 1, R, nseg, slot, ctx_end, st));
+                    B2_TRY(latent_mixer(m, kv, L, W, S, KS, in1, x, rm, 1, R, nseg, slot, ctx_end, st));
                 } else if (d.type == B2_MIXER_GQA_ATTN) {
                     B2_TRY(gqa_mixer(m, kv, L, W, S, in1, x, rm, 1, R, nseg, slot, ctx_end, st, ride));
                 } else if (d.type == B2_MIXER_MLSTM || d.type == B2_MIXER_DELTA) {
@@ -1032,7 +1044,7 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
                 } else if (d.type == B2_MIXER_GLA) {
                     B2_TRY(gla_mixer(m, L, W, S, in1, x, rm, 1, R, nseg, st, ride));
                 } else {
-                    B2_TRY(hgrn2_mixer(m, L, W, S, in1.h, x, rm, 1, R, nseg, st));
+                    B2_TRY(hgrn2_mixer(m, L, W, S, in1, x, rm, 1, R, nseg, st));
                 }
                 if (early) B2_TRY(gelu_down(m, L, W, x, rm, 1, R, st));
                 else if (d.ff > 0 && ride == nullptr) B2_TRY(seq_feed_forward(m, L, W, in2, x, rm, 1, R, st));
@@ -1040,24 +1052,30 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
                     B2_CUDA_CHECK(cudaMemcpyAsync(resid_out + ri * (size_t)R * width, x, (size_t)R * width * F4, cudaMemcpyDeviceToDevice, st));
                 continue;
             }
-            if (pre) B2_TRY(rms_scalar_f32(x, nullptr, W.norm1.as<float>(), pass_add, pass_vec, xn, R, width, eps, st));
+            // (the normed rows of a prompt leave rounded as well: what the products, and the experts' gather, read)
+            void* h16 = pre && R > 1 && s.h1_16.p != nullptr && lin.tensor_cores(32, width, s.proj.as<float>(), 32, R) ? s.h1_16.p : nullptr;
+            if (pre) B2_TRY(rms_scalar_f32(x, nullptr, W.norm1.as<float>(), pass_add, pass_vec, xn, R, width, eps, st, h16));
             else B2_TRY(sandwich_input(s, post, W.norm1, W.canon1, S.canon1, R, nseg, max_n, st, &h));
+            SubIn in(h);
+            in.h16 = h16;
             if (d.type == B2_MIXER_LATENT_ATTN) {
                 SeqLayerState& KS = d.la_kv_from > 0 ? state.layer[s.runs[ri].kv_run] : S;
-                B2_TRY(latent_mixer(m, kv, L, W, S, KS, h, target, alpha, acc, R, nseg, slot, ctx_end, st));
+                B2_TRY(latent_mixer(m, kv, L, W, S, KS, in, target, alpha, acc, R, nseg, slot, ctx_end, st));
             } else if (d.type == B2_MIXER_GQA_ATTN) {
-                B2_TRY(gqa_mixer(m, kv, L, W, S, h, target, alpha, acc, R, nseg, slot, ctx_end, st));
+                B2_TRY(gqa_mixer(m, kv, L, W, S, in, target, alpha, acc, R, nseg, slot, ctx_end, st));
             } else if (d.type == B2_MIXER_GLA) {
-                B2_TRY(gla_mixer(m, L, W, S, h, target, alpha, acc, R, nseg, st));
+                B2_TRY(gla_mixer(m, L, W, S, in, target, alpha, acc, R, nseg, st));
             } else {
-                B2_TRY(hgrn2_mixer(m, L, W, S, h, target, alpha, acc, R, nseg, st));
+                B2_TRY(hgrn2_mixer(m, L, W, S, in, target, alpha, acc, R, nseg, st));
             }
             post = sandwich ? W.norm1_b.as<float>() : nullptr;
             if (d.ff > 0) {
                 h = xn;
-                if (pre) B2_TRY(rms_scalar_f32(x, nullptr, W.norm2.as<float>(), nullptr, nullptr, xn, R, width, eps, st));
+                if (pre) B2_TRY(rms_scalar_f32(x, nullptr, W.norm2.as<float>(), nullptr, nullptr, xn, R, width, eps, st, h16));
                 else if (sandwich) B2_TRY(sandwich_input(s, post, W.norm2, W.canon2, S.canon2, R, nseg, max_n, st, &h));
-                B2_TRY(seq_feed_forward(m, L, W, h, target, alpha, acc, R, st));
+                SubIn in2(h);
+                in2.h16 = h16;
+                B2_TRY(seq_feed_forward(m, L, W, in2, target, alpha, acc, R, st));
                 post = sandwich ? W.norm2_b.as<float>() : nullptr;
             }
             if (post != nullptr && (resid_out != nullptr || ri + 1 == s.runs.size())) {   // the last sublayer's output joins x now
@@ -1748,7 +1766,7 @@ int seq_finalize(b2_model* m) {
     if (s.d.block == B2_BLOCK_PARALLEL2) B2_TRY(s.h2.alloc(R * width * F4));
     if (den_w > 0) B2_TRY(s.den.alloc(R * den_w * F4));
     if (s.d.compute == B2_COMPUTE_BF16) {
-        if (dyt || s.d.block == B2_BLOCK_PARALLEL_RMS || s.d.block == B2_BLOCK_PARALLEL2) B2_TRY(s.h1_16.alloc(R * width * 2));
+        if (dyt || s.d.block == B2_BLOCK_PARALLEL_RMS || s.d.block == B2_BLOCK_PARALLEL2 || (s.d.block == B2_BLOCK_PRE_RMS1 && width % 8 == 0)) B2_TRY(s.h1_16.alloc(R * width * 2));
         if (dyt) B2_TRY(s.h2_16.alloc(R * width * 2));
         if (gelu) B2_TRY(s.f16.alloc(R * fw * 2));
     }

@@ -451,3 +451,18 @@ def test_sampled_generation_repeats_with_the_seed_and_rejects_bad_input():
         model.generate(torch.tensor([[cfg["vocab"] + 3, 1, 2]]), max_new_tokens=2)
     with pytest.raises(ValueError):
         model.generate(p, max_new_tokens=4000)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("width", [36, 40, 510, 512, 520, 2052, 2056])
+@pytest.mark.parametrize("rows", [2, 63, 64, 129])
+def test_rows_of_norms_and_experts(width, rows, dtype):
+    """Whole-row norms with and without a rounded copy, gathered rows and the sum of one to three choices, around the widths of their 16-byte forms"""
+    cfg = config([layer(LAT, MOE if rows % 2 else MOE_SINGLES), layer(HG, MOE_ONE)], width=width, softcap=None)
+    model, w = build(cfg, dtype, max_batch=1, max_seq=rows + 1, max_rows=rows)
+    toks = tokens_for(cfg, rows)
+    got = model._ensure_engine().append_tokens(model._ensure_engine().new_kv(1, rows + 1), 0, toks, restart=True, residuals=True)[1]
+    ref = O.forward(cfg, w, toks)[1]
+    model.invalidate_engine()
+    for a, b in zip(got, ref):
+        assert close(a, b, dtype)
