@@ -1,6 +1,6 @@
 // bf16 GEMM whose K is cut over the CTAs of a cluster: C[M,N] = epilogue(A[M,K] · W[N,K]^T) for shapes whose output tiles do not fill the SMs
-// (short prompts, one or two pictures). The plain kernel (gemm_tcgen05.cu) then walks a long K on a few SMs, bound by what ONE SM can take
-// out of L2; here S = 2 or 4 CTAs of a cluster take a slice of K each, with the same TMA ring and tcgen05 products, and their partial tiles meet
+// (short prompts, one to four pictures). The plain kernel (gemm_tcgen05.cu) then walks a long K on a few SMs, bound by what ONE SM can take
+// out of L2; here S = 2 to 4 CTAs of a cluster take a slice of K each, with the same TMA ring and tcgen05 products, and their partial tiles meet
 // in distributed shared memory: every CTA puts its accumulator into its drained ring, the cluster synchronises, and CTA r adds up its 1/S of
 // the columns from all S rings in rank order (deterministic, fp32) and runs the epilogue for them. No workspace, no second launch.
 // M = 64, N = 2048, K = 5120: 23.0 us on 32 SMs -> 11.4 us on 128; N = 4096, K = 11008: 46.4 -> 21.6 us.
@@ -19,7 +19,7 @@ constexpr int KS_BM = 128, KS_BK = 64, KS_THREADS = 320, KS_A = KS_BM * KS_BK * 
 
 template <int BN>
 struct KsCfg {
-    static constexpr int STAGE = KS_A + BN * KS_BK * 2, STAGES = BN == 128 ? 6 : 8, SMEM = STAGES * STAGE + 1024 + 256;
+    static constexpr int STAGE = KS_A + BN * KS_BK * 2, STAGES = BN == 256 ? 4 : BN == 128 ? 6 : 8, SMEM = STAGES * STAGE + 1024 + 256;
     static_assert(KS_BM * BN * 4 <= STAGES * STAGE, "the partial tile lies in the drained ring");
 };
 
@@ -140,10 +140,9 @@ __global__ void __launch_bounds__(KS_THREADS, 1) gemm_splitk_kernel(const __grid
     cluster_sync();
     if (warp >= 2) {
         pdl_wait();   // residual and output may be written by the kernels in front
-        const int t = threadIdx.x - 64, row = t & 127, per = BN / S / 8;   // 8-column groups of this CTA's share
+        const int t = threadIdx.x - 64, row = t & 127, g1 = BN / 8 * (rank + 1) / S;   // 8-column groups of this CTA's share
         const uint32_t base = smem_u32(smem);
-        for (int j = t >> 7; j < per && m0 + row < M; j += 2) {
-            const int c8 = rank * per + j;   // group of 8 columns inside the tile
+        for (int c8 = BN / 8 * rank / S + (t >> 7); c8 < g1 && m0 + row < M; c8 += 2) {   // group of 8 columns inside the tile
             float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             for (int s = 0; s < S; ++s) {
                 const float4 u = ks_ld_remote(base + (uint32_t)((2 * c8) * KS_BM + row) * 16, s), w = ks_ld_remote(base + (uint32_t)((2 * c8 + 1) * KS_BM + row) * 16, s);
@@ -209,7 +208,7 @@ int splitk_act(const GemmArgs& g, int S, const KsEpi& ep, cudaStream_t st) {
 }  // namespace
 
 int gemm_bf16_splitk(const GemmArgs& g, int bn, int S, cudaStream_t st) {
-    B2_CHECK_ARG((bn == 64 || bn == 128) && (S == 2 || S == 4) && S <= (g.K + KS_BK - 1) / KS_BK && g.tile_group == nullptr, "gemm(split K): bad plan bn=%d S=%d K=%d", bn, S, g.K);
+    B2_CHECK_ARG((bn == 64 || bn == 128 || bn == 256) && S >= 2 && S <= 4 && S <= (g.K + KS_BK - 1) / KS_BK && g.tile_group == nullptr, "gemm(split K): bad plan bn=%d S=%d K=%d", bn, S, g.K);
     // (a gated unit's output has half the product's columns: without its epilogue here, the plain one would write past every row)
     B2_CHECK_ARG(g.act == ACT_NONE || g.act == ACT_QUICK_GELU || g.act == ACT_GELU_ERF, "gemm(split K): activation %d has no epilogue here", g.act);
     KsEpi ep;
@@ -218,7 +217,7 @@ int gemm_bf16_splitk(const GemmArgs& g, int bn, int S, cudaStream_t st) {
     ep.bias = reinterpret_cast<const __nv_bfloat16*>(g.bias); ep.residual = reinterpret_cast<const __nv_bfloat16*>(g.residual);
     ep.out = g.out; ep.ld_out = g.ld_out; ep.ld_res = g.ld_res; ep.out_fp32 = g.out_fp32;
     ep.post = g.out_fp32 ? g.post : 0; ep.alpha = g.out_fp32 ? g.alpha : 1.f; ep.accumulate = g.out_fp32 ? g.accumulate : 0;
-    return bn == 64 ? splitk_act<64>(g, S, ep, st) : splitk_act<128>(g, S, ep, st);
+    return bn == 64 ? splitk_act<64>(g, S, ep, st) : bn == 128 ? splitk_act<128>(g, S, ep, st) : splitk_act<256>(g, S, ep, st);
 }
 
 }  // namespace b2

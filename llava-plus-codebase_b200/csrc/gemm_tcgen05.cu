@@ -668,7 +668,11 @@ int gemm_bf16(const GemmArgs& g, cudaStream_t stream) {
     const bool grouped = g.tile_group != nullptr, glu = g.act == ACT_SWIGLU || g.act == ACT_GLU;
     B2_CHECK_ARG(!grouped || (g.groups >= 1 && (g.act == ACT_NONE || g.act == ACT_GLU) && g.bias == nullptr && g.residual == nullptr && g.M % BM == 0),
                  "gemm: a grouped product takes whole tiles of %d rows, no bias, residual or fused activation but the gated unit", BM);
-    if (g.bn_override >= 1000 && !grouped) return gemm_bf16_splitk(g, g.bn_override % 1000, g.bn_override / 1000, stream);
+    if (g.bn_override >= 1000 && !grouped) {
+        const int bn = g.bn_override % 1000, S = g.bn_override / 1000;
+        B2_CHECK_ARG((bn == 64 || bn == 128) && (S == 2 || S == 4) && !glu, "gemm(split K): no plan bn=%d S=%d activation=%d", bn, S, g.act);
+        return gemm_bf16_splitk(g, bn, S, stream);
+    }
     if (g.bn_override == 2 && !grouped) return gemm_bf16_2cta(g, stream);  // CTA-pair kernel (cta_group::2, 256x256 pair tiles)
 
     // Tile-N choice. Cost model fitted to profiles/r1b_gemm_sweep.json: a tile costs ~BN / rel(BN) (rel = tensor-pipe
@@ -701,11 +705,15 @@ int gemm_bf16(const GemmArgs& g, cudaStream_t stream) {
         float split_best = 0.f;
         const int kb = (g.K + BK - 1) / BK;
         if (g.bn_override == 0 && !grouped && !glu) {
-            for (int c = 2; c < 4; ++c)
-                for (int s = 2; s <= 4; s *= 2) {
-                    const long long ctas = (long long)num_m * ((g.N + cand[c] - 1) / cand[c]) * s;
-                    if (ctas > (s == 2 ? num_sms() : 128) || kb < 4 * s) continue;
-                    const float cost = (float)cand[c] / rel[c] / s + 24.f + 1154.f / kb;
+            // Three slices, of which the GPCs hold 45 clusters, take 0.9 us more to meet, and 256 columns 1.2 more again; where two of them leave
+            // SMs idle and four come in two turns they are the best: M = 577, N = 1024, K = 4096 14.6 -> 12.2 us (K = 1024: uncut 6.9, 7.9), M = 16,
+            // N = K = 5120 16.4 -> 14.0, M = 1154, N = 1024, K = 4096 (256 columns) 21.1 uncut -> 17.2.
+            for (int c = 0; c < 4; ++c)
+                for (int s = 2; s <= 4; ++s) {
+                    if (c == 1 || (c == 0 && s != 3) || (c == 3 && s == 3)) continue;
+                    const long long tiles = (long long)num_m * ((g.N + cand[c] - 1) / cand[c]);
+                    if (tiles > (s == 2 ? num_sms() / 2 : s == 3 ? 45 : 32) || kb < 4 * s) continue;
+                    const float cost = (float)cand[c] / rel[c] / s + 24.f + (1154.f + (s == 3 ? 700.f : 0.f) + (c == 0 ? 920.f : 0.f)) / kb;
                     if (split_bn == 0 || cost < split_best) { split_best = cost; split_bn = cand[c]; split_s = s; }
                 }
         }

@@ -67,7 +67,7 @@ int projector_fused_bf16(const void* X, int ldx, const void* W1, const void* b1,
                          void* out, int ld_out, int M, int K1, int N1, int N2, int* row_done, cudaStream_t stream);
 // CTA-pair (cta_group::2, 256x256 pair tiles) variant, gemm_2cta.cu (chosen by gemm_bf16's cost model, or bn_override == 2)
 int gemm_bf16_2cta(const GemmArgs& g, cudaStream_t stream);
-// K cut over clusters of S CTAs, tiles of 128 x bn (gemm_splitk.cu; chosen by gemm_bf16, or bn_override == 1000 * S + bn)
+// K cut over clusters of S CTAs, tiles of 128 x bn (gemm_splitk.cu; chosen by gemm_bf16, or bn_override == 1000 * S + bn for bn 64, 128 and S 2, 4)
 int gemm_bf16_splitk(const GemmArgs& g, int bn, int S, cudaStream_t stream);
 
 // ---- swap-AB stream-K GEMM for decode at batch 7..128 (gemm_skinny.cu): fp8 steps, and bf16 steps of wide models (stream_k_step, model.cu) ----

@@ -38,6 +38,12 @@ def test_split_k(M, N, K, act, f32, bias, residual, plan):
     assert bool(((out - ref).abs() <= tol).all()), float(((out - ref).abs() - tol).max())
 
 
+@pytest.mark.parametrize("M,N,K,act,f32,bias,residual", [(1154, 1024, 4096, 0, 0, 1, 1), (1027, 1000, 4104, 1, 0, 1, 0), (16, 5120, 1544, 0, 1, 0, 0), (500, 1160, 2568, 2, 0, 1, 1)])
+def test_split_in_three(M, N, K, act, f32, bias, residual):
+    """Tiles of 256 columns (the first two) and of 128 whose column groups don't divide by three, through the rule."""
+    test_split_k(M, N, K, act, f32, bias, residual, 0)
+
+
 def test_plans_that_do_not_fit_are_refused():
     A = torch.zeros(16, 128, device="cuda", dtype=torch.bfloat16)
     W = torch.zeros(64, 128, device="cuda", dtype=torch.bfloat16)
