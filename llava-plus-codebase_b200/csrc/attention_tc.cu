@@ -22,6 +22,8 @@
 #include <math.h>
 #include <stdlib.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -30,7 +32,6 @@ namespace {
 
 constexpr int TC_BM = 128;  // queries per CTA
 constexpr int TC_BN = 64;   // keys per tile
-constexpr int TC_THREADS = 192;
 
 __device__ __forceinline__ void tma_load_4d(void* smem_dst, const void* tmap, uint64_t* bar, int c0, int c1, int c2,
                                             int c3) {
@@ -49,6 +50,11 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&v
         "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]),
         "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
         : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
 }
 // MUFU.EX2 without exp2f's denormal-range fix-up (inputs here are <= 8, results feed a bf16 / an fp32 sum)
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -89,20 +95,20 @@ struct FlashTcParams {
     float scale_log2;
 };
 
-template <int D>
+template <int D, int WGS>
 struct TcCfg {
-    static constexpr int Q_BYTES = TC_BM * D * 2, TILE = TC_BN * D * 2, STAGES = D == 64 ? 3 : 2;   // of K and of V each
-    static constexpr int SMEM = Q_BYTES + 2 * STAGES * TILE + 1024 /*align*/ + 256 /*barriers*/;
+    static constexpr int Q_BYTES = TC_BM * D * 2, TILE = TC_BN * D * 2, STAGES = WGS == 2 ? 4 : D == 64 ? 3 : 2;   // of K and of V each
+    static constexpr int SMEM = Q_BYTES + 2 * STAGES * TILE + 1024 /*align*/ + 256 /*barriers*/ + (WGS == 2 ? 2 * TC_BM * 8 : 0) /*maxima and sums of both groups*/;
 };
 
-template <int D, bool CAUSAL>
-__global__ void __launch_bounds__(TC_THREADS, 2)
+template <int D, bool CAUSAL, int WGS>
+__global__ void __launch_bounds__(64 + 128 * WGS, 3 - WGS)
 flash_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, FlashTcParams p) {
-    using Cfg = TcCfg<D>;
+    using Cfg = TcCfg<D, WGS>;
     constexpr int SLABS = D / 64, STAGES = Cfg::STAGES;   // 64-wide (128 B) slabs of the head dim
     constexpr int Q_SLAB = TC_BM * 128, KV_SLAB = TC_BN * 128;
-    constexpr int TMEM_COLS = 256, TM_O = 2 * TC_BN;      // S / P: columns [0, 64) and [64, 128), O: [128, 128 + D)
+    constexpr int NBUF = 2 * WGS, TMEM_COLS = 256 * WGS, TM_O = NBUF * TC_BN;   // S_t / P_t: columns [64 (t % NBUF), + 64), then O of each group of warps
 
     extern __shared__ uint8_t tc_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tc_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -110,8 +116,8 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     uint8_t* sK = sQ + Cfg::Q_BYTES;
     uint8_t* sV = sK + STAGES * Cfg::TILE;
     uint64_t* bars = reinterpret_cast<uint64_t*>(sV + STAGES * Cfg::TILE);
-    uint64_t *q_full = bars, *s_full = bars + 1 /*[2]*/, *p_full = bars + 3 /*[2]*/, *o_done = bars + 5, *o_last = bars + 6;
-    uint64_t *k_full = bars + 7, *k_empty = k_full + STAGES, *v_full = k_empty + STAGES, *v_empty = v_full + STAGES;
+    uint64_t *q_full = bars, *s_full = bars + 1, *p_full = s_full + NBUF, *o_done = p_full + NBUF /*[WGS]*/, *o_last = o_done + WGS;
+    uint64_t *k_full = o_last + WGS, *k_empty = k_full + STAGES, *v_full = k_empty + STAGES, *v_empty = v_full + STAGES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(v_empty + STAGES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -123,12 +129,14 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         tma_prefetch_desc(&tm_k);
         tma_prefetch_desc(&tm_v);
         mbar_init(q_full, 1);
-        for (int s = 0; s < 2; ++s) {
+        for (int s = 0; s < NBUF; ++s) {
             mbar_init(&s_full[s], 1);
-            mbar_init(&p_full[s], 4);  // one arrive per softmax warp; two of them, as P_(t+1) may be announced before anyone waited for P_t
+            mbar_init(&p_full[s], 4);  // one arrive per softmax warp of the group; one a buffer, as P_(t+1) may be announced before anyone waited for P_t
         }
-        mbar_init(o_done, 1);
-        mbar_init(o_last, 1);
+        for (int w = 0; w < WGS; ++w) {
+            mbar_init(&o_done[w], 1);
+            mbar_init(&o_last[w], 1);
+        }
         for (int s = 0; s < 4 * STAGES; ++s) mbar_init(&k_full[s], 1);
         fence_barrier_init();
     }
@@ -145,24 +153,25 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const int len = p.seq_lens != nullptr ? p.seq_lens[b] : p.S;
     const int kv_end = CAUSAL ? min(len, q0 + TC_BM) : len;
     const int T = (max(kv_end, 0) + TC_BN - 1) / TC_BN;  // 0: a request without keys, whose rows are zeros
+    const bool stub = kv_end - (T - 1) * TC_BN <= 16;   // the last tile has a sixteenth of a tile or less (a class token behind 24 x 24 patches)
 
     if (warp == 0) {
         if (lane == 0) {
-            // ---------------- TMA producer: K runs two tiles ahead of V, as the scores do ----------------
+            // ---------------- TMA producer: K runs NBUF tiles ahead of V, as the scores do ----------------
             mbar_arrive_expect_tx(q_full, Cfg::Q_BYTES);
             for (int sl = 0; sl < SLABS; ++sl) {
                 tma_load_4d(sQ + sl * Q_SLAB, &tm_q, q_full, sl * 64, q0, head, b);
                 tma_load_4d(sQ + sl * Q_SLAB + KV_SLAB, &tm_q, q_full, sl * 64, q0 + TC_BN, head, b);
             }
-            for (int t = 0; t < T + 2; ++t) {
+            for (int t = 0; t < T + NBUF; ++t) {
                 if (t < T) {
                     const int s = t % STAGES;
                     mbar_wait(&k_empty[s], ((t / STAGES) & 1) ^ 1);
                     mbar_arrive_expect_tx(&k_full[s], Cfg::TILE);
                     for (int sl = 0; sl < SLABS; ++sl) tma_load_4d(sK + s * Cfg::TILE + sl * KV_SLAB, &tm_k, &k_full[s], sl * 64, t * TC_BN, head, b);
                 }
-                if (t >= 2) {
-                    const int u = t - 2, s = u % STAGES;
+                if (t >= NBUF) {
+                    const int u = t - NBUF, s = u % STAGES;
                     mbar_wait(&v_empty[s], ((u / STAGES) & 1) ^ 1);
                     mbar_arrive_expect_tx(&v_full[s], Cfg::TILE);
                     for (int sl = 0; sl < SLABS; ++sl) tma_load_4d(sV + s * Cfg::TILE + sl * KV_SLAB, &tm_v, &v_full[s], sl * 64, u * TC_BN, head, b);
@@ -183,64 +192,67 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 if (leader)
 #pragma unroll
                 for (int k = 0; k < D / 16; ++k)
-                    umma_bf16(tm + (t & 1) * TC_BN, q_desc + ((k >> 2) * (Q_SLAB >> 4) + (k & 3) * 2), k_desc + ((k >> 2) * (KV_SLAB >> 4) + (k & 3) * 2), idesc_s,
+                    umma_bf16(tm + (t % NBUF) * TC_BN, q_desc + ((k >> 2) * (Q_SLAB >> 4) + (k & 3) * 2), k_desc + ((k >> 2) * (KV_SLAB >> 4) + (k & 3) * 2), idesc_s,
                               k != 0 ? 1u : 0u);
                 if (leader) {
                     umma_commit(&k_empty[s]);
-                    umma_commit(&s_full[t & 1]);
+                    umma_commit(&s_full[t % NBUF]);
                 }
                 __syncwarp();
             };
             mbar_wait(q_full, 0);
 #pragma unroll 1
-            for (int t = -2; t < T; ++t) {
+            for (int t = -NBUF; t < T; ++t) {
                 if (t >= 0) {   // O += P_t V_t once the softmax warps have written P_t (and rescaled O)
-                    const int s = t % STAGES;
+                    const int s = t % STAGES, w = t % WGS;
                     mbar_wait(&v_full[s], (t / STAGES) & 1);
-                    mbar_wait(&p_full[t & 1], (t >> 1) & 1);
+                    mbar_wait(&p_full[t % NBUF], (t / NBUF) & 1);
                     tc_fence_after();
                     const uint64_t v_desc = make_sw128_mnmajor_desc(smem_u32(sV + s * Cfg::TILE), KV_SLAB);
                     if (leader)
 #pragma unroll
-                    for (int k = 0; k < TC_BN / 16; ++k)
-                        umma_ts(tm + TM_O, tm + (t & 1) * TC_BN + k * 8, v_desc + k * 128, idesc_o, (t | k) != 0 ? 1u : 0u);   // 16 key rows of 128 B per step
+                    for (int k = 0; k < TC_BN / 16; ++k)   // 16 key rows of 128 B per step
+                        if (k == 0 || t + 1 < T || !stub) umma_ts(tm + TM_O + w * D, tm + (t % NBUF) * TC_BN + k * 8, v_desc + k * 128, idesc_o, (t >= WGS || k != 0) ? 1u : 0u);
                     if (leader) umma_commit(&v_empty[s]);
                     // the last product has a barrier of its own: its waiters may come while the one before is still under way, and would
                     // take the parity of the one before that for theirs
-                    if (leader) umma_commit(t + 1 < T ? o_done : o_last);
+                    if (leader) umma_commit(t + WGS < T ? &o_done[w] : &o_last[w]);
                     __syncwarp();
-                    if (t + 2 < T) mbar_wait(o_done, t & 1);   // S_(t+2) takes the buffer that P_t was read from
+                    if (t + NBUF < T) mbar_wait(&o_done[w], (t / WGS) & 1);   // S_(t+NBUF) takes the buffer that P_t was read from
                 }
-                if (t + 2 < T) scores(t + 2);
+                if (t + NBUF < T) scores(t + NBUF);
             }
         }
     } else {
         // ---------------- softmax / correction / epilogue: thread r <-> query row q0 + r ----------------
-        const int quad = warp & 3;
+        const int quad = warp & 3, w = WGS == 2 ? (warp - 2) >> 2 : 0;   // group w: tiles w, w + WGS, ... and an O, a maximum and a sum of its own
         const int r = quad * 32 + lane;
         const int qrow = q0 + r;
-        const uint32_t lanes = tm + (static_cast<uint32_t>(quad * 32) << 16);
+        const uint32_t lanes = tm + (static_cast<uint32_t>(quad * 32) << 16), tm_o = lanes + TM_O + w * D;
         float m_run = -INFINITY, l_run = 0.f;
-        for (int t = 0; t < T; ++t) {
+        auto softmax = [&](int t, auto cols) {   // of the first COLS keys of tile t
+            constexpr int COLS = decltype(cols)::value;
             const int key0 = t * TC_BN;
-            const uint32_t buf = lanes + (t & 1) * TC_BN;
-            mbar_wait(&s_full[t & 1], (t >> 1) & 1);
-            tc_fence_after();
-            uint32_t v[2][32];
+            const uint32_t buf = lanes + (t % NBUF) * TC_BN;
+            uint32_t v[COLS];
             __syncwarp();
-            tmem_ld_32x32(buf, v[0]);
-            tmem_ld_32x32(buf + 32, v[1]);
+            if constexpr (COLS == 64) {
+                tmem_ld_32x32(buf, reinterpret_cast<uint32_t(&)[32]>(v[0]));
+                tmem_ld_32x32(buf + 32, reinterpret_cast<uint32_t(&)[32]>(v[32]));
+            } else {
+                tmem_ld_cols(buf, v);
+            }
             tmem_ld_wait();
             // interior tiles need no per-key mask (CTA-uniform test: every key valid for every query row of this CTA)
-            if (!(key0 + TC_BN <= len && (!CAUSAL || key0 + TC_BN - 1 <= q0))) {
+            if (!(key0 + COLS <= len && (!CAUSAL || key0 + COLS - 1 <= q0))) {
                 const int last = (CAUSAL ? min(len - 1, qrow) : len - 1) - key0;   // last visible key of the tile
 #pragma unroll
-                for (int i = 0; i < 64; ++i)
-                    if (i > last) v[i >> 5][i & 31] = __float_as_uint(-INFINITY);
+                for (int i = 0; i < COLS; ++i)
+                    if (i > last) v[i] = __float_as_uint(-INFINITY);
             }
             float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-            for (int i = 0; i < 64; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(v[i >> 5][i & 31]));
+            for (int i = 0; i < COLS; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(v[i]));
             const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;  // scale > 0: max commutes with the scaling (-inf stays -inf)
             // lazy rescale: keep the stale max while the new one is < 2^8 above it (P <= 256: exact enough in bf16 / fp32;
             // the stale max cancels in O / l)
@@ -248,63 +260,90 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             const float m_new = grow ? mx : m_run;
             const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
             const float corr = grow ? exp2f(m_run - m_use) : 1.0f;  // m_run = -inf -> 0
-            if (t > 0 && __any_sync(0xffffffffu, corr != 1.0f)) {   // rescale the running output (in TMEM) once the previous P·V has landed
-                mbar_wait(o_done, (t - 1) & 1);
+            if (t >= WGS && __any_sync(0xffffffffu, corr != 1.0f)) {   // rescale the running output (in TMEM) once the previous P·V has landed
+                mbar_wait(&o_done[w], (t / WGS - 1) & 1);
                 tc_fence_after();
 #pragma unroll 1
                 for (int c = 0; c < D / 32; ++c) {
                     uint32_t o[32];
                     __syncwarp();
-                    tmem_ld_32x32(lanes + TM_O + c * 32, o);
+                    tmem_ld_32x32(tm_o + c * 32, o);
                     tmem_ld_wait();
 #pragma unroll
                     for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
-                    tmem_st_32x32(lanes + TM_O + c * 32, o);
+                    tmem_st_32x32(tm_o + c * 32, o);
                 }
             }
             l_run *= corr;
             m_run = m_new;
             float rs[4] = {0.f, 0.f, 0.f, 0.f};
-            uint32_t pk[32];
+            uint32_t pk[COLS / 2];
 #pragma unroll
-            for (int i = 0; i < 64; i += 2) {
-                const float p0 = ex2_approx(fmaf(__uint_as_float(v[i >> 5][i & 31]), p.scale_log2, -m_use));   // -inf -> +0
-                const float p1 = ex2_approx(fmaf(__uint_as_float(v[i >> 5][(i & 31) + 1]), p.scale_log2, -m_use));
+            for (int i = 0; i < COLS; i += 2) {
+                const float p0 = ex2_approx(fmaf(__uint_as_float(v[i]), p.scale_log2, -m_use));   // -inf -> +0
+                const float p1 = ex2_approx(fmaf(__uint_as_float(v[i + 1]), p.scale_log2, -m_use));
                 rs[(i >> 1) & 3] += p0 + p1;
                 pk[i >> 1] = pack_bf16(p0, p1);
             }
             l_run += (rs[0] + rs[1]) + (rs[2] + rs[3]);
             __syncwarp();
-            tmem_st_32x32(buf, pk);   // over the scores of this row
+            if constexpr (COLS == 64) tmem_st_32x32(buf, pk);   // over the scores of this row
+            else tmem_st_32x8(buf, pk);
             tmem_st_wait();
+        };
+        const bool idle = q0 + quad * 32 >= p.S;   // no query in this warp's rows: nothing of O is read there
+        for (int t = w; t < T; t += WGS) {
+            mbar_wait(&s_full[t % NBUF], (t / NBUF) & 1);
+            tc_fence_after();
+            if (!idle) {
+                if (stub && t + 1 == T) softmax(t, std::integral_constant<int, 16>());
+                else softmax(t, std::integral_constant<int, 64>());
+            }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&p_full[t & 1]);
+            if (lane == 0) mbar_arrive(&p_full[t % NBUF]);
         }
         // ---- epilogue: O / l (no key: no product to wait for, and nothing of O to read) ----
-        if (T > 0) mbar_wait(o_last, 0);
+        float corr[WGS];   // of each group's O, 1 / l included
+        if constexpr (WGS == 2) {
+            float2* ml = reinterpret_cast<float2*>(tmem_slot + 2);
+            ml[w * TC_BM + r] = make_float2(m_run, l_run);
+            __syncwarp();
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            const float2 a = ml[r], c = ml[TC_BM + r];
+            const float m = fmaxf(a.x, c.x);
+            corr[0] = a.x == -INFINITY ? 0.f : exp2f(a.x - m);
+            corr[1] = c.x == -INFINITY ? 0.f : exp2f(c.x - m);
+            const float l = a.y * corr[0] + c.y * corr[1], inv = l > 0.f ? 1.f / l : 0.f;
+            corr[0] *= inv;
+            corr[1] *= inv;
+        } else {
+            corr[0] = l_run > 0.f ? 1.f / l_run : 0.f;
+        }
+        for (int i = 0; i < WGS; ++i)
+            if (T > i) mbar_wait(&o_last[i], 0);
         tc_fence_after();
-        const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
         __nv_bfloat16* orow = p.o + b * p.o_bs + (int64_t)qrow * p.o_ts + head * p.o_hs;
 #pragma unroll
-        for (int c = 0; c < D / 32; ++c) {
+        for (int i = 0; i < D / 32 / WGS; ++i) {   // two groups: half of the columns each
+            const int c = w * (D / 32 / WGS) + i;
+            float x[32];
             uint32_t v[32];
             __syncwarp();
             tmem_ld_32x32(lanes + TM_O + c * 32, v);
             tmem_ld_wait();
-            if (T == 0) {
 #pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = 0u;
+            for (int j = 0; j < 32; ++j) x[j] = T == 0 ? 0.f : __uint_as_float(v[j]) * corr[0];
+            if (WGS == 2 && T > 1) {
+                tmem_ld_32x32(lanes + TM_O + D + c * 32, v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 32; ++j) x[j] = fmaf(__uint_as_float(v[j]), corr[WGS - 1], x[j]);
             }
             if (qrow < p.S) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    *reinterpret_cast<uint4*>(orow + c * 32 + i * 8) = make_uint4(
-                        pack_bf16(__uint_as_float(v[i * 8 + 0]) * inv, __uint_as_float(v[i * 8 + 1]) * inv),
-                        pack_bf16(__uint_as_float(v[i * 8 + 2]) * inv, __uint_as_float(v[i * 8 + 3]) * inv),
-                        pack_bf16(__uint_as_float(v[i * 8 + 4]) * inv, __uint_as_float(v[i * 8 + 5]) * inv),
-                        pack_bf16(__uint_as_float(v[i * 8 + 6]) * inv, __uint_as_float(v[i * 8 + 7]) * inv));
-                }
+                for (int j = 0; j < 32; j += 8)
+                    *reinterpret_cast<uint4*>(orow + c * 32 + j) = make_uint4(pack_bf16(x[j], x[j + 1]), pack_bf16(x[j + 2], x[j + 3]), pack_bf16(x[j + 4], x[j + 5]), pack_bf16(x[j + 6], x[j + 7]));
             }
         }
     }
@@ -355,7 +394,7 @@ int make_tmap_4d(CUtensorMap* map, const void* ptr, int D, int S, int H, int B, 
     return 0;
 }
 
-template <int D, bool CAUSAL>
+template <int D, bool CAUSAL, int WGS>
 int launch_tc(const FlashArgs& a, cudaStream_t stream) {
     CUtensorMap tq, tk, tv;
     B2_TRY(make_tmap_4d(&tq, a.q, D, a.S, a.H, a.B, a.q_ts, a.q_hs, a.q_bs));
@@ -367,11 +406,11 @@ int launch_tc(const FlashArgs& a, cudaStream_t stream) {
     p.o_bs = a.o_bs; p.o_ts = a.o_ts; p.o_hs = a.o_hs;
     p.S = a.S;
     p.scale_log2 = a.scale * 1.4426950408889634f;
-    constexpr int smem = TcCfg<D>::SMEM;
-    auto kern = flash_tc_kernel<D, CAUSAL>;
+    constexpr int smem = TcCfg<D, WGS>::SMEM;
+    auto kern = flash_tc_kernel<D, CAUSAL, WGS>;
     B2_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     dim3 grid(a.H, a.B, (a.S + TC_BM - 1) / TC_BM);
-    B2_CUDA_CHECK(launch_pdl(kern, grid, dim3(TC_THREADS), (size_t)smem, stream, tq, tk, tv, p));
+    B2_CUDA_CHECK(launch_pdl(kern, grid, dim3(64 + 128 * WGS), (size_t)smem, stream, tq, tk, tv, p));
     B2_LAUNCH_CHECK();
     return 0;
 }
@@ -382,8 +421,14 @@ int flash_attn_tc_bf16(const FlashArgs& a, cudaStream_t stream) {
     B2_CHECK_ARG(a.D == 64 || a.D == 128, "flash_attn(tc): head_dim must be 64 or 128 (got %d)", a.D);
     B2_CHECK_ARG((a.o_ts % 8) == 0 && (a.o_hs % 8) == 0 && (a.o_bs % 8) == 0 && (reinterpret_cast<uintptr_t>(a.o) & 15) == 0,
                  "flash_attn(tc): output must be 16B aligned with 16B-multiple strides");
-    if (a.D == 64) return a.causal ? launch_tc<64, true>(a, stream) : launch_tc<64, false>(a, stream);
-    return a.causal ? launch_tc<128, true>(a, stream) : launch_tc<128, false>(a, stream);
+    // at most one CTA an SM, and more than one tile of keys: two groups of softmax warps take the tiles in turn
+    const bool two = (long long)a.H * a.B * ((a.S + TC_BM - 1) / TC_BM) <= num_sms() && a.S > TC_BN;
+    if (a.D == 64) {
+        if (two) return a.causal ? launch_tc<64, true, 2>(a, stream) : launch_tc<64, false, 2>(a, stream);
+        return a.causal ? launch_tc<64, true, 1>(a, stream) : launch_tc<64, false, 1>(a, stream);
+    }
+    if (two) return a.causal ? launch_tc<128, true, 2>(a, stream) : launch_tc<128, false, 2>(a, stream);
+    return a.causal ? launch_tc<128, true, 1>(a, stream) : launch_tc<128, false, 1>(a, stream);
 }
 
 }  // namespace b2

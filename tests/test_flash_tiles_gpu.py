@@ -49,6 +49,33 @@ def test_tile_edges(S, D, causal, growing):
 
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("causal", [0, 1])
+@pytest.mark.parametrize("H", [3, 79])
+@pytest.mark.parametrize("S", [64, 80, 81, 208, 337, 400, 577])
+@pytest.mark.parametrize("growing", [False, True])
+def test_two_groups_and_one(S, H, D, causal, growing):
+    """Few and many CTAs (tiles in turn by two groups of warps, or one), last tiles of at most 16 keys and of one more, a last query tile with warps that have no row."""
+    from llava import _b2
+
+    lib, P = _b2.init(0), _b2.ptr
+    B = 2
+    g = torch.Generator(device="cuda").manual_seed(S + D + H)
+    q, k, v = (torch.randn(B, S, H, D, device="cuda", generator=g).bfloat16() for _ in range(3))
+    if growing:
+        q[..., 0] = 8.0
+        k[..., 0] = torch.arange(S, device="cuda").div(16, rounding_mode="floor").clamp(max=200).bfloat16()[None, :, None]
+    scale = 1 / math.sqrt(D)
+    for lens in (None, torch.tensor([S, max(1, S - 63)], dtype=torch.int32, device="cuda")):
+        o = torch.empty_like(q)
+        _b2.check(lib.b2_op_flash_attn(P(q), P(k), P(v), P(o), P(lens), B, S, H, D, causal, scale, _b2.stream_ptr()))
+        ref = attend(q, k, v, lens, causal, scale)
+        tol = 2 ** -8 * float(v.abs().max()) + 2 ** -8   # as above
+        for b in range(B):
+            n = S if lens is None or not causal else int(lens[b])
+            assert float((o[b, :n].double() - ref[b, :n]).abs().max()) <= tol
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [0, 1])
 def test_requests_without_keys(D, causal):
     """A length of 0 (or below) leaves its rows zeros and the other requests of the call as they are."""
     from llava import _b2
