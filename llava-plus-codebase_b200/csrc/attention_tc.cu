@@ -4,19 +4,21 @@
 // Replaces the eager attention of the reference's HF path, which materialises the [B,H,S,S] score matrix
 // (transformers modeling_llama.py:199-221 eager_attention_forward; modeling_clip.py:261-279).
 //
-// CTA = one (batch, head, 128-query tile), 192 threads, TWO CTAs per SM (256 TMEM columns each):
+// CTA = one (batch, head, 128-query tile), 192 threads, TWO CTAs per SM (256 TMEM columns each; two groups of softmax warps: 320, one, 512):
 //   warp 0 / lane 0 : TMA producer — Q once, then K_t / V_t tiles of 64 keys into rings (4-D tensor maps over the strided [b, t, h, d]
 //                     views: the same kernel reads the fused qkv activation buffer of the ViT and the [B, H, Smax, 128] KV cache
 //                     of the decoder)
 //   warp 1          : MMA issuer — S_t = Q K_t^T  (UMMA 128x64xD, both operands K-major, SWIZZLE_128B), into one of two TMEM buffers
 //                                  O += P_t V_t (UMMA 128xDx64; P from TMEM, V straight from its [keys, d] tile as an MN-major operand)
-//   warps 2..5      : softmax — thread r owns query row r: tcgen05.ld the S row, scale/mask, running max / sum, P = exp2(s - m) as bf16
+//   warps 2..5 (..9): softmax — thread r owns query row r: tcgen05.ld the S row, scale/mask, running max / sum, P = exp2(s - m) as bf16
 //                     back into TMEM over the score row it came from; O in TMEM is rescaled only when a row's max grew by more
 //                     than 2^8 (lazy rescale: P and l keep using the stale max, which cancels in O / l), finally O / l -> global.
 // S_(t+1) is there before softmax t ends, and S_(t+2) is issued when O_t has read P_t out of its buffer: the softmax warps never wait for a
 // product of their own tile. They are what bounds the kernel (at d = 64 the special-function unit alone needs 1024 clk for 128 x 128 exponentials,
 // the products 640). Before: tiles of 128 keys, one score buffer, P through shared memory, every tile a chain of product, softmax and product.
-// Measured, before -> now: [B, S, H, d] = [1, 577, 16, 64] 18.4 -> 11.9 us, [32, 577, 16, 64] 214 -> 106 us (204 -> 411 TFLOP/s),
+// A CTA alone on its SM is bound by the latency of a tile (1310 clk of which the exponentials' unit needs 512), so there two groups of four softmax warps
+// take the tiles in turn, each with buffers, an O, a maximum and a sum of its own, which meet in the epilogue (launch rule at the end).
+// Measured, before -> now: [B, S, H, d] = [1, 577, 16, 64] 18.4 -> 11.9 -> 8.9 us (two groups), [32, 577, 16, 64] 214 -> 104 us (204 -> 419 TFLOP/s),
 // causal [1, 704, 32, 128] 32.9 -> 15.0 us, [4, 2048, 32, 128] 441 -> 172 us (797 TFLOP/s of the 0.5 S^2 that is visible).
 #include <cuda.h>
 #include <math.h>
@@ -421,8 +423,9 @@ int flash_attn_tc_bf16(const FlashArgs& a, cudaStream_t stream) {
     B2_CHECK_ARG(a.D == 64 || a.D == 128, "flash_attn(tc): head_dim must be 64 or 128 (got %d)", a.D);
     B2_CHECK_ARG((a.o_ts % 8) == 0 && (a.o_hs % 8) == 0 && (a.o_bs % 8) == 0 && (reinterpret_cast<uintptr_t>(a.o) & 15) == 0,
                  "flash_attn(tc): output must be 16B aligned with 16B-multiple strides");
-    // at most one CTA an SM, and more than one tile of keys: two groups of softmax warps take the tiles in turn
-    const bool two = (long long)a.H * a.B * ((a.S + TC_BM - 1) / TC_BM) <= num_sms() && a.S > TC_BN;
+    // at most one CTA an SM, and three tiles of keys or more: two groups of softmax warps take the tiles in turn. One group / two, us: [1, 577, 16, 64]
+    // 12.0 / 8.9, [1, 1024, 16, 64] 17.8 / 12.7, causal [1, 300, 32, 64] 7.4 / 6.2 (two tiles: 4.7 / 4.4; two such CTAs do not fit an SM: [2, 577, 16, 64] 12.9 / 15.8).
+    const bool two = (long long)a.H * a.B * ((a.S + TC_BM - 1) / TC_BM) <= num_sms() && a.S > 2 * TC_BN;
     if (a.D == 64) {
         if (two) return a.causal ? launch_tc<64, true, 2>(a, stream) : launch_tc<64, false, 2>(a, stream);
         return a.causal ? launch_tc<64, true, 1>(a, stream) : launch_tc<64, false, 1>(a, stream);
