@@ -318,12 +318,26 @@ rope_kv_write_kernel(__nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict_
 }
 
 // ------------------------------------------------------------------------------------------------
-// decode attention: grid (nsplit, H, B), 128 threads. D = 128 fixed: a half-warp (16 lanes x 8 elems)
-// covers one K/V row with one 16-byte load per lane.
+// decode attention: grid (nsplit, H, B), 128 threads. D = 128 fixed: a half-warp (16 lanes x 8 elems) covers one K/V row.
+// The keys and values of a split lie in one piece each: a thread asks for them in bulk copies of 24 rows as soon as the length is known, into a ring
+// of two stages, and the rotation of q and of the new key runs while the first are on their way. What bounds it is HBM where contexts are long
+// (64 requests of 32 heads, 800 keys: 0.99 of the copy rate), and for short ones the chain of a CTA (length, copies, merge; 40 keys: 7.7 us against
+// 3.2 of bytes): seven CTAs an SM hide more of it than fewer with deeper rings. us, rows loaded to registers by every half-warp, four keys at
+// a time with an online softmax each -> now, at the split counts then and now: 8 x 32 heads, 800 keys 24.5 -> 23.1; 16, 110 12.0 -> 8.5;
+// 32, 110 18.3 -> 13.2; 32, 800 76.3 -> 68.3; 64, 800 139.5 -> 127.0; 128, 300 127.6 -> 96.6; 8 x 40, 2000 75.2 -> 55.2. Rings of 2 / 3 / 4
+// stages of 32 rows (6 / 4 / 3 CTAs): 14.6 / 15.9 / 17.4 at 32, 110 and 74 / 66 / 77 at 32, 800; 3 stages of 16 12.8 and 69.5.
 // ------------------------------------------------------------------------------------------------
 constexpr int DA_D = 128;
 constexpr int DA_THREADS = 128;
-constexpr int DA_UNROLL = 4;
+constexpr int DA_KEYS = 24, DA_U = DA_KEYS / 8;   // keys per stage and half-warp
+constexpr int DA_STAGES = 2, DA_CTAS = 7;         // per SM: registers and shared memory
+constexpr int DA_TILE = DA_KEYS * DA_D * 2;
+constexpr int DA_SMEM = DA_STAGES * 2 * DA_TILE + 128 /*align*/;
+
+__device__ __forceinline__ void da_bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
 
 struct DecodeAttnParams {
     const __nv_bfloat16* qkv;
@@ -337,32 +351,60 @@ struct DecodeAttnParams {
     float theta, scale_log2;
 };
 
-__global__ void __launch_bounds__(DA_THREADS) decode_attn_kernel(DecodeAttnParams p) {
+__global__ void __launch_bounds__(DA_THREADS, DA_CTAS) decode_attn_kernel(DecodeAttnParams p) {
     const int split = blockIdx.x, head = blockIdx.y, b = blockIdx.z;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int hw = (warp << 1) | (lane >> 4);  // half-warp id 0..7
     const int c = lane & 15;                   // 8-element chunk of the head dim
+    extern __shared__ uint8_t da_raw[];
+    uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(da_raw) + 127) & ~static_cast<uintptr_t>(127));
+    __shared__ __align__(8) uint64_t s_full[DA_STAGES], s_empty[DA_STAGES];
+    __shared__ float s_q[DA_D];
+    __shared__ float s_knew[DA_D];
+    __shared__ float s_m[8], s_l[8];
+    __shared__ float s_o[8][DA_D];
+    __shared__ int s_last;
+    if (tid == 0) {
+        for (int i = 0; i < DA_STAGES; ++i) {
+            mbar_init(&s_full[i], 1);
+            mbar_init(&s_empty[i], DA_THREADS / 32);
+        }
+        fence_barrier_init();
+    }
     pdl_trigger();
     pdl_wait();                                // qkv (previous GEMM) and cur_len (previous step) are upstream outputs
     const int pos = p.cur_len[b];              // position of the new token == number of cached keys
     const int total = pos + 1;
     const int hd = p.H * DA_D;
 
-    __shared__ float s_q[DA_D];
-    __shared__ float s_knew[DA_D];
-    __shared__ float s_m[8], s_l[8];
-    __shared__ float s_o[8][DA_D];
-    __shared__ int s_last;
+    // key range of this split (device-side: the launch grid is fixed so the step can live in a CUDA graph); the new token's row is not read back
+    const int chunk = (total + p.nsplit - 1) / p.nsplit;
+    const int k_begin = split * chunk;
+    const int k_end = min(k_begin + chunk, total);
+    const bool owns_new = (pos >= k_begin) && (pos < k_end);
+    const int n = max(min(k_end, pos) - k_begin, 0), tiles = (n + DA_KEYS - 1) / DA_KEYS;
+
+    const size_t cbase = ((size_t)b * p.H + head) * p.Smax * DA_D;
+    auto load = [&](int t) {
+        uint8_t* dst = ring + (t % DA_STAGES) * 2 * DA_TILE;
+        const uint32_t bytes = min(n - t * DA_KEYS, DA_KEYS) * DA_D * 2;
+        const size_t at = cbase + (size_t)(k_begin + t * DA_KEYS) * DA_D;
+        mbar_arrive_expect_tx(&s_full[t % DA_STAGES], 2 * bytes);
+        da_bulk_g2s(dst, p.kcache + at, bytes, &s_full[t % DA_STAGES]);
+        da_bulk_g2s(dst + DA_TILE, p.vcache + at, bytes, &s_full[t % DA_STAGES]);
+    };
+    if (tid == 0)
+        for (int t = 0; t < min(tiles, DA_STAGES); ++t) load(t);
 
     // ---- RoPE on q and the new k (every CTA: 128 threads, one element each) ----
     {
         const __nv_bfloat16* qrow = p.qkv + (size_t)b * 3 * hd + head * DA_D;
         const __nv_bfloat16* krow = qrow + hd;
         const int i = tid & 63;
-        float cs, sn;
-        rope_cos_sin(pos, i, DA_D, p.theta, cs, sn);
         const float q1 = __bfloat162float(qrow[i]), q2 = __bfloat162float(qrow[i + 64]);
         const float k1 = __bfloat162float(krow[i]), k2 = __bfloat162float(krow[i + 64]);
+        float cs, sn;
+        rope_cos_sin(pos, i, DA_D, p.theta, cs, sn);
         if (tid < 64) {
             s_q[i] = rope_apply(q1, -q2, cs, sn);
             s_knew[i] = rope_apply(k1, -k2, cs, sn);
@@ -373,13 +415,6 @@ __global__ void __launch_bounds__(DA_THREADS) decode_attn_kernel(DecodeAttnParam
     }
     __syncthreads();
 
-    // key range of this split (device-side: the launch grid is fixed so the step can live in a CUDA graph)
-    const int chunk = (total + p.nsplit - 1) / p.nsplit;
-    const int k_begin = split * chunk;
-    const int k_end = min(k_begin + chunk, total);
-    const bool owns_new = (pos >= k_begin) && (pos < k_end);
-
-    const size_t cbase = ((size_t)b * p.H + head) * p.Smax * DA_D;
     if (owns_new) {
         // append the new token's k (roped) and v to the cache; exactly one CTA per (b, head) does this
         const __nv_bfloat16* vrow = p.qkv + (size_t)b * 3 * hd + 2 * hd + head * DA_D;
@@ -396,64 +431,79 @@ __global__ void __launch_bounds__(DA_THREADS) decode_attn_kernel(DecodeAttnParam
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[e] = 0.f;
 
-    const __nv_bfloat16* kb = p.kcache + cbase + c * 8;
-    const __nv_bfloat16* vb = p.vcache + cbase + c * 8;
-    const __nv_bfloat16* vnew = p.qkv + (size_t)b * 3 * hd + 2 * hd + head * DA_D + c * 8;
-
-    // each half-warp walks keys k_begin + hw, +8, ...; DA_UNROLL keys (2*DA_UNROLL 16B loads) in flight
+    // each half-warp takes keys hw, hw + 8, hw + 16 of a stage: their scores, one maximum and one correction of what it holds
     // (trip count is CTA-uniform: the shuffles below use the full warp mask)
-    for (int kbase = k_begin; kbase < k_end; kbase += 8 * DA_UNROLL) {
-        const int k0 = kbase + hw;
-        uint4 kraw[DA_UNROLL], vraw[DA_UNROLL];
+#pragma unroll 1
+    for (int t = 0; t < tiles; ++t) {
+        const int st = t % DA_STAGES, left = n - t * DA_KEYS;
+        const uint4* kt = reinterpret_cast<const uint4*>(ring + st * 2 * DA_TILE) + hw * 16 + c;
+        const uint4* vt = kt + DA_TILE / 16;
+        mbar_wait(&s_full[st], (t / DA_STAGES) & 1);
+        float sc[DA_U];
 #pragma unroll
-        for (int u = 0; u < DA_UNROLL; ++u) {
-            const int key = k0 + u * 8;
-            if (key < k_end && key != pos) {
-                kraw[u] = ld_stream_16(kb + (size_t)key * DA_D);
-                vraw[u] = ld_stream_16(vb + (size_t)key * DA_D);
-            } else {
-                kraw[u] = make_uint4(0, 0, 0, 0);
-                vraw[u] = make_uint4(0, 0, 0, 0);
-            }
+        for (int u = 0; u < DA_U; ++u) {
+            const uint4 k = hw + u * 8 < left ? kt[u * 128] : make_uint4(0, 0, 0, 0);
+            float d0 = qreg[0] * bf16_lo(k.x);
+            d0 = fmaf(qreg[1], bf16_hi(k.x), d0); d0 = fmaf(qreg[2], bf16_lo(k.y), d0); d0 = fmaf(qreg[3], bf16_hi(k.y), d0);
+            d0 = fmaf(qreg[4], bf16_lo(k.z), d0); d0 = fmaf(qreg[5], bf16_hi(k.z), d0); d0 = fmaf(qreg[6], bf16_lo(k.w), d0);
+            sc[u] = fmaf(qreg[7], bf16_hi(k.w), d0);
         }
+        // reduce over the 16 lanes of the half-warp (xor 8,4,2,1 stays inside the half)
 #pragma unroll
-        for (int u = 0; u < DA_UNROLL; ++u) {
-            const int key = k0 + u * 8;
-            const bool valid = key < k_end;  // uniform across the half-warp
-            float kf[8], vf[8];
-            if (key == pos) {
-                // the new token: k from smem (already roped, bf16-rounded), v straight from qkv
+        for (int o = 8; o > 0; o >>= 1)
 #pragma unroll
-                for (int e = 0; e < 8; ++e) kf[e] = round_bf16(s_knew[c * 8 + e]);
-                const uint4 vv = *reinterpret_cast<const uint4*>(vnew);
-                vf[0] = bf16_lo(vv.x); vf[1] = bf16_hi(vv.x); vf[2] = bf16_lo(vv.y); vf[3] = bf16_hi(vv.y);
-                vf[4] = bf16_lo(vv.z); vf[5] = bf16_hi(vv.z); vf[6] = bf16_lo(vv.w); vf[7] = bf16_hi(vv.w);
-            } else {
-                kf[0] = bf16_lo(kraw[u].x); kf[1] = bf16_hi(kraw[u].x); kf[2] = bf16_lo(kraw[u].y);
-                kf[3] = bf16_hi(kraw[u].y); kf[4] = bf16_lo(kraw[u].z); kf[5] = bf16_hi(kraw[u].z);
-                kf[6] = bf16_lo(kraw[u].w); kf[7] = bf16_hi(kraw[u].w);
-                vf[0] = bf16_lo(vraw[u].x); vf[1] = bf16_hi(vraw[u].x); vf[2] = bf16_lo(vraw[u].y);
-                vf[3] = bf16_hi(vraw[u].y); vf[4] = bf16_lo(vraw[u].z); vf[5] = bf16_hi(vraw[u].z);
-                vf[6] = bf16_lo(vraw[u].w); vf[7] = bf16_hi(vraw[u].w);
+            for (int u = 0; u < DA_U; ++u) sc[u] += __shfl_xor_sync(0xffffffffu, sc[u], o);
+        if (hw < left) {
+            float m_new = m_run;
+#pragma unroll
+            for (int u = 0; u < DA_U; ++u) {
+                sc[u] = hw + u * 8 < left ? sc[u] * p.scale_log2 : -INFINITY;
+                m_new = fmaxf(m_new, sc[u]);
             }
-            float dot = 0.f;
+            const float m_use = m_new == -INFINITY ? 0.f : m_new;
+            const float corr = exp2f(m_run - m_use);
+            l_run *= corr;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) dot += qreg[e] * kf[e];
-            // reduce over the 16 lanes of the half-warp (xor 8,4,2,1 stays inside the half)
-            dot += __shfl_xor_sync(0xffffffffu, dot, 8);
-            dot += __shfl_xor_sync(0xffffffffu, dot, 4);
-            dot += __shfl_xor_sync(0xffffffffu, dot, 2);
-            dot += __shfl_xor_sync(0xffffffffu, dot, 1);
-            if (valid) {
-                const float sc = dot * p.scale_log2;
-                const float m_new = fmaxf(m_run, sc);
-                const float corr = exp2f(m_run - m_new);
-                const float pr = exp2f(sc - m_new);
-                l_run = l_run * corr + pr;
+            for (int e = 0; e < 8; ++e) acc[e] *= corr;
 #pragma unroll
-                for (int e = 0; e < 8; ++e) acc[e] = acc[e] * corr + pr * vf[e];
-                m_run = m_new;
+            for (int u = 0; u < DA_U; ++u)
+                if (hw + u * 8 < left) {
+                    const uint4 v = vt[u * 128];
+                    const float pr = exp2f(sc[u] - m_use);
+                    l_run += pr;
+                    acc[0] = fmaf(pr, bf16_lo(v.x), acc[0]); acc[1] = fmaf(pr, bf16_hi(v.x), acc[1]);
+                    acc[2] = fmaf(pr, bf16_lo(v.y), acc[2]); acc[3] = fmaf(pr, bf16_hi(v.y), acc[3]);
+                    acc[4] = fmaf(pr, bf16_lo(v.z), acc[4]); acc[5] = fmaf(pr, bf16_hi(v.z), acc[5]);
+                    acc[6] = fmaf(pr, bf16_lo(v.w), acc[6]); acc[7] = fmaf(pr, bf16_hi(v.w), acc[7]);
+                }
+            m_run = m_new;
+        }
+        if (t + DA_STAGES < tiles) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_empty[st]);
+            if (tid == 0) {
+                mbar_wait(&s_empty[st], (t / DA_STAGES) & 1);
+                load(t + DA_STAGES);
             }
+            __syncwarp();
+        }
+    }
+    if (owns_new) {   // the new token: k from smem (roped, bf16-rounded), v straight from qkv; the first half-warp counts it
+        const uint4 v = *reinterpret_cast<const uint4*>(p.qkv + (size_t)b * 3 * hd + 2 * hd + head * DA_D + c * 8);
+        float sc = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sc = fmaf(qreg[e], round_bf16(s_knew[c * 8 + e]), sc);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) sc += __shfl_xor_sync(0xffffffffu, sc, o);
+        if (hw == 0) {
+            sc *= p.scale_log2;
+            const float m_new = fmaxf(m_run, sc), m_use = m_new == -INFINITY ? 0.f : m_new;
+            const float corr = exp2f(m_run - m_use), pr = exp2f(sc - m_use);
+            const float vf[8] = {bf16_lo(v.x), bf16_hi(v.x), bf16_lo(v.y), bf16_hi(v.y), bf16_lo(v.z), bf16_hi(v.z), bf16_lo(v.w), bf16_hi(v.w)};
+            l_run = l_run * corr + pr;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[e] = acc[e] * corr + pr * vf[e];
+            m_run = m_new;
         }
     }
 
@@ -473,6 +523,10 @@ __global__ void __launch_bounds__(DA_THREADS) decode_attn_kernel(DecodeAttnParam
         o_cta += s_o[i][tid] * w;
     }
     const int bh = b * p.H + head;
+    if (p.nsplit == 1) {
+        p.out[(size_t)b * hd + head * DA_D + tid] = __float2bfloat16_rn(o_cta / l_cta);
+        return;
+    }
     float* part = p.partial + ((size_t)bh * p.nsplit + split) * (DA_D + 2);
     part[tid] = o_cta;
     if (tid == 0) { part[DA_D] = m_cta; part[DA_D + 1] = l_cta; }
@@ -566,12 +620,13 @@ int rope_kv_write(void* qkv, void* kcache, void* vcache, int B, int S, int H, in
     return 0;
 }
 
-// resident CTAs of decode_attn_kernel per SM (register-limited: 79 registers x 128 threads -> 6), for the split heuristic
+// resident CTAs of decode_attn_kernel per SM, for the split heuristic
 int decode_attn_ctas_per_sm() {
     static int occ = 0;
     if (occ == 0) {
         int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, decode_attn_kernel, DA_THREADS, 0) != cudaSuccess || n < 1) n = 6;
+        if (cudaFuncSetAttribute(decode_attn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DA_SMEM) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, decode_attn_kernel, DA_THREADS, DA_SMEM) != cudaSuccess || n < 1) n = DA_CTAS;
         occ = n;
     }
     return occ;
@@ -592,7 +647,8 @@ int decode_attn_bf16(const DecodeAttnArgs& a, cudaStream_t stream) {
     p.theta = a.theta;
     p.scale_log2 = a.scale * 1.4426950408889634f;
     dim3 grid(a.nsplit, a.H, a.B);
-    B2_CUDA_CHECK(launch_pdl(decode_attn_kernel, grid, dim3(DA_THREADS), 0, stream, p));
+    B2_CUDA_CHECK(cudaFuncSetAttribute(decode_attn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DA_SMEM));
+    B2_CUDA_CHECK(launch_pdl(decode_attn_kernel, grid, dim3(DA_THREADS), DA_SMEM, stream, p));
     B2_LAUNCH_CHECK();
     return 0;
 }

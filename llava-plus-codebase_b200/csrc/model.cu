@@ -164,20 +164,16 @@ bool use_skinny(const b2_kv* kv, int B) {
 }
 
 int decode_nsplit(int B, int H, int max_seq) {
-    // Split-KV factor of the multi-kernel decode step. The kernel is register-limited to `occ` resident CTAs per SM (6), so
-    // one wave is occ*SMs = 888 CTAs. Measured over the ladder (profiles/r2j_*, r2k_decode_ab_nsplit_stages.jsonl, 7B, ctx ~800):
-    // B=8 (256 pairs): n=3 4.19 ms vs n=5 4.32 / n=10 4.38; B=16: n=3 4.80 vs n=1 5.05 / n=5 4.90; B=32: n=3 6.50 vs n=2 6.55 /
-    // n=6 6.68; B=64: n=1..3 equal. Few pairs: fill one wave; otherwise 3 splits (short enough ranges for the tail wave to
-    // overlap, few enough partials for the merge to stay cheap).
+    // Split-KV factor of the multi-kernel decode step: as many splits as fill one wave of resident CTAs (seven an SM, 1036), with room for at least 128 keys
+    // each: a split's partial sums and the merge cost 2 us or more. us with 1 / 2 / 3 / 4 / 8 splits: 2 requests of 32 heads, 100 keys 5.5 / 7.1 / 7.2 / 7.5; 4, 800
+    // 24.3 / 18.5 / 18.9 / 16.2 / 14.3; 8, 800 31.0 / 23.2 / 23.3 / 23.1 / 23.8; 16, 800 37.4 / 37.3 / 40.1 / 39.4; 32, 110 13.2 / 17.4 / 18.2 / 21.4; 64, 800 127 / 129 / 130.
     const char* e = getenv("B2_DECODE_NSPLIT");
     if (e != nullptr && atoi(e) >= 1) return atoi(e) > 32 ? 32 : atoi(e);
     const int cap = decode_attn_ctas_per_sm() * num_sms();
     int n = cap / (B * H);
-    if (n < 3) n = 3;
     if (n > 16) n = 16;
-    const int n_hi = max_seq / 64;  // keep >= 64 keys per split at the cache's capacity
-    if (n > n_hi) n = n_hi < 1 ? 1 : n_hi;
-    return n;
+    if (n > max_seq / 128) n = max_seq / 128;
+    return n < 1 ? 1 : n;
 }
 
 // ------------------------------------------------------------------------------------------------------
