@@ -44,7 +44,7 @@ __device__ __forceinline__ float warp_max(float v) {
 
 // the last write of one output entry: its own sigmoid gate, when there is one, and the form the output is wanted in
 __device__ __forceinline__ void store_out(const BiasAttnArgs& a, int row, int head, int d, float v) {
-    if (a.chan_gate != nullptr) v /= 1.f + expf(-a.chan_gate[(size_t)row * a.ldg + (size_t)head * a.dv + d]);
+    if (a.chan_gate != nullptr) v /= 1.f + expf(-a.chan_gate[(size_t)row * a.ldg + (a.chan_step ? (size_t)head * a.dv + d : head)]);
     const size_t at = (size_t)row * a.ldo + (size_t)head * a.dv + d;
     if (a.out16 != nullptr) reinterpret_cast<__nv_bfloat16*>(a.out16)[at] = __float2bfloat16_rn(v);
     else a.out[at] = v;

@@ -161,7 +161,7 @@ __device__ __noinline__ void attn_plain(const SplitParams& p, int row, int head,
         inv = c0 / fmaf(l, c0, expf(sk - mf));
     }
     if (a.head_gate != nullptr) inv /= 1.f + expf(-a.head_gate[(size_t)row * a.ldg + head]);
-    const float* cg = a.chan_gate != nullptr ? a.chan_gate + (size_t)row * a.ldg + (size_t)head * a.dv : nullptr;
+    const float* cg = a.chan_gate != nullptr ? a.chan_gate + (size_t)row * a.ldg + (size_t)head * (a.chan_step ? a.dv : 1) : nullptr;
     const size_t at = (size_t)row * a.ldo + (size_t)head * a.dv;
     for (int d = d0; d < d1; d += 16) {
         float o[16];
@@ -182,14 +182,14 @@ __device__ __noinline__ void attn_plain(const SplitParams& p, int row, int head,
         for (int c = 0; c < 16; ++c) {
             if (d + c >= d1) continue;
             float y = o[c] * inv;
-            if (cg != nullptr) y = sigmoid_times(cg[d + c], y);
+            if (cg != nullptr) y = sigmoid_times(cg[(d + c) * a.chan_step], y);
             if (a.out16 != nullptr) reinterpret_cast<__nv_bfloat16*>(a.out16)[at + d + c] = __float2bfloat16_rn(y);
             else a.out[at + d + c] = y;
         }
     }
 }
 
-template <int DKS, int DVS, int KT, bool EXTRA, int SOFT>   // EXTRA: soft-cap or distance bias; SOFT: softmax warps, 8 or 16
+template <int DKS, int DVS, int KT, bool EXTRA, int SOFT, bool ONE = false>   // EXTRA: soft-cap or distance bias; SOFT: softmax warps, 8 or 16; ONE: one channel gate a head
 __global__ void __launch_bounds__(64 + 32 * SOFT, 1) attn_split_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                                                                    const __grid_constant__ SplitParams p) {
     using Cfg = SplitCfg<DKS, DVS, KT>;
@@ -445,7 +445,12 @@ __global__ void __launch_bounds__(64 + 32 * SOFT, 1) attn_split_kernel(const __g
             }
             if (a.head_gate != nullptr) inv /= 1.f + expf(-a.head_gate[(size_t)row * a.ldg + head]);
             const int d0 = share * CQ;
-            const float* cg = a.chan_gate != nullptr ? a.chan_gate + (size_t)row * a.ldg + (size_t)head * a.dv : nullptr;
+            const float* cg = a.chan_gate != nullptr ? a.chan_gate + (size_t)row * a.ldg + (size_t)head * (a.chan_step ? a.dv : 1) : nullptr;
+            if constexpr (ONE) {
+                const float den = 1.f + expf(-cg[0]);
+#pragma unroll
+                for (int c = 0; c < CQ; ++c) o[c] = o[c] * inv / den;
+            }
             const size_t at = (size_t)row * a.ldo + (size_t)head * a.dv;
             const bool vec = a.dv % 4 == 0 && a.ldo % 4 == 0 &&
                              (a.out16 != nullptr ? (reinterpret_cast<uintptr_t>(a.out16) & 7) == 0 : (reinterpret_cast<uintptr_t>(a.out) & 15) == 0);
@@ -455,8 +460,8 @@ __global__ void __launch_bounds__(64 + 32 * SOFT, 1) attn_split_kernel(const __g
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int d = d0 + c + i;
-                    y[i] = o[c + i] * inv;
-                    if (cg != nullptr && d < a.dv) y[i] = sigmoid_times(cg[d], y[i]);
+                    y[i] = ONE ? o[c + i] : o[c + i] * inv;
+                    if (!ONE && cg != nullptr && d < a.dv) y[i] = sigmoid_times(cg[d], y[i]);
                 }
                 if (vec && d0 + c + 4 <= a.dv) {
                     if (a.out16 != nullptr) *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(a.out16) + at + d0 + c) = make_uint2(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]));
@@ -488,7 +493,10 @@ int launch_split(const SplitParams& p, const SplitSrc& k, const SplitSrc& v, int
     // there on two, whose exchanges are fewer (260 rows 241.0 / 240.2, 1000 rows 324.8 / 321.0, 2048 rows 336 / 332). 18 warps leave a thread 96 registers:
     // with value heads of 128 the four-thread form spills (208 / 148 bytes stored / loaded at <2, 2, 64, true, 16>, 132 / 140 without cap and bias).
     const bool extra = p.a.softcap > 0.f || p.a.rel != nullptr, wide = extra || nkeys <= FEW_KEYS;
-    auto kernel = extra ? attn_split_kernel<DKS, DVS, KT, true, 16> : wide ? attn_split_kernel<DKS, DVS, KT, false, 16> : attn_split_kernel<DKS, DVS, KT, false, 8>;
+    const bool one = p.a.chan_gate != nullptr && p.a.chan_step == 0;   // (a kernel of its own: in the others its divisions cost 1 % of a layer without them)
+    auto kernel = extra ? (one ? attn_split_kernel<DKS, DVS, KT, true, 16, true> : attn_split_kernel<DKS, DVS, KT, true, 16>)
+                  : wide ? (one ? attn_split_kernel<DKS, DVS, KT, false, 16, true> : attn_split_kernel<DKS, DVS, KT, false, 16>)
+                         : (one ? attn_split_kernel<DKS, DVS, KT, false, 8, true> : attn_split_kernel<DKS, DVS, KT, false, 8>);
     B2_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));
     launch_pdl(kernel, dim3(((p.a.rows + p.QT - 1) / p.QT) * p.a.G), dim3(64 + 32 * (wide ? 16 : 8)), Cfg::SMEM, st, tk, tv, p);
     B2_LAUNCH_CHECK();

@@ -632,6 +632,7 @@ struct BiasAttnArgs {
                                                   // (the maps of differential attention: G = maps * Gv key heads over one set of values)
     const float* head_gate = nullptr; int64_t ldg = 0;   // non-null ([rows, ldg], entry h): a head's output is multiplied by sigmoid(head_gate[r, h])
     const float* chan_gate = nullptr;             // non-null ([rows, ldg], entry h * dv + d): every entry of the output has a sigmoid gate of its own
+    int chan_step = 1;                            // 0: entry h for all of a head's outputs, each divided by itself (head_gate goes into the weights' common factor: other roundings)
     void* out16 = nullptr;                        // non-null: the output is written as bf16 (pitch ldo) instead of fp32: the operand of a product
     float* partial = nullptr; int nsplit = 1;     // split-KV scratch [rows*H*nsplit*(dv+2)] when nsplit > 1
     int tile_rows = 0;                            // consecutive rows that share a slot (a prompt portion: its rows; a decode step: 1);

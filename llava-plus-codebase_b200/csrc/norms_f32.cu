@@ -310,7 +310,8 @@ __global__ void rms_scalar_kernel(float* __restrict__ x, const int32_t* __restri
     const float mul = g[0] / sqrtf(block_sum(q, red) / (float)cols + eps);
     for (int c = threadIdx.x; c < cols; c += blockDim.x) out[r * cols + c] = xr[c] * mul;
 }
-// a row of up to V * blockDim * 4 entries in registers: one pass over it
+// a row of up to V * blockDim entries in registers: one pass over it, and the sum of squares in the order of the kernel above (columns t, t + blockDim, ... of a
+// thread: experts are chosen from what these rows give, and a near tie falls as it did)
 template <int V>
 __global__ void __launch_bounds__(256) rms_scalar_reg_kernel(float* __restrict__ x, const int32_t* __restrict__ row_index, const float* __restrict__ g, const float* __restrict__ add,
                                                              const float* __restrict__ vec, float* __restrict__ out, int cols, float eps, __nv_bfloat16* __restrict__ out16) {
@@ -318,35 +319,32 @@ __global__ void __launch_bounds__(256) rms_scalar_reg_kernel(float* __restrict__
     __shared__ float red[33];
     const size_t r = blockIdx.x, src = row_index != nullptr ? (size_t)row_index[r] : r;
     float* xr = x + src * cols;
-    float4 v[V];
-    float q = 0.f;
+    float v[V], q = 0.f;
 #pragma unroll
     for (int u = 0; u < V; ++u) {
-        const int c = (threadIdx.x + u * blockDim.x) * 4;
-        v[u] = c < cols ? *reinterpret_cast<const float4*>(xr + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const int c = threadIdx.x + u * blockDim.x;
+        v[u] = c < cols ? xr[c] : 0.f;
     }
     if (add != nullptr || vec != nullptr) {
 #pragma unroll
         for (int u = 0; u < V; ++u) {
-            const int c = (threadIdx.x + u * blockDim.x) * 4;
+            const int c = threadIdx.x + u * blockDim.x;
             if (c >= cols) continue;
-            const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-            const float4 p = add != nullptr ? *reinterpret_cast<const float4*>(add + src * cols + c) : zero, w = vec != nullptr ? *reinterpret_cast<const float4*>(vec + c) : zero;
-            v[u].x += p.x + w.x; v[u].y += p.y + w.y; v[u].z += p.z + w.z; v[u].w += p.w + w.w;
-            *reinterpret_cast<float4*>(xr + c) = v[u];
+            v[u] += (add != nullptr ? add[src * cols + c] : 0.f) + (vec != nullptr ? vec[c] : 0.f);
+            xr[c] = v[u];
         }
     }
     if (out == nullptr) return;   // only the update of x was asked for
 #pragma unroll
-    for (int u = 0; u < V; ++u) { q = fmaf(v[u].x, v[u].x, q); q = fmaf(v[u].y, v[u].y, q); q = fmaf(v[u].z, v[u].z, q); q = fmaf(v[u].w, v[u].w, q); }
+    for (int u = 0; u < V; ++u) q = fmaf(v[u], v[u], q);
     const float mul = g[0] / sqrtf(block_sum(q, red) / (float)cols + eps);
 #pragma unroll
     for (int u = 0; u < V; ++u) {
-        const int c = (threadIdx.x + u * blockDim.x) * 4;
+        const int c = threadIdx.x + u * blockDim.x;
         if (c >= cols) continue;
-        const float4 y = make_float4(v[u].x * mul, v[u].y * mul, v[u].z * mul, v[u].w * mul);
-        *reinterpret_cast<float4*>(out + r * cols + c) = y;
-        if (out16 != nullptr) *reinterpret_cast<uint2*>(out16 + r * cols + c) = make_uint2(pack_bf16(y.x, y.y), pack_bf16(y.z, y.w));
+        const float y = v[u] * mul;
+        out[r * cols + c] = y;
+        if (out16 != nullptr) out16[r * cols + c] = __float2bfloat16_rn(y);
     }
 }
 
@@ -823,16 +821,16 @@ int sigmoid_gate_f32(const float* a, int64_t lda, const float* g, int64_t ldg, f
 int rms_scalar_f32(float* x, const int32_t* row_index, const float* g, const float* add, const float* vec, float* out, int rows, int cols,
                    float eps, cudaStream_t st, void* out16) {
     B2_CHECK_ARG(x && rows > 0 && cols > 0 && ((g && out) || (!out && (add || vec))), "rms_scalar: bad argument");
-    const uintptr_t align = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(add) | reinterpret_cast<uintptr_t>(vec) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out16);
-    if (cols % 4 == 0 && (align & 15) == 0 && cols <= 8192) {   // 1536 rows of 2048: 9.5 us, and 6.7 for a cast; now 5.6 with the bf16 rows
+    if (cols <= 8192) {   // 1536 rows of 2048: 9.5 us, and 6.7 for a cast; now 6.2 with the bf16 rows
         __nv_bfloat16* o16 = reinterpret_cast<__nv_bfloat16*>(out16);
-        if (cols <= 512) launch_pdl(rms_scalar_reg_kernel<1>, dim3(rows), dim3(128), 0, st, x, row_index, g, add, vec, out, cols, eps, o16);
-        else if (cols <= 2048) launch_pdl(rms_scalar_reg_kernel<2>, dim3(rows), dim3(256), 0, st, x, row_index, g, add, vec, out, cols, eps, o16);
-        else launch_pdl(rms_scalar_reg_kernel<8>, dim3(rows), dim3(256), 0, st, x, row_index, g, add, vec, out, cols, eps, o16);
+        const dim3 threads(cols >= 1024 ? 256 : 128);
+        if (cols <= 2048) launch_pdl(rms_scalar_reg_kernel<8>, dim3(rows), threads, 0, st, x, row_index, g, add, vec, out, cols, eps, o16);
+        else if (cols <= 4096) launch_pdl(rms_scalar_reg_kernel<16>, dim3(rows), threads, 0, st, x, row_index, g, add, vec, out, cols, eps, o16);
+        else launch_pdl(rms_scalar_reg_kernel<32>, dim3(rows), threads, 0, st, x, row_index, g, add, vec, out, cols, eps, o16);
         B2_LAUNCH_CHECK();
         return 0;
     }
-    B2_CHECK_ARG(out16 == nullptr, "rms_scalar: bf16 rows in whole fours on 16 bytes");
+    B2_CHECK_ARG(out16 == nullptr, "rms_scalar: bf16 rows of at most 8192 columns");
     launch_pdl(rms_scalar_kernel, dim3(rows), dim3(cols >= 1024 ? 256 : 128), 0, st, x, row_index, g, add, vec, out, cols, eps);
     B2_LAUNCH_CHECK();
     return 0;

@@ -390,7 +390,7 @@ static int latent_mixer(b2_model* m, b2_kv* kv, const SeqLayerInfo& L, SeqWeight
         }
         // the heads' sigmoid gates ride in the attention's last write, and the output leaves as the bf16 operand of W_o where that product reads those (19 us
         // of gating and casting before, 1536 rows of 16 heads of 128)
-        if (gate) { ah.head_gate = gates; ah.ldg = L.pproj_ld; }
+        if (gate) { ah.chan_gate = gates; ah.chan_step = 0; ah.ldg = L.pproj_ld; }   // (each output divided, as by a pass of its own: experts are chosen behind this layer, and near ties fall as they did)
         const void* o16 = lin.tensor_cores(width, L.pv, target, width, R) ? s.a16.p : nullptr;
         if (o16 != nullptr) ah.out16 = s.a16.p;
         B2_TRY(attn_bias_f32(ah, st));
