@@ -290,7 +290,11 @@ struct RowMap {
     int32_t* row_pos = nullptr;   // device [rows]; -1 = idle row
 };
 // one segment: rows [0, n) of slot `slot`; its start position is read on the device from len[slot] (and len[slot] += n)
-int rowmap_portion(const RowMap& rm, int32_t* len, int slot, int n, int restart, cudaStream_t stream);
+// (want[i] = want_host[i], i < n_want, rides along: up to 128 of them as kernel parameters, a copy of their own was 4.6 us behind the last layer)
+int rowmap_portion(const RowMap& rm, int32_t* len, int slot, int n, int restart, int32_t* want, const int32_t* want_host, int n_want, cudaStream_t stream);
+// dst = src, as a kernel that starts and ends like its neighbours (cudaMemcpyAsync of 41 rows of 2048 between two layers: 3.7 us and the next kernel's start in full
+// behind it); n a multiple of 4, both 16-byte aligned
+int copy_f32(float* dst, const float* src, size_t n, cudaStream_t stream);
 // B segments of one row each for slots slot0 .. slot0+B-1 at positions len[slot]; with sstate->per_row set, slots whose
 // rows_state entry is not active become idle rows
 struct DecodeRows { RowMap rm; const int32_t* len = nullptr; const SampleState* sstate = nullptr; const RowState* rows_state = nullptr; int slot0 = 0; };

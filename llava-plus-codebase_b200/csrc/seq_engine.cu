@@ -976,6 +976,17 @@ static int seq_feed_forward(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, c
     return moe_combine_f32(target, s.moe_y.as<float>(), width, pos, s.moe_w.as<float>(), R, top, width, alpha, st, h, width);
 }
 
+// the residual stream behind a layer run: by a kernel where the caller's buffer is memory of this device that it can write in 16-byte pieces
+static int keep_residual(float* dst, const float* x, size_t n, cudaStream_t st) {
+    cudaPointerAttributes attr;
+    int dev = -1;
+    const bool here = n % 4 == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0 && cudaGetDevice(&dev) == cudaSuccess &&
+                      cudaPointerGetAttributes(&attr, dst) == cudaSuccess && attr.type == cudaMemoryTypeDevice && attr.device == dev;
+    if (here) return copy_f32(dst, x, n, st);
+    cudaGetLastError();
+    B2_CUDA_CHECK(cudaMemcpyAsync(dst, x, n * F4, cudaMemcpyDeviceToDevice, st));
+    return 0;
+}
 // ------------------------------------------------------------------------------------------------------------------
 // forward over R rows described by the model's row map (nseg segments). x holds the embedded rows on entry.
 // ------------------------------------------------------------------------------------------------------------------
@@ -1049,7 +1060,7 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
                 if (early) B2_TRY(gelu_down(m, L, W, x, rm, 1, R, st));
                 else if (d.ff > 0 && ride == nullptr) B2_TRY(seq_feed_forward(m, L, W, in2, x, rm, 1, R, st));
                 if (resid_out != nullptr)
-                    B2_CUDA_CHECK(cudaMemcpyAsync(resid_out + ri * (size_t)R * width, x, (size_t)R * width * F4, cudaMemcpyDeviceToDevice, st));
+                    B2_TRY(keep_residual(resid_out + ri * (size_t)R * width, x, (size_t)R * width, st));
                 continue;
             }
             // (the normed rows of a prompt leave rounded as well: what the products, and the experts' gather, read)
@@ -1085,7 +1096,7 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
                 post = nullptr;
             }
             if (resid_out != nullptr)
-                B2_CUDA_CHECK(cudaMemcpyAsync(resid_out + ri * (size_t)R * width, x, (size_t)R * width * F4, cudaMemcpyDeviceToDevice, st));
+                B2_TRY(keep_residual(resid_out + ri * (size_t)R * width, x, (size_t)R * width, st));
             continue;
         }
         if (pass >= 0) B2_TRY(rms_scalar_f32(x, nullptr, nullptr, pass_add, pass_vec, nullptr, R, width, eps, st));
@@ -1171,7 +1182,7 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
             B2_TRY(layernorm_add_f32(x, mix, W.norm2.as<float>(), W.norm2_b.as<float>(), R, width, eps, st));
         }
         if (resid_out != nullptr)
-            B2_CUDA_CHECK(cudaMemcpyAsync(resid_out + ri * (size_t)R * width, x, (size_t)R * width * F4, cudaMemcpyDeviceToDevice, st));
+            B2_TRY(keep_residual(resid_out + ri * (size_t)R * width, x, (size_t)R * width, st));
     }
     return 0;
 }
@@ -2250,11 +2261,10 @@ int b2_append_tokens(b2_model* m, b2_kv* kv, int slot, const int32_t* tokens_hos
     B2_CUDA_CHECK(cudaMemcpyAsync(s.tok.p, tokens_host, (size_t)n * 4, cudaMemcpyHostToDevice, st));
     RowMap rm{s.segs.as<SeqSeg>(), s.row_slot.as<int32_t>(), s.row_pos.as<int32_t>()};
     // a slot that starts over begins from position 0 whatever its device-side length says
-    B2_TRY(rowmap_portion(rm, kv->len_dev.as<int32_t>(), slot, n, start == 0 ? 1 : 0, st));
+    B2_TRY(rowmap_portion(rm, kv->len_dev.as<int32_t>(), slot, n, start == 0 ? 1 : 0, s.want.as<int32_t>(), want_host, n_want, st));
     B2_TRY(seq_embed(m, kv, s.tok.as<int32_t>(), n, 1, st));
     B2_TRY(seq_forward(m, kv, n, 1, slot, start + n, resid_out, st));
     if (n_want > 0) {
-        B2_CUDA_CHECK(cudaMemcpyAsync(s.want.p, want_host, (size_t)n_want * 4, cudaMemcpyHostToDevice, st));
         cudaPointerAttributes attr;
         bool dev_out = cudaPointerGetAttributes(&attr, logits_out) == cudaSuccess && (attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged);
         cudaGetLastError();

@@ -66,3 +66,28 @@ def test_steps_from_and_into_any_memory(width):
         got.append((out.view(3, 101).clone(), nxt.cpu()))
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
     assert torch.equal(got[0][0].argmax(-1).cpu().int(), got[0][1])
+
+
+@pytest.mark.parametrize("n", [1, 7, 130])
+def test_residuals_and_wanted_rows_of_any_layout(n):
+    """Residual rows into a buffer that no 16-byte boundary begins and one that does; up to 128 wanted rows as kernel parameters,
+    more of them as a copy."""
+    from llava import _b2
+
+    cfg = S.config([S.layer(S.GLA, None), S.layer(S.GLA, None)], width=40, vocab=101)
+    model, _ = S.build(cfg, torch.bfloat16, max_batch=1, max_seq=160, max_rows=160)
+    eng, P = model._ensure_engine(), _b2.ptr
+    kv, toks = eng.new_kv(1, 160), S.tokens_for(cfg, n)
+    ctoks = (C.c_int32 * n)(*toks)
+    size = 2 * n * 40
+    got = []
+    for at, k in ((0, n), (1, n), (4, 1), (2, 1)):
+        want = list(range(n))[-k:]
+        resid, logits = torch.full((size + 8,), 7.0, device="cuda"), torch.empty(k, 101, device="cuda")
+        _b2.check(eng.lib.b2_append_tokens(eng.handle, kv.handle, 0, ctoks, n, 1, (C.c_int32 * k)(*want), k, P(logits), P(resid[at:]), _b2.stream_ptr()))
+        assert resid[:at].eq(7).all() and resid[at + size:].eq(7).all()
+        got.append((resid[at:at + size].clone(), logits[-1:].clone(), logits))
+    assert all(torch.equal(g[0], got[0][0]) for g in got)
+    assert torch.equal(got[0][2], got[1][2]) and torch.equal(got[2][1], got[3][1])
+    # (one row of logits is a product of its own: bf16 operands, fp32 sums in another order)
+    assert torch.allclose(got[0][1], got[2][1], atol=2 ** -8 * float(got[0][1].abs().max()))
