@@ -160,7 +160,7 @@ __global__ void gather_rows_bf16_kernel(const float* __restrict__ A, int64_t lda
 }
 
 // ... rows that are bf16 already: whole 16 bytes (5120 rows of 2048 from 1536: 17.9 us from fp32 rows, 5.6)
-__global__ void __launch_bounds__(256) gather_rows16_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const int32_t* __restrict__ src_row, __nv_bfloat16* __restrict__ out,
+__global__ void __launch_bounds__(256) gather_rows16_kernel(const __nv_bfloat16* A, int64_t lda, const int32_t* src_row, __nv_bfloat16* __restrict__ out,
                                                             int64_t ld_out, int rows, int chunks) {
     pdl_enter_late();
     const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
@@ -173,8 +173,8 @@ __global__ void __launch_bounds__(256) gather_rows16_kernel(const __nv_bfloat16*
 // x[r] += alpha * sum_k w[r, k] * y[pair_pos[r * top + k]] (a negative position: h[r] in y's place). V: columns per thread; the rows of two choices
 // are on their way at a time
 template <int V>
-__global__ void __launch_bounds__(256) moe_combine_kernel(float* __restrict__ x, const float* __restrict__ y, int64_t ldy, const int32_t* __restrict__ pair_pos,
-                                                          const float* __restrict__ w, int top, int cols, float alpha, const float* __restrict__ h, int64_t ldh) {
+__global__ void __launch_bounds__(256) moe_combine_kernel(float* __restrict__ x, const float* y, int64_t ldy, const int32_t* pair_pos,
+                                                          const float* w, int top, int cols, float alpha, const float* h, int64_t ldh) {
     pdl_enter_late();
     const size_t r = blockIdx.y;
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * V;

@@ -14,7 +14,7 @@ constexpr int kWarpsPerBlock = 4;
 // read behind the statistics, one row a warp and registers for 2048 columns took 10.6 us for 9232 rows of 1024 and 3.6 for 577 (from one kernel's end to the next); now 9.2 and 2.7.
 template <int VEC>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-layernorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
+layernorm_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma,
                  const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y, int rows, int cols,
                  float eps) {
     pdl_trigger();
@@ -122,7 +122,7 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, const 
 // dependent L2 round trips: 11 us measured for 11 MB of traffic). Same arithmetic and rounding points as rmsnorm_kernel;
 // cols % 8 == 0, cols <= 8192.
 __global__ void __launch_bounds__(256)
-rmsnorm_row_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, const int32_t* __restrict__ row_index,
+rmsnorm_row_kernel(const __nv_bfloat16* x, int64_t x_row_stride, const int32_t* row_index,
                    const __nv_bfloat16* __restrict__ gamma, __nv_bfloat16* __restrict__ y, int cols, float eps) {
     __shared__ float s_part[8];
     const int row = blockIdx.x, tid = threadIdx.x;
