@@ -91,3 +91,18 @@ def test_residuals_and_wanted_rows_of_any_layout(n):
     assert torch.equal(got[0][2], got[1][2]) and torch.equal(got[2][1], got[3][1])
     # (one row of logits is a product of its own: bf16 operands, fp32 sums in another order)
     assert torch.allclose(got[0][1], got[2][1], atol=2 ** -8 * float(got[0][1].abs().max()))
+
+
+@pytest.mark.parametrize("width", [500, 512, 516, 1022, 1024, 1028, 2048, 2052])
+def test_rows_normed_in_registers(width):
+    """LayerNorm onto the residual stream and in front of the head, at the widths where its register forms begin and end."""
+    import test_katadra_gpu as K
+
+    cfg = K.config([K.MAMBA], width=width)
+    model, w = K.build(cfg, torch.float32, max_batch=1)
+    toks = K.tokens_for(cfg, 11)
+    logits, hidden = model.forward(torch.tensor([toks]), output_hidden_states=True)
+    ref, layers = K.O.forward(cfg, w, toks, return_layers=True)
+    # fp32 sums of up to 2052 terms (2^-24 of a term each, growing with the root of their number) in two products and the norms behind them
+    assert K.err(hidden[0, 0], layers[0]) <= 2 ** -24 * 4 * 2052 ** 0.5
+    assert K.err(logits[0], ref) <= 2 ** -24 * 8 * 2052 ** 0.5
