@@ -616,7 +616,7 @@ int expert_sum_f32(const ExpertSumArgs& a, cudaStream_t st) {
 }
 
 namespace {
-__global__ void cast_rows_bf16_kernel(const float* __restrict__ A, int64_t lda, __nv_bfloat16* __restrict__ out, int64_t ld_out, int K) {
+__global__ void cast_rows_bf16_kernel(const float* A, int64_t lda, __nv_bfloat16* __restrict__ out, int64_t ld_out, int K) {
     pdl_enter();
     const size_t r = blockIdx.y;
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) * 2;

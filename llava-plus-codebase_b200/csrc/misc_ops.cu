@@ -45,7 +45,7 @@ __global__ void splice_embed_kernel(const int32_t* __restrict__ src_index, const
     }
 }
 
-__global__ void embed_tokens_kernel(const int32_t* __restrict__ tokens, const uint4* __restrict__ table,
+__global__ void embed_tokens_kernel(const int32_t* tokens, const uint4* __restrict__ table,
                                     uint4* __restrict__ out, int vec_per_row, int vocab, int* err_flag) {
     const int row = blockIdx.x;
     pdl_trigger();

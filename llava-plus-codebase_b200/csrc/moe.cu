@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int32_t* __restric
 }
 
 // out[r, c] = act(in[r, c], in[r, ff + c]): the gated unit (SiLU(g) u, or its bounded and shifted form)
-__global__ void glu_rows_kernel(const float* __restrict__ in, int64_t ld_in, float* __restrict__ out, int64_t ld_out, int ff,
+__global__ void glu_rows_kernel(const float* in, int64_t ld_in, float* __restrict__ out, int64_t ld_out, int ff,
                                 __nv_bfloat16* __restrict__ out16, int64_t ld_out16, GluAct act) {
     pdl_enter_late();
     const size_t r = blockIdx.y;
@@ -145,7 +145,7 @@ __global__ void glu_rows_kernel(const float* __restrict__ in, int64_t ld_in, flo
     }
 }
 
-__global__ void gather_rows_bf16_kernel(const float* __restrict__ A, int64_t lda, const int32_t* __restrict__ src_row, __nv_bfloat16* __restrict__ out,
+__global__ void gather_rows_bf16_kernel(const float* A, int64_t lda, const int32_t* src_row, __nv_bfloat16* __restrict__ out,
                                         int64_t ld_out, int K) {
     pdl_enter_late();
     const size_t p = blockIdx.y;

@@ -98,9 +98,9 @@ void launch_layernorm_rows(float* x, const float* y, const int32_t* row_index, c
 __device__ __forceinline__ float silu_f(float v) { return v / (1.f + expf(-v)); }
 
 // one warp per (row, group)
-__global__ void gated_group_rmsnorm_kernel(const float* __restrict__ y, int64_t ldy, const float* __restrict__ z, int64_t ldz,
+__global__ void gated_group_rmsnorm_kernel(const float* y, int64_t ldy, const float* z, int64_t ldz,
                                            const float* __restrict__ gamma, float* __restrict__ out, int64_t ldo, int rows, int groups, int group,
-                                           int gate_first, int gamma_shared, float eps, int sigmoid_gate, const float* __restrict__ den,
+                                           int gate_first, int gamma_shared, float eps, int sigmoid_gate, const float* den,
                                            __nv_bfloat16* __restrict__ out16, int64_t ldo16) {
     pdl_enter();
     const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -130,10 +130,10 @@ __global__ void gated_group_rmsnorm_kernel(const float* __restrict__ y, int64_t 
 // Groups of up to 128 NV channels, 16 bytes at a time: a lane requests all that it will use of a group before it computes anything. The loop
 // above is a chain of dependent 4-byte loads: a step's row of 1024 channels in groups of 256 8.8 -> 5.5 us, 1900 rows 30.7 -> 10.3 us.
 template <int NV>
-__global__ void __launch_bounds__(256) gated_group_rmsnorm_vec_kernel(const float* __restrict__ y, int64_t ldy, const float* __restrict__ z, int64_t ldz,
+__global__ void __launch_bounds__(256) gated_group_rmsnorm_vec_kernel(const float* y, int64_t ldy, const float* z, int64_t ldz,
                                                                       const float* __restrict__ gamma, float* __restrict__ out, int64_t ldo, int rows,
                                                                       int groups, int group, int gate_first, int gamma_shared, float eps, int sigmoid_gate,
-                                                                      const float* __restrict__ den, __nv_bfloat16* __restrict__ out16, int64_t ldo16) {
+                                                                      const float* den, __nv_bfloat16* __restrict__ out16, int64_t ldo16) {
     pdl_enter();
     const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (w >= rows * groups) return;
@@ -195,7 +195,7 @@ int launch_group_norm(const float* y, int64_t ldy, const float* z, int64_t ldz, 
 struct DytOuts { DytOut o[2]; };
 __device__ __forceinline__ float dyt_f(float x, float alpha, float w, float b) { return fmaf(tanhf(alpha * x), w, b); }
 template <bool VEC>
-__global__ void __launch_bounds__(256) dyt_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ row_index, DytOuts outs, int n_outs,
+__global__ void __launch_bounds__(256) dyt_rows_kernel(const float* x, const int32_t* row_index, DytOuts outs, int n_outs,
                                                        int cols) {
     pdl_enter();
     const size_t r = blockIdx.y;
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(256) dyt_rows_kernel(const float* __restrict__
     }
 }
 
-__global__ void __launch_bounds__(256) concat_rows_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out,
+__global__ void __launch_bounds__(256) concat_rows_kernel(const float* a, const float* b, float* __restrict__ out,
                                                           __nv_bfloat16* __restrict__ out16, int cols) {
     pdl_enter();
     const size_t r = blockIdx.y;
@@ -310,7 +310,7 @@ __global__ void embed_rows_kernel(const int32_t* tokens, const TT* __restrict__ 
     }
 }
 
-__global__ void sigmoid_gate_kernel(const float* __restrict__ a, int64_t lda, const float* __restrict__ g, int64_t ldg, float* __restrict__ out,
+__global__ void sigmoid_gate_kernel(const float* a, int64_t lda, const float* g, int64_t ldg, float* __restrict__ out,
                                     int64_t ldo, int cols) {
     pdl_enter();
     const size_t r = blockIdx.y;
@@ -321,7 +321,7 @@ __global__ void sigmoid_gate_kernel(const float* __restrict__ a, int64_t lda, co
 // ---- pre-norm blocks with a one-number RMS norm -----------------------------------------------------------------------------
 // out[i] = x[row_index[i]] / sqrt(mean(x^2) + eps) * g[0]; with `add`/`vec` the row is first updated in place:
 // x += add[row] + vec (the opening of a pass of a looped block of layers)
-__global__ void rms_scalar_kernel(float* __restrict__ x, const int32_t* __restrict__ row_index, const float* __restrict__ g,
+__global__ void rms_scalar_kernel(float* __restrict__ x, const int32_t* row_index, const float* __restrict__ g,
                                   const float* __restrict__ add, const float* __restrict__ vec, float* __restrict__ out, int cols, float eps) {
     pdl_enter();
     __shared__ float red[33];
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(256) rms_scalar_reg_kernel(float* __restrict__
 }
 
 // weighted RMS norm of a (gathered) row; accumulate: added onto out
-__global__ void rms_weight_kernel(const float* __restrict__ in, int64_t ld_in, const int32_t* __restrict__ row_index, const float* __restrict__ w,
+__global__ void rms_weight_kernel(const float* __restrict__ in, int64_t ld_in, const int32_t* row_index, const float* __restrict__ w,
                                   float* __restrict__ out, int64_t ld_out, int accumulate, int cols, float eps, __nv_bfloat16* __restrict__ out16) {
     pdl_enter();
     __shared__ float red[33];
@@ -400,7 +400,7 @@ __global__ void rms_weight_kernel(const float* __restrict__ in, int64_t ld_in, c
 // the same for rows of whole 16-byte pieces, at most V per thread: a row is read once, stays in registers, and its weights are loaded in
 // front of the reduction (in and out may be the same rows)
 template <int V>
-__global__ void __launch_bounds__(256) rms_weight_reg_kernel(const float* in, int64_t ld_in, const int32_t* __restrict__ row_index,
+__global__ void __launch_bounds__(256) rms_weight_reg_kernel(const float* in, int64_t ld_in, const int32_t* row_index,
                                                              const float* __restrict__ w, float* out, int64_t ld_out, int accumulate, int cols, float eps,
                                                              __nv_bfloat16* __restrict__ out16) {
     pdl_enter();
@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(256) rms_weight_reg_kernel(const float* in, in
 
 // token row -> weighted RMS norm of the table's row (the residual stream of a model whose embedding is normed)
 template <typename TT>
-__global__ void embed_norm_kernel(const int32_t* __restrict__ tokens, const TT* __restrict__ table, float* __restrict__ x, int cols, int vocab,
+__global__ void embed_norm_kernel(const int32_t* tokens, const TT* __restrict__ table, float* __restrict__ x, int cols, int vocab,
                                   int* err_flag, const float* __restrict__ w, float eps) {
     pdl_enter();
     __shared__ float red[33];
@@ -467,7 +467,7 @@ __device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
     return make_float4(__uint_as_float(t.x << 16), __uint_as_float(t.x & 0xffff0000u), __uint_as_float(t.y << 16), __uint_as_float(t.y & 0xffff0000u));
 }
 template <typename TT, int V>
-__global__ void __launch_bounds__(256) embed_norm_reg_kernel(const int32_t* __restrict__ tokens, const TT* __restrict__ table, float* __restrict__ x,
+__global__ void __launch_bounds__(256) embed_norm_reg_kernel(const int32_t* tokens, const TT* __restrict__ table, float* __restrict__ x,
                                                              int cols, int vocab, int* err_flag, const float* __restrict__ w, float eps) {
     pdl_enter();
     __shared__ float red[33];
@@ -649,7 +649,7 @@ __global__ void transpose_blocks_kernel(const T* __restrict__ src, T* __restrict
 }
 
 // PolyNorm: out = a N(z) + b N(z^2) + c N(z^3) + e with z = in + bias, powers element-wise, N = division by the row's root mean square
-__global__ void polynorm_kernel(const float* __restrict__ in, int64_t ld_in, const float* __restrict__ bias, const float* __restrict__ coef,
+__global__ void polynorm_kernel(const float* in, int64_t ld_in, const float* __restrict__ bias, const float* __restrict__ coef,
                                 float* __restrict__ out, int64_t ld_out, int cols, float eps, int vec) {
     pdl_enter();
     __shared__ float red[33];
@@ -706,7 +706,7 @@ __global__ void softcap_kernel(float* __restrict__ x, size_t n, float cap) {
 }
 
 // out[r, h * dv + d] = a[r, h * dv + d] * sigmoid(g[r, h]): one gate per head
-__global__ void head_gate_kernel(const float* __restrict__ a, int64_t lda, const float* __restrict__ g, int64_t ldg, float* __restrict__ out,
+__global__ void head_gate_kernel(const float* a, int64_t lda, const float* g, int64_t ldg, float* __restrict__ out,
                                  int64_t ldo, int heads, int dv) {
     pdl_enter();
     const size_t r = blockIdx.y;
@@ -718,7 +718,7 @@ __global__ void head_gate_kernel(const float* __restrict__ a, int64_t lda, const
 // token of a sequence takes row `buckets`. The previous token of a call's first row is the slot's carried token, which the same
 // block then replaces by the segment's last token. x0 (nullable) receives a copy of the rows.
 template <typename TT>
-__global__ void embed_bigram_kernel(const int32_t* __restrict__ tokens, const SeqSeg* __restrict__ segs, const TT* __restrict__ table,
+__global__ void embed_bigram_kernel(const int32_t* tokens, const SeqSeg* segs, const TT* __restrict__ table,
                                     const TT* __restrict__ bigram, int32_t* __restrict__ last_tok, float* __restrict__ x, float* __restrict__ x0,
                                     int cols, int vocab, int buckets, int mul_prev, int mul_cur, int* err_flag) {
     pdl_enter();
@@ -750,8 +750,8 @@ __global__ void embed_bigram_kernel(const int32_t* __restrict__ tokens, const Se
 }
 
 // latent[slot][pos] = unit_rms(in[r]) * gamma: the normalised low-rank row that a token leaves in the cache
-__global__ void latent_append_kernel(const float* __restrict__ in, int64_t ld_in, const float* __restrict__ gamma, float* __restrict__ cache,
-                                     const int32_t* __restrict__ row_slot, const int32_t* __restrict__ row_pos, int rank, int Smax, float eps) {
+__global__ void latent_append_kernel(const float* in, int64_t ld_in, const float* __restrict__ gamma, float* __restrict__ cache,
+                                     const int32_t* row_slot, const int32_t* row_pos, int rank, int Smax, float eps) {
     pdl_enter();
     __shared__ float red[33];
     const size_t r = blockIdx.x;

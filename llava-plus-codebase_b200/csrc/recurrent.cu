@@ -19,7 +19,7 @@ template <int FLAGS>   // CONV_SILU | CONV_ADD_INPUT; own_tail: every segment is
 __global__ void __launch_bounds__(128) causal_conv_kernel(const float* __restrict__ in, int64_t ld_in, const float* __restrict__ w,
                                                           const float* __restrict__ bias, float* __restrict__ tail,
                                                           float* __restrict__ out, int64_t ld_out, int C, int taps,
-                                                          const SeqSeg* __restrict__ segs, int own_tail) {
+                                                          const SeqSeg* segs, int own_tail) {
     pdl_enter();
     const SeqSeg sg = segs[blockIdx.z];
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(const float* __restric
 }
 // tail[j] := input of token n - (taps-1) + j of the segment; tokens before the call come from the old tail (or zero)
 __global__ void __launch_bounds__(128) causal_conv_tail_kernel(const float* __restrict__ in, int64_t ld_in, float* __restrict__ tail, int C,
-                                                               int taps, const SeqSeg* __restrict__ segs) {
+                                                               int taps, const SeqSeg* segs) {
     pdl_enter();
     const SeqSeg sg = segs[blockIdx.y];
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -99,8 +99,8 @@ __global__ void __launch_bounds__(128) causal_conv_tail_kernel(const float* __re
 // ---- token shift: out[s][t] = x[t] + (x[t-1] - x[t]) * mu[s]; x[-1] of a call is the carried row (zero at a sequence start) ---
 constexpr int SHIFT_MAX_MIX = 8, SHIFT_TILE = 8;
 __global__ void __launch_bounds__(128) token_shift_mix_kernel(const float* __restrict__ x, const float* __restrict__ mu,
-                                                              const float* __restrict__ prev, float* __restrict__ out, int64_t out_stride,
-                                                              int cols, int n_mix, const SeqSeg* __restrict__ segs) {
+                                                              const float* prev, float* __restrict__ out, int64_t out_stride,
+                                                              int cols, int n_mix, const SeqSeg* segs) {
     pdl_enter();
     const SeqSeg sg = segs[blockIdx.z];
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -123,8 +123,8 @@ __global__ void __launch_bounds__(128) token_shift_mix_kernel(const float* __res
         }
     }
 }
-__global__ void __launch_bounds__(128) token_shift_carry_kernel(const float* __restrict__ x, float* __restrict__ prev, int cols,
-                                                                const SeqSeg* __restrict__ segs) {
+__global__ void __launch_bounds__(128) token_shift_carry_kernel(const float* x, float* __restrict__ prev, int cols,
+                                                                const SeqSeg* segs) {
     pdl_enter();
     const SeqSeg sg = segs[blockIdx.y];
     const int c = blockIdx.x * blockDim.x + threadIdx.x;

@@ -155,9 +155,9 @@ __global__ void __launch_bounds__(256) rotate_rows_block_kernel(RotateParts ps) 
 }
 
 // cache[slot][pos] = [ unit_rms(in[r, :rank]) * gamma | the rot entries behind them, their first `pairs` pairs turned by pos ]
-__global__ void __launch_bounds__(128) latent_rot_append_kernel(const float* __restrict__ in, int64_t ld_in, const float* __restrict__ gamma,
-                                                                float* __restrict__ cache, const int32_t* __restrict__ row_slot,
-                                                                const int32_t* __restrict__ row_pos, int rank, int rot, int pairs,
+__global__ void __launch_bounds__(128) latent_rot_append_kernel(const float* in, int64_t ld_in, const float* __restrict__ gamma,
+                                                                float* __restrict__ cache, const int32_t* row_slot,
+                                                                const int32_t* row_pos, int rank, int rot, int pairs,
                                                                 const float2* __restrict__ table, int Smax, float eps) {
     pdl_enter_late();
     __shared__ float red[4];

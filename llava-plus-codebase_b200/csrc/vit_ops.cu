@@ -10,7 +10,7 @@ namespace b2 {
 namespace {
 
 // one CTA per patch; threads sweep the kpad output elements (k = c*ps*ps + i*ps + j)
-__global__ void vit_im2col_kernel(const __nv_bfloat16* __restrict__ pix, __nv_bfloat16* __restrict__ out, int img,
+__global__ void vit_im2col_kernel(const __nv_bfloat16* pix, __nv_bfloat16* __restrict__ out, int img,
                                   int ps, int kpad) {
     pdl_trigger();
     pdl_wait();  // inputs are outputs of the upstream kernel (programmatic dependent launch)
@@ -35,7 +35,7 @@ __global__ void vit_im2col_kernel(const __nv_bfloat16* __restrict__ pix, __nv_bf
 
 // one warp per token row; D % 256 == 0, D <= 2048
 __global__ void __launch_bounds__(128)
-vit_embed_ln_kernel(const __nv_bfloat16* __restrict__ patch_out, const __nv_bfloat16* __restrict__ cls,
+vit_embed_ln_kernel(const __nv_bfloat16* patch_out, const __nv_bfloat16* __restrict__ cls,
                     const __nv_bfloat16* __restrict__ pos, const __nv_bfloat16* __restrict__ gamma,
                     const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ hidden, int B, int P,
                     int D, float eps) {
@@ -99,7 +99,7 @@ vit_embed_ln_kernel(const __nv_bfloat16* __restrict__ patch_out, const __nv_bflo
     }
 }
 
-__global__ void vit_drop_cls_kernel(const uint4* __restrict__ hidden, uint4* __restrict__ out, int P, int vec_per_row,
+__global__ void vit_drop_cls_kernel(const uint4* hidden, uint4* __restrict__ out, int P, int vec_per_row,
                                     int64_t total_vec) {
     pdl_trigger();
     pdl_wait();  // inputs are outputs of the upstream kernel (programmatic dependent launch)
