@@ -299,18 +299,21 @@ int interleave_gate_up(const void* gate, const void* up, void* out, int I, int h
 }
 
 // What stands around one decode step, in a launch each instead of copies and a fill (4-5 us apiece between a step's graph and the next)
+// (the next step's first launch comes while the last step's end drains)
 __global__ void decode_begin_kernel(int32_t* tok, const int32_t* tokens, int B, int32_t* step_counter) {
+    pdl_wait();
     for (int b = threadIdx.x; b < B; b += blockDim.x) tok[b] = tokens[b];
     if (threadIdx.x == 0) *step_counter = 0;
 }
 __global__ void __launch_bounds__(256) decode_end_kernel(float* logits_out, const float* logits, int64_t n, int32_t* next, const int32_t* tok, int B) {
+    pdl_trigger();
     const int64_t n4 = n / 4, step = (int64_t)gridDim.x * blockDim.x, i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     for (int64_t i = i0; i < n4; i += step) reinterpret_cast<float4*>(logits_out)[i] = reinterpret_cast<const float4*>(logits)[i];
     for (int64_t i = 4 * n4 + i0; i < n; i += step) logits_out[i] = logits[i];
     for (int64_t b = i0; b < B; b += step) next[b] = tok[b];
 }
 int decode_begin(int32_t* tok, const int32_t* tokens, int B, int32_t* step_counter, cudaStream_t stream) {
-    decode_begin_kernel<<<1, 128, 0, stream>>>(tok, tokens, B, step_counter);
+    B2_CUDA_CHECK(launch_pdl(decode_begin_kernel, dim3(1), dim3(128), 0, stream, tok, tokens, B, step_counter));
     B2_LAUNCH_CHECK();
     return 0;
 }
