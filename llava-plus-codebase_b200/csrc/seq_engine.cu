@@ -1207,9 +1207,10 @@ static int seq_cap_logits(const SeqModel& s, float* logits, int n, int64_t ld, c
     B2_CHECK_ARG(ld == s.d.vocab, "seq_head: soft-capped logits are contiguous rows");
     return softcap_f32(logits, (size_t)n * s.d.vocab, s.d.logit_softcap, st);
 }
-// rows `index` (null: all) of x -> final norm -> head -> soft-cap: fp32 logits [n, vocab]
-static int seq_head(b2_model* m, const int32_t* index, int n, float* logits, int64_t ld, cudaStream_t st) {
+// rows `index` (null: n rows from `row` on) of x -> final norm -> head -> soft-cap: fp32 logits [n, vocab]
+static int seq_head(b2_model* m, const int32_t* index, int n, float* logits, int64_t ld, cudaStream_t st, int row = 0) {
     SeqModel& s = *m->seq;
+    float* x = s.x.as<float>() + (size_t)row * s.d.width;
     const Lin lin{m, st};
     const DevBuf& head = s.d.tied_head ? s.embed : s.head;
     const float lscale = s.d.logit_scale != 0.f ? s.d.logit_scale : 1.f;
@@ -1220,18 +1221,18 @@ static int seq_head(b2_model* m, const int32_t* index, int n, float* logits, int
         DytOut o;
         o.norm = dn = dyt_of(s.final_a, s.final_w, s.final_b);
         if (index == nullptr && lin.fuses_norm(s.d.width, n)) {   // a decode step: the rows are normed on their way into the product
-            in = s.x.as<float>();
+            in = x;
         } else {
             dn.alpha = nullptr;
             if (lin.tensor_cores(s.d.vocab, s.d.width, logits, ld, n)) o.out16 = const_cast<void*>(in16 = s.a16.p);
             else o.out = s.xn.as<float>();
-            B2_TRY(dyt_rows_f32(s.x.as<float>(), index, &o, 1, n, s.d.width, st));
+            B2_TRY(dyt_rows_f32(x, index, &o, 1, n, s.d.width, st));
         }
     } else if (s.d.block == B2_BLOCK_PRE_RMS1)
-        B2_TRY(rms_scalar_f32(s.x.as<float>(), index, s.final_w.as<float>(), nullptr, nullptr, s.xn.as<float>(), n, s.d.width, s.d.norm_eps, st));
+        B2_TRY(rms_scalar_f32(x, index, s.final_w.as<float>(), nullptr, nullptr, s.xn.as<float>(), n, s.d.width, s.d.norm_eps, st));
     else if (s.d.block == B2_BLOCK_SANDWICH_RMS || s.d.block == B2_BLOCK_PARALLEL_RMS || s.d.block == B2_BLOCK_PARALLEL2) {
         if (n == 1 && index == nullptr && tc_enabled()) {   // one row is normed on its way into the head
-            LinearArgs a = lin.args(s.x.as<float>(), s.d.width, head, s.d.vocab, s.d.width, logits, ld, 1, LIN_NONE, lscale);
+            LinearArgs a = lin.args(x, s.d.width, head, s.d.vocab, s.d.width, logits, ld, 1, LIN_NONE, lscale);
             a.rms_w = s.final_w.as<float>(); a.rms_eps = s.d.norm_eps;
             if (linear_stream_norms(a)) {
                 B2_TRY(linear_stream_f32(a, st));
@@ -1239,9 +1240,9 @@ static int seq_head(b2_model* m, const int32_t* index, int n, float* logits, int
             }
         }
         if (s.a16.p != nullptr && lin.tensor_cores(s.d.vocab, s.d.width, logits, ld, n)) in16 = s.a16.p;   // (several rows: as the head reads them)
-        B2_TRY(rms_weight_f32(s.x.as<float>(), s.d.width, index, s.final_w.as<float>(), s.xn.as<float>(), s.d.width, 0, n, s.d.width, s.d.norm_eps, st, const_cast<void*>(in16)));
+        B2_TRY(rms_weight_f32(x, s.d.width, index, s.final_w.as<float>(), s.xn.as<float>(), s.d.width, 0, n, s.d.width, s.d.norm_eps, st, const_cast<void*>(in16)));
     } else
-        B2_TRY(layernorm_gather_f32(s.x.as<float>(), index, s.final_w.as<float>(), s.final_b.as<float>(), s.xn.as<float>(), n, s.d.width, s.d.norm_eps, st));
+        B2_TRY(layernorm_gather_f32(x, index, s.final_w.as<float>(), s.final_b.as<float>(), s.xn.as<float>(), n, s.d.width, s.d.norm_eps, st));
     B2_TRY(lin(in, s.d.width, head, s.d.vocab, s.d.width, logits, ld, n, LIN_NONE, lscale, 0, nullptr, 0, nullptr, in16, dn.alpha != nullptr ? &dn : nullptr));
     return seq_cap_logits(s, logits, n, ld, st);
 }
@@ -2269,7 +2270,9 @@ int b2_append_tokens(b2_model* m, b2_kv* kv, int slot, const int32_t* tokens_hos
         bool dev_out = cudaPointerGetAttributes(&attr, logits_out) == cudaSuccess && (attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged);
         cudaGetLastError();
         if (dev_out) {
-            B2_TRY(seq_head(m, s.want.as<int32_t>(), n_want, logits_out, s.d.vocab, st));
+            // (one row, by its address: normed on its way into the head where a decode step's is)
+            if (n_want == 1) B2_TRY(seq_head(m, nullptr, 1, logits_out, s.d.vocab, st, want_host[0]));
+            else B2_TRY(seq_head(m, s.want.as<int32_t>(), n_want, logits_out, s.d.vocab, st));
         } else {
             // host destination: through the projection workspace, in pieces of what it holds
             const int per = (int)std::max<size_t>(1, ((size_t)s.rows * s.proj_w) / s.d.vocab);
