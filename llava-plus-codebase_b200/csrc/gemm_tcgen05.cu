@@ -670,7 +670,7 @@ int gemm_bf16(const GemmArgs& g, cudaStream_t stream) {
                  "gemm: a grouped product takes whole tiles of %d rows, no bias, residual or fused activation but the gated unit", BM);
     if (g.bn_override >= 1000 && !grouped) {
         const int bn = g.bn_override % 1000, S = g.bn_override / 1000;
-        B2_CHECK_ARG((bn == 64 || bn == 128) && (S == 2 || S == 4) && !glu, "gemm(split K): no plan bn=%d S=%d activation=%d", bn, S, g.act);
+        B2_CHECK_ARG((bn == 64 || bn == 128) && (S == 2 || S == 4), "gemm(split K): no plan bn=%d S=%d", bn, S);
         return gemm_bf16_splitk(g, bn, S, stream);
     }
     if (g.bn_override == 2 && !grouped) return gemm_bf16_2cta(g, stream);  // CTA-pair kernel (cta_group::2, 256x256 pair tiles)
