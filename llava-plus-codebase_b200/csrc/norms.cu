@@ -9,9 +9,9 @@ namespace {
 
 constexpr int kWarpsPerBlock = 4;
 
-// cols % 256 == 0 (each lane handles cols/32 elements in 16 B vectors); cols <= 256 * VEC. A warp takes rows row0, row0 + warps, ...: weight and bias stay in
-// registers, and the next row is on its way while this one is normed. The kernel stands between two products and is bound by its chain: weights
-// read behind the statistics, one row a warp and registers for 2048 columns took 10.6 us for 9232 rows of 1024 and 3.6 for 577 (from one kernel's end to the next); now 9.2 and 2.7.
+// cols % 256 == 0 (each lane handles cols/32 elements in 16 B vectors); cols <= 256 * VEC. Weight and bias are asked for with the row: between two products the
+// kernel is bound by its chain of loads and sums (577 rows of 1024, from one kernel's end to the next: 3.6 us with the weights behind the statistics and
+// registers for 2048 columns at every width, now 2.6; back to back 9232 rows 10.5 -> 8.9, 36928 32.8 -> 27.0). Several rows a warp with the weights kept lost: 18464 rows 18.0 -> 35.4 us, 36928 32.8 -> 65.9.
 template <int VEC>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 layernorm_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma,
@@ -19,8 +19,8 @@ layernorm_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma
                  float eps) {
     pdl_trigger();
     pdl_wait();  // inputs are outputs of the upstream kernel (programmatic dependent launch)
-    int row = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31, step = gridDim.x * kWarpsPerBlock;
+    const int row = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
     if (row >= rows) return;
     const int nvec = cols / 256;
     uint4 u[VEC], g[VEC], b[VEC];
@@ -33,46 +33,42 @@ layernorm_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma
             g[i] = *reinterpret_cast<const uint4*>(gamma + i * 256 + lane * 8);
             b[i] = *reinterpret_cast<const uint4*>(beta + i * 256 + lane * 8);
         }
-#pragma unroll 1
-    for (; row < rows; row += step) {
-        float v[VEC][8];
-        float sum = 0.f;
+    float v[VEC][8];
+    float sum = 0.f;
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) {
-            if (i < nvec) {
-                v[i][0] = bf16_lo(u[i].x); v[i][1] = bf16_hi(u[i].x); v[i][2] = bf16_lo(u[i].y); v[i][3] = bf16_hi(u[i].y);
-                v[i][4] = bf16_lo(u[i].z); v[i][5] = bf16_hi(u[i].z); v[i][6] = bf16_lo(u[i].w); v[i][7] = bf16_hi(u[i].w);
-                if (row + step < rows) u[i] = *reinterpret_cast<const uint4*>(x + (size_t)(row + step) * cols + i * 256 + lane * 8);
+    for (int i = 0; i < VEC; ++i) {
+        if (i < nvec) {
+            v[i][0] = bf16_lo(u[i].x); v[i][1] = bf16_hi(u[i].x); v[i][2] = bf16_lo(u[i].y); v[i][3] = bf16_hi(u[i].y);
+            v[i][4] = bf16_lo(u[i].z); v[i][5] = bf16_hi(u[i].z); v[i][6] = bf16_lo(u[i].w); v[i][7] = bf16_hi(u[i].w);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) sum += v[i][e];
+            for (int e = 0; e < 8; ++e) sum += v[i][e];
+        }
+    }
+    const float mean = warp_sum(sum) / cols;
+    float var = 0.f;
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+        if (i < nvec) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float d = v[i][e] - mean;
+                var += d * d;
             }
         }
-        const float mean = warp_sum(sum) / cols;
-        float var = 0.f;
+    }
+    const float rstd = rsqrtf(warp_sum(var) / cols + eps);
+    __nv_bfloat16* yr = y + (size_t)row * cols;
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) {
-            if (i < nvec) {
+    for (int i = 0; i < VEC; ++i) {
+        if (i < nvec) {
+            const float gg[8] = {bf16_lo(g[i].x), bf16_hi(g[i].x), bf16_lo(g[i].y), bf16_hi(g[i].y),
+                                 bf16_lo(g[i].z), bf16_hi(g[i].z), bf16_lo(g[i].w), bf16_hi(g[i].w)};
+            const float bb[8] = {bf16_lo(b[i].x), bf16_hi(b[i].x), bf16_lo(b[i].y), bf16_hi(b[i].y),
+                                 bf16_lo(b[i].z), bf16_hi(b[i].z), bf16_lo(b[i].w), bf16_hi(b[i].w)};
+            float o[8];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const float d = v[i][e] - mean;
-                    var += d * d;
-                }
-            }
-        }
-        const float rstd = rsqrtf(warp_sum(var) / cols + eps);
-        __nv_bfloat16* yr = y + (size_t)row * cols;
-#pragma unroll
-        for (int i = 0; i < VEC; ++i) {
-            if (i < nvec) {
-                const float gg[8] = {bf16_lo(g[i].x), bf16_hi(g[i].x), bf16_lo(g[i].y), bf16_hi(g[i].y),
-                                     bf16_lo(g[i].z), bf16_hi(g[i].z), bf16_lo(g[i].w), bf16_hi(g[i].w)};
-                const float bb[8] = {bf16_lo(b[i].x), bf16_hi(b[i].x), bf16_lo(b[i].y), bf16_hi(b[i].y),
-                                     bf16_lo(b[i].z), bf16_hi(b[i].z), bf16_lo(b[i].w), bf16_hi(b[i].w)};
-                float o[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) o[e] = (v[i][e] - mean) * rstd * gg[e] + bb[e];
-                *reinterpret_cast<uint4*>(yr + i * 256 + lane * 8) = make_uint4(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]), pack_bf16(o[6], o[7]));
-            }
+            for (int e = 0; e < 8; ++e) o[e] = (v[i][e] - mean) * rstd * gg[e] + bb[e];
+            *reinterpret_cast<uint4*>(yr + i * 256 + lane * 8) = make_uint4(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]), pack_bf16(o[6], o[7]));
         }
     }
 }
@@ -178,8 +174,7 @@ int layernorm_bf16(const void* x, const void* gamma, const void* beta, void* y, 
                    cudaStream_t stream) {
     B2_CHECK_ARG(rows > 0 && cols > 0 && cols % 256 == 0 && cols <= 2048,
                  "layernorm: cols must be a multiple of 256 and <= 2048 (cols=%d rows=%d)", cols, rows);
-    // as many rows a warp as leave five blocks an SM or fewer, shared evenly
-    const int blocks = (rows + kWarpsPerBlock - 1) / kWarpsPerBlock, turns = (blocks + 5 * num_sms() - 1) / (5 * num_sms()), grid = (blocks + turns - 1) / turns;
+    const int grid = (rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
     B2_CUDA_CHECK(launch_pdl(cols <= 1024 ? layernorm_kernel<4> : layernorm_kernel<8>, dim3(grid), dim3(kWarpsPerBlock * 32), 0, stream,
         reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(gamma),
         reinterpret_cast<const __nv_bfloat16*>(beta), reinterpret_cast<__nv_bfloat16*>(y), rows, cols, eps));

@@ -1,4 +1,4 @@
-"""bf16 LayerNorm (csrc/norms.cu) where its warps take several rows each: row counts around whole turns of the grid, every register count."""
+"""bf16 LayerNorm (csrc/norms.cu) in both of its register forms, at row counts around whole blocks and far above one wave of them."""
 import pytest
 import torch
 
