@@ -779,7 +779,10 @@ __global__ void rowmap_portion_kernel(SeqSeg* segs, int32_t* row_slot, int32_t* 
 
 // dst = src: two groups of four numbers a thread
 __global__ void __launch_bounds__(256) copy_f32_kernel(float4* __restrict__ dst, const float4* src, size_t n4) {
-    pdl_enter_late();   // (pdl_enter: a prompt of 41 rows through four layers 338 us instead of 309)
+    // and no trigger: the next kernel may be the head, whose one CTA an SM find their places best on empty SMs (let in among the CTAs of the layer's last
+    // product: 70 rows through one layer of width 2048 97 -> 120 us with the weights in L2; a prompt of 41 rows through four layers, us: plain copies
+    // 316, a trigger at once 338, behind the wait 310, none 309)
+    pdl_wait();
     const size_t i = (size_t)blockIdx.x * 512 + threadIdx.x;
     float4 a, b;
     if (i < n4) a = src[i];
