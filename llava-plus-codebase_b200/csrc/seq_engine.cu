@@ -191,8 +191,8 @@ int tc_min_rows() {
     const int v = e != nullptr ? atoi(e) : 0;
     // (the streamed products read bf16 rows twice as fast, and a norm on its way in keeps them on the FMA kernels. us a step of four layers, 2 and 3 rows, from
     // 4 rows on / from 2: mixed layers of width 2048 199 / 182 and 197 / 181; dynamic-tanh norms of 2048 299 / 208 and 328 / 211; parallel experts of 2048 219 /
-    // 209 and 243 / 239; other designs within 1 %)
-    return v >= 1 ? v : 2;
+    // 209 and 243 / 239; other designs within 1 %. One row streams its fp32 rows whatever the variable says: bf16 rows alone would not be read)
+    return v >= 2 ? v : 2;
 }
 
 struct Lin {  // one Linear call on the model's compute dtype

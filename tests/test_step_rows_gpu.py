@@ -106,3 +106,25 @@ def test_rows_normed_in_registers(width):
     # fp32 sums of up to 2052 terms (2^-24 of a term each, growing with the root of their number) in two products and the norms behind them
     assert K.err(hidden[0, 0], layers[0]) <= 2 ** -24 * 4 * 2052 ** 0.5
     assert K.err(logits[0], ref) <= 2 ** -24 * 8 * 2052 ** 0.5
+
+
+@pytest.mark.parametrize("name", ["gla", "diff", "win", "memory"])
+def test_one_row_steps_where_every_row_counts_as_a_tensor_core_one(name, monkeypatch):
+    """B2_SEQ_TC_MIN_ROWS=1: the step of one row streams its fp32 rows all the same, so nothing in front of it may leave bf16 rows alone."""
+    import test_ramosun_gpu as R
+
+    if name == "memory":
+        mod, cfg = R, R.CFG_MAIN
+    else:
+        mix = {"gla": S.gla(2, 32, 32), "diff": S.diff(2, 1, 32, 32, None, None, 32), "win": S.win(2, 1, 32, 32, None, None, 32)}[name]
+        mod, cfg = S, S.config([S.layer(mix, {"kind": "dense", "ff": 64, "limit": 1.25})] * 2, width=64)
+    toks, got = mod.tokens_for(cfg, 9), []
+    for rows in ("1", "2"):
+        monkeypatch.setenv("B2_SEQ_TC_MIN_ROWS", rows)
+        model, _ = mod.build(cfg, torch.bfloat16, max_batch=1, max_seq=32, max_rows=16)
+        eng = model._ensure_engine()
+        kv = eng.new_kv(1, 32)
+        eng.append_tokens(kv, 0, toks[:5], restart=True)
+        got.append(torch.cat([eng.decode_step(kv, torch.tensor([t], dtype=torch.int32)).clone().view(1, -1) for t in toks[5:]]))
+        model.invalidate_engine()
+    assert torch.equal(got[0], got[1])
