@@ -466,3 +466,20 @@ def test_rows_of_norms_and_experts(width, rows, dtype):
     model.invalidate_engine()
     for a, b in zip(got, ref):
         assert close(a, b, dtype)
+
+
+@pytest.mark.parametrize("width", [8192, 8200])
+def test_widths_around_the_register_form_of_the_norm(width):
+    """Two rows of a prompt and of a step, whose norms leave a rounded copy beside the fp32 rows, at the widest row held in registers and above it."""
+    cfg = config([layer(HG, None), layer(LAT, MOE)], width=width, softcap=None)
+    model, w = build(cfg, torch.bfloat16, max_batch=2, max_seq=8, max_rows=2)
+    eng, toks = model._ensure_engine(), tokens_for(cfg, 3)
+    kv = eng.new_kv(2, 8)
+    for slot in range(2):
+        got = eng.append_tokens(kv, slot, toks[:2], restart=True, residuals=True)[1]
+    logits = eng.decode_step(kv, torch.tensor([toks[2]] * 2, dtype=torch.int32))
+    ref_logits, ref = O.forward(cfg, w, toks)[:2]
+    for a, b in zip(got, ref):
+        assert close(a, np.asarray(b)[:2], torch.bfloat16)
+    assert close(logits, np.stack([np.asarray(ref_logits)[2]] * 2), torch.bfloat16)
+    model.invalidate_engine()
