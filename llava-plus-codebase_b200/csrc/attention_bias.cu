@@ -189,7 +189,7 @@ constexpr int TL_KT = 32, TL_WARPS = 8, TL_PPW = 4;
 // dst[r * dpitch + c] = src[r * spitch + c] for r < nrows, c < 4 * n4, 16 bytes at a time; a thread issues N loads before its
 // first store, so the copy is bound by bandwidth and not by one memory round trip per element
 template <int N>
-__device__ __forceinline__ void copy_rows_f4(float* __restrict__ dst, int dpitch, const float* __restrict__ src, size_t spitch, int nrows, int n4,
+__device__ __forceinline__ void copy_rows_f4(float* __restrict__ dst, int dpitch, const float* src, size_t spitch, int nrows, int n4,
                                              int tid) {
     const int total = nrows * n4;
     for (int base = 0; base < total; base += TL_WARPS * 32 * N) {

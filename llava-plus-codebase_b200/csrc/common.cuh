@@ -54,8 +54,9 @@ extern unsigned long long g_launch_count;  // kernels launched by this library (
 // is still draining; everything it does BEFORE pdl_wait() must not touch memory the predecessor writes or reads-then-expects
 // unchanged. Kernels of the decode step use the window to fetch WEIGHTS (which no kernel writes) into shared memory.
 // ----------------------------------------------------------------------------------------------
-// What another kernel writes is not read through a `const __restrict__` parameter: such loads count as constant over the kernel's life, and the compiler may
-// move them in front of the wait (seen in a norm with its row in registers, 8 loads a thread: stale rows with programmatic launches, none without).
+// What another kernel writes is not read through a `const __restrict__` parameter or __ldg: such loads count as constant over the kernel's life, and the
+// compiler may move them in front of the wait (seen in a norm with its row in registers, 8 loads a thread: stale rows with programmatic launches, none
+// without). tests/test_launch_order_host.py lists the parameters that may be: weights and tables.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

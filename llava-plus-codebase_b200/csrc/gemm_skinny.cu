@@ -334,7 +334,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
                         const int b = c * 32 + j;
-                        acc[j] *= ws * (b < B ? __ldg(ep.x_scale + b) : 0.f);
+                        acc[j] *= ws * (b < B ? ep.x_scale[b] : 0.f);
                     }
                 }
                 if constexpr (ACT == ACT_SWIGLU) {

@@ -49,7 +49,7 @@ __device__ __forceinline__ void ld_w8(const __nv_bfloat16* p, float (&w)[8]) {
 // is bf16: whole (K <= kc_max) and then shared by every column group the CTA walks, or kc_max columns at a time for one group.
 constexpr int RW_COLS = 2, RW_SMEM_FLOATS = 16384;
 template <typename TW>
-__global__ void __launch_bounds__(256) linear_rows_vec_kernel(const float* __restrict__ A, int64_t lda, const TW* __restrict__ W, int64_t ldw,
+__global__ void __launch_bounds__(256) linear_rows_vec_kernel(const float* A, int64_t lda, const TW* __restrict__ W, int64_t ldw,
                                                               const float* __restrict__ bias, float* __restrict__ out, int64_t ld_out, int M, int N,
                                                               int K, int kc_max, int act, float alpha, int accumulate, int round_a, DytNorm norm) {
     pdl_enter();
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(256) linear_rows_vec_kernel(const float* __res
 // column meet in shared memory in a fixed order.
 constexpr int R1_U = 4;
 template <typename TW, int WPC, bool NORM>
-__global__ void __launch_bounds__(256) linear_one_row_kernel(const float* __restrict__ A, const TW* __restrict__ W, int64_t ldw,
+__global__ void __launch_bounds__(256) linear_one_row_kernel(const float* A, const TW* __restrict__ W, int64_t ldw,
                                                              const float* __restrict__ bias, float* __restrict__ out, int N, int K, int act,
                                                              float alpha, int accumulate, int round_a, DytNorm norm) {
     pdl_enter();
@@ -209,7 +209,7 @@ int launch_one_row(const LinearArgs& a, cudaStream_t st) {
 
 // any K and alignment: one warp per output column, scalar loads
 template <typename TW>
-__global__ void __launch_bounds__(256) linear_rows_kernel(const float* __restrict__ A, int64_t lda, const TW* __restrict__ W, int64_t ldw,
+__global__ void __launch_bounds__(256) linear_rows_kernel(const float* A, int64_t lda, const TW* __restrict__ W, int64_t ldw,
                                                           const float* __restrict__ bias, float* __restrict__ out, int64_t ld_out, int M, int N,
                                                           int K, int act, float alpha, int accumulate, int round_a) {
     pdl_enter();
@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(256) linear_rows_kernel(const float* __restric
 // ---- portions of a prompt: 64 x 64 output tile, K in steps of 16, 4 x 4 outputs per thread -------------------------------
 constexpr int TB = 64, TK = 16;
 template <typename TW>
-__global__ void __launch_bounds__(256) linear_tiled_kernel(const float* __restrict__ A, int64_t lda, const TW* __restrict__ W, int64_t ldw,
+__global__ void __launch_bounds__(256) linear_tiled_kernel(const float* A, int64_t lda, const TW* __restrict__ W, int64_t ldw,
                                                            const float* __restrict__ bias, float* __restrict__ out, int64_t ld_out, int M, int N,
                                                            int K, int act, float alpha, int accumulate, int round_a) {
     pdl_enter();
@@ -517,9 +517,9 @@ int launch_expert_sum(const ExpertSumArgs& a, cudaStream_t st) {
 // batched small Linears of a decode step: block = 8 output columns of one batch entry (a head), one warp per column; the
 // weight row is read once and multiplied with every row of the step
 template <typename TW, bool VEC>
-__global__ void __launch_bounds__(256) linear_batched_rows_kernel(const float* __restrict__ A, int64_t lda, int64_t a_bs, const TW* __restrict__ W,
+__global__ void __launch_bounds__(256) linear_batched_rows_kernel(const float* A, int64_t lda, int64_t a_bs, const TW* __restrict__ W,
                                                                   int64_t w_bs, float* __restrict__ out, int64_t ld_out, int64_t o_bs, int M, int N,
-                                                                  int K, int round_a, const float* __restrict__ gate, int64_t ldg) {
+                                                                  int K, int round_a, const float* gate, int64_t ldg) {
     pdl_enter();
     const int b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = blockIdx.x * 8 + warp;

@@ -39,7 +39,7 @@ struct LxCfg {
 };
 
 // rows of fp32 -> [part][rows][pitch] bf16, entries past K zero
-__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ in, int64_t ld, int rows, int K, int pitch, __nv_bfloat16* __restrict__ out, int vec) {
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* in, int64_t ld, int rows, int K, int pitch, __nv_bfloat16* __restrict__ out, int vec) {
     pdl_enter();
     const int chunks = pitch >> 3;
     const int64_t total = (int64_t)rows * chunks, plane = (int64_t)rows * pitch;

@@ -104,7 +104,7 @@ __global__ void moe_route_kernel(MoeRouteArgs a) {
 // One block. pairs = rows * top (token, choice) pairs with their expert in idx. Every expert gets its pairs in consecutive
 // positions, padded to a multiple of `tile` rows: pair_pos[pair] = position, src_row[position] = token row (-1: padding),
 // tile_group[t] = expert of tile t (-1: unused), for max_tiles tiles. A pair with a negative index has no expert: position -1.
-__global__ void __launch_bounds__(1024) moe_plan_kernel(const int32_t* __restrict__ idx, int pairs, int top, int experts, int tile, int max_tiles,
+__global__ void __launch_bounds__(1024) moe_plan_kernel(const int32_t* idx, int pairs, int top, int experts, int tile, int max_tiles,
                                                         int32_t* __restrict__ pair_pos, int32_t* __restrict__ src_row,
                                                         int32_t* __restrict__ tile_group) {
     pdl_enter_late();

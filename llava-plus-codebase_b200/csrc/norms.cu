@@ -74,7 +74,7 @@ layernorm_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma
 }
 
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, const int32_t* row_index,
+rmsnorm_kernel(const __nv_bfloat16* x, int64_t x_row_stride, const int32_t* row_index,
                const __nv_bfloat16* __restrict__ gamma, __nv_bfloat16* __restrict__ y, int rows, int cols,
                float eps) {
     pdl_trigger();

@@ -322,7 +322,7 @@ __global__ void sigmoid_gate_kernel(const float* a, int64_t lda, const float* g,
 // out[i] = x[row_index[i]] / sqrt(mean(x^2) + eps) * g[0]; with `add`/`vec` the row is first updated in place:
 // x += add[row] + vec (the opening of a pass of a looped block of layers)
 __global__ void rms_scalar_kernel(float* __restrict__ x, const int32_t* row_index, const float* __restrict__ g,
-                                  const float* __restrict__ add, const float* __restrict__ vec, float* __restrict__ out, int cols, float eps,
+                                  const float* add, const float* __restrict__ vec, float* __restrict__ out, int cols, float eps,
                                   __nv_bfloat16* __restrict__ out16) {
     pdl_enter();
     __shared__ float red[33];
@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(256) rms_scalar_reg_kernel(float* __restrict__
 }
 
 // weighted RMS norm of a (gathered) row; accumulate: added onto out
-__global__ void rms_weight_kernel(const float* __restrict__ in, int64_t ld_in, const int32_t* row_index, const float* __restrict__ w,
+__global__ void rms_weight_kernel(const float* in, int64_t ld_in, const int32_t* row_index, const float* __restrict__ w,
                                   float* __restrict__ out, int64_t ld_out, int accumulate, int cols, float eps, __nv_bfloat16* __restrict__ out16) {
     pdl_enter();
     __shared__ float red[33];

@@ -16,7 +16,7 @@ namespace {
 // second small kernel replaces it afterwards, so tiles never race with the update.
 constexpr int CONV_MAX_TAPS = 16, CONV_TILE = 32;
 template <int FLAGS>   // CONV_SILU | CONV_ADD_INPUT; own_tail: every segment is ONE tile, whose thread replaces the carried inputs itself
-__global__ void __launch_bounds__(128) causal_conv_kernel(const float* __restrict__ in, int64_t ld_in, const float* __restrict__ w,
+__global__ void __launch_bounds__(128) causal_conv_kernel(const float* in, int64_t ld_in, const float* __restrict__ w,
                                                           const float* __restrict__ bias, float* __restrict__ tail,
                                                           float* __restrict__ out, int64_t ld_out, int C, int taps,
                                                           const SeqSeg* segs, int own_tail) {
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(const float* __restric
     }
 }
 // tail[j] := input of token n - (taps-1) + j of the segment; tokens before the call come from the old tail (or zero)
-__global__ void __launch_bounds__(128) causal_conv_tail_kernel(const float* __restrict__ in, int64_t ld_in, float* __restrict__ tail, int C,
+__global__ void __launch_bounds__(128) causal_conv_tail_kernel(const float* in, int64_t ld_in, float* __restrict__ tail, int C,
                                                                int taps, const SeqSeg* segs) {
     pdl_enter();
     const SeqSeg sg = segs[blockIdx.y];
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(128) causal_conv_tail_kernel(const float* __re
 
 // ---- token shift: out[s][t] = x[t] + (x[t-1] - x[t]) * mu[s]; x[-1] of a call is the carried row (zero at a sequence start) ---
 constexpr int SHIFT_MAX_MIX = 8, SHIFT_TILE = 8;
-__global__ void __launch_bounds__(128) token_shift_mix_kernel(const float* __restrict__ x, const float* __restrict__ mu,
+__global__ void __launch_bounds__(128) token_shift_mix_kernel(const float* x, const float* __restrict__ mu,
                                                               const float* prev, float* __restrict__ out, int64_t out_stride,
                                                               int cols, int n_mix, const SeqSeg* segs) {
     pdl_enter();

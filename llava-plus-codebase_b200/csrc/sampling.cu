@@ -156,7 +156,7 @@ __device__ __forceinline__ uint32_t radix_select(const float* s_x, int V, unsign
 }
 
 __global__ void __launch_bounds__(SP_THREADS, 1)
-sample_publish_kernel(const float* __restrict__ logits, int V, int B, SampleState* st, RowState* rows, int32_t* tok, int32_t* out_tokens,
+sample_publish_kernel(const float* logits, int V, int B, SampleState* st, RowState* rows, int32_t* tok, int32_t* out_tokens,
                       int32_t* step_counter, int32_t* cur_len, volatile int32_t* ring, int ring_cap, int flags,
                       int step_offset) {
     extern __shared__ __align__(16) uint8_t sp_smem[];

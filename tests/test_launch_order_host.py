@@ -44,3 +44,39 @@ def test_cluster_barriers_take_whole_warps(repo_root):
             seen += 1
             assert re.search(r"__syncwarp\(\);\s*asm volatile\(\"$", src[:m.start()]), os.path.basename(path)
     assert seen >= 1
+
+
+# `const __restrict__` parameters of kernels that wait for the one in front: a model's weights and tables, which no kernel of a pass writes
+WEIGHTS = {
+    "linear_rows_vec_kernel": "W bias", "linear_one_row_kernel": "W bias", "linear_rows_kernel": "W bias", "linear_tiled_kernel": "W bias",
+    "linear_batched_rows_kernel": "W", "embed_tokens_kernel": "table", "layernorm_kernel": "gamma beta", "rmsnorm_kernel": "gamma",
+    "rmsnorm_row_kernel": "gamma", "layernorm_rows_kernel": "gamma beta", "gated_group_rmsnorm_kernel": "gamma", "gated_group_rmsnorm_vec_kernel": "gamma",
+    "embed_rows_kernel": "table", "rms_scalar_kernel": "g vec", "rms_scalar_reg_kernel": "g vec", "rms_weight_kernel": "w", "rms_weight_reg_kernel": "w",
+    "embed_norm_kernel": "table w", "embed_norm_reg_kernel": "table w", "polynorm_kernel": "bias coef", "embed_bigram_kernel": "table bigram",
+    "latent_append_kernel": "gamma", "causal_conv_kernel": "w bias", "token_shift_mix_kernel": "mu", "latent_rot_append_kernel": "gamma table",
+    "vit_embed_ln_kernel": "cls pos gamma beta",
+}
+READ_ONLY = {"io.gamma", "tab", "ep.w_scale"}   # what __ldg reads: norm weights, cosines and sines, scales of weights
+
+
+def waiting_parameters(src):
+    """(kernel, its `const __restrict__` parameters, what it reads by __ldg) of every kernel that waits for the one in front of it"""
+    src = re.sub(r"//[^\n]*|/\*.*?\*/", "", src, flags=re.S)
+    for m in re.finditer(r"__global__\b", src):
+        at = src.index("{", m.end())
+        head, body = src[m.end():at], next(body for _, body in kernels(src[m.start():]))
+        if re.search(r"\bpdl_(wait|enter)", body):
+            yield (re.findall(r"(\w+_kernel)\b", head)[0], set(re.findall(r"const\s+[\w:]+\s*\*\s*__restrict__\s+(\w+)", head)),
+                   set(re.findall(r"__ldg\((?:reinterpret_cast<[^>]*>\()?([\w.]+)", body)))
+
+
+def test_rows_that_other_kernels_write_are_not_read_as_constants(repo_root):
+    """The compiler may move a load through a `const __restrict__` parameter in front of griddepcontrol.wait, and then reads what the kernel in front
+    has not written yet."""
+    seen = 0
+    for path in glob.glob(os.path.join(repo_root, "llava-plus-codebase_b200", "csrc", "*.cu")):
+        for name, params, ldg in waiting_parameters(open(path).read()):
+            seen += 1
+            assert params <= set(WEIGHTS.get(name, "").split()), f"{os.path.basename(path)}: {name} reads {params} as constants"
+            assert ldg <= READ_ONLY, f"{os.path.basename(path)}: {name} reads {ldg} as constants"
+    assert seen >= 60
