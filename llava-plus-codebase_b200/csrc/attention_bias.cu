@@ -481,6 +481,12 @@ __device__ __forceinline__ void st_turn(const StepAppend& r, const float* norm_w
     }
 }
 
+// The block's warps meet, each with its first rows on their way or none to ask for: a barrier by number counts warps, wherever in the program they come to it
+__device__ __forceinline__ void st_meet() {
+    __syncwarp();
+    asm volatile("bar.sync 1, %0;" ::"n"(ST_WARPS * 32) : "memory");
+}
+
 // grid (C, G * chunks, rows), clusters along x; NH >= query heads of a chunk
 template <int NH, bool APPEND>
 __global__ void __launch_bounds__(ST_WARPS * 32, 1) attn_step_kernel(BiasAttnArgs a, int C) {
@@ -535,7 +541,7 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 1) attn_step_kernel(BiasAttnArg
             const int i = min(b + e, k1 - 1), v = i < nA ? i : first + i - nA;
             vf[e] = lane * 4 < dv && b + e < k1 ? *reinterpret_cast<const float4*>(V + (size_t)v * dv + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        if (!met) { __syncthreads(); met = true; }
+        if (!met) { st_meet(); met = true; }
 #pragma unroll
         for (int h = 0; h < NH; ++h) {
             float s[2], p[2];
@@ -576,7 +582,7 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 1) attn_step_kernel(BiasAttnArg
             }
         }
     }
-    if (!met) __syncthreads();
+    if (!met) st_meet();
     if (APPEND && rank == C - 1) {   // the CTA with the fewest keys: the newest one, by the warp that has had the fewest turns; both rows into the caches
         const float* vn = a.append.v + (size_t)r * a.ldq + (size_t)(g % Gv) * dv;
         if (warp == ST_WARPS - 1) {

@@ -80,3 +80,22 @@ def test_rows_that_other_kernels_write_are_not_read_as_constants(repo_root):
             assert params <= set(WEIGHTS.get(name, "").split()), f"{os.path.basename(path)}: {name} reads {params} as constants"
             assert ldg <= READ_ONLY, f"{os.path.basename(path)}: {name} reads {ldg} as constants"
     assert seen >= 60
+
+
+# conditions around a __syncthreads of one line, the same in every thread of a block: sizes and modes of the launch
+UNIFORM = {"S > 1", "MODE == SCAN_SSD || MODE == SCAN_HGRN2 || p.prepared == 0"}
+
+
+def test_block_barriers_are_reached_by_the_whole_block_at_one_place(repo_root):
+    """__syncthreads asks for all threads of the block at the same call. Warps that meet at different places use a barrier by number (bar.sync)."""
+    seen = 0
+    for path in glob.glob(os.path.join(repo_root, "llava-plus-codebase_b200", "csrc", "*.cu")):
+        src = re.sub(r"//[^\n]*|/\*.*?\*/", "", open(path).read(), flags=re.S)
+        for m in re.finditer(r"__syncthreads\(\)", src):
+            seen += 1
+            line = src[:m.start()].rsplit("\n", 2)
+            cond = re.search(r"\bif (?:constexpr )?\((.*)\)\s*(?:\{[^}]*)?$", line[-1])
+            if cond is None and re.search(r"\belse\s*(?:\{[^}]*)?$", line[-1]):
+                cond = re.search(r"\bif \((.*?)\) [^;]*;\s*$", line[-2])
+            assert cond is None or cond.group(1) in UNIFORM, f"{os.path.basename(path)}: a barrier behind if ({cond.group(1)})"
+    assert seen >= 50
