@@ -14,13 +14,21 @@
 namespace b2 {
 typedef __nv_bfloat16 bf16;
 
+// Makes room on the current device for an allocation of `need` bytes that was refused, out of what models keep only to be faster (seq_engine.cu);
+// false: there is not enough of that, and nothing was given back.
+bool give_back_spare(size_t need);
+
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
-    int alloc(size_t n) {
+    int alloc(size_t n, bool spare = false) {   // spare: nothing depends on it
         free();
         if (n == 0) return 0;
         cudaError_t e = cudaMalloc(&p, n);
+        if (e == cudaErrorMemoryAllocation && !spare) {
+            cudaGetLastError();
+            if (give_back_spare(n)) e = cudaMalloc(&p, n);
+        }
         if (e != cudaSuccess) {
             p = nullptr;
             cudaGetLastError();  // a refusal, not a fault: the next launch must not report it as its own

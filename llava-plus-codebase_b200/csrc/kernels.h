@@ -330,9 +330,11 @@ constexpr int LINEAR_SPLIT_MIN_ROWS = 9;
 bool linear_splits(const LinearArgs& a);
 size_t linear_split_bytes(int rows, int K);
 int linear_split_f32(const LinearArgs& a, cudaStream_t stream);
-// *other := 1 if a value of w is not a bf16 one (n % 4 == 0; other is not cleared); the high halves of fp32 values, which are the values then
-int bf16_values(const float* w, int64_t n, int* other, cudaStream_t stream);
-int high_halves(const float* w, int64_t n, void* out, cudaStream_t stream);
+// Matrices of fp32, on 16 bytes and in whole fours, listed in device memory: other[i] := 1 if a value of matrix i is not a bf16 one (other is not
+// cleared); out of each := the high halves of its values, which are the values then
+struct Fp32Matrix { const uint4* w = nullptr; int64_t fours = 0; uint2* out = nullptr; };
+int bf16_values(const Fp32Matrix* list, int n, int* other, cudaStream_t stream);
+int high_halves(const Fp32Matrix* list, int n, cudaStream_t stream);
 // A handful of rows on bf16 weights (linear_stream.cu): whether a call is one of those that stream their weights through registers
 constexpr int LINEAR_STREAM_MAX = 16;
 bool linear_streams(const LinearArgs& a);

@@ -298,18 +298,20 @@ int launch_tiles(const LinearArgs& a, const __nv_bfloat16* pa, const __nv_bfloat
 
 int pitch_of(int K) { return (K + 7) / 8 * 8; }
 
-__global__ void __launch_bounds__(256) bf16_values_kernel(const uint4* __restrict__ w, int64_t n4, int* __restrict__ other) {
+__global__ void __launch_bounds__(256) bf16_values_kernel(const Fp32Matrix* __restrict__ list, int* __restrict__ other) {
+    const Fp32Matrix m = list[blockIdx.y];
     int bad = 0;
-    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (int64_t)gridDim.x * 256) {
-        const uint4 v = w[i];
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < m.fours; i += (int64_t)gridDim.x * 256) {
+        const uint4 v = m.w[i];
         bad |= ((v.x | v.y | v.z | v.w) & 0xffffu) != 0;
     }
-    if (__syncthreads_or(bad) && threadIdx.x == 0) *other = 1;
+    if (__syncthreads_or(bad) && threadIdx.x == 0) other[blockIdx.y] = 1;
 }
-__global__ void __launch_bounds__(256) high_halves_kernel(const uint4* __restrict__ w, int64_t n4, uint2* __restrict__ out) {
-    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (int64_t)gridDim.x * 256) {
-        const uint4 v = w[i];
-        out[i] = make_uint2(v.x >> 16 | (v.y & 0xffff0000u), v.z >> 16 | (v.w & 0xffff0000u));
+__global__ void __launch_bounds__(256) high_halves_kernel(const Fp32Matrix* __restrict__ list) {
+    const Fp32Matrix m = list[blockIdx.y];
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < m.fours; i += (int64_t)gridDim.x * 256) {
+        const uint4 v = m.w[i];
+        m.out[i] = make_uint2(v.x >> 16 | (v.y & 0xffff0000u), v.z >> 16 | (v.w & 0xffff0000u));
     }
 }
 }  // namespace
@@ -342,15 +344,15 @@ int linear_split_f32(const LinearArgs& a, cudaStream_t st) {
     return 0;
 }
 
-int bf16_values(const float* w, int64_t n, int* other, cudaStream_t st) {
-    B2_CHECK_ARG(n % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0, "bf16_values: whole fours on 16 bytes");
-    bf16_values_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((n / 4 + 255) / 256, 8 * num_sms())), 256, 0, st>>>(reinterpret_cast<const uint4*>(w), n / 4, other);
+int bf16_values(const Fp32Matrix* list, int n, int* other, cudaStream_t st) {
+    B2_CHECK_ARG(list && other && n >= 1 && n <= 65535, "bf16_values: 1..65535 matrices");
+    bf16_values_kernel<<<dim3(2 * num_sms(), n), 256, 0, st>>>(list, other);
     B2_LAUNCH_CHECK();
     return 0;
 }
-int high_halves(const float* w, int64_t n, void* out, cudaStream_t st) {
-    B2_CHECK_ARG(n % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0, "high_halves: whole fours on 16 bytes");
-    high_halves_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((n / 4 + 255) / 256, 8 * num_sms())), 256, 0, st>>>(reinterpret_cast<const uint4*>(w), n / 4, reinterpret_cast<uint2*>(out));
+int high_halves(const Fp32Matrix* list, int n, cudaStream_t st) {
+    B2_CHECK_ARG(list && n >= 1 && n <= 65535, "high_halves: 1..65535 matrices");
+    high_halves_kernel<<<dim3(2 * num_sms(), n), 256, 0, st>>>(list);
     B2_LAUNCH_CHECK();
     return 0;
 }

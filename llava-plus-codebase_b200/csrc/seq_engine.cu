@@ -6,8 +6,11 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#include <algorithm>
 
 #include <map>
+#include <mutex>
+#include <vector>
 
 #include "engine.h"
 
@@ -79,10 +82,13 @@ struct SeqModel {
     DevBuf x, proj, act, y, gated, mixout, mixes, rp, wl1, wlog, ff, xn, tok, want;
     DevBuf lin_parts;                  // fp32 compute: bf16 parts of a product's operands (linear_split.cu)
     // fp32 compute: the matrices whose values all are bf16 ones (a bf16 checkpoint), as bf16 beside the fp32 ones: their products take half as many
-    // steps and no parts are made of them. Read by prompt portions only, and not from when a weight is set until the model is finalized again: the
-    // graph of a decode step goes on reading the fp32 matrices, which are set in place.
-    std::map<const void*, DevBuf> w16;
-    bool w16_valid = false, portion = false;
+    // steps and no parts are made of them. Spare memory, in one piece: read by prompt portions only (portion16: one is being issued), given back when a
+    // weight is set (until the model is finalized again) or when an allocation that something depends on finds no room. The graph of a decode step,
+    // and one that a caller captures, goes on reading the fp32 matrices, which are set in place. (w16_mem, w16, w16_users: under w16_lock)
+    DevBuf w16_mem;
+    std::map<const void*, const __nv_bfloat16*> w16;
+    int w16_users = 0, w16_device = 0;
+    bool portion16 = false;
     DevBuf scan_chunks;                // chunk states of a long prompt's recurrences (recurrent.cu)
     DevBuf attn_parts;                 // bf16 parts of the keys and values that a prompt portion sees (attention_split.cu); grows with the longest cache
     DevBuf a16;                        // bf16 copy of a GEMM's A operand (tensor-core path of the bf16 compute mode)
@@ -123,7 +129,7 @@ void alloc_spare(DevBuf& b, size_t bytes) {
     size_t free_bytes = 0, total = 0;
     if (bytes <= b.bytes) return;
     DevBuf n;
-    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || free_bytes < bytes + SPARE_RESERVE || n.alloc(bytes) != 0) {
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || free_bytes < bytes + SPARE_RESERVE || n.alloc(bytes, true) != 0) {
         cudaGetLastError();
         return;
     }
@@ -131,6 +137,42 @@ void alloc_spare(DevBuf& b, size_t bytes) {
     b.free();
     b = n;
 }
+
+// The models that hold bf16 copies of weights. A model whose prompt is being issued by another thread (w16_users) keeps its copies.
+std::mutex w16_lock;
+std::vector<SeqModel*> w16_holders;
+void free_bf16_weights(SeqModel& s) {   // under w16_lock
+    s.w16_mem.free();
+    s.w16.clear();
+    w16_holders.erase(std::remove(w16_holders.begin(), w16_holders.end(), &s), w16_holders.end());
+}
+void drop_bf16_weights(SeqModel& s) {
+    std::lock_guard<std::mutex> lk(w16_lock);
+    if (s.w16_mem.p == nullptr) return;
+    cudaDeviceSynchronize();   // calls in flight may use them
+    free_bf16_weights(s);
+}
+struct Bf16Weights {   // a prompt portion is being issued: its products read the copies, which stay until it is
+    SeqModel& s;
+    Bf16Weights(SeqModel& model, cudaStream_t st) : s(model) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        std::lock_guard<std::mutex> lk(w16_lock);
+        if (s.w16.empty()) return;
+        if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+            cudaGetLastError();
+            return;
+        }
+        s.portion16 = true;
+        ++s.w16_users;
+    }
+    ~Bf16Weights() {
+        if (!s.portion16) return;
+        std::lock_guard<std::mutex> lk(w16_lock);
+        s.portion16 = false;
+        --s.w16_users;
+    }
+    Bf16Weights(const Bf16Weights&) = delete;
+};
 
 int64_t numel(const int64_t* shape, int ndim) {
     int64_t n = 1;
@@ -221,9 +263,9 @@ struct Lin {  // one Linear call on the model's compute dtype
         if (norm != nullptr) a.norm = *norm;
         a.A16 = a16;
         a.parts = s.lin_parts.p; a.parts_bytes = s.lin_parts.bytes;
-        if (s.portion && s.w16_valid && K % 8 == 0) {
+        if (s.portion16 && K % 8 == 0) {
             const auto it = s.w16.find(W.p);
-            if (it != s.w16.end()) a.W16 = it->second.as<__nv_bfloat16>() + w_row0 * (size_t)K;
+            if (it != s.w16.end()) a.W16 = it->second + w_row0 * (size_t)K;
         }
         return a;
     }
@@ -1250,7 +1292,6 @@ static int seq_head(b2_model* m, const int32_t* index, int n, float* logits, int
 // one decode step over the slots [slot0, slot0 + B): kv->tok -> logits (m->logits) -> token selection, lengths += 1
 int seq_decode_launch(b2_model* m, b2_kv* kv, int B, int slot0, cudaStream_t st) {
     SeqModel& s = *m->seq;
-    s.portion = false;
     DecodeRows rows;   // (the row map is made where the rows are embedded: a launch between the graph's first and the next took 4.6 us of a step)
     rows.rm = RowMap{s.segs.as<SeqSeg>(), s.row_slot.as<int32_t>(), s.row_pos.as<int32_t>()};
     rows.len = kv->len_dev.as<int32_t>(); rows.sstate = kv->sstate.as<SampleState>(); rows.rows_state = kv->rows_dev.as<RowState>(); rows.slot0 = slot0;
@@ -1268,7 +1309,7 @@ int seq_decode_launch(b2_model* m, b2_kv* kv, int B, int slot0, cudaStream_t st)
 // ------------------------------------------------------------------------------------------------------------------
 int seq_set_weight(b2_model* m, const char* key, const void* ptr, const int64_t* shape, int ndim, int dt) {
     SeqModel& s = *m->seq;
-    s.w16_valid = false;
+    drop_bf16_weights(s);
     const int width = s.d.width, V = s.d.vocab, WD = s.w_dtype;
     const std::string k(key);
     if (k == "embed") { B2_TRY(want_shape(key, shape, ndim, V, width)); s.got[k] = 1; return put_tensor(s.embed, WD, (size_t)((V + 7) / 8 * 8) * width, 0, ptr, dt, (int64_t)V * width); }
@@ -1652,40 +1693,87 @@ static std::vector<std::string> required_of(const SeqLayerInfo& L, const b2_seq_
     return v;
 }
 
-// The fp32 matrices that prompt portions multiply with, where all their values are bf16 ones, once more as bf16
-static int copy_bf16_weights(SeqModel& s) {
-    if (!s.w16.empty()) cudaDeviceSynchronize();   // calls in flight may use the old ones
-    for (auto& e : s.w16) e.second.free();
-    s.w16.clear();
-    std::vector<const DevBuf*> mats;
+// The fp32 matrices that prompt portions multiply with, where all their values are bf16 ones, once more as bf16: as many as fit into an eighth of what
+// the device has free. (One pass of two launches over all of them and one allocation: a launch, a question for the free memory and an
+// allocation for each took half as long as finalizing the model did without.)
+static int copy_bf16_weights(SeqModel& s, int device) {
+    drop_bf16_weights(s);
+    std::vector<Fp32Matrix> mats;
+    const auto add = [&](const DevBuf& b) {
+        if (b.p == nullptr || b.bytes % 16 != 0) return;
+        Fp32Matrix m;
+        m.w = b.as<uint4>(); m.fours = (int64_t)(b.bytes / 16);
+        mats.push_back(m);
+    };
     for (const SeqWeights& W : s.w)
         for (const DevBuf* b : {&W.in_w, &W.o_w, &W.lproj_w, &W.lo_w, &W.r_w, &W.k_w, &W.v_w, &W.g_w, &W.w1, &W.w2, &W.ro_w, &W.up_w, &W.down_w, &W.qdg_w, &W.uk_w, &W.uv_w,
                                 &W.qfv_w, &W.router_w, &W.sgu_w, &W.sd_w, &W.uq_w, &W.ukx_w, &W.gla_w, &W.a2_w, &W.mem_w})
-            if (b->p != nullptr && b->bytes % 16 == 0) mats.push_back(b);
-    for (const DevBuf* b : {s.d.tied_head ? &s.embed : &s.head, &s.loop_in})
-        if (b->p != nullptr && b->bytes % 16 == 0) mats.push_back(b);
-    if (mats.empty()) return 0;
+            add(*b);
+    add(s.d.tied_head ? s.embed : s.head);
+    add(s.loop_in);
+    const size_t list_bytes = mats.size() * sizeof(Fp32Matrix), flag_bytes = mats.size() * sizeof(int);
+    if (mats.empty() || mats.size() > 65535 || s.lin_parts.bytes < list_bytes + flag_bytes) return 0;
     std::vector<int> other(mats.size(), 0);
-    DevBuf flags;
-    B2_TRY(flags.alloc(other.size() * 4));
-    cudaError_t e = cudaMemset(flags.p, 0, other.size() * 4);
-    int r = 0;
-    for (size_t i = 0; i < mats.size() && r == 0; ++i) r = bf16_values(mats[i]->as<float>(), (int64_t)(mats[i]->bytes / F4), flags.as<int>() + i, 0);
-    if (e == cudaSuccess) e = cudaMemcpy(other.data(), flags.p, other.size() * 4, cudaMemcpyDeviceToHost);
-    flags.free();
-    B2_TRY(r);
-    B2_CUDA_CHECK(e);
-    for (size_t i = 0; i < mats.size(); ++i) {
-        if (other[i] != 0) continue;
-        DevBuf c;
-        alloc_spare(c, mats[i]->bytes / 2);
-        if (c.p == nullptr) continue;
-        s.w16[mats[i]->p] = c;
-        B2_TRY(high_halves(mats[i]->as<float>(), (int64_t)(mats[i]->bytes / F4), c.p, 0));
+    DevBuf copies;
+    const DevBuf& list = s.lin_parts;   // (the parts' scratch, behind the calls in flight)
+    int* flags = reinterpret_cast<int*>(list.as<char>() + list_bytes);
+    std::vector<Fp32Matrix> taken;
+    const auto run = [&]() -> int {
+        B2_CUDA_CHECK(cudaDeviceSynchronize());
+        B2_CUDA_CHECK(cudaMemcpy(list.p, mats.data(), list_bytes, cudaMemcpyHostToDevice));
+        B2_CUDA_CHECK(cudaMemset(flags, 0, flag_bytes));
+        B2_TRY(bf16_values(list.as<Fp32Matrix>(), (int)mats.size(), flags, 0));
+        B2_CUDA_CHECK(cudaMemcpy(other.data(), flags, flag_bytes, cudaMemcpyDeviceToHost));
+        size_t free_bytes = 0, total = 0, bytes = 0;
+        B2_CUDA_CHECK(cudaMemGetInfo(&free_bytes, &total));
+        const auto size = [](const Fp32Matrix& m) { return ((size_t)m.fours * 8 + 255) / 256 * 256; };
+        for (size_t i = 0; i < mats.size(); ++i)
+            if (other[i] == 0 && bytes + size(mats[i]) <= free_bytes / 8 && free_bytes >= bytes + size(mats[i]) + SPARE_RESERVE) {
+                taken.push_back(mats[i]);
+                bytes += size(mats[i]);
+            }
+        if (bytes == 0 || copies.alloc(bytes, true) != 0) {
+            cudaGetLastError();
+            return 0;
+        }
+        size_t at = 0;
+        for (Fp32Matrix& m : taken) {
+            m.out = reinterpret_cast<uint2*>(copies.as<char>() + at);
+            at += size(m);
+        }
+        B2_CUDA_CHECK(cudaMemcpy(list.p, taken.data(), taken.size() * sizeof(Fp32Matrix), cudaMemcpyHostToDevice));
+        B2_TRY(high_halves(list.as<Fp32Matrix>(), (int)taken.size(), 0));
+        B2_CUDA_CHECK(cudaStreamSynchronize(0));
+        return 0;
+    };
+    const int r = run();
+    if (r != 0 || copies.p == nullptr) {
+        copies.free();
+        return r;
     }
-    B2_CUDA_CHECK(cudaStreamSynchronize(0));
-    s.w16_valid = true;
+    std::lock_guard<std::mutex> lk(w16_lock);
+    s.w16_mem = copies;
+    s.w16_device = device;
+    for (const Fp32Matrix& m : taken) s.w16[m.w] = reinterpret_cast<const __nv_bfloat16*>(m.out);
+    w16_holders.push_back(&s);
     return 0;
+}
+
+bool give_back_spare(size_t need) {
+    int device = 0;
+    size_t free_bytes = 0, total = 0, held = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) return false;
+    std::lock_guard<std::mutex> lk(w16_lock);
+    std::vector<SeqModel*> idle;
+    for (SeqModel* s : w16_holders)
+        if (s->w16_device == device && s->w16_users == 0) {
+            idle.push_back(s);
+            held += s->w16_mem.bytes;
+        }
+    if (idle.empty() || free_bytes + held < need) return false;
+    cudaDeviceSynchronize();   // calls in flight may use them
+    for (SeqModel* s : idle) free_bf16_weights(*s);
+    return true;
 }
 
 int seq_finalize(b2_model* m) {
@@ -1836,7 +1924,7 @@ int seq_finalize(b2_model* m) {
     alloc_spare(s.scan_chunks, chunk_floats * F4);
     if (s.d.compute != B2_COMPUTE_BF16) {
         alloc_spare(s.lin_parts, linear_split_bytes((int)R, s.a16_w) + ((size_t)64 << 20));   // (with room for the weights in blocks of rows)
-        B2_TRY(copy_bf16_weights(s));
+        B2_TRY(copy_bf16_weights(s, m->device));
     }
     return 0;
 }
@@ -1858,7 +1946,7 @@ void seq_model_free(b2_model* m) {
                     &s.rlogit, &s.moe_idx, &s.moe_w, &s.moe_pos, &s.moe_src, &s.moe_tile, &s.moe_h, &s.moe_a, &s.moe_y, &s.moe_a16, &s.zero_idx, &s.hin, &s.final_a, &s.loop_in, &s.cat,
                     &s.h2, &s.h1_16, &s.h2_16, &s.f16, &s.den, &s.embed_nw, &s.scan_chunks, &s.lin_parts, &s.attn_parts};
     for (DevBuf* b : bs) b->free();
-    for (auto& e : s.w16) e.second.free();
+    drop_bf16_weights(s);
     delete m->seq;
     m->seq = nullptr;
 }
@@ -2258,7 +2346,7 @@ int b2_append_tokens(b2_model* m, b2_kv* kv, int slot, const int32_t* tokens_hos
     for (int i = 0; i < n_want; ++i) B2_CHECK_ARG(want_host[i] >= 0 && want_host[i] < n, "b2_append_tokens: wanted index %d outside the %d tokens", want_host[i], n);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     B2_TRY(ws_enter(m, st));
-    s.portion = true;
+    const Bf16Weights weights16(s, st);
     B2_CUDA_CHECK(cudaMemcpyAsync(s.tok.p, tokens_host, (size_t)n * 4, cudaMemcpyHostToDevice, st));
     RowMap rm{s.segs.as<SeqSeg>(), s.row_slot.as<int32_t>(), s.row_pos.as<int32_t>()};
     // a slot that starts over begins from position 0 whatever its device-side length says

@@ -92,3 +92,27 @@ def test_a_refused_cache_leaves_the_calls_behind_it_alone():
         eng.new_kv(1, 60_000_000)      # 245 GB of keys
     assert torch.equal(prompt(eng, kv, toks), ref)
     model.invalidate_engine()
+
+
+def test_copies_of_weights_give_way_to_a_cache():
+    """True fp32 on weights that are bf16 values: their bf16 copies are given back for a cache that finds no room beside them."""
+    cfg = S.config([S.layer(S.win(8, 8, 128, 128, None, None, 0), {"kind": "dense", "ff": 16384, "limit": 1.25})], width=1024)
+    model, _ = S.build(cfg, torch.float32, max_batch=1, max_seq=64, max_rows=64)
+    eng, toks = model._ensure_engine(), S.tokens_for(cfg, 50)
+    first = eng.new_kv(1, 64)
+    ref = prompt(eng, first, toks)
+    seq = 20000
+    own = 8 * seq * (128 + 128) * 4
+    copies = 3 * 16384 * 1024 * 2
+    again = eng.new_kv(1, 64)
+    assert torch.equal(prompt(eng, again, toks), ref)
+    again.close()
+    with device_with(own - copies // 2):
+        kv = eng.new_kv(1, seq)
+        got = prompt(eng, kv, toks)
+        torch.cuda.synchronize()
+        kv.close()
+    assert S.err(got, ref) <= 2e-5      # three products of parts or six of them, fp32 sums in another order
+    assert torch.equal(prompt(eng, first, toks), got)
+    first.close()
+    model.invalidate_engine()
