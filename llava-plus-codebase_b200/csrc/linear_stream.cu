@@ -233,11 +233,7 @@ __global__ void __launch_bounds__(LS_WARPS * 32, 16 / LS_WARPS) linear_stream_tw
 
 // Whether a launch of `tiles` tiles of `units` units runs as one CTA of 16 warps an SM, not two of 8
 template <int NT>
-bool wide_ctas(int tiles, int units, bool side = false) {
-    // Side by side, few units: rounds of tiles that fill the SMs with 16 warps, and not with 8 (a first product of gated linear attention of width 2048 and its
-    // gated unit, 1025 tiles, 2 / 4 / 8 slots: a step of one layer 85 / 87 / 89 us with 8 warps, 81 / 84 / 86 with 16)
-    const int full = (tiles + num_sms() - 1) / num_sms() * num_sms(), full2 = (tiles + 2 * num_sms() - 1) / (2 * num_sms()) * 2 * num_sms();
-    if (side && units <= 20 && tiles >= 0.94 * full && tiles < 0.9 * full2) return true;
+bool wide_ctas(int tiles, int units) {
     // Two CTAs of 8 warps on an SM, or one of 16: the shorter one of the longest chains that a warp walks, in half units of weights. The end of a tile
     // (two barriers, the warps' sums) takes about half a unit's time, with more than 8 rows a whole one's; in a long stream of tiles whose last units
     // leave some of 8 warps idle (a head of 32000 outputs, K = 1536: 12 units), 16 warps were the faster form all the same. us a step, always 8 warps /
@@ -260,9 +256,18 @@ int launch_stream(const LinearArgs& a, cudaStream_t st) {
 template <int NT, bool A16, int FORM, bool RMS = false>
 int launch_two(const LinearArgs& a, const LinearArgs& b, cudaStream_t st) {
     const int tiles = (a.N + LS_N - 1) / LS_N + (FORM == LS_SIDE ? (b.N + LS_N / 2 - 1) / (LS_N / 2) : 0);
-    const int units = (a.K + LS_UNIT - 1) / LS_UNIT + (FORM == LS_SUM ? (b.K + LS_UNIT - 1) / LS_UNIT : 0);
-    if (wide_ctas<NT>(tiles, units, FORM == LS_SIDE)) B2_CUDA_CHECK(launch_pdl(linear_stream_two_kernel<NT, A16, FORM, RMS, 16>, dim3(std::min(tiles, num_sms())), dim3(512), 0, st, a, b));
-    else B2_CUDA_CHECK(launch_pdl(linear_stream_two_kernel<NT, A16, FORM, RMS, 8>, dim3(std::min(tiles, 2 * num_sms())), dim3(256), 0, st, a, b));
+    // A product and a gated unit side by side have tiles in plenty (3.6 rounds of two CTAs an SM at width 1024, 1024 outputs and a unit of 2560) and run as two
+    // CTAs of 8 warps, whose ends of tiles fall between each other's. us a layer in a chain of 3 to 12, 8 / 16 warps: gated linear attention of width 1024, 2 slots
+    // 19.8 / 22.6, of 2048, one slot 36.8 / 38.7, 8 slots 39.9 / 40.3, of 2304, 4 slots 45.2 / 48.0; window attention of 2560, one slot 45.6 / 48.4, of 4096, 16
+    // slots 101 / 103; of 135 measured (widths 1024 to 4096, 1 to 16 slots) 16 warps were ahead by more than 1 % in 3, by 2.4 % at most (1536, 4 slots 30.1 / 29.4).
+    if constexpr (FORM == LS_SUM) {
+        if (wide_ctas<NT>(tiles, (a.K + LS_UNIT - 1) / LS_UNIT + (b.K + LS_UNIT - 1) / LS_UNIT)) {
+            B2_CUDA_CHECK(launch_pdl(linear_stream_two_kernel<NT, A16, FORM, RMS, 16>, dim3(std::min(tiles, num_sms())), dim3(512), 0, st, a, b));
+            B2_LAUNCH_CHECK();
+            return 0;
+        }
+    }
+    B2_CUDA_CHECK(launch_pdl(linear_stream_two_kernel<NT, A16, FORM, RMS, 8>, dim3(std::min(tiles, 2 * num_sms())), dim3(256), 0, st, a, b));
     B2_LAUNCH_CHECK();
     return 0;
 }

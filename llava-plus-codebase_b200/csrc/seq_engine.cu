@@ -497,9 +497,11 @@ static LinearArgs glu_rows_args(const Lin& lin, const SeqLayerInfo& L, SeqWeight
 
 // A handful of rows through a parallel block: mixer and feed-forward read the same rows and add onto the same ones, so the feed-forward's two
 // products ride in the launches of the mixer's first and last (linear_stream.cu): two launches a layer fewer, each 1.5 to 3 us of start, ragged last
-// tiles and end. 48 steps of four mixed layers, width 2048 (us, before -> now): one slot 9773 -> 9436, 8 slots 12293 -> 12106. Wider layers spend their time
-// on the weights, and a sum's units then fit the SMs no better (a step of four layers, apart / together: width 2560, 4 slots 237 / 239; 3072, 12 slots
-// 377 / 390): one row rides always, more up to 8192 inputs of the sum.
+// tiles and end. us a layer in a chain of 3 to 12, apart / together: gated linear attention of width 1024, 2 slots 24.7 / 19.8, of 2048, one slot 42.5 / 36.8, 8
+// slots 42.5 / 39.9, of 4096, 4 slots 89.8 / 86.5; window attention of 3072, 8 slots 56.6 / 56.0. Up to 8 rows ride at every width (of 81 measured,
+// 1024 to 4096, 2 to 8 slots, 2 lost more than 1.5 %: 1536, 4 slots 28.8 / 30.1, 3072, 2 slots 61.4 / 63.0). More rows spend their time on the tiles' ends and products, and a
+// wide sum then fits the SMs no better (a step of four mixed layers: width 2048, 12 slots 213 / 207, 16 221 / 215; 2560 271 / 284, 297 / 310; 3072, 12 slots
+// 321 / 333): they ride up to 8192 inputs of the sum.
 struct RowFeedForward { LinearArgs up, down; };
 static LinearArgs gqa_first(const Lin& lin, const SeqLayerInfo& L, SeqWeights& W, const SubIn& in, int R) {
     const SeqModel& s = *lin.m->seq;
@@ -525,7 +527,7 @@ static bool row_feed_forward(const Lin& lin, const SeqLayerInfo& L, SeqWeights& 
     const bool gqa = d.type == B2_MIXER_GQA_ATTN;
     const int inner = gqa ? L.ng : L.pv;
     const LinearArgs first = gqa ? gqa_first(lin, L, W, in, R) : gla_first(lin, L, W, in, R);
-    if (R > 1 && inner + ff > 8192) return false;
+    if (R > 8 && inner + ff > 8192) return false;
     return first.A16 == f.up.A16 && linear_streams(first) && linear_streams(f.up) && linear_streams(f.down) &&
            linear_streams(lin.args(s.gated.as<float>(), inner, W.o_w, width, inner, target, width, R, LIN_NONE, alpha, 1));
 }

@@ -139,3 +139,11 @@ def test_one_row_normed_on_its_way_in(mixer, width, monkeypatch):
     cfg = config([dict(mix, mlp={"kind": "dense", "ff": 72, "limit": 7.0})], width=width, vocab=1003)
     w = O.random_weights(cfg, seed=6)
     both_ways(lambda: residuals(cfg, w, 5, 3), monkeypatch, bound(width, 72, 3 * 40, 2 * 40))
+
+
+@pytest.mark.parametrize("n", [2, 8, 9])
+def test_wide_sums_share_a_launch_up_to_eight_rows(n, monkeypatch):
+    """A sum of more than 8192 inputs: in one launch for 2 and 8 rows, in two for 9"""
+    cfg = config([dict(win(5, 1, 24, 40, 11, 3, 8), mlp={"kind": "dense", "ff": 8200, "limit": 7.0})], width=264, vocab=101)
+    w = O.random_weights(cfg, seed=5)
+    both_ways(lambda: residuals(cfg, w, n, 2), monkeypatch, bound(264, 8200, 5 * 40))
