@@ -1020,14 +1020,18 @@ static int seq_feed_forward(b2_model* m, const SeqLayerInfo& L, SeqWeights& W, c
     return moe_combine_f32(target, s.moe_y.as<float>(), width, pos, s.moe_w.as<float>(), R, top, width, alpha, st, h, width);
 }
 
-// the residual stream behind a layer run: by a kernel where the caller's buffer is memory of this device that it can write in 16-byte pieces
-static int keep_residual(float* dst, const float* x, size_t n, cudaStream_t st) {
+// The residual stream behind a layer run leaves by a kernel where the caller's buffer (rows of every run, n numbers each) is memory of this device that takes
+// 16-byte pieces; asked once a call
+static bool writes_rows(const float* out, size_t n) {
     cudaPointerAttributes attr;
     int dev = -1;
-    const bool here = n % 4 == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0 && cudaGetDevice(&dev) == cudaSuccess &&
-                      cudaPointerGetAttributes(&attr, dst) == cudaSuccess && attr.type == cudaMemoryTypeDevice && attr.device == dev;
-    if (here) return copy_f32(dst, x, n, st);
+    if (n % 4 != 0 || (reinterpret_cast<uintptr_t>(out) & 15) != 0) return false;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaPointerGetAttributes(&attr, out) == cudaSuccess) return attr.type == cudaMemoryTypeDevice && attr.device == dev;
     cudaGetLastError();
+    return false;
+}
+static int keep_residual(float* dst, const float* x, size_t n, bool by_kernel, cudaStream_t st) {
+    if (by_kernel) return copy_f32(dst, x, n, st);
     B2_CUDA_CHECK(cudaMemcpyAsync(dst, x, n * F4, cudaMemcpyDeviceToDevice, st));
     return 0;
 }
@@ -1050,6 +1054,7 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
     const bool direct = pre || parallel;   // a sublayer's last product adds residual_mult * its output onto x
     const float rm = s.d.residual_mult;
     float* xn = s.xn.as<float>();
+    const bool by_kernel = resid_out != nullptr && writes_rows(resid_out, (size_t)R * width);
     const float* post = nullptr;   // sandwich block: weight of the sublayer output in `mix` that has not joined x yet
     for (size_t ri = 0; ri < s.runs.size(); ++ri) {
         const size_t li = (size_t)s.runs[ri].layer;
@@ -1104,7 +1109,7 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
                 if (early) B2_TRY(gelu_down(m, L, W, x, rm, 1, R, st));
                 else if (d.ff > 0 && ride == nullptr) B2_TRY(seq_feed_forward(m, L, W, in2, x, rm, 1, R, st));
                 if (resid_out != nullptr)
-                    B2_TRY(keep_residual(resid_out + ri * (size_t)R * width, x, (size_t)R * width, st));
+                    B2_TRY(keep_residual(resid_out + ri * (size_t)R * width, x, (size_t)R * width, by_kernel, st));
                 continue;
             }
             // (the normed rows of a prompt leave rounded as well: what the products, and the experts' gather, read)
@@ -1140,7 +1145,7 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
                 post = nullptr;
             }
             if (resid_out != nullptr)
-                B2_TRY(keep_residual(resid_out + ri * (size_t)R * width, x, (size_t)R * width, st));
+                B2_TRY(keep_residual(resid_out + ri * (size_t)R * width, x, (size_t)R * width, by_kernel, st));
             continue;
         }
         if (pass >= 0) B2_TRY(rms_scalar_f32(x, nullptr, nullptr, pass_add, pass_vec, nullptr, R, width, eps, st));
@@ -1226,7 +1231,7 @@ static int seq_forward(b2_model* m, b2_kv* kv, int R, int nseg, int slot, int ct
             B2_TRY(layernorm_add_f32(x, mix, W.norm2.as<float>(), W.norm2_b.as<float>(), R, width, eps, st));
         }
         if (resid_out != nullptr)
-            B2_TRY(keep_residual(resid_out + ri * (size_t)R * width, x, (size_t)R * width, st));
+            B2_TRY(keep_residual(resid_out + ri * (size_t)R * width, x, (size_t)R * width, by_kernel, st));
     }
     return 0;
 }
