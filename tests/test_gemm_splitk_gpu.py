@@ -1,5 +1,8 @@
 """The GEMM whose K is cut over a cluster (csrc/gemm_splitk.cu) against 64-bit products of the same bf16 operands, at the edges of its tiles and
 k-slices, with every epilogue, in every plan and through the rule that chooses one."""
+import json
+import re
+
 import pytest
 import torch
 import torch.nn.functional as F
@@ -38,10 +41,25 @@ def test_split_k(M, N, K, act, f32, bias, residual, plan):
     assert bool(((out - ref).abs() <= tol).all()), float(((out - ref).abs() - tol).max())
 
 
-@pytest.mark.parametrize("M,N,K,act,f32,bias,residual", [(1154, 1024, 4096, 0, 0, 1, 1), (1027, 1000, 4104, 1, 0, 1, 0), (16, 5120, 1544, 0, 1, 0, 0), (500, 1160, 2568, 2, 0, 1, 1)])
+@pytest.mark.parametrize("M,N,K,act,f32,bias,residual", [(1154, 1024, 4096, 0, 0, 1, 1), (1153, 1000, 4104, 1, 0, 1, 0), (16, 5120, 2568, 0, 1, 0, 0), (500, 1160, 2568, 2, 0, 1, 1)])
 def test_split_in_three(M, N, K, act, f32, bias, residual):
     """Tiles of 256 columns (the first two) and of 128 whose column groups don't divide by three, through the rule."""
     test_split_k(M, N, K, act, f32, bias, residual, 0)
+
+
+@pytest.mark.parametrize("M,N,K,bn", [(1154, 1024, 4096, 256), (1153, 1000, 4104, 256), (16, 5120, 2568, 128), (500, 1160, 2568, 128)])
+def test_the_rule_takes_three_slices_there(M, N, K, bn, tmp_path):
+    """The shapes of the test above are those of the plans that it means: no plan number names these."""
+    A, W = (torch.zeros(n, K, device="cuda", dtype=torch.bfloat16) for n in (M, N))
+    product(A, W, None, None, False, 0, 0)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        product(A, W, None, None, False, 0, 0)
+        torch.cuda.synchronize()
+    prof.export_chrome_trace(str(tmp_path / "trace.json"))
+    ran = [e for e in json.load(open(tmp_path / "trace.json"))["traceEvents"] if e.get("cat") == "kernel" and "gemm" in e["name"]]
+    assert len(ran) == 1 and re.search(r"gemm_splitk_kernel<(\(int\))?%d\b" % bn, ran[0]["name"]), [e["name"] for e in ran]
+    grid = ran[0]["args"]["grid"]
+    assert grid[0] * grid[1] * grid[2] == 3 * -(-M // 128) * -(-N // bn)
 
 
 def test_plans_that_do_not_fit_are_refused():
