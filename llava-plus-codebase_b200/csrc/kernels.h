@@ -608,7 +608,8 @@ int matrix_memory_f32(const MemoryArgs& a, cudaStream_t stream);
 // ---- attention with unit-RMS q/k, query temperature, tanh soft-cap and a bucketed distance bias (attention_bias.cu) -----
 enum { MASK_CAUSAL = 0, MASK_WINDOW = 1, MASK_CHUNK = 2 };
 // One row per slot whose queries and newest key are still as the projection left them: the attention norms and turns them itself (as RotateArgs do it), attends
-// to that key and its value and appends both to the caches (attn_bias_appends says where)
+// to that key and its value and appends both to the caches. For calls that attn_bias_appends accepts, with norms over a head's own entries (not over all
+// heads of a row) and values that are not turned.
 struct StepAppend {
     const float *k = nullptr, *v = nullptr;       // [rows, G*dk], [rows, Gv*dv], both of pitch ldq; null: they are in the caches
     const float *q_norm = nullptr, *k_norm = nullptr; float eps = 0.f;   // weights of the heads' norm over dk, or null
@@ -656,7 +657,7 @@ constexpr int ATTN_SPLIT_MIN_ROWS = 16, ATTN_SPLIT_MIN_KEYS = 40;
 bool attn_split_fits(const BiasAttnArgs& a);                       // the call runs on the tensor cores
 size_t attn_split_bytes_per_key(int G, int Gv, int dk, int dv);    // scratch per visible key position
 int attn_split_f32(const BiasAttnArgs& a, cudaStream_t stream);
-int attn_bias_f32(const BiasAttnArgs& a, cudaStream_t stream);
-bool attn_bias_appends(const BiasAttnArgs& a);   // whether a.append is served for a call of these sizes     // causal softmax attention of every row against its slot's cache
+int attn_bias_f32(const BiasAttnArgs& a, cudaStream_t stream);     // causal softmax attention of every row against its slot's cache
+bool attn_bias_appends(const BiasAttnArgs& a);                     // whether a call of these sizes takes a.append
 
 }  // namespace b2
