@@ -334,11 +334,6 @@ constexpr int DA_STAGES = 2, DA_CTAS = 7;         // per SM: registers and share
 constexpr int DA_TILE = DA_KEYS * DA_D * 2;
 constexpr int DA_SMEM = DA_STAGES * 2 * DA_TILE + 128 /*align*/;
 
-__device__ __forceinline__ void da_bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
-
 struct DecodeAttnParams {
     const __nv_bfloat16* qkv;
     __nv_bfloat16* kcache;
@@ -390,8 +385,8 @@ __global__ void __launch_bounds__(DA_THREADS, DA_CTAS) decode_attn_kernel(Decode
         const uint32_t bytes = min(n - t * DA_KEYS, DA_KEYS) * DA_D * 2;
         const size_t at = cbase + (size_t)(k_begin + t * DA_KEYS) * DA_D;
         mbar_arrive_expect_tx(&s_full[t % DA_STAGES], 2 * bytes);
-        da_bulk_g2s(dst, p.kcache + at, bytes, &s_full[t % DA_STAGES]);
-        da_bulk_g2s(dst + DA_TILE, p.vcache + at, bytes, &s_full[t % DA_STAGES]);
+        bulk_g2s(dst, p.kcache + at, bytes, &s_full[t % DA_STAGES]);
+        bulk_g2s(dst + DA_TILE, p.vcache + at, bytes, &s_full[t % DA_STAGES]);
     };
     if (tid == 0)
         for (int t = 0; t < min(tiles, DA_STAGES); ++t) load(t);

@@ -74,14 +74,6 @@ __device__ __forceinline__ void grid_sync(unsigned int* counter, unsigned int ta
     cons_sync();
 }
 
-// 1-D TMA bulk copy global -> shared, completion (bytes) signalled on an mbarrier
-__device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(smem_dst)),
-                 "l"(gsrc), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-
 // One GEMV phase as seen by a CTA. Output units (rows; SwiGLU: channels = a gate row + its up row) are cut into
 // gridDim.x contiguous ranges that differ by at most ONE unit, so every SM streams the same number of bytes to
 // within 1-4% (a split in whole 8-row blocks left +-1 block = 6-16% skew per phase in front of every grid barrier:

@@ -92,13 +92,6 @@ __device__ __forceinline__ unsigned long long sk_now() {
 }
 #define SK_STAMP(slot) do { if (ep.trace != nullptr) ep.trace[(size_t)blockIdx.x * 16 + (slot)] = sk_now(); } while (0)
 
-// 1-D bulk copy global -> shared, completion (bytes) on an mbarrier
-__device__ __forceinline__ void sk_bulk_g2s(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem_dst)),
-                 "l"(gsrc), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 2, 128;" ::: "memory"); }
 
 // CTA that owns global k-block unit u when `total` units are cut into `grid` ranges [total*c/grid, total*(c+1)/grid)
@@ -266,7 +259,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                     asm volatile("fence.proxy.async;" ::: "memory");  // other CTAs' generic-proxy stores -> async-proxy reads
                     mbar_arrive_expect_tx(fix_bar, (uint32_t)nseg * (BN * SK_BM * 4));
                     for (int sidx = 0; sidx < nseg; ++sidx)
-                        sk_bulk_g2s(smem + (size_t)sidx * (BN * SK_BM * 4), slot0 + (size_t)sidx * (BN * SK_BM), BN * SK_BM * 4, fix_bar);
+                        bulk_g2s(smem + (size_t)sidx * (BN * SK_BM * 4), slot0 + (size_t)sidx * (BN * SK_BM), BN * SK_BM * 4, fix_bar);
                 }
                 if (et == 0 && t == t_last) SK_STAMP(6);  // partial published / finaliser elected
                 if (et == 0 && finalize) ++n_final;

@@ -190,10 +190,6 @@ __global__ void __launch_bounds__(SB_THREADS, 2) sb_prepare_kernel(ScanArgs a, B
     if (tid == 0) p.bad_in[bh] = any;
 }
 
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
 // 128 columns of V, transposed: a row of 64 tokens per column. Returns whether a value is one that the parts do not hold.
 __device__ __forceinline__ bool put_values(const ScanArgs& a, uint8_t* sv, size_t row0, int nt, int h, int col0) {
     bool bad = false;
@@ -252,7 +248,7 @@ __global__ void __launch_bounds__(SB_THREADS, 2) sb_states_kernel(ScanArgs a, Bl
     const int t0 = p.t0 + b * SB_TOK, nt = min(SB_TOK, p.t0 + p.n - t0), col0 = ct * 128;
     if (threadIdx.x == 0) {
         mbar_arrive_expect_tx(full, Cfg::K);
-        bulk_load(sk, p.k + bh * Cfg::K, Cfg::K, full);
+        bulk_g2s(sk, p.k + bh * Cfg::K, Cfg::K, full);
     }
     const bool bad = put_values(a, sv, (size_t)sg.row0 + t0, nt, h, col0);
     fence_proxy_async();
@@ -367,7 +363,7 @@ __global__ void __launch_bounds__(SB_THREADS, 2) sb_output_kernel(ScanArgs a, Bl
     for (int blk = 0; blk <= KB; ++blk) {
         if (threadIdx.x == 0) {   // (the products that read it last are done)
             mbar_arrive_expect_tx(full, SB_OUT_B);
-            bulk_load(sb, blk < KB ? p.q + (bh * KB + blk) * SB_OUT_B : p.a + bh * SB_OUT_B, SB_OUT_B, full);
+            bulk_g2s(sb, blk < KB ? p.q + (bh * KB + blk) * SB_OUT_B : p.a + bh * SB_OUT_B, SB_OUT_B, full);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
