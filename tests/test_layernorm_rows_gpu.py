@@ -1,4 +1,4 @@
-"""bf16 LayerNorm (csrc/norms.cu) in both of its register forms, at row counts around whole blocks and far above one wave of them."""
+"""bf16 LayerNorm (csrc/norms.cu) in both of its register forms, at row counts around whole blocks of four and above one wave of them."""
 import pytest
 import torch
 
@@ -6,7 +6,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("cols", [256, 1024, 1280, 2048])
-@pytest.mark.parametrize("rows", [1, 3, 2959, 2960, 2961, 5923, 9232])
+@pytest.mark.parametrize("rows", [1, 3, 4, 5, 577, 9232, 9233])
 def test_layernorm_rows(rows, cols):
     from llava import _b2
 
