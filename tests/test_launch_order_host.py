@@ -99,3 +99,17 @@ def test_block_barriers_are_reached_by_the_whole_block_at_one_place(repo_root):
                 cond = re.search(r"\bif \((.*?)\) [^;]*;\s*$", line[-2])
             assert cond is None or cond.group(1) in UNIFORM, f"{os.path.basename(path)}: a barrier behind if ({cond.group(1)})"
     assert seen >= 50
+
+
+def test_pairs_leave_together_behind_the_release_of_tensor_memory(repo_root):
+    """Tensor memory of a CTA pair (cta_group::2) is released by both CTAs. If one could exit in between, the next kernel's CTA on its SM would allocate
+    while the other's release is under way."""
+    seen = 0
+    for path in glob.glob(os.path.join(repo_root, "llava-plus-codebase_b200", "csrc", "*.cu")):
+        for name, body in kernels(open(path).read()):
+            free = re.search(r"\btmem_dealloc_2sm\(", body)
+            if free is None:
+                continue
+            seen += 1
+            assert re.search(r"\bcluster_sync\(\)", body[free.end():]), f"{os.path.basename(path)}: {name} lets a CTA go before its pair has released"
+    assert seen >= 1
