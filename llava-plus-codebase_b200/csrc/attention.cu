@@ -326,6 +326,8 @@ rope_kv_write_kernel(__nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict_
 // a time with an online softmax each -> now, at the split counts then and now: 8 x 32 heads, 800 keys 24.5 -> 23.1; 16, 110 12.0 -> 8.5;
 // 32, 110 18.3 -> 13.2; 32, 800 76.3 -> 68.3; 64, 800 139.5 -> 127.0; 128, 300 127.6 -> 96.6; 8 x 40, 2000 75.2 -> 55.2. Rings of 2 / 3 / 4
 // stages of 32 rows (6 / 4 / 3 CTAs): 14.6 / 15.9 / 17.4 at 32, 110 and 74 / 66 / 77 at 32, 800; 3 stages of 16 12.8 and 69.5.
+// The merge asks for eight splits at a time: as a loop unrolled by eight, two to seven splits were a chain of round trips (8 x 32 heads, 100 keys in four
+// 9.4 -> 8.0; 2 x 32, 100 in seven 10.2 -> 6.7).
 // ------------------------------------------------------------------------------------------------
 constexpr int DA_D = 128;
 constexpr int DA_THREADS = 128;
@@ -537,16 +539,33 @@ __global__ void __launch_bounds__(DA_THREADS, DA_CTAS) decode_attn_kernel(Decode
     if (s_last) {
         __threadfence();
         const float* pb = p.partial + (size_t)bh * p.nsplit * (DA_D + 2);
+        // eight splits at a time, whatever their number: what a group reads is asked for at once, where the rest of a loop unrolled by eight was a chain
+        constexpr int U = 8;
         float m_all = -INFINITY;
-#pragma unroll 8
-        for (int s = 0; s < p.nsplit; ++s) m_all = fmaxf(m_all, __ldcg(pb + (size_t)s * (DA_D + 2) + DA_D));
+        for (int s0 = 0; s0 < p.nsplit; s0 += U) {
+            float ms[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) ms[u] = s0 + u < p.nsplit ? __ldcg(pb + (size_t)(s0 + u) * (DA_D + 2) + DA_D) : -INFINITY;
+#pragma unroll
+            for (int u = 0; u < U; ++u) m_all = fmaxf(m_all, ms[u]);
+        }
         float l_all = 0.f, o_all = 0.f;
-#pragma unroll 8
-        for (int s = 0; s < p.nsplit; ++s) {  // independent loads: unrolled so they overlap instead of chaining
-            const float ms = __ldcg(pb + (size_t)s * (DA_D + 2) + DA_D);
-            const float w = (ms == -INFINITY) ? 0.f : exp2f(ms - m_all);
-            l_all += __ldcg(pb + (size_t)s * (DA_D + 2) + DA_D + 1) * w;
-            o_all += __ldcg(pb + (size_t)s * (DA_D + 2) + tid) * w;
+        for (int s0 = 0; s0 < p.nsplit; s0 += U) {
+            float ms[U], ls[U], os[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const float* ps = pb + (size_t)(s0 + u) * (DA_D + 2);
+                const bool there = s0 + u < p.nsplit;
+                ms[u] = there ? __ldcg(ps + DA_D) : -INFINITY;
+                ls[u] = there ? __ldcg(ps + DA_D + 1) : 0.f;
+                os[u] = there ? __ldcg(ps + tid) : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const float w = ms[u] == -INFINITY ? 0.f : exp2f(ms[u] - m_all);
+                l_all += ls[u] * w;
+                o_all += os[u] * w;
+            }
         }
         p.out[(size_t)b * hd + head * DA_D + tid] = __float2bfloat16_rn(o_all / l_all);
         if (tid == 0) p.counters[bh] = 0;  // self-reset for the next launch

@@ -164,16 +164,20 @@ bool use_skinny(const b2_kv* kv, int B) {
 }
 
 int decode_nsplit(int B, int H, int max_seq) {
-    // Split-KV factor of the multi-kernel decode step: as many splits as fill one wave of resident CTAs (seven an SM, 1036), with room for at least 128 keys
-    // each: a split's partial sums and the merge cost 2 us or more. us with 1 / 2 / 3 / 4 / 8 splits: 2 requests of 32 heads, 100 keys 5.5 / 7.1 / 7.2 / 7.5; 4, 800
-    // 24.3 / 18.5 / 18.9 / 16.2 / 14.3; 8, 800 31.0 / 23.2 / 23.3 / 23.1 / 23.8; 16, 800 37.4 / 37.3 / 40.1 / 39.4; 32, 110 13.2 / 17.4 / 18.2 / 21.4; 64, 800 127 / 129 / 130.
+    // Split-KV factor of the multi-kernel decode step (fixed at capture, so by the cache's capacity and not by the lengths). As many splits as fill one wave of
+    // resident CTAs (seven an SM, 1036), but six at most, of 64 keys of capacity or more: from 96 pairs on more of them only add partial sums. Few pairs (48
+    // and less) gain from up to 16, of 128 keys. Where the pairs are a little more than a wave, its rest would be a second one of lone CTAs: two splits, if
+    // contexts can be long. us a step of four layers of the 7B width, cold caches, 1 / 2 / 3 / 6 / 10 splits: 3 requests, 1000 keys 545 / 508 / 492 / 483 / 489, 1800
+    // 627 / 553 / 525 / 507 / 512; 4, 1800 639 / 568 / 544 / 534 / 552; 16, 1000 603 / 574 / 582 / 582; 20, 600 533 / 565 / 546, 1800 769 / 842 / 762; 32, 1800 972 / 985 / 986.
+    // 1 / 2 splits: 33 (1056 pairs), 64 keys 440 / 460, 600 651 / 645, 1800 1136 / 1039; 44, 250 550 / 555, 1800 1255 / 1168; 48, 600 726 / 735, 1800 1286 / 1266.
     const char* e = getenv("B2_DECODE_NSPLIT");
     if (e != nullptr && atoi(e) >= 1) return atoi(e) > 32 ? 32 : atoi(e);
-    const int cap = decode_attn_ctas_per_sm() * num_sms();
-    int n = cap / (B * H);
-    if (n > 16) n = 16;
-    if (n > max_seq / 128) n = max_seq / 128;
-    return n < 1 ? 1 : n;
+    const int cap = decode_attn_ctas_per_sm() * num_sms(), pairs = B * H;
+    if (pairs > cap && 10 * pairs < 14 * cap && max_seq >= 1024) return 2;
+    const int most = std::max(6, std::min(16, 512 / pairs));
+    int n = std::min(cap / pairs, most);
+    if (n > 6) n = std::max(6, std::min(n, max_seq / 128));
+    return std::max(1, std::min(n, max_seq / 64));
 }
 
 // ------------------------------------------------------------------------------------------------------

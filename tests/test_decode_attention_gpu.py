@@ -44,3 +44,8 @@ def test_decode_attention_tiles(nsplit, growing):
             # row n is written, and nothing else
             assert torch.equal(vc[b, :, n], qkv[b, 2]) and torch.equal(kc[b, :, n, 32:64], qkv[b, 1, :, 32:64])
             assert torch.equal(kc[b, :, :n], kc0[b, :, :n]) and torch.equal(kc[b, :, n + 1:], kc0[b, :, n + 1:])
+
+
+@pytest.mark.parametrize("nsplit", [7, 8, 9])
+def test_splits_meet_in_groups_of_eight(nsplit):
+    test_decode_attention_tiles(nsplit, True)
