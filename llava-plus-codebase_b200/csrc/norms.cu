@@ -12,8 +12,11 @@ constexpr int kWarpsPerBlock = 4;
 // cols % 256 == 0 (each lane handles cols/32 elements in 16 B vectors); cols <= 256 * VEC. Weight and bias are asked for with the row: between two products the
 // kernel is bound by its chain of loads and sums (577 rows of 1024, from one kernel's end to the next: 3.6 us with the weights behind the statistics and
 // registers for 2048 columns at every width, now 2.6; back to back 9232 rows 10.5 -> 8.9, 36928 32.8 -> 27.0). Several rows a warp with the weights kept lost: 18464 rows 18.0 -> 35.4 us, 36928 32.8 -> 65.9.
-template <int VEC>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+// Rows wider than 1024 have a kernel for each width, so that no registers stand for columns that are not there, and 2048 columns spill a few for a fourth CTA on the
+// SM: 18464 rows of 1280 / 1536 / 1792 / 2048 20.4 / 26.7 / 28.3 / 29.7 us with the weights behind the statistics, 24.7 / 26.8 / 28.8 / 30.8 with them in front in
+// registers for 2048 columns, 18.4 / 22.5 / 24.8 / 29.2 now.
+template <int VEC, int CTAS = 1>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, CTAS)
 layernorm_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma,
                  const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y, int rows, int cols,
                  float eps) {
@@ -175,7 +178,8 @@ int layernorm_bf16(const void* x, const void* gamma, const void* beta, void* y, 
     B2_CHECK_ARG(rows > 0 && cols > 0 && cols % 256 == 0 && cols <= 2048,
                  "layernorm: cols must be a multiple of 256 and <= 2048 (cols=%d rows=%d)", cols, rows);
     const int grid = (rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
-    B2_CUDA_CHECK(launch_pdl(cols <= 1024 ? layernorm_kernel<4> : layernorm_kernel<8>, dim3(grid), dim3(kWarpsPerBlock * 32), 0, stream,
+    const auto kernel = cols <= 1024 ? layernorm_kernel<4> : cols == 1280 ? layernorm_kernel<5> : cols == 1536 ? layernorm_kernel<6> : cols == 1792 ? layernorm_kernel<7> : layernorm_kernel<8, 4>;
+    B2_CUDA_CHECK(launch_pdl(kernel, dim3(grid), dim3(kWarpsPerBlock * 32), 0, stream,
         reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(gamma),
         reinterpret_cast<const __nv_bfloat16*>(beta), reinterpret_cast<__nv_bfloat16*>(y), rows, cols, eps));
     B2_LAUNCH_CHECK();

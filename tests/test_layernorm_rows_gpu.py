@@ -1,11 +1,11 @@
-"""bf16 LayerNorm (csrc/norms.cu) in both of its register forms, at row counts around whole blocks of four and above one wave of them."""
+"""bf16 LayerNorm (csrc/norms.cu) in all of its register forms, at row counts around whole blocks of four and above one wave of them."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("cols", [256, 1024, 1280, 2048])
+@pytest.mark.parametrize("cols", [256, 1024, 1280, 1536, 1792, 2048])
 @pytest.mark.parametrize("rows", [1, 3, 4, 5, 577, 9232, 9233])
 def test_layernorm_rows(rows, cols):
     from llava import _b2
