@@ -343,7 +343,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     }
     // The pair's TMEM is given back by both CTAs together, so neither leaves its SM to the next kernel before both have done so: else a CTA that comes in on the
     // one SM may take TMEM while the other's half is still to come. (Prompts of 512 rows at the 7B width, the one size where the next kernel asks for half of
-    // the columns between two pair kernels: without this barrier two of three runs of 65 of them stood still for good, none of nine with it. No time.)
+    // the columns between two pair kernels: without this barrier two of three runs of 65 of them stood still for good, none of nine with it. 0.25 us a launch.)
     cluster_sync();
 }
 
