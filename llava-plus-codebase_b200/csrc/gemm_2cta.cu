@@ -167,6 +167,9 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         }
         fence_barrier_init();
     }
+    // The allocation below is the pair's: both CTAs must be there, and one may start long before the other (without this barrier prompts of 512 rows at the 7B width,
+    // whose pair kernels come in while the last CTAs of tile GEMMs leave, stood still for good within 300 of them; none of 7200 did with it)
+    cluster_sync();
     if (warp == 1) tmem_alloc_2sm(tmem_slot, P_TMEM_COLS);  // collective over the pair: one warp in each CTA
     tc_fence_before();
     cluster_sync();  // barriers initialised and TMEM allocated in both CTAs before anyone signals across
@@ -341,10 +344,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         tc_fence_after();
         tmem_dealloc_2sm(tmem_base, P_TMEM_COLS);
     }
-    // The pair's TMEM is given back by both CTAs together, so neither leaves its SM to the next kernel before both have done so: else a CTA that comes in on the
-    // one SM may take TMEM while the other's half is still to come. (Prompts of 512 rows at the 7B width, the one size where the next kernel asks for half of
-    // the columns between two pair kernels: without this barrier two of three runs of 65 of them stood still for good, none of nine with it. 0.25 us a launch.)
-    cluster_sync();
+    cluster_sync();  // so is the release: neither CTA leaves its SM to the next kernel before both have released
 }
 
 template <int ACT, bool F32 = false>

@@ -101,15 +101,17 @@ def test_block_barriers_are_reached_by_the_whole_block_at_one_place(repo_root):
     assert seen >= 50
 
 
-def test_pairs_leave_together_behind_the_release_of_tensor_memory(repo_root):
-    """Tensor memory of a CTA pair (cta_group::2) is released by both CTAs. If one could exit in between, the next kernel's CTA on its SM would allocate
-    while the other's release is under way."""
+def test_pairs_are_together_while_they_take_and_release_tensor_memory(repo_root):
+    """Tensor memory of a CTA pair (cta_group::2) is taken and released by both CTAs: the pair meets in front of the one, as a CTA may start long before its
+    peer, and behind the other, as one may leave before its peer."""
     seen = 0
     for path in glob.glob(os.path.join(repo_root, "llava-plus-codebase_b200", "csrc", "*.cu")):
         for name, body in kernels(open(path).read()):
-            free = re.search(r"\btmem_dealloc_2sm\(", body)
-            if free is None:
+            take, free = re.search(r"\btmem_alloc_2sm\(", body), re.search(r"\btmem_dealloc_2sm\(", body)
+            if take is None:
                 continue
             seen += 1
-            assert re.search(r"\bcluster_sync\(\)", body[free.end():]), f"{os.path.basename(path)}: {name} lets a CTA go before its pair has released"
+            meet = r"\bcluster_sync\(\)"
+            assert re.search(meet, body[:take.start()]), f"{os.path.basename(path)}: {name} takes tensor memory before its pair has met"
+            assert re.search(meet, body[free.end():]), f"{os.path.basename(path)}: {name} lets a CTA go before its pair has released"
     assert seen >= 1
