@@ -168,7 +168,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         fence_barrier_init();
     }
     // The allocation below is the pair's: both CTAs must be there, and one may start long before the other (without this barrier prompts of 512 rows at the 7B width,
-    // whose pair kernels come in while the last CTAs of tile GEMMs leave, stood still for good within 300 of them; none of 7200 did with it)
+    // whose pair kernels come in while the last CTAs of tile GEMMs leave, stood still for good within 300 of them; none of 14400 did with it)
     cluster_sync();
     if (warp == 1) tmem_alloc_2sm(tmem_slot, P_TMEM_COLS);  // collective over the pair: one warp in each CTA
     tc_fence_before();
@@ -344,7 +344,6 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         tc_fence_after();
         tmem_dealloc_2sm(tmem_base, P_TMEM_COLS);
     }
-    cluster_sync();  // so is the release: neither CTA leaves its SM to the next kernel before both have released
 }
 
 template <int ACT, bool F32 = false>
